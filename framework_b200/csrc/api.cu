@@ -7,6 +7,7 @@
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <mutex>
@@ -62,8 +63,8 @@ float powi_f32(float x, uint32_t n) {
 
 // Largest M*N*K*batch for which the two gradient products of a backward call are issued side by side.
 double overlap_work_limit() {
-    const char *v = getenv("MNI_B200_BWD_OVERLAP_WORK");
-    return v && *v ? atof(v) : 4.0e9;   // measured: helps up to the attention-shaped products (1.6e9), neutral beyond
+    const char *v = env_value("MNI_B200_BWD_OVERLAP_WORK");
+    return v ? atof(v) : 4.0e9;   // measured: helps up to the attention-shaped products (1.6e9), neutral beyond
 }
 
 // Row counts up to which the streaming kernels beat the tensor path (measured at K = N = 4096 with a weight
@@ -71,10 +72,7 @@ double overlap_work_limit() {
 // 17.0 at 12).  The forward's limit depends on which of its two kernels can run: skinny_fwd_row_limit.
 constexpr int64_t kSkinnyDxRows = 5, kSkinnyDwRows = 8;
 
-bool env_flag(const char *name, int dflt) {
-    const char *v = getenv(name);
-    return (v && *v ? atoi(v) : dflt) != 0;
-}
+bool env_flag(const char *name, int dflt) { return env_int(name, dflt) != 0; }
 
 // Bump allocator over the device's scratch.  In dry mode nothing is touched: the
 // same host logic runs and only the byte count is produced (workspace_query).
@@ -680,6 +678,7 @@ int bwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const mni_
 // Runs `body` twice: a dry pass that sizes the scratch, then the real pass.
 template <class Body>
 int with_scratch(uint32_t flags, void *stream, Body body) {
+    EnvScope env;
     DeviceState *st = nullptr;
     int rc = device_state(&st);
     if (rc) return rc;
@@ -720,6 +719,42 @@ int device_sm_count() {
 bool pdl_enabled() {
     static const bool on = env_flag("MNI_B200_PDL", 1);
     return on;
+}
+
+// The switches found by the innermost open EnvScope of this thread: pointers into the environment block, valid while
+// the call runs under the same rule as getenv's results.
+namespace {
+constexpr int kMaxSwitches = 48;
+struct EnvSnapshot {
+    int depth = 0, count = 0;
+    const char *entry[kMaxSwitches];      // "NAME=value"
+};
+thread_local EnvSnapshot t_env;
+}  // namespace
+
+EnvScope::EnvScope() {
+    if (t_env.depth++ != 0) return;
+    t_env.count = 0;
+    for (char **e = environ; e && *e; ++e)
+        if ((*e)[0] == 'M' && strncmp(*e, "MNI_B200_", 9) == 0 && t_env.count < kMaxSwitches) t_env.entry[t_env.count++] = *e;
+}
+EnvScope::~EnvScope() { --t_env.depth; }
+
+const char *env_value(const char *name) {
+    const char *v = nullptr;
+    if (t_env.depth == 0) {
+        v = getenv(name);
+    } else {
+        for (int i = 0; i < t_env.count; ++i) {
+            const size_t n = strlen(name);
+            if (strncmp(t_env.entry[i], name, n) == 0 && t_env.entry[i][n] == '=') { v = t_env.entry[i] + n + 1; break; }
+        }
+    }
+    return v && *v ? v : nullptr;
+}
+int env_int(const char *name, int dflt) {
+    const char *v = env_value(name);
+    return v ? atoi(v) : dflt;
 }
 
 int fail(int status, const char *fmt, ...) {

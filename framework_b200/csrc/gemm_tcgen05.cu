@@ -1251,11 +1251,6 @@ EncodeTiledFn encode_fn() {
     return fn;
 }
 
-int env_int(const char *name, int dflt) {
-    const char *v = getenv(name);
-    return v && *v ? atoi(v) : dflt;
-}
-
 // Encoded tensor maps are a pure function of (pointer, extents, strides, box, swizzle): a training loop calls with
 // the same handful of buffers every step, so each host thread keeps the maps it has built (bounded; dropped
 // wholesale when full) and an eager call pays a hash lookup instead of three or four driver encodes.
@@ -1269,9 +1264,14 @@ struct MapKey {
 };
 struct MapKeyHash {
     size_t operator()(const MapKey &k) const {
-        const unsigned char *b = reinterpret_cast<const unsigned char *>(&k);
-        uint64_t h = 1469598103934665603ull;            // FNV-1a over the key's bytes
-        for (size_t i = 0; i < sizeof(MapKey); ++i) { h ^= b[i]; h *= 1099511628211ull; }
+        static_assert(sizeof(MapKey) % 8 == 0, "hashed in 8-byte words");
+        uint64_t h = 1469598103934665603ull;
+        for (size_t i = 0; i < sizeof(MapKey); i += 8) {
+            uint64_t w;
+            memcpy(&w, reinterpret_cast<const unsigned char *>(&k) + i, 8);
+            h = (h ^ w) * 0x9e3779b97f4a7c15ull;
+            h ^= h >> 29;
+        }
         return static_cast<size_t>(h);
     }
 };
@@ -1775,8 +1775,8 @@ int launch_gemm_tc(const GemmProblem &p0, float *partial, uint32_t *err_word, in
     {
         // Tests shorten the limit of the device-side waits; the withhold hook (a stage that never fills, so
         // that the waits do run out) is honoured only together with a limit of at most ~0.1 s.
-        const char *w = getenv("MNI_B200_WAIT_CYCLES");
-        const long long wc = w && *w ? atoll(w) : 0;
+        const char *w = env_value("MNI_B200_WAIT_CYCLES");
+        const long long wc = w ? atoll(w) : 0;
         k.wait_cycles = wc > 0 ? wc : kWaitCycles;
         k.withhold_at = k.wait_cycles <= 200000000LL ? env_int("MNI_B200_TEST_WITHHOLD_KBLOCK", 0) : 0;
     }

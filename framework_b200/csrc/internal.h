@@ -50,6 +50,19 @@ cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, si
 // error plumbing
 // ---------------------------------------------------------------------------
 int fail(int status, const char *fmt, ...);          // records the thread-local message, returns status
+
+// The MNI_B200_* switches.  A call consults some forty of them (the planner runs once to size the scratch and once to
+// launch), and getenv walks the whole environment each time -- 3 of the 6 us a small product's call spent on the
+// host.  An entry point opens an EnvScope, which walks the environment once; env_value then looks among the
+// switches found, normally none.  Outside a scope env_value reads the environment itself.
+struct EnvScope {
+    EnvScope();
+    ~EnvScope();
+    EnvScope(const EnvScope &) = delete;
+    EnvScope &operator=(const EnvScope &) = delete;
+};
+const char *env_value(const char *name);              // value, or nullptr if unset or empty
+int env_int(const char *name, int dflt);
 int device_sm_count();                                // SM count of the current device (cached per device)
 extern std::atomic<uint64_t> g_launches;              // kernels launched by this library
 

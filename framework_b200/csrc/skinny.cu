@@ -605,8 +605,7 @@ skinny_dx_sliced_kernel(const float *__restrict__ dy, long long lddy, const floa
 // Which dx kernel runs.  The sliced kernel is opt-in (MNI_B200_SKINNY_DX_SLICED=1): measured inside the
 // benchmark step at 4 rows, K = N = 4096, it needs ~28 us against ~18 us for the row-pair kernel.
 int dx_sliced_mode() {
-    const char *v = getenv("MNI_B200_SKINNY_DX_SLICED");
-    return v && *v ? atoi(v) : -1;
+    return env_int("MNI_B200_SKINNY_DX_SLICED", -1);
 }
 
 int pick_mt(int64_t M) { return M <= 1 ? 1 : M <= 2 ? 2 : M <= 4 ? 4 : M <= 8 ? 8 : 16; }
@@ -767,8 +766,7 @@ int launch_skinny_dx(const float *dy, int64_t lddy, const float *W, int64_t ldw,
 #define MNI_SKINNY_DXS(MT, P_, B_)                                                                              \
     skinny_dx_sliced_kernel<MT, P_, B_><<<sblocks, 32 * kDxsWarps, 0, stream>>>(dy, lddy, W, ldw, dx, lddx,       \
                                                                                accumulate ? 1 : 0, (int)M, N, K)
-        const char *vv = getenv("MNI_B200_DXS_VARIANT");      // register / slice-width variants of the 4- and 8-row forms
-        const int variant = vv && *vv ? atoi(vv) : 0;
+        const int variant = env_int("MNI_B200_DXS_VARIANT", 0);      // register / slice-width variants of the 4- and 8-row forms
         switch (mt) {
             case 1: MNI_SKINNY_DXS(1, 4, 2); break;
             case 2: MNI_SKINNY_DXS(2, 4, 2); break;
