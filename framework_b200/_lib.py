@@ -112,7 +112,17 @@ def lib() -> C.CDLL:
 
 def check(status: int) -> None:
     if status != 0:
-        raise MniError(status, lib().mni_b200_last_error().decode("utf-8", "replace"))
+        raise_status(status)
+
+
+def raise_status(status: int, message: str | None = None) -> None:
+    raise MniError(status, lib().mni_b200_last_error().decode("utf-8", "replace") if message is None else message)
+
+
+def addresses() -> dict:
+    """Address of every entry point of the loaded library, for the native host side."""
+    handle = lib()
+    return {name: C.cast(getattr(handle, name), C.c_void_p).value for name in _SIGNATURES}
 
 
 def make_view(ptr: int, shape, strides) -> View:

@@ -1,7 +1,10 @@
-"""Builds ``libmni_b200.so`` in-tree with nvcc for sm_100a (cross-compiles without a GPU)."""
+"""Builds the native parts in-tree: ``libmni_b200.so`` with nvcc for sm_100a (cross-compiles without a GPU) and the
+host extension ``_host.so`` (tensor object and operator front end) with g++ against torch's headers."""
 from __future__ import annotations
 
 import glob
+import importlib.machinery
+import importlib.util
 import os
 import subprocess
 import sys
@@ -10,6 +13,8 @@ _PKG = os.path.dirname(os.path.abspath(__file__))
 _ROOT = os.path.dirname(_PKG)
 CSRC = os.path.join(_PKG, "csrc")
 LIB_PATH = os.path.join(_PKG, "lib", "libmni_b200.so")
+HOST_SRC = os.path.join(CSRC, "host", "host.cpp")
+HOST_PATH = os.path.join(_PKG, "lib", "_host.so")
 
 NVCC_FLAGS = [
     "-O3", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
@@ -91,5 +96,67 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
     return LIB_PATH
 
 
+def host_source_hash() -> str:
+    """sha256 of what the host extension is built from: its source, the C ABI header, the torch and Python versions."""
+    import hashlib
+    import torch
+    h = hashlib.sha256(f"{torch.__version__} {sys.version_info[:3]}".encode())
+    for path in [HOST_SRC] + sorted(glob.glob(os.path.join(_ROOT, "include", "*.h"))):
+        with open(path, "rb") as f:
+            h.update(f.read())
+    return h.hexdigest()
+
+
+def _hash_file() -> str:
+    return HOST_PATH + ".id"
+
+
+def host_is_stale() -> bool:
+    try:
+        with open(_hash_file()) as f:
+            return f.read().strip() != host_source_hash() or not os.path.exists(HOST_PATH)
+    except OSError:
+        return True
+
+
+def build_host(force: bool = False) -> str:
+    """Compiles the host extension into lib/_host.so (about ten seconds); returns its path.  The file is put in place
+    by a rename, so that processes that build it at the same time each see a whole one."""
+    if not force and not host_is_stale():
+        return HOST_PATH
+    import sysconfig
+    import torch
+    root = os.path.dirname(torch.__file__)
+    inc = [os.path.join(_ROOT, "include"), os.path.join(root, "include"),
+           os.path.join(root, "include", "torch", "csrc", "api", "include"), sysconfig.get_paths()["include"],
+           os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")]
+    os.makedirs(os.path.dirname(HOST_PATH), exist_ok=True)
+    tmp = f"{HOST_PATH}.{os.getpid()}.tmp"
+    subprocess.check_call(
+        ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+         f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+         f'-DMNI_HOST_SOURCE_HASH="{host_source_hash()}"', *[f"-I{d}" for d in inc], HOST_SRC, "-o", tmp,
+         "-L" + os.path.join(root, "lib"), "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10"])
+    os.replace(tmp, HOST_PATH)
+    with open(f"{tmp}.id", "w") as f:
+        f.write(host_source_hash() + "\n")
+    os.replace(f"{tmp}.id", _hash_file())
+    return HOST_PATH
+
+
+def load_host():
+    """The host extension as a module, compiled first if it is missing or was built from another source."""
+    import torch  # noqa: F401  (the extension links against torch's libraries, which torch loads)
+    build_host()
+    loader = importlib.machinery.ExtensionFileLoader("_host", HOST_PATH)
+    spec = importlib.util.spec_from_file_location("_host", HOST_PATH, loader=loader)
+    module = importlib.util.module_from_spec(spec)
+    loader.exec_module(module)
+    if module.source_hash != host_source_hash():
+        raise ImportError(f"{HOST_PATH} was built from another source than {HOST_SRC}; delete it and import again")
+    return module
+
+
 if __name__ == "__main__":
     print(build_library(force="--force" in sys.argv, verbose="-v" in sys.argv))
+    print(build_host(force="--force" in sys.argv))

@@ -2,16 +2,17 @@
 
 Names, argument meaning and error behaviour follow src/native/src/ops/matmul.rs
 and the bias branch of src/native/src/ops/elementwise.rs; every function is a thin
-call into the C ABI of ``libmni_b200.so``.  Outputs are allocated here the way the
+call into the C ABI of ``libmni_b200.so``, made by the native host side
+(csrc/host/host.cpp): it checks the arguments, allocates the outputs the way the
 reference's ``store.zeros`` does (uninitialised memory is fine: the kernels
-overwrite every element).
+overwrite every element) and names the current stream.
 """
 from __future__ import annotations
 
 from typing import Optional, Sequence, Tuple
 
 from . import _lib
-from .tensor import DeviceTensor, current_stream, row_major_strides, shape_size
+from .tensor import DeviceTensor, _host, current_stream, row_major_strides
 
 
 def broadcast_shape(a: Sequence[int], b: Sequence[int]) -> tuple:
@@ -43,17 +44,7 @@ def _matmul_out_shape(a: DeviceTensor, b: DeviceTensor) -> tuple:
 def matmul(a: DeviceTensor, b: DeviceTensor, bias: Optional[DeviceTensor] = None, *, flags: int = 0,
            out: Optional[DeviceTensor] = None) -> DeviceTensor:
     """``ops::matmul::matmul`` (ops/matmul.rs:83-197).  ``bias`` fuses the Linear bias add."""
-    oshape = _matmul_out_shape(a, b)
-    if bias is not None and (bias.ndim != 1 or bias.shape[0] != oshape[-1] or not bias.is_contiguous()):
-        raise ValueError("bias must be a contiguous [N] vector")
-    if out is None:
-        out = DeviceTensor.empty(oshape, a.storage.device)
-    elif out.shape != oshape or not out.is_contiguous():
-        raise ValueError("out must be contiguous with the broadcast output shape")
-    va, vb = a.view_struct(), b.view_struct()
-    _lib.check(_lib.lib().mni_b200_matmul_fwd(va, vb, out.ptr, bias.ptr if bias is not None else None,
-                                              flags, current_stream()))
-    return out
+    return _host.matmul(a, b, bias, flags, out)
 
 
 def matmul_backward(grad: DeviceTensor, a: DeviceTensor, b: DeviceTensor, *, flags: int = 0,
@@ -61,119 +52,46 @@ def matmul_backward(grad: DeviceTensor, a: DeviceTensor, b: DeviceTensor, *, fla
                     da: Optional[DeviceTensor] = None, db: Optional[DeviceTensor] = None,
                     dbias: Optional[DeviceTensor] = None):
     """``ops::matmul::matmul_backward`` (ops/matmul.rs:225-255) -> (grad_a, grad_b[, dbias])."""
-    oshape = _matmul_out_shape(a, b)
-    if grad.shape != oshape:
-        raise ValueError(f"grad has shape {grad.shape}, forward output is {oshape}")
-    dev = a.storage.device
-    if need_da and da is None:
-        da = DeviceTensor.empty(a.shape, dev)
-    if need_db and db is None:
-        db = DeviceTensor.empty(b.shape, dev)
-    if want_dbias and dbias is None:
-        dbias = DeviceTensor.empty((oshape[-1],), dev)
-    va, vb, vg = a.view_struct(), b.view_struct(), grad.view_struct()
-    _lib.check(_lib.lib().mni_b200_matmul_bwd(
-        va, vb, vg, da.ptr if need_da else None, db.ptr if need_db else None,
-        dbias.ptr if want_dbias else None, flags, current_stream()))
-    if want_dbias:
-        return da, db, dbias
-    return da, db
+    return _host.matmul_backward(grad, a, b, flags, need_da, need_db, want_dbias, da, db, dbias)
 
 
 def add(a: DeviceTensor, b: DeviceTensor) -> DeviceTensor:
     """Bias branch of ``ops::elementwise::add`` (ops/elementwise.rs:105-130): [.., N] + [N]."""
-    if not (b.ndim == 1 and a.ndim >= 1 and a.shape[-1] == b.shape[0]):
-        raise NotImplementedError("only the Linear bias add ([..., N] + [N]) is on this path")
-    a = a.contiguous()
-    b = b.contiguous()
-    out = DeviceTensor.empty(a.shape, a.storage.device)
-    n = a.shape[-1]
-    rows = shape_size(a.shape[:-1])
-    _lib.check(_lib.lib().mni_b200_add_bias(a.ptr, b.ptr, out.ptr, rows, n, current_stream()))
-    return out
+    return _host.add(a, b)
 
 
 def add_backward(grad: DeviceTensor, a_shape: Sequence[int], b_shape: Sequence[int], *,
                  flags: int = 0) -> Tuple[DeviceTensor, DeviceTensor]:
     """``add_backward`` for the bias branch (ops/elementwise.rs:213-231) -> (grad_a, grad_bias)."""
-    if tuple(grad.shape) != tuple(a_shape) or len(b_shape) != 1 or b_shape[0] != grad.shape[-1]:
-        raise NotImplementedError("only the Linear bias add ([..., N] + [N]) is on this path")
-    g = grad.contiguous()
-    ga = DeviceTensor.empty(a_shape, g.storage.device)
-    gb = DeviceTensor.empty(b_shape, g.storage.device)
-    n = g.shape[-1]
-    rows = shape_size(g.shape[:-1])
-    _lib.check(_lib.lib().mni_b200_add_bias_bwd(g.ptr, ga.ptr, gb.ptr, rows, n, flags, current_stream()))
-    return ga, gb
+    return _host.add_backward(grad, a_shape, b_shape, flags)
 
 
 def bias_gelu(x: DeviceTensor, bias: DeviceTensor) -> DeviceTensor:
     """``ops::fused::bias_gelu`` (ops/fused.rs:279-314): gelu(x + bias) with bias over the last dim."""
-    if bias.ndim != 1 or x.ndim < 1 or x.shape[-1] != bias.shape[0]:
-        raise ValueError("bias must be a [C] vector matching x's last dim")
-    x, bias = x.contiguous(), bias.contiguous()
-    out = DeviceTensor.empty(x.shape, x.storage.device)
-    n = x.shape[-1]
-    _lib.check(_lib.lib().mni_b200_bias_gelu(x.ptr, bias.ptr, out.ptr, shape_size(x.shape[:-1]), n, current_stream()))
-    return out
+    return _host.bias_gelu(x, bias)
 
 
 def bias_gelu_backward(grad: DeviceTensor, x: DeviceTensor, bias: DeviceTensor, *,
                        flags: int = 0) -> Tuple[DeviceTensor, DeviceTensor]:
     """``ops::fused::bias_gelu_backward`` (ops/fused.rs:354-392) -> (dx, dbias)."""
-    if tuple(grad.shape) != tuple(x.shape) or bias.shape != (x.shape[-1],):
-        raise ValueError("grad must have x's shape and bias must be [C]")
-    g, x, bias = grad.contiguous(), x.contiguous(), bias.contiguous()
-    dx = DeviceTensor.empty(x.shape, x.storage.device)
-    dbias = DeviceTensor.empty(bias.shape, x.storage.device)
-    n = x.shape[-1]
-    _lib.check(_lib.lib().mni_b200_bias_gelu_bwd(g.ptr, x.ptr, bias.ptr, dx.ptr, dbias.ptr,
-                                                 shape_size(x.shape[:-1]), n, flags, current_stream()))
-    return dx, dbias
+    return _host.bias_gelu_backward(grad, x, bias, flags)
 
 
 def matmul_bias_gelu(a: DeviceTensor, b: DeviceTensor, bias: DeviceTensor, *, flags: int = 0,
                      want_pre: bool = True) -> Tuple[Optional[DeviceTensor], DeviceTensor]:
     """matmul followed by bias_gelu in one GEMM launch -> (pre = a.b or None, out = gelu(pre + bias))."""
-    oshape = _matmul_out_shape(a, b)
-    if bias.ndim != 1 or bias.shape[0] != oshape[-1] or not bias.is_contiguous():
-        raise ValueError("bias must be a contiguous [N] vector")
-    dev = a.storage.device
-    pre = DeviceTensor.empty(oshape, dev) if want_pre else None
-    out = DeviceTensor.empty(oshape, dev)
-    va, vb = a.view_struct(), b.view_struct()
-    _lib.check(_lib.lib().mni_b200_matmul_bias_gelu_fwd(va, vb, bias.ptr, pre.ptr if pre is not None else None,
-                                                        out.ptr, flags, current_stream()))
-    return pre, out
-
-
-def _softmax_split(shape: Sequence[int], dim: int) -> Tuple[int, int, int]:
-    d = dim + len(shape) if dim < 0 else dim
-    if not 0 <= d < len(shape):
-        raise IndexError(f"softmax dim {dim} out of range for shape {tuple(shape)}")
-    return max(shape_size(shape[:d]), 1) if d else 1, shape[d], max(shape_size(shape[d + 1:]), 1)
+    return _host.matmul_bias_gelu(a, b, bias, flags, want_pre)
 
 
 def softmax(a: DeviceTensor, dim: int = -1) -> DeviceTensor:
     """``ops::norm::softmax`` (ops/norm.rs:52-89).  A strided input is gathered first, as the reference's
     ``dev_ptr`` read assumes row-major data."""
-    a = a if a.is_contiguous() else a.contiguous()
-    outer, size, inner = _softmax_split(a.shape, dim)
-    out = DeviceTensor.empty(a.shape, a.storage.device)
-    _lib.check(_lib.lib().mni_b200_softmax_fwd(a.ptr, out.ptr, outer, size, inner, current_stream()))
-    return out
+    return _host.softmax(a, dim)
 
 
 def softmax_backward(grad: DeviceTensor, out: DeviceTensor, dim: int = -1) -> DeviceTensor:
     """``ops::norm::softmax_backward`` (ops/norm.rs:125-163) from the saved forward output."""
-    if tuple(grad.shape) != tuple(out.shape):
-        raise ValueError("grad and out must have the same shape")
-    grad = grad if grad.is_contiguous() else grad.contiguous()
-    out = out if out.is_contiguous() else out.contiguous()
-    outer, size, inner = _softmax_split(out.shape, dim)
-    dx = DeviceTensor.empty(out.shape, out.storage.device)
-    _lib.check(_lib.lib().mni_b200_softmax_bwd(grad.ptr, out.ptr, dx.ptr, outer, size, inner, current_stream()))
-    return dx
+    return _host.softmax_backward(grad, out, dim)
 
 
 def _grad_sumsq(grads: Sequence[DeviceTensor]) -> "torch.Tensor":
@@ -237,12 +155,7 @@ def permute(a: DeviceTensor, dims: Sequence[int]) -> DeviceTensor:
 def permute_backward(grad: DeviceTensor, dims: Sequence[int], orig_shape: Sequence[int]) -> DeviceTensor:
     """``ops::layout::permute_backward`` (ops/layout.rs:198-212): the gradient of the permuted tensor, put
     back into the original layout -- one device gather of the inverse-permuted view."""
-    if tuple(grad.shape) != tuple(orig_shape[d] for d in dims):
-        raise ValueError(f"grad has shape {grad.shape}, expected {tuple(orig_shape[d] for d in dims)}")
-    inv = [0] * len(dims)
-    for i, d in enumerate(dims):
-        inv[d] = i
-    return grad.permute(inv).contiguous()
+    return _host.permute_backward(grad, dims, orig_shape)
 
 
 class Linear:

@@ -13,7 +13,9 @@ from typing import Sequence
 import numpy as np
 import torch
 
-from . import _lib
+from . import _lib, build
+
+_host = build.load_host()
 
 
 def row_major_strides(shape: Sequence[int]) -> tuple:
@@ -33,26 +35,22 @@ def shape_size(shape: Sequence[int]) -> int:
 
 
 def current_stream() -> int:
-    return int(torch.cuda.current_stream().cuda_stream)
+    """Address of the current CUDA stream of the current device."""
+    return _host.current_stream()
 
 
-class DeviceTensor:
-    """f32 tensor on the current CUDA device: flat storage, shape, element strides."""
+class DeviceTensor(_host.Tensor):
+    """f32 tensor on the current CUDA device: flat `storage`, `shape`, element `strides`.
 
-    __slots__ = ("storage", "shape", "strides")
+    ``DeviceTensor(storage, shape, strides=None)``; the object itself, with `size`, `ndim`, `ptr`,
+    `is_contiguous()`, `permute(dims)` and `contiguous()`, is native (csrc/host/host.cpp)."""
 
-    def __init__(self, storage: torch.Tensor, shape: Sequence[int], strides: Sequence[int] | None = None):
-        if storage.dtype != torch.float32 or not storage.is_cuda or storage.dim() != 1:
-            raise TypeError("storage must be a flat float32 CUDA tensor")
-        self.storage = storage
-        self.shape = tuple(int(s) for s in shape)
-        self.strides = tuple(int(s) for s in strides) if strides is not None else row_major_strides(self.shape)
+    __slots__ = ()
 
     # -- construction ------------------------------------------------------
     @staticmethod
     def empty(shape: Sequence[int], device=None) -> "DeviceTensor":
-        n = max(shape_size(shape), 1)
-        return DeviceTensor(torch.empty(n, dtype=torch.float32, device=device or "cuda"), shape)
+        return _host.empty(shape, device)
 
     @staticmethod
     def from_numpy(a: np.ndarray, device=None) -> "DeviceTensor":
@@ -71,33 +69,10 @@ class DeviceTensor:
             base, t.storage_offset(), (max(_span(t), 1),), (1,))
         return DeviceTensor(flat, tuple(t.shape), tuple(t.stride()))
 
-    # -- properties --------------------------------------------------------
-    @property
-    def size(self) -> int:
-        return shape_size(self.shape)
-
-    @property
-    def ndim(self) -> int:
-        return len(self.shape)
-
-    @property
-    def ptr(self) -> int:
-        return int(self.storage.data_ptr())
-
-    def is_contiguous(self) -> bool:
-        """tensor.rs:77-89."""
-        return self.strides == row_major_strides(self.shape)
-
     def view_struct(self) -> "_lib.View":
         return _lib.make_view(self.ptr, self.shape, self.strides)
 
     # -- layout ops (ops/layout.rs) ------------------------------------------
-    def permute(self, dims: Sequence[int]) -> "DeviceTensor":
-        """Stride-only permutation sharing the storage (no kernel, no copy)."""
-        if sorted(dims) != list(range(self.ndim)):
-            raise ValueError(f"invalid permutation {list(dims)}")
-        return DeviceTensor(self.storage, [self.shape[d] for d in dims], [self.strides[d] for d in dims])
-
     def narrow(self, dim: int, start: int, length: int) -> "DeviceTensor":
         """The sub-tensor [start, start + length) of dimension `dim`, as a view of the same storage (pointer
         offset + same strides): how row or column panels of an operand reach the kernels without a copy."""
@@ -107,15 +82,6 @@ class DeviceTensor:
         shape = list(self.shape)
         shape[d] = length
         return DeviceTensor(self.storage[start * self.strides[d]:], shape, self.strides)
-
-    def contiguous(self) -> "DeviceTensor":
-        """ops/layout.rs:218-231 / tensor.rs:510-517, done on the device."""
-        if self.is_contiguous():
-            return self
-        out = DeviceTensor.empty(self.shape, self.storage.device)
-        v = self.view_struct()
-        _lib.check(_lib.lib().mni_b200_contiguous(v, out.ptr, current_stream()))
-        return out
 
     def view(self, shape: Sequence[int]) -> "DeviceTensor":
         """ops/layout.rs:80-89: reshape of the contiguous data (shares storage when already contiguous)."""
@@ -138,3 +104,11 @@ def _span(t: torch.Tensor) -> int:
     if t.numel() == 0:
         return 0
     return 1 + sum((s - 1) * st for s, st in zip(t.shape, t.stride()))
+
+
+_host.setup(DeviceTensor, lambda: _host.bind(_lib.addresses()), _lib.raise_status, lambda a, b: _product_shape(a, b))
+
+
+def _product_shape(a, b) -> tuple:
+    from .ops import _matmul_out_shape
+    return _matmul_out_shape(a, b)
