@@ -70,6 +70,10 @@ _SIGNATURES = {
     "mni_b200_adamw_step": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_float, C.c_float,
                                       C.c_float, C.c_float, C.c_float, C.c_uint32, C.c_void_p, C.c_float, C.c_int,
                                       C.c_void_p]),
+    "mni_b200_grad_norm_sq": (C.c_int, [C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
+    "mni_b200_clip_and_step": (C.c_int, [C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_float,
+                                         C.c_float, C.c_float, C.c_float, C.c_float, C.c_uint32, C.c_float, C.c_void_p,
+                                         C.c_void_p]),
     "mni_b200_contiguous": (C.c_int, [C.POINTER(View), C.c_void_p, C.c_void_p]),
     "mni_b200_sm_reserve": (C.c_int, [C.c_int]),
     "mni_b200_workspace_set": (C.c_int, [C.c_void_p, C.c_size_t]),

@@ -10,8 +10,10 @@
 #include <unistd.h>
 
 #include <algorithm>
+#include <cmath>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <vector>
 
 namespace mni {
@@ -170,6 +172,62 @@ int scratch_base(DeviceState &st, size_t bytes, cudaStream_t stream, uint8_t **b
     *base = st.ws;
     return MNI_B200_OK;
 }
+
+// Where a kernel leaves a number for the host: slots of pinned memory, one per call that is waiting.  The pool is
+// process-wide (portable pinned memory), bounded, and a slot goes back when its call returns.
+struct NormSlotLease {
+    NormSlot *slot = nullptr;
+    unsigned seq = 0;
+    static constexpr int kSlots = 64;
+    struct Pool {
+        std::mutex mu;
+        NormSlot *base = nullptr;
+        uint64_t used = 0;         // bit per slot
+        unsigned next_seq = 0;
+    };
+    static Pool &pool() { static Pool p; return p; }
+    int take() {
+        Pool &p = pool();
+        std::unique_lock<std::mutex> lock(p.mu);
+        if (!p.base) {
+            void *m = nullptr;
+            const cudaError_t e = cudaHostAlloc(&m, kSlots * sizeof(NormSlot), cudaHostAllocPortable | cudaHostAllocMapped);
+            if (e != cudaSuccess) return fail(MNI_B200_ERR_CUDA, "cudaHostAlloc: %s", cudaGetErrorString(e));
+            memset(m, 0, kSlots * sizeof(NormSlot));
+            p.base = static_cast<NormSlot *>(m);
+        }
+        while (~p.used == 0) {                // every slot is out: some call returns its own soon
+            lock.unlock();
+            std::this_thread::yield();
+            lock.lock();
+        }
+        const int i = __builtin_ctzll(~p.used);
+        p.used |= 1ull << i;
+        slot = p.base + i;
+        if (++p.next_seq == 0) ++p.next_seq;
+        seq = p.next_seq;
+        return MNI_B200_OK;
+    }
+    // Waits until the kernel has written the slot, or until the stream has ended without doing so.
+    int wait(cudaStream_t stream) {
+        volatile unsigned *const arrived = &slot->seq;
+        for (uint64_t spins = 1; *arrived != seq; ++spins) {
+            if ((spins & 0x3fff) != 0) continue;
+            const cudaError_t e = cudaStreamQuery(stream);
+            if (e == cudaErrorNotReady) continue;
+            if (e == cudaSuccess && *arrived == seq) break;
+            return fail(MNI_B200_ERR_CUDA, "the norm did not arrive: %s", cudaGetErrorString(e));
+        }
+        std::atomic_thread_fence(std::memory_order_acquire);
+        return MNI_B200_OK;
+    }
+    ~NormSlotLease() {
+        if (!slot) return;
+        Pool &p = pool();
+        std::lock_guard<std::mutex> lock(p.mu);
+        p.used &= ~(1ull << (slot - p.base));
+    }
+};
 
 // ------------------------------------------------------------------ shapes
 int64_t prod(const int64_t *s, int n) {
@@ -893,11 +951,18 @@ int mni_b200_grad_sumsq(const float *grad, int64_t n, double *sumsq, uint32_t fl
     if (n < 0) return fail(MNI_B200_ERR_ARG, "negative extent");
     if (!sumsq) return fail(MNI_B200_ERR_ARG, "sumsq is null");
     if (n > 0 && !grad) return fail(MNI_B200_ERR_ARG, "grad is null");
-    return with_scratch(flags, stream, [&](Call &c) -> int {
-        const size_t poff = c.arena.reserve(sumsq_partial_bytes(n, c.st->sm_count));
-        if (c.dry()) return MNI_B200_OK;
-        return launch_sumsq(grad, n, sumsq, (flags & MNI_B200_ACCUMULATE_C) != 0, c.at(poff), c.st->sm_count, c.stream);
-    });
+    DeviceState *st = nullptr;
+    int rc = device_state(&st);
+    if (rc) return rc;
+    return launch_sumsq_list(1, &grad, &n, sumsq, (flags & MNI_B200_ACCUMULATE_C) != 0, nullptr, 0, st->sm_count,
+                             static_cast<cudaStream_t>(stream));
+}
+
+// bias corrections of ops/optimizer.rs:26-27: 1 - beta.powi(step) in f32
+static AdamWArgs adamw_args(float lr, float beta1, float beta2, float eps, float weight_decay, uint32_t step,
+                            const double *sumsq, float max_norm, int write_clipped_grad) {
+    return AdamWArgs{lr, beta1, beta2, eps, 1.0f - lr * weight_decay, 1.0f - powi_f32(beta1, step),
+                     1.0f - powi_f32(beta2, step), sumsq, max_norm, write_clipped_grad ? 1 : 0};
 }
 
 int mni_b200_adamw_step(float *param, float *m, float *v, float *grad, int64_t n, float lr, float beta1, float beta2,
@@ -910,10 +975,59 @@ int mni_b200_adamw_step(float *param, float *m, float *v, float *grad, int64_t n
     DeviceState *st = nullptr;
     int rc = device_state(&st);
     if (rc) return rc;
-    // bias corrections of ops/optimizer.rs:26-27: 1 - beta.powi(step) in f32
-    const float p1 = powi_f32(beta1, step), p2 = powi_f32(beta2, step);
-    return launch_adamw(param, m, v, grad, n, lr, beta1, beta2, eps, weight_decay, 1.0f - p1, 1.0f - p2, grad_sumsq,
-                        max_grad_norm, write_clipped_grad != 0, static_cast<cudaStream_t>(stream));
+    return launch_adamw_list(adamw_args(lr, beta1, beta2, eps, weight_decay, step, grad_sumsq, max_grad_norm, write_clipped_grad),
+                             1, &param, &m, &v, &grad, &n, false, static_cast<cudaStream_t>(stream));
+}
+
+int mni_b200_grad_norm_sq(int64_t count, const float *const *grads, const int64_t *n, double *sumsq, void *stream) {
+    if (count < 0) return fail(MNI_B200_ERR_ARG, "negative count");
+    if (!sumsq || (count > 0 && (!grads || !n))) return fail(MNI_B200_ERR_ARG, "null pointer");
+    for (int64_t i = 0; i < count; ++i) {
+        if (n[i] < 0) return fail(MNI_B200_ERR_ARG, "negative extent");
+        if (n[i] > 0 && !grads[i]) return fail(MNI_B200_ERR_ARG, "grad is null");
+    }
+    DeviceState *st = nullptr;
+    int rc = device_state(&st);
+    if (rc) return rc;
+    return launch_sumsq_list(count, grads, n, sumsq, false, nullptr, 0, st->sm_count, static_cast<cudaStream_t>(stream));
+}
+
+int mni_b200_clip_and_step(int64_t count, float *const *params, float *const *ms, float *const *vs, float *const *grads,
+                           const int64_t *n, float lr, float beta1, float beta2, float eps, float weight_decay,
+                           uint32_t step, float max_grad_norm, float *norm, void *stream) {
+    if (count < 0) return fail(MNI_B200_ERR_ARG, "negative count");
+    if (count > 0 && (!params || !ms || !vs || !grads || !n)) return fail(MNI_B200_ERR_ARG, "null pointer");
+    for (int64_t i = 0; i < count; ++i) {
+        if (n[i] < 0) return fail(MNI_B200_ERR_ARG, "negative extent");
+        if (n[i] > 0 && (!params[i] || !ms[i] || !vs[i] || !grads[i])) return fail(MNI_B200_ERR_ARG, "null pointer");
+    }
+    if (step == 0) return fail(MNI_B200_ERR_ARG, "step counts from 1");
+    DeviceState *st = nullptr;
+    int rc = device_state(&st);
+    if (rc) return rc;
+    cudaStream_t const s = static_cast<cudaStream_t>(stream);
+    if (norm && stream_is_capturing(s))
+        return fail(MNI_B200_ERR_ARG, "the norm cannot be read while the stream is capturing: pass no norm");
+    double *sumsq = norm_sumsq_ptr();
+    if (!sumsq) return fail(MNI_B200_ERR_CUDA, "norm accumulator unavailable");
+    NormSlotLease lease;
+    if (norm) {
+        rc = lease.take();
+        if (rc) return rc;
+    }
+    {
+        std::lock_guard<std::mutex> lock(st->mu);      // the two launches of a call stay together
+        rc = launch_sumsq_list(count, grads, n, sumsq, false, lease.slot, lease.seq, st->sm_count, s);
+        if (rc == MNI_B200_OK)
+            rc = launch_adamw_list(adamw_args(lr, beta1, beta2, eps, weight_decay, step, sumsq, max_grad_norm, 1), count,
+                                   params, ms, vs, grads, n, true, s);
+    }
+    if (!norm) return rc;
+    // The norm arrives while the step still runs: the host waits for it alone, not for the stream.
+    const int waited = lease.wait(s);
+    if (rc || waited) return rc ? rc : waited;
+    *norm = sqrtf(static_cast<float>(lease.slot->sumsq));
+    return MNI_B200_OK;
 }
 
 int mni_b200_contiguous(const mni_b200_view *src, float *dst, void *stream) {
@@ -987,12 +1101,10 @@ int mni_b200_workspace_query(const mni_b200_view *a, const mni_b200_view *b, uin
     // bias + GELU forward without a `pre` output: when the epilogue cannot be fused the product needs a temporary
     rc = dry([&](Call &c) { return fwd_gelu_body(c, a, b, fake, nullptr, fake); });
     if (rc) return rc;
-    // the pointwise entry points on the forward output: column-sum partials, gradient-norm partials
+    // the pointwise entry points on the forward output: column-sum partials
     const int64_t rows = s.batch * s.M;
     need = std::max(need, (colsum_partial_bytes(std::max<int64_t>(rows, 1), std::max<int64_t>(s.N, 1), st->sm_count) + 255) &
                               ~static_cast<size_t>(255));
-    const int64_t biggest = std::max({s.a_batch * s.M * s.K, s.b_batch * s.K * s.N, rows * s.N, int64_t{1}});
-    need = std::max(need, (sumsq_partial_bytes(biggest, st->sm_count) + 255) & ~static_cast<size_t>(255));
     *bytes = need;
     return MNI_B200_OK;
 }

@@ -50,7 +50,8 @@ struct Api {
     decltype(&mni_b200_softmax_fwd) softmax_fwd;
     decltype(&mni_b200_softmax_bwd) softmax_bwd;
     decltype(&mni_b200_contiguous) contiguous;
-    decltype(&mni_b200_adamw_step) adamw_step;
+    decltype(&mni_b200_grad_norm_sq) grad_norm_sq;
+    decltype(&mni_b200_clip_and_step) clip_and_step;
 };
 Api g_api;
 bool g_bound = false;
@@ -730,6 +731,70 @@ PyObject *op_permute_backward(PyObject *, PyObject *const *args, Py_ssize_t narg
     return reinterpret_cast<PyObject *>(out);
 }
 
+// ------------------------------------------------------------------ optimizer
+// Addresses and sizes of a list of contiguous tensors.
+struct TensorList {
+    std::vector<float *> ptr;
+    std::vector<int64_t> n;
+    bool parse(PyObject *seq, const char *not_contiguous) {
+        PyObject *fast = PySequence_Fast(seq, "expected a sequence of tensors");
+        if (!fast) return false;
+        const Py_ssize_t count = PySequence_Fast_GET_SIZE(fast);
+        ptr.reserve(static_cast<size_t>(count));
+        n.reserve(static_cast<size_t>(count));
+        for (Py_ssize_t i = 0; i < count; ++i) {
+            TensorObj *t = as_tensor(PySequence_Fast_GET_ITEM(fast, i), "every element");
+            if (t && !t->contiguous) { PyErr_SetString(PyExc_ValueError, not_contiguous); t = nullptr; }
+            if (!t) { Py_DECREF(fast); return false; }
+            ptr.push_back(data(t));
+            n.push_back(numel(t->shape));
+        }
+        Py_DECREF(fast);
+        return true;
+    }
+};
+
+// grad_norm_sq(grads, address of a device double)
+PyObject *op_grad_norm_sq(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
+    ARGS(2, "grad_norm_sq(grads, out)");
+    TensorList grads;
+    if (!grads.parse(args[0], "gradients must be contiguous")) return nullptr;
+    double *out = static_cast<double *>(PyLong_AsVoidPtr(args[1]));
+    if (!out && PyErr_Occurred()) return nullptr;
+    void *stream = current_stream();
+    CALL(g_api.grad_norm_sq(static_cast<int64_t>(grads.ptr.size()), grads.ptr.data(), grads.n.data(), out, stream));
+    Py_RETURN_NONE;
+}
+
+// clip_and_step(params, ms, vs, grads, lr, beta1, beta2, eps, weight_decay, step, max_grad_norm) -> norm
+PyObject *op_clip_and_step(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
+    ARGS(11, "clip_and_step(params, ms, vs, grads, lr, beta1, beta2, eps, weight_decay, step, max_grad_norm)");
+    TensorList p, m, v, g;
+    const char *text = "adamw_step needs contiguous tensors";
+    if (!g.parse(args[3], "gradients must be contiguous") || !p.parse(args[0], text) || !m.parse(args[1], text) ||
+        !v.parse(args[2], text))
+        return nullptr;
+    const size_t count = p.ptr.size();
+    if (m.ptr.size() != count || v.ptr.size() != count || g.ptr.size() != count) {
+        PyErr_SetString(PyExc_ValueError, "params, ms, vs and grads must have the same length");
+        return nullptr;
+    }
+    if (p.n != m.n || p.n != v.n || p.n != g.n) {
+        PyErr_SetString(PyExc_ValueError, "param, m, v and grad must have the same size");
+        return nullptr;
+    }
+    float hyper[5];
+    for (int i = 0; i < 5; ++i) hyper[i] = static_cast<float>(PyFloat_AsDouble(args[4 + i]));
+    const uint32_t step = static_cast<uint32_t>(PyLong_AsUnsignedLongMask(args[9]));
+    const float max_norm = static_cast<float>(PyFloat_AsDouble(args[10]));
+    if (PyErr_Occurred()) return nullptr;
+    float norm = 0.f;
+    void *stream = current_stream();
+    CALL(g_api.clip_and_step(static_cast<int64_t>(count), p.ptr.data(), m.ptr.data(), v.ptr.data(), g.ptr.data(), p.n.data(),
+                             hyper[0], hyper[1], hyper[2], hyper[3], hyper[4], step, max_norm, &norm, stream));
+    return PyFloat_FromDouble(static_cast<double>(norm));
+}
+
 // ------------------------------------------------------------------ module
 // setup(cls, loader, raise_status, check_shapes): the Python side of the bindings
 PyObject *setup(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
@@ -750,7 +815,8 @@ PyObject *bind(PyObject *, PyObject *table) {
     struct { const char *name; void **slot; } entries[] = {
 #define ENTRY(field) {"mni_b200_" #field, reinterpret_cast<void **>(&g_api.field)}
         ENTRY(matmul_fwd), ENTRY(matmul_bwd), ENTRY(matmul_bias_gelu_fwd), ENTRY(add_bias), ENTRY(add_bias_bwd),
-        ENTRY(bias_gelu), ENTRY(bias_gelu_bwd), ENTRY(softmax_fwd), ENTRY(softmax_bwd), ENTRY(contiguous), ENTRY(adamw_step),
+        ENTRY(bias_gelu), ENTRY(bias_gelu_bwd), ENTRY(softmax_fwd), ENTRY(softmax_bwd), ENTRY(contiguous),
+        ENTRY(grad_norm_sq), ENTRY(clip_and_step),
 #undef ENTRY
     };
     for (auto &e : entries) {
@@ -784,6 +850,8 @@ PyMethodDef module_methods[] = {
     FAST("softmax", op_softmax, "ops.softmax"),
     FAST("softmax_backward", op_softmax_backward, "ops.softmax_backward"),
     FAST("permute_backward", op_permute_backward, "ops.permute_backward"),
+    FAST("grad_norm_sq", op_grad_norm_sq, "squared global gradient norm into a device double"),
+    FAST("clip_and_step", op_clip_and_step, "ops.clip_and_step"),
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_host", "native host side of the operator interface", -1, module_methods,
                           nullptr, nullptr, nullptr, nullptr};

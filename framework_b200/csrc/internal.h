@@ -159,15 +159,25 @@ size_t colsum_partial_bytes(int64_t rows, int64_t n, int sm_count);
 int launch_colsum(const float *dy, int64_t ld, float *out, int64_t rows, int64_t n, bool accumulate,
                   float *partial, int sm_count, cudaStream_t stream);
 int launch_copy(const float *src, float *dst, int64_t n, cudaStream_t stream);
-int launch_adamw(float *param, float *m, float *v, float *grad, int64_t n, float lr, float beta1, float beta2,
-                 float eps, float weight_decay, float bc1, float bc2, const double *sumsq, float max_norm,
-                 bool write_grad, cudaStream_t stream);
 int launch_softmax_fwd(const float *x, float *out, int64_t outer, int64_t dim, int64_t inner, cudaStream_t stream);
 int launch_softmax_bwd(const float *dy, const float *out, float *dx, int64_t outer, int64_t dim, int64_t inner,
                        cudaStream_t stream);
-size_t sumsq_partial_bytes(int64_t n, int sm_count);
-int launch_sumsq(const float *grad, int64_t n, double *out, bool accumulate, void *partial, int sm_count,
-                 cudaStream_t stream);
+// AdamW over a list of tensors, and the f64 sum of squares of a list of gradients (optimizer.cu).
+struct AdamWArgs {
+    float lr, beta1, beta2, eps, decay, bc1, bc2;
+    const double *sumsq;           // squared gradient norm on the device, or null
+    float max_norm;
+    int write_grad;
+};
+struct NormSlot {                  // in pinned host memory: the squared norm, then the sequence number of the call
+    double sumsq;
+    unsigned seq;
+};
+double *norm_sumsq_ptr();          // device address of clip_and_step's squared norm
+int launch_adamw_list(const AdamWArgs &a, int64_t count, float *const *param, float *const *m, float *const *v,
+                      float *const *grad, const int64_t *n, bool dependent, cudaStream_t stream);
+int launch_sumsq_list(int64_t count, const float *const *grad, const int64_t *n, double *out, bool accumulate,
+                      NormSlot *slot, unsigned seq, int sm_count, cudaStream_t stream);
 // out = gelu_tanh(x + bias[col]);  dx = grad * gelu'(x + bias), dbias = column sums of dx (partial: colsum_partial_bytes)
 int launch_bias_gelu(const float *x, const float *bias, float *out, int64_t rows, int64_t n, cudaStream_t stream);
 int launch_bias_gelu_bwd(const float *grad, const float *x, const float *bias, float *dx, float *dbias,

@@ -98,11 +98,7 @@ def _grad_sumsq(grads: Sequence[DeviceTensor]) -> "torch.Tensor":
     """Squared global gradient norm as a one-element f64 device tensor (no host read)."""
     import torch
     sumsq = torch.empty(1, dtype=torch.float64, device=grads[0].storage.device)
-    for i, g in enumerate(grads):
-        if not g.is_contiguous():
-            raise ValueError("gradients must be contiguous")
-        flags = _lib.ACCUMULATE_C if i else 0
-        _lib.check(_lib.lib().mni_b200_grad_sumsq(g.ptr, g.size, sumsq.data_ptr(), flags, current_stream()))
+    _host.grad_norm_sq(grads, sumsq.data_ptr())
     return sumsq
 
 
@@ -134,10 +130,13 @@ def clip_and_step(params: Sequence[DeviceTensor], ms: Sequence[DeviceTensor], vs
                   grads: Sequence[DeviceTensor], *, lr: float, beta1: float = 0.9, beta2: float = 0.999,
                   eps: float = 1e-8, weight_decay: float = 0.0, step: int = 1, max_grad_norm: float = 0.0) -> float:
     """``ops::optimizer::clip_and_step`` (ops/optimizer.rs:247-276): global-norm clip and AdamW over all
-    parameters; returns the norm before clipping.  The norm stays on the device until every step kernel is
-    queued; the read that returns it is the call's only synchronisation."""
+    parameters; returns the norm before clipping.  The call waits for the norm alone: the step it has queued by
+    then may still run, in stream order with whatever follows."""
     if not params:
         return 0.0
+    if len(params) == len(ms) == len(vs) == len(grads):
+        return _host.clip_and_step(params, ms, vs, grads, lr, beta1, beta2, eps, weight_decay, int(step), max_grad_norm)
+    # more gradients than parameters (or the other way round): the norm is over all of them, the step over the pairs
     import numpy as np
     sumsq = _grad_sumsq(grads)
     for p, m, v, g in zip(params, ms, vs, grads):

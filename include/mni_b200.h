@@ -202,6 +202,23 @@ MNI_B200_API int mni_b200_adamw_step(float *param, float *m, float *v, float *gr
                                      void *stream);
 
 /*
+ * The same over a model's parameters, a list of `count` tensors (host arrays of device pointers and element counts):
+ * the squared global gradient norm (ops/optimizer.rs:126-171) into a device double ...
+ */
+MNI_B200_API int mni_b200_grad_norm_sq(int64_t count, const float *const *grads, const int64_t *n, double *sumsq,
+                                       void *stream);
+/*
+ * ... and clip_and_step (ops/optimizer.rs:247-276): the norm over all gradients, then the clipped AdamW step of every
+ * tensor, gradients left scaled as grad_clip_f32 leaves them.  One launch each for lists of up to 512 tensors.  With a
+ * non-null `norm` (host memory) the call waits until the norm before clipping is known and stores it there; the
+ * step itself may still be running, in stream order with whatever follows.
+ */
+MNI_B200_API int mni_b200_clip_and_step(int64_t count, float *const *params, float *const *ms, float *const *vs,
+                                        float *const *grads, const int64_t *n, float lr, float beta1, float beta2,
+                                        float eps, float weight_decay, uint32_t step, float max_grad_norm, float *norm,
+                                        void *stream);
+
+/*
  * Same result as mni_b200_add_bias_bwd, for callers that must never see this library
  * allocate device memory: a runtime that owns the device's memory budget through its own
  * allocator, or a step loop that cannot take the device-wide stall of cudaMalloc/cudaFree.
@@ -237,8 +254,8 @@ MNI_B200_API int mni_b200_contiguous(const mni_b200_view *src, float *dst, void 
  * alignment count), over: mni_b200_matmul_fwd; mni_b200_matmul_bias_gelu_fwd
  * with or without a `pre` output; mni_b200_matmul_bwd with da, db and dbias and
  * ANY view of the output gradient (contiguous, or strided so that it has to be
- * gathered first); and the pointwise entry points (add_bias_bwd, bias_gelu_bwd,
- * grad_sumsq) applied to tensors no larger than a, b or the forward output.
+ * gathered first); and the pointwise entry points (add_bias_bwd, bias_gelu_bwd)
+ * applied to tensors no larger than a, b or the forward output.
  * The flags given are the flags the later calls must use.
  *
  * CUDA graphs.  Every call may be recorded by a capturing stream (the side stream

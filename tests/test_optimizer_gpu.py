@@ -102,3 +102,32 @@ def test_adamw_rejects_step_zero(F):
     t = _dev(F, np.zeros(8, np.float32))
     with pytest.raises(Exception):
         F.adamw_step(t, t, t, t, lr=1e-3, step=0)
+
+
+@pytest.mark.parametrize("sizes,misalign", [([1, 4095, 4096, 4097, 8192, 12289], 0), ([0, 5000, 0, 7], 0), ([4096, 9000], 1),
+                                            ([130] * 17, 0), ([33] * 129, 2), ([1000, 3] * 300, 0)])
+def test_parameter_lists_around_the_chunk_and_launch_limits(F, oracle, sizes, misalign):
+    """One launch covers a list of tensors in chunks of 4096 elements: sizes at the chunk's edges, empty tensors, starts
+    that are not 16-byte aligned, and lists on both sides of the 16 / 128 / 512 tensors a launch is compiled for."""
+    import torch
+    rng = np.random.default_rng(len(sizes))
+    host = {}
+    dev = {}
+    for name, scale in (("p", 1.0), ("m", 0.1), ("v", 0.01), ("g", 1.0)):
+        host[name] = [(scale * rng.standard_normal(n)).astype(np.float32) for n in sizes]
+        if name == "v":
+            host[name] = [np.abs(a) for a in host[name]]
+        dev[name] = []
+        for a in host[name]:
+            flat = torch.zeros(a.size + misalign + 1, device="cuda")[misalign:misalign + max(a.size, 1)]
+            flat[:a.size].copy_(torch.from_numpy(a))
+            dev[name].append(F.DeviceTensor(flat, (a.size,)))
+    cfg = dict(lr=1e-3, beta1=0.9, beta2=0.999, eps=1e-8, weight_decay=0.01, step=3, max_grad_norm=1.0)
+    want = oracle.clip_and_step(host["p"], host["m"], host["v"], host["g"], **cfg)
+    launches = F.launch_count()
+    got = F.clip_and_step(dev["p"], dev["m"], dev["v"], dev["g"], **cfg)
+    assert F.launch_count() - launches == 2 * ((len(sizes) + 511) // 512)
+    assert abs(got - want) <= 1e-6 * want          # the CPU backend's own sum is f64 over rounded f32 squares
+    for name in "pmvg":
+        for d, r in zip(dev[name], host[name]):
+            assert r.size == 0 or float(np.max(np.abs(d.numpy() - r))) <= 2e-6 * (1 + float(np.abs(r).max())), name
