@@ -11,6 +11,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <initializer_list>
 #include <mutex>
 #include <string>
 #include <thread>
@@ -332,35 +333,46 @@ struct Call {
     float *at(size_t off) const { return reinterpret_cast<float *>(base + off); }
 };
 
-// Gathers a view into scratch as [batch_flat, R, C] with the last dim padded to a multiple of 4.
-int pack_view(Call &c, const mni_b200_view &v, mni_b200_view *packed, size_t *offset) {
-    const int nd = v.ndim;
-    const int64_t cols = v.shape[nd - 1], rows = v.shape[nd - 2];
-    const int64_t ld = std::max<int64_t>(4, round_up(cols, 4));
-    const int64_t batch = prod(v.shape, nd - 2);
-    const size_t bytes = static_cast<size_t>(batch * rows * ld) * sizeof(float);
-    const size_t off = c.arena.reserve(bytes);
-    *offset = off;
-    packed->ndim = 3;
-    packed->shape[0] = batch; packed->shape[1] = rows; packed->shape[2] = cols;
-    packed->stride[0] = rows * ld; packed->stride[1] = ld; packed->stride[2] = 1;
-    packed->ptr = c.dry() ? reinterpret_cast<const float *>(static_cast<uintptr_t>(256)) : c.at(off);
-    c.note("gather of a strided operand into scratch");
-    if (c.dry()) return MNI_B200_OK;
-    return launch_pack(v, c.at(off), ld, c.stream);
+// Gathers views into scratch as [batch_flat, R, C] with the last dim padded to a multiple of 4, all in one launch.
+// Each *use[i] is replaced by the view of its packed copy, which `packed[i]` holds.
+int pack_views(Call &c, const mni_b200_view **const *use, mni_b200_view *packed, int count) {
+    GatherView jobs[kMaxGathers];
+    for (int i = 0; i < count; ++i) {
+        const mni_b200_view &v = **use[i];
+        const int nd = v.ndim;
+        const int64_t cols = v.shape[nd - 1], rows = v.shape[nd - 2];
+        const int64_t ld = std::max<int64_t>(4, round_up(cols, 4));
+        const int64_t batch = prod(v.shape, nd - 2);
+        const size_t off = c.arena.reserve(static_cast<size_t>(batch * rows * ld) * sizeof(float));
+        mni_b200_view &q = packed[i];
+        q.ndim = 3;
+        q.shape[0] = batch; q.shape[1] = rows; q.shape[2] = cols;
+        q.stride[0] = rows * ld; q.stride[1] = ld; q.stride[2] = 1;
+        q.ptr = c.dry() ? reinterpret_cast<const float *>(static_cast<uintptr_t>(256)) : c.at(off);
+        jobs[i] = GatherView{&v, c.dry() ? nullptr : c.at(off), ld};
+        c.note("gather of a strided operand into scratch");
+    }
+    int rc = MNI_B200_OK;
+    if (!c.dry()) rc = launch_gather(jobs, count, c.stream);
+    for (int i = 0; i < count; ++i) *use[i] = &packed[i];
+    return rc;
 }
 
-// Operand from a view, packing it into scratch when TMA cannot describe it.
-int make_operand(Call &c, const mni_b200_view &v, bool transposed, Operand &op) {
-    const bool force_pack = (c.flags & MNI_B200_FORCE_PACK) != 0;
-    if (!force_pack && view_to_operand(v, transposed, op)) return MNI_B200_OK;
-    mni_b200_view packed;
-    size_t off;
-    int rc = pack_view(c, v, &packed, &off);
-    if (rc) return rc;
-    if (!view_to_operand(packed, transposed, op)) return fail(MNI_B200_ERR_ARG, "packed operand is not describable");
-    // The packed copy is flat in the batch: keep the original flat batch count.
-    return MNI_B200_OK;
+// The operands TMA cannot describe (or all of them, under the test flag) are gathered first.  A gathered operand serves
+// every product of the call, whichever of its two matrix dims is contracted: the copy is describable either way.
+int pack_undescribable(Call &c, std::initializer_list<const mni_b200_view **> uses, mni_b200_view *packed) {
+    const mni_b200_view **need[kMaxGathers];
+    int count = 0;
+    for (const mni_b200_view **u : uses) {
+        Operand probe;
+        if ((c.flags & MNI_B200_FORCE_PACK) != 0 || !view_to_operand(**u, false, probe)) need[count++] = u;
+    }
+    return count ? pack_views(c, need, packed, count) : static_cast<int>(MNI_B200_OK);
+}
+
+int make_operand(const mni_b200_view &v, bool transposed, Operand &op) {
+    return view_to_operand(v, transposed, op) ? static_cast<int>(MNI_B200_OK)
+                                              : fail(MNI_B200_ERR_ARG, "operand is not describable");
 }
 
 int run_gemm(Call &c, GemmProblem &p) {
@@ -443,9 +455,12 @@ int fwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, float *out
     }
 
     GemmProblem p;
-    rc = make_operand(c, *a, false, p.A);
+    mni_b200_view packed[kMaxGathers];
+    rc = pack_undescribable(c, {&a, &b}, packed);
     if (rc) return rc;
-    rc = make_operand(c, *b, true, p.B);
+    rc = make_operand(*a, false, p.A);
+    if (rc) return rc;
+    rc = make_operand(*b, true, p.B);
     if (rc) return rc;
     p.A.batch = s.a_batch;
     p.B.batch = s.b_batch;
@@ -475,9 +490,12 @@ int fwd_gelu_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const
                         ((c.flags & MNI_B200_FORCE_TENSOR_PATH) == 0 && s.M <= skinny_fwd_row_limit(s.N));
     if (s.K > 0 && !skinny) {
         GemmProblem p;
-        rc = make_operand(c, *a, false, p.A);
+        mni_b200_view packed[kMaxGathers];
+        rc = pack_undescribable(c, {&a, &b}, packed);
         if (rc) return rc;
-        rc = make_operand(c, *b, true, p.B);
+        rc = make_operand(*a, false, p.A);
+        if (rc) return rc;
+        rc = make_operand(*b, true, p.B);
         if (rc) return rc;
         p.A.batch = s.a_batch;
         p.B.batch = s.b_batch;
@@ -606,6 +624,16 @@ int bwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const mni_
     const bool share_sms = overlap && da_wanted && db_wanted && !skinny_dx && !skinny_dw && env_flag("MNI_B200_BWD_SHARE_SMS", 1);
     if (share_sms) c.sm_share = 2;
     cudaStream_t const main_stream = c.stream;
+    // Operands of the tensor path that have to be gathered: once each, before the streams part.
+    mni_b200_view packed[kMaxGathers];
+    const bool da_tensor = da_wanted && !skinny_dx, db_tensor = db_wanted && !skinny_dw;
+    const mni_b200_view *const dc_given = dc, *const a_given = a, *const b_given = b;
+    c.label = "operands: ";
+    if (da_tensor && db_tensor) rc = pack_undescribable(c, {&dc, &b, &a}, packed);
+    else if (da_tensor) rc = pack_undescribable(c, {&dc, &b}, packed);
+    else if (db_tensor) rc = pack_undescribable(c, {&dc, &a}, packed);
+    c.label = "";
+    if (rc) return rc;
     const bool fork = !c.dry() && (overlap || side_dbias);
     if (fork) {
         MNI_CUDA(cudaEventRecord(c.st->ev_fork, main_stream));
@@ -635,29 +663,27 @@ int bwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const mni_
             rc = zero_or_bias_fill(c, dbias, 1, s.N, nullptr, acc_dbias);
             if (rc) return rc;
         } else {
-            mni_b200_view flat = *dc;
-            const float *src = dc->ptr;
-            int64_t ld = s.N;
-            bool contiguous = true;
-            {
+            // a gathered dc serves here too: its rows follow one another at the padded pitch
+            mni_b200_view flat;
+            const mni_b200_view *rows_of = dc;
+            if (dc == dc_given) {
+                bool contiguous = true;
                 int64_t expect = 1;
                 for (int d = gn - 1; d >= 0; --d) {
                     if (dc->shape[d] != 1 && dc->stride[d] != expect) contiguous = false;
                     expect *= dc->shape[d];
                 }
-            }
-            if (!contiguous) {
-                size_t off;
-                rc = pack_view(c, *dc, &flat, &off);
+                const mni_b200_view **use = &rows_of;
+                if (!contiguous) rc = pack_views(c, &use, &flat, 1);
                 if (rc) return rc;
-                src = flat.ptr;
-                ld = flat.stride[1];
             }
+            const float *src = rows_of->ptr;
+            const int64_t ld = rows_of == dc_given ? s.N : rows_of->stride[1];
             const size_t pbytes = colsum_partial_bytes(rows, s.N, c.st->sm_count);
             const size_t poff = c.arena.reserve(pbytes);
             c.note(side_dbias ? "column sums, on the side stream" : "column sums");
             if (!c.dry()) {
-                rc = launch_colsum(src, ld, dbias, rows, s.N, acc_dbias, c.at(poff), c.st->sm_count, c.stream);
+                rc = launch_colsum(src, ld, nullptr, dbias, rows, s.N, acc_dbias, c.at(poff), c.st->sm_count, c.stream);
                 if (rc) return rc;
             }
         }
@@ -674,23 +700,23 @@ int bwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const mni_
         } else if (skinny_dx) {
             c.note("streaming (skinny) input-gradient kernel");
             if (!c.dry()) {
-                rc = launch_skinny_dx(dc->ptr, dc->stride[gn - 2], b->ptr, b->stride[b->ndim - 2], da, s.K, acc_da,
+                rc = launch_skinny_dx(dc_given->ptr, dc_given->stride[gn - 2], b_given->ptr, b_given->stride[b_given->ndim - 2], da, s.K, acc_da,
                                       s.M, s.N, s.K, c.stream);
                 if (rc) return rc;
             }
         } else {
             int64_t ob[MNI_B200_MAX_DIMS];
-            const int onb = broadcast_shape(dc->shape, gn - 2, b->shape, b->ndim - 2, ob);
+            const int onb = broadcast_shape(dc_given->shape, gn - 2, b_given->shape, b_given->ndim - 2, ob);
             if (onb < 0) return fail(MNI_B200_ERR_BROADCAST, "dc and b batch shapes are not broadcastable");
             Operand X, Y;
-            rc = make_operand(c, *dc, false, X);   // rows M, contraction N
+            rc = make_operand(*dc, false, X);   // rows M, contraction N
             if (rc) return rc;
-            rc = make_operand(c, *b, false, Y);    // rows K, contraction N
+            rc = make_operand(*b, false, Y);    // rows K, contraction N
             if (rc) return rc;
             X.batch = g_batch;
             Y.batch = s.b_batch;
             c.dep_mode = pair ? 1 : 0;
-            rc = grad_gemm(c, X, Y, s.M, s.K, s.N, ob, onb, *a, da, acc_da);
+            rc = grad_gemm(c, X, Y, s.M, s.K, s.N, ob, onb, *a_given, da, acc_da);
             c.dep_mode = 0;
             if (rc) return rc;
         }
@@ -706,26 +732,23 @@ int bwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const mni_
         } else if (skinny_dw) {
             c.note("streaming (skinny) weight-gradient kernel");
             if (!c.dry()) {
-                rc = launch_skinny_dw(a->ptr, a->stride[a->ndim - 2], dc->ptr, dc->stride[gn - 2], db, s.N, acc_db,
+                rc = launch_skinny_dw(a_given->ptr, a_given->stride[a_given->ndim - 2], dc_given->ptr, dc_given->stride[gn - 2], db, s.N, acc_db,
                                       s.M, s.N, s.K, c.stream);
                 if (rc) return rc;
             }
         } else {
             int64_t ob[MNI_B200_MAX_DIMS];
-            const int onb = broadcast_shape(a->shape, a->ndim - 2, dc->shape, gn - 2, ob);
+            const int onb = broadcast_shape(a_given->shape, a_given->ndim - 2, dc_given->shape, gn - 2, ob);
             if (onb < 0) return fail(MNI_B200_ERR_BROADCAST, "a and dc batch shapes are not broadcastable");
             Operand X, Y;
-            const size_t used_before = c.arena.used;
-            rc = make_operand(c, *a, true, X);     // rows K, contraction M
+            rc = make_operand(*a, true, X);     // rows K, contraction M
             if (rc) return rc;
-            rc = make_operand(c, *dc, true, Y);    // rows N, contraction M
+            rc = make_operand(*dc, true, Y);    // rows N, contraction M
             if (rc) return rc;
             X.batch = s.a_batch;
             Y.batch = g_batch;
-            // An operand that had to be gathered first makes this product depend on the gather kernel just
-            // launched: then it waits like any other launch.
-            if (pair && c.arena.used == used_before) { c.dep_mode = 2; c.flag_bank = 1; }
-            rc = grad_gemm(c, X, Y, s.K, s.N, s.M, ob, onb, *b, db, acc_db);
+            if (pair) { c.dep_mode = 2; c.flag_bank = 1; }
+            rc = grad_gemm(c, X, Y, s.K, s.N, s.M, ob, onb, *b_given, db, acc_db);
             c.dep_mode = 0;
             if (rc) return rc;
         }
@@ -880,16 +903,12 @@ int mni_b200_add_bias_bwd(const float *dy, float *d_y, float *dbias, int64_t row
     if (rows < 0 || n < 0) return fail(MNI_B200_ERR_ARG, "negative extent");
     if (!dy && rows * n > 0) return fail(MNI_B200_ERR_ARG, "dy is null");
     return with_scratch(flags, stream, [&](Call &c) -> int {
-        if (d_y && d_y != dy && !c.dry()) {
-            int rc = launch_copy(dy, d_y, rows * n, c.stream);
-            if (rc) return rc;
-        }
-        if (!dbias || n == 0) return MNI_B200_OK;
+        if (!dbias || n == 0) return c.dry() ? static_cast<int>(MNI_B200_OK) : launch_copy(dy, d_y, rows * n, c.stream);
         const bool acc = (flags & MNI_B200_ACCUMULATE_DBIAS) != 0;
         if (rows == 0) return zero_or_bias_fill(c, dbias, 1, n, nullptr, acc);
         const size_t poff = c.arena.reserve(colsum_partial_bytes(rows, n, c.st->sm_count));
         if (c.dry()) return MNI_B200_OK;
-        return launch_colsum(dy, n, dbias, rows, n, acc, c.at(poff), c.st->sm_count, c.stream);
+        return launch_colsum(dy, n, d_y != dy ? d_y : nullptr, dbias, rows, n, acc, c.at(poff), c.st->sm_count, c.stream);
     });
 }
 
@@ -1038,7 +1057,8 @@ int mni_b200_contiguous(const mni_b200_view *src, float *dst, void *stream) {
     DeviceState *st = nullptr;
     rc = device_state(&st);
     if (rc) return rc;
-    return launch_pack(*src, dst, src->shape[src->ndim - 1], static_cast<cudaStream_t>(stream));
+    const GatherView job{src, dst, src->shape[src->ndim - 1]};
+    return launch_gather(&job, 1, static_cast<cudaStream_t>(stream));
 }
 
 int mni_b200_sm_reserve(int sms) {

@@ -46,6 +46,30 @@ cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, si
 }
 #endif
 
+// Division by a launch-time constant as a multiply-high and a shift (exact for 0 <= n < 2^31): every role
+// decodes every tile it visits, and with short contractions a handful of hardware divisions per tile showed
+// up as 1 250 cycles of a 3 000-cycle main loop.  mul = ceil(2^(31 + ceil(log2 d)) / d), shr = ceil(log2 d) - 1.
+struct FastDiv {
+    uint32_t mul, shr, d;
+};
+inline FastDiv make_fastdiv(long long d_in) {
+    FastDiv f;
+    const uint32_t d = static_cast<uint32_t>(d_in < 1 ? 1 : d_in);
+    f.d = d;
+    if (d == 1) { f.mul = 0; f.shr = 0; return f; }
+    uint32_t l = 0;
+    while ((1ull << l) < d) ++l;
+    const uint32_t p = 31 + l;
+    f.mul = static_cast<uint32_t>(((1ull << p) + d - 1) / d);
+    f.shr = p - 32;
+    return f;
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ int fd_div(int n, const FastDiv &f) {
+    return f.d == 1 ? n : static_cast<int>(__umulhi(static_cast<uint32_t>(n), f.mul) >> f.shr);
+}
+#endif
+
 // ---------------------------------------------------------------------------
 // error plumbing
 // ---------------------------------------------------------------------------
@@ -156,7 +180,8 @@ int launch_skinny_dw(const float *x, int64_t ldx, const float *dy, int64_t lddy,
 int launch_add_bias(const float *y, const float *bias, float *out, int64_t rows, int64_t n,
                     cudaStream_t stream);
 size_t colsum_partial_bytes(int64_t rows, int64_t n, int sm_count);
-int launch_colsum(const float *dy, int64_t ld, float *out, int64_t rows, int64_t n, bool accumulate,
+// out = column sums of dy[rows, n] (row pitch ld); copy != null also receives dy (pitch n) in the same pass
+int launch_colsum(const float *dy, int64_t ld, float *copy, float *out, int64_t rows, int64_t n, bool accumulate,
                   float *partial, int sm_count, cudaStream_t stream);
 int launch_copy(const float *src, float *dst, int64_t n, cudaStream_t stream);
 int launch_softmax_fwd(const float *x, float *out, int64_t outer, int64_t dim, int64_t inner, cudaStream_t stream);
@@ -183,8 +208,14 @@ int launch_bias_gelu(const float *x, const float *bias, float *out, int64_t rows
 int launch_bias_gelu_bwd(const float *grad, const float *x, const float *bias, float *dx, float *dbias,
                          int64_t rows, int64_t n, bool accumulate, float *partial, int sm_count,
                          cudaStream_t stream);
-// dst[row-major, ld_dst on the last dim] = gather of a strided view
-int launch_pack(const mni_b200_view &src, float *dst, int64_t ld_dst, cudaStream_t stream);
+// dst[row-major, ld_dst on the last dim] = gather of a strided view; several views of a call in one launch (gather.cu)
+struct GatherView {
+    const mni_b200_view *src;
+    float *dst;
+    int64_t ld_dst;
+};
+constexpr int kMaxGathers = 3;
+int launch_gather(const GatherView *views, int count, cudaStream_t stream);
 // device-side utils::unbroadcast: out[orig] (+)= sum over broadcast dims of grad[gshape]
 int launch_unbroadcast(const float *grad, const int64_t *gshape, int gnd, const int64_t *oshape, int ond,
                        float *out, bool accumulate, cudaStream_t stream);

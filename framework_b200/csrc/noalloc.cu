@@ -93,14 +93,10 @@ extern "C" MNI_B200_API int mni_b200_add_bias_bwd_noalloc(const float *dy, float
                              "holds %zu; use mni_b200_add_bias_bwd for this size",
                              (long long)rows, (long long)n, need, kNoAllocScratchBytes);
     }
-    if (d_y && d_y != dy) {
-        rc = mni::launch_copy(dy, d_y, rows * n, s);
-        if (rc) return rc;
-    }
-    if (!dbias || n == 0) return MNI_B200_OK;
+    if (!dbias || n == 0) return mni::launch_copy(dy, d_y, rows * n, s);
     if (rows == 0) {
         if (!accumulate) MNI_CUDA(cudaMemsetAsync(dbias, 0, static_cast<size_t>(n) * sizeof(float), s));
         return MNI_B200_OK;
     }
-    return mni::launch_colsum(dy, n, dbias, rows, n, accumulate, st->scratch, st->sm_count, s);
+    return mni::launch_colsum(dy, n, d_y != dy ? d_y : nullptr, dbias, rows, n, accumulate, st->scratch, st->sm_count, s);
 }
