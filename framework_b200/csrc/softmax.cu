@@ -2,8 +2,8 @@
 // attention-shaped use of the batched GEMM (ops/norm.rs:52-89, :125-163; kernels/softmax.cu).
 // HBM-bound: the forward reads x once and writes out once (8 bytes per element), the backward reads
 // dy and out once and writes dx once (12 bytes per element).  A row that fits a warp's registers
-// (<= 2048 elements, length a multiple of 4) never leaves them between the max, the sum and the
-// division; other shapes take a block-per-row or a block-per-32-columns loop over the same arithmetic.
+// (<= 2048 elements; <= 1024 where rows are not 16-byte aligned, as with an odd length) never leaves them between
+// the max, the sum and the division; other shapes take a block-per-row or a block-per-32-columns loop over the same arithmetic.
 #include "internal.h"
 
 #include <algorithm>
@@ -26,70 +26,84 @@ __device__ __forceinline__ float warp_sum(float x) {
     return x;
 }
 
-// Row in registers: lane l holds float4 chunks l, l+32, ... (CH of them; chunk index < len4 is live).
-template <int CH>
+// Row in registers: lane l holds units l, l+32, ... (CH of them; unit index < len is live).  A unit is a float4 where the
+// rows are 16-byte aligned, a float where they are not (an odd length): the warp's loads are contiguous either way.
+__device__ __forceinline__ float unit_max(const float &v) { return v; }
+__device__ __forceinline__ float unit_max(const float4 &v) { return fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)); }
+__device__ __forceinline__ float unit_exp(float &v, float mx) { v = expf(v - mx); return v; }
+__device__ __forceinline__ float unit_exp(float4 &v, float mx) {
+    v.x = expf(v.x - mx); v.y = expf(v.y - mx);
+    v.z = expf(v.z - mx); v.w = expf(v.w - mx);
+    return (v.x + v.y) + (v.z + v.w);
+}
+__device__ __forceinline__ float unit_div(const float &v, float s) { return v / s; }
+__device__ __forceinline__ float4 unit_div(const float4 &v, float s) { return make_float4(v.x / s, v.y / s, v.z / s, v.w / s); }
+__device__ __forceinline__ float unit_dot(const float &g, const float &s) { return g * s; }
+__device__ __forceinline__ float unit_dot(const float4 &g, const float4 &s) { return (g.x * s.x + g.y * s.y) + (g.z * s.z + g.w * s.w); }
+__device__ __forceinline__ float unit_grad(const float &g, const float &s, float dot) { return s * (g - dot); }
+__device__ __forceinline__ float4 unit_grad(const float4 &g, const float4 &s, float dot) {
+    return make_float4(s.x * (g.x - dot), s.y * (g.y - dot), s.z * (g.z - dot), s.w * (g.w - dot));
+}
+
+template <typename V, int CH>
 __global__ void __launch_bounds__(kRowsPerBlock * 32)
-softmax_rows_fwd_kernel(const float4 *__restrict__ x, float4 *__restrict__ out, long long rows, int len4) {
+softmax_rows_fwd_kernel(const V *__restrict__ x, V *__restrict__ out, long long rows, int len) {
+    grid_dependency_trigger();
     const long long row = blockIdx.x * static_cast<long long>(kRowsPerBlock) + (threadIdx.x >> 5);
-    if (row >= rows) return;
     const int lane = threadIdx.x & 31;
-    const float4 *xr = x + row * len4;
-    float4 v[CH];
+    grid_dependency_wait();
+    if (row >= rows) return;
+    const V *xr = x + row * len;
+    V v[CH];
     float mx = kNegInf;
 #pragma unroll
     for (int c = 0; c < CH; ++c) {
         const int i = c * 32 + lane;
-        if (i < len4) {
+        if (i < len) {
             v[c] = __ldcs(xr + i);
-            mx = fmaxf(fmaxf(fmaxf(mx, v[c].x), fmaxf(v[c].y, v[c].z)), v[c].w);
+            mx = fmaxf(mx, unit_max(v[c]));
         }
     }
     mx = warp_max(mx);
     float sum = 0.f;
 #pragma unroll
-    for (int c = 0; c < CH; ++c) {
-        if (c * 32 + lane < len4) {
-            v[c].x = expf(v[c].x - mx); v[c].y = expf(v[c].y - mx);
-            v[c].z = expf(v[c].z - mx); v[c].w = expf(v[c].w - mx);
-            sum += (v[c].x + v[c].y) + (v[c].z + v[c].w);
-        }
-    }
+    for (int c = 0; c < CH; ++c)
+        if (c * 32 + lane < len) sum += unit_exp(v[c], mx);
     sum = warp_sum(sum);
-    float4 *orow = out + row * len4;
+    V *orow = out + row * len;
 #pragma unroll
     for (int c = 0; c < CH; ++c) {
         const int i = c * 32 + lane;
-        if (i < len4) orow[i] = make_float4(v[c].x / sum, v[c].y / sum, v[c].z / sum, v[c].w / sum);
+        if (i < len) orow[i] = unit_div(v[c], sum);
     }
 }
 
-template <int CH>
+template <typename V, int CH>
 __global__ void __launch_bounds__(kRowsPerBlock * 32)
-softmax_rows_bwd_kernel(const float4 *__restrict__ dy, const float4 *__restrict__ out, float4 *__restrict__ dx,
-                        long long rows, int len4) {
+softmax_rows_bwd_kernel(const V *__restrict__ dy, const V *__restrict__ out, V *__restrict__ dx, long long rows, int len) {
+    grid_dependency_trigger();
     const long long row = blockIdx.x * static_cast<long long>(kRowsPerBlock) + (threadIdx.x >> 5);
-    if (row >= rows) return;
     const int lane = threadIdx.x & 31;
-    const float4 *gr = dy + row * len4, *sr = out + row * len4;
-    float4 g[CH], s[CH];
+    grid_dependency_wait();
+    if (row >= rows) return;
+    const V *gr = dy + row * len, *sr = out + row * len;
+    V g[CH], s[CH];
     float dot = 0.f;
 #pragma unroll
     for (int c = 0; c < CH; ++c) {
         const int i = c * 32 + lane;
-        if (i < len4) {
+        if (i < len) {
             g[c] = __ldcs(gr + i);
             s[c] = __ldcs(sr + i);
-            dot += (g[c].x * s[c].x + g[c].y * s[c].y) + (g[c].z * s[c].z + g[c].w * s[c].w);
+            dot += unit_dot(g[c], s[c]);
         }
     }
     dot = warp_sum(dot);
-    float4 *drow = dx + row * len4;
+    V *drow = dx + row * len;
 #pragma unroll
     for (int c = 0; c < CH; ++c) {
         const int i = c * 32 + lane;
-        if (i < len4)
-            drow[i] = make_float4(s[c].x * (g[c].x - dot), s[c].y * (g[c].y - dot), s[c].z * (g[c].z - dot),
-                                  s[c].w * (g[c].w - dot));
+        if (i < len) drow[i] = unit_grad(g[c], s[c], dot);
     }
 }
 
@@ -194,11 +208,59 @@ softmax_cols_bwd_kernel(const float *__restrict__ dy, const float *__restrict__ 
 
 bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-int chunks_for(long long len) {          // float4 chunks per lane, rounded up to a compiled variant
-    const long long need = (len / 4 + 31) / 32;
-    for (int ch : {1, 2, 4, 8, 16})
-        if (need <= ch) return ch;
+// Units per lane of a row of `units`, rounded up to a compiled variant (0: the row does not fit `most` of them).
+int chunks_for(long long units, int most) {
+    const long long need = (units + 31) / 32;
+    for (int ch : {1, 2, 4, 8, 16, 32})
+        if (need <= ch) return ch <= most ? ch : 0;
     return 0;
+}
+
+template <typename V>
+using RowsFwd = void (*)(const V *, V *, long long, int);
+template <typename V>
+using RowsBwd = void (*)(const V *, const V *, V *, long long, int);
+template <typename V>
+RowsFwd<V> rows_fwd(int ch) {
+    switch (ch) {
+        case 1: return softmax_rows_fwd_kernel<V, 1>;
+        case 2: return softmax_rows_fwd_kernel<V, 2>;
+        case 4: return softmax_rows_fwd_kernel<V, 4>;
+        case 8: return softmax_rows_fwd_kernel<V, 8>;
+        case 16: return softmax_rows_fwd_kernel<V, 16>;
+        default: return softmax_rows_fwd_kernel<V, sizeof(V) == 4 ? 32 : 16>;
+    }
+}
+template <typename V>
+RowsBwd<V> rows_bwd(int ch) {
+    switch (ch) {
+        case 1: return softmax_rows_bwd_kernel<V, 1>;
+        case 2: return softmax_rows_bwd_kernel<V, 2>;
+        case 4: return softmax_rows_bwd_kernel<V, 4>;
+        case 8: return softmax_rows_bwd_kernel<V, 8>;
+        case 16: return softmax_rows_bwd_kernel<V, sizeof(V) == 4 ? 16 : 8>;
+        default: return softmax_rows_bwd_kernel<V, sizeof(V) == 4 ? 32 : 8>;
+    }
+}
+
+template <typename V>
+int launch_rows_fwd(const float *x, float *out, int64_t rows, int64_t dim, int ch, cudaStream_t stream) {
+    const dim3 grid(static_cast<unsigned>((rows + kRowsPerBlock - 1) / kRowsPerBlock));
+    const cudaError_t e = launch_dependent(rows_fwd<V>(ch), grid, dim3(kRowsPerBlock * 32), 0, stream, reinterpret_cast<const V *>(x),
+                                           reinterpret_cast<V *>(out), rows, static_cast<int>(dim * sizeof(float) / sizeof(V)));
+    if (e != cudaSuccess) return fail(MNI_B200_ERR_CUDA, "softmax launch failed: %s", cudaGetErrorString(e));
+    MNI_LAUNCH_CHECK("softmax_rows_fwd");
+    return MNI_B200_OK;
+}
+template <typename V>
+int launch_rows_bwd(const float *dy, const float *out, float *dx, int64_t rows, int64_t dim, int ch, cudaStream_t stream) {
+    const dim3 grid(static_cast<unsigned>((rows + kRowsPerBlock - 1) / kRowsPerBlock));
+    const cudaError_t e = launch_dependent(rows_bwd<V>(ch), grid, dim3(kRowsPerBlock * 32), 0, stream, reinterpret_cast<const V *>(dy),
+                                           reinterpret_cast<const V *>(out), reinterpret_cast<V *>(dx), rows,
+                                           static_cast<int>(dim * sizeof(float) / sizeof(V)));
+    if (e != cudaSuccess) return fail(MNI_B200_ERR_CUDA, "softmax launch failed: %s", cudaGetErrorString(e));
+    MNI_LAUNCH_CHECK("softmax_rows_bwd");
+    return MNI_B200_OK;
 }
 
 }  // namespace
@@ -206,22 +268,10 @@ int chunks_for(long long len) {          // float4 chunks per lane, rounded up t
 int launch_softmax_fwd(const float *x, float *out, int64_t outer, int64_t dim, int64_t inner, cudaStream_t stream) {
     if (outer * dim * inner == 0) return MNI_B200_OK;
     if (inner == 1) {
-        const int ch = (dim % 4 == 0 && aligned16(x) && aligned16(out)) ? chunks_for(dim) : 0;
-        if (ch) {
-            const int len4 = static_cast<int>(dim / 4);
-            const unsigned blocks = static_cast<unsigned>((outer + kRowsPerBlock - 1) / kRowsPerBlock);
-            const float4 *x4 = reinterpret_cast<const float4 *>(x);
-            float4 *o4 = reinterpret_cast<float4 *>(out);
-            switch (ch) {
-                case 1: softmax_rows_fwd_kernel<1><<<blocks, kRowsPerBlock * 32, 0, stream>>>(x4, o4, outer, len4); break;
-                case 2: softmax_rows_fwd_kernel<2><<<blocks, kRowsPerBlock * 32, 0, stream>>>(x4, o4, outer, len4); break;
-                case 4: softmax_rows_fwd_kernel<4><<<blocks, kRowsPerBlock * 32, 0, stream>>>(x4, o4, outer, len4); break;
-                case 8: softmax_rows_fwd_kernel<8><<<blocks, kRowsPerBlock * 32, 0, stream>>>(x4, o4, outer, len4); break;
-                default: softmax_rows_fwd_kernel<16><<<blocks, kRowsPerBlock * 32, 0, stream>>>(x4, o4, outer, len4); break;
-            }
-            MNI_LAUNCH_CHECK("softmax_rows_fwd");
-            return MNI_B200_OK;
-        }
+        // a lane holds up to 16 16-byte units (2048 elements a row), or up to 32 elements (1024) of a row that is not aligned
+        const bool aligned = dim % 4 == 0 && aligned16(x) && aligned16(out);
+        if (const int ch = aligned ? chunks_for(dim / 4, 16) : 0) return launch_rows_fwd<float4>(x, out, outer, dim, ch, stream);
+        if (const int ch = aligned ? 0 : chunks_for(dim, 32)) return launch_rows_fwd<float>(x, out, outer, dim, ch, stream);
         softmax_long_fwd_kernel<<<static_cast<unsigned>(outer), kBlockThreads, 0, stream>>>(x, out, dim);
         MNI_LAUNCH_CHECK("softmax_long_fwd");
         return MNI_B200_OK;
@@ -237,21 +287,10 @@ int launch_softmax_bwd(const float *dy, const float *out, float *dx, int64_t out
                        cudaStream_t stream) {
     if (outer * dim * inner == 0) return MNI_B200_OK;
     if (inner == 1) {
-        const int ch = (dim % 4 == 0 && aligned16(dy) && aligned16(out) && aligned16(dx)) ? chunks_for(dim) : 0;
-        if (ch && ch <= 8) {              // two rows live in registers here: 1024 elements at most
-            const int len4 = static_cast<int>(dim / 4);
-            const unsigned blocks = static_cast<unsigned>((outer + kRowsPerBlock - 1) / kRowsPerBlock);
-            const float4 *g4 = reinterpret_cast<const float4 *>(dy), *s4 = reinterpret_cast<const float4 *>(out);
-            float4 *d4 = reinterpret_cast<float4 *>(dx);
-            switch (ch) {
-                case 1: softmax_rows_bwd_kernel<1><<<blocks, kRowsPerBlock * 32, 0, stream>>>(g4, s4, d4, outer, len4); break;
-                case 2: softmax_rows_bwd_kernel<2><<<blocks, kRowsPerBlock * 32, 0, stream>>>(g4, s4, d4, outer, len4); break;
-                case 4: softmax_rows_bwd_kernel<4><<<blocks, kRowsPerBlock * 32, 0, stream>>>(g4, s4, d4, outer, len4); break;
-                default: softmax_rows_bwd_kernel<8><<<blocks, kRowsPerBlock * 32, 0, stream>>>(g4, s4, d4, outer, len4); break;
-            }
-            MNI_LAUNCH_CHECK("softmax_rows_bwd");
-            return MNI_B200_OK;
-        }
+        const bool aligned = dim % 4 == 0 && aligned16(dy) && aligned16(out) && aligned16(dx);
+        // two rows live in registers here: 1024 elements at most
+        if (const int ch = aligned ? chunks_for(dim / 4, 8) : 0) return launch_rows_bwd<float4>(dy, out, dx, outer, dim, ch, stream);
+        if (const int ch = aligned ? 0 : chunks_for(dim, 32)) return launch_rows_bwd<float>(dy, out, dx, outer, dim, ch, stream);
         softmax_long_bwd_kernel<<<static_cast<unsigned>(outer), kBlockThreads, 0, stream>>>(dy, out, dx, dim);
         MNI_LAUNCH_CHECK("softmax_long_bwd");
         return MNI_B200_OK;
