@@ -65,28 +65,6 @@ constexpr long long kWaitCycles = 4000000000LL;            // default limit of e
 enum OperandMode { kKMajor = 0, kMnMultiBox = 1, kMnSingleBox = 2 };
 enum EpilogueMode { kEpiPlainStores = 0, kEpiTmaStore = 1, kEpiTmaReduce = 2, kEpiVectorStores = 3 };
 
-// Division by a launch-time constant as a multiply-high and a shift (exact for 0 <= n < 2^31): every role
-// decodes every tile it visits, and with short contractions a handful of hardware divisions per tile showed
-// up as 1 250 cycles of a 3 000-cycle main loop.  mul = ceil(2^(31 + ceil(log2 d)) / d), shr = ceil(log2 d) - 1.
-struct FastDiv {
-    uint32_t mul, shr, d;
-};
-__host__ inline FastDiv make_fastdiv(long long d_in) {
-    FastDiv f;
-    const uint32_t d = static_cast<uint32_t>(d_in < 1 ? 1 : d_in);
-    f.d = d;
-    if (d == 1) { f.mul = 0; f.shr = 0; return f; }
-    uint32_t l = 0;
-    while ((1ull << l) < d) ++l;
-    const uint32_t p = 31 + l;
-    f.mul = static_cast<uint32_t>(((1ull << p) + d - 1) / d);
-    f.shr = p - 32;
-    return f;
-}
-__device__ __forceinline__ int fd_div(int n, const FastDiv &f) {
-    return f.d == 1 ? n : static_cast<int>(__umulhi(static_cast<uint32_t>(n), f.mul) >> f.shr);
-}
-
 struct KParams {
     int M, N;
     int tiles_m, tiles_n, group_m;
@@ -111,7 +89,8 @@ struct KParams {
     uint32_t a_kstep, b_kstep;       // descriptor address advance (16-byte units) per 8-deep k-step
     float *C;
     long long ldc, c_bstride;
-    float *partial;            // split-K: [split][batch][M][N]
+    float *partial;            // split-K: [split][batch][M][partial_ld]
+    long long partial_ld;      // N rounded up to a multiple of 4, so that partials always leave through TMA
     const float *bias;
     int accumulate;
     int transpose_out;         // the kernel computes C^T (operands exchanged): patches are stored transposed, bias is per row
@@ -1079,43 +1058,69 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     } else if (use_tma) {
                         emit(&tmC, (p.epi_mode == kEpiTmaReduce && fuse) || add_piece);
                     } else {
-                        const int row = row0 + lane;
-                        if (row < p.M) {
-                            float *out = fuse ? p.C + static_cast<long long>(t.bt) * p.c_bstride + static_cast<long long>(row) * p.ldc
-                                              : p.partial + (static_cast<long long>(cbatch) * p.M + row) * p.N;
-                            if (p.epi_mode == kEpiVectorStores && col0 + 32 <= p.N) {
-                                // Each lane owns one row: four 32-byte stores write whole sectors, no staging.
-                                float *dst = out + col0;
+                        float *out0 = fuse ? p.C + static_cast<long long>(t.bt) * p.c_bstride + static_cast<long long>(row0) * p.ldc
+                                           : p.partial + (static_cast<long long>(cbatch) * p.M + row0) * p.partial_ld;
+                        const long long pitch = fuse ? p.ldc : p.partial_ld;
+                        const bool add = (fuse && p.accumulate) || add_piece;
+                        if (p.epi_mode == kEpiVectorStores && col0 + 32 <= p.N) {
+                            // Each lane owns one row: four 32-byte stores write whole sectors, no staging.
+                            if (row0 + lane >= p.M) continue;
+                            float *dst = out0 + lane * pitch + col0;
 #pragma unroll
-                                for (int j = 0; j < 4; ++j) {
-                                    float y[8];
+                            for (int j = 0; j < 4; ++j) {
+                                float y[8];
 #pragma unroll
-                                    for (int e = 0; e < 8; ++e) y[e] = __uint_as_float(v[8 * j + e]);
-                                    if ((fuse && p.accumulate) || add_piece) {
-                                        float o[8];
-                                        asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                                                     : "=f"(o[0]), "=f"(o[1]), "=f"(o[2]), "=f"(o[3]), "=f"(o[4]), "=f"(o[5]),
-                                                       "=f"(o[6]), "=f"(o[7])
-                                                     : "l"(dst + 8 * j));
+                                for (int e = 0; e < 8; ++e) y[e] = __uint_as_float(v[8 * j + e]);
+                                if (add) {
+                                    float o[8];
+                                    asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                                                 : "=f"(o[0]), "=f"(o[1]), "=f"(o[2]), "=f"(o[3]), "=f"(o[4]), "=f"(o[5]),
+                                                   "=f"(o[6]), "=f"(o[7])
+                                                 : "l"(dst + 8 * j));
 #pragma unroll
-                                        for (int e = 0; e < 8; ++e) y[e] += o[e];
-                                    }
-                                    asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst + 8 * j),
-                                                 "f"(y[0]), "f"(y[1]), "f"(y[2]), "f"(y[3]), "f"(y[4]), "f"(y[5]), "f"(y[6]),
-                                                 "f"(y[7])
-                                                 : "memory");
+                                    for (int e = 0; e < 8; ++e) y[e] += o[e];
                                 }
-                                continue;
+                                asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst + 8 * j),
+                                             "f"(y[0]), "f"(y[1]), "f"(y[2]), "f"(y[3]), "f"(y[4]), "f"(y[5]), "f"(y[6]),
+                                             "f"(y[7])
+                                             : "memory");
                             }
+                            continue;
+                        }
+                        // Rows that are not 16-byte aligned (an odd width): the patch is turned in the warp's staging
+                        // buffer, so that every store covers 32 neighbouring columns of one row.  Stored straight from
+                        // the accumulator's row-per-lane order each instruction touched 32 rows (attention scores of
+                        // length 333: 75 us a product).
+                        uint8_t *mine = my_stage + lane * 128;
 #pragma unroll
-                            for (int j = 0; j < 32; ++j) {
-                                if (col0 + j < p.N) {
-                                    float y = __uint_as_float(v[j]);
-                                    if ((fuse && p.accumulate) || add_piece) y += out[col0 + j];
-                                    out[col0 + j] = y;
+                        for (int j = 0; j < 8; ++j)
+                            *reinterpret_cast<float4 *>(mine + ((j ^ (lane & 7)) << 4)) =
+                                make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
+                                            __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
+                        __syncwarp();
+                        const int rows = min(32, p.M - row0);
+                        if (col0 + lane < p.N) {
+                            float *dst = out0 + col0 + lane;
+                            const uint8_t *src = my_stage + ((lane & 3) << 2);
+#pragma unroll
+                            for (int r8 = 0; r8 < 32; r8 += 8) {
+                                float y[8];
+#pragma unroll
+                                for (int r = 0; r < 8; ++r)
+                                    y[r] = *reinterpret_cast<const float *>(src + (r8 + r) * 128 + (((lane >> 2) ^ r) << 4));
+                                if (add) {
+                                    float o[8];
+#pragma unroll
+                                    for (int r = 0; r < 8; ++r) o[r] = r8 + r < rows ? dst[(r8 + r) * pitch] : 0.f;
+#pragma unroll
+                                    for (int r = 0; r < 8; ++r) y[r] += o[r];
                                 }
+#pragma unroll
+                                for (int r = 0; r < 8; ++r)
+                                    if (r8 + r < rows) dst[(r8 + r) * pitch] = y[r];
                             }
                         }
+                        __syncwarp();                  // the staging buffer is free again
                     }
                 }
             }
@@ -1177,59 +1182,74 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 }
 
 // Deterministic split-K finish: C = sum_s partial[s] (+ bias) (+ C), splits added in ascending order.
-// One thread per vector of the output (two divisions per thread, none per element); the partials of
-// four splits are in flight at a time.
-template <typename V, typename I>
+// One thread per 16-byte vector of the partials (rows of `pld` floats); the partials of four splits are in flight at a
+// time.  VEC: the output's rows are whole aligned vectors too.  Otherwise (an odd width) a warp turns its 128
+// columns through shared memory, so that its stores cover 32 neighbouring elements.
+template <bool VEC, typename I>
 __global__ void __launch_bounds__(256)
 splitk_reduce_kernel(const float *__restrict__ partial, float *__restrict__ C, long long ldc, long long c_bstride,
-                     const float *__restrict__ bias, int accumulate, int splits, long long rows, int M, int N) {
-    constexpr int W = sizeof(V) / sizeof(float);
+                     const float *__restrict__ bias, int accumulate, int splits, long long rows, int M, int N, int pld) {
+    __shared__ float turn[VEC ? 1 : 256 * 4];
     grid_dependency_trigger();
     grid_dependency_wait();                      // the partials come from the grid before this one
-    const I per_row = static_cast<I>(N / W);
+    const I per_row = static_cast<I>(pld / 4);
+    const I items = static_cast<I>(rows) * per_row;
     const I item = static_cast<I>(blockIdx.x) * 256 + threadIdx.x;
-    if (item >= static_cast<I>(rows) * per_row) return;
-    const I row = item / per_row;
-    const int col = static_cast<int>(item - row * per_row) * W;
-    const I bt = row / static_cast<I>(M);
-    const int m = static_cast<int>(row - bt * static_cast<I>(M));
-    const long long slab = rows * N;
-    const float *src = partial + static_cast<long long>(row) * N + col;
-    float acc[W];
+    if (VEC && item >= items) return;
+    const long long slab = rows * pld;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (item < items) {
+        const float4 *src = reinterpret_cast<const float4 *>(partial) + item;
+        int sp = 0;
+        for (; sp + 4 <= splits; sp += 4) {
+            float4 t[4];
 #pragma unroll
-    for (int e = 0; e < W; ++e) acc[e] = 0.f;
-    int sp = 0;
-    for (; sp + 4 <= splits; sp += 4) {
-        V t[4];
+            for (int u = 0; u < 4; ++u) t[u] = __ldcg(src + (sp + u) * (slab / 4));
 #pragma unroll
-        for (int u = 0; u < 4; ++u) t[u] = __ldcg(reinterpret_cast<const V *>(src + (sp + u) * slab));
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const float *tv = reinterpret_cast<const float *>(&t[u]);
-#pragma unroll
-            for (int e = 0; e < W; ++e) acc[e] += tv[e];
+            for (int u = 0; u < 4; ++u) { acc.x += t[u].x; acc.y += t[u].y; acc.z += t[u].z; acc.w += t[u].w; }
+        }
+        for (; sp < splits; ++sp) {
+            const float4 t = __ldcg(src + sp * (slab / 4));
+            acc.x += t.x; acc.y += t.y; acc.z += t.z; acc.w += t.w;
         }
     }
-    for (; sp < splits; ++sp) {
-        const V t = __ldcg(reinterpret_cast<const V *>(src + sp * slab));
-        const float *tv = reinterpret_cast<const float *>(&t);
-#pragma unroll
-        for (int e = 0; e < W; ++e) acc[e] += tv[e];
+    if (VEC) {
+        const I row = item / per_row;
+        const int col = static_cast<int>(item - row * per_row) * 4;
+        const I bt = row / static_cast<I>(M);
+        const int m = static_cast<int>(row - bt * static_cast<I>(M));
+        if (bias) {
+            const float4 b = __ldg(reinterpret_cast<const float4 *>(bias + col));
+            acc.x += b.x; acc.y += b.y; acc.z += b.z; acc.w += b.w;
+        }
+        float4 *out = reinterpret_cast<float4 *>(C + static_cast<long long>(bt) * c_bstride + static_cast<long long>(m) * ldc + col);
+        if (accumulate) {
+            const float4 c0 = *out;
+            acc.x += c0.x; acc.y += c0.y; acc.z += c0.z; acc.w += c0.w;
+        }
+        *out = acc;
+        return;
     }
-    if (bias) {
-        const V b = __ldg(reinterpret_cast<const V *>(bias + col));
-        const float *bv = reinterpret_cast<const float *>(&b);
+    const int lane = threadIdx.x & 31;
+    float *mine = turn + (threadIdx.x & ~31) * 4;
+    reinterpret_cast<float4 *>(mine)[lane] = acc;
+    __syncwarp();
 #pragma unroll
-        for (int e = 0; e < W; ++e) acc[e] += bv[e];
+    for (int j = 0; j < 4; ++j) {
+        const int e = j * 32 + lane;                           // element within the warp's 128
+        const I at = (item - lane) + e / 4;                    // its vector
+        if (at >= items) continue;
+        const I row = at / per_row;
+        const int col = static_cast<int>(at - row * per_row) * 4 + (e & 3);
+        if (col >= N) continue;
+        const I bt = row / static_cast<I>(M);
+        const int m = static_cast<int>(row - bt * static_cast<I>(M));
+        float *out = C + static_cast<long long>(bt) * c_bstride + static_cast<long long>(m) * ldc + col;
+        float y = mine[e];
+        if (bias) y += __ldg(bias + col);
+        if (accumulate) y += *out;
+        *out = y;
     }
-    V *out = reinterpret_cast<V *>(C + static_cast<long long>(bt) * c_bstride + static_cast<long long>(m) * ldc + col);
-    if (accumulate) {
-        const V c0 = *out;
-        const float *cv = reinterpret_cast<const float *>(&c0);
-#pragma unroll
-        for (int e = 0; e < W; ++e) acc[e] += cv[e];
-    }
-    *out = *reinterpret_cast<const V *>(acc);
 }
 
 // ------------------------------------------------------------------ host side
@@ -1631,13 +1651,15 @@ bool gemm_tc_can_fuse_activation(const GemmProblem &p, int sm_count) {
            env_int("MNI_B200_NO_TMA_STORE", 0) == 0 && env_int("MNI_B200_EPI_VECTOR", 0) == 0;
 }
 
+static int64_t partial_pitch(int64_t n) { return (n + 3) / 4 * 4; }
+
 size_t gemm_tc_partial_bytes(const GemmProblem &p0, int sm_count) {
     bool transposed = false;
     const GemmProblem p = kernel_view(p0, &transposed);
     const Plan pl = make_plan(p, sm_count);
     if (pl.sk) return static_cast<size_t>(pl.grid) * 2 * BM * pl.bn * sizeof(float);   // two parked accumulators per CTA
     if (pl.splits <= 1) return 0;
-    return static_cast<size_t>(pl.splits) * p.batch * p.M * p.N * sizeof(float);
+    return static_cast<size_t>(pl.splits) * p.batch * p0.M * partial_pitch(p0.N) * sizeof(float);
 }
 
 std::string gemm_tc_describe(const GemmProblem &p0, int sm_count) {
@@ -1687,8 +1709,9 @@ int launch_gemm_tc(const GemmProblem &p0, float *partial, uint32_t *err_word, in
 
     // Epilogue: TMA store when the destination rows are 16-byte aligned, plain stores otherwise.
     float *dst = pl.splits > 1 ? partial : p.C;
-    const int64_t dst_ld = pl.splits > 1 ? oN : p.ldc;
-    const int64_t dst_bs = pl.splits > 1 ? p.M * p.N : p.c_bstride;
+    const int64_t pld = partial_pitch(oN);
+    const int64_t dst_ld = pl.splits > 1 ? pld : p.ldc;
+    const int64_t dst_bs = pl.splits > 1 ? oM * pld : p.c_bstride;
     const int64_t dst_batches = pl.splits > 1 ? static_cast<int64_t>(pl.splits) * p.batch : p.batch;
     const bool tma_ok = (reinterpret_cast<uintptr_t>(dst) & 15) == 0 && dst_ld % 4 == 0 && dst_bs % 4 == 0 &&
                         env_int("MNI_B200_NO_TMA_STORE", 0) == 0;
@@ -1769,6 +1792,7 @@ int launch_gemm_tc(const GemmProblem &p0, float *partial, uint32_t *err_word, in
     k.ldc = p.ldc;
     k.c_bstride = p.c_bstride;
     k.partial = partial;
+    k.partial_ld = pld;
     k.bias = p.bias;
     k.accumulate = p.accumulate;
     k.err = err_word;
@@ -1837,20 +1861,15 @@ int launch_gemm_tc(const GemmProblem &p0, float *partial, uint32_t *err_word, in
     if (pl.splits > 1) {
         const long long rows = static_cast<long long>(p.batch) * oM;
         const bool vec = oN % 4 == 0 && p.ldc % 4 == 0 && p.c_bstride % 4 == 0 &&
-                         ((reinterpret_cast<uintptr_t>(p.C) | reinterpret_cast<uintptr_t>(partial) |
-                           reinterpret_cast<uintptr_t>(p.bias)) & 15) == 0;
-        const long long items = rows * (vec ? oN / 4 : oN);
+                         ((reinterpret_cast<uintptr_t>(p.C) | reinterpret_cast<uintptr_t>(p.bias)) & 15) == 0;
+        const long long items = rows * (pld / 4);
         const unsigned blocks = static_cast<unsigned>((items + 255) / 256);
         const bool small = items < (1LL << 31) - 256;
-#define MNI_REDUCE(V_, I_)                                                                                          \
-    e = launch_dependent(splitk_reduce_kernel<V_, I_>, dim3(blocks), dim3(256), 0, stream, partial, p.C, p.ldc,        \
-                         p.c_bstride, p.bias, p.accumulate ? 1 : 0, pl.splits, rows, static_cast<int>(oM),          \
-                         static_cast<int>(oN))
-        if (vec && small) MNI_REDUCE(float4, unsigned);
-        else if (vec) MNI_REDUCE(float4, long long);
-        else if (small) MNI_REDUCE(float, unsigned);
-        else MNI_REDUCE(float, long long);
-#undef MNI_REDUCE
+        auto reduce = vec ? (small ? splitk_reduce_kernel<true, unsigned> : splitk_reduce_kernel<true, long long>)
+                          : (small ? splitk_reduce_kernel<false, unsigned> : splitk_reduce_kernel<false, long long>);
+        e = launch_dependent(reduce, dim3(blocks), dim3(256), 0, stream, partial, p.C, p.ldc, p.c_bstride, p.bias,
+                             p.accumulate ? 1 : 0, pl.splits, rows, static_cast<int>(oM), static_cast<int>(oN),
+                             static_cast<int>(pld));
         if (e != cudaSuccess) return fail(MNI_B200_ERR_CUDA, "splitk_reduce_kernel launch failed: %s", cudaGetErrorString(e));
         MNI_LAUNCH_CHECK("splitk_reduce_kernel");
     }

@@ -1,0 +1,89 @@
+"""Forms of the memory-bound kernels at the sizes where they change or can go wrong: gathers of permuted views, column
+sums with their copy, the bias pass, softmax rows that are not 16-byte aligned, and products whose output rows are not."""
+import numpy as np
+import pytest
+
+from conftest import Guarded, regression_bound_3xtf32, rel_fro
+
+pytestmark = pytest.mark.gpu
+
+
+def _rng(*key):
+    return np.random.default_rng(list(key))
+
+
+@pytest.mark.parametrize("shape,dims", [
+    ((2, 5, 3, 64), (0, 2, 1, 3)),          # rows of 16-byte units
+    ((2, 7, 3, 65), (0, 2, 1, 3)),          # odd rows: an element per unit
+    ((2, 3, 65, 33), (0, 1, 3, 2)),         # transposing tiles, both extents past a tile's edge
+    ((3, 64, 32), (0, 2, 1)),               # exactly one tile each
+    ((2, 3, 8, 130), (0, 3, 1, 2)),         # tiles with dimensions between
+    ((130, 7), (1, 0)),                     # too narrow for tiles
+    ((5, 1, 9), (2, 1, 0)), ((1, 1, 1), (2, 0, 1)), ((4, 6), (0, 1))])
+def test_gather_of_permuted_views(F, shape, dims):
+    a = _rng(1, *shape).standard_normal(shape).astype(np.float32)
+    view = F.DeviceTensor.from_numpy(a).permute(dims)
+    want = np.ascontiguousarray(a.transpose(dims))
+    out = Guarded(F, want.shape)
+    F._lib.check(F._lib.lib().mni_b200_contiguous(view.view_struct(), out.tensor.ptr, 0))
+    out.check("gather")
+    assert np.array_equal(out.tensor.numpy(), want)
+    assert np.array_equal(view.contiguous().numpy(), want)
+    back = F.permute_backward(F.DeviceTensor.from_numpy(want), dims, shape)
+    assert np.array_equal(back.numpy(), a)
+
+
+@pytest.mark.parametrize("rows,n,misalign", [(1, 1, 0), (63, 4, 0), (65, 130, 0), (64, 128, 0), (1000, 516, 0), (129, 260, 1),
+                                             (777, 131, 0), (5000, 33, 0), (40, 200_000, 0)])
+def test_bias_add_and_its_backward(F, rows, n, misalign):
+    rng = _rng(2, rows, n)
+    y, b = rng.standard_normal((rows, n)).astype(np.float32), rng.standard_normal(n).astype(np.float32)
+    dy = Guarded(F, (rows, n), init=y, misalign=misalign)
+    bias = F.DeviceTensor.from_numpy(b)
+    lib, check = F._lib.lib(), F._lib.check
+    out = Guarded(F, (rows, n), misalign=misalign)
+    check(lib.mni_b200_add_bias(dy.tensor.ptr, bias.ptr, out.tensor.ptr, rows, n, 0))
+    out.check("bias add")
+    assert np.array_equal(out.tensor.numpy(), y + b)
+    copy, sums = Guarded(F, (rows, n), misalign=misalign), Guarded(F, (n,))
+    check(lib.mni_b200_add_bias_bwd(dy.tensor.ptr, copy.tensor.ptr, sums.tensor.ptr, rows, n, 0, 0))
+    copy.check("copy of dy")
+    sums.check("column sums")
+    assert np.array_equal(copy.tensor.numpy(), y)
+    exact = y.astype(np.float64).sum(0)
+    bound = 1e-6 * np.sqrt(rows) * np.abs(y).max() + 1e-6
+    assert np.max(np.abs(sums.tensor.numpy() - exact)) <= bound * 8
+    check(lib.mni_b200_add_bias_bwd(dy.tensor.ptr, None, sums.tensor.ptr, rows, n, F._lib.ACCUMULATE_DBIAS, 0))
+    assert np.max(np.abs(sums.tensor.numpy() - 2 * exact)) <= bound * 16
+
+
+@pytest.mark.parametrize("length", [31, 33, 333, 511, 1023, 1025, 2047])
+def test_softmax_rows_of_odd_length(F, length):
+    rng = _rng(3, length)
+    x, dy = (rng.standard_normal((19, length)).astype(np.float32) * 3 for _ in range(2))
+    e = np.exp(x.astype(np.float64) - x.max(-1, keepdims=True))
+    p = e / e.sum(-1, keepdims=True)
+    got = F.softmax(F.DeviceTensor.from_numpy(x))
+    assert np.max(np.abs(got.numpy() - p)) <= 4e-7 + 4e-6 * p.max()
+    s = got.numpy().astype(np.float64)
+    want = s * (dy - (dy * s).sum(-1, keepdims=True))
+    dx = F.softmax_backward(F.DeviceTensor.from_numpy(dy), got)
+    assert np.max(np.abs(dx.numpy() - want)) <= 1e-6 * (1 + np.abs(want).max())
+
+
+@pytest.mark.parametrize("m,k,n,batch,flags", [
+    (130, 64, 257, (), 0), (70, 40, 333, (3,), 0),           # one piece, rows of 257 / 333 floats
+    (256, 1700, 301, (), 0),                                 # pieces added to unaligned rows
+    (300, 512, 129, (), 3 << 16), (64, 260, 777, (2,), 2 << 16)])   # split contraction, padded partials
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_products_with_unaligned_output_rows(F, m, k, n, batch, flags, accumulate):
+    rng = _rng(4, m, k, n)
+    a, b = rng.standard_normal(batch + (m, k)).astype(np.float32), rng.standard_normal(batch + (k, n)).astype(np.float32)
+    bias, c0 = rng.standard_normal(n).astype(np.float32), rng.standard_normal(batch + (m, n)).astype(np.float32)
+    want = a.astype(np.float64) @ b.astype(np.float64) + bias + (c0 if accumulate else 0)
+    out = Guarded(F, want.shape, init=c0 if accumulate else None)
+    F.matmul(F.DeviceTensor.from_numpy(a), F.DeviceTensor.from_numpy(b), F.DeviceTensor.from_numpy(bias), out=out.tensor,
+             flags=flags | F._lib.FORCE_TENSOR_PATH | (F._lib.ACCUMULATE_C if accumulate else 0))
+    F.device_status()
+    out.check("product", fully_written=not accumulate)
+    assert rel_fro(out.tensor.numpy(), want) <= regression_bound_3xtf32(k)
