@@ -75,6 +75,11 @@ double overlap_work_limit() {
 // 17.0 at 12).  The forward's limit depends on which of its two kernels can run: skinny_fwd_row_limit.
 constexpr int64_t kSkinnyDxRows = 5, kSkinnyDwRows = 8;
 
+// Rows up to which the warp-level streaming kernels (rows.cu) take a product the FFMA kernels above do not.  From 16
+// rows, the narrowest tile of the tensor path, that path wastes nothing on an aligned weight; one whose rows are not
+// 16-byte aligned it would have to gather first.
+constexpr int64_t kRowsAligned = 15, kRowsUnaligned = 16;
+
 bool env_flag(const char *name, int dflt) { return env_int(name, dflt) != 0; }
 
 // Bump allocator over the device's scratch.  In dry mode nothing is touched: the
@@ -318,8 +323,10 @@ struct Call {
     cudaStream_t stream;
     uint32_t flags;
     uint8_t *base = nullptr;   // resolved scratch base (real mode, second pass)
+    bool capturing = false;    // the stream records into a graph
     int flag_bank = 0;         // 1 while launches go to the library's side stream / for the second product of a pair
     int dep_mode = 0;          // GemmProblem::dep_mode of the tensor-path launches issued now
+    GemmFinish *defer = nullptr;       // where the next product leaves its split-K finish instead of launching it
     int sm_share = 1;          // 2 while grad_a and grad_b run side by side: each is planned for half of the SMs
     std::string *plan_log = nullptr;   // mni_b200_plan_describe: one line per launch the call would make
     const char *label = "";            // which product the launches logged now belong to
@@ -389,7 +396,7 @@ int run_gemm(Call &c, GemmProblem &p) {
     if (pbytes) poff = c.arena.reserve(pbytes);
     if (c.plan_log) c.note(gemm_tc_describe(p, c.gemm_sms()));
     if (c.dry()) return MNI_B200_OK;
-    return launch_gemm_tc(p, pbytes ? c.at(poff) : nullptr, c.st->err_word, c.gemm_sms(), c.stream);
+    return launch_gemm_tc(p, pbytes ? c.at(poff) : nullptr, c.st->err_word, c.gemm_sms(), c.stream, c.defer);
 }
 
 int zero_or_bias_fill(Call &c, float *out, int64_t rows, int64_t n, const float *bias, bool accumulate) {
@@ -425,6 +432,16 @@ int analyse(const mni_b200_view *a, const mni_b200_view *b, Shapes &s) {
     return MNI_B200_OK;
 }
 
+// Few rows against one weight, not forced onto another path.
+bool rows_wanted(uint32_t flags, const Shapes &s, const mni_b200_view &w) {
+    const int64_t s0 = w.stride[w.ndim - 2], s1 = w.stride[w.ndim - 1];
+    const bool aligned = (reinterpret_cast<uintptr_t>(w.ptr) & 15) == 0 && (s1 == 1 ? s0 : s1) % 4 == 0 &&
+                         (s1 == 1 ? s.N : s.K) % 4 == 0;
+    return (flags & (MNI_B200_FORCE_TENSOR_PATH | MNI_B200_FORCE_SKINNY_PATH | MNI_B200_FORCE_PACK)) == 0 &&
+           ((flags >> 16) & 0xffu) == 0 && s.batch == 1 && s.a_batch == 1 && s.b_batch == 1 &&
+           s.M <= (aligned ? kRowsAligned : kRowsUnaligned);
+}
+
 // ------------------------------------------------------------------ forward
 int fwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, float *out, const float *bias) {
     Shapes s;
@@ -451,6 +468,17 @@ int fwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, float *out
             const int64_t ldw = s.K == 1 ? round_up(s.N, 4) : b->stride[bn - 2];
             return launch_skinny_fwd(a->ptr, a->stride[an - 2], b->ptr, ldw, out, s.N, bias, accumulate, s.M, s.N,
                                      s.K, c.at(poff), c.st->sm_count, c.stream);
+        }
+    }
+
+    if (rows_wanted(c.flags, s, *b) && rows_supported(s.M, s.N, s.K, c.st->sm_count) && (a->stride[a->ndim - 1] == 1 || s.K == 1)) {
+        const int64_t ldx = a->stride[a->ndim - 2], sk = b->stride[b->ndim - 2], sn = b->stride[b->ndim - 1];
+        if (sn == 1 || sk == 1) {                      // W as stored [K, N], or [N, K] seen through a transposing view
+            c.note("streaming (few rows) forward kernel");
+            if (c.dry()) return MNI_B200_OK;
+            auto launch = sn == 1 ? launch_rows_fwd : launch_rows_bt_fwd;
+            return launch(a->ptr, ldx, b->ptr, sn == 1 ? sk : sn, out, s.N, bias, accumulate, s.M, s.N, s.K,
+                          c.st->sm_count, c.stream);
         }
     }
 
@@ -524,21 +552,26 @@ int fwd_gelu_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const
 }
 
 // ------------------------------------------------------------------ backward
+// Whether the target's batch dims, right-aligned against ob, are all equal to it (`same`), or hold a single matrix: then
+// one product writes the gradient, with no unbroadcast after it.
+bool single_product(const int64_t *ob, int onb, const mni_b200_view &target, bool *same) {
+    const int tnb = target.ndim - 2;
+    *same = tnb <= onb;
+    for (int i = 0; *same && i < onb; ++i) {
+        const int64_t td = i < onb - tnb ? 1 : target.shape[i - (onb - tnb)];
+        if (td != ob[i]) *same = false;
+    }
+    return *same || prod(ob, onb) == 1 || prod(target.shape, tnb) == 1;
+}
+
 // One gradient: G[ob.., R, Cn] = X . Y (a GEMM over `kdim`) reduced to `target`'s shape.
 //   X supplies the rows, Y the columns; both already as Operands with flat batch counts.
 int grad_gemm(Call &c, Operand X, Operand Y, int64_t R, int64_t Cn, int64_t kdim, const int64_t *ob, int onb,
               const mni_b200_view &target, float *out, bool accumulate) {
     const int64_t obatch = prod(ob, onb);
-    const int tnb = target.ndim - 2;
-    const int64_t tbatch = prod(target.shape, tnb);
-    bool same = true;
-    {   // target batch dims, right-aligned against ob, all equal?
-        if (tnb > onb) same = false;
-        for (int i = 0; same && i < onb; ++i) {
-            const int64_t td = i < onb - tnb ? 1 : target.shape[i - (onb - tnb)];
-            if (td != ob[i]) same = false;
-        }
-    }
+    const int64_t tbatch = prod(target.shape, target.ndim - 2);
+    bool same = false;
+    single_product(ob, onb, target, &same);
     GemmProblem p;
     p.A = X; p.B = Y;
     p.M = R; p.N = Cn; p.K = kdim;
@@ -601,32 +634,50 @@ int bwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const mni_
                            s.batch == 1 && g_batch == 1 && s.M <= 16 && (a->stride[a->ndim - 1] == 1 || s.K == 1) &&
                            (dc->stride[gn - 1] == 1 || s.N == 1);
 
+    // ... and those of the remaining few-row products that stream the weight through the warp-level kernels
+    const bool rows_ok = rows_wanted(c.flags, s, *b) && g_batch == 1 && (dc->stride[gn - 1] == 1 || s.N == 1);
+    const int64_t b_sk = b->stride[b->ndim - 2], b_sn = b->stride[b->ndim - 1];
+    const bool rows_dx = da_wanted && !skinny_dx && rows_ok && rows_supported(s.M, s.K, s.N, c.st->sm_count) && (b_sn == 1 || b_sk == 1);
+    const bool rows_dw = db_wanted && !skinny_dw && rows_ok && (a->stride[a->ndim - 1] == 1 || s.K == 1);
+    const bool streamed_dx = skinny_dx || rows_dx, streamed_dw = skinny_dw || rows_dw;
+
     // grad_a and grad_b do not depend on each other.  grad_b of a small problem goes to the library's side stream
     // next to grad_a and is joined before returning (event fork / join, also valid under stream capture).  The
     // column sums of the bias gradient are HBM-bound and always go to the side stream, where they run beside the
     // tensor-bound products instead of in front of them.
-    // MNI_B200_BWD_PAIR=1 selects the one-stream alternative for two tensor-core products: launched back to back
-    // as an independent pair (GemmProblem::dep_mode), the second starts on the SMs the first leaves free with no
-    // event in between.  Measured, it does not pay: 512^3 30.9 vs 28.8 us per step under graph replay (the second
-    // product can only start once every CTA of the first has passed its own dependency wait), 58.9 vs 60.8 us
-    // eager, the Linear step 406 vs 405 us -- so it stays off.
+    // Two tensor-core products of a small problem are launched back to back on ONE stream as an independent pair
+    // (GemmProblem::dep_mode: the second starts as soon as every CTA of the first has passed its own dependency wait), then
+    // their finishes.  Under stream capture they go to two branches of the graph instead.  Measured: events between
+    // streams cost an eager call 4-20 us (16 rows x 4096^2: 87 -> 66 us a step; 512^3: 35.0 -> 31.6) but a graph nothing
+    // (512^3: pair 32.1, branches 26.7).  MNI_B200_BWD_PAIR=0 / 1 never / always pairs.
     const double work = static_cast<double>(s.M) * static_cast<double>(s.N) * static_cast<double>(s.K) *
                         static_cast<double>(std::max<int64_t>(g_batch, 1));
     // The decisions are the same in the sizing pass and in the real pass (they change the plans, hence the scratch);
     // only the stream operations are skipped while sizing.
     const bool side_on = env_flag("MNI_B200_BWD_OVERLAP", 1);
-    const bool pair = side_on && da_wanted && db_wanted && !skinny_dx && !skinny_dw && env_flag("MNI_B200_BWD_PAIR", 0);
-    const bool overlap = side_on && !pair && da && db && a_elems > 0 && b_elems > 0 && work > 0 && work <= overlap_work_limit();
+    const bool two_tensor = da_wanted && db_wanted && !streamed_dx && !streamed_dw;
+    const bool small = work > 0 && work <= overlap_work_limit();
+    bool pairable = false;
+    if (side_on && two_tensor) {
+        int64_t oa[MNI_B200_MAX_DIMS], ob[MNI_B200_MAX_DIMS];
+        bool same;
+        const int na = broadcast_shape(dc->shape, gn - 2, b->shape, b->ndim - 2, oa);
+        const int nb = broadcast_shape(a->shape, a->ndim - 2, dc->shape, gn - 2, ob);
+        pairable = na >= 0 && nb >= 0 && single_product(oa, na, *a, &same) && single_product(ob, nb, *b, &same);
+    }
+    const int pair_env = env_int("MNI_B200_BWD_PAIR", -1);
+    const bool pair = pairable && (pair_env > 0 || (pair_env < 0 && small && !c.capturing));
+    const bool overlap = side_on && !pair && da && db && a_elems > 0 && b_elems > 0 && small;
     const bool side_dbias = side_on && dbias && (da || db) && work > 0;
     // Two tensor-core products side by side: each persistent grid is planned for half of the SMs, so that both are
     // resident at once instead of the second queueing behind the first's CTAs (measured under graph replay: 512^3
     // 29.2 -> 24.6 us per step, 1024^3 55.3 -> 45.3 us).
-    const bool share_sms = overlap && da_wanted && db_wanted && !skinny_dx && !skinny_dw && env_flag("MNI_B200_BWD_SHARE_SMS", 1);
+    const bool share_sms = (overlap || pair) && small && two_tensor && env_flag("MNI_B200_BWD_SHARE_SMS", 1);
     if (share_sms) c.sm_share = 2;
     cudaStream_t const main_stream = c.stream;
     // Operands of the tensor path that have to be gathered: once each, before the streams part.
     mni_b200_view packed[kMaxGathers];
-    const bool da_tensor = da_wanted && !skinny_dx, db_tensor = db_wanted && !skinny_dw;
+    const bool da_tensor = da_wanted && !streamed_dx, db_tensor = db_wanted && !streamed_dw;
     const mni_b200_view *const dc_given = dc, *const a_given = a, *const b_given = b;
     c.label = "operands: ";
     if (da_tensor && db_tensor) rc = pack_undescribable(c, {&dc, &b, &a}, packed);
@@ -644,6 +695,7 @@ int bwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const mni_
         ~Join() {
             c.flag_bank = 0;
             c.dep_mode = 0;
+            c.defer = nullptr;
             c.sm_share = 1;
             c.label = "";
             if (!on) return;
@@ -691,6 +743,7 @@ int bwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const mni_
 
     c.stream = main_stream;
 
+    GemmFinish finish_a, finish_b;     // of a pair: launched after both products
     // grad_a = unbroadcast(dc . b^T, a.shape)   (ops/matmul.rs:231-240)
     c.label = "grad_a: ";
     if (da && a_elems > 0) {
@@ -702,6 +755,14 @@ int bwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const mni_
             if (!c.dry()) {
                 rc = launch_skinny_dx(dc_given->ptr, dc_given->stride[gn - 2], b_given->ptr, b_given->stride[b_given->ndim - 2], da, s.K, acc_da,
                                       s.M, s.N, s.K, c.stream);
+                if (rc) return rc;
+            }
+        } else if (rows_dx) {
+            c.note("streaming (few rows) input-gradient kernel");
+            if (!c.dry()) {
+                auto launch = b_sn == 1 ? launch_rows_dx : launch_rows_bt_dx;
+                rc = launch(dc_given->ptr, dc_given->stride[gn - 2], b_given->ptr, b_sn == 1 ? b_sk : b_sn, da, s.K, nullptr, acc_da,
+                            s.M, s.N, s.K, c.st->sm_count, c.stream);
                 if (rc) return rc;
             }
         } else {
@@ -716,6 +777,7 @@ int bwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const mni_
             X.batch = g_batch;
             Y.batch = s.b_batch;
             c.dep_mode = pair ? 1 : 0;
+            c.defer = pair ? &finish_a : nullptr;
             rc = grad_gemm(c, X, Y, s.M, s.K, s.N, ob, onb, *a_given, da, acc_da);
             c.dep_mode = 0;
             if (rc) return rc;
@@ -724,6 +786,7 @@ int bwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const mni_
 
     // grad_b = unbroadcast(a^T . dc, b.shape)   (ops/matmul.rs:242-251)
     if (overlap) { if (!c.dry()) c.stream = c.st->side; c.flag_bank = 1; }
+    c.defer = nullptr;
     c.label = "grad_b: ";
     if (db && b_elems > 0) {
         if (!db_wanted) {
@@ -734,6 +797,13 @@ int bwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const mni_
             if (!c.dry()) {
                 rc = launch_skinny_dw(a_given->ptr, a_given->stride[a_given->ndim - 2], dc_given->ptr, dc_given->stride[gn - 2], db, s.N, acc_db,
                                       s.M, s.N, s.K, c.stream);
+                if (rc) return rc;
+            }
+        } else if (rows_dw) {
+            c.note("streaming (few rows) weight-gradient kernel");
+            if (!c.dry()) {
+                rc = launch_rows_dw(a_given->ptr, a_given->stride[a_given->ndim - 2], dc_given->ptr, dc_given->stride[gn - 2], db,
+                                    s.N, acc_db, s.M, s.N, s.K, c.st->sm_count, c.stream);
                 if (rc) return rc;
             }
         } else {
@@ -747,13 +817,17 @@ int bwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const mni_
             if (rc) return rc;
             X.batch = s.a_batch;
             Y.batch = g_batch;
-            if (pair) { c.dep_mode = 2; c.flag_bank = 1; }
+            if (pair) { c.dep_mode = 2; c.flag_bank = 1; c.defer = &finish_b; }
             rc = grad_gemm(c, X, Y, s.K, s.N, s.M, ob, onb, *b_given, db, acc_db);
             c.dep_mode = 0;
             if (rc) return rc;
         }
     }
-    return MNI_B200_OK;
+    if (!c.dry()) {
+        if (finish_a.splits) rc = launch_gemm_finish(finish_a, c.stream);
+        if (rc == MNI_B200_OK && finish_b.splits) rc = launch_gemm_finish(finish_b, c.stream);
+    }
+    return rc;
 }
 
 // Runs `body` twice: a dry pass that sizes the scratch, then the real pass.
@@ -764,11 +838,14 @@ int with_scratch(uint32_t flags, void *stream, Body body) {
     int rc = device_state(&st);
     if (rc) return rc;
     std::lock_guard<std::mutex> lock(st->mu);
+    const bool capturing = stream_is_capturing(static_cast<cudaStream_t>(stream));
     Call dry;
+    dry.capturing = capturing;
     dry.st = st; dry.arena.st = st; dry.arena.dry = true; dry.stream = static_cast<cudaStream_t>(stream); dry.flags = flags;
     rc = body(dry);
     if (rc) return rc;
     Call real;
+    real.capturing = capturing;
     real.st = st; real.arena.st = st; real.arena.dry = false; real.stream = static_cast<cudaStream_t>(stream); real.flags = flags;
     if (dry.arena.used > 0) {
         rc = scratch_base(*st, dry.arena.used, real.stream, &real.base);

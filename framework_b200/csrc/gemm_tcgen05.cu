@@ -1683,8 +1683,26 @@ std::string gemm_tc_describe(const GemmProblem &p0, int sm_count) {
     return buf;
 }
 
+int launch_gemm_finish(const GemmFinish &f, cudaStream_t stream) {
+    const long long rows = static_cast<long long>(f.batch) * f.M;
+    const int64_t pld = partial_pitch(f.N);
+    const bool vec = f.N % 4 == 0 && f.ldc % 4 == 0 && f.c_bstride % 4 == 0 &&
+                     ((reinterpret_cast<uintptr_t>(f.C) | reinterpret_cast<uintptr_t>(f.bias)) & 15) == 0;
+    const long long items = rows * (pld / 4);
+    const unsigned blocks = static_cast<unsigned>((items + 255) / 256);
+    const bool small = items < (1LL << 31) - 256;
+    auto reduce = vec ? (small ? splitk_reduce_kernel<true, unsigned> : splitk_reduce_kernel<true, long long>)
+                      : (small ? splitk_reduce_kernel<false, unsigned> : splitk_reduce_kernel<false, long long>);
+    const cudaError_t e = launch_dependent(reduce, dim3(blocks), dim3(256), 0, stream, f.partial, f.C, f.ldc, f.c_bstride, f.bias,
+                                           f.accumulate ? 1 : 0, f.splits, rows, static_cast<int>(f.M), static_cast<int>(f.N),
+                                           static_cast<int>(pld));
+    if (e != cudaSuccess) return fail(MNI_B200_ERR_CUDA, "splitk_reduce_kernel launch failed: %s", cudaGetErrorString(e));
+    MNI_LAUNCH_CHECK("splitk_reduce_kernel");
+    return MNI_B200_OK;
+}
+
 int launch_gemm_tc(const GemmProblem &p0, float *partial, uint32_t *err_word, int sm_count,
-                   cudaStream_t stream) {
+                   cudaStream_t stream, GemmFinish *defer) {
     if (p0.M <= 0 || p0.N <= 0 || p0.batch <= 0) return MNI_B200_OK;
     bool transposed = false;
     const GemmProblem p = kernel_view(p0, &transposed);       // p.M / p.N are the kernel's; oM / oN the output's
@@ -1859,19 +1877,9 @@ int launch_gemm_tc(const GemmProblem &p0, float *partial, uint32_t *err_word, in
     if (e != cudaSuccess) return fail(MNI_B200_ERR_CUDA, "gemm_tc_kernel set-up failed: %s", cudaGetErrorString(e));
     MNI_LAUNCH_CHECK("gemm_tc_kernel");
     if (pl.splits > 1) {
-        const long long rows = static_cast<long long>(p.batch) * oM;
-        const bool vec = oN % 4 == 0 && p.ldc % 4 == 0 && p.c_bstride % 4 == 0 &&
-                         ((reinterpret_cast<uintptr_t>(p.C) | reinterpret_cast<uintptr_t>(p.bias)) & 15) == 0;
-        const long long items = rows * (pld / 4);
-        const unsigned blocks = static_cast<unsigned>((items + 255) / 256);
-        const bool small = items < (1LL << 31) - 256;
-        auto reduce = vec ? (small ? splitk_reduce_kernel<true, unsigned> : splitk_reduce_kernel<true, long long>)
-                          : (small ? splitk_reduce_kernel<false, unsigned> : splitk_reduce_kernel<false, long long>);
-        e = launch_dependent(reduce, dim3(blocks), dim3(256), 0, stream, partial, p.C, p.ldc, p.c_bstride, p.bias,
-                             p.accumulate ? 1 : 0, pl.splits, rows, static_cast<int>(oM), static_cast<int>(oN),
-                             static_cast<int>(pld));
-        if (e != cudaSuccess) return fail(MNI_B200_ERR_CUDA, "splitk_reduce_kernel launch failed: %s", cudaGetErrorString(e));
-        MNI_LAUNCH_CHECK("splitk_reduce_kernel");
+        const GemmFinish f{partial, p.C, p.ldc, p.c_bstride, p.batch, oM, oN, p.bias, p.accumulate, pl.splits};
+        if (defer) *defer = f;
+        else return launch_gemm_finish(f, stream);
     }
     return MNI_B200_OK;
 }

@@ -147,8 +147,18 @@ size_t gemm_tc_partial_bytes(const GemmProblem &p, int sm_count);
 
 // Tensor-core path: TMA -> smem -> (hi/lo split) -> tcgen05.mma -> TMEM -> global.
 // `partial` must hold gemm_tc_partial_bytes() bytes when that is non-zero.
+// `defer` != null: the finish of a split contraction is not launched but described there (splits stays 0 if there is none).
+struct GemmFinish {
+    const float *partial = nullptr;
+    float *C = nullptr;
+    int64_t ldc = 0, c_bstride = 0, batch = 0, M = 0, N = 0;
+    const float *bias = nullptr;
+    bool accumulate = false;
+    int splits = 0;
+};
 int launch_gemm_tc(const GemmProblem &p, float *partial, uint32_t *err_word, int sm_count,
-                   cudaStream_t stream);
+                   cudaStream_t stream, GemmFinish *defer = nullptr);
+int launch_gemm_finish(const GemmFinish &f, cudaStream_t stream);
 // One line of text naming the kernel variant, tiling, split and grid launch_gemm_tc would use for this problem
 // on a device with `sm_count` SMs.  Pure host arithmetic: touches no device.
 std::string gemm_tc_describe(const GemmProblem &p, int sm_count);
@@ -175,6 +185,16 @@ int launch_skinny_dx(const float *dy, int64_t lddy, const float *W, int64_t ldw,
 //   dW[K,N] = x[M,K]^T . dy[M,N]                                     M <= 16
 int launch_skinny_dw(const float *x, int64_t ldx, const float *dy, int64_t lddy, float *dW, int64_t lddw,
                      bool accumulate, int64_t M, int64_t N, int64_t K, cudaStream_t stream);
+
+// A few rows (M <= 16) in the split TF32 arithmetic of the tensor path, any alignment of the weight's rows (rows.cu).
+// outs / total: outputs per row and length of the contraction (forward: N, K; dx: K, N).
+bool rows_supported(int64_t M, int64_t outs, int64_t total, int sm_count);
+using RowsLaunch = int(const float *x, int64_t ldx, const float *W, int64_t ldw, float *out, int64_t ldout, const float *bias,
+                       bool accumulate, int64_t M, int64_t N, int64_t K, int sm_count, cudaStream_t stream);
+RowsLaunch launch_rows_fwd, launch_rows_dx;            // W as stored [K, N]
+RowsLaunch launch_rows_bt_fwd, launch_rows_bt_dx;      // W stored [N, K], seen through a transposing view
+int launch_rows_dw(const float *x, int64_t ldx, const float *dy, int64_t lddy, float *dW, int64_t lddw, bool accumulate,
+                   int64_t M, int64_t N, int64_t K, int sm_count, cudaStream_t stream);
 
 // Pointwise / reduction helpers.
 int launch_add_bias(const float *y, const float *bias, float *out, int64_t rows, int64_t n,

@@ -1,0 +1,431 @@
+// A few rows (at most 16) against a large weight, in the split TF32 arithmetic of the tensor path:
+//
+//   forward : y[M,N]  = x[M,K] . W[K,N] (+ bias)
+//   dx      : dx[M,K] = dy[M,N] . W[K,N]^T
+//   dW      : dW[K,N] = x[M,K]^T . dy[M,N]
+//
+// Bound by HBM: the weight is read (dW: written) once, 67 MB = 10.3 us at K = N = 4096 of the measured copy rate.  The
+// warp-level mma.sync is the right matrix instruction here although tcgen05 is several times faster per SM: the
+// 805 M multiply-adds of 16 rows are 5 us of it spread over the warps that stream the weight, with no tensor memory to
+// allocate, no descriptors, no operand staging beyond the ring and an accumulator that is already in registers.  The
+// tcgen05 path takes the same products in 64-wide tiles with a split contraction and a second kernel that sums it, and
+// gathers a weight with an odd row length into scratch first.  Nine rows x 4096 x 4096: forward 20.1 -> 18.0 us, dx 19.9 ->
+// 18.0, the step 79 -> 55; 4096 x 4095: forward 53 -> 30 us, dx 44 -> 34, the step 153 -> 96.
+//
+// Split as in the tensor path: hi = x with the low 13 mantissa bits cut, lo = x - hi, products lo.hi + hi.lo + hi.hi.
+// A chain in the tensor core's accumulator, which truncates, is kFlush elements long; longer sums are added up in
+// registers, and the slices of the contraction in ascending order.
+#include "device_utils.h"
+#include "internal.h"
+
+#include <algorithm>
+
+namespace mni {
+
+namespace {
+
+constexpr int kWarps = 4;                    // each streams 32 x 32 tiles of the weight
+constexpr int kThreads = 32 * kWarps;
+constexpr int kDwCols = 32 * kWarps;         // columns of dW per block
+constexpr int kDepth = 4;                    // 32 x 32 weight tiles held per warp, three in flight: 96 KB per SM with two blocks
+constexpr int kRows = 16;
+constexpr int kFlush = 256;                  // contraction elements summed in one tensor-core accumulator
+constexpr int kMaxSlice = 2048;              // contraction per block (its x is staged whole: 131 KB)
+constexpr int kMaxSlices = 8;                // slices of a strip: one portable cluster
+
+__device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void split(float x, uint32_t &hi, uint32_t &lo) {
+    hi = __float_as_uint(x) & 0xFFFFE000u;
+    lo = __float_as_uint(x - __uint_as_float(hi));
+}
+// acc += a . b in three passes, for the four 8-column tiles of a warp.
+__device__ __forceinline__ void mma_split(float (&acc)[4][4], const uint32_t (&ah)[4], const uint32_t (&al)[4],
+                                          const float (&b0)[4], const float (&b1)[4]) {
+    uint32_t h0[4], l0[4], h1[4], l1[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) { split(b0[j], h0[j], l0[j]); split(b1[j], h1[j], l1[j]); }
+    // pass by pass, so that neighbouring instructions work on different accumulators
+#pragma unroll
+    for (int j = 0; j < 4; ++j) mma_tf32(acc[j], al, h0[j], h1[j]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) mma_tf32(acc[j], ah, l0[j], l1[j]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) mma_tf32(acc[j], ah, h0[j], h1[j]);
+}
+
+// out[m, o] = sum_c x[m, c] . w(c, o), with w(c, o) = W[c, o] (forward) or W[o, c] (DX).
+// grid = (strips of outputs, contraction slices), the slices of a strip one cluster.  WK = 1: the block's four warps take
+// 32 outputs each of a 128-wide strip; WK = 4: they share a 32-wide strip and take every fourth tile of the slice each,
+// which keeps more of the chip busy when the outputs are few.  Every warp streams its part of W through a private ring of 32 x 32 tiles (cp.async: 16-byte pieces where the rows of W are
+// aligned, single floats where they are not -- the loads are contiguous along the row either way), x is staged once per
+// block.  The tile pitch makes the fragment reads conflict-free: 40 floats for 16-byte reads of four neighbouring
+// outputs (forward), 36 for reads down a column (DX).  The slices' sums meet through distributed shared memory.
+template <bool DX, bool VEC, int WK>
+__global__ void __launch_bounds__(kThreads, 2)
+rows_kernel(const float *__restrict__ x, long long ldx, const float *__restrict__ W, long long ldw, float *__restrict__ y,
+            long long ldy, const float *__restrict__ bias, int accumulate, int M, long long outs, long long total, int k_per,
+            int x_vec, int y_vec) {
+    constexpr int PITCH = DX ? 36 : 40;
+    constexpr int OUTS = 32 * (kWarps / WK), SUM_PITCH = OUTS + 4;      // outputs per block
+    extern __shared__ __align__(16) float smem[];
+    const int xp = k_per + 4;                               // = 4 mod 32: the A fragments' scalar reads hit all banks
+    float *xs = smem;                                       // [kRows][xp]
+    float *ring = smem + kRows * xp;                        // [warps][depth][32][PITCH]; later the block's sums
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    const long long k0 = static_cast<long long>(blockIdx.y) * k_per;
+    const int kc = static_cast<int>(min(static_cast<long long>(k_per), total - k0));
+    const int ow = warp / WK, kw = warp % WK;               // this warp's 32 outputs within the block, its share of the tiles
+    const long long o0 = static_cast<long long>(blockIdx.x) * OUTS + ow * 32;
+    const int nb = ((kc + 31) / 32 - kw + WK - 1) / WK;     // tiles kw, kw + WK, ... of the slice
+    float *mine = ring + warp * (kDepth * 32 * PITCH);
+    // extents of this warp's part of W, as rows and columns of W
+    const int rows_live = DX ? static_cast<int>(max(0ll, min(32ll, outs - o0))) : kc;
+    const int cols_live = DX ? kc : static_cast<int>(max(0ll, min(32ll, outs - o0)));
+    const float *wp = DX ? W + o0 * ldw + k0 : W + k0 * ldw + o0;
+    grid_dependency_trigger();
+    grid_dependency_wait();
+    auto issue = [&](int b) {
+        if (b < nb) {
+            float *slot = mine + (b % kDepth) * (32 * PITCH);
+            const int at = (b * WK + kw) * 32, r0 = DX ? 0 : at, c0 = DX ? at : 0;
+            if (VEC) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int r = i * 4 + (lane >> 3), c = (lane & 7) * 4;
+                    const bool ok = r0 + r < rows_live && c0 + c < cols_live;
+                    cp_async16(slot + r * PITCH + c, ok ? wp + (r0 + r) * ldw + c0 + c : W, ok);
+                }
+            } else {
+#pragma unroll 8
+                for (int r = 0; r < 32; ++r) {
+                    const bool ok = r0 + r < rows_live && c0 + lane < cols_live;
+                    cp_async4(slot + r * PITCH + lane, ok ? wp + (r0 + r) * ldw + c0 + lane : W, ok);
+                }
+            }
+        }
+        cp_async_commit();                                  // empty groups keep the count uniform
+    };
+    if (x_vec) {
+        const int quads = k_per / 4;
+        for (int i = threadIdx.x; i < kRows * quads; i += kThreads) {
+            const int m = i / quads, kk = (i - m * quads) * 4;
+            const int valid = m < M ? max(0, min(4, kc - kk)) : 0;
+            const unsigned dst = static_cast<unsigned>(__cvta_generic_to_shared(xs + m * xp + kk));
+            const float *src = valid > 0 ? x + m * ldx + k0 + kk : x;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid * 4) : "memory");
+        }
+    } else {
+        for (int m = 0; m < kRows; ++m)
+            for (int kk = threadIdx.x; kk < k_per; kk += kThreads) {
+                const bool ok = m < M && kk < kc;
+                cp_async4(xs + m * xp + kk, ok ? x + m * ldx + k0 + kk : x, ok);
+            }
+    }
+    cp_async_commit();
+#pragma unroll
+    for (int b = 0; b < kDepth - 1; ++b) issue(b);
+    cp_async_wait<kDepth - 1>();                            // x (the oldest group) has landed
+    __syncthreads();
+    float acc[4][4], sum[4][4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[j][e] = sum[j][e] = 0.f;
+    for (int b = 0; b < nb; ++b) {
+        __syncwarp();                                       // every lane is done with the slot that is filled next
+        issue(b + kDepth - 1);
+        cp_async_wait<kDepth - 1>();                        // tile b has landed, for this lane ...
+        __syncwarp();                                       // ... and for the others
+        const float *slot = mine + (b % kDepth) * (32 * PITCH);
+        const float *xr = xs + g * xp + (b * WK + kw) * 32 + t;
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+            uint32_t ah[4], al[4];
+            split(xr[s * 8], ah[0], al[0]);
+            split(xr[s * 8 + 8 * xp], ah[1], al[1]);
+            split(xr[s * 8 + 4], ah[2], al[2]);
+            split(xr[s * 8 + 4 + 8 * xp], ah[3], al[3]);
+            float b0[4], b1[4];
+            if (DX) {                                       // tile j, column n = g: W row 8j + g
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    b0[j] = slot[(j * 8 + g) * PITCH + s * 8 + t];
+                    b1[j] = slot[(j * 8 + g) * PITCH + s * 8 + t + 4];
+                }
+            } else {                                        // tile j, column n = g: W column 4g + j, four tiles in one read
+                const float4 v0 = *reinterpret_cast<const float4 *>(slot + (s * 8 + t) * PITCH + g * 4);
+                const float4 v1 = *reinterpret_cast<const float4 *>(slot + (s * 8 + t + 4) * PITCH + g * 4);
+                b0[0] = v0.x; b0[1] = v0.y; b0[2] = v0.z; b0[3] = v0.w;
+                b1[0] = v1.x; b1[1] = v1.y; b1[2] = v1.z; b1[3] = v1.w;
+            }
+            mma_split(acc, ah, al, b0, b1);
+        }
+        if ((b + 1) % (kFlush / 32) == 0 || b + 1 == nb) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) { sum[j][e] += acc[j][e]; acc[j][e] = 0.f; }
+        }
+    }
+    cp_async_wait<0>();
+    __syncthreads();                                        // the ring is free: it takes the block's sums
+    float *sums = ring;                                     // [WK][kRows][SUM_PITCH]
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        float *row = sums + (kw * kRows + g + 8 * h) * SUM_PITCH + ow * 32;
+        if (DX) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                *reinterpret_cast<float2 *>(row + j * 8 + 2 * t) = make_float2(sum[j][2 * h], sum[j][2 * h + 1]);
+        } else {
+            *reinterpret_cast<float4 *>(row + 8 * t) = make_float4(sum[0][2 * h], sum[1][2 * h], sum[2][2 * h], sum[3][2 * h]);
+            *reinterpret_cast<float4 *>(row + 8 * t + 4) =
+                make_float4(sum[0][2 * h + 1], sum[1][2 * h + 1], sum[2][2 * h + 1], sum[3][2 * h + 1]);
+        }
+    }
+    const int ranks = static_cast<int>(gridDim.y);
+    if (WK > 1) {                                           // the warps of a strip first, into the first one's place
+        __syncthreads();
+        for (int i = threadIdx.x; i < kRows * (OUTS / 4); i += kThreads) {
+            float4 *at = reinterpret_cast<float4 *>(sums + (i / (OUTS / 4)) * SUM_PITCH + (i % (OUTS / 4)) * 4);
+            float4 v = *at;
+#pragma unroll
+            for (int k = 1; k < WK; ++k) {
+                const float4 p = at[k * kRows * SUM_PITCH / 4];
+                v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
+            }
+            *at = v;
+        }
+    }
+    if (ranks > 1) cluster_sync_all();
+    else __syncthreads();
+    for (int i = static_cast<int>(blockIdx.y) * kThreads + threadIdx.x; i < M * (OUTS / 4); i += ranks * kThreads) {
+        const int m = i / (OUTS / 4), q = (i - m * (OUTS / 4)) * 4;
+        const long long o = static_cast<long long>(blockIdx.x) * OUTS + q;
+        if (o >= outs) continue;
+        const float *at = sums + m * SUM_PITCH + q;
+        const float4 v = ranks > 1 ? cluster_sum_f4(at, ranks) : *reinterpret_cast<const float4 *>(at);
+        float out[4] = {v.x, v.y, v.z, v.w};
+        float *dst = y + m * ldy + o;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            if (o + e >= outs) continue;
+            if (bias) out[e] += __ldg(bias + o + e);
+            if (accumulate) out[e] += dst[e];
+        }
+        if (y_vec && o + 3 < outs) {
+            *reinterpret_cast<float4 *>(dst) = make_float4(out[0], out[1], out[2], out[3]);
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (o + e < outs) dst[e] = out[e];
+        }
+    }
+    if (ranks > 1) cluster_sync_all();                      // no block leaves while its sums may still be read
+}
+
+// dW[k, n] = sum_m x[m, k] . dy[m, n]: bound by the write of dW.  grid = (strips of 128 columns, slabs of K); a warp keeps
+// the fragments of dy for its 32 columns in registers, walks the slab's rows 16 at a time and writes 32 bytes per
+// thread and row, a warp 128 contiguous bytes of each of eight rows.  WIDTH: floats per store; 1 turns the patch in
+// shared memory first (rows that are not 16-byte aligned).
+constexpr int kSlabRows = 224;               // rows of dW per block at most
+template <int WIDTH>
+__global__ void __launch_bounds__(kThreads)
+rows_dw_kernel(const float *__restrict__ x, long long ldx, const float *__restrict__ dy, long long lddy, float *__restrict__ dW,
+               long long lddw, int accumulate, int M, long long N, long long K, int k_per) {
+    constexpr int XP = kSlabRows + 8;                       // = 8 mod 32: the A fragments' reads hit all banks
+    __shared__ float xs[kRows * XP];
+    __shared__ float patch[WIDTH == 1 ? kWarps * 16 * 33 : 1];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    const long long k0 = static_cast<long long>(blockIdx.y) * k_per;
+    const int kc = static_cast<int>(min(static_cast<long long>(k_per), K - k0));
+    const long long n0 = static_cast<long long>(blockIdx.x) * kDwCols + warp * 32;
+    grid_dependency_trigger();
+    grid_dependency_wait();
+    for (int m = 0; m < kRows; ++m)
+        for (int k = threadIdx.x; k < XP; k += kThreads) xs[m * XP + k] = (m < M && k < kc) ? __ldg(x + m * ldx + k0 + k) : 0.f;
+    // B fragments: tile j, column g is column 4g + j of the warp's 32; batches t, t + 4 of either half of the rows
+    float b0[2][4], b1[2][4];
+#pragma unroll
+    for (int s = 0; s < 2; ++s)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const long long n = n0 + 4 * g + j;
+            const int m0 = 8 * s + t, m1 = m0 + 4;
+            b0[s][j] = (n < N && m0 < M) ? __ldg(dy + m0 * lddy + n) : 0.f;
+            b1[s][j] = (n < N && m1 < M) ? __ldg(dy + m1 * lddy + n) : 0.f;
+        }
+    __syncthreads();
+    const int halves = M > 8 ? 2 : 1;
+    for (int r0 = 0; r0 < kc; r0 += 16) {
+        float acc[4][4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[j][e] = 0.f;
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+            if (s >= halves) break;
+            uint32_t ah[4], al[4];
+            const float *xr = xs + (8 * s + t) * XP + r0 + g;
+            split(xr[0], ah[0], al[0]);
+            split(xr[8], ah[1], al[1]);
+            split(xr[4 * XP], ah[2], al[2]);
+            split(xr[4 * XP + 8], ah[3], al[3]);
+            mma_split(acc, ah, al, b0[s], b1[s]);
+        }
+        if constexpr (WIDTH == 1) {
+            float *mine = patch + warp * (16 * 33);
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    mine[(g + 8 * h) * 33 + 8 * t + j] = acc[j][2 * h];
+                    mine[(g + 8 * h) * 33 + 8 * t + 4 + j] = acc[j][2 * h + 1];
+                }
+            __syncwarp();
+            if (n0 + lane < N) {
+#pragma unroll 4
+                for (int r = 0; r < 16; ++r) {
+                    if (r0 + r >= kc) break;
+                    float *dst = dW + (k0 + r0 + r) * lddw + n0 + lane;
+                    const float v = mine[r * 33 + lane];
+                    __stcs(dst, accumulate ? *dst + v : v);
+                }
+            }
+            __syncwarp();
+        } else
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int r = r0 + g + 8 * h;
+            const long long n = n0 + 8 * t;
+            if (r >= kc || n >= N) continue;
+            float *dst = dW + (k0 + r) * lddw + n;
+            float v[8];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) { v[j] = acc[j][2 * h]; v[4 + j] = acc[j][2 * h + 1]; }
+            const bool second = n + 4 < N;                  // N is a multiple of 4 here
+            if (accumulate) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e)
+                    if (e < 4 || second) v[e] += dst[e];
+            }
+            if (WIDTH == 8 && second) {
+                asm volatile("st.global.cs.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "f"(v[0]), "f"(v[1]),
+                             "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+                             : "memory");
+            } else {
+                __stcs(reinterpret_cast<float4 *>(dst), make_float4(v[0], v[1], v[2], v[3]));
+                if (second) __stcs(reinterpret_cast<float4 *>(dst + 4), make_float4(v[4], v[5], v[6], v[7]));
+            }
+        }
+    }
+}
+
+bool aligned(const void *p, size_t bytes) { return (reinterpret_cast<uintptr_t>(p) & (bytes - 1)) == 0; }
+
+// How a product is cut: strips of 128 outputs, or of 32 where those leave most SMs without a block; about two blocks per
+// SM in all, slices of at least 64 (256 where four warps share one), at most kMaxSlices of them.
+struct RowsPlan { int outs, k_per; unsigned strips, slices; };
+RowsPlan plan_rows(int64_t outs, int64_t total, int sm_count) {
+    RowsPlan p;
+    p.outs = (outs + 127) / 128 * kMaxSlices >= sm_count ? 128 : 32;
+    const int64_t strips = (outs + p.outs - 1) / p.outs;
+    int64_t slices = std::max<int64_t>((total + kMaxSlice - 1) / kMaxSlice, (2LL * sm_count + strips - 1) / strips);
+    slices = std::min<int64_t>({slices, kMaxSlices, std::max<int64_t>(1, total / (p.outs == 128 ? 64 : 256))});
+    p.k_per = static_cast<int>(((total + slices - 1) / slices + 31) / 32 * 32);
+    p.strips = static_cast<unsigned>(strips);
+    p.slices = static_cast<unsigned>((total + p.k_per - 1) / p.k_per);
+    return p;
+}
+
+template <bool DX>
+int launch_rows(const float *x, int64_t ldx, const float *W, int64_t ldw, float *y, int64_t ldy, const float *bias,
+                bool accumulate, int64_t M, int64_t outs, int64_t total, int64_t w_cols, int sm_count, cudaStream_t stream) {
+    const RowsPlan pl = plan_rows(outs, total, sm_count);
+    const int k_per = pl.k_per;
+    const bool vec = aligned(W, 16) && ldw % 4 == 0 && w_cols % 4 == 0, narrow = pl.outs == 32;
+    const size_t smem = (static_cast<size_t>(kRows) * (k_per + 4) + static_cast<size_t>(kWarps) * kDepth * 32 * (DX ? 36 : 40)) * sizeof(float);
+    auto kernel = narrow ? (vec ? rows_kernel<DX, true, kWarps> : rows_kernel<DX, false, kWarps>)
+                         : (vec ? rows_kernel<DX, true, 1> : rows_kernel<DX, false, 1>);
+    static std::atomic<uint64_t> opted_in[2][2];            // per device, as in launch_variant of the tensor path
+    std::atomic<uint64_t> &done = opted_in[narrow][vec];
+    int dev = 0;
+    MNI_CUDA(cudaGetDevice(&dev));
+    const uint64_t bit = 1ull << (dev & 63);
+    if ((done.load(std::memory_order_acquire) & bit) == 0) {
+        MNI_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+        done.fetch_or(bit, std::memory_order_release);
+    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(pl.strips, pl.slices);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attrs[2];
+    attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+    attrs[1].id = cudaLaunchAttributeClusterDimension;
+    attrs[1].val.clusterDim.x = 1;
+    attrs[1].val.clusterDim.y = pl.slices;
+    attrs[1].val.clusterDim.z = 1;
+    cfg.attrs = attrs;
+    cfg.numAttrs = pl.slices > 1 ? 2 : 1;
+    const int x_vec = (ldx % 4 == 0 || M == 1) && aligned(x, 16) ? 1 : 0, y_vec = ldy % 4 == 0 && aligned(y, 16) ? 1 : 0;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, x, static_cast<long long>(ldx), W, static_cast<long long>(ldw), y,
+                                             static_cast<long long>(ldy), bias, accumulate ? 1 : 0, static_cast<int>(M),
+                                             static_cast<long long>(outs), static_cast<long long>(total), k_per, x_vec, y_vec);
+    if (e != cudaSuccess) return fail(MNI_B200_ERR_CUDA, "rows_kernel launch failed: %s", cudaGetErrorString(e));
+    MNI_LAUNCH_CHECK("rows_kernel");
+    return MNI_B200_OK;
+}
+
+}  // namespace
+
+// The streaming kernel wins where its blocks cover the chip in 128-wide strips, or where the contraction is short enough
+// for the 32-wide ones (measured against the tensor path, 9 rows: 4096 x 4096 18.0 / 20.1 us, 512 x 8192 6.7 / 10.3,
+// 600 x 601 6.2 / 11.9; but 8192 x 512 17.4 / 13.5, 8190 x 1030 41 / 32).
+bool rows_supported(int64_t M, int64_t outs, int64_t total, int sm_count) {
+    return M >= 1 && M <= kRows && total >= 1 && total <= static_cast<int64_t>(kMaxSlice) * kMaxSlices && outs >= 1 &&
+           outs <= 0x7fffffffLL && ((outs + 127) / 128 * kMaxSlices >= sm_count || total <= 1024);
+}
+
+int launch_rows_fwd(const float *x, int64_t ldx, const float *W, int64_t ldw, float *y, int64_t ldy, const float *bias,
+                    bool accumulate, int64_t M, int64_t N, int64_t K, int sm_count, cudaStream_t stream) {
+    return launch_rows<false>(x, ldx, W, ldw, y, ldy, bias, accumulate, M, N, K, N, sm_count, stream);
+}
+// ... with the weight stored [N, K] and seen through a transposing view
+int launch_rows_bt_fwd(const float *x, int64_t ldx, const float *W, int64_t ldw, float *y, int64_t ldy, const float *bias,
+                       bool accumulate, int64_t M, int64_t N, int64_t K, int sm_count, cudaStream_t stream) {
+    return launch_rows<true>(x, ldx, W, ldw, y, ldy, bias, accumulate, M, N, K, K, sm_count, stream);
+}
+int launch_rows_dx(const float *dy, int64_t lddy, const float *W, int64_t ldw, float *dx, int64_t lddx, const float *bias,
+                   bool accumulate, int64_t M, int64_t N, int64_t K, int sm_count, cudaStream_t stream) {
+    return launch_rows<true>(dy, lddy, W, ldw, dx, lddx, bias, accumulate, M, K, N, N, sm_count, stream);
+}
+int launch_rows_bt_dx(const float *dy, int64_t lddy, const float *W, int64_t ldw, float *dx, int64_t lddx, const float *bias,
+                      bool accumulate, int64_t M, int64_t N, int64_t K, int sm_count, cudaStream_t stream) {
+    return launch_rows<false>(dy, lddy, W, ldw, dx, lddx, bias, accumulate, M, K, N, K, sm_count, stream);
+}
+int launch_rows_dw(const float *x, int64_t ldx, const float *dy, int64_t lddy, float *dW, int64_t lddw, bool accumulate,
+                   int64_t M, int64_t N, int64_t K, int sm_count, cudaStream_t stream) {
+    const int64_t strips = (N + kDwCols - 1) / kDwCols;
+    // about six blocks of 128 threads per SM
+    int64_t k_per = (K * strips + 6LL * sm_count - 1) / (6LL * sm_count);
+    k_per = std::min<int64_t>(kSlabRows, std::max<int64_t>(16, (k_per + 15) / 16 * 16));
+    const dim3 grid(static_cast<unsigned>(strips), static_cast<unsigned>((K + k_per - 1) / k_per));
+    const bool v4 = aligned(dW, 16) && lddw % 4 == 0 && N % 4 == 0, v8 = v4 && aligned(dW, 32) && lddw % 8 == 0;
+    const cudaError_t e = launch_dependent(v8 ? rows_dw_kernel<8> : v4 ? rows_dw_kernel<4> : rows_dw_kernel<1>, grid, dim3(kThreads),
+                                           0, stream, x, ldx, dy, lddy, dW, lddw, accumulate ? 1 : 0, static_cast<int>(M), N, K,
+                                           static_cast<int>(k_per));
+    if (e != cudaSuccess) return fail(MNI_B200_ERR_CUDA, "rows_dw_kernel launch failed: %s", cudaGetErrorString(e));
+    MNI_LAUNCH_CHECK("rows_dw_kernel");
+    return MNI_B200_OK;
+}
+
+}  // namespace mni

@@ -6,6 +6,7 @@
 //   fwd : y[M,N]  = x[M,K] . W[K,N] (+bias)        W streamed once, split-K partials, fused finish
 //   dW  : dW[K,N] = x[M,K]^T . dy[M,N]             dW written once
 //   dx  : dx[M,K] = dy[M,N] . W[K,N]^T             W streamed once, one warp per two rows of W
+#include "device_utils.h"
 #include "internal.h"
 
 #include <algorithm>
@@ -201,30 +202,6 @@ constexpr int kRingGroups = 8;                              // k-groups per bloc
 constexpr int kRingDepth = 4;                               // batches held by the ring, all but one in flight
 constexpr size_t kRingXBytes = 40 * 1024;                   // cap on the staged x slice: two blocks per SM
 
-__device__ __forceinline__ void cp_async16(void *smem, const void *gmem, bool valid) {
-    const unsigned dst = static_cast<unsigned>(__cvta_generic_to_shared(smem));
-    const int bytes = valid ? 16 : 0;                       // 0: nothing is read, the slot is zero-filled
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(gmem), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-// Thread-block-cluster helpers for the ring kernel's finish: the K splits of a strip form one cluster, every
-// CTA leaves its block sums in its own shared memory and the sums are added straight from there.
-__device__ __forceinline__ void cluster_sync_all() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ float4 ld_cluster_f4(const void *own_smem, unsigned rank) {
-    const unsigned local = static_cast<unsigned>(__cvta_generic_to_shared(own_smem));
-    unsigned remote;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(rank));
-    float4 v;
-    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(remote) : "memory");
-    return v;
-}
-
 // Requires N % 4 == 0, W 16-byte aligned with ldw % 4 == 0, k_per a multiple of kRingUnit.
 // cluster != 0: launched as clusters of gridDim.y CTAs along y (at most 8); the finish then goes through
 // distributed shared memory instead of scratch, fence and ticket, in the same ascending split order.
@@ -337,11 +314,7 @@ skinny_fwd_ring_kernel(const float *__restrict__ x, long long ldx, const float *
         const int ranks = static_cast<int>(gridDim.y);
         if (live) {
             for (int m = static_cast<int>(blockIdx.y) * GROUPS + kg; m < M; m += ranks * GROUPS) {
-                float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
-                for (int r = 0; r < ranks; ++r) {
-                    const float4 t = ld_cluster_f4(mine_sums + m * COLS + ct, static_cast<unsigned>(r));
-                    sum.x += t.x; sum.y += t.y; sum.z += t.z; sum.w += t.w;
-                }
+                const float4 sum = cluster_sum_f4(mine_sums + m * COLS + ct, ranks);
                 const float sv[4] = {sum.x, sum.y, sum.z, sum.w};
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {

@@ -1,0 +1,41 @@
+"""The warp-level streaming kernels of a few rows: edges of tiles, slices and strips, aligned and unaligned weights, weights
+seen through a transposing view, bias and accumulation, against float64 inside guard zones."""
+import numpy as np
+import pytest
+
+from conftest import Guarded, regression_bound_3xtf32, rel_fro
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("m,k,n", [(9, 4096, 2404), (15, 1000, 2500), (1, 65, 2433), (16, 31, 33), (3, 1024, 129), (12, 33, 4096),
+                                   (10, 2401, 2390), (5, 16384, 2370), (9, 64, 32), (2, 1, 1)])
+@pytest.mark.parametrize("transposed", [False, True])
+def test_few_rows_forward_and_backward(F, m, k, n, transposed):
+    rng = np.random.default_rng([m, k, n])
+    x, dy = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((m, n)).astype(np.float32)
+    w, bias = rng.standard_normal((k, n)).astype(np.float32), rng.standard_normal(n).astype(np.float32)
+    t = F.DeviceTensor.from_numpy
+    wd = t(np.ascontiguousarray(w.T)).permute((1, 0)) if transposed else t(w)
+    x64, w64, dy64 = (a.astype(np.float64) for a in (x, w, dy))
+    c0 = [rng.standard_normal(s).astype(np.float32) for s in ((m, n), (m, k), (k, n))]
+    for accumulate in (False, True):
+        y, dx, dw = (Guarded(F, c.shape, init=c if accumulate else None) for c in c0)
+        flags = (F._lib.ACCUMULATE_C | F._lib.ACCUMULATE_DA | F._lib.ACCUMULATE_DB) if accumulate else 0
+        F.matmul(t(x), wd, t(bias), out=y.tensor, flags=flags)
+        F.matmul_backward(t(dy), t(x), wd, da=dx.tensor, db=dw.tensor, flags=flags)
+        F.device_status()
+        for got, want, c, length in ((y, x64 @ w64 + bias, c0[0], k), (dx, dy64 @ w64.T, c0[1], n), (dw, x64.T @ dy64, c0[2], m)):
+            got.check(fully_written=not accumulate)
+            ref = want + (c if accumulate else 0)
+            assert rel_fro(got.tensor.numpy(), ref) <= regression_bound_3xtf32(length), (accumulate, length)
+
+
+def test_few_rows_plans(F):
+    """Which calls stream the weight: few rows that the FFMA kernels do not take, enough outputs for the strips or a short
+    contraction; 16 aligned rows are the tensor path's."""
+    def kernel(m, k, n):
+        return F.plan_describe((m, k), (k, n))[0]
+    assert "few rows" in kernel(9, 4096, 4096) and "few rows" in kernel(16, 4096, 4093) and "few rows" in kernel(3, 600, 601)
+    assert "skinny" in kernel(3, 4096, 4096)
+    assert "tensor" in kernel(16, 4096, 4096) and "tensor" in kernel(9, 8192, 512)
