@@ -63,6 +63,7 @@ constexpr int kBarBytes = (3 * kMaxStages + 4) * 8 + 16;
 constexpr long long kWaitCycles = 4000000000LL;            // default limit of every device-side wait: ~2 s at 2 GHz
 
 enum OperandMode { kKMajor = 0, kMnMultiBox = 1, kMnSingleBox = 2 };
+enum TailMode { kWholeTiles = 0, kBalanced = 1, kCutTiles = 2 };
 enum EpilogueMode { kEpiPlainStores = 0, kEpiTmaStore = 1, kEpiTmaReduce = 2, kEpiVectorStores = 3 };
 
 struct KParams {
@@ -105,6 +106,10 @@ struct KParams {
     // Balanced tail ("stream-K"): tiles [sk_first_tile, tiles) are not dealt out whole; their k-blocks are
     // cut into one contiguous range per CTA (pair), so a ragged last wave costs its share, not a full wave.
     int sk;                    // 0 = off
+    // Split tail: units below `tail_unit` are whole tiles, the rest are the last wave's tiles cut into `tail_ways` units each,
+    // whose partial tiles go to scratch (through tmP) for tail_finish_kernel.  units = all of them.
+    int units, tail_unit, tail_ways;
+    FastDiv fd_ways;
     int sk_first_tile;         // tiles below this index are dealt out whole, round-robin
     float *sk_partial;         // two parked accumulator tiles per CTA: [cta][2][epilogue warp][chunk][8][lane] float4
     unsigned int *sk_flags;    // ready flags [cta][2][epilogue warp] (1 = parked), then tickets [tile][rank][epilogue warp]
@@ -325,13 +330,25 @@ struct TileCoord {
     int shared;      // balanced tail: this unit is only a range of the tile's k-blocks
     int park;        // shared: which of the CTA's two parking places it uses (0 = first unit of its range)
     int tile;        // flat tile index
+    int part;        // >= 0: index of this unit among the split tail's
     int chunk;       // > 0: a later piece of a unit whose contraction is summed in several accumulators (added to the output)
 };
 
+template <int TAIL>
 __device__ __forceinline__ TileCoord decode_unit(const KParams &p, int unit) {
     TileCoord t;
-    const int tile = fd_div(unit, p.fd_splits);
-    t.split = unit - tile * p.splits;
+    t.part = TAIL == kCutTiles ? unit - p.tail_unit : -1;
+    int tile, ways;
+    if (t.part >= 0) {
+        const int q = fd_div(t.part, p.fd_ways);
+        ways = p.tail_ways;
+        tile = p.tail_unit + q;                    // whole tiles before the tail: unit == tile there
+        t.split = t.part - q * ways;
+    } else {
+        ways = p.splits;
+        tile = fd_div(unit, p.fd_splits);
+        t.split = unit - tile * ways;
+    }
     t.shared = 0;
     t.park = 0;
     t.chunk = 0;
@@ -347,12 +364,12 @@ __device__ __forceinline__ TileCoord decode_unit(const KParams &p, int unit) {
     t.tn = gm == p.group_m ? fd_div(rin, p.fd_group_m) : fd_div(rin, p.fd_last_gm);
     t.tm = first_m + (rin - t.tn * gm);
     const int total = p.fold * p.kiters;
-    if (p.splits == 1) {
+    if (ways == 1) {
         t.it0 = 0;
         t.it1 = total;
     } else {
-        t.it0 = static_cast<int>(static_cast<long long>(total) * t.split / p.splits);
-        t.it1 = static_cast<int>(static_cast<long long>(total) * (t.split + 1) / p.splits);
+        t.it0 = static_cast<int>(static_cast<long long>(total) * t.split / ways);
+        t.it1 = static_cast<int>(static_cast<long long>(total) * (t.split + 1) / ways);
     }
     return t;
 }
@@ -377,7 +394,7 @@ __device__ __forceinline__ WorkIter work_begin(const KParams &p, int slot, int n
     WorkIter wi;
     wi.unit = slot;
     wi.unit_step = nslots;
-    wi.unit_end = p.sk ? p.sk_first_tile : p.batch * p.tiles_m * p.tiles_n * p.splits;
+    wi.unit_end = p.sk ? p.sk_first_tile : p.units;
     wi.w0 = wi.w = wi.w1 = 0;
     wi.piece_it = wi.piece_end = wi.piece_len = wi.piece_no = 0;
     if (p.sk) {
@@ -386,7 +403,6 @@ __device__ __forceinline__ WorkIter work_begin(const KParams &p, int slot, int n
     }
     return wi;
 }
-__device__ __forceinline__ TileCoord decode_unit(const KParams &p, int unit);
 // Cuts a long unit into equal pieces of at most p.chunk_iters k-blocks: `t` becomes the first piece, the iterator
 // remembers the rest.
 __device__ __forceinline__ void first_piece(const KParams &p, WorkIter &wi, TileCoord &t) {
@@ -401,6 +417,7 @@ __device__ __forceinline__ void first_piece(const KParams &p, WorkIter &wi, Tile
         wi.piece_it = t.it1;
     }
 }
+template <int TAIL>
 __device__ __forceinline__ bool work_next(const KParams &p, WorkIter &wi, TileCoord &t) {
     if (wi.piece_it < wi.piece_end) {          // next piece of the current unit
         t = wi.cur;
@@ -411,17 +428,17 @@ __device__ __forceinline__ bool work_next(const KParams &p, WorkIter &wi, TileCo
         return true;
     }
     if (wi.unit < wi.unit_end) {
-        t = decode_unit(p, wi.unit);
+        t = decode_unit<TAIL>(p, wi.unit);
         wi.unit += wi.unit_step;
         first_piece(p, wi, t);
         return true;
     }
-    if (wi.w < wi.w1) {
+    if (TAIL == kBalanced && wi.w < wi.w1) {
         const int per_tile = p.fold * p.kiters;
         const int rel = static_cast<int>(wi.w / per_tile);
         const int it0 = static_cast<int>(wi.w - static_cast<long long>(rel) * per_tile);
         const int it1 = static_cast<int>(min(static_cast<long long>(per_tile), it0 + (wi.w1 - wi.w)));
-        t = decode_unit(p, p.sk_first_tile + rel);          // splits == 1 here: unit == tile
+        t = decode_unit<TAIL>(p, p.sk_first_tile + rel);          // splits == 1 here: unit == tile
         t.it0 = it0;
         t.it1 = it1;
         t.shared = (it0 != 0 || it1 != per_tile) ? 1 : 0;
@@ -463,14 +480,16 @@ __device__ __forceinline__ void load_operand(int mode, uint32_t dst, const CUten
 // The split warps read each landed A row once, and store hi and lo with tcgen05.st into a TMEM slot
 // of the stage (columns 2*BN + stage*64: 32 of hi, 32 of lo); no lo copy of A is written to shared
 // memory and no MMA re-reads A from it, which is what bounds narrow tiles otherwise.
-// SK = true compiles the balanced-tail epilogue (parking / reducing shared tiles) in; the other
-// instantiations carry none of its code or registers.
+// TAIL: what the last wave may be.  kWholeTiles; kBalanced compiles the balanced tail's epilogue (parking / reducing
+// shared tiles) in; kCutTiles the split tail's (partial tiles to scratch).  Each instantiation carries only its own
+// code and registers (2 % of a single-pass 8192^3 product otherwise).
 // SG = 2 (TA only): the split warps work as two groups on alternate k-blocks (see the split role).
-template <int BN, int BK, bool FAST, int NS, int CG, bool TA = false, bool SK = false, int SG = 1>
+template <int BN, int BK, bool FAST, int NS, int CG, bool TA = false, int TAIL = kWholeTiles, int SG = 1>
 __global__ void __launch_bounds__(32 * (2 + NS + kEpiWarps), 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmD,
-               const KParams p) {
+               const __grid_constant__ CUtensorMap tmP, const __grid_constant__ KParams p) {
+    constexpr bool SK = TAIL == kBalanced, CUT = TAIL == kCutTiles;
     constexpr int BNL = BN / CG;                           // B rows staged by this CTA
     constexpr uint32_t A_BYTES = BM * BK * 4;
     constexpr uint32_t B_BYTES = BNL * BK * 4;
@@ -570,7 +589,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             uint32_t dstA = dstA0;
             WorkIter wi = work_begin(p, unit0, unit_step);
             TileCoord t;
-            while (ok && work_next(p, wi, t)) {
+            while (ok && work_next<TAIL>(p, wi, t)) {
                 int f = 0, kk = t.it0;
                 if (t.it0 >= p.kiters) {
                     f = t.it0 / p.kiters;
@@ -639,7 +658,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             const uint32_t ready0 = (FAST && CG == 1) ? bar_full : bar_xform;
             WorkIter wi = work_begin(p, unit0, unit_step);
             TileCoord wt;
-            while (ok && work_next(p, wi, wt)) {
+            while (ok && work_next<TAIL>(p, wi, wt)) {
                 const int iters = wt.it1 - wt.it0;
                 const int buf = acc_it & 1;
                 const uint32_t acc_phase = (acc_it >> 1) & 1;
@@ -734,7 +753,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             constexpr int U = !EXACT ? 1 : (PER % 4 == 0) ? 4 : (PER % 2 == 0 ? 2 : 1);
             WorkIter wi = work_begin(p, unit0, unit_step);
             TileCoord wt;
-            while (ok && work_next(p, wi, wt)) {
+            while (ok && work_next<TAIL>(p, wi, wt)) {
                 const int iters = wt.it1 - wt.it0;
                 for (int it = 0; it < iters; ++it) {
                     if (SG == 2 && ((kb++ & 1) != group)) {    // the other group's k-block
@@ -840,16 +859,18 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         WorkIter wi = work_begin(p, unit0, unit_step);
         TileCoord t;
         const int my_cta = static_cast<int>(blockIdx.x);                 // slot * CG + rank in the pair
-        while (ok && work_next(p, wi, t)) {
+        while (ok && work_next<TAIL>(p, wi, t)) {
             const int buf = acc_it & 1;
             const uint32_t acc_phase = (acc_it >> 1) & 1;
             ok = mbar_wait(bar_acc_full + 8u * buf, acc_phase, abort_flag, p.err, 0x500u | buf, waited, timed, p.wait_cycles);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             tc_fence_after();
-            const bool fuse = p.splits == 1;
+            const bool part = CUT && t.part >= 0;            // of the split tail: a raw partial tile, always through TMA
+            const bool fuse = p.splits == 1 && !part;
+            const bool tma_here = use_tma || part;
             const bool add_piece = t.chunk > 0;       // a later piece of this unit's contraction: added to what the earlier ones wrote
-            if (add_piece && use_tma) {
+            if (add_piece && tma_here) {
                 // this warp's earlier stores to the same patches must have completed, not just been read
                 if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
                 in_flight = 0;
@@ -1019,9 +1040,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         __syncwarp();
                         if (lane == 0) {
                             const uint32_t src = smem_u32(my_stage + patch * kEpiBufBytes);
-                            const int c0 = p.transpose_out ? row0 : col0, c1 = p.transpose_out ? col0 : row0;
-                            if (reduce) tma_reduce_add_5d(map, src, c0, c1, cbatch);
-                            else tma_store_5d(map, src, c0, c1, cbatch);
+                            const int c0 = part ? chunk * 32 : p.transpose_out ? row0 : col0;
+                            const int c1 = part ? static_cast<int>(cta_rank) * BM + q * 32 : p.transpose_out ? col0 : row0;
+                            const int c2 = part ? t.part : cbatch;
+                            if (reduce) tma_reduce_add_5d(map, src, c0, c1, c2);
+                            else tma_store_5d(map, src, c0, c1, c2);
                             asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                             ++in_flight;
                         }
@@ -1055,6 +1078,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 #pragma unroll
                         for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(gelu_tanh_f(__uint_as_float(v[j])));
                         emit(&tmD, false);
+                    } else if (part) {
+                        emit(&tmP, add_piece);
                     } else if (use_tma) {
                         emit(&tmC, (p.epi_mode == kEpiTmaReduce && fuse) || add_piece);
                     } else {
@@ -1102,22 +1127,19 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         if (col0 + lane < p.N) {
                             float *dst = out0 + col0 + lane;
                             const uint8_t *src = my_stage + ((lane & 3) << 2);
+#pragma unroll 2
+                            for (int r4 = 0; r4 < 32; r4 += 4) {
+                                float y[4];
 #pragma unroll
-                            for (int r8 = 0; r8 < 32; r8 += 8) {
-                                float y[8];
-#pragma unroll
-                                for (int r = 0; r < 8; ++r)
-                                    y[r] = *reinterpret_cast<const float *>(src + (r8 + r) * 128 + (((lane >> 2) ^ r) << 4));
+                                for (int r = 0; r < 4; ++r)
+                                    y[r] = *reinterpret_cast<const float *>(src + (r4 + r) * 128 + (((lane >> 2) ^ ((r4 + r) & 7)) << 4));
                                 if (add) {
-                                    float o[8];
 #pragma unroll
-                                    for (int r = 0; r < 8; ++r) o[r] = r8 + r < rows ? dst[(r8 + r) * pitch] : 0.f;
-#pragma unroll
-                                    for (int r = 0; r < 8; ++r) y[r] += o[r];
+                                    for (int r = 0; r < 4; ++r) y[r] += r4 + r < rows ? dst[(r4 + r) * pitch] : 0.f;
                                 }
 #pragma unroll
-                                for (int r = 0; r < 8; ++r)
-                                    if (r8 + r < rows) dst[(r8 + r) * pitch] = y[r];
+                                for (int r = 0; r < 4; ++r)
+                                    if (r4 + r < rows) dst[(r4 + r) * pitch] = y[r];
                             }
                         }
                         __syncwarp();                  // the staging buffer is free again
@@ -1152,7 +1174,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
         // The staging patches must have been read before the CTA gives up its shared memory; the global
         // writes themselves complete with the grid like any other store.
-        if (use_tma && lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        if ((use_tma || CUT) && lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
         if (p.prof && warp == 2 + NS && lane == 0) {
             atomicAdd(p.prof + 4, static_cast<unsigned long long>(waited));
             atomicAdd(p.prof + 7, static_cast<unsigned long long>(t_wg));
@@ -1248,6 +1270,74 @@ splitk_reduce_kernel(const float *__restrict__ partial, float *__restrict__ C, l
         float y = mine[e];
         if (bias) y += __ldg(bias + col);
         if (accumulate) y += *out;
+        *out = y;
+    }
+}
+
+// Finish of a split tail: adds the `tail_ways` partial tiles of each of the last wave's tiles in ascending order and runs
+// what the GEMM epilogue does to a whole tile (bias, C += ..., gelu into the second output).  grid = (tile rows / 4, tail
+// tiles); a row of the tile is 64 vectors, two warps.
+template <bool VEC>
+__global__ void __launch_bounds__(256)
+tail_finish_kernel(const float *__restrict__ partial, float *__restrict__ D, int bn, int tile_rows,
+                   const __grid_constant__ KParams p) {
+    __shared__ float turn[VEC ? 1 : 256 * 4];
+    grid_dependency_trigger();
+    const TileCoord t = decode_unit<kCutTiles>(p, p.tail_unit + static_cast<int>(blockIdx.y) * p.tail_ways);
+    const int r = static_cast<int>(blockIdx.x) * 4 + (threadIdx.x >> 6), c4 = threadIdx.x & 63;
+    const int row = t.tm * tile_rows + r, col = t.tn * bn + c4 * 4;
+    grid_dependency_wait();                      // the partials come from the grid before this one
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (row < p.M && col < p.N) {
+        const float4 *src = reinterpret_cast<const float4 *>(partial) +
+                            ((static_cast<long long>(blockIdx.y) * p.tail_ways) * tile_rows + r) * (bn / 4) + c4;
+        float4 x[4];
+        const long long step = static_cast<long long>(tile_rows) * (bn / 4);
+        for (int w0 = 0; w0 < p.tail_ways; w0 += 4) {
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (w0 + u < p.tail_ways) x[u] = __ldcg(src + (w0 + u) * step);
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (w0 + u < p.tail_ways) { acc.x += x[u].x; acc.y += x[u].y; acc.z += x[u].z; acc.w += x[u].w; }
+        }
+    }
+    const long long at = static_cast<long long>(t.bt) * p.c_bstride + static_cast<long long>(row) * p.ldc;
+    if (VEC) {
+        if (row >= p.M || col >= p.N) return;
+        float v[4] = {acc.x, acc.y, acc.z, acc.w};
+        if (D && p.C) *reinterpret_cast<float4 *>(p.C + at + col) = acc;       // the raw product, what the tape saves
+        if (p.bias) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[e] += __ldg(p.bias + col + e);
+        }
+        float4 *out = reinterpret_cast<float4 *>((D ? D : p.C) + at + col);
+        if (D) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[e] = gelu_tanh_f(v[e]);
+        } else if (p.accumulate) {
+            const float4 c0 = *out;
+            v[0] += c0.x; v[1] += c0.y; v[2] += c0.z; v[3] += c0.w;
+        }
+        *out = make_float4(v[0], v[1], v[2], v[3]);
+        return;
+    }
+    // rows that are not whole aligned vectors: a warp turns its 128 columns, so that a store covers 32 neighbours
+    const int lane = threadIdx.x & 31;
+    float *mine = turn + (threadIdx.x & ~31) * 4;
+    reinterpret_cast<float4 *>(mine)[lane] = acc;
+    __syncwarp();
+    if (row >= p.M) return;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int cc = t.tn * bn + (threadIdx.x & 32) * 4 + j * 32 + lane;
+        if (cc >= p.N) continue;
+        float y = mine[j * 32 + lane];
+        if (D && p.C) p.C[at + cc] = y;
+        if (p.bias) y += __ldg(p.bias + cc);
+        float *out = (D ? D : p.C) + at + cc;
+        if (D) y = gelu_tanh_f(y);
+        else if (p.accumulate) y += *out;
         *out = y;
     }
 }
@@ -1414,6 +1504,7 @@ struct Plan {
     bool ta;                                                  // A operand of the MMAs from tensor memory
     bool sk;                                                  // balanced tail: the last, ragged wave is cut by k-blocks
     int sk_first_tile;
+    int tail_ways, tail_tiles;                                // split tail: the last wave's tiles, cut into this many units each (0: none)
     size_t smem;
 };
 
@@ -1506,10 +1597,24 @@ Plan make_plan(const GemmProblem &p, int sm_count) {
     // boundary are summed in the owner's epilogue, in slot order).
     pl.sk = false;
     pl.sk_first_tile = 0;
+    pl.tail_ways = pl.tail_tiles = 0;
     // MNI_B200_STREAMK: unset = on when the whole-tile schedule would idle more than a fifth of the slot-rounds
     // (measured: below that the idle SMs of a ragged wave are power headroom for the busy ones at the 1 kW cap
     // and the balanced tail does not pay); 1 = on from 8 % idle; 0 = never.
     const int sk_env = env_int("MNI_B200_STREAMK", -1);
+    // Split tail: after at least one whole round, a last wave that fills at most half of the CTA pairs is cut into two to
+    // four units per tile, whose partial tiles one small kernel adds.  2048 x 3072, K = 768 (96 tiles on 74 pairs): two
+    // rounds 49.7 us, the balanced tail 51.9 (17 of it parking and adding in the last CTAs), this 41.
+    if (splits == 1 && sk_env < 0 && p.force_splits <= 0 && pl.cg == 2 && pl.bn == 256) {
+        const long long full = tiles / slots, rem = tiles - full * slots;
+        const long long ways = rem > 0 ? std::min<long long>(slots / rem, 4) : 1;
+        const double eff = static_cast<double>(tiles) / static_cast<double>((full + 1) * slots);
+        if (full >= 1 && ways >= 2 && eff < 0.80 && iters / ways * pl.bk >= 128) {
+            pl.tail_ways = static_cast<int>(ways);
+            pl.tail_tiles = static_cast<int>(rem);
+            return pl;
+        }
+    }
     if (splits == 1 && p.D == nullptr && sk_env != 0) {
         const long long full_rounds = tiles / slots, rem = tiles - full_rounds * slots;
         const double eff = static_cast<double>(tiles) / static_cast<double>((full_rounds + 1) * slots);
@@ -1547,9 +1652,9 @@ uint32_t desc_hi_bits(uint32_t sbo_bytes, uint32_t layout_type) {
     return ((sbo_bytes >> 4) & 0x3FFFu) | (1u << 14) | (layout_type << 29);
 }
 
-template <int BN, int BK, bool FAST, int NS, int CG, bool TA = false, bool SK = false, int SG = 1>
+template <int BN, int BK, bool FAST, int NS, int CG, bool TA = false, int TAIL = kWholeTiles, int SG = 1>
 cudaError_t launch_variant(const Plan &pl, const CUtensorMap &tmA, const CUtensorMap &tmB, const CUtensorMap &tmC,
-                           const CUtensorMap &tmD, const KParams &k, cudaStream_t stream) {
+                           const CUtensorMap &tmD, const CUtensorMap &tmP, const KParams &k, cudaStream_t stream) {
     // The shared-memory opt-in is an attribute of the function on ONE device: set once per device of the process
     // (a bit per device ordinal; setting it twice from two threads is harmless).
     static std::atomic<uint64_t> opted_in{0};
@@ -1558,7 +1663,7 @@ cudaError_t launch_variant(const Plan &pl, const CUtensorMap &tmA, const CUtenso
     if (attr != cudaSuccess) return attr;
     const uint64_t bit = 1ull << (dev & 63);
     if ((opted_in.load(std::memory_order_acquire) & bit) == 0) {
-        attr = cudaFuncSetAttribute(gemm_tc_kernel<BN, BK, FAST, NS, CG, TA, SK, SG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        attr = cudaFuncSetAttribute(gemm_tc_kernel<BN, BK, FAST, NS, CG, TA, TAIL, SG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     227 * 1024);
         if (attr != cudaSuccess) return attr;
         opted_in.fetch_or(bit, std::memory_order_release);
@@ -1577,7 +1682,7 @@ cudaError_t launch_variant(const Plan &pl, const CUtensorMap &tmA, const CUtenso
     attrs[1].val.clusterDim.z = 1;
     cfg.attrs = attrs;
     cfg.numAttrs = CG == 2 ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, gemm_tc_kernel<BN, BK, FAST, NS, CG, TA, SK, SG>, tmA, tmB, tmC, tmD, k);
+    return cudaLaunchKernelEx(&cfg, gemm_tc_kernel<BN, BK, FAST, NS, CG, TA, TAIL, SG>, tmA, tmB, tmC, tmD, tmP, k);
 }
 
 }  // namespace
@@ -1658,6 +1763,7 @@ size_t gemm_tc_partial_bytes(const GemmProblem &p0, int sm_count) {
     const GemmProblem p = kernel_view(p0, &transposed);
     const Plan pl = make_plan(p, sm_count);
     if (pl.sk) return static_cast<size_t>(pl.grid) * 2 * BM * pl.bn * sizeof(float);   // two parked accumulators per CTA
+    if (pl.tail_ways) return static_cast<size_t>(pl.tail_tiles) * pl.tail_ways * BM * pl.cg * pl.bn * sizeof(float);
     if (pl.splits <= 1) return 0;
     return static_cast<size_t>(pl.splits) * p.batch * p0.M * partial_pitch(p0.N) * sizeof(float);
 }
@@ -1675,11 +1781,11 @@ std::string gemm_tc_describe(const GemmProblem &p0, int sm_count) {
     char buf[320];
     snprintf(buf, sizeof(buf),
              "tensor m=%lld n=%lld k=%lld batch=%lld fold=%lld bn=%d bk=%d pair=%d tmem_a=%d stages=%d splits=%d "
-             "tail=%d grid=%d exchanged=%d single_pass=%d pieces=%d mma_n=%d",
+             "tail=%d grid=%d exchanged=%d single_pass=%d pieces=%d mma_n=%d tail_ways=%d",
              static_cast<long long>(p.M), static_cast<long long>(p.N), static_cast<long long>(p.K),
              static_cast<long long>(p.batch), static_cast<long long>(p.fold), pl.bn, pl.bk, pl.cg == 2 ? 1 : 0,
-             pl.ta ? 1 : 0, pl.stages, pl.splits, pl.sk ? 1 : 0, pl.grid, transposed ? 1 : 0, p.fast_tf32 ? 1 : 0,
-             pieces, mma_n_for(p, pl));
+             pl.ta ? 1 : 0, pl.stages, pl.splits, pl.sk || pl.tail_ways ? 1 : 0, pl.grid, transposed ? 1 : 0, p.fast_tf32 ? 1 : 0,
+             pieces, mma_n_for(p, pl), pl.tail_ways);
     return buf;
 }
 
@@ -1709,11 +1815,11 @@ int launch_gemm_tc(const GemmProblem &p0, float *partial, uint32_t *err_word, in
     const int64_t oM = p0.M, oN = p0.N;
     const Plan pl = make_plan(p, sm_count);
     if (p.K <= 0) return fail(MNI_B200_ERR_ARG, "empty contraction reached the tensor-core launcher");
-    if ((pl.splits > 1 || pl.sk) && partial == nullptr)
+    if ((pl.splits > 1 || pl.sk || pl.tail_ways) && partial == nullptr)
         return fail(MNI_B200_ERR_WORKSPACE, "split-K launch without partial storage");
 
     KParams k{};
-    CUtensorMap tmA, tmB, tmC, tmD;
+    CUtensorMap tmA, tmB, tmC, tmD, tmP;
     if (p.D != nullptr && !gemm_tc_can_fuse_activation(p, sm_count))
         return fail(MNI_B200_ERR_ARG, "fused activation requested for a problem that cannot carry it");
     int rc = make_operand_map(&tmA, p.A, BM, pl.bk, &k.a_mode);
@@ -1757,6 +1863,13 @@ int launch_gemm_tc(const GemmProblem &p0, float *partial, uint32_t *err_word, in
         k.store_pre = p.C != nullptr ? 1 : 0;
     }
 
+    tmP = tmC;
+    if (pl.tail_ways) {      // partial tiles one after the other, rows of pl.bn floats
+        rc = make_output_map(&tmP, partial, pl.bn, BM * pl.cg, static_cast<int64_t>(pl.tail_tiles) * pl.tail_ways, pl.bn,
+                             static_cast<int64_t>(BM) * pl.cg * pl.bn);
+        if (rc) return rc;
+    }
+
     k.M = static_cast<int>(p.M);
     k.N = static_cast<int>(p.N);
     k.transpose_out = transposed ? 1 : 0;
@@ -1789,6 +1902,13 @@ int launch_gemm_tc(const GemmProblem &p0, float *partial, uint32_t *err_word, in
         k.fd_last_gm = make_fastdiv(last_gm);
         k.fd_a_cnt = make_fastdiv(k.a_batch); k.fd_a_d1 = make_fastdiv(k.a_d1); k.fd_a_d2 = make_fastdiv(k.a_d2);
         k.fd_b_cnt = make_fastdiv(k.b_batch); k.fd_b_d1 = make_fastdiv(k.b_d1); k.fd_b_d2 = make_fastdiv(k.b_d2);
+    }
+    {
+        const int tiles = k.batch * k.tiles_m * k.tiles_n;
+        k.tail_ways = pl.tail_ways;
+        k.fd_ways = make_fastdiv(pl.tail_ways);
+        k.tail_unit = pl.tail_ways ? tiles - pl.tail_tiles : 0x7fffffff;
+        k.units = pl.tail_ways ? k.tail_unit + pl.tail_tiles * pl.tail_ways : tiles * pl.splits;
     }
     k.stages = pl.stages;
     k.epi_patches = pl.patches;
@@ -1846,29 +1966,34 @@ int launch_gemm_tc(const GemmProblem &p0, float *partial, uint32_t *err_word, in
     }
     cudaError_t e = cudaErrorInvalidValue;
     if (pl.sk) {
-        if (pl.ta && pl.bn == 64 && split_groups == 2) e = launch_variant<64, 32, false, 8, 1, true, true, 2>(pl, tmA, tmB, tmC, tmD, k, stream);
-        else if (pl.ta && pl.bn == 64) e = launch_variant<64, 32, false, 8, 1, true, true>(pl, tmA, tmB, tmC, tmD, k, stream);
-        else if (pl.ta && pl.bn == 128 && split_groups == 2) e = launch_variant<128, 32, false, 8, 1, true, true, 2>(pl, tmA, tmB, tmC, tmD, k, stream);
-        else if (pl.ta && pl.bn == 128) e = launch_variant<128, 32, false, 8, 1, true, true>(pl, tmA, tmB, tmC, tmD, k, stream);
-        else if (!p.fast_tf32 && pl.bk == 16) e = launch_variant<256, 16, false, 8, 2, false, true>(pl, tmA, tmB, tmC, tmD, k, stream);
-        else if (!p.fast_tf32 && pl.bk == 32) e = launch_variant<256, 32, false, 8, 2, false, true>(pl, tmA, tmB, tmC, tmD, k, stream);
-        else if (pl.bk == 16) e = launch_variant<256, 16, true, 4, 2, false, true>(pl, tmA, tmB, tmC, tmD, k, stream);
-        else e = launch_variant<256, 32, true, 4, 2, false, true>(pl, tmA, tmB, tmC, tmD, k, stream);
+        if (pl.ta && pl.bn == 64 && split_groups == 2) e = launch_variant<64, 32, false, 8, 1, true, kBalanced, 2>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+        else if (pl.ta && pl.bn == 64) e = launch_variant<64, 32, false, 8, 1, true, kBalanced>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+        else if (pl.ta && pl.bn == 128 && split_groups == 2) e = launch_variant<128, 32, false, 8, 1, true, kBalanced, 2>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+        else if (pl.ta && pl.bn == 128) e = launch_variant<128, 32, false, 8, 1, true, kBalanced>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+        else if (!p.fast_tf32 && pl.bk == 16) e = launch_variant<256, 16, false, 8, 2, false, kBalanced>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+        else if (!p.fast_tf32 && pl.bk == 32) e = launch_variant<256, 32, false, 8, 2, false, kBalanced>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+        else if (pl.bk == 16) e = launch_variant<256, 16, true, 4, 2, false, kBalanced>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+        else e = launch_variant<256, 32, true, 4, 2, false, kBalanced>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+    } else if (pl.tail_ways) {
+        if (!p.fast_tf32 && pl.bk == 16) e = launch_variant<256, 16, false, 8, 2, false, kCutTiles>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+        else if (!p.fast_tf32) e = launch_variant<256, 32, false, 8, 2, false, kCutTiles>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+        else if (pl.bk == 16) e = launch_variant<256, 16, true, 4, 2, false, kCutTiles>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+        else e = launch_variant<256, 32, true, 4, 2, false, kCutTiles>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
     } else if (pl.ta) {
-        if (pl.bn == 64 && split_groups == 2) e = launch_variant<64, 32, false, 8, 1, true, false, 2>(pl, tmA, tmB, tmC, tmD, k, stream);
-        else if (pl.bn == 64) e = launch_variant<64, 32, false, 8, 1, true>(pl, tmA, tmB, tmC, tmD, k, stream);
-        else if (split_groups == 2) e = launch_variant<128, 32, false, 8, 1, true, false, 2>(pl, tmA, tmB, tmC, tmD, k, stream);
-        else e = launch_variant<128, 32, false, 8, 1, true>(pl, tmA, tmB, tmC, tmD, k, stream);
+        if (pl.bn == 64 && split_groups == 2) e = launch_variant<64, 32, false, 8, 1, true, kWholeTiles, 2>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+        else if (pl.bn == 64) e = launch_variant<64, 32, false, 8, 1, true>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+        else if (split_groups == 2) e = launch_variant<128, 32, false, 8, 1, true, kWholeTiles, 2>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+        else e = launch_variant<128, 32, false, 8, 1, true>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
     }
 #define MNI_VARIANT(BN_, BK_)                                                                         \
     if (pl.cg == 1 && !pl.ta && pl.bn == BN_ && pl.bk == BK_) {                                                 \
-        if (p.fast_tf32) e = launch_variant<BN_, BK_, true, 4, 1>(pl, tmA, tmB, tmC, tmD, k, stream);      \
-        else e = launch_variant<BN_, BK_, false, 8, 1>(pl, tmA, tmB, tmC, tmD, k, stream);                 \
+        if (p.fast_tf32) e = launch_variant<BN_, BK_, true, 4, 1>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);      \
+        else e = launch_variant<BN_, BK_, false, 8, 1>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);                 \
     }
 #define MNI_PAIR_VARIANT(BN_, BK_)                                                                    \
-    if (pl.cg == 2 && !pl.sk && pl.bn == BN_ && pl.bk == BK_) {                                                 \
-        if (p.fast_tf32) e = launch_variant<BN_, BK_, true, 4, 2>(pl, tmA, tmB, tmC, tmD, k, stream);      \
-        else e = launch_variant<BN_, BK_, false, 8, 2>(pl, tmA, tmB, tmC, tmD, k, stream);                 \
+    if (pl.cg == 2 && !pl.sk && !pl.tail_ways && pl.bn == BN_ && pl.bk == BK_) {                                                 \
+        if (p.fast_tf32) e = launch_variant<BN_, BK_, true, 4, 2>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);      \
+        else e = launch_variant<BN_, BK_, false, 8, 2>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);                 \
     }
     MNI_PAIR_VARIANT(64, 32) MNI_PAIR_VARIANT(128, 32) MNI_PAIR_VARIANT(256, 16) MNI_PAIR_VARIANT(256, 32)
 #undef MNI_PAIR_VARIANT
@@ -1876,6 +2001,15 @@ int launch_gemm_tc(const GemmProblem &p0, float *partial, uint32_t *err_word, in
 #undef MNI_VARIANT
     if (e != cudaSuccess) return fail(MNI_B200_ERR_CUDA, "gemm_tc_kernel set-up failed: %s", cudaGetErrorString(e));
     MNI_LAUNCH_CHECK("gemm_tc_kernel");
+    if (pl.tail_ways) {
+        const bool vec = oN % 4 == 0 && p.ldc % 4 == 0 && p.c_bstride % 4 == 0 &&
+                         ((reinterpret_cast<uintptr_t>(p.C) | reinterpret_cast<uintptr_t>(p.D)) & 15) == 0;
+        const dim3 grid(static_cast<unsigned>(BM * pl.cg / 4), static_cast<unsigned>(pl.tail_tiles));
+        e = launch_dependent(vec ? tail_finish_kernel<true> : tail_finish_kernel<false>, grid, dim3(256), 0, stream, partial, p.D,
+                             pl.bn, BM * pl.cg, k);
+        if (e != cudaSuccess) return fail(MNI_B200_ERR_CUDA, "tail_finish_kernel launch failed: %s", cudaGetErrorString(e));
+        MNI_LAUNCH_CHECK("tail_finish_kernel");
+    }
     if (pl.splits > 1) {
         const GemmFinish f{partial, p.C, p.ldc, p.c_bstride, p.batch, oM, oN, p.bias, p.accumulate, pl.splits};
         if (defer) *defer = f;

@@ -87,3 +87,35 @@ def test_products_with_unaligned_output_rows(F, m, k, n, batch, flags, accumulat
     F.device_status()
     out.check("product", fully_written=not accumulate)
     assert rel_fro(out.tensor.numpy(), want) <= regression_bound_3xtf32(k)
+
+
+@pytest.mark.parametrize("m,k,n,batch", [
+    (2048, 416, 3072, ()),        # 96 tiles of 256 x 256: 22 of them cut into three units
+    (2000, 420, 3001, ()),        # ragged edges, unaligned rows
+    (2304, 2048, 2050, ()),       # 81 tiles: 7 cut into four units of 512
+    (512, 700, 1000, (12,))])     # batched
+@pytest.mark.parametrize("mode", ["plain", "accumulate", "gelu", "single pass"])
+def test_last_wave_cut_into_units(F, m, k, n, batch, mode):
+    """After a whole round, the tiles of a half-empty last wave are computed by several units each, and a finish kernel adds
+    their partial tiles with everything the epilogue does to a whole one."""
+    rng = _rng(5, m, k, n)
+    a, b = rng.standard_normal(batch + (m, k)).astype(np.float32), rng.standard_normal(batch + (k, n)).astype(np.float32)
+    bias, c0 = rng.standard_normal(n).astype(np.float32), rng.standard_normal(batch + (m, n)).astype(np.float32)
+    ad, bd, biasd = (F.DeviceTensor.from_numpy(x) for x in (a, b, bias))
+    assert "tail_ways=0" not in F.plan_describe(a.shape, b.shape)[0]
+    want = a.astype(np.float64) @ b.astype(np.float64)
+    if mode == "gelu":
+        pre, got = F.matmul_bias_gelu(ad, bd, biasd)
+        F.device_status()
+        assert rel_fro(pre.numpy(), want) <= regression_bound_3xtf32(k)
+        v = want + bias
+        want = 0.5 * v * (1 + np.tanh(0.7978845608028654 * (v + 0.044715 * v ** 3)))
+        assert rel_fro(got.numpy(), want) <= regression_bound_3xtf32(k)
+        return
+    out = Guarded(F, want.shape, init=c0 if mode == "accumulate" else None)
+    flags = {"plain": 0, "accumulate": F._lib.ACCUMULATE_C, "single pass": F._lib.PRECISION_TF32}[mode]
+    F.matmul(ad, bd, biasd, out=out.tensor, flags=flags)
+    F.device_status()
+    out.check("product", fully_written=mode != "accumulate")
+    want = want + bias + (c0 if mode == "accumulate" else 0)
+    assert rel_fro(out.tensor.numpy(), want) <= (2e-3 if mode == "single pass" else regression_bound_3xtf32(k))
