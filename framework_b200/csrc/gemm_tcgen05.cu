@@ -63,7 +63,7 @@ constexpr int kBarBytes = (3 * kMaxStages + 4) * 8 + 16;
 constexpr long long kWaitCycles = 4000000000LL;            // default limit of every device-side wait: ~2 s at 2 GHz
 
 enum OperandMode { kKMajor = 0, kMnMultiBox = 1, kMnSingleBox = 2 };
-enum TailMode { kWholeTiles = 0, kBalanced = 1, kCutTiles = 2 };
+enum TailMode { kWholeTiles = 0, kBalanced = 1, kCutTiles = 2, kRunningSum = 3 };
 enum EpilogueMode { kEpiPlainStores = 0, kEpiTmaStore = 1, kEpiTmaReduce = 2, kEpiVectorStores = 3 };
 
 struct KParams {
@@ -315,6 +315,15 @@ __device__ __forceinline__ void tmem_ld32_issue(uint32_t taddr, uint32_t (&v)[32
         : "r"(taddr)
         : "memory");
 }
+__device__ __forceinline__ void tmem_ld16_issue(uint32_t taddr, uint32_t (&v)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+        : "r"(taddr)
+        : "memory");
+}
 __device__ __forceinline__ void tmem_ld_wait() {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
@@ -481,11 +490,22 @@ __device__ __forceinline__ void load_operand(int mode, uint32_t dst, const CUten
 // of the stage (columns 2*BN + stage*64: 32 of hi, 32 of lo); no lo copy of A is written to shared
 // memory and no MMA re-reads A from it, which is what bounds narrow tiles otherwise.
 // TAIL: what the last wave may be.  kWholeTiles; kBalanced compiles the balanced tail's epilogue (parking / reducing
-// shared tiles) in; kCutTiles the split tail's (partial tiles to scratch).  Each instantiation carries only its own
-// code and registers (2 % of a single-pass 8192^3 product otherwise).
+// shared tiles) in; kCutTiles the split tail's (partial tiles to scratch).  kRunningSum: whole tiles whose contraction is
+// summed in several pieces, added up in the epilogue's registers instead of in memory (256-wide pairs, TMA stores, no
+// activation): 8192^3 single-pass 5.97 -> 5.53 ms a step, 3xTF32 1 %; its wide epilogue costs single-piece tiles 15 %.
+// Each instantiation carries only its own code and registers (2 % of a single-pass 8192^3 product otherwise).
 // SG = 2 (TA only): the split warps work as two groups on alternate k-blocks (see the split role).
+__host__ __device__ constexpr int gemm_threads(int ns, bool run) { return 32 * ((run ? 4 : 2) + ns + kEpiWarps); }
+// Register shares of the running-sum variants, in registers per thread, out of what the launch gives each thread (96 of
+// 640 threads, 128 of 512 in single-pass mode): two epilogue warpgroups, the split's and the one that issues.
+template <bool FAST>
+struct RegShare {
+    static constexpr int kEpilogue = FAST ? 216 : 168, kSplit = FAST ? 40 : 48, kIssue = FAST ? 40 : 48;
+    static constexpr int kSplitGroups = FAST ? 1 : 2, kLaunch = FAST ? 128 : 96;
+    static_assert(2 * kEpilogue + kSplitGroups * kSplit + kIssue <= (3 + kSplitGroups) * kLaunch, "more registers than the launch has");
+};
 template <int BN, int BK, bool FAST, int NS, int CG, bool TA = false, int TAIL = kWholeTiles, int SG = 1>
-__global__ void __launch_bounds__(32 * (2 + NS + kEpiWarps), 1)
+__global__ void __launch_bounds__(gemm_threads(NS, TAIL == kRunningSum), 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmD,
                const __grid_constant__ CUtensorMap tmP, const __grid_constant__ KParams p) {
@@ -494,6 +514,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     constexpr uint32_t A_BYTES = BM * BK * 4;
     constexpr uint32_t B_BYTES = BNL * BK * 4;
     constexpr uint32_t RAW_BYTES = A_BYTES + B_BYTES;
+    // RUN: a unit's running sum over its pieces takes 128 registers of every epilogue thread, so the warps are laid out in
+    // whole warpgroups -- TMA and MMA (and two idle), split, epilogue -- that trade registers.
+    constexpr bool RUN = TAIL == kRunningSum;
+    static_assert(!RUN || (BN == 256 && CG == 2), "running sums are built for 256-wide pairs");
+    constexpr int SPLIT0 = RUN ? 4 : 2, EPI0 = SPLIT0 + NS;   // first split and first epilogue warp
     static_assert(!TA || (!FAST && CG == 1 && BK == 32 && NS == 8 && BN <= 128), "unsupported A-from-TMEM variant");
     constexpr uint32_t STAGE_BYTES = FAST ? RAW_BYTES : (TA ? A_BYTES + 2 * B_BYTES : 2 * RAW_BYTES);
     constexpr uint32_t STAGE16 = STAGE_BYTES >> 4;
@@ -575,6 +600,393 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     if (p.dep_mode == 1 && threadIdx.x == 0) grid_dependency_trigger();
 
 
+    // The epilogue comes first: it is the branch whose register share the running-sum variants raise.
+    if (warp >= EPI0) {
+        // RUN: the warpgroups trade registers; the increase waits for the others' decrease
+        if constexpr (RUN) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(RegShare<FAST>::kEpilogue));
+        // ------------------------------------------------------------ epilogue
+        const int q = warp & 3;                       // TMEM lane quarter this warp may read
+        const int ew = warp - EPI0;               // 0..7: warps ew and ew+4 share a lane quarter ...
+        constexpr int CHUNKS = BN / 32 / (kEpiWarps / 4);   // ... and take half of the tile's 32-column chunks each
+        const int chunk_lo = (ew >> 2) * CHUNKS;
+        uint8_t *my_stage = epi_base + ew * p.epi_patches * kEpiBufBytes;
+        int acc_it = 0;
+        int patch = 0;                                // staging buffer to use next
+        int in_flight = 0;                            // bulk groups committed by lane 0 and not yet waited for
+        bool ok = true;
+        long long waited = 0, t_ld = 0, t_wg = 0;
+        const bool use_tma = p.epi_mode == kEpiTmaStore || p.epi_mode == kEpiTmaReduce;
+        const bool bias_vec = (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0;
+        WorkIter wi = work_begin(p, unit0, unit_step);
+        TileCoord t;
+        const int my_cta = static_cast<int>(blockIdx.x);                 // slot * CG + rank in the pair
+        uint32_t run[RUN ? CHUNKS : 1][32];           // RUN: sum of the unit's pieces so far
+        while (ok && work_next<TAIL>(p, wi, t)) {
+            const int buf = acc_it & 1;
+            const uint32_t acc_phase = (acc_it >> 1) & 1;
+            ok = mbar_wait(bar_acc_full + 8u * buf, acc_phase, abort_flag, p.err, 0x500u | buf, waited, timed, p.wait_cycles);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            tc_fence_after();
+            const bool part = CUT && t.part >= 0;            // of the split tail: a raw partial tile, always through TMA
+            const bool fuse = p.splits == 1 && !part;
+            const bool tma_here = use_tma || part;
+            const bool later_piece = t.chunk > 0;     // a later piece of this unit's contraction: added to the earlier ones
+            const bool last_piece = wi.piece_it >= wi.piece_end;
+            const bool add_piece = !RUN && later_piece;   // ... through memory
+            if (add_piece && tma_here) {
+                // this warp's earlier stores to the same patches must have completed, not just been read
+                if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+                in_flight = 0;
+                __syncwarp();
+            }
+            const int row0 = t.tm * (BM * CG) + static_cast<int>(cta_rank) * BM + q * 32;
+            const int cbatch = fuse ? t.bt : t.split * p.batch + t.bt;
+            const uint32_t tbase = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(buf * BN);
+            // Shared tile of the balanced tail.  Each (tile, CTA rank, epilogue warp) region has a ticket; the
+            // units of the tile arrive in any order, all but the last park their accumulator (and raise a
+            // ready flag), the last one adds the parked ones to its own in slot order -- the sum does not
+            // depend on who came last -- and runs the usual epilogue.
+            int seg_first = 0, seg_count = 1;          // slots sharing the tile: seg_first .. seg_first + seg_count - 1
+            bool reducer = false;
+            const int nslots = static_cast<int>(gridDim.x) / CG;
+            if (SK && t.shared) {
+                const long long per_tile = p.fold * p.kiters;
+                const long long tile_begin = static_cast<long long>(t.tile - p.sk_first_tile) * per_tile;
+                const long long tile_end = tile_begin + per_tile;
+                seg_first = unit0;
+                while (seg_first > 0 && sk_range_begin(p, seg_first, nslots) > tile_begin) --seg_first;
+                int last = unit0;
+                while (last + 1 < nslots && sk_range_begin(p, last + 1, nslots) < tile_end) ++last;
+                seg_count = last - seg_first + 1;
+            }
+            bool waited_contrib = false, parked = false;
+            unsigned int *ticket = nullptr;
+            if (SK && t.shared && seg_count > 1 && row0 < p.M && t.tn * BN + chunk_lo * 32 < p.N) {
+                const size_t region = (static_cast<size_t>(t.tile - p.sk_first_tile) * CG + cta_rank) * kEpiWarps + ew;
+                ticket = p.sk_flags + static_cast<size_t>(gridDim.x) * 2 * kEpiWarps + region;
+                unsigned int old = 0;
+                if (lane == 0) old = atomicAdd(ticket, 1u);
+                old = __shfl_sync(0xffffffffu, old, 0);
+                reducer = old == static_cast<unsigned int>(seg_count - 1);
+            }
+            const bool park_it = SK && t.shared && seg_count > 1 && !reducer;
+            // The reducer's list of the tile's other units, in slot order: index of their parking place
+            // ((cta * 2 + place) * warps + warp, also the index of its ready flag).
+            size_t others[kSkMaxShare - 1];
+            int n_others = 0, n_before = 0;
+            if (SK && reducer) {
+                const long long tile_begin = static_cast<long long>(t.tile - p.sk_first_tile) * (p.fold * p.kiters);
+                for (int j = seg_first; j < seg_first + seg_count; ++j) {
+                    if (j == unit0) continue;
+                    const int idx = (j == seg_first && sk_range_begin(p, j, nslots) < tile_begin) ? 1 : 0;
+                    others[n_others++] = (static_cast<size_t>(j * CG + static_cast<int>(cta_rank)) * 2 + idx) * kEpiWarps + ew;
+                    if (j < unit0) ++n_before;
+                }
+            }
+            if constexpr (RUN) {
+                __syncwarp();                          // tcgen05.ld is warp-collective
+                const long long t_ld0 = p.prof ? clock64() : 0;
+                if (!later_piece) {
+#pragma unroll
+                    for (int c = 0; c < CHUNKS; ++c) tmem_ld32_issue(tbase + (chunk_lo + c) * 32, run[c]);
+                    tmem_ld_wait();
+                } else {
+#pragma unroll
+                    for (int c = 0; c < 2 * CHUNKS; ++c) {
+                        uint32_t x[16];
+                        tmem_ld16_issue(tbase + chunk_lo * 32 + c * 16, x);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int e = 0; e < 16; ++e) {
+                            uint32_t &r = run[c / 2][(c & 1) * 16 + e];
+                            r = __float_as_uint(__uint_as_float(r) + __uint_as_float(x[e]));
+                        }
+                    }
+                }
+                if (p.prof) t_ld += clock64() - t_ld0;
+                // the accumulator has been read: the MMA warp may refill it while this sum goes out
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    if (CG == 2 && cta_rank != 0) mbar_arrive_cta(bar_acc_empty + 8u * buf, 0u);
+                    else mbar_arrive(bar_acc_empty + 8u * buf);
+                }
+                ++acc_it;
+                if (!last_piece) continue;
+            }
+            if (row0 < p.M) {
+#pragma unroll(RUN ? CHUNKS : 1)
+                for (int c = 0; c < CHUNKS; ++c) {
+                    const int chunk = chunk_lo + c;
+                    const int col0 = t.tn * BN + chunk * 32;
+                    if (col0 >= p.N) break;           // warp-uniform
+                    uint32_t loaded[32];
+                    uint32_t (&v)[32] = RUN ? run[RUN ? c : 0] : loaded;
+                    if constexpr (!RUN) {
+                        __syncwarp();                  // tcgen05.ld is warp-collective
+                        const long long t_ld0 = p.prof ? clock64() : 0;
+                        tmem_ld32_issue(tbase + chunk * 32, v);
+                        tmem_ld_wait();
+                        if (p.prof) t_ld += clock64() - t_ld0;
+                    }
+                    if (park_it) {
+                        // [j][lane] order: one instruction of the warp writes 512 contiguous bytes
+                        float4 *dst = reinterpret_cast<float4 *>(
+                            p.sk_partial + (((static_cast<size_t>(my_cta) * 2 + t.park) * kEpiWarps + ew) * CHUNKS + (chunk - chunk_lo)) * 1024) + lane;
+#pragma unroll
+                        for (int j = 0; j < 8; ++j)
+                            __stcg(dst + j * 32, make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
+                                                        __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3])));
+                        parked = true;
+                        continue;
+                    }
+                    if (SK && reducer) {
+                        if (!waited_contrib) {
+                            // Bounded wait for the ready flag of every other unit of the tile (they took their
+                            // tickets earlier, so they are at most one parking pass behind).
+                            for (int o = 0; ok && o < n_others; ++o) {
+                                const unsigned int *flag = p.sk_flags + others[o];
+                                const long long tw0 = clock64();
+                                unsigned int seen = 0;
+                                while (true) {
+                                    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(flag) : "memory");
+                                    if (seen != 0u) break;
+                                    if (*abort_flag || clock64() - tw0 > p.wait_cycles) {
+                                        *abort_flag = 1u;
+                                        atomicCAS(p.err, 0u, 0x600u);
+                                        ok = false;
+                                        break;
+                                    }
+                                }
+                            }
+                            ok = __all_sync(0xffffffffu, ok);
+                            waited_contrib = true;
+                            if (!ok) break;
+                        }
+                        // Sum in slot (= ascending k) order; this warp's own accumulator takes its place in it.
+                        // Each parked tile is fetched with independent 16-byte loads, half a chunk at a time.
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            float4 pre[4];
+                            for (int o = 0; o < n_before; ++o) {
+                                const float4 *src = reinterpret_cast<const float4 *>(
+                                                        p.sk_partial + (others[o] * CHUNKS + (chunk - chunk_lo)) * 1024) + h * 128 + lane;
+                                float4 x[4];
+#pragma unroll
+                                for (int u = 0; u < 4; ++u) x[u] = __ldcg(src + u * 32);
+#pragma unroll
+                                for (int u = 0; u < 4; ++u) {
+                                    if (o == 0) pre[u] = x[u];
+                                    else { pre[u].x += x[u].x; pre[u].y += x[u].y; pre[u].z += x[u].z; pre[u].w += x[u].w; }
+                                }
+                            }
+                            if (n_before > 0) {
+#pragma unroll
+                                for (int u = 0; u < 4; ++u) {
+                                    const int b = 16 * h + 4 * u;
+                                    v[b + 0] = __float_as_uint(pre[u].x + __uint_as_float(v[b + 0]));
+                                    v[b + 1] = __float_as_uint(pre[u].y + __uint_as_float(v[b + 1]));
+                                    v[b + 2] = __float_as_uint(pre[u].z + __uint_as_float(v[b + 2]));
+                                    v[b + 3] = __float_as_uint(pre[u].w + __uint_as_float(v[b + 3]));
+                                }
+                            }
+                            for (int o = n_before; o < n_others; ++o) {
+                                const float4 *src = reinterpret_cast<const float4 *>(
+                                                        p.sk_partial + (others[o] * CHUNKS + (chunk - chunk_lo)) * 1024) + h * 128 + lane;
+                                float4 x[4];
+#pragma unroll
+                                for (int u = 0; u < 4; ++u) x[u] = __ldcg(src + u * 32);
+#pragma unroll
+                                for (int u = 0; u < 4; ++u) {
+                                    const int b = 16 * h + 4 * u;
+                                    v[b + 0] = __float_as_uint(__uint_as_float(v[b + 0]) + x[u].x);
+                                    v[b + 1] = __float_as_uint(__uint_as_float(v[b + 1]) + x[u].y);
+                                    v[b + 2] = __float_as_uint(__uint_as_float(v[b + 2]) + x[u].z);
+                                    v[b + 3] = __float_as_uint(__uint_as_float(v[b + 3]) + x[u].w);
+                                }
+                            }
+                        }
+                    }
+                    // Stages the 32 values of this lane's row into the warp's next patch and hands the
+                    // patch to the TMA unit (store, or reduce-add for C += ...).
+                    auto emit = [&](const CUtensorMap *map, bool reduce) {
+                        const long long t_wg0 = p.prof ? clock64() : 0;
+                        if (lane == 0 && in_flight == p.epi_patches) {   // the patch must have been read by its store
+                            if (p.epi_patches == 1) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                            else if (p.epi_patches == 2) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+                            else if (p.epi_patches == 4) asm volatile("cp.async.bulk.wait_group.read 3;" ::: "memory");
+                            else asm volatile("cp.async.bulk.wait_group.read 7;" ::: "memory");
+                            --in_flight;
+                        }
+                        __syncwarp();
+                        if (p.prof) t_wg += clock64() - t_wg0;
+                        if (!RUN && p.transpose_out) {
+                            // patch row j = this chunk's column j, float `lane` of it = this lane's row:
+                            // the 32 lanes fill one 128-byte line per store, conflict-free
+                            uint8_t *dst = my_stage + patch * kEpiBufBytes + ((lane & 3) << 2);
+#pragma unroll
+                            for (int j = 0; j < 32; ++j)
+                                *reinterpret_cast<uint32_t *>(dst + j * 128 + (((lane >> 2) ^ (j & 7)) << 4)) = v[j];
+                        } else {
+                            uint8_t *dst = my_stage + patch * kEpiBufBytes + lane * 128;
+#pragma unroll
+                            for (int j = 0; j < 8; ++j)
+                                *reinterpret_cast<float4 *>(dst + ((j ^ (lane & 7)) << 4)) =
+                                    make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
+                                                __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
+                        }
+                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                        __syncwarp();
+                        if (lane == 0) {
+                            const uint32_t src = smem_u32(my_stage + patch * kEpiBufBytes);
+                            const int c0 = part ? chunk * 32 : (!RUN && p.transpose_out) ? row0 : col0;
+                            const int c1 = part ? static_cast<int>(cta_rank) * BM + q * 32 : (!RUN && p.transpose_out) ? col0 : row0;
+                            const int c2 = part ? t.part : cbatch;
+                            if (reduce) tma_reduce_add_5d(map, src, c0, c1, c2);
+                            else tma_store_5d(map, src, c0, c1, c2);
+                            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                            ++in_flight;
+                        }
+                        if (++patch == p.epi_patches) patch = 0;
+                    };
+                    const bool do_act = !RUN && fuse && p.act != 0;          // host guarantees use_tma in this mode
+                    if (do_act && p.store_pre) emit(&tmC, false);    // the raw product, what the tape saves
+                    if (fuse && p.bias != nullptr && add_piece) {
+                        // the bias went in with the first piece
+                    } else if (!RUN && fuse && p.bias != nullptr && p.transpose_out) {
+                        const float b = row0 + lane < p.M ? __ldg(p.bias + row0 + lane) : 0.f;   // one bias value per row here
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + b);
+                    } else if (fuse && p.bias != nullptr) {
+                        if (bias_vec && col0 + 32 <= p.N) {
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) {
+                                const float4 b = __ldg(reinterpret_cast<const float4 *>(p.bias + col0) + j);
+                                v[4 * j + 0] = __float_as_uint(__uint_as_float(v[4 * j + 0]) + b.x);
+                                v[4 * j + 1] = __float_as_uint(__uint_as_float(v[4 * j + 1]) + b.y);
+                                v[4 * j + 2] = __float_as_uint(__uint_as_float(v[4 * j + 2]) + b.z);
+                                v[4 * j + 3] = __float_as_uint(__uint_as_float(v[4 * j + 3]) + b.w);
+                            }
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < 32; ++j)
+                                if (col0 + j < p.N) v[j] = __float_as_uint(__uint_as_float(v[j]) + __ldg(p.bias + col0 + j));
+                        }
+                    }
+                    if (do_act) {
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(gelu_tanh_f(__uint_as_float(v[j])));
+                        emit(&tmD, false);
+                    } else if (part) {
+                        emit(&tmP, add_piece);
+                    } else if (RUN || use_tma) {
+                        emit(&tmC, (p.epi_mode == kEpiTmaReduce && fuse) || add_piece);
+                    } else {
+                        float *out0 = fuse ? p.C + static_cast<long long>(t.bt) * p.c_bstride + static_cast<long long>(row0) * p.ldc
+                                           : p.partial + (static_cast<long long>(cbatch) * p.M + row0) * p.partial_ld;
+                        const long long pitch = fuse ? p.ldc : p.partial_ld;
+                        const bool add = (fuse && p.accumulate) || add_piece;
+                        if (p.epi_mode == kEpiVectorStores && col0 + 32 <= p.N) {
+                            // Each lane owns one row: four 32-byte stores write whole sectors, no staging.
+                            if (row0 + lane >= p.M) continue;
+                            float *dst = out0 + lane * pitch + col0;
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                float y[8];
+#pragma unroll
+                                for (int e = 0; e < 8; ++e) y[e] = __uint_as_float(v[8 * j + e]);
+                                if (add) {
+                                    float o[8];
+                                    asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                                                 : "=f"(o[0]), "=f"(o[1]), "=f"(o[2]), "=f"(o[3]), "=f"(o[4]), "=f"(o[5]),
+                                                   "=f"(o[6]), "=f"(o[7])
+                                                 : "l"(dst + 8 * j));
+#pragma unroll
+                                    for (int e = 0; e < 8; ++e) y[e] += o[e];
+                                }
+                                asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst + 8 * j),
+                                             "f"(y[0]), "f"(y[1]), "f"(y[2]), "f"(y[3]), "f"(y[4]), "f"(y[5]), "f"(y[6]),
+                                             "f"(y[7])
+                                             : "memory");
+                            }
+                            continue;
+                        }
+                        // Rows that are not 16-byte aligned (an odd width): the patch is turned in the warp's staging
+                        // buffer, so that every store covers 32 neighbouring columns of one row.  Stored straight from
+                        // the accumulator's row-per-lane order each instruction touched 32 rows (attention scores of
+                        // length 333: 75 us a product).
+                        uint8_t *mine = my_stage + lane * 128;
+#pragma unroll
+                        for (int j = 0; j < 8; ++j)
+                            *reinterpret_cast<float4 *>(mine + ((j ^ (lane & 7)) << 4)) =
+                                make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
+                                            __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
+                        __syncwarp();
+                        const int rows = min(32, p.M - row0);
+                        if (col0 + lane < p.N) {
+                            float *dst = out0 + col0 + lane;
+                            const uint8_t *src = my_stage + ((lane & 3) << 2);
+#pragma unroll 2
+                            for (int r4 = 0; r4 < 32; r4 += 4) {
+                                float y[4];
+#pragma unroll
+                                for (int r = 0; r < 4; ++r)
+                                    y[r] = *reinterpret_cast<const float *>(src + (r4 + r) * 128 + (((lane >> 2) ^ ((r4 + r) & 7)) << 4));
+                                if (add) {
+#pragma unroll
+                                    for (int r = 0; r < 4; ++r) y[r] += r4 + r < rows ? dst[(r4 + r) * pitch] : 0.f;
+                                }
+#pragma unroll
+                                for (int r = 0; r < 4; ++r)
+                                    if (r4 + r < rows) dst[(r4 + r) * pitch] = y[r];
+                            }
+                        }
+                        __syncwarp();                  // the staging buffer is free again
+                    }
+                }
+            }
+            if (!ok) break;
+            if (parked) {
+                // publish: every lane's stores are fenced, then one release store of the ready flag
+                __threadfence();
+                __syncwarp();
+                if (lane == 0) {
+                    unsigned int *flag = p.sk_flags + ((static_cast<size_t>(my_cta) * 2 + t.park) * kEpiWarps + ew);
+                    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(flag), "r"(1u) : "memory");
+                }
+            } else if (SK && reducer) {
+                // every lane has read the parked tiles: ticket and ready flags go back to zero for the next launch
+                __syncwarp();
+                if (lane == 0) {
+                    *ticket = 0u;
+                    if (waited_contrib)
+                        for (int o = 0; o < n_others; ++o) p.sk_flags[others[o]] = 0u;
+                }
+            }
+            if constexpr (!RUN) {
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    if (CG == 2 && cta_rank != 0) mbar_arrive_cta(bar_acc_empty + 8u * buf, 0u);
+                    else mbar_arrive(bar_acc_empty + 8u * buf);
+                }
+                ++acc_it;
+            }
+        }
+        // The staging patches must have been read before the CTA gives up its shared memory; the global
+        // writes themselves complete with the grid like any other store.
+        if ((use_tma || CUT) && lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        if (p.prof && warp == EPI0 && lane == 0) {
+            atomicAdd(p.prof + 4, static_cast<unsigned long long>(waited));
+            atomicAdd(p.prof + 7, static_cast<unsigned long long>(t_wg));
+            atomicAdd(p.prof + 1, static_cast<unsigned long long>(t_ld));
+        }
+    } else {
+    if constexpr (RUN) {
+        if (warp < SPLIT0) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(RegShare<FAST>::kIssue));
+        else asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(RegShare<FAST>::kSplit));
+    }
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
         // The whole warp runs the loop; one elected lane issues the copies.
@@ -727,7 +1139,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 atomicAdd(p.prof + 2, static_cast<unsigned long long>(waited));
             }
         }
-    } else if (warp < 2 + NS) {
+    } else if (RUN && warp < SPLIT0) {
+        // idle: the rest of the first warpgroup
+    } else {
         // ------------------------------------------------------------ hi/lo split
         // In single-pass mode there is nothing to split; for a CTA pair these warps still relay "my
         // CTA's tile has landed" to the leader's barrier.
@@ -739,8 +1153,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             // two k-blocks in flight.  The host picks SG = 2 for long contractions.
             static_assert(SG == 1 || (SG == 2 && TA), "two split groups exist for the tensor-memory A variants only");
             constexpr int GROUPS = SG;
-            const int group = TA ? (warp - 2) >> 2 : 0;   // SG = 1: the k-half this warp splits; SG = 2: its group
-            const int tid = (threadIdx.x - 64) & (32 * NS / GROUPS - 1);   // index within the group
+            const int group = TA ? (warp - SPLIT0) >> 2 : 0;   // SG = 1: the k-half this warp splits; SG = 2: its group
+            const int tid = (threadIdx.x - 32 * SPLIT0) & (32 * NS / GROUPS - 1);   // index within the group
             int stage = 0;
             int kb = 0;                                   // k-blocks this CTA has seen: the group takes those of its parity
             uint32_t phase = 0;
@@ -842,344 +1256,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             }
             if (p.prof && tid == 0) atomicAdd(p.prof + 3, static_cast<unsigned long long>(waited));
         }
-    } else {
-        // ------------------------------------------------------------ epilogue
-        const int q = warp & 3;                       // TMEM lane quarter this warp may read
-        const int ew = warp - (2 + NS);               // 0..7: warps ew and ew+4 share a lane quarter ...
-        constexpr int CHUNKS = BN / 32 / (kEpiWarps / 4);   // ... and take half of the tile's 32-column chunks each
-        const int chunk_lo = (ew >> 2) * CHUNKS;
-        uint8_t *my_stage = epi_base + ew * p.epi_patches * kEpiBufBytes;
-        int acc_it = 0;
-        int patch = 0;                                // staging buffer to use next
-        int in_flight = 0;                            // bulk groups committed by lane 0 and not yet waited for
-        bool ok = true;
-        long long waited = 0, t_ld = 0, t_wg = 0;
-        const bool use_tma = p.epi_mode == kEpiTmaStore || p.epi_mode == kEpiTmaReduce;
-        const bool bias_vec = (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0;
-        WorkIter wi = work_begin(p, unit0, unit_step);
-        TileCoord t;
-        const int my_cta = static_cast<int>(blockIdx.x);                 // slot * CG + rank in the pair
-        while (ok && work_next<TAIL>(p, wi, t)) {
-            const int buf = acc_it & 1;
-            const uint32_t acc_phase = (acc_it >> 1) & 1;
-            ok = mbar_wait(bar_acc_full + 8u * buf, acc_phase, abort_flag, p.err, 0x500u | buf, waited, timed, p.wait_cycles);
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) break;
-            tc_fence_after();
-            const bool part = CUT && t.part >= 0;            // of the split tail: a raw partial tile, always through TMA
-            const bool fuse = p.splits == 1 && !part;
-            const bool tma_here = use_tma || part;
-            const bool add_piece = t.chunk > 0;       // a later piece of this unit's contraction: added to what the earlier ones wrote
-            if (add_piece && tma_here) {
-                // this warp's earlier stores to the same patches must have completed, not just been read
-                if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-                in_flight = 0;
-                __syncwarp();
-            }
-            const int row0 = t.tm * (BM * CG) + static_cast<int>(cta_rank) * BM + q * 32;
-            const int cbatch = fuse ? t.bt : t.split * p.batch + t.bt;
-            const uint32_t tbase = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(buf * BN);
-            // Shared tile of the balanced tail.  Each (tile, CTA rank, epilogue warp) region has a ticket; the
-            // units of the tile arrive in any order, all but the last park their accumulator (and raise a
-            // ready flag), the last one adds the parked ones to its own in slot order -- the sum does not
-            // depend on who came last -- and runs the usual epilogue.
-            int seg_first = 0, seg_count = 1;          // slots sharing the tile: seg_first .. seg_first + seg_count - 1
-            bool reducer = false;
-            const int nslots = static_cast<int>(gridDim.x) / CG;
-            if (SK && t.shared) {
-                const long long per_tile = p.fold * p.kiters;
-                const long long tile_begin = static_cast<long long>(t.tile - p.sk_first_tile) * per_tile;
-                const long long tile_end = tile_begin + per_tile;
-                seg_first = unit0;
-                while (seg_first > 0 && sk_range_begin(p, seg_first, nslots) > tile_begin) --seg_first;
-                int last = unit0;
-                while (last + 1 < nslots && sk_range_begin(p, last + 1, nslots) < tile_end) ++last;
-                seg_count = last - seg_first + 1;
-            }
-            bool waited_contrib = false, parked = false;
-            unsigned int *ticket = nullptr;
-            if (SK && t.shared && seg_count > 1 && row0 < p.M && t.tn * BN + chunk_lo * 32 < p.N) {
-                const size_t region = (static_cast<size_t>(t.tile - p.sk_first_tile) * CG + cta_rank) * kEpiWarps + ew;
-                ticket = p.sk_flags + static_cast<size_t>(gridDim.x) * 2 * kEpiWarps + region;
-                unsigned int old = 0;
-                if (lane == 0) old = atomicAdd(ticket, 1u);
-                old = __shfl_sync(0xffffffffu, old, 0);
-                reducer = old == static_cast<unsigned int>(seg_count - 1);
-            }
-            const bool park_it = SK && t.shared && seg_count > 1 && !reducer;
-            // The reducer's list of the tile's other units, in slot order: index of their parking place
-            // ((cta * 2 + place) * warps + warp, also the index of its ready flag).
-            size_t others[kSkMaxShare - 1];
-            int n_others = 0, n_before = 0;
-            if (SK && reducer) {
-                const long long tile_begin = static_cast<long long>(t.tile - p.sk_first_tile) * (p.fold * p.kiters);
-                for (int j = seg_first; j < seg_first + seg_count; ++j) {
-                    if (j == unit0) continue;
-                    const int idx = (j == seg_first && sk_range_begin(p, j, nslots) < tile_begin) ? 1 : 0;
-                    others[n_others++] = (static_cast<size_t>(j * CG + static_cast<int>(cta_rank)) * 2 + idx) * kEpiWarps + ew;
-                    if (j < unit0) ++n_before;
-                }
-            }
-            if (row0 < p.M) {
-                for (int chunk = chunk_lo; chunk < chunk_lo + CHUNKS; ++chunk) {
-                    const int col0 = t.tn * BN + chunk * 32;
-                    if (col0 >= p.N) break;           // warp-uniform
-                    uint32_t v[32];
-                    __syncwarp();                      // tcgen05.ld is warp-collective
-                    const long long t_ld0 = p.prof ? clock64() : 0;
-                    tmem_ld32_issue(tbase + chunk * 32, v);
-                    tmem_ld_wait();
-                    if (p.prof) t_ld += clock64() - t_ld0;
-                    if (park_it) {
-                        // [j][lane] order: one instruction of the warp writes 512 contiguous bytes
-                        float4 *dst = reinterpret_cast<float4 *>(
-                            p.sk_partial + (((static_cast<size_t>(my_cta) * 2 + t.park) * kEpiWarps + ew) * CHUNKS + (chunk - chunk_lo)) * 1024) + lane;
-#pragma unroll
-                        for (int j = 0; j < 8; ++j)
-                            __stcg(dst + j * 32, make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
-                                                        __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3])));
-                        parked = true;
-                        continue;
-                    }
-                    if (SK && reducer) {
-                        if (!waited_contrib) {
-                            // Bounded wait for the ready flag of every other unit of the tile (they took their
-                            // tickets earlier, so they are at most one parking pass behind).
-                            for (int o = 0; ok && o < n_others; ++o) {
-                                const unsigned int *flag = p.sk_flags + others[o];
-                                const long long tw0 = clock64();
-                                unsigned int seen = 0;
-                                while (true) {
-                                    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(flag) : "memory");
-                                    if (seen != 0u) break;
-                                    if (*abort_flag || clock64() - tw0 > p.wait_cycles) {
-                                        *abort_flag = 1u;
-                                        atomicCAS(p.err, 0u, 0x600u);
-                                        ok = false;
-                                        break;
-                                    }
-                                }
-                            }
-                            ok = __all_sync(0xffffffffu, ok);
-                            waited_contrib = true;
-                            if (!ok) break;
-                        }
-                        // Sum in slot (= ascending k) order; this warp's own accumulator takes its place in it.
-                        // Each parked tile is fetched with independent 16-byte loads, half a chunk at a time.
-#pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            float4 pre[4];
-                            for (int o = 0; o < n_before; ++o) {
-                                const float4 *src = reinterpret_cast<const float4 *>(
-                                                        p.sk_partial + (others[o] * CHUNKS + (chunk - chunk_lo)) * 1024) + h * 128 + lane;
-                                float4 x[4];
-#pragma unroll
-                                for (int u = 0; u < 4; ++u) x[u] = __ldcg(src + u * 32);
-#pragma unroll
-                                for (int u = 0; u < 4; ++u) {
-                                    if (o == 0) pre[u] = x[u];
-                                    else { pre[u].x += x[u].x; pre[u].y += x[u].y; pre[u].z += x[u].z; pre[u].w += x[u].w; }
-                                }
-                            }
-                            if (n_before > 0) {
-#pragma unroll
-                                for (int u = 0; u < 4; ++u) {
-                                    const int b = 16 * h + 4 * u;
-                                    v[b + 0] = __float_as_uint(pre[u].x + __uint_as_float(v[b + 0]));
-                                    v[b + 1] = __float_as_uint(pre[u].y + __uint_as_float(v[b + 1]));
-                                    v[b + 2] = __float_as_uint(pre[u].z + __uint_as_float(v[b + 2]));
-                                    v[b + 3] = __float_as_uint(pre[u].w + __uint_as_float(v[b + 3]));
-                                }
-                            }
-                            for (int o = n_before; o < n_others; ++o) {
-                                const float4 *src = reinterpret_cast<const float4 *>(
-                                                        p.sk_partial + (others[o] * CHUNKS + (chunk - chunk_lo)) * 1024) + h * 128 + lane;
-                                float4 x[4];
-#pragma unroll
-                                for (int u = 0; u < 4; ++u) x[u] = __ldcg(src + u * 32);
-#pragma unroll
-                                for (int u = 0; u < 4; ++u) {
-                                    const int b = 16 * h + 4 * u;
-                                    v[b + 0] = __float_as_uint(__uint_as_float(v[b + 0]) + x[u].x);
-                                    v[b + 1] = __float_as_uint(__uint_as_float(v[b + 1]) + x[u].y);
-                                    v[b + 2] = __float_as_uint(__uint_as_float(v[b + 2]) + x[u].z);
-                                    v[b + 3] = __float_as_uint(__uint_as_float(v[b + 3]) + x[u].w);
-                                }
-                            }
-                        }
-                    }
-                    // Stages the 32 values of this lane's row into the warp's next patch and hands the
-                    // patch to the TMA unit (store, or reduce-add for C += ...).
-                    auto emit = [&](const CUtensorMap *map, bool reduce) {
-                        const long long t_wg0 = p.prof ? clock64() : 0;
-                        if (lane == 0 && in_flight == p.epi_patches) {   // the patch must have been read by its store
-                            if (p.epi_patches == 1) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-                            else if (p.epi_patches == 2) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-                            else if (p.epi_patches == 4) asm volatile("cp.async.bulk.wait_group.read 3;" ::: "memory");
-                            else asm volatile("cp.async.bulk.wait_group.read 7;" ::: "memory");
-                            --in_flight;
-                        }
-                        __syncwarp();
-                        if (p.prof) t_wg += clock64() - t_wg0;
-                        if (p.transpose_out) {
-                            // patch row j = this chunk's column j, float `lane` of it = this lane's row:
-                            // the 32 lanes fill one 128-byte line per store, conflict-free
-                            uint8_t *dst = my_stage + patch * kEpiBufBytes + ((lane & 3) << 2);
-#pragma unroll
-                            for (int j = 0; j < 32; ++j)
-                                *reinterpret_cast<uint32_t *>(dst + j * 128 + (((lane >> 2) ^ (j & 7)) << 4)) = v[j];
-                        } else {
-                            uint8_t *dst = my_stage + patch * kEpiBufBytes + lane * 128;
-#pragma unroll
-                            for (int j = 0; j < 8; ++j)
-                                *reinterpret_cast<float4 *>(dst + ((j ^ (lane & 7)) << 4)) =
-                                    make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
-                                                __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
-                        }
-                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                        __syncwarp();
-                        if (lane == 0) {
-                            const uint32_t src = smem_u32(my_stage + patch * kEpiBufBytes);
-                            const int c0 = part ? chunk * 32 : p.transpose_out ? row0 : col0;
-                            const int c1 = part ? static_cast<int>(cta_rank) * BM + q * 32 : p.transpose_out ? col0 : row0;
-                            const int c2 = part ? t.part : cbatch;
-                            if (reduce) tma_reduce_add_5d(map, src, c0, c1, c2);
-                            else tma_store_5d(map, src, c0, c1, c2);
-                            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-                            ++in_flight;
-                        }
-                        if (++patch == p.epi_patches) patch = 0;
-                    };
-                    const bool do_act = fuse && p.act != 0;          // host guarantees use_tma in this mode
-                    if (do_act && p.store_pre) emit(&tmC, false);    // the raw product, what the tape saves
-                    if (fuse && p.bias != nullptr && add_piece) {
-                        // the bias went in with the first piece
-                    } else if (fuse && p.bias != nullptr && p.transpose_out) {
-                        const float b = row0 + lane < p.M ? __ldg(p.bias + row0 + lane) : 0.f;   // one bias value per row here
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + b);
-                    } else if (fuse && p.bias != nullptr) {
-                        if (bias_vec && col0 + 32 <= p.N) {
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) {
-                                const float4 b = __ldg(reinterpret_cast<const float4 *>(p.bias + col0) + j);
-                                v[4 * j + 0] = __float_as_uint(__uint_as_float(v[4 * j + 0]) + b.x);
-                                v[4 * j + 1] = __float_as_uint(__uint_as_float(v[4 * j + 1]) + b.y);
-                                v[4 * j + 2] = __float_as_uint(__uint_as_float(v[4 * j + 2]) + b.z);
-                                v[4 * j + 3] = __float_as_uint(__uint_as_float(v[4 * j + 3]) + b.w);
-                            }
-                        } else {
-#pragma unroll
-                            for (int j = 0; j < 32; ++j)
-                                if (col0 + j < p.N) v[j] = __float_as_uint(__uint_as_float(v[j]) + __ldg(p.bias + col0 + j));
-                        }
-                    }
-                    if (do_act) {
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(gelu_tanh_f(__uint_as_float(v[j])));
-                        emit(&tmD, false);
-                    } else if (part) {
-                        emit(&tmP, add_piece);
-                    } else if (use_tma) {
-                        emit(&tmC, (p.epi_mode == kEpiTmaReduce && fuse) || add_piece);
-                    } else {
-                        float *out0 = fuse ? p.C + static_cast<long long>(t.bt) * p.c_bstride + static_cast<long long>(row0) * p.ldc
-                                           : p.partial + (static_cast<long long>(cbatch) * p.M + row0) * p.partial_ld;
-                        const long long pitch = fuse ? p.ldc : p.partial_ld;
-                        const bool add = (fuse && p.accumulate) || add_piece;
-                        if (p.epi_mode == kEpiVectorStores && col0 + 32 <= p.N) {
-                            // Each lane owns one row: four 32-byte stores write whole sectors, no staging.
-                            if (row0 + lane >= p.M) continue;
-                            float *dst = out0 + lane * pitch + col0;
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) {
-                                float y[8];
-#pragma unroll
-                                for (int e = 0; e < 8; ++e) y[e] = __uint_as_float(v[8 * j + e]);
-                                if (add) {
-                                    float o[8];
-                                    asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                                                 : "=f"(o[0]), "=f"(o[1]), "=f"(o[2]), "=f"(o[3]), "=f"(o[4]), "=f"(o[5]),
-                                                   "=f"(o[6]), "=f"(o[7])
-                                                 : "l"(dst + 8 * j));
-#pragma unroll
-                                    for (int e = 0; e < 8; ++e) y[e] += o[e];
-                                }
-                                asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst + 8 * j),
-                                             "f"(y[0]), "f"(y[1]), "f"(y[2]), "f"(y[3]), "f"(y[4]), "f"(y[5]), "f"(y[6]),
-                                             "f"(y[7])
-                                             : "memory");
-                            }
-                            continue;
-                        }
-                        // Rows that are not 16-byte aligned (an odd width): the patch is turned in the warp's staging
-                        // buffer, so that every store covers 32 neighbouring columns of one row.  Stored straight from
-                        // the accumulator's row-per-lane order each instruction touched 32 rows (attention scores of
-                        // length 333: 75 us a product).
-                        uint8_t *mine = my_stage + lane * 128;
-#pragma unroll
-                        for (int j = 0; j < 8; ++j)
-                            *reinterpret_cast<float4 *>(mine + ((j ^ (lane & 7)) << 4)) =
-                                make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
-                                            __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
-                        __syncwarp();
-                        const int rows = min(32, p.M - row0);
-                        if (col0 + lane < p.N) {
-                            float *dst = out0 + col0 + lane;
-                            const uint8_t *src = my_stage + ((lane & 3) << 2);
-#pragma unroll 2
-                            for (int r4 = 0; r4 < 32; r4 += 4) {
-                                float y[4];
-#pragma unroll
-                                for (int r = 0; r < 4; ++r)
-                                    y[r] = *reinterpret_cast<const float *>(src + (r4 + r) * 128 + (((lane >> 2) ^ ((r4 + r) & 7)) << 4));
-                                if (add) {
-#pragma unroll
-                                    for (int r = 0; r < 4; ++r) y[r] += r4 + r < rows ? dst[(r4 + r) * pitch] : 0.f;
-                                }
-#pragma unroll
-                                for (int r = 0; r < 4; ++r)
-                                    if (r4 + r < rows) dst[(r4 + r) * pitch] = y[r];
-                            }
-                        }
-                        __syncwarp();                  // the staging buffer is free again
-                    }
-                }
-            }
-            if (!ok) break;
-            if (parked) {
-                // publish: every lane's stores are fenced, then one release store of the ready flag
-                __threadfence();
-                __syncwarp();
-                if (lane == 0) {
-                    unsigned int *flag = p.sk_flags + ((static_cast<size_t>(my_cta) * 2 + t.park) * kEpiWarps + ew);
-                    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(flag), "r"(1u) : "memory");
-                }
-            } else if (SK && reducer) {
-                // every lane has read the parked tiles: ticket and ready flags go back to zero for the next launch
-                __syncwarp();
-                if (lane == 0) {
-                    *ticket = 0u;
-                    if (waited_contrib)
-                        for (int o = 0; o < n_others; ++o) p.sk_flags[others[o]] = 0u;
-                }
-            }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) {
-                if (CG == 2 && cta_rank != 0) mbar_arrive_cta(bar_acc_empty + 8u * buf, 0u);
-                else mbar_arrive(bar_acc_empty + 8u * buf);
-            }
-            ++acc_it;
-        }
-        // The staging patches must have been read before the CTA gives up its shared memory; the global
-        // writes themselves complete with the grid like any other store.
-        if ((use_tma || CUT) && lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-        if (p.prof && warp == 2 + NS && lane == 0) {
-            atomicAdd(p.prof + 4, static_cast<unsigned long long>(waited));
-            atomicAdd(p.prof + 7, static_cast<unsigned long long>(t_wg));
-            atomicAdd(p.prof + 1, static_cast<unsigned long long>(t_ld));
-        }
+    }
     }
 
     tc_fence_before();
@@ -1670,7 +1747,7 @@ cudaError_t launch_variant(const Plan &pl, const CUtensorMap &tmA, const CUtenso
     }
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(static_cast<unsigned>(pl.grid));
-    cfg.blockDim = dim3(32 * (2 + NS + kEpiWarps));
+    cfg.blockDim = dim3(gemm_threads(NS, TAIL == kRunningSum));
     cfg.dynamicSmemBytes = pl.smem;
     cfg.stream = stream;
     cudaLaunchAttribute attrs[2];
@@ -1964,6 +2041,11 @@ int launch_gemm_tc(const GemmProblem &p0, float *partial, uint32_t *err_word, in
         const int sg_env = env_int("MNI_B200_SPLIT_GROUPS", 0);
         split_groups = (sg_env == 1 || sg_env == 2) ? sg_env : (unit_iters >= 12 ? 2 : 1);
     }
+    // Units summed in several pieces keep their running sum in registers where that is built (the kernel's first_piece
+    // rule decides what is cut).
+    const long long unit_len = (static_cast<long long>(k.fold) * k.kiters + pl.splits - 1) / pl.splits;
+    const bool running = pl.cg == 2 && pl.bn == 256 && pl.bk == (p.fast_tf32 ? 32 : 16) && !pl.sk && !pl.tail_ways && k.chunk_iters > 0 &&
+                         unit_len > k.chunk_iters + (k.chunk_iters >> 1) && (k.epi_mode == kEpiTmaStore || k.epi_mode == kEpiTmaReduce);
     cudaError_t e = cudaErrorInvalidValue;
     if (pl.sk) {
         if (pl.ta && pl.bn == 64 && split_groups == 2) e = launch_variant<64, 32, false, 8, 1, true, kBalanced, 2>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
@@ -1974,6 +2056,10 @@ int launch_gemm_tc(const GemmProblem &p0, float *partial, uint32_t *err_word, in
         else if (!p.fast_tf32 && pl.bk == 32) e = launch_variant<256, 32, false, 8, 2, false, kBalanced>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
         else if (pl.bk == 16) e = launch_variant<256, 16, true, 4, 2, false, kBalanced>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
         else e = launch_variant<256, 32, true, 4, 2, false, kBalanced>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+    } else if (running && p.fast_tf32) {
+        e = launch_variant<256, 32, true, 4, 2, false, kRunningSum>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+    } else if (running) {
+        e = launch_variant<256, 16, false, 8, 2, false, kRunningSum>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
     } else if (pl.tail_ways) {
         if (!p.fast_tf32 && pl.bk == 16) e = launch_variant<256, 16, false, 8, 2, false, kCutTiles>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
         else if (!p.fast_tf32) e = launch_variant<256, 32, false, 8, 2, false, kCutTiles>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
@@ -1991,7 +2077,7 @@ int launch_gemm_tc(const GemmProblem &p0, float *partial, uint32_t *err_word, in
         else e = launch_variant<BN_, BK_, false, 8, 1>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);                 \
     }
 #define MNI_PAIR_VARIANT(BN_, BK_)                                                                    \
-    if (pl.cg == 2 && !pl.sk && !pl.tail_ways && pl.bn == BN_ && pl.bk == BK_) {                                                 \
+    if (pl.cg == 2 && !pl.sk && !pl.tail_ways && !running && pl.bn == BN_ && pl.bk == BK_) {                                                 \
         if (p.fast_tf32) e = launch_variant<BN_, BK_, true, 4, 2>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);      \
         else e = launch_variant<BN_, BK_, false, 8, 2>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);                 \
     }
