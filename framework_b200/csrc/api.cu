@@ -80,6 +80,12 @@ constexpr int64_t kSkinnyDxRows = 5, kSkinnyDwRows = 8;
 // 16-byte aligned it would have to gather first.
 constexpr int64_t kRowsAligned = 15, kRowsUnaligned = 16;
 
+// Limits of the one-launch f32 kernel (tiny.cu): it needs about 1.9 us and 1 us per 64 contraction elements, whatever the
+// rest of the shape, up to M * N * K = 8 M (192^3: forward 5.0 us against 7.7, backward 5.8 against 8.9; 256^3 is level;
+// K = 512 loses).  Up to 8 rows the streaming kernels are the competition.
+constexpr int64_t kTinyContraction = 320, kTinyContractionFewRows = 128;
+constexpr int kTinyWork = 1 << 23;
+
 bool env_flag(const char *name, int dflt) { return env_int(name, dflt) != 0; }
 
 // Bump allocator over the device's scratch.  In dry mode nothing is touched: the
@@ -442,6 +448,18 @@ bool rows_wanted(uint32_t flags, const Shapes &s, const mni_b200_view &w) {
            s.M <= (aligned ? kRowsAligned : kRowsUnaligned);
 }
 
+// Small enough for the one-launch f32 kernel: a single matrix product whose longest contraction (forward K, backward
+// M and N) and whose work are both small, operands readable along one of their dims.  MNI_B200_TINY overrides the limit on
+// M * N * K (0: never).
+bool tiny_wanted(uint32_t flags, const Shapes &s, const mni_b200_view &a, const mni_b200_view &b, const mni_b200_view *dc) {
+    auto readable = [](const mni_b200_view &v) { return v.stride[v.ndim - 1] == 1 || v.stride[v.ndim - 2] == 1; };
+    const uint32_t forced = MNI_B200_FORCE_TENSOR_PATH | MNI_B200_FORCE_SKINNY_PATH | MNI_B200_FORCE_PACK | MNI_B200_PRECISION_TF32;
+    return (flags & forced) == 0 && ((flags >> 16) & 0xffu) == 0 && s.batch == 1 && s.a_batch == 1 && s.b_batch == 1 &&
+           (dc ? std::max(s.M, s.N) : s.K) <= (s.M <= 8 ? kTinyContractionFewRows : kTinyContraction) &&
+           std::max({s.M, s.N, s.K}) <= kTinyWork && s.M * s.N * s.K <= env_int("MNI_B200_TINY", kTinyWork) && readable(a) &&
+           readable(b) && (!dc || readable(*dc));
+}
+
 // ------------------------------------------------------------------ forward
 int fwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, float *out, const float *bias) {
     Shapes s;
@@ -453,6 +471,14 @@ int fwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, float *out
     if (s.K == 0) return zero_or_bias_fill(c, out, s.batch * s.M, s.N, bias, accumulate);
 
     if (!*c.label) c.label = "forward: ";
+    if (tiny_wanted(c.flags, s, *a, *b, nullptr)) {
+        c.note("small f32 kernel");
+        if (c.dry()) return MNI_B200_OK;
+        const TinyProduct p{a->ptr, b->ptr, out, bias, static_cast<int>(s.M), static_cast<int>(s.N), static_cast<int>(s.K),
+                            accumulate ? 1 : 0, a->stride[a->ndim - 2], a->stride[a->ndim - 1], b->stride[b->ndim - 2],
+                            b->stride[b->ndim - 1], s.N};
+        return launch_tiny(&p, 1, nullptr, c.stream);
+    }
     const bool want_skinny = (c.flags & MNI_B200_FORCE_SKINNY_PATH) != 0 ||
                              ((c.flags & MNI_B200_FORCE_TENSOR_PATH) == 0 && s.M <= skinny_fwd_row_limit(s.N));
     if (want_skinny && s.batch == 1 && skinny_fwd_supported(s.M, s.N, s.K)) {
@@ -514,7 +540,7 @@ int fwd_gelu_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const
     if (!bias || !out) return fail(MNI_B200_ERR_ARG, "bias and out must not be null");
     const uint32_t saved_flags = c.flags;
     c.flags &= ~static_cast<uint32_t>(MNI_B200_ACCUMULATE_C);
-    const bool skinny = (c.flags & MNI_B200_FORCE_SKINNY_PATH) != 0 ||
+    const bool skinny = (c.flags & MNI_B200_FORCE_SKINNY_PATH) != 0 || tiny_wanted(c.flags, s, *a, *b, nullptr) ||
                         ((c.flags & MNI_B200_FORCE_TENSOR_PATH) == 0 && s.M <= skinny_fwd_row_limit(s.N));
     if (s.K > 0 && !skinny) {
         GemmProblem p;
@@ -622,6 +648,22 @@ int bwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const mni_
     // Which kernel each gradient takes.
     const bool da_wanted = da && a_elems > 0 && s.N > 0 && g_batch > 0;
     const bool db_wanted = db && b_elems > 0 && s.M > 0 && g_batch > 0;
+    if (g_batch == 1 && s.M > 0 && s.N > 0 && s.K > 0 && (da || db) && (!dbias || dc->stride[gn - 1] == 1) &&
+        tiny_wanted(c.flags, s, *a, *b, dc)) {
+        c.label = "grad_a, grad_b, grad_bias: ";
+        c.note("small f32 kernel");
+        c.label = "";
+        if (c.dry()) return MNI_B200_OK;
+        const int M = static_cast<int>(s.M), N = static_cast<int>(s.N), K = static_cast<int>(s.K);
+        const long long a_m = a->stride[a->ndim - 2], a_k = a->stride[a->ndim - 1], b_k = b->stride[b->ndim - 2],
+                        b_n = b->stride[b->ndim - 1], g_m = dc->stride[gn - 2], g_n = dc->stride[gn - 1];
+        TinyProduct p[kMaxTiny];
+        int count = 0;
+        if (da) p[count++] = TinyProduct{dc->ptr, b->ptr, da, nullptr, M, K, N, acc_da ? 1 : 0, g_m, g_n, b_n, b_k, s.K};
+        if (db) p[count++] = TinyProduct{a->ptr, dc->ptr, db, nullptr, K, N, M, acc_db ? 1 : 0, a_k, a_m, g_m, g_n, s.N};
+        const TinyColumns columns{dc->ptr, dbias, g_m, M, N, acc_dbias ? 1 : 0};
+        return launch_tiny(p, count, dbias ? &columns : nullptr, c.stream);
+    }
     const bool skinny_dx = da_wanted &&
                            ((c.flags & MNI_B200_FORCE_SKINNY_PATH) != 0 ||
                             ((c.flags & MNI_B200_FORCE_TENSOR_PATH) == 0 && s.M <= kSkinnyDxRows)) &&

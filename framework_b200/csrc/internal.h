@@ -196,6 +196,25 @@ RowsLaunch launch_rows_bt_fwd, launch_rows_bt_dx;      // W stored [N, K], seen 
 int launch_rows_dw(const float *x, int64_t ldx, const float *dy, int64_t lddy, float *dW, int64_t lddw, bool accumulate,
                    int64_t M, int64_t N, int64_t K, int sm_count, cudaStream_t stream);
 
+// Products too small for the tensor path, all of a call's in one launch (tiny.cu):
+//   c[m, n] = sum_k a[m, k] . b[k, n] (+ bias) (+ c), each operand with a unit stride in one of its dims
+struct TinyProduct {
+    const float *a, *b;
+    float *c;
+    const float *bias;
+    int M, N, K, accumulate;
+    long long a_m, a_k, b_k, b_n, ldc;
+};
+//   out[j] (+)= sum_r src[r, j]
+struct TinyColumns {
+    const float *src;
+    float *out;
+    long long ld;
+    int rows, n, accumulate;
+};
+constexpr int kMaxTiny = 2;
+int launch_tiny(const TinyProduct *products, int count, const TinyColumns *columns, cudaStream_t stream);
+
 // Pointwise / reduction helpers.
 int launch_add_bias(const float *y, const float *bias, float *out, int64_t rows, int64_t n,
                     cudaStream_t stream);

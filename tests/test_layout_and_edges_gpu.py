@@ -119,3 +119,31 @@ def test_last_wave_cut_into_units(F, m, k, n, batch, mode):
     out.check("product", fully_written=mode != "accumulate")
     want = want + bias + (c0 if mode == "accumulate" else 0)
     assert rel_fro(out.tensor.numpy(), want) <= (2e-3 if mode == "single pass" else regression_bound_3xtf32(k))
+
+
+@pytest.mark.parametrize("m,k,n", [(1, 1, 1), (9, 8, 7), (31, 33, 32), (32, 64, 32), (33, 65, 31), (64, 128, 5), (100, 300, 120),
+                                   (320, 9, 320), (192, 192, 192), (5, 100, 1000)])
+@pytest.mark.parametrize("layout", ["plain", "a transposed", "b transposed", "dc transposed"])
+def test_small_products_in_one_launch(F, m, k, n, layout):
+    """Plain f32 tiles: edges of the 32 x 32 tile and of the 8 x 8 contraction steps, every side a transposing view, bias,
+    accumulation, all three gradients in one launch."""
+    rng = _rng(6, m, k, n)
+    a, b = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((k, n)).astype(np.float32)
+    g, bias = rng.standard_normal((m, n)).astype(np.float32), rng.standard_normal(n).astype(np.float32)
+
+    def dev(x, transposed):
+        t = F.DeviceTensor.from_numpy
+        return t(np.ascontiguousarray(x.T)).permute((1, 0)) if transposed else t(x)
+    ad, bd, gd = dev(a, layout[0] == "a"), dev(b, layout[0] == "b"), dev(g, layout[0] == "d")
+    a64, b64, g64 = (x.astype(np.float64) for x in (a, b, g))
+    c0 = [rng.standard_normal(s).astype(np.float32) for s in ((m, n), (m, k), (k, n), (n,))]
+    lib = F._lib
+    for accumulate in (False, True):
+        y, da, db, dbias = (Guarded(F, c.shape, init=c if accumulate else None) for c in c0)
+        F.matmul(ad, bd, F.DeviceTensor.from_numpy(bias), out=y.tensor, flags=lib.ACCUMULATE_C if accumulate else 0)
+        F.matmul_backward(gd, ad, bd, da=da.tensor, db=db.tensor, dbias=dbias.tensor, want_dbias=True,
+                          flags=lib.ACCUMULATE_DA | lib.ACCUMULATE_DB | lib.ACCUMULATE_DBIAS if accumulate else 0)
+        F.device_status()
+        for got, want, c in zip((y, da, db, dbias), (a64 @ b64 + bias, g64 @ b64.T, a64.T @ g64, g64.sum(0)), c0):
+            got.check(fully_written=not accumulate)
+            assert rel_fro(got.tensor.numpy(), want + (c if accumulate else 0)) <= regression_bound_3xtf32(max(m, k, n))
