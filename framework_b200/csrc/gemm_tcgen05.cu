@@ -416,7 +416,7 @@ __device__ __forceinline__ WorkIter work_begin(const KParams &p, int slot, int n
 // remembers the rest.
 __device__ __forceinline__ void first_piece(const KParams &p, WorkIter &wi, TileCoord &t) {
     const int len = t.it1 - t.it0;
-    if (p.chunk_iters > 0 && len > p.chunk_iters + (p.chunk_iters >> 1)) {
+    if (p.chunk_iters > 0 && len > p.chunk_iters + (p.chunk_iters >> 3)) {
         const int pieces = (len + p.chunk_iters - 1) / p.chunk_iters;
         wi.cur = t;
         wi.piece_len = (len + pieces - 1) / pieces;
@@ -1587,6 +1587,16 @@ struct Plan {
 
 constexpr size_t kFixedSmemNoEpi = 1024 + kBarBytes;
 
+// Split tail of `tiles` 256-wide pair tiles: after at least one whole round, a last wave that fills at most half of the
+// slots, in a schedule that would idle more than a fifth of them, is cut into two to four units per tile of at least 128
+// contraction elements each.  1: no cut.
+long long cut_ways(long long tiles, long long slots, long long k) {
+    const long long full = tiles / slots, rem = tiles - full * slots;
+    const long long ways = rem > 0 ? std::min<long long>(slots / rem, 4) : 1;
+    const double eff = static_cast<double>(tiles) / static_cast<double>((full + 1) * slots);
+    return full >= 1 && ways >= 2 && eff < 0.80 && k / ways >= 128 ? ways : 1;
+}
+
 Plan make_plan(const GemmProblem &p, int sm_count) {
     Plan pl;
     pl.bn = p.N <= 64 ? 64 : (p.N <= 128 ? 128 : 256);
@@ -1621,6 +1631,29 @@ Plan make_plan(const GemmProblem &p, int sm_count) {
                 const double t = rounds * (k_eff / sp) * c_ns + (sp > 1 ? 1500.0 + (sp + 1) * out_bytes / 3000.0 : 0.0);
                 if (t < best) { best = t; pl.bn = bn; model_splits = sp; }
             }
+        }
+    }
+    // Problems of several rounds: a round costs the main loop of a tile (nanoseconds per k element) plus its own overhead,
+    // or the time to write the round's tiles where the contraction is short, half as much again if the output's rows are
+    // not 16-byte aligned.  Fitted to products of 64 .. 1024 in every dimension; it decides against 256-wide tiles where
+    // they would compute and write mostly padding (48 x [333 x 64 x 333]: 36.5 us in 256-wide pairs, 25.8 in 128-wide tiles).
+    if (bn_env == 0 && p.force_splits <= 0 && !p.fast_tf32 && p.N > 128 && tiles256 >= sm_count && env_int("MNI_B200_PLAN_MODEL", 1) != 0) {
+        const double k_us = static_cast<double>(p.K) * static_cast<double>(p.fold) * 1e-3;
+        const double unaligned = (p.ldc % 4 != 0 || p.c_bstride % 4 != 0) ? 1.45 : 1.0;
+        double best = 1e300;
+        for (int bn : {256, 128, 64}) {
+            const int cg = pair_for(bn);
+            const long long tiles = static_cast<long long>(p.batch) * ((p.M + BM * cg - 1) / (BM * cg)) * ((p.N + bn - 1) / bn);
+            const long long slots = std::max(1, sm_count / cg);
+            const double loop = k_us * (bn == 256 ? (cg == 2 ? 30.0 : 33.0) : (bn == 128 ? 19.0 : 13.0)) + (bn == 256 ? 0.5 : (bn == 128 ? 1.0 : 0.65));
+            const double write = unaligned * (bn == 256 ? (cg == 2 ? 3.7 : 4.5) : (bn == 128 ? 2.2 : 1.5));
+            double rounds = static_cast<double>((tiles + slots - 1) / slots);
+            if (bn == 256 && cg == 2) {
+                const long long ways = cut_ways(tiles, slots, p.fold * ((p.K + 15) / 16) * 16);
+                if (ways > 1) rounds += 1.0 / static_cast<double>(ways) - 0.75;
+            }
+            const double t = rounds * std::max(loop, write);
+            if (t < best) { best = t; pl.bn = bn; }
         }
     }
     pl.cg = pair_for(pl.bn);
@@ -1669,34 +1702,30 @@ Plan make_plan(const GemmProblem &p, int sm_count) {
     pl.splits = splits;
     const long long units = tiles * splits;
     pl.grid = static_cast<int>(std::min<long long>(units, slots)) * pl.cg;
-    // Balanced tail: when the last wave of whole tiles would leave more than 8 % of the slots idle, its
-    // k-blocks are dealt out evenly instead (every slot gets one contiguous range; tiles cut by a range
-    // boundary are summed in the owner's epilogue, in slot order).
+    // Balanced tail: the k-blocks of the last wave are dealt out evenly (every slot gets one contiguous range; tiles cut by
+    // a range boundary are summed in the owner's epilogue, in slot order).
     pl.sk = false;
     pl.sk_first_tile = 0;
     pl.tail_ways = pl.tail_tiles = 0;
-    // MNI_B200_STREAMK: unset = on when the whole-tile schedule would idle more than a fifth of the slot-rounds
-    // (measured: below that the idle SMs of a ragged wave are power headroom for the busy ones at the 1 kW cap
-    // and the balanced tail does not pay); 1 = on from 8 % idle; 0 = never.
+    // MNI_B200_STREAMK=1 turns it on where whole tiles would idle more than 8 % of the slot-rounds.  Off by default: parking
+    // and adding the shared tiles costs more than the idle slots at every size measured (24 x [512 x 512 x 64] 19.9 us
+    // against 12.4, 6 x 700^3 42.1 / 29.0, 3000 x 1000 x 900 45.8 / 37.7, 1000 x 2000 x 3000 63.8 / 65.4).
+    // MNI_B200_STREAMK=0 turns the split tail below off as well.
     const int sk_env = env_int("MNI_B200_STREAMK", -1);
-    // Split tail: after at least one whole round, a last wave that fills at most half of the CTA pairs is cut into two to
-    // four units per tile, whose partial tiles one small kernel adds.  2048 x 3072, K = 768 (96 tiles on 74 pairs): two
+    // The split tail's partial tiles are added by one small kernel.  2048 x 3072, K = 768 (96 tiles on 74 pairs): two
     // rounds 49.7 us, the balanced tail 51.9 (17 of it parking and adding in the last CTAs), this 41.
     if (splits == 1 && sk_env < 0 && p.force_splits <= 0 && pl.cg == 2 && pl.bn == 256) {
-        const long long full = tiles / slots, rem = tiles - full * slots;
-        const long long ways = rem > 0 ? std::min<long long>(slots / rem, 4) : 1;
-        const double eff = static_cast<double>(tiles) / static_cast<double>((full + 1) * slots);
-        if (full >= 1 && ways >= 2 && eff < 0.80 && iters / ways * pl.bk >= 128) {
+        const long long ways = cut_ways(tiles, slots, iters * pl.bk);
+        if (ways > 1) {
             pl.tail_ways = static_cast<int>(ways);
-            pl.tail_tiles = static_cast<int>(rem);
+            pl.tail_tiles = static_cast<int>(tiles % slots);
             return pl;
         }
     }
-    if (splits == 1 && p.D == nullptr && sk_env != 0) {
+    if (splits == 1 && p.D == nullptr && sk_env > 0) {
         const long long full_rounds = tiles / slots, rem = tiles - full_rounds * slots;
         const double eff = static_cast<double>(tiles) / static_cast<double>((full_rounds + 1) * slots);
-        const double eff_limit = sk_env > 0 ? 0.92 : 0.80;
-        if (rem > 0 && eff < eff_limit && iters >= 8 && tiles * 2 > slots) {
+        if (rem > 0 && eff < 0.92 && iters >= 8 && tiles * 2 > slots) {
             // the tail takes one whole round along when there is one, so that a range is at least a tile long
             const long long whole = full_rounds > 0 ? full_rounds - 1 : 0;
             const long long range = (tiles - whole * slots) * iters / slots;
@@ -1854,7 +1883,7 @@ std::string gemm_tc_describe(const GemmProblem &p0, int sm_count) {
     const long long iters = p.fold * ((p.K + pl.bk - 1) / pl.bk);
     const long long len = (iters + pl.splits - 1) / pl.splits;
     const long long ci = (chunk_k > 0 && p.D == nullptr) ? std::max(1, chunk_k / pl.bk) : 0;
-    const int pieces = (ci > 0 && len > ci + ci / 2) ? static_cast<int>((len + ci - 1) / ci) : 1;
+    const int pieces = (ci > 0 && len > ci + ci / 8) ? static_cast<int>((len + ci - 1) / ci) : 1;
     char buf[320];
     snprintf(buf, sizeof(buf),
              "tensor m=%lld n=%lld k=%lld batch=%lld fold=%lld bn=%d bk=%d pair=%d tmem_a=%d stages=%d splits=%d "
@@ -2045,7 +2074,7 @@ int launch_gemm_tc(const GemmProblem &p0, float *partial, uint32_t *err_word, in
     // rule decides what is cut).
     const long long unit_len = (static_cast<long long>(k.fold) * k.kiters + pl.splits - 1) / pl.splits;
     const bool running = pl.cg == 2 && pl.bn == 256 && pl.bk == (p.fast_tf32 ? 32 : 16) && !pl.sk && !pl.tail_ways && k.chunk_iters > 0 &&
-                         unit_len > k.chunk_iters + (k.chunk_iters >> 1) && (k.epi_mode == kEpiTmaStore || k.epi_mode == kEpiTmaReduce);
+                         unit_len > k.chunk_iters + (k.chunk_iters >> 3) && (k.epi_mode == kEpiTmaStore || k.epi_mode == kEpiTmaReduce);
     cudaError_t e = cudaErrorInvalidValue;
     if (pl.sk) {
         if (pl.ta && pl.bn == 64 && split_groups == 2) e = launch_variant<64, 32, false, 8, 1, true, kBalanced, 2>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
