@@ -699,22 +699,47 @@ int bwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const mni_
     const bool side_on = env_flag("MNI_B200_BWD_OVERLAP", 1);
     const bool two_tensor = da_wanted && db_wanted && !streamed_dx && !streamed_dw;
     const bool small = work > 0 && work <= overlap_work_limit();
-    bool pairable = false;
+    bool pairable = false, beside = small;
     if (side_on && two_tensor) {
         int64_t oa[MNI_B200_MAX_DIMS], ob[MNI_B200_MAX_DIMS];
         bool same;
         const int na = broadcast_shape(dc->shape, gn - 2, b->shape, b->ndim - 2, oa);
         const int nb = broadcast_shape(a->shape, a->ndim - 2, dc->shape, gn - 2, ob);
         pairable = na >= 0 && nb >= 0 && single_product(oa, na, *a, &same) && single_product(ob, nb, *b, &same);
+        if (pairable && !small) {
+            // Larger products go side by side where the cost model says so by a margin: where one of them, or both, would
+            // leave SMs idle on its own or need a split of the contraction to fill them (2048 x 3072 x 768: 97.6 -> 81.4 us).
+            auto estimate = [&](int64_t rows, int64_t cols, int64_t k, const int64_t *batch_dims, int nd, const mni_b200_view &target,
+                                float *out, int share) {
+                bool is_same;
+                single_product(batch_dims, nd, target, &is_same);
+                const int64_t count = prod(batch_dims, nd);
+                GemmProblem p;
+                p.M = rows; p.N = cols; p.K = k;
+                p.batch = is_same ? count : 1;
+                p.fold = is_same ? 1 : count;
+                p.C = out; p.ldc = cols; p.c_bstride = rows * cols;
+                p.fast_tf32 = (c.flags & MNI_B200_PRECISION_TF32) != 0;
+                p.force_splits = static_cast<int>((c.flags >> 16) & 0xffu);
+                c.sm_share = share;
+                const double us = gemm_tc_estimate_us(p, c.gemm_sms());
+                c.sm_share = 1;
+                return us;
+            };
+            auto of_da = [&](int share) { return estimate(s.M, s.K, s.N, oa, na, *a, da, share); };
+            auto of_db = [&](int share) { return estimate(s.K, s.N, s.M, ob, nb, *b, db, share); };
+            const double whole_a = of_da(1), whole_b = of_db(1), half_a = of_da(2), half_b = of_db(2);
+            beside = whole_a > 0 && whole_b > 0 && half_a > 0 && half_b > 0 && std::max(half_a, half_b) < 0.92 * (whole_a + whole_b);
+        }
     }
     const int pair_env = env_int("MNI_B200_BWD_PAIR", -1);
-    const bool pair = pairable && (pair_env > 0 || (pair_env < 0 && small && !c.capturing));
-    const bool overlap = side_on && !pair && da && db && a_elems > 0 && b_elems > 0 && small;
+    const bool pair = pairable && (pair_env > 0 || (pair_env < 0 && beside && !c.capturing));
+    const bool overlap = side_on && !pair && da && db && a_elems > 0 && b_elems > 0 && beside;
     const bool side_dbias = side_on && dbias && (da || db) && work > 0;
     // Two tensor-core products side by side: each persistent grid is planned for half of the SMs, so that both are
     // resident at once instead of the second queueing behind the first's CTAs (measured under graph replay: 512^3
     // 29.2 -> 24.6 us per step, 1024^3 55.3 -> 45.3 us).
-    const bool share_sms = (overlap || pair) && small && two_tensor && env_flag("MNI_B200_BWD_SHARE_SMS", 1);
+    const bool share_sms = (overlap || pair) && beside && two_tensor && env_flag("MNI_B200_BWD_SHARE_SMS", 1);
     if (share_sms) c.sm_share = 2;
     cudaStream_t const main_stream = c.stream;
     // Operands of the tensor path that have to be gathered: once each, before the streams part.
@@ -866,8 +891,9 @@ int bwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const mni_
         }
     }
     if (!c.dry()) {
-        if (finish_a.splits) rc = launch_gemm_finish(finish_a, c.stream);
-        if (rc == MNI_B200_OK && finish_b.splits) rc = launch_gemm_finish(finish_b, c.stream);
+        const bool both = finish_a.splits && finish_b.splits;
+        if (finish_a.splits) rc = launch_gemm_finish(finish_a, both ? 1 : 0, c.stream);
+        if (rc == MNI_B200_OK && finish_b.splits) rc = launch_gemm_finish(finish_b, both ? 2 : 0, c.stream);
     }
     return rc;
 }

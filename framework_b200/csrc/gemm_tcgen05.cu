@@ -41,6 +41,7 @@
 // Every wait on an mbarrier or flag is bounded: after KParams::wait_cycles clock cycles (~2 s unless a
 // test shortens it) the waiter records a code in a global error word, raises a CTA-wide abort flag and
 // all roles drain to the common exit, where TMEM is released.  Nothing traps.
+#include "activation.h"
 #include "internal.h"
 
 #include <stdio.h>
@@ -326,12 +327,6 @@ __device__ __forceinline__ void tmem_ld16_issue(uint32_t taddr, uint32_t (&v)[16
 }
 __device__ __forceinline__ void tmem_ld_wait() {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-// gelu(v) = 0.5 v (1 + tanh(sqrt(2/pi) (v + 0.044715 v^3)))   (kernels/fused_ops.cu:66-82)
-__device__ __forceinline__ float gelu_tanh_f(float v) {
-    const float inner = 0.7978845608028654f * (v + 0.044715f * v * v * v);
-    return 0.5f * v * (1.0f + tanhf(inner));
 }
 
 struct TileCoord {
@@ -876,7 +871,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     }
                     if (do_act) {
 #pragma unroll
-                        for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(gelu_tanh_f(__uint_as_float(v[j])));
+                        for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(gelu_tanh(__uint_as_float(v[j])));
                         emit(&tmD, false);
                     } else if (part) {
                         emit(&tmP, add_piece);
@@ -1280,22 +1275,31 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     if (p.dep_mode == 2 && threadIdx.x == 0) grid_dependency_wait();
 }
 
+// Divisors of the finish kernel: multiply-high and shift below 2^31 items, plain 64-bit beyond.
+__device__ __forceinline__ uint32_t divisor(const FastDiv &f) { return f.d; }
+__device__ __forceinline__ long long divisor(long long d) { return d; }
+__device__ __forceinline__ unsigned divide(unsigned n, const FastDiv &f) { return static_cast<unsigned>(fd_div(static_cast<int>(n), f)); }
+__device__ __forceinline__ long long divide(long long n, long long d) { return n / d; }
 // Deterministic split-K finish: C = sum_s partial[s] (+ bias) (+ C), splits added in ascending order.
 // One thread per 16-byte vector of the partials (rows of `pld` floats); the partials of four splits are in flight at a
 // time.  VEC: the output's rows are whole aligned vectors too.  Otherwise (an odd width) a warp turns its 128
 // columns through shared memory, so that its stores cover 32 neighbouring elements.
-template <bool VEC, typename I>
+// dep_mode 1 / 2: first / second of two finishes launched back to back that need nothing from each other; the second starts
+// once every block of the first has seen the products complete, and waits for the first only before it ends (as the pair of
+// products does; a backward of 1000 x 333 x 777: 5 us less than one after the other).
+template <bool VEC, typename I, typename D>
 __global__ void __launch_bounds__(256)
 splitk_reduce_kernel(const float *__restrict__ partial, float *__restrict__ C, long long ldc, long long c_bstride,
-                     const float *__restrict__ bias, int accumulate, int splits, long long rows, int M, int N, int pld) {
+                     const float *__restrict__ bias, int accumulate, int splits, long long rows, D rows_per_batch, D vectors,
+                     int M, int N, int dep_mode) {
     __shared__ float turn[VEC ? 1 : 256 * 4];
-    grid_dependency_trigger();
-    grid_dependency_wait();                      // the partials come from the grid before this one
-    const I per_row = static_cast<I>(pld / 4);
+    if (dep_mode != 1) grid_dependency_trigger();
+    if (dep_mode != 2) grid_dependency_wait();   // the partials come from the grids before this one
+    if (dep_mode == 1) grid_dependency_trigger();
+    const I per_row = static_cast<I>(divisor(vectors));
     const I items = static_cast<I>(rows) * per_row;
     const I item = static_cast<I>(blockIdx.x) * 256 + threadIdx.x;
-    if (VEC && item >= items) return;
-    const long long slab = rows * pld;
+    const long long slab = rows * per_row;       // in vectors
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     if (item < items) {
         const float4 *src = reinterpret_cast<const float4 *>(partial) + item;
@@ -1303,52 +1307,55 @@ splitk_reduce_kernel(const float *__restrict__ partial, float *__restrict__ C, l
         for (; sp + 4 <= splits; sp += 4) {
             float4 t[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) t[u] = __ldcg(src + (sp + u) * (slab / 4));
+            for (int u = 0; u < 4; ++u) t[u] = __ldcg(src + (sp + u) * slab);
 #pragma unroll
             for (int u = 0; u < 4; ++u) { acc.x += t[u].x; acc.y += t[u].y; acc.z += t[u].z; acc.w += t[u].w; }
         }
         for (; sp < splits; ++sp) {
-            const float4 t = __ldcg(src + sp * (slab / 4));
+            const float4 t = __ldcg(src + sp * slab);
             acc.x += t.x; acc.y += t.y; acc.z += t.z; acc.w += t.w;
         }
     }
     if (VEC) {
-        const I row = item / per_row;
-        const int col = static_cast<int>(item - row * per_row) * 4;
-        const I bt = row / static_cast<I>(M);
-        const int m = static_cast<int>(row - bt * static_cast<I>(M));
-        if (bias) {
-            const float4 b = __ldg(reinterpret_cast<const float4 *>(bias + col));
-            acc.x += b.x; acc.y += b.y; acc.z += b.z; acc.w += b.w;
+        if (item < items) {
+            const I row = divide(item, vectors);
+            const int col = static_cast<int>(item - row * per_row) * 4;
+            const I bt = divide(row, rows_per_batch);
+            const int m = static_cast<int>(row - bt * static_cast<I>(M));
+            if (bias) {
+                const float4 b = __ldg(reinterpret_cast<const float4 *>(bias + col));
+                acc.x += b.x; acc.y += b.y; acc.z += b.z; acc.w += b.w;
+            }
+            float4 *out = reinterpret_cast<float4 *>(C + static_cast<long long>(bt) * c_bstride + static_cast<long long>(m) * ldc + col);
+            if (accumulate) {
+                const float4 c0 = *out;
+                acc.x += c0.x; acc.y += c0.y; acc.z += c0.z; acc.w += c0.w;
+            }
+            *out = acc;
         }
-        float4 *out = reinterpret_cast<float4 *>(C + static_cast<long long>(bt) * c_bstride + static_cast<long long>(m) * ldc + col);
-        if (accumulate) {
-            const float4 c0 = *out;
-            acc.x += c0.x; acc.y += c0.y; acc.z += c0.z; acc.w += c0.w;
-        }
-        *out = acc;
-        return;
-    }
-    const int lane = threadIdx.x & 31;
-    float *mine = turn + (threadIdx.x & ~31) * 4;
-    reinterpret_cast<float4 *>(mine)[lane] = acc;
-    __syncwarp();
+    } else {
+        const int lane = threadIdx.x & 31;
+        float *mine = turn + (threadIdx.x & ~31) * 4;
+        reinterpret_cast<float4 *>(mine)[lane] = acc;
+        __syncwarp();
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        const int e = j * 32 + lane;                           // element within the warp's 128
-        const I at = (item - lane) + e / 4;                    // its vector
-        if (at >= items) continue;
-        const I row = at / per_row;
-        const int col = static_cast<int>(at - row * per_row) * 4 + (e & 3);
-        if (col >= N) continue;
-        const I bt = row / static_cast<I>(M);
-        const int m = static_cast<int>(row - bt * static_cast<I>(M));
-        float *out = C + static_cast<long long>(bt) * c_bstride + static_cast<long long>(m) * ldc + col;
-        float y = mine[e];
-        if (bias) y += __ldg(bias + col);
-        if (accumulate) y += *out;
-        *out = y;
+        for (int j = 0; j < 4; ++j) {
+            const int e = j * 32 + lane;                           // element within the warp's 128
+            const I at = (item - lane) + e / 4;                    // its vector
+            if (at >= items) continue;
+            const I row = divide(at, vectors);
+            const int col = static_cast<int>(at - row * per_row) * 4 + (e & 3);
+            if (col >= N) continue;
+            const I bt = divide(row, rows_per_batch);
+            const int m = static_cast<int>(row - bt * static_cast<I>(M));
+            float *out = C + static_cast<long long>(bt) * c_bstride + static_cast<long long>(m) * ldc + col;
+            float y = mine[e];
+            if (bias) y += __ldg(bias + col);
+            if (accumulate) y += *out;
+            *out = y;
+        }
     }
+    if (dep_mode == 2) grid_dependency_wait();
 }
 
 // Finish of a split tail: adds the `tail_ways` partial tiles of each of the last wave's tiles in ascending order and runs
@@ -1391,7 +1398,7 @@ tail_finish_kernel(const float *__restrict__ partial, float *__restrict__ D, int
         float4 *out = reinterpret_cast<float4 *>((D ? D : p.C) + at + col);
         if (D) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) v[e] = gelu_tanh_f(v[e]);
+            for (int e = 0; e < 4; ++e) v[e] = gelu_tanh(v[e]);
         } else if (p.accumulate) {
             const float4 c0 = *out;
             v[0] += c0.x; v[1] += c0.y; v[2] += c0.z; v[3] += c0.w;
@@ -1413,7 +1420,7 @@ tail_finish_kernel(const float *__restrict__ partial, float *__restrict__ D, int
         if (D && p.C) p.C[at + cc] = y;
         if (p.bias) y += __ldg(p.bias + cc);
         float *out = (D ? D : p.C) + at + cc;
-        if (D) y = gelu_tanh_f(y);
+        if (D) y = gelu_tanh(y);
         else if (p.accumulate) y += *out;
         *out = y;
     }
@@ -1581,6 +1588,7 @@ struct Plan {
     bool ta;                                                  // A operand of the MMAs from tensor memory
     bool sk;                                                  // balanced tail: the last, ragged wave is cut by k-blocks
     int sk_first_tile;
+    double est_us;                                            // the cost model's time for this plan (0: it has none)
     int tail_ways, tail_tiles;                                // split tail: the last wave's tiles, cut into this many units each (0: none)
     size_t smem;
 };
@@ -1611,6 +1619,8 @@ Plan make_plan(const GemmProblem &p, int sm_count) {
     // nanoseconds per k element of one tile (30 / 33 for a 256-wide pair / lone CTA, 15.4 for 128, 13.5
     // for 64), 1.5 us for the reduce launch and its traffic at 3 TB/s.
     int model_splits = 0;
+    pl.est_us = 0.0;
+    constexpr double kFixedUs = 5.0;                          // launch, pipeline fill, last epilogue
     const long long tiles256 = static_cast<long long>(p.batch) * ((p.M + BM - 1) / BM) * ((p.N + 255) / 256);
     if (bn_env == 0 && p.force_splits <= 0 && tiles256 < sm_count && env_int("MNI_B200_PLAN_MODEL", 1) != 0) {
         const double k_eff = static_cast<double>(p.K) * static_cast<double>(p.fold);
@@ -1632,6 +1642,7 @@ Plan make_plan(const GemmProblem &p, int sm_count) {
                 if (t < best) { best = t; pl.bn = bn; model_splits = sp; }
             }
         }
+        pl.est_us = best * 1e-3 + kFixedUs;
     }
     // Problems of several rounds: a round costs the main loop of a tile (nanoseconds per k element) plus its own overhead,
     // or the time to write the round's tiles where the contraction is short, half as much again if the output's rows are
@@ -1655,6 +1666,7 @@ Plan make_plan(const GemmProblem &p, int sm_count) {
             const double t = rounds * std::max(loop, write);
             if (t < best) { best = t; pl.bn = bn; }
         }
+        pl.est_us = best + kFixedUs;
     }
     pl.cg = pair_for(pl.bn);
     pl.bk = (pl.bn == 256 && !p.fast_tf32) ? 16 : 32;
@@ -1874,6 +1886,11 @@ size_t gemm_tc_partial_bytes(const GemmProblem &p0, int sm_count) {
     return static_cast<size_t>(pl.splits) * p.batch * p0.M * partial_pitch(p0.N) * sizeof(float);
 }
 
+double gemm_tc_estimate_us(const GemmProblem &p, int sm_count) {
+    bool transposed = false;
+    return p.fast_tf32 ? 0.0 : make_plan(kernel_view(p, &transposed), sm_count).est_us;
+}
+
 std::string gemm_tc_describe(const GemmProblem &p0, int sm_count) {
     bool transposed = false;
     const GemmProblem p = kernel_view(p0, &transposed);
@@ -1895,7 +1912,7 @@ std::string gemm_tc_describe(const GemmProblem &p0, int sm_count) {
     return buf;
 }
 
-int launch_gemm_finish(const GemmFinish &f, cudaStream_t stream) {
+int launch_gemm_finish(const GemmFinish &f, int dep_mode, cudaStream_t stream) {
     const long long rows = static_cast<long long>(f.batch) * f.M;
     const int64_t pld = partial_pitch(f.N);
     const bool vec = f.N % 4 == 0 && f.ldc % 4 == 0 && f.c_bstride % 4 == 0 &&
@@ -1903,11 +1920,17 @@ int launch_gemm_finish(const GemmFinish &f, cudaStream_t stream) {
     const long long items = rows * (pld / 4);
     const unsigned blocks = static_cast<unsigned>((items + 255) / 256);
     const bool small = items < (1LL << 31) - 256;
-    auto reduce = vec ? (small ? splitk_reduce_kernel<true, unsigned> : splitk_reduce_kernel<true, long long>)
-                      : (small ? splitk_reduce_kernel<false, unsigned> : splitk_reduce_kernel<false, long long>);
-    const cudaError_t e = launch_dependent(reduce, dim3(blocks), dim3(256), 0, stream, f.partial, f.C, f.ldc, f.c_bstride, f.bias,
-                                           f.accumulate ? 1 : 0, f.splits, rows, static_cast<int>(f.M), static_cast<int>(f.N),
-                                           static_cast<int>(pld));
+    const int acc = f.accumulate ? 1 : 0, m = static_cast<int>(f.M), n = static_cast<int>(f.N);
+    cudaError_t e;
+    if (small) {
+        auto reduce = vec ? splitk_reduce_kernel<true, unsigned, FastDiv> : splitk_reduce_kernel<false, unsigned, FastDiv>;
+        e = launch_dependent(reduce, dim3(blocks), dim3(256), 0, stream, f.partial, f.C, f.ldc, f.c_bstride, f.bias, acc, f.splits,
+                             rows, make_fastdiv(f.M), make_fastdiv(pld / 4), m, n, dep_mode);
+    } else {
+        auto reduce = vec ? splitk_reduce_kernel<true, long long, long long> : splitk_reduce_kernel<false, long long, long long>;
+        e = launch_dependent(reduce, dim3(blocks), dim3(256), 0, stream, f.partial, f.C, f.ldc, f.c_bstride, f.bias, acc, f.splits,
+                             rows, f.M, pld / 4, m, n, dep_mode);
+    }
     if (e != cudaSuccess) return fail(MNI_B200_ERR_CUDA, "splitk_reduce_kernel launch failed: %s", cudaGetErrorString(e));
     MNI_LAUNCH_CHECK("splitk_reduce_kernel");
     return MNI_B200_OK;
@@ -2128,7 +2151,7 @@ int launch_gemm_tc(const GemmProblem &p0, float *partial, uint32_t *err_word, in
     if (pl.splits > 1) {
         const GemmFinish f{partial, p.C, p.ldc, p.c_bstride, p.batch, oM, oN, p.bias, p.accumulate, pl.splits};
         if (defer) *defer = f;
-        else return launch_gemm_finish(f, stream);
+        else return launch_gemm_finish(f, 0, stream);
     }
     return MNI_B200_OK;
 }

@@ -158,7 +158,10 @@ struct GemmFinish {
 };
 int launch_gemm_tc(const GemmProblem &p, float *partial, uint32_t *err_word, int sm_count,
                    cudaStream_t stream, GemmFinish *defer = nullptr);
-int launch_gemm_finish(const GemmFinish &f, cudaStream_t stream);
+// dep_mode 1 / 2: first / second of two finishes that do not depend on each other, launched back to back
+int launch_gemm_finish(const GemmFinish &f, int dep_mode, cudaStream_t stream);
+// The plan's cost model for this problem in microseconds (0: the model does not cover it).
+double gemm_tc_estimate_us(const GemmProblem &p, int sm_count);
 // One line of text naming the kernel variant, tiling, split and grid launch_gemm_tc would use for this problem
 // on a device with `sm_count` SMs.  Pure host arithmetic: touches no device.
 std::string gemm_tc_describe(const GemmProblem &p, int sm_count);

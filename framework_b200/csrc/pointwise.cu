@@ -1,4 +1,5 @@
 // HBM-bound helpers around the GEMM: bias add, column sums (dbias), bias + GELU, device-side unbroadcast.
+#include "activation.h"
 #include "internal.h"
 
 #include <algorithm>
@@ -138,20 +139,6 @@ colsum_kernel(const float *__restrict__ dy, long long ld, float *__restrict__ co
 }
 
 // ---- bias + GELU (tanh form), the fused pointwise op that follows the MLP up-projection --------
-// gelu(v) = 0.5 v (1 + tanh(sqrt(2/pi) (v + 0.044715 v^3))), v = x + bias   (kernels/fused_ops.cu:66-82)
-__device__ __forceinline__ float gelu_tanh(float v) {
-    const float inner = 0.7978845608028654f * (v + 0.044715f * v * v * v);
-    return 0.5f * v * (1.0f + tanhf(inner));
-}
-// d gelu / d v                                                             (kernels/fused_ops.cu:96-103)
-__device__ __forceinline__ float gelu_tanh_grad(float v) {
-    const float inner = 0.7978845608028654f * (v + 0.044715f * v * v * v);
-    const float th = tanhf(inner);
-    const float sech2 = 1.0f - th * th;
-    const float d_inner = 0.7978845608028654f * (1.0f + 3.0f * 0.044715f * v * v);
-    return 0.5f * (1.0f + th) + 0.5f * v * sech2 * d_inner;
-}
-
 // out[r, j] = f(y[r, j] + bias[j]), f the identity or GELU.  The tensor is one flat run, so four consecutive elements are
 // a unit whatever n is; only the bias index wraps.  QUADS: the pointers allow 16-byte units (else an element each);
 // ALIGNED: a unit's bias values are one aligned 16-byte load too.  `units` per launch stays below 2^31.
