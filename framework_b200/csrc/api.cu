@@ -699,18 +699,16 @@ int bwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const mni_
     const bool side_on = env_flag("MNI_B200_BWD_OVERLAP", 1);
     const bool two_tensor = da_wanted && db_wanted && !streamed_dx && !streamed_dw;
     const bool small = work > 0 && work <= overlap_work_limit();
-    bool pairable = false, beside = small;
+    bool pairable = false, beside = small, b_first = false;
     if (side_on && two_tensor) {
         int64_t oa[MNI_B200_MAX_DIMS], ob[MNI_B200_MAX_DIMS];
         bool same;
         const int na = broadcast_shape(dc->shape, gn - 2, b->shape, b->ndim - 2, oa);
         const int nb = broadcast_shape(a->shape, a->ndim - 2, dc->shape, gn - 2, ob);
         pairable = na >= 0 && nb >= 0 && single_product(oa, na, *a, &same) && single_product(ob, nb, *b, &same);
-        if (pairable && !small) {
-            // Larger products go side by side where the cost model says so by a margin: where one of them, or both, would
-            // leave SMs idle on its own or need a split of the contraction to fill them (2048 x 3072 x 768: 97.6 -> 81.4 us).
-            auto estimate = [&](int64_t rows, int64_t cols, int64_t k, const int64_t *batch_dims, int nd, const mni_b200_view &target,
-                                float *out, int share) {
+        if (pairable) {
+            auto problem = [&](int64_t rows, int64_t cols, int64_t k, const int64_t *batch_dims, int nd, const mni_b200_view &target,
+                               float *out) {
                 bool is_same;
                 single_product(batch_dims, nd, target, &is_same);
                 const int64_t count = prod(batch_dims, nd);
@@ -721,15 +719,23 @@ int bwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const mni_
                 p.C = out; p.ldc = cols; p.c_bstride = rows * cols;
                 p.fast_tf32 = (c.flags & MNI_B200_PRECISION_TF32) != 0;
                 p.force_splits = static_cast<int>((c.flags >> 16) & 0xffu);
-                c.sm_share = share;
-                const double us = gemm_tc_estimate_us(p, c.gemm_sms());
-                c.sm_share = 1;
-                return us;
+                return p;
             };
-            auto of_da = [&](int share) { return estimate(s.M, s.K, s.N, oa, na, *a, da, share); };
-            auto of_db = [&](int share) { return estimate(s.K, s.N, s.M, ob, nb, *b, db, share); };
-            const double whole_a = of_da(1), whole_b = of_db(1), half_a = of_da(2), half_b = of_db(2);
-            beside = whole_a > 0 && whole_b > 0 && half_a > 0 && half_b > 0 && std::max(half_a, half_b) < 0.92 * (whole_a + whole_b);
+            const GemmProblem pa = problem(s.M, s.K, s.N, oa, na, *a, da), pb = problem(s.K, s.N, s.M, ob, nb, *b, db);
+            const int all = c.gemm_sms();
+            c.sm_share = 2;
+            const int half = c.gemm_sms();
+            c.sm_share = 1;
+            if (!small) {
+                // Larger products go side by side where the cost model says so by a margin: where one of them, or both, would
+                // leave SMs idle on its own or need a split of the contraction to fill them (2048 x 3072 x 768: 97.6 -> 81.4 us).
+                const double whole_a = gemm_tc_estimate_us(pa, all), whole_b = gemm_tc_estimate_us(pb, all);
+                const double half_a = gemm_tc_estimate_us(pa, half), half_b = gemm_tc_estimate_us(pb, half);
+                beside = whole_a > 0 && whole_b > 0 && half_a > 0 && half_b > 0 && std::max(half_a, half_b) < 0.9 * (whole_a + whole_b);
+            }
+            // CTA pairs take both SMs of a unit, lone CTAs are dealt out one to a unit: launched first, these would leave
+            // the pairs hardly a whole unit until they end (16 rows x 4096^2, grad_b in pairs after grad_a: 47 us against 37).
+            b_first = beside && !gemm_tc_uses_pairs(pa, half) && gemm_tc_uses_pairs(pb, half);
         }
     }
     const int pair_env = env_int("MNI_B200_BWD_PAIR", -1);
@@ -810,10 +816,21 @@ int bwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const mni_
 
     c.stream = main_stream;
 
-    GemmFinish finish_a, finish_b;     // of a pair: launched after both products
+    GemmFinish finish[2];              // of a pair: launched after both products
+    // What the first (0) or second (1) product issued is launched with: an independent pair on one stream, or the second
+    // on the side stream.
+    auto place = [&](int at) {
+        c.dep_mode = pair ? at + 1 : 0;
+        c.defer = pair ? &finish[at] : nullptr;
+        if (at == 1 && overlap && !c.dry()) c.stream = c.st->side;
+        c.flag_bank = at == 1 && (overlap || pair) ? 1 : 0;
+    };
+
     // grad_a = unbroadcast(dc . b^T, a.shape)   (ops/matmul.rs:231-240)
-    c.label = "grad_a: ";
-    if (da && a_elems > 0) {
+    auto grad_a = [&](int at) -> int {
+        c.label = "grad_a: ";
+        place(at);
+        if (!da || a_elems == 0) return MNI_B200_OK;
         if (!da_wanted) {
             rc = zero_or_bias_fill(c, da, a_elems, 1, nullptr, acc_da);
             if (rc) return rc;
@@ -843,19 +860,17 @@ int bwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const mni_
             if (rc) return rc;
             X.batch = g_batch;
             Y.batch = s.b_batch;
-            c.dep_mode = pair ? 1 : 0;
-            c.defer = pair ? &finish_a : nullptr;
             rc = grad_gemm(c, X, Y, s.M, s.K, s.N, ob, onb, *a_given, da, acc_da);
-            c.dep_mode = 0;
             if (rc) return rc;
         }
-    }
+        return MNI_B200_OK;
+    };
 
     // grad_b = unbroadcast(a^T . dc, b.shape)   (ops/matmul.rs:242-251)
-    if (overlap) { if (!c.dry()) c.stream = c.st->side; c.flag_bank = 1; }
-    c.defer = nullptr;
-    c.label = "grad_b: ";
-    if (db && b_elems > 0) {
+    auto grad_b = [&](int at) -> int {
+        c.label = "grad_b: ";
+        place(at);
+        if (!db || b_elems == 0) return MNI_B200_OK;
         if (!db_wanted) {
             rc = zero_or_bias_fill(c, db, b_elems, 1, nullptr, acc_db);
             if (rc) return rc;
@@ -884,17 +899,17 @@ int bwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const mni_
             if (rc) return rc;
             X.batch = s.a_batch;
             Y.batch = g_batch;
-            if (pair) { c.dep_mode = 2; c.flag_bank = 1; c.defer = &finish_b; }
             rc = grad_gemm(c, X, Y, s.K, s.N, s.M, ob, onb, *b_given, db, acc_db);
-            c.dep_mode = 0;
             if (rc) return rc;
         }
-    }
-    if (!c.dry()) {
-        const bool both = finish_a.splits && finish_b.splits;
-        if (finish_a.splits) rc = launch_gemm_finish(finish_a, both ? 1 : 0, c.stream);
-        if (rc == MNI_B200_OK && finish_b.splits) rc = launch_gemm_finish(finish_b, both ? 2 : 0, c.stream);
-    }
+        return MNI_B200_OK;
+    };
+    rc = b_first ? grad_b(0) : grad_a(0);
+    if (rc == MNI_B200_OK) rc = b_first ? grad_a(1) : grad_b(1);
+    c.dep_mode = 0;
+    const bool both = finish[0] && finish[1];
+    if (rc == MNI_B200_OK && finish[0]) rc = finish[0](both ? 1 : 0, c.stream);
+    if (rc == MNI_B200_OK && finish[1]) rc = finish[1](both ? 2 : 0, c.stream);
     return rc;
 }
 

@@ -1363,14 +1363,19 @@ splitk_reduce_kernel(const float *__restrict__ partial, float *__restrict__ C, l
 // tiles); a row of the tile is 64 vectors, two warps.
 template <bool VEC>
 __global__ void __launch_bounds__(256)
-tail_finish_kernel(const float *__restrict__ partial, float *__restrict__ D, int bn, int tile_rows,
+tail_finish_kernel(const float *__restrict__ partial, float *__restrict__ D, int bn, int tile_rows, int dep_mode,
                    const __grid_constant__ KParams p) {
     __shared__ float turn[VEC ? 1 : 256 * 4];
-    grid_dependency_trigger();
+    if (dep_mode != 1) grid_dependency_trigger();
     const TileCoord t = decode_unit<kCutTiles>(p, p.tail_unit + static_cast<int>(blockIdx.y) * p.tail_ways);
     const int r = static_cast<int>(blockIdx.x) * 4 + (threadIdx.x >> 6), c4 = threadIdx.x & 63;
     const int row = t.tm * tile_rows + r, col = t.tn * bn + c4 * 4;
-    grid_dependency_wait();                      // the partials come from the grid before this one
+    if (dep_mode != 2) grid_dependency_wait();   // the partials come from the grids before this one
+    if (dep_mode == 1) grid_dependency_trigger();
+    struct AtEnd {                               // dep_mode 2: see splitk_reduce_kernel
+        bool wait;
+        __device__ ~AtEnd() { if (wait) grid_dependency_wait(); }
+    } at_end{dep_mode == 2};
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     if (row < p.M && col < p.N) {
         const float4 *src = reinterpret_cast<const float4 *>(partial) +
@@ -1886,6 +1891,11 @@ size_t gemm_tc_partial_bytes(const GemmProblem &p0, int sm_count) {
     return static_cast<size_t>(pl.splits) * p.batch * p0.M * partial_pitch(p0.N) * sizeof(float);
 }
 
+bool gemm_tc_uses_pairs(const GemmProblem &p, int sm_count) {
+    bool transposed = false;
+    return make_plan(kernel_view(p, &transposed), sm_count).cg == 2;
+}
+
 double gemm_tc_estimate_us(const GemmProblem &p, int sm_count) {
     bool transposed = false;
     return p.fast_tf32 ? 0.0 : make_plan(kernel_view(p, &transposed), sm_count).est_us;
@@ -1912,7 +1922,16 @@ std::string gemm_tc_describe(const GemmProblem &p0, int sm_count) {
     return buf;
 }
 
-int launch_gemm_finish(const GemmFinish &f, int dep_mode, cudaStream_t stream) {
+namespace {
+struct SplitFinish {
+    const float *partial;
+    float *C;
+    int64_t ldc, c_bstride, batch, M, N;
+    const float *bias;
+    bool accumulate;
+    int splits;
+};
+int launch_split_finish(const SplitFinish &f, int dep_mode, cudaStream_t stream) {
     const long long rows = static_cast<long long>(f.batch) * f.M;
     const int64_t pld = partial_pitch(f.N);
     const bool vec = f.N % 4 == 0 && f.ldc % 4 == 0 && f.c_bstride % 4 == 0 &&
@@ -1935,6 +1954,17 @@ int launch_gemm_finish(const GemmFinish &f, int dep_mode, cudaStream_t stream) {
     MNI_LAUNCH_CHECK("splitk_reduce_kernel");
     return MNI_B200_OK;
 }
+int launch_tail_finish(const GemmProblem &p, const Plan &pl, const KParams &k, const float *partial, int dep_mode, cudaStream_t stream) {
+    const bool vec = p.N % 4 == 0 && p.ldc % 4 == 0 && p.c_bstride % 4 == 0 &&
+                     ((reinterpret_cast<uintptr_t>(p.C) | reinterpret_cast<uintptr_t>(p.D)) & 15) == 0;
+    const dim3 grid(static_cast<unsigned>(BM * pl.cg / 4), static_cast<unsigned>(pl.tail_tiles));
+    const cudaError_t e = launch_dependent(vec ? tail_finish_kernel<true> : tail_finish_kernel<false>, grid, dim3(256), 0, stream,
+                                           partial, p.D, pl.bn, BM * pl.cg, dep_mode, k);
+    if (e != cudaSuccess) return fail(MNI_B200_ERR_CUDA, "tail_finish_kernel launch failed: %s", cudaGetErrorString(e));
+    MNI_LAUNCH_CHECK("tail_finish_kernel");
+    return MNI_B200_OK;
+}
+}  // namespace
 
 int launch_gemm_tc(const GemmProblem &p0, float *partial, uint32_t *err_word, int sm_count,
                    cudaStream_t stream, GemmFinish *defer) {
@@ -2139,19 +2169,14 @@ int launch_gemm_tc(const GemmProblem &p0, float *partial, uint32_t *err_word, in
 #undef MNI_VARIANT
     if (e != cudaSuccess) return fail(MNI_B200_ERR_CUDA, "gemm_tc_kernel set-up failed: %s", cudaGetErrorString(e));
     MNI_LAUNCH_CHECK("gemm_tc_kernel");
+    // (a split tail only ever comes with whole rows of CTA pairs: its operands are not exchanged)
     if (pl.tail_ways) {
-        const bool vec = oN % 4 == 0 && p.ldc % 4 == 0 && p.c_bstride % 4 == 0 &&
-                         ((reinterpret_cast<uintptr_t>(p.C) | reinterpret_cast<uintptr_t>(p.D)) & 15) == 0;
-        const dim3 grid(static_cast<unsigned>(BM * pl.cg / 4), static_cast<unsigned>(pl.tail_tiles));
-        e = launch_dependent(vec ? tail_finish_kernel<true> : tail_finish_kernel<false>, grid, dim3(256), 0, stream, partial, p.D,
-                             pl.bn, BM * pl.cg, k);
-        if (e != cudaSuccess) return fail(MNI_B200_ERR_CUDA, "tail_finish_kernel launch failed: %s", cudaGetErrorString(e));
-        MNI_LAUNCH_CHECK("tail_finish_kernel");
-    }
-    if (pl.splits > 1) {
-        const GemmFinish f{partial, p.C, p.ldc, p.c_bstride, p.batch, oM, oN, p.bias, p.accumulate, pl.splits};
-        if (defer) *defer = f;
-        else return launch_gemm_finish(f, 0, stream);
+        if (!defer) return launch_tail_finish(p, pl, k, partial, 0, stream);
+        *defer = [p, pl, k, partial](int dep_mode, cudaStream_t st) { return launch_tail_finish(p, pl, k, partial, dep_mode, st); };
+    } else if (pl.splits > 1) {
+        const SplitFinish f{partial, p.C, p.ldc, p.c_bstride, p.batch, oM, oN, p.bias, p.accumulate, pl.splits};
+        if (!defer) return launch_split_finish(f, 0, stream);
+        *defer = [f](int dep_mode, cudaStream_t st) { return launch_split_finish(f, dep_mode, st); };
     }
     return MNI_B200_OK;
 }

@@ -8,6 +8,7 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <functional>
 #include <string>
 
 #include "mni_b200.h"
@@ -147,19 +148,13 @@ size_t gemm_tc_partial_bytes(const GemmProblem &p, int sm_count);
 
 // Tensor-core path: TMA -> smem -> (hi/lo split) -> tcgen05.mma -> TMEM -> global.
 // `partial` must hold gemm_tc_partial_bytes() bytes when that is non-zero.
-// `defer` != null: the finish of a split contraction is not launched but described there (splits stays 0 if there is none).
-struct GemmFinish {
-    const float *partial = nullptr;
-    float *C = nullptr;
-    int64_t ldc = 0, c_bstride = 0, batch = 0, M = 0, N = 0;
-    const float *bias = nullptr;
-    bool accumulate = false;
-    int splits = 0;
-};
+// `defer` != null: a finish kernel (of a split contraction or a split tail) is not launched but left there; calling it
+// launches it.  dep_mode 1 / 2: first / second of two finishes that do not depend on each other, launched back to back.
+using GemmFinish = std::function<int(int dep_mode, cudaStream_t stream)>;
 int launch_gemm_tc(const GemmProblem &p, float *partial, uint32_t *err_word, int sm_count,
                    cudaStream_t stream, GemmFinish *defer = nullptr);
-// dep_mode 1 / 2: first / second of two finishes that do not depend on each other, launched back to back
-int launch_gemm_finish(const GemmFinish &f, int dep_mode, cudaStream_t stream);
+// Whether the problem is computed by CTA pairs.
+bool gemm_tc_uses_pairs(const GemmProblem &p, int sm_count);
 // The plan's cost model for this problem in microseconds (0: the model does not cover it).
 double gemm_tc_estimate_us(const GemmProblem &p, int sm_count);
 // One line of text naming the kernel variant, tiling, split and grid launch_gemm_tc would use for this problem
