@@ -838,7 +838,7 @@ int bwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const mni_
             c.note("streaming (skinny) input-gradient kernel");
             if (!c.dry()) {
                 rc = launch_skinny_dx(dc_given->ptr, dc_given->stride[gn - 2], b_given->ptr, b_given->stride[b_given->ndim - 2], da, s.K, acc_da,
-                                      s.M, s.N, s.K, c.stream);
+                                      s.M, s.N, s.K, !overlap, c.stream);
                 if (rc) return rc;
             }
         } else if (rows_dx) {

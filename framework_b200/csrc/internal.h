@@ -31,7 +31,7 @@ __device__ __forceinline__ void grid_dependency_trigger() {
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <typename... KArgs, typename... Args>
-cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+cudaError_t launch_dependent(bool dependent, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
                              Args &&...args) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
@@ -40,10 +40,14 @@ cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, si
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+    attr[0].val.programmaticStreamSerializationAllowed = dependent && pdl_enabled() ? 1 : 0;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+template <typename... KArgs, typename... Args>
+cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args &&...args) {
+    return launch_dependent(true, kernel, grid, block, smem, stream, static_cast<Args &&>(args)...);
 }
 #endif
 
@@ -178,8 +182,10 @@ int launch_skinny_fwd(const float *x, int64_t ldx, const float *W, int64_t ldw, 
                       float *partial, int sm_count, cudaStream_t stream);
 //   dx[M,K] = dy[M,N] . W[K,N]^T                                    M <= 8
 bool skinny_dx_supported(const float *dy, int64_t lddy, const float *W, int64_t ldw, int64_t M, int64_t N);
+//   (dependent: as a programmatic dependent launch -- not beside a product on another stream, whose blocks would find
+//   the waiting ones of this kernel in their places)
 int launch_skinny_dx(const float *dy, int64_t lddy, const float *W, int64_t ldw, float *dx, int64_t lddx,
-                     bool accumulate, int64_t M, int64_t N, int64_t K, cudaStream_t stream);
+                     bool accumulate, int64_t M, int64_t N, int64_t K, bool dependent, cudaStream_t stream);
 //   dW[K,N] = x[M,K]^T . dy[M,N]                                     M <= 16
 int launch_skinny_dw(const float *x, int64_t ldx, const float *dy, int64_t lddy, float *dW, int64_t lddw,
                      bool accumulate, int64_t M, int64_t N, int64_t K, cudaStream_t stream);

@@ -737,7 +737,7 @@ bool skinny_dx_supported(const float *dy, int64_t lddy, const float *W, int64_t 
 }
 
 int launch_skinny_dx(const float *dy, int64_t lddy, const float *W, int64_t ldw, float *dx, int64_t lddx,
-                     bool accumulate, int64_t M, int64_t N, int64_t K, cudaStream_t stream) {
+                     bool accumulate, int64_t M, int64_t N, int64_t K, bool dependent, cudaStream_t stream) {
     const int mt = pick_mt(M);
     const int sliced = dx_sliced_mode();
     if (sliced > 0) {
@@ -771,8 +771,8 @@ int launch_skinny_dx(const float *dy, int64_t lddy, const float *W, int64_t ldw,
     cudaError_t e = cudaErrorInvalidValue;
 #define MNI_SKINNY_DX(MT)                                                                              \
     case MT:                                                                                           \
-        e = launch_dependent(full ? skinny_dx_kernel<MT, true> : skinny_dx_kernel<MT, false>, dim3(blocks), dim3(kDxThreads), 0, \
-                             stream, dy, lddy, W, ldw, dx, lddx, accumulate ? 1 : 0, static_cast<int>(M), N, K); \
+        e = launch_dependent(dependent, full ? skinny_dx_kernel<MT, true> : skinny_dx_kernel<MT, false>, dim3(blocks), \
+                             dim3(kDxThreads), 0, stream, dy, lddy, W, ldw, dx, lddx, accumulate ? 1 : 0, static_cast<int>(M), N, K); \
         break;
     switch (mt) {
         MNI_SKINNY_DX(1) MNI_SKINNY_DX(2) MNI_SKINNY_DX(4) MNI_SKINNY_DX(8)
