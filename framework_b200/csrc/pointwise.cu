@@ -3,6 +3,7 @@
 #include "internal.h"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace mni {
 
@@ -193,7 +194,7 @@ bias_kernel(const float *__restrict__ y, const float *__restrict__ bias, float *
 
 // Backward: dx = grad * gelu'(x + bias) written once, and the column sums of dx (same block shape and fixed summation
 // order as colsum_kernel; no atomics on values).
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 4)      // four blocks per SM is what colsum_slabs plans for: one wave
 bias_gelu_bwd_kernel(const float *__restrict__ grad, const float *__restrict__ x, const float *__restrict__ bias,
                      float *__restrict__ dx, float *__restrict__ partial, float *__restrict__ dbias, long long rows,
                      long long n, long long rows_per, int accumulate) {
@@ -214,27 +215,29 @@ bias_gelu_bwd_kernel(const float *__restrict__ grad, const float *__restrict__ x
             if (col + e < n) b[e] = __ldg(bias + col + e);
         long long r = r0 + warp;
         if (vec) {
-            constexpr int U = 4;              // rows in flight per thread
-            for (; r < r1; r += 8 * U) {
-                float4 g[U], v[U];
+            auto batch = [&](auto rows_in_flight) {
+                constexpr int U = decltype(rows_in_flight)::value;
+                for (; r + 8 * (U - 1) < r1; r += 8 * U) {
+                    float4 g[U], v[U];
 #pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const long long off = min(r + 8 * u, r1 - 1) * n + col;
-                    g[u] = __ldcs(reinterpret_cast<const float4 *>(grad + off));
-                    v[u] = __ldcs(reinterpret_cast<const float4 *>(x + off));
-                }
+                    for (int u = 0; u < U; ++u) {
+                        g[u] = __ldcs(reinterpret_cast<const float4 *>(grad + (r + 8 * u) * n + col));
+                        v[u] = __ldcs(reinterpret_cast<const float4 *>(x + (r + 8 * u) * n + col));
+                    }
 #pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    if (r + 8 * u >= r1) break;
-                    float4 d;
-                    d.x = g[u].x * gelu_tanh_grad(v[u].x + b[0]);
-                    d.y = g[u].y * gelu_tanh_grad(v[u].y + b[1]);
-                    d.z = g[u].z * gelu_tanh_grad(v[u].z + b[2]);
-                    d.w = g[u].w * gelu_tanh_grad(v[u].w + b[3]);
-                    *reinterpret_cast<float4 *>(dx + (r + 8 * u) * n + col) = d;
-                    acc.x += d.x; acc.y += d.y; acc.z += d.z; acc.w += d.w;
+                    for (int u = 0; u < U; ++u) {
+                        float4 d;
+                        d.x = g[u].x * gelu_tanh_grad(v[u].x + b[0]);
+                        d.y = g[u].y * gelu_tanh_grad(v[u].y + b[1]);
+                        d.z = g[u].z * gelu_tanh_grad(v[u].z + b[2]);
+                        d.w = g[u].w * gelu_tanh_grad(v[u].w + b[3]);
+                        *reinterpret_cast<float4 *>(dx + (r + 8 * u) * n + col) = d;
+                        acc.x += d.x; acc.y += d.y; acc.z += d.z; acc.w += d.w;
+                    }
                 }
-            }
+            };
+            batch(std::integral_constant<int, 2>{});      // rows in flight per thread (four spill at 64 registers)
+            batch(std::integral_constant<int, 1>{});
         } else {
             for (; r < r1; r += 8) {
                 const long long off = r * n + col;

@@ -25,8 +25,8 @@
  *     with MNI_B200_ERR_DEVICE.
  *   - Threads and streams.  Calls may come from any host thread; state is per
  *     device and guarded by a per-device lock.  The scratch buffer, the finish
- *     tickets of the split-K / streaming kernels and the flags of the balanced
- *     tail are ONE set per device, shared by every stream: two calls whose
+ *     tickets of the streaming kernels, the column sums and the gradient norm, and
+ *     the flags of the balanced tail are ONE set per device, shared by every stream: two calls whose
  *     kernels can run at the same time on one device (different streams with no
  *     event between them) race on them.  Keep a device's calls on one stream --
  *     what the reference does (device.rs:37) -- or order the streams with events.
