@@ -15,14 +15,19 @@ namespace {
 
 constexpr int kMaxDims = MNI_B200_MAX_DIMS;
 constexpr int kThreads = 256;
-constexpr int kItems = 4;                       // units per thread of the row forms, all in flight together
+// Units per thread of the row forms, all in flight together.  One up to 16 blocks per SM, where a second unit only takes
+// warps away (4 MB head merge 4.5 us at four units, 3.2 at two, 2.6 at one); two beyond, where it covers the latency of
+// the first (12.6 MB 6.2 / 4.9 / 5.0, 48x333x333 padded to 336 by 1.2 us faster at two than at four).
+constexpr int kMaxItems = 2;
+constexpr int kOneItemBlocksPerSm = 16;
 constexpr int kTileU = 32, kTileI = 64;         // transposing form: source-contiguous x destination-contiguous
 
 enum GatherKind {
     kRowsVec = 0,        // rows contiguous and aligned on both sides: a 16-byte unit each way
     kRowsQuad = 1,       // source rows contiguous, not aligned; destination padded to whole 16-byte units (pads become 0)
-    kElements = 2,       // anything else, an element per unit
-    kTranspose = 3,      // another dimension is the contiguous one of the source: tiles through shared memory
+    kFlatQuad = 2,       // dense destination, any source: four consecutive elements per unit, which may cross rows
+    kElements = 3,       // anything else, an element per unit
+    kTranspose = 4,      // another dimension is the contiguous one of the source: tiles through shared memory
 };
 
 struct Gather {
@@ -38,6 +43,7 @@ struct Gather {
     long long s_inner, d_u;             // source stride of the last dimension, destination stride of the other
     long long ld;                       // destination pitch of a row
     int items;                          // row forms: total units
+    int elements;                       // kFlatQuad: total elements
     unsigned first;                     // first block of this gather
 };
 struct GatherList {
@@ -45,6 +51,21 @@ struct GatherList {
     int count;
 };
 
+// Source address of the start of a row.
+__device__ __forceinline__ const float *row_source(const Gather &g, int row) {
+    const float *src = g.src;
+    for (int d = g.nd - 1; d >= 0; --d) {
+        const int q = fd_div(row, g.ext[d]);
+        src += (row - q * static_cast<int>(g.ext[d].d)) * g.sstr[d];
+        row = q;
+    }
+    return src;
+}
+
+// FLAT: some gather of the list is kFlatQuad, whose row crossings cost 8 registers a thread that the other forms keep for
+// occupancy (12.6 MB head merge 6.1 us with them, 5.1 without).  Against an element per unit, four with one store take a
+// permuted 500x333x65 from 48 us to 31.5.
+template <int ITEMS, bool FLAT>
 __global__ void __launch_bounds__(kThreads)
 gather_kernel(const __grid_constant__ GatherList list) {
     __shared__ float tile[kTileI][kTileU + 1];
@@ -90,22 +111,34 @@ gather_kernel(const __grid_constant__ GatherList list) {
         }
         return;
     }
-    const int base = block * (kThreads * kItems) + threadIdx.x;
-    long long to[kItems];
-    float4 v[kItems];
+    const int base = block * (kThreads * ITEMS) + threadIdx.x;
+    long long to[ITEMS];
+    float4 v[ITEMS];
 #pragma unroll
-    for (int u = 0; u < kItems; ++u) {
+    for (int u = 0; u < ITEMS; ++u) {
         const int item = base + u * kThreads;
         if (item >= g.items) continue;
-        int rem = fd_div(item, g.units);
-        const int c = item - rem * static_cast<int>(g.units.d);
-        const float *src = g.src;
-        to[u] = rem * g.ld;
-        for (int d = g.nd - 1; d >= 0; --d) {
-            const int q = fd_div(rem, g.ext[d]);
-            src += (rem - q * static_cast<int>(g.ext[d].d)) * g.sstr[d];
-            rem = q;
+        if (FLAT && g.kind == kFlatQuad) {
+            const int at = 4 * item;
+            int row = fd_div(at, g.units), c = at - row * static_cast<int>(g.units.d);
+            const float *src = row_source(g, row);
+            to[u] = at;
+            float e[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                if (at + k >= g.elements) break;
+                e[k] = __ldg(src + c * g.s_inner);
+                if (++c == static_cast<int>(g.units.d) && k < 3 && at + k + 1 < g.elements) {
+                    c = 0;
+                    src = row_source(g, ++row);
+                }
+            }
+            v[u] = make_float4(e[0], e[1], e[2], e[3]);
+            continue;
         }
+        const int row = fd_div(item, g.units), c = item - row * static_cast<int>(g.units.d);
+        const float *src = row_source(g, row);
+        to[u] = row * g.ld;
         if (g.kind == kElements) {
             to[u] += c;
             v[u].x = __ldg(src + c * g.s_inner);
@@ -124,10 +157,19 @@ gather_kernel(const __grid_constant__ GatherList list) {
         }
     }
 #pragma unroll
-    for (int u = 0; u < kItems; ++u) {
-        if (base + u * kThreads >= g.items) continue;
-        if (g.kind == kElements) g.dst[to[u]] = v[u].x;
-        else *reinterpret_cast<float4 *>(g.dst + to[u]) = v[u];
+    for (int u = 0; u < ITEMS; ++u) {
+        const int item = base + u * kThreads;
+        if (item >= g.items) continue;
+        if (g.kind == kElements) {
+            g.dst[to[u]] = v[u].x;
+        } else if (FLAT && g.kind == kFlatQuad && 4 * item + 4 > g.elements) {
+            const float e[3] = {v[u].x, v[u].y, v[u].z};
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+                if (4 * item + k < g.elements) g.dst[4 * item + k] = e[k];
+        } else {
+            *reinterpret_cast<float4 *>(g.dst + to[u]) = v[u];
+        }
     }
 }
 
@@ -159,7 +201,8 @@ gather_wide_kernel(const float *__restrict__ src, float *__restrict__ dst, const
 
 bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-// Fills `g` for one view; returns the number of blocks.  The view has fewer than 2^31 elements, none of its extents is 0.
+// Fills `g` for one view; returns its tiles (transposing form, a block each) or units (the others).  The view has fewer
+// than 2^31 elements, none of its extents is 0.
 unsigned plan_gather(const GatherView &view, Gather &g) {
     const mni_b200_view &v = *view.src;
     // Dimensions outermost first: extent, source stride, destination stride.
@@ -227,12 +270,14 @@ unsigned plan_gather(const GatherView &view, Gather &g) {
     }
     const bool units4 = (ss[last] == 1 || ext[last] == 1) && aligned16(view.dst) && (rows == 1 || ld % 4 == 0);
     if (units4 && aligned && ext[last] % 4 == 0) g.kind = kRowsVec;
-    else if (units4 && (rows == 1 ? ext[last] % 4 == 0 : ld - ext[last] < 4)) g.kind = kRowsQuad;
+    else if (units4 && (rows == 1 ? ext[last] % 4 == 0 : ld - ext[last] < 4 && ld != ext[last])) g.kind = kRowsQuad;
+    else if (aligned16(view.dst) && (rows == 1 || ld == ext[last])) g.kind = kFlatQuad;
     else g.kind = kElements;
-    const int64_t units = g.kind == kElements ? ext[last] : (ext[last] + 3) / 4;
+    g.elements = static_cast<int>(rows * ext[last]);
+    const int64_t units = g.kind == kElements || g.kind == kFlatQuad ? ext[last] : (ext[last] + 3) / 4;
     g.units = make_fastdiv(units);
-    g.items = static_cast<int>(rows * units);
-    return static_cast<unsigned>((rows * units + kThreads * kItems - 1) / (kThreads * kItems));
+    g.items = static_cast<int>(g.kind == kFlatQuad ? (rows * ext[last] + 3) / 4 : rows * units);
+    return static_cast<unsigned>(g.items);
 }
 
 }  // namespace
@@ -240,13 +285,15 @@ unsigned plan_gather(const GatherView &view, Gather &g) {
 int launch_gather(const GatherView *views, int count, cudaStream_t stream) {
     GatherList list;
     list.count = 0;
-    unsigned blocks = 0;
+    unsigned sizes[kMaxGathers];
+    long long units = 0;
+    bool flat = false;
     for (int i = 0; i < count; ++i) {
         const mni_b200_view &v = *views[i].src;
         long long total = 1;
         for (int d = 0; d < v.ndim; ++d) total *= v.shape[d];
         if (total == 0) continue;
-        if (total >= (1LL << 31) - kThreads * kItems || views[i].ld_dst >= (1LL << 31)) {
+        if (total >= (1LL << 31) - 4 * kThreads * kMaxItems || views[i].ld_dst >= (1LL << 31)) {
             WideGather a{};
             a.nd = v.ndim;
             for (int d = 0; d < v.ndim; ++d) { a.shape[d] = v.shape[d]; a.stride[d] = v.stride[d]; }
@@ -258,12 +305,22 @@ int launch_gather(const GatherView *views, int count, cudaStream_t stream) {
             MNI_LAUNCH_CHECK("gather_wide_kernel");
             continue;
         }
-        Gather &g = list.g[list.count++];
-        g.first = blocks;
-        blocks += plan_gather(views[i], g);
+        sizes[list.count] = plan_gather(views[i], list.g[list.count]);
+        if (list.g[list.count].kind != kTranspose) units += sizes[list.count];
+        if (list.g[list.count].kind == kFlatQuad) flat = true;
+        ++list.count;
+    }
+    const bool one = units <= static_cast<long long>(device_sm_count()) * kOneItemBlocksPerSm * kThreads;
+    const unsigned per_block = kThreads * (one ? 1 : kMaxItems);
+    unsigned blocks = 0;
+    for (int i = 0; i < list.count; ++i) {
+        list.g[i].first = blocks;
+        blocks += list.g[i].kind == kTranspose ? sizes[i] : (sizes[i] + per_block - 1) / per_block;
     }
     if (blocks == 0) return MNI_B200_OK;
-    const cudaError_t e = launch_dependent(gather_kernel, dim3(blocks), dim3(kThreads), 0, stream, list);
+    const auto kernel = one ? (flat ? gather_kernel<1, true> : gather_kernel<1, false>)
+                            : (flat ? gather_kernel<kMaxItems, true> : gather_kernel<kMaxItems, false>);
+    const cudaError_t e = launch_dependent(kernel, dim3(blocks), dim3(kThreads), 0, stream, list);
     if (e != cudaSuccess) return fail(MNI_B200_ERR_CUDA, "gather_kernel launch failed: %s", cudaGetErrorString(e));
     MNI_LAUNCH_CHECK("gather_kernel");
     return MNI_B200_OK;

@@ -33,6 +33,23 @@ def test_gather_of_permuted_views(F, shape, dims):
     assert np.array_equal(back.numpy(), a)
 
 
+@pytest.mark.parametrize("shape,dims", [
+    ((7, 5, 3), (1, 0, 2)),                 # rows of 3 in units of 4, a remainder of 1
+    ((3, 5, 2), (1, 0, 2)), ((9, 7, 1, 5), (1, 0, 2, 3)), ((2, 3), (1, 0)), ((31, 3, 17), (2, 1, 0)),
+    ((150, 333, 65), (1, 0, 2)),            # two units per thread, the last one partial
+    ((4, 12, 640, 79), (0, 2, 1, 3)),
+    ((8, 400, 12, 64), (0, 2, 1, 3))])      # two aligned units per thread
+def test_gather_in_units_across_rows(F, shape, dims):
+    a = _rng(7, *shape).standard_normal(shape).astype(np.float32)
+    view = F.DeviceTensor.from_numpy(a).permute(dims)
+    want = np.ascontiguousarray(a.transpose(dims))
+    for misalign in (0, 1):
+        out = Guarded(F, want.shape, misalign=misalign)
+        F._lib.check(F._lib.lib().mni_b200_contiguous(view.view_struct(), out.tensor.ptr, 0))
+        out.check("gather")
+        assert np.array_equal(out.tensor.numpy(), want)
+
+
 @pytest.mark.parametrize("rows,n,misalign", [(1, 1, 0), (63, 4, 0), (65, 130, 0), (64, 128, 0), (1000, 516, 0), (129, 260, 1),
                                              (777, 131, 0), (5000, 33, 0), (40, 200_000, 0)])
 def test_bias_add_and_its_backward(F, rows, n, misalign):
