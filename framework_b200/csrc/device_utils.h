@@ -10,6 +10,11 @@ __device__ __forceinline__ void cp_async16(void *smem, const void *gmem, bool va
     const int bytes = valid ? 16 : 0;                       // 0: nothing is read, the slot is zero-filled
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(gmem), "r"(bytes) : "memory");
 }
+// ... of which only the first `bytes` are read, the rest of the slot is zero-filled.
+__device__ __forceinline__ void cp_async16_part(void *smem, const void *gmem, int bytes) {
+    const unsigned dst = static_cast<unsigned>(__cvta_generic_to_shared(smem));
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(gmem), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
@@ -41,13 +46,6 @@ __device__ __forceinline__ float4 cluster_sum_f4(const void *own_smem, int ranks
     for (int r = 1; r < kMaxClusterRanks; ++r)
         if (r < ranks) { sum.x += p[r].x; sum.y += p[r].y; sum.z += p[r].z; sum.w += p[r].w; }
     return sum;
-}
-
-// Four bytes, for rows that are not 16-byte aligned.
-__device__ __forceinline__ void cp_async4(void *smem, const void *gmem, bool valid) {
-    const unsigned dst = static_cast<unsigned>(__cvta_generic_to_shared(smem));
-    const int bytes = valid ? 4 : 0;
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(gmem), "r"(bytes) : "memory");
 }
 
 }  // namespace mni

@@ -10,7 +10,7 @@
 // allocate, no descriptors, no operand staging beyond the ring and an accumulator that is already in registers.  The
 // tcgen05 path takes the same products in 64-wide tiles with a split contraction and a second kernel that sums it, and
 // gathers a weight with an odd row length into scratch first.  Nine rows x 4096 x 4096: forward 20.1 -> 18.0 us, dx 19.9 ->
-// 18.0, the step 79 -> 55; 4096 x 4095: forward 53 -> 30 us, dx 44 -> 34, the step 153 -> 96.
+// 18.0, the step 79 -> 55; 4096 x 4095: forward 53 -> 21 us, dx 44 -> 22, the step 153 -> 83.
 //
 // Split as in the tensor path: hi = x with the low 13 mantissa bits cut, lo = x - hi, products lo.hi + hi.lo + hi.hi.
 // A chain in the tensor core's accumulator, which truncates, is kFlush elements long; longer sums are added up in
@@ -61,15 +61,18 @@ __device__ __forceinline__ void mma_split(float (&acc)[4][4], const uint32_t (&a
 // out[m, o] = sum_c x[m, c] . w(c, o), with w(c, o) = W[c, o] (forward) or W[o, c] (DX).
 // grid = (strips of outputs, contraction slices), the slices of a strip one cluster.  WK = 1: the block's four warps take
 // 32 outputs each of a 128-wide strip; WK = 4: they share a 32-wide strip and take every fourth tile of the slice each,
-// which keeps more of the chip busy when the outputs are few.  Every warp streams its part of W through a private ring of 32 x 32 tiles (cp.async: 16-byte pieces where the rows of W are
-// aligned, single floats where they are not -- the loads are contiguous along the row either way), x is staged once per
-// block.  The tile pitch makes the fragment reads conflict-free: 40 floats for 16-byte reads of four neighbouring
-// outputs (forward), 36 for reads down a column (DX).  The slices' sums meet through distributed shared memory.
+// which keeps more of the chip busy when the outputs are few.  Every warp streams its part of W through a private ring of
+// 32 x 32 tiles by cp.async of 16-byte units; x is staged once per block in the same way.  Rows that are not 16-byte
+// aligned (VEC = false) are copied from the boundary before them, nine units for 32 words, and keep their shift in shared
+// memory, where the fragment reads add it.  (Copied word by word they took the load path 26 cycles per 128 bytes: 16 rows x
+// 4096 x 4095 forward 30 -> 20.8 us, dx 34 -> 22; 3 rows x 5486 x 7657 127 -> 85.)  The tile pitch makes the fragment
+// reads of aligned rows conflict-free: 40 floats for 16-byte reads of four neighbouring outputs (forward), 36 for reads
+// down a column (DX).  The slices' sums meet through distributed shared memory.
 template <bool DX, bool VEC, int WK>
 __global__ void __launch_bounds__(kThreads, 2)
 rows_kernel(const float *__restrict__ x, long long ldx, const float *__restrict__ W, long long ldw, float *__restrict__ y,
             long long ldy, const float *__restrict__ bias, int accumulate, int M, long long outs, long long total, int k_per,
-            int x_vec, int y_vec) {
+            int y_vec) {
     constexpr int PITCH = DX ? 36 : 40;
     constexpr int OUTS = 32 * (kWarps / WK), SUM_PITCH = OUTS + 4;      // outputs per block
     extern __shared__ __align__(16) float smem[];
@@ -83,10 +86,16 @@ rows_kernel(const float *__restrict__ x, long long ldx, const float *__restrict_
     const long long o0 = static_cast<long long>(blockIdx.x) * OUTS + ow * 32;
     const int nb = ((kc + 31) / 32 - kw + WK - 1) / WK;     // tiles kw, kw + WK, ... of the slice
     float *mine = ring + warp * (kDepth * 32 * PITCH);
-    // extents of this warp's part of W, as rows and columns of W
+    // extents of this warp's part of W, as rows and columns of W (tiles start at multiples of 32 of either)
     const int rows_live = DX ? static_cast<int>(max(0ll, min(32ll, outs - o0))) : kc;
     const int cols_live = DX ? kc : static_cast<int>(max(0ll, min(32ll, outs - o0)));
     const float *wp = DX ? W + o0 * ldw + k0 : W + k0 * ldw + o0;
+    // Words by which a row starts past a 16-byte boundary; rows four apart are alike, so the row that a lane copies or
+    // multiplies has one shift throughout.
+    const int w_at = static_cast<int>((reinterpret_cast<uintptr_t>(wp) >> 2) & 3), w_step = static_cast<int>(ldw & 3);
+    auto shift_of = [&](int row) { return VEC ? 0 : (w_at + row * w_step) & 3; };
+    const int x_at = static_cast<int>((reinterpret_cast<uintptr_t>(x) >> 2) & 3), x_step = static_cast<int>(ldx & 3);
+    auto x_shift = [&](int m) { return (x_at + m * x_step) & 3; };
     grid_dependency_trigger();
     grid_dependency_wait();
     auto issue = [&](int b) {
@@ -101,30 +110,26 @@ rows_kernel(const float *__restrict__ x, long long ldx, const float *__restrict_
                     cp_async16(slot + r * PITCH + c, ok ? wp + (r0 + r) * ldw + c0 + c : W, ok);
                 }
             } else {
-#pragma unroll 8
-                for (int r = 0; r < 32; ++r) {
-                    const bool ok = r0 + r < rows_live && c0 + lane < cols_live;
-                    cp_async4(slot + r * PITCH + lane, ok ? wp + (r0 + r) * ldw + c0 + lane : W, ok);
-                }
+                // whole 16-byte units from the boundary before the row's part: nine cover 32 words at any shift
+                const int end = min(32, cols_live - c0);
+                auto unit = [&](int r, int q, int sh) {
+                    const int words = r0 + r < rows_live && end > 0 ? max(0, min(4, end + sh - 4 * q)) : 0;
+                    const float *src = words > 0 ? wp + (r0 + r) * ldw + c0 - sh + 4 * q : x - x_at;
+                    cp_async16_part(slot + r * PITCH + 4 * q, src, 4 * words);
+                };
+                const int sh = shift_of(lane >> 3), sh_last = shift_of(lane);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) unit(i * 4 + (lane >> 3), lane & 7, sh);
+                if (sh_last > 0) unit(lane, 8, sh_last);
             }
         }
         cp_async_commit();                                  // empty groups keep the count uniform
     };
-    if (x_vec) {
-        const int quads = k_per / 4;
-        for (int i = threadIdx.x; i < kRows * quads; i += kThreads) {
-            const int m = i / quads, kk = (i - m * quads) * 4;
-            const int valid = m < M ? max(0, min(4, kc - kk)) : 0;
-            const unsigned dst = static_cast<unsigned>(__cvta_generic_to_shared(xs + m * xp + kk));
-            const float *src = valid > 0 ? x + m * ldx + k0 + kk : x;
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid * 4) : "memory");
-        }
-    } else {
-        for (int m = 0; m < kRows; ++m)
-            for (int kk = threadIdx.x; kk < k_per; kk += kThreads) {
-                const bool ok = m < M && kk < kc;
-                cp_async4(xs + m * xp + kk, ok ? x + m * ldx + k0 + kk : x, ok);
-            }
+    const int quads = k_per / 4 + 1;
+    for (int i = threadIdx.x; i < kRows * quads; i += kThreads) {
+        const int m = i / quads, q = i - m * quads, sh = x_shift(m);
+        const int words = m < M ? max(0, min(4, kc + sh - 4 * q)) : 0;
+        cp_async16_part(xs + m * xp + 4 * q, words > 0 ? x + m * ldx + k0 - sh + 4 * q : x - x_at, 4 * words);
     }
     cp_async_commit();
 #pragma unroll
@@ -142,7 +147,8 @@ rows_kernel(const float *__restrict__ x, long long ldx, const float *__restrict_
         cp_async_wait<kDepth - 1>();                        // tile b has landed, for this lane ...
         __syncwarp();                                       // ... and for the others
         const float *slot = mine + (b % kDepth) * (32 * PITCH);
-        const float *xr = xs + g * xp + (b * WK + kw) * 32 + t;
+        const float *xr = xs + g * xp + x_shift(g) + (b * WK + kw) * 32 + t;
+        const float *rows = slot + shift_of(DX ? g : t);    // of the row whose elements this lane multiplies
 #pragma unroll
         for (int s = 0; s < 4; ++s) {
             uint32_t ah[4], al[4];
@@ -154,8 +160,14 @@ rows_kernel(const float *__restrict__ x, long long ldx, const float *__restrict_
             if (DX) {                                       // tile j, column n = g: W row 8j + g
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    b0[j] = slot[(j * 8 + g) * PITCH + s * 8 + t];
-                    b1[j] = slot[(j * 8 + g) * PITCH + s * 8 + t + 4];
+                    b0[j] = rows[(j * 8 + g) * PITCH + s * 8 + t];
+                    b1[j] = rows[(j * 8 + g) * PITCH + s * 8 + t + 4];
+                }
+            } else if (!VEC) {                              // tile j, column n = g: W column 8j + g
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    b0[j] = rows[(s * 8 + t) * PITCH + j * 8 + g];
+                    b1[j] = rows[(s * 8 + t + 4) * PITCH + j * 8 + g];
                 }
             } else {                                        // tile j, column n = g: W column 4g + j, four tiles in one read
                 const float4 v0 = *reinterpret_cast<const float4 *>(slot + (s * 8 + t) * PITCH + g * 4);
@@ -178,7 +190,7 @@ rows_kernel(const float *__restrict__ x, long long ldx, const float *__restrict_
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         float *row = sums + (kw * kRows + g + 8 * h) * SUM_PITCH + ow * 32;
-        if (DX) {
+        if (DX || !VEC) {
 #pragma unroll
             for (int j = 0; j < 4; ++j)
                 *reinterpret_cast<float2 *>(row + j * 8 + 2 * t) = make_float2(sum[j][2 * h], sum[j][2 * h + 1]);
@@ -376,10 +388,10 @@ int launch_rows(const float *x, int64_t ldx, const float *W, int64_t ldw, float 
     attrs[1].val.clusterDim.z = 1;
     cfg.attrs = attrs;
     cfg.numAttrs = pl.slices > 1 ? 2 : 1;
-    const int x_vec = (ldx % 4 == 0 || M == 1) && aligned(x, 16) ? 1 : 0, y_vec = ldy % 4 == 0 && aligned(y, 16) ? 1 : 0;
+    const int y_vec = ldy % 4 == 0 && aligned(y, 16) ? 1 : 0;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, x, static_cast<long long>(ldx), W, static_cast<long long>(ldw), y,
                                              static_cast<long long>(ldy), bias, accumulate ? 1 : 0, static_cast<int>(M),
-                                             static_cast<long long>(outs), static_cast<long long>(total), k_per, x_vec, y_vec);
+                                             static_cast<long long>(outs), static_cast<long long>(total), k_per, y_vec);
     if (e != cudaSuccess) return fail(MNI_B200_ERR_CUDA, "rows_kernel launch failed: %s", cudaGetErrorString(e));
     MNI_LAUNCH_CHECK("rows_kernel");
     return MNI_B200_OK;

@@ -39,3 +39,26 @@ def test_few_rows_plans(F):
     assert "few rows" in kernel(9, 4096, 4096) and "few rows" in kernel(16, 4096, 4093) and "few rows" in kernel(9, 1000, 4001)
     assert "skinny" in kernel(3, 4096, 4096)
     assert "tensor" in kernel(16, 4096, 4096) and "tensor" in kernel(9, 8192, 512)
+
+
+@pytest.mark.parametrize("m,k,n", [(2, 97, 130), (7, 129, 1001), (16, 70, 63), (13, 1030, 2434), (4, 33, 4100)])
+@pytest.mark.parametrize("offset", [0, 1, 2, 3])
+def test_few_rows_units_from_before_a_row(F, m, k, n, offset):
+    """Rows at every shift against the 16-byte units that they are copied in; NaNs around the operands must not leak in."""
+    rng = np.random.default_rng([m, k, n, offset])
+
+    def inside(a, at):
+        buf = np.full(a.size + 8, np.nan, np.float32)
+        buf[at:at + a.size] = a.ravel()
+        return F.DeviceTensor(F.DeviceTensor.from_numpy(buf).torch_view()[at:at + a.size], a.shape)
+
+    x, dy = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((m, n)).astype(np.float32)
+    w = rng.standard_normal((k, n)).astype(np.float32)
+    x64, w64, dy64 = (a.astype(np.float64) for a in (x, w, dy))
+    for transposed in (False, True):
+        wd = inside(np.ascontiguousarray(w.T), offset).permute((1, 0)) if transposed else inside(w, offset)
+        y = F.matmul(inside(x, (offset + 1) % 4), wd)
+        dx, dw = F.matmul_backward(inside(dy, (offset + 2) % 4), inside(x, (offset + 1) % 4), wd)
+        F.device_status()
+        for got, want, length in ((y, x64 @ w64, k), (dx, dy64 @ w64.T, n), (dw, x64.T @ dy64, m)):
+            assert rel_fro(got.numpy(), want) <= regression_bound_3xtf32(length)
