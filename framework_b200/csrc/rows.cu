@@ -30,7 +30,11 @@ constexpr int kDwCols = 32 * kWarps;         // columns of dW per block
 constexpr int kDepth = 4;                    // 32 x 32 weight tiles held per warp, three in flight: 96 KB per SM with two blocks
 constexpr int kRows = 16;
 constexpr int kFlush = 256;                  // contraction elements summed in one tensor-core accumulator
-constexpr int kMaxSlice = 2048;              // contraction per block (its x is staged whole: 131 KB)
+// Contraction elements of x staged at a time, in two buffers where a block's slice is longer.  128-wide strips: 33 KB
+// either way, which leaves room for two blocks per SM; 32-wide ones, whose warps take every fourth tile each, need chunks of
+// four tiles per warp for the copies to be in time.
+constexpr int kChunk = 256, kChunkNarrow = 512;
+constexpr int64_t kMaxTotal = 16384;         // longest contraction taken here
 constexpr int kMaxSlices = 8;                // slices of a strip: one portable cluster
 
 __device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
@@ -76,9 +80,11 @@ rows_kernel(const float *__restrict__ x, long long ldx, const float *__restrict_
     constexpr int PITCH = DX ? 36 : 40;
     constexpr int OUTS = 32 * (kWarps / WK), SUM_PITCH = OUTS + 4;      // outputs per block
     extern __shared__ __align__(16) float smem[];
-    const int xp = k_per + 4;                               // = 4 mod 32: the A fragments' scalar reads hit all banks
-    float *xs = smem;                                       // [kRows][xp]
-    float *ring = smem + kRows * xp;                        // [warps][depth][32][PITCH]; later the block's sums
+    constexpr int CHUNK = WK == 1 ? kChunk : kChunkNarrow;
+    const int xk = k_per <= 512 ? k_per : CHUNK;            // contraction per chunk of x
+    const int xp = xk + 4;                                  // = 4 mod 32: the A fragments' scalar reads hit all banks
+    float *xs = smem;                                       // [1 or 2][kRows][xp]
+    float *ring = smem + kRows * xp * (k_per <= 512 ? 1 : 2);   // [warps][depth][32][PITCH]; later the block's sums
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
     const long long k0 = static_cast<long long>(blockIdx.y) * k_per;
     const int kc = static_cast<int>(min(static_cast<long long>(k_per), total - k0));
@@ -125,12 +131,17 @@ rows_kernel(const float *__restrict__ x, long long ldx, const float *__restrict_
         }
         cp_async_commit();                                  // empty groups keep the count uniform
     };
-    const int quads = k_per / 4 + 1;
-    for (int i = threadIdx.x; i < kRows * quads; i += kThreads) {
-        const int m = i / quads, q = i - m * quads, sh = x_shift(m);
-        const int words = m < M ? max(0, min(4, kc + sh - 4 * q)) : 0;
-        cp_async16_part(xs + m * xp + 4 * q, words > 0 ? x + m * ldx + k0 - sh + 4 * q : x - x_at, 4 * words);
-    }
+    const int quads = xk / 4 + 1;
+    auto stage_x = [&](int chunk) {
+        const int at = chunk * xk, live = min(xk, kc - at);
+        float *dst = xs + (chunk & 1) * (kRows * xp);
+        for (int i = threadIdx.x; i < kRows * quads; i += kThreads) {
+            const int m = i / quads, q = i - m * quads, sh = x_shift(m);
+            const int words = m < M ? max(0, min(4, live + sh - 4 * q)) : 0;
+            cp_async16_part(dst + m * xp + 4 * q, words > 0 ? x + m * ldx + k0 + at - sh + 4 * q : x - x_at, 4 * words);
+        }
+    };
+    stage_x(0);
     cp_async_commit();
 #pragma unroll
     for (int b = 0; b < kDepth - 1; ++b) issue(b);
@@ -141,13 +152,27 @@ rows_kernel(const float *__restrict__ x, long long ldx, const float *__restrict_
     for (int j = 0; j < 4; ++j)
 #pragma unroll
         for (int e = 0; e < 4; ++e) acc[j][e] = sum[j][e] = 0.f;
-    for (int b = 0; b < nb; ++b) {
+    // the same for all warps; a slice of one chunk never comes to its end
+    const int rounds = ((kc + 31) / 32 + WK - 1) / WK, chunk_tiles = k_per <= 512 ? rounds : CHUNK / (32 * WK);
+    const float *xr = xs + g * xp + x_shift(g) + kw * 32 + t;
+    int turn = 0, chunk = 0;                                // the tile with which the next chunk of x begins
+    for (int b = 0; b < rounds; ++b, xr += 32 * WK) {
         __syncwarp();                                       // every lane is done with the slot that is filled next
         issue(b + kDepth - 1);
         cp_async_wait<kDepth - 1>();                        // tile b has landed, for this lane ...
+        if (b == turn) {
+            // This chunk of x, staged at least four groups ago, has landed for every thread, and every warp is done with the
+            // chunk before: the next one takes its place, as part of the next tile's group.
+            if (chunk > 0) {
+                __syncthreads();
+                xr += ((chunk & 1) ? kRows * xp : -kRows * xp) - xk;
+            }
+            turn += chunk_tiles;
+            if (++chunk * xk < kc) stage_x(chunk);
+        }
         __syncwarp();                                       // ... and for the others
+        if (WK > 1 && b >= nb) continue;
         const float *slot = mine + (b % kDepth) * (32 * PITCH);
-        const float *xr = xs + g * xp + x_shift(g) + (b * WK + kw) * 32 + t;
         const float *rows = slot + shift_of(DX ? g : t);    // of the row whose elements this lane multiplies
 #pragma unroll
         for (int s = 0; s < 4; ++s) {
@@ -341,18 +366,27 @@ rows_dw_kernel(const float *__restrict__ x, long long ldx, const float *__restri
 
 bool aligned(const void *p, size_t bytes) { return (reinterpret_cast<uintptr_t>(p) & (bytes - 1)) == 0; }
 
-// How a product is cut: strips of 128 outputs, or of 32 where those leave most SMs without a block; about two blocks per
-// SM in all, slices of at least 64 (256 where four warps share one), at most kMaxSlices of them.
+// How a product is cut: strips of 128 outputs, or of 32 where those leave most SMs without a block; slices of at least 64
+// (256 where four warps share one), at most kMaxSlices of them, as many as finish first on two blocks per SM (a block costs
+// about 64 elements more than its slice).  With x staged whole and slices for two blocks per SM on average, 9 rows x 5488 x
+// 7656 ran one block per SM, a few of them in a third round: forward 72.6 -> 47 us, dx 78.6 -> 44.
 struct RowsPlan { int outs, k_per; unsigned strips, slices; };
 RowsPlan plan_rows(int64_t outs, int64_t total, int sm_count) {
-    RowsPlan p;
+    RowsPlan p{};
     p.outs = (outs + 127) / 128 * kMaxSlices >= sm_count ? 128 : 32;
     const int64_t strips = (outs + p.outs - 1) / p.outs;
-    int64_t slices = std::max<int64_t>((total + kMaxSlice - 1) / kMaxSlice, (2LL * sm_count + strips - 1) / strips);
-    slices = std::min<int64_t>({slices, kMaxSlices, std::max<int64_t>(1, total / (p.outs == 128 ? 64 : 256))});
-    p.k_per = static_cast<int>(((total + slices - 1) / slices + 31) / 32 * 32);
+    const int64_t most = std::min<int64_t>(kMaxSlices, std::max<int64_t>(1, total / (p.outs == 128 ? 64 : 256)));
+    int64_t best = 0;
+    for (int64_t n = 1; n <= most; ++n) {
+        const int64_t k_per = ((total + n - 1) / n + 31) / 32 * 32, slices = (total + k_per - 1) / k_per;
+        const int64_t per_sm = p.outs == 128 || k_per <= 512 ? 2 : 1;
+        const int64_t cost = ((strips * slices + per_sm * sm_count - 1) / (per_sm * sm_count)) * per_sm * (k_per + 64);
+        if (best != 0 && cost >= best) continue;
+        best = cost;
+        p.k_per = static_cast<int>(k_per);
+        p.slices = static_cast<unsigned>(slices);
+    }
     p.strips = static_cast<unsigned>(strips);
-    p.slices = static_cast<unsigned>((total + p.k_per - 1) / p.k_per);
     return p;
 }
 
@@ -362,7 +396,8 @@ int launch_rows(const float *x, int64_t ldx, const float *W, int64_t ldw, float 
     const RowsPlan pl = plan_rows(outs, total, sm_count);
     const int k_per = pl.k_per;
     const bool vec = aligned(W, 16) && ldw % 4 == 0 && w_cols % 4 == 0, narrow = pl.outs == 32;
-    const size_t smem = (static_cast<size_t>(kRows) * (k_per + 4) + static_cast<size_t>(kWarps) * kDepth * 32 * (DX ? 36 : 40)) * sizeof(float);
+    const int x_floats = k_per <= 512 ? k_per + 4 : 2 * ((narrow ? kChunkNarrow : kChunk) + 4);
+    const size_t smem = (static_cast<size_t>(kRows) * x_floats + static_cast<size_t>(kWarps) * kDepth * 32 * (DX ? 36 : 40)) * sizeof(float);
     auto kernel = narrow ? (vec ? rows_kernel<DX, true, kWarps> : rows_kernel<DX, false, kWarps>)
                          : (vec ? rows_kernel<DX, true, 1> : rows_kernel<DX, false, 1>);
     static std::atomic<uint64_t> opted_in[2][2];            // per device, as in launch_variant of the tensor path
@@ -403,7 +438,7 @@ int launch_rows(const float *x, int64_t ldx, const float *W, int64_t ldw, float 
 // for the 32-wide ones (measured against the tensor path, 9 rows: 4096 x 4096 18.0 / 20.1 us, 512 x 8192 6.7 / 10.3,
 // 600 x 601 6.2 / 11.9; but 8192 x 512 17.4 / 13.5, 8190 x 1030 41 / 32).
 bool rows_supported(int64_t M, int64_t outs, int64_t total, int sm_count) {
-    return M >= 1 && M <= kRows && total >= 1 && total <= static_cast<int64_t>(kMaxSlice) * kMaxSlices && outs >= 1 &&
+    return M >= 1 && M <= kRows && total >= 1 && total <= kMaxTotal && outs >= 1 &&
            outs <= 0x7fffffffLL && ((outs + 127) / 128 * kMaxSlices >= sm_count || total <= 1024);
 }
 
