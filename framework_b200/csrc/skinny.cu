@@ -369,8 +369,10 @@ skinny_fwd_ring_kernel(const float *__restrict__ x, long long ldx, const float *
     if (threadIdx.x == 0) g_skinny_tickets[blockIdx.x] = 0u;
 }
 
-// grid = (n strips of 512 columns, k slabs).  dy[M, 4 cols] lives in registers; each
-// k row of dW is one float4 store per thread.
+// grid = (n strips of 512 columns, k slabs).  dy[M, 4 cols] lives in registers; each k row of dW is one float4 store per
+// thread.  Rows of dW that are not 16-byte aligned are taken in up to four classes of equal shift, the strip's columns moved
+// back by the shift so that the stores stay whole; a class loads its dy anew, from L1 (word by word stores: 1 row x 4097 x
+// 4097 30 us, 1 x 5486 x 7657 70).
 template <int MT>
 __global__ void __launch_bounds__(kSkinnyThreads)
 skinny_dw_kernel(const float *__restrict__ x, long long ldx, const float *__restrict__ dy, long long lddy,
@@ -385,32 +387,39 @@ skinny_dw_kernel(const float *__restrict__ x, long long ldx, const float *__rest
         xs[kk * MT + m] = m < M ? __ldg(x + m * ldx + k0 + kk) : 0.f;
     }
     __syncthreads();
-    const long long col = (static_cast<long long>(blockIdx.x) * kSkinnyThreads + threadIdx.x) * 4;
-    if (col >= N) return;
-    float g[MT][4];
+    const int classes = (lddw & 3) == 0 ? 1 : (lddw & 1) == 0 ? 2 : 4;
+    for (int cls = 0; cls < classes; ++cls) {
+        const int shift = static_cast<int>(((reinterpret_cast<uintptr_t>(dW) >> 2) + (k0 + cls) * lddw) & 3);
+        const long long col = (static_cast<long long>(blockIdx.x) * kSkinnyThreads + threadIdx.x) * 4 - shift;
+        if (col >= N) continue;
+        float g[MT][4];
 #pragma unroll
-    for (int m = 0; m < MT; ++m)
-        for (int e = 0; e < 4; ++e) g[m][e] = (m < M && col + e < N) ? __ldg(dy + m * lddy + col + e) : 0.f;
-    const bool vec = (col + 3 < N) && ((lddw & 3) == 0) && ((reinterpret_cast<uintptr_t>(dW) & 15) == 0);
-    for (int kk = 0; kk < kc; ++kk) {
-        float o[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int m = 0; m < MT; ++m)
 #pragma unroll
-        for (int m = 0; m < MT; ++m) {
-            const float xv = xs[kk * MT + m];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) o[e] = fmaf(xv, g[m][e], o[e]);
-        }
-        float *dst = dW + (k0 + kk) * lddw + col;
-        if (vec) {
-            float4 v = make_float4(o[0], o[1], o[2], o[3]);
-            if (accumulate) {
-                const float4 old = *reinterpret_cast<const float4 *>(dst);
-                v.x += old.x; v.y += old.y; v.z += old.z; v.w += old.w;
-            }
-            __stcs(reinterpret_cast<float4 *>(dst), v);
-        } else {
             for (int e = 0; e < 4; ++e)
-                if (col + e < N) dst[e] = accumulate ? dst[e] + o[e] : o[e];
+                g[m][e] = (m < M && col + e >= 0 && col + e < N) ? __ldg(dy + m * lddy + col + e) : 0.f;
+        const bool vec = col >= 0 && col + 3 < N;
+        for (int kk = cls; kk < kc; kk += classes) {
+            float o[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int m = 0; m < MT; ++m) {
+                const float xv = xs[kk * MT + m];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) o[e] = fmaf(xv, g[m][e], o[e]);
+            }
+            float *dst = dW + (k0 + kk) * lddw + col;
+            if (vec) {
+                float4 v = make_float4(o[0], o[1], o[2], o[3]);
+                if (accumulate) {
+                    const float4 old = *reinterpret_cast<const float4 *>(dst);
+                    v.x += old.x; v.y += old.y; v.z += old.z; v.w += old.w;
+                }
+                __stcs(reinterpret_cast<float4 *>(dst), v);
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (col + e >= 0 && col + e < N) dst[e] = accumulate ? dst[e] + o[e] : o[e];
+            }
         }
     }
 }
@@ -787,7 +796,8 @@ int launch_skinny_dx(const float *dy, int64_t lddy, const float *W, int64_t ldw,
 int launch_skinny_dw(const float *x, int64_t ldx, const float *dy, int64_t lddy, float *dW, int64_t lddw,
                      bool accumulate, int64_t M, int64_t N, int64_t K, cudaStream_t stream) {
     const int mt = pick_mt(M);
-    const int strips = static_cast<int>((N + 4 * kSkinnyThreads - 1) / (4 * kSkinnyThreads));
+    const int moved = lddw % 4 == 0 && (reinterpret_cast<uintptr_t>(dW) & 15) == 0 ? 0 : 3;      // columns that a shift adds
+    const int strips = static_cast<int>((N + moved + 4 * kSkinnyThreads - 1) / (4 * kSkinnyThreads));
     long long slabs = std::max<long long>(1, (device_sm_count() * 8LL) / strips);
     long long k_per = std::max<long long>(8, (K + slabs - 1) / slabs);
     k_per = std::min<long long>(k_per, 1024);

@@ -58,7 +58,10 @@ def test_few_rows_units_from_before_a_row(F, m, k, n, offset):
     for transposed in (False, True):
         wd = inside(np.ascontiguousarray(w.T), offset).permute((1, 0)) if transposed else inside(w, offset)
         y = F.matmul(inside(x, (offset + 1) % 4), wd)
-        dx, dw = F.matmul_backward(inside(dy, (offset + 2) % 4), inside(x, (offset + 1) % 4), wd)
+        dx, dw = F.DeviceTensor.empty((m, k)), Guarded(F, (k, n), misalign=offset)
+        F.matmul_backward(inside(dy, (offset + 2) % 4), inside(x, (offset + 1) % 4), wd, da=dx, db=dw.tensor)
         F.device_status()
+        dw.check("dw")
+        dw = dw.tensor
         for got, want, length in ((y, x64 @ w64, k), (dx, dy64 @ w64.T, n), (dw, x64.T @ dy64, m)):
             assert rel_fro(got.numpy(), want) <= regression_bound_3xtf32(length)
