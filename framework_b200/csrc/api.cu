@@ -71,8 +71,8 @@ double overlap_work_limit() {
 }
 
 // Row counts up to which the streaming kernels beat the tensor path (measured at K = N = 4096 with a weight
-// that is not in L2: dx 19.4 vs 23.6 us at 5 rows and 31.0 vs 23.7 at 8; dW 13.5 vs 16.9 at 8 rows and 21.8 vs
-// 17.0 at 12).  The forward's limit depends on which of its two kernels can run: skinny_fwd_row_limit.
+// that is not in L2: dx 19.4 vs 23.6 us at 5 rows and 31.0 vs 23.7 at 8; dW 14 vs 16.9 at 8 rows, 15.5 at 12, 20.7 at
+// 15: beyond 8 rows it goes with the rows.cu kernels, whose dx it runs in front of).  The forward's limit depends on which of its two kernels can run: skinny_fwd_row_limit.
 constexpr int64_t kSkinnyDxRows = 5, kSkinnyDwRows = 8;
 
 // Rows up to which the warp-level streaming kernels (rows.cu) take a product the FFMA kernels above do not.  From 16
@@ -670,18 +670,17 @@ int bwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const mni_
                            s.batch == 1 && g_batch == 1 && s.a_batch == 1 && s.b_batch == 1 &&
                            dc->stride[gn - 1] == 1 && b->stride[b->ndim - 1] == 1 && s.K > 1 &&
                            skinny_dx_supported(dc->ptr, dc->stride[gn - 2], b->ptr, b->stride[b->ndim - 2], s.M, s.N);
+    const bool rows_ok = rows_wanted(c.flags, s, *b) && g_batch == 1 && (dc->stride[gn - 1] == 1 || s.N == 1);
     const bool skinny_dw = db_wanted &&
-                           ((c.flags & MNI_B200_FORCE_SKINNY_PATH) != 0 ||
+                           ((c.flags & MNI_B200_FORCE_SKINNY_PATH) != 0 || rows_ok ||
                             ((c.flags & MNI_B200_FORCE_TENSOR_PATH) == 0 && s.M <= kSkinnyDwRows)) &&
                            s.batch == 1 && g_batch == 1 && s.M <= 16 && (a->stride[a->ndim - 1] == 1 || s.K == 1) &&
                            (dc->stride[gn - 1] == 1 || s.N == 1);
 
     // ... and those of the remaining few-row products that stream the weight through the warp-level kernels
-    const bool rows_ok = rows_wanted(c.flags, s, *b) && g_batch == 1 && (dc->stride[gn - 1] == 1 || s.N == 1);
     const int64_t b_sk = b->stride[b->ndim - 2], b_sn = b->stride[b->ndim - 1];
     const bool rows_dx = da_wanted && !skinny_dx && rows_ok && rows_supported(s.M, s.K, s.N, c.st->sm_count) && (b_sn == 1 || b_sk == 1);
-    const bool rows_dw = db_wanted && !skinny_dw && rows_ok && (a->stride[a->ndim - 1] == 1 || s.K == 1);
-    const bool streamed_dx = skinny_dx || rows_dx, streamed_dw = skinny_dw || rows_dw;
+    const bool streamed_dx = skinny_dx || rows_dx, streamed_dw = skinny_dw;
 
     // grad_a and grad_b do not depend on each other.  grad_b of a small problem goes to the library's side stream
     // next to grad_a and is joined before returning (event fork / join, also valid under stream capture).  The
@@ -879,13 +878,6 @@ int bwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const mni_
             if (!c.dry()) {
                 rc = launch_skinny_dw(a_given->ptr, a_given->stride[a_given->ndim - 2], dc_given->ptr, dc_given->stride[gn - 2], db, s.N, acc_db,
                                       s.M, s.N, s.K, c.stream);
-                if (rc) return rc;
-            }
-        } else if (rows_dw) {
-            c.note("streaming (few rows) weight-gradient kernel");
-            if (!c.dry()) {
-                rc = launch_rows_dw(a_given->ptr, a_given->stride[a_given->ndim - 2], dc_given->ptr, dc_given->stride[gn - 2], db,
-                                    s.N, acc_db, s.M, s.N, s.K, c.st->sm_count, c.stream);
                 if (rc) return rc;
             }
         } else {

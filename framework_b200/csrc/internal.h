@@ -197,8 +197,6 @@ using RowsLaunch = int(const float *x, int64_t ldx, const float *W, int64_t ldw,
                        bool accumulate, int64_t M, int64_t N, int64_t K, int sm_count, cudaStream_t stream);
 RowsLaunch launch_rows_fwd, launch_rows_dx;            // W as stored [K, N]
 RowsLaunch launch_rows_bt_fwd, launch_rows_bt_dx;      // W stored [N, K], seen through a transposing view
-int launch_rows_dw(const float *x, int64_t ldx, const float *dy, int64_t lddy, float *dW, int64_t lddw, bool accumulate,
-                   int64_t M, int64_t N, int64_t K, int sm_count, cudaStream_t stream);
 
 // Products too small for the tensor path, all of a call's in one launch (tiny.cu):
 //   c[m, n] = sum_k a[m, k] . b[k, n] (+ bias) (+ c), each operand with a unit stride in one of its dims

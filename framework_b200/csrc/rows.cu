@@ -2,15 +2,14 @@
 //
 //   forward : y[M,N]  = x[M,K] . W[K,N] (+ bias)
 //   dx      : dx[M,K] = dy[M,N] . W[K,N]^T
-//   dW      : dW[K,N] = x[M,K]^T . dy[M,N]
 //
-// Bound by HBM: the weight is read (dW: written) once, 67 MB = 10.3 us at K = N = 4096 of the measured copy rate.  The
+// Bound by HBM: the weight is read once, 67 MB = 10.3 us at K = N = 4096 of the measured copy rate.  The
 // warp-level mma.sync is the right matrix instruction here although tcgen05 is several times faster per SM: the
 // 805 M multiply-adds of 16 rows are 5 us of it spread over the warps that stream the weight, with no tensor memory to
 // allocate, no descriptors, no operand staging beyond the ring and an accumulator that is already in registers.  The
 // tcgen05 path takes the same products in 64-wide tiles with a split contraction and a second kernel that sums it, and
 // gathers a weight with an odd row length into scratch first.  Nine rows x 4096 x 4096: forward 20.1 -> 18.0 us, dx 19.9 ->
-// 18.0, the step 79 -> 55; 4096 x 4095: forward 53 -> 21 us, dx 44 -> 22, the step 153 -> 83.
+// 18.0; 4096 x 4095: forward 53 -> 21 us, dx 44 -> 22.
 //
 // Split as in the tensor path: hi = x with the low 13 mantissa bits cut, lo = x - hi, products lo.hi + hi.lo + hi.hi.
 // A chain in the tensor core's accumulator, which truncates, is kFlush elements long; longer sums are added up in
@@ -26,7 +25,6 @@ namespace {
 
 constexpr int kWarps = 4;                    // each streams 32 x 32 tiles of the weight
 constexpr int kThreads = 32 * kWarps;
-constexpr int kDwCols = 32 * kWarps;         // columns of dW per block
 constexpr int kDepth = 4;                    // 32 x 32 weight tiles held per warp, three in flight: 96 KB per SM with two blocks
 constexpr int kRows = 16;
 constexpr int kFlush = 256;                  // contraction elements summed in one tensor-core accumulator
@@ -266,104 +264,6 @@ rows_kernel(const float *__restrict__ x, long long ldx, const float *__restrict_
     if (ranks > 1) cluster_sync_all();                      // no block leaves while its sums may still be read
 }
 
-// dW[k, n] = sum_m x[m, k] . dy[m, n]: bound by the write of dW.  grid = (strips of 128 columns, slabs of K); a warp keeps
-// the fragments of dy for its 32 columns in registers, walks the slab's rows 16 at a time and writes 32 bytes per
-// thread and row, a warp 128 contiguous bytes of each of eight rows.  WIDTH: floats per store; 1 turns the patch in
-// shared memory first (rows that are not 16-byte aligned).
-constexpr int kSlabRows = 224;               // rows of dW per block at most
-template <int WIDTH>
-__global__ void __launch_bounds__(kThreads)
-rows_dw_kernel(const float *__restrict__ x, long long ldx, const float *__restrict__ dy, long long lddy, float *__restrict__ dW,
-               long long lddw, int accumulate, int M, long long N, long long K, int k_per) {
-    constexpr int XP = kSlabRows + 8;                       // = 8 mod 32: the A fragments' reads hit all banks
-    __shared__ float xs[kRows * XP];
-    __shared__ float patch[WIDTH == 1 ? kWarps * 16 * 33 : 1];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-    const long long k0 = static_cast<long long>(blockIdx.y) * k_per;
-    const int kc = static_cast<int>(min(static_cast<long long>(k_per), K - k0));
-    const long long n0 = static_cast<long long>(blockIdx.x) * kDwCols + warp * 32;
-    grid_dependency_trigger();
-    grid_dependency_wait();
-    for (int m = 0; m < kRows; ++m)
-        for (int k = threadIdx.x; k < XP; k += kThreads) xs[m * XP + k] = (m < M && k < kc) ? __ldg(x + m * ldx + k0 + k) : 0.f;
-    // B fragments: tile j, column g is column 4g + j of the warp's 32; batches t, t + 4 of either half of the rows
-    float b0[2][4], b1[2][4];
-#pragma unroll
-    for (int s = 0; s < 2; ++s)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const long long n = n0 + 4 * g + j;
-            const int m0 = 8 * s + t, m1 = m0 + 4;
-            b0[s][j] = (n < N && m0 < M) ? __ldg(dy + m0 * lddy + n) : 0.f;
-            b1[s][j] = (n < N && m1 < M) ? __ldg(dy + m1 * lddy + n) : 0.f;
-        }
-    __syncthreads();
-    const int halves = M > 8 ? 2 : 1;
-    for (int r0 = 0; r0 < kc; r0 += 16) {
-        float acc[4][4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) acc[j][e] = 0.f;
-#pragma unroll
-        for (int s = 0; s < 2; ++s) {
-            if (s >= halves) break;
-            uint32_t ah[4], al[4];
-            const float *xr = xs + (8 * s + t) * XP + r0 + g;
-            split(xr[0], ah[0], al[0]);
-            split(xr[8], ah[1], al[1]);
-            split(xr[4 * XP], ah[2], al[2]);
-            split(xr[4 * XP + 8], ah[3], al[3]);
-            mma_split(acc, ah, al, b0[s], b1[s]);
-        }
-        if constexpr (WIDTH == 1) {
-            float *mine = patch + warp * (16 * 33);
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    mine[(g + 8 * h) * 33 + 8 * t + j] = acc[j][2 * h];
-                    mine[(g + 8 * h) * 33 + 8 * t + 4 + j] = acc[j][2 * h + 1];
-                }
-            __syncwarp();
-            if (n0 + lane < N) {
-#pragma unroll 4
-                for (int r = 0; r < 16; ++r) {
-                    if (r0 + r >= kc) break;
-                    float *dst = dW + (k0 + r0 + r) * lddw + n0 + lane;
-                    const float v = mine[r * 33 + lane];
-                    __stcs(dst, accumulate ? *dst + v : v);
-                }
-            }
-            __syncwarp();
-        } else
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int r = r0 + g + 8 * h;
-            const long long n = n0 + 8 * t;
-            if (r >= kc || n >= N) continue;
-            float *dst = dW + (k0 + r) * lddw + n;
-            float v[8];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) { v[j] = acc[j][2 * h]; v[4 + j] = acc[j][2 * h + 1]; }
-            const bool second = n + 4 < N;                  // N is a multiple of 4 here
-            if (accumulate) {
-#pragma unroll
-                for (int e = 0; e < 8; ++e)
-                    if (e < 4 || second) v[e] += dst[e];
-            }
-            if (WIDTH == 8 && second) {
-                asm volatile("st.global.cs.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "f"(v[0]), "f"(v[1]),
-                             "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
-                             : "memory");
-            } else {
-                __stcs(reinterpret_cast<float4 *>(dst), make_float4(v[0], v[1], v[2], v[3]));
-                if (second) __stcs(reinterpret_cast<float4 *>(dst + 4), make_float4(v[4], v[5], v[6], v[7]));
-            }
-        }
-    }
-}
-
 bool aligned(const void *p, size_t bytes) { return (reinterpret_cast<uintptr_t>(p) & (bytes - 1)) == 0; }
 
 // How a product is cut: strips of 128 outputs, or of 32 where those leave most SMs without a block; slices of at least 64
@@ -458,21 +358,6 @@ int launch_rows_dx(const float *dy, int64_t lddy, const float *W, int64_t ldw, f
 int launch_rows_bt_dx(const float *dy, int64_t lddy, const float *W, int64_t ldw, float *dx, int64_t lddx, const float *bias,
                       bool accumulate, int64_t M, int64_t N, int64_t K, int sm_count, cudaStream_t stream) {
     return launch_rows<false>(dy, lddy, W, ldw, dx, lddx, bias, accumulate, M, K, N, K, sm_count, stream);
-}
-int launch_rows_dw(const float *x, int64_t ldx, const float *dy, int64_t lddy, float *dW, int64_t lddw, bool accumulate,
-                   int64_t M, int64_t N, int64_t K, int sm_count, cudaStream_t stream) {
-    const int64_t strips = (N + kDwCols - 1) / kDwCols;
-    // about six blocks of 128 threads per SM
-    int64_t k_per = (K * strips + 6LL * sm_count - 1) / (6LL * sm_count);
-    k_per = std::min<int64_t>(kSlabRows, std::max<int64_t>(16, (k_per + 15) / 16 * 16));
-    const dim3 grid(static_cast<unsigned>(strips), static_cast<unsigned>((K + k_per - 1) / k_per));
-    const bool v4 = aligned(dW, 16) && lddw % 4 == 0 && N % 4 == 0, v8 = v4 && aligned(dW, 32) && lddw % 8 == 0;
-    const cudaError_t e = launch_dependent(v8 ? rows_dw_kernel<8> : v4 ? rows_dw_kernel<4> : rows_dw_kernel<1>, grid, dim3(kThreads),
-                                           0, stream, x, ldx, dy, lddy, dW, lddw, accumulate ? 1 : 0, static_cast<int>(M), N, K,
-                                           static_cast<int>(k_per));
-    if (e != cudaSuccess) return fail(MNI_B200_ERR_CUDA, "rows_dw_kernel launch failed: %s", cudaGetErrorString(e));
-    MNI_LAUNCH_CHECK("rows_dw_kernel");
-    return MNI_B200_OK;
 }
 
 }  // namespace mni

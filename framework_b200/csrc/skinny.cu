@@ -369,22 +369,40 @@ skinny_fwd_ring_kernel(const float *__restrict__ x, long long ldx, const float *
     if (threadIdx.x == 0) g_skinny_tickets[blockIdx.x] = 0u;
 }
 
+// acc += a * b for two neighbouring columns, each rounded as fmaf rounds it.
+__device__ __forceinline__ void fma2(unsigned long long &acc, unsigned long long a, unsigned long long b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+    unsigned long long v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+    return v;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+    float2 f;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+    return f;
+}
+
 // grid = (n strips of 512 columns, k slabs).  dy[M, 4 cols] lives in registers; each k row of dW is one float4 store per
-// thread.  Rows of dW that are not 16-byte aligned are taken in up to four classes of equal shift, the strip's columns moved
-// back by the shift so that the stores stay whole; a class loads its dy anew, from L1 (word by word stores: 1 row x 4097 x
-// 4097 30 us, 1 x 5486 x 7657 70).
+// thread.  Bound by the write of dW up to 8 rows (4096 x 4096: 11.9 us at one row, 10.1 of the copy rate); beyond, packed
+// multiply-adds and x stored twice, so that a 16-byte read feeds four of them, keep the issue slots out of the way (9 rows
+// 15.0 us, 15 rows 20.7; warp-level matrix instructions took 21.5 and 24).  Rows of dW that are not 16-byte aligned are
+// taken in up to four classes of equal shift, the strip's columns moved back by the shift so that the stores stay whole; a
+// class loads its dy anew, from L1 (word by word stores: 1 row x 4097 x 4097 30 us against 14.7, 1 x 5486 x 7657 70 / 34).
 template <int MT>
 __global__ void __launch_bounds__(kSkinnyThreads)
 skinny_dw_kernel(const float *__restrict__ x, long long ldx, const float *__restrict__ dy, long long lddy,
                  float *__restrict__ dW, long long lddw, int accumulate, int M, long long N, long long K,
                  long long k_per) {
-    extern __shared__ float xs[];   // [k_per][MT]
+    extern __shared__ __align__(16) float2 xs[];   // [k_per][MT], each element twice: the operand of a packed multiply-add
     const long long k0 = blockIdx.y * k_per;
     const long long k1 = min(K, k0 + k_per);
     const int kc = static_cast<int>(k1 - k0);
     for (int i = threadIdx.x; i < MT * kc; i += kSkinnyThreads) {
         const int kk = i % kc, m = i / kc;
-        xs[kk * MT + m] = m < M ? __ldg(x + m * ldx + k0 + kk) : 0.f;
+        const float v = m < M ? __ldg(x + m * ldx + k0 + kk) : 0.f;
+        xs[kk * MT + m] = make_float2(v, v);
     }
     __syncthreads();
     const int classes = (lddw & 3) == 0 ? 1 : (lddw & 1) == 0 ? 2 : 4;
@@ -392,21 +410,40 @@ skinny_dw_kernel(const float *__restrict__ x, long long ldx, const float *__rest
         const int shift = static_cast<int>(((reinterpret_cast<uintptr_t>(dW) >> 2) + (k0 + cls) * lddw) & 3);
         const long long col = (static_cast<long long>(blockIdx.x) * kSkinnyThreads + threadIdx.x) * 4 - shift;
         if (col >= N) continue;
-        float g[MT][4];
-#pragma unroll
-        for (int m = 0; m < MT; ++m)
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-                g[m][e] = (m < M && col + e >= 0 && col + e < N) ? __ldg(dy + m * lddy + col + e) : 0.f;
+        auto dy_at = [&](int m, int e) { return (m < M && col + e >= 0 && col + e < N) ? __ldg(dy + m * lddy + col + e) : 0.f; };
         const bool vec = col >= 0 && col + 3 < N;
-        for (int kk = cls; kk < kc; kk += classes) {
-            float o[4] = {0.f, 0.f, 0.f, 0.f};
+        const bool dy_vec = (lddy & 3) == 0 && ((reinterpret_cast<uintptr_t>(dy + col)) & 15) == 0;
+        unsigned long long g[MT][2];
 #pragma unroll
-            for (int m = 0; m < MT; ++m) {
-                const float xv = xs[kk * MT + m];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) o[e] = fmaf(xv, g[m][e], o[e]);
+        for (int m = 0; m < MT; ++m) {
+            if (vec && dy_vec) {
+                const float4 v = m < M ? __ldg(reinterpret_cast<const float4 *>(dy + m * lddy + col)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                g[m][0] = pack2(v.x, v.y);
+                g[m][1] = pack2(v.z, v.w);
+            } else {
+                g[m][0] = pack2(dy_at(m, 0), dy_at(m, 1));
+                g[m][1] = pack2(dy_at(m, 2), dy_at(m, 3));
             }
+        }
+        for (int kk = cls; kk < kc; kk += classes) {
+            unsigned long long acc[2] = {0, 0};
+            const float2 *xr = xs + kk * MT;
+            if constexpr (MT == 1) {
+                const unsigned long long xv = *reinterpret_cast<const unsigned long long *>(xr);
+                fma2(acc[0], xv, g[0][0]);
+                fma2(acc[1], xv, g[0][1]);
+            } else {
+#pragma unroll
+                for (int m = 0; m < MT; m += 2) {
+                    const ulonglong2 xv = *reinterpret_cast<const ulonglong2 *>(xr + m);
+                    fma2(acc[0], xv.x, g[m][0]);
+                    fma2(acc[1], xv.x, g[m][1]);
+                    fma2(acc[0], xv.y, g[m + 1][0]);
+                    fma2(acc[1], xv.y, g[m + 1][1]);
+                }
+            }
+            const float2 lo = unpack2(acc[0]), hi = unpack2(acc[1]);
+            const float o[4] = {lo.x, lo.y, hi.x, hi.y};
             float *dst = dW + (k0 + kk) * lddw + col;
             if (vec) {
                 float4 v = make_float4(o[0], o[1], o[2], o[3]);
@@ -795,25 +832,28 @@ int launch_skinny_dx(const float *dy, int64_t lddy, const float *W, int64_t ldw,
 
 int launch_skinny_dw(const float *x, int64_t ldx, const float *dy, int64_t lddy, float *dW, int64_t lddw,
                      bool accumulate, int64_t M, int64_t N, int64_t K, cudaStream_t stream) {
-    const int mt = pick_mt(M);
+    const int mt = M > 8 && M <= 12 ? 12 : pick_mt(M);
     const int moved = lddw % 4 == 0 && (reinterpret_cast<uintptr_t>(dW) & 15) == 0 ? 0 : 3;      // columns that a shift adds
     const int strips = static_cast<int>((N + moved + 4 * kSkinnyThreads - 1) / (4 * kSkinnyThreads));
-    long long slabs = std::max<long long>(1, (device_sm_count() * 8LL) / strips);
+    long long slabs = std::max<long long>(1, static_cast<long long>(device_sm_count()) * (mt > 8 ? 5 : 8) / strips);
     long long k_per = std::max<long long>(8, (K + slabs - 1) / slabs);
-    k_per = std::min<long long>(k_per, 1024);
+    k_per = std::min<long long>(k_per, mt > 8 ? 512 : 1024);
     slabs = (K + k_per - 1) / k_per;
     dim3 grid(strips, static_cast<unsigned>(slabs));
-    const size_t smem = static_cast<size_t>(mt) * k_per * sizeof(float);
-    // launched the ordinary way: its blocks come in several waves, and a dependent's blocks waiting beside them would
+    const size_t smem = static_cast<size_t>(mt) * k_per * sizeof(float2);
+    // 8 blocks per SM, or 5 above 8 rows, as many as are resident then: each block first loads dy (9 rows x 4096 x 4096 15.0 us
+    // at 5, 17.4 at 8; 11 x 5509 x 1792 11.5 / 16.6).
+    // Launched the ordinary way: its blocks come in several waves, and a dependent's blocks waiting beside them would
     // take their places (4096 x 4096, 1 row: 11.9 us this way, 16.6 as a dependent launch)
 #define MNI_SKINNY_DW(MT)                                                                              \
     case MT:                                                                                           \
-        cudaFuncSetAttribute(skinny_dw_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024); \
+        if (smem > 48 * 1024)                                                                          \
+            cudaFuncSetAttribute(skinny_dw_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024); \
         skinny_dw_kernel<MT><<<grid, kSkinnyThreads, smem, stream>>>(x, ldx, dy, lddy, dW, lddw,       \
                                                                      accumulate ? 1 : 0, (int)M, N, K, k_per); \
         break;
     switch (mt) {
-        MNI_SKINNY_DW(1) MNI_SKINNY_DW(2) MNI_SKINNY_DW(4) MNI_SKINNY_DW(8) MNI_SKINNY_DW(16)
+        MNI_SKINNY_DW(1) MNI_SKINNY_DW(2) MNI_SKINNY_DW(4) MNI_SKINNY_DW(8) MNI_SKINNY_DW(12) MNI_SKINNY_DW(16)
     }
 #undef MNI_SKINNY_DW
     MNI_LAUNCH_CHECK("skinny_dw_kernel");
