@@ -1595,6 +1595,7 @@ struct Plan {
     int sk_first_tile;
     double est_us;                                            // the cost model's time for this plan (0: it has none)
     int tail_ways, tail_tiles;                                // split tail: the last wave's tiles, cut into this many units each (0: none)
+    bool running;                                             // units of several pieces are summed in the epilogue's registers
     size_t smem;
 };
 
@@ -1608,6 +1609,13 @@ long long cut_ways(long long tiles, long long slots, long long k) {
     const long long ways = rem > 0 ? std::min<long long>(slots / rem, 4) : 1;
     const double eff = static_cast<double>(tiles) / static_cast<double>((full + 1) * slots);
     return full >= 1 && ways >= 2 && eff < 0.80 && k / ways >= 128 ? ways : 1;
+}
+
+// Longest accumulation chain in tensor memory, in k-blocks (MNI_B200_CHUNK_K contraction elements; 0 = no limit).  The fused
+// activation needs the whole sum in one accumulator.
+int chunk_iters_for(const GemmProblem &p, int bk) {
+    const int chunk_k = env_int("MNI_B200_CHUNK_K", 1024);
+    return (chunk_k > 0 && p.D == nullptr) ? std::max(1, chunk_k / bk) : 0;
 }
 
 Plan make_plan(const GemmProblem &p, int sm_count) {
@@ -1724,6 +1732,7 @@ Plan make_plan(const GemmProblem &p, int sm_count) {
     pl.sk = false;
     pl.sk_first_tile = 0;
     pl.tail_ways = pl.tail_tiles = 0;
+    pl.running = false;
     // MNI_B200_STREAMK=1 turns it on where whole tiles would idle more than 8 % of the slot-rounds.  Off by default: parking
     // and adding the shared tiles costs more than the idle slots at every size measured (24 x [512 x 512 x 64] 19.9 us
     // against 12.4, 6 x 700^3 42.1 / 29.0, 3000 x 1000 x 900 45.8 / 37.7, 1000 x 2000 x 3000 63.8 / 65.4).
@@ -1731,7 +1740,9 @@ Plan make_plan(const GemmProblem &p, int sm_count) {
     const int sk_env = env_int("MNI_B200_STREAMK", -1);
     // The split tail's partial tiles are added by one small kernel.  2048 x 3072, K = 768 (96 tiles on 74 pairs): two
     // rounds 49.7 us, the balanced tail 51.9 (17 of it parking and adding in the last CTAs), this 41.
-    if (splits == 1 && sk_env < 0 && p.force_splits <= 0 && pl.cg == 2 && pl.bn == 256) {
+    // Neither it nor the running sum is built for exchanged operands, whose patches leave transposed (the planner's own
+    // choice there is a 64-wide tile; MNI_B200_BN=256 makes it a 256-wide pair).
+    if (splits == 1 && sk_env < 0 && p.force_splits <= 0 && pl.cg == 2 && pl.bn == 256 && !p.exchanged) {
         const long long ways = cut_ways(tiles, slots, iters * pl.bk);
         if (ways > 1) {
             pl.tail_ways = static_cast<int>(ways);
@@ -1756,6 +1767,10 @@ Plan make_plan(const GemmProblem &p, int sm_count) {
             }
         }
     }
+    // Units summed in several pieces (the kernel's first_piece rule) keep their running sum in registers where that is built.
+    const long long chunk = chunk_iters_for(p, pl.bk), unit_len = (iters + splits - 1) / splits;
+    pl.running = pl.cg == 2 && pl.bn == 256 && pl.bk == (p.fast_tf32 ? 32 : 16) && !pl.sk && !p.exchanged && chunk > 0 &&
+                 unit_len > chunk + (chunk >> 3);
     return pl;
 }
 
@@ -1868,6 +1883,7 @@ GemmProblem kernel_view(const GemmProblem &p, bool *transposed) {
     GemmProblem q = p;
     std::swap(q.A, q.B);
     std::swap(q.M, q.N);
+    q.exchanged = true;
     *transposed = true;
     return q;
 }
@@ -1905,20 +1921,19 @@ std::string gemm_tc_describe(const GemmProblem &p0, int sm_count) {
     bool transposed = false;
     const GemmProblem p = kernel_view(p0, &transposed);
     const Plan pl = make_plan(p, sm_count);
-    const int chunk_k = env_int("MNI_B200_CHUNK_K", 1024);
     // pieces a whole unit's contraction is summed in (the kernel's first_piece rule)
     const long long iters = p.fold * ((p.K + pl.bk - 1) / pl.bk);
     const long long len = (iters + pl.splits - 1) / pl.splits;
-    const long long ci = (chunk_k > 0 && p.D == nullptr) ? std::max(1, chunk_k / pl.bk) : 0;
+    const long long ci = chunk_iters_for(p, pl.bk);
     const int pieces = (ci > 0 && len > ci + ci / 8) ? static_cast<int>((len + ci - 1) / ci) : 1;
     char buf[320];
     snprintf(buf, sizeof(buf),
              "tensor m=%lld n=%lld k=%lld batch=%lld fold=%lld bn=%d bk=%d pair=%d tmem_a=%d stages=%d splits=%d "
-             "tail=%d grid=%d exchanged=%d single_pass=%d pieces=%d mma_n=%d tail_ways=%d",
+             "tail=%d grid=%d exchanged=%d single_pass=%d pieces=%d mma_n=%d tail_ways=%d running=%d",
              static_cast<long long>(p.M), static_cast<long long>(p.N), static_cast<long long>(p.K),
              static_cast<long long>(p.batch), static_cast<long long>(p.fold), pl.bn, pl.bk, pl.cg == 2 ? 1 : 0,
              pl.ta ? 1 : 0, pl.stages, pl.splits, pl.sk || pl.tail_ways ? 1 : 0, pl.grid, transposed ? 1 : 0, p.fast_tf32 ? 1 : 0,
-             pieces, mma_n_for(p, pl), pl.tail_ways);
+             pieces, mma_n_for(p, pl), pl.tail_ways, pl.running ? 1 : 0);
     return buf;
 }
 
@@ -1974,6 +1989,8 @@ int launch_gemm_tc(const GemmProblem &p0, float *partial, uint32_t *err_word, in
     const int64_t oM = p0.M, oN = p0.N;
     const Plan pl = make_plan(p, sm_count);
     if (p.K <= 0) return fail(MNI_B200_ERR_ARG, "empty contraction reached the tensor-core launcher");
+    if (transposed && (pl.tail_ways || pl.running))
+        return fail(MNI_B200_ERR_ARG, "internal: a plan that stores no transposed patches for exchanged operands");
     if ((pl.splits > 1 || pl.sk || pl.tail_ways) && partial == nullptr)
         return fail(MNI_B200_ERR_WORKSPACE, "split-K launch without partial storage");
 
@@ -2040,12 +2057,7 @@ int launch_gemm_tc(const GemmProblem &p0, float *partial, uint32_t *err_word, in
     k.fold = static_cast<int>(p.fold);
     k.splits = pl.splits;
     k.dep_mode = p.dep_mode;
-    {
-        // Longest accumulation chain in tensor memory, in contraction elements (MNI_B200_CHUNK_K, 0 = unlimited).
-        // The fused activation needs the whole sum in one accumulator.
-        const int chunk_k = env_int("MNI_B200_CHUNK_K", 1024);
-        k.chunk_iters = (chunk_k > 0 && p.D == nullptr) ? std::max(1, chunk_k / pl.bk) : 0;
-    }
+    k.chunk_iters = chunk_iters_for(p, pl.bk);
     k.a_batch = static_cast<int>(p.A.batch);
     k.a_d1 = static_cast<int>(p.A.bshape[1]);
     k.a_d2 = static_cast<int>(p.A.bshape[2]);
@@ -2123,11 +2135,7 @@ int launch_gemm_tc(const GemmProblem &p0, float *partial, uint32_t *err_word, in
         const int sg_env = env_int("MNI_B200_SPLIT_GROUPS", 0);
         split_groups = (sg_env == 1 || sg_env == 2) ? sg_env : (unit_iters >= 12 ? 2 : 1);
     }
-    // Units summed in several pieces keep their running sum in registers where that is built (the kernel's first_piece
-    // rule decides what is cut).
-    const long long unit_len = (static_cast<long long>(k.fold) * k.kiters + pl.splits - 1) / pl.splits;
-    const bool running = pl.cg == 2 && pl.bn == 256 && pl.bk == (p.fast_tf32 ? 32 : 16) && !pl.sk && !pl.tail_ways && k.chunk_iters > 0 &&
-                         unit_len > k.chunk_iters + (k.chunk_iters >> 3) && (k.epi_mode == kEpiTmaStore || k.epi_mode == kEpiTmaReduce);
+    const bool running = pl.running && (k.epi_mode == kEpiTmaStore || k.epi_mode == kEpiTmaReduce);
     cudaError_t e = cudaErrorInvalidValue;
     if (pl.sk) {
         if (pl.ta && pl.bn == 64 && split_groups == 2) e = launch_variant<64, 32, false, 8, 1, true, kBalanced, 2>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
@@ -2169,7 +2177,6 @@ int launch_gemm_tc(const GemmProblem &p0, float *partial, uint32_t *err_word, in
 #undef MNI_VARIANT
     if (e != cudaSuccess) return fail(MNI_B200_ERR_CUDA, "gemm_tc_kernel set-up failed: %s", cudaGetErrorString(e));
     MNI_LAUNCH_CHECK("gemm_tc_kernel");
-    // (a split tail only ever comes with whole rows of CTA pairs: its operands are not exchanged)
     if (pl.tail_ways) {
         if (!defer) return launch_tail_finish(p, pl, k, partial, 0, stream);
         *defer = [p, pl, k, partial](int dep_mode, cudaStream_t st) { return launch_tail_finish(p, pl, k, partial, dep_mode, st); };

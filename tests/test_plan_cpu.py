@@ -159,6 +159,21 @@ def test_mma_width_follows_the_output_width(plan):
     assert (wide["bn"], wide["pair"], wide["mma_n"]) == (256, 1, 256)
 
 
+@pytest.mark.parametrize("flags", [0, 1])
+def test_exchanged_operands_keep_to_the_plans_that_store_transposed(plan, monkeypatch, flags):
+    """Few rows and many columns are computed as C^T.  At a forced width of 256 that is a 256-wide pair problem, but the split
+    tail and the running sum store no transposed patches: neither may be planned, whatever the last wave and the contraction."""
+    monkeypatch.setenv("MNI_B200_BN", "256")
+    from framework_b200 import _lib
+    for m, k, n in ((48, 512, 20480), (64, 2048, 20000), (32, 8192, 4096), (32, 8000, 32768), (17, 256, 19200)):
+        f = tensor_plan(plan((m, k), (k, n), flags=flags | _lib.FORCE_TENSOR_PATH), "forward")
+        assert (f["exchanged"], f["bn"], f["pair"], f["tail_ways"], f["running"]) == (1, 256, 1, 0, 0), f
+    plain = tensor_plan(plan((8192, 8192), (8192, 8192), flags=flags), "forward")
+    assert (plain["exchanged"], plain["running"]) == (0, 1)
+    cut = tensor_plan(plan((2048, 768), (768, 3072), flags=flags), "forward")
+    assert (cut["exchanged"], cut["tail_ways"]) == (0, 3)
+
+
 def test_errors_are_the_calls_own(plan):
     from framework_b200 import _lib
     with pytest.raises(_lib.MniError) as ei:

@@ -113,6 +113,20 @@ def test_transposed_output_form_delivers_the_split(F, oracle):
     _assert_separated(e3, e1, k, "transposed output")
 
 
+@pytest.mark.parametrize("m,k,n", [(48, 512, 20480), (32, 4096, 4096)])
+def test_transposed_output_form_in_wide_pairs(F, monkeypatch, m, k, n):
+    """The same at a forced width of 256: a ragged last wave, and a contraction of several pieces."""
+    monkeypatch.setenv("MNI_B200_BN", "256")
+    rng = np.random.default_rng([61, m])
+    a = rng.standard_normal((m, k), dtype=np.float32)
+    b = rng.standard_normal((k, n), dtype=np.float32)
+    out = Guarded(F, (m, n))
+    F.matmul(F.DeviceTensor.from_numpy(a), F.DeviceTensor.from_numpy(b), out=out.tensor, flags=F._lib.FORCE_TENSOR_PATH)
+    F.device_status()
+    out.check()
+    assert rel_fro(out.tensor.numpy(), a.astype(np.float64) @ b.astype(np.float64)) <= regression_bound_3xtf32(k)
+
+
 def test_backward_products_deliver_the_split(F, oracle):
     """dA = dC . B^T (both operands K-major) and dB = A^T . dC (both MN-major), and the weight gradient of a
     broadcast weight, whose batch is folded into the contraction (K' = batch * M)."""
