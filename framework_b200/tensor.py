@@ -8,6 +8,7 @@ to own device memory and to name the current stream.
 """
 from __future__ import annotations
 
+import copyreg
 from typing import Sequence
 
 import numpy as np
@@ -68,6 +69,16 @@ class DeviceTensor(_host.Tensor):
         flat = torch.empty(0, dtype=torch.float32, device=t.device).set_(
             base, t.storage_offset(), (max(_span(t), 1),), (1,))
         return DeviceTensor(flat, tuple(t.shape), tuple(t.stride()))
+
+    # -- copies and checkpoints --------------------------------------------
+    def __reduce_ex__(self, protocol):
+        """copy.copy shares the storage; copy.deepcopy and pickle (torch.save) carry it.  The state is the one a Python class
+        with these three slots has, (instance dictionary or None, slot values), so that files of either kind load."""
+        if protocol < 2:
+            return super().__reduce_ex__(protocol)           # refused, as for any class with slots
+        names = ["storage", "shape", "strides", *copyreg._slotnames(type(self))]
+        slots = {name: getattr(self, name) for name in names if getattr(self, name, None) is not None}
+        return copyreg.__newobj__, (type(self),), (getattr(self, "__dict__", None) or None, slots)
 
     def view_struct(self) -> "_lib.View":
         return _lib.make_view(self.ptr, self.shape, self.strides)
