@@ -432,7 +432,18 @@ bool output(PyObject *given, const Dims &shape, const at::Device &device, const 
     Py_END_ALLOW_THREADS                    \
     if (!check(rc)) return nullptr
 
-uint32_t flags_of(PyObject *o) { return static_cast<uint32_t>(PyLong_AsUnsignedLongMask(o)); }
+// Flags and truth values.  Anything else than a number (or a value without a truth) is an error before anything is launched.
+bool parse_flags(PyObject *o, uint32_t &out) {
+    const unsigned long v = PyLong_AsUnsignedLongMask(o);
+    if (v == static_cast<unsigned long>(-1) && PyErr_Occurred()) return false;
+    out = static_cast<uint32_t>(v);
+    return true;
+}
+bool parse_truth(PyObject *o, bool &out) {
+    const int v = PyObject_IsTrue(o);
+    out = v == 1;
+    return v >= 0;
+}
 
 // matmul(a, b, bias, flags, out)
 PyObject *op_matmul(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
@@ -440,7 +451,8 @@ PyObject *op_matmul(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     TENSOR(a, 0, "a");
     TENSOR(b, 1, "b");
     Dims shape;
-    if (!product_shape(a, b, shape)) return nullptr;
+    uint32_t flags;
+    if (!product_shape(a, b, shape) || !parse_flags(args[3], flags)) return nullptr;
     TensorObj *bias = nullptr;
     if (args[2] != Py_None) {
         bias = as_tensor(args[2], "bias");
@@ -460,7 +472,6 @@ PyObject *op_matmul(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     if (!make_view(a, va) || !make_view(b, vb)) return nullptr;
     float *c = data(out.t);
     const float *bias_ptr = bias ? data(bias) : nullptr;
-    const uint32_t flags = flags_of(args[3]);
     void *stream = current_stream();
     CALL(g_api.matmul_fwd(&va, &vb, c, bias_ptr, flags, stream));
     return out.release();
@@ -481,8 +492,11 @@ PyObject *op_matmul_backward(PyObject *, PyObject *const *args, Py_ssize_t nargs
         Py_XDECREF(want);
         return nullptr;
     }
-    const bool need_da = PyObject_IsTrue(args[4]) == 1, need_db = PyObject_IsTrue(args[5]) == 1;
-    const bool want_dbias = PyObject_IsTrue(args[6]) == 1;
+    uint32_t flags;
+    bool need_da, need_db, want_dbias;
+    if (!parse_flags(args[3], flags) || !parse_truth(args[4], need_da) || !parse_truth(args[5], need_db) ||
+        !parse_truth(args[6], want_dbias))
+        return nullptr;
     const at::Device device = a->flat.device();
     Ref da, db, dbias;
     if (need_da && !output(args[7], a->shape, device, "da", da)) return nullptr;
@@ -491,7 +505,6 @@ PyObject *op_matmul_backward(PyObject *, PyObject *const *args, Py_ssize_t nargs
     mni_b200_view va, vb, vg;
     if (!make_view(a, va) || !make_view(b, vb) || !make_view(grad, vg)) return nullptr;
     float *pa = da ? data(da.t) : nullptr, *pb = db ? data(db.t) : nullptr, *pbias = dbias ? data(dbias.t) : nullptr;
-    const uint32_t flags = flags_of(args[3]);
     void *stream = current_stream();
     CALL(g_api.matmul_bwd(&va, &vb, &vg, pa, pb, pbias, flags, stream));
     // a gradient that is not needed comes back as it was passed in
@@ -543,7 +556,8 @@ PyObject *op_add_backward(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     ARGS(4, "add_backward(grad, a_shape, b_shape, flags)");
     TENSOR(grad, 0, "grad");
     Dims a_shape, b_shape;
-    if (!parse_ints(args[1], a_shape) || !parse_ints(args[2], b_shape)) return nullptr;
+    uint32_t flags;
+    if (!parse_ints(args[1], a_shape) || !parse_ints(args[2], b_shape) || !parse_flags(args[3], flags)) return nullptr;
     if (grad->shape != a_shape || b_shape.size() != 1 || grad->shape.empty() || b_shape[0] != grad->shape.back()) {
         PyErr_SetString(PyExc_NotImplementedError, "only the Linear bias add ([..., N] + [N]) is on this path");
         return nullptr;
@@ -555,7 +569,6 @@ PyObject *op_add_backward(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     const float *pg = data(g.t);
     float *pa = data(ga.t), *pb = data(gb.t);
     const int64_t rows = leading_rows(a_shape), n = b_shape[0];
-    const uint32_t flags = flags_of(args[3]);
     void *stream = current_stream();
     CALL(g_api.add_bias_bwd(pg, pa, pb, rows, n, flags, stream));
     return pair_of(ga, gb);
@@ -592,6 +605,8 @@ PyObject *op_bias_gelu_backward(PyObject *, PyObject *const *args, Py_ssize_t na
         PyErr_SetString(PyExc_ValueError, "grad must have x's shape and bias must be [C]");
         return nullptr;
     }
+    uint32_t flags;
+    if (!parse_flags(args[3], flags)) return nullptr;
     Ref g(contiguous_of(g0)), x(g ? contiguous_of(x0) : nullptr), b(x ? contiguous_of(b0) : nullptr);
     if (!g || !x || !b) return nullptr;
     const at::Device device = x.t->flat.device();
@@ -600,7 +615,6 @@ PyObject *op_bias_gelu_backward(PyObject *, PyObject *const *args, Py_ssize_t na
     const float *pg = data(g.t), *px = data(x.t), *pb = data(b.t);
     float *pdx = data(dx.t), *pdb = data(dbias.t);
     const int64_t rows = leading_rows(x.t->shape), n = x.t->shape.back();
-    const uint32_t flags = flags_of(args[3]);
     void *stream = current_stream();
     CALL(g_api.bias_gelu_bwd(pg, px, pb, pdx, pdb, rows, n, flags, stream));
     return pair_of(dx, dbias);
@@ -618,7 +632,9 @@ PyObject *op_matmul_bias_gelu(PyObject *, PyObject *const *args, Py_ssize_t narg
         PyErr_SetString(PyExc_ValueError, "bias must be a contiguous [N] vector");
         return nullptr;
     }
-    const bool want_pre = PyObject_IsTrue(args[4]) == 1;
+    uint32_t flags;
+    bool want_pre;
+    if (!parse_flags(args[3], flags) || !parse_truth(args[4], want_pre)) return nullptr;
     Ref pre, out;
     if (want_pre) {
         pre.reset(new_tensor(shape, a->flat.device()));
@@ -630,7 +646,6 @@ PyObject *op_matmul_bias_gelu(PyObject *, PyObject *const *args, Py_ssize_t narg
     if (!make_view(a, va) || !make_view(b, vb)) return nullptr;
     const float *pb = data(bias);
     float *pp = pre ? data(pre.t) : nullptr, *po = data(out.t);
-    const uint32_t flags = flags_of(args[3]);
     void *stream = current_stream();
     CALL(g_api.matmul_bias_gelu_fwd(&va, &vb, pb, pp, po, flags, stream));
     PyObject *tuple = PyTuple_New(2);
