@@ -76,6 +76,26 @@ bool check(int status) {
 
 void *current_stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 
+// A C++ exception (torch's: no driver, no device, out of memory) becomes a Python one instead of ending the process.
+template <PyObject *(*FN)(PyObject *, PyObject *)>
+PyObject *guarded(PyObject *self, PyObject *arg) {
+    try {
+        return FN(self, arg);
+    } catch (...) {
+        torch::translate_exception_to_python(std::current_exception());
+        return nullptr;
+    }
+}
+template <PyObject *(*FN)(PyObject *, PyObject *const *, Py_ssize_t)>
+PyObject *guarded_fast(PyObject *self, PyObject *const *args, Py_ssize_t nargs) {
+    try {
+        return FN(self, args, nargs);
+    } catch (...) {
+        torch::translate_exception_to_python(std::current_exception());
+        return nullptr;
+    }
+}
+
 // ------------------------------------------------------------------ tensor object
 bool row_major(const Dims &shape, const Dims &stride) {
     if (shape.size() != stride.size()) return false;
@@ -101,6 +121,12 @@ void set_row_major(TensorObj *t) {
     t->contiguous = true;
 }
 float *data(const TensorObj *t) { return static_cast<float *>(t->flat.data_ptr()); }
+// Whether the tensor has been given its storage (an object that was created without being initialised has none).
+bool has_storage(const TensorObj *t) {
+    if (t->flat.defined()) return true;
+    PyErr_SetString(PyExc_AttributeError, "storage");
+    return false;
+}
 
 bool parse_ints(PyObject *seq, Dims &out) {
     PyObject *fast = PySequence_Fast(seq, "expected a sequence of integers");
@@ -207,7 +233,8 @@ TensorObj *as_tensor(PyObject *o, const char *what) {
         PyErr_Format(PyExc_TypeError, "%s must be a DeviceTensor, not %s", what, Py_TYPE(o)->tp_name);
         return nullptr;
     }
-    return reinterpret_cast<TensorObj *>(o);
+    TensorObj *t = reinterpret_cast<TensorObj *>(o);
+    return has_storage(t) ? t : nullptr;
 }
 
 bool make_view(const TensorObj *t, mni_b200_view &v) {
@@ -229,7 +256,8 @@ bool make_view(const TensorObj *t, mni_b200_view &v) {
 
 // ------------------------------------------------------------------ tensor methods
 PyObject *get_storage(PyObject *self, void *) {
-    return THPVariable_Wrap(reinterpret_cast<TensorObj *>(self)->flat);
+    TensorObj *t = reinterpret_cast<TensorObj *>(self);
+    return has_storage(t) ? THPVariable_Wrap(t->flat) : nullptr;
 }
 int put_storage(PyObject *self, PyObject *value, void *) {
     if (!value) { PyErr_SetString(PyExc_AttributeError, "storage cannot be deleted"); return -1; }
@@ -254,7 +282,10 @@ PyObject *get_size(PyObject *self, void *) { return PyLong_FromLongLong(numel(re
 PyObject *get_ndim(PyObject *self, void *) {
     return PyLong_FromSize_t(reinterpret_cast<TensorObj *>(self)->shape.size());
 }
-PyObject *get_ptr(PyObject *self, void *) { return PyLong_FromVoidPtr(data(reinterpret_cast<TensorObj *>(self))); }
+PyObject *get_ptr(PyObject *self, void *) {
+    TensorObj *t = reinterpret_cast<TensorObj *>(self);
+    return has_storage(t) ? PyLong_FromVoidPtr(data(t)) : nullptr;
+}
 PyObject *is_contiguous(PyObject *self, PyObject *) {
     return PyBool_FromLong(reinterpret_cast<TensorObj *>(self)->contiguous);
 }
@@ -288,14 +319,14 @@ PyObject *permuted(TensorObj *t, const Dims &dims) {
 }
 PyObject *permute(PyObject *self, PyObject *arg) {
     Dims dims;
-    if (!parse_ints(arg, dims)) return nullptr;
+    if (!has_storage(reinterpret_cast<TensorObj *>(self)) || !parse_ints(arg, dims)) return nullptr;
     return permuted(reinterpret_cast<TensorObj *>(self), dims);
 }
 
 // New reference to `t` itself when it is contiguous, else to a gathered copy.
 TensorObj *contiguous_of(TensorObj *t) {
     if (t->contiguous) { Py_INCREF(t); return t; }
-    if (!ensure_bound()) return nullptr;
+    if (!has_storage(t) || !ensure_bound()) return nullptr;
     TensorObj *out = new_tensor(t->shape, t->flat.device());
     mni_b200_view v;
     if (!out || !make_view(t, v)) { Py_XDECREF(out); return nullptr; }
@@ -361,8 +392,8 @@ PyGetSetDef tensor_getset[] = {
     {nullptr, nullptr, nullptr, nullptr, nullptr}};
 PyMethodDef tensor_methods[] = {
     {"is_contiguous", is_contiguous, METH_NOARGS, "whether the strides are row-major (tensor.rs:77-89)"},
-    {"permute", permute, METH_O, "stride-only permutation sharing the storage (no kernel, no copy)"},
-    {"contiguous", contiguous, METH_NOARGS, "the tensor itself, or a device gather of it (ops/layout.rs:218-231)"},
+    {"permute", guarded<permute>, METH_O, "stride-only permutation sharing the storage (no kernel, no copy)"},
+    {"contiguous", guarded<contiguous>, METH_NOARGS, "the tensor itself, or a device gather of it (ops/layout.rs:218-231)"},
     {nullptr, nullptr, 0, nullptr}};
 PyTypeObject tensor_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
 
@@ -448,11 +479,12 @@ bool parse_truth(PyObject *o, bool &out) {
 // matmul(a, b, bias, flags, out)
 PyObject *op_matmul(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     ARGS(5, "matmul(a, b, bias, flags, out)");
+    uint32_t flags;
+    if (!parse_flags(args[3], flags)) return nullptr;
     TENSOR(a, 0, "a");
     TENSOR(b, 1, "b");
     Dims shape;
-    uint32_t flags;
-    if (!product_shape(a, b, shape) || !parse_flags(args[3], flags)) return nullptr;
+    if (!product_shape(a, b, shape)) return nullptr;
     TensorObj *bias = nullptr;
     if (args[2] != Py_None) {
         bias = as_tensor(args[2], "bias");
@@ -480,6 +512,11 @@ PyObject *op_matmul(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
 // matmul_backward(grad, a, b, flags, need_da, need_db, want_dbias, da, db, dbias)
 PyObject *op_matmul_backward(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     ARGS(10, "matmul_backward(grad, a, b, flags, need_da, need_db, want_dbias, da, db, dbias)");
+    uint32_t flags;
+    bool need_da, need_db, want_dbias;
+    if (!parse_flags(args[3], flags) || !parse_truth(args[4], need_da) || !parse_truth(args[5], need_db) ||
+        !parse_truth(args[6], want_dbias))
+        return nullptr;
     TENSOR(grad, 0, "grad");
     TENSOR(a, 1, "a");
     TENSOR(b, 2, "b");
@@ -492,11 +529,6 @@ PyObject *op_matmul_backward(PyObject *, PyObject *const *args, Py_ssize_t nargs
         Py_XDECREF(want);
         return nullptr;
     }
-    uint32_t flags;
-    bool need_da, need_db, want_dbias;
-    if (!parse_flags(args[3], flags) || !parse_truth(args[4], need_da) || !parse_truth(args[5], need_db) ||
-        !parse_truth(args[6], want_dbias))
-        return nullptr;
     const at::Device device = a->flat.device();
     Ref da, db, dbias;
     if (need_da && !output(args[7], a->shape, device, "da", da)) return nullptr;
@@ -554,10 +586,11 @@ PyObject *op_add(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
 // add_backward(grad, a_shape, b_shape, flags)
 PyObject *op_add_backward(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     ARGS(4, "add_backward(grad, a_shape, b_shape, flags)");
+    uint32_t flags;
+    if (!parse_flags(args[3], flags)) return nullptr;
     TENSOR(grad, 0, "grad");
     Dims a_shape, b_shape;
-    uint32_t flags;
-    if (!parse_ints(args[1], a_shape) || !parse_ints(args[2], b_shape) || !parse_flags(args[3], flags)) return nullptr;
+    if (!parse_ints(args[1], a_shape) || !parse_ints(args[2], b_shape)) return nullptr;
     if (grad->shape != a_shape || b_shape.size() != 1 || grad->shape.empty() || b_shape[0] != grad->shape.back()) {
         PyErr_SetString(PyExc_NotImplementedError, "only the Linear bias add ([..., N] + [N]) is on this path");
         return nullptr;
@@ -598,6 +631,8 @@ PyObject *op_bias_gelu(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
 // bias_gelu_backward(grad, x, bias, flags)
 PyObject *op_bias_gelu_backward(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     ARGS(4, "bias_gelu_backward(grad, x, bias, flags)");
+    uint32_t flags;
+    if (!parse_flags(args[3], flags)) return nullptr;
     TENSOR(g0, 0, "grad");
     TENSOR(x0, 1, "x");
     TENSOR(b0, 2, "bias");
@@ -605,8 +640,6 @@ PyObject *op_bias_gelu_backward(PyObject *, PyObject *const *args, Py_ssize_t na
         PyErr_SetString(PyExc_ValueError, "grad must have x's shape and bias must be [C]");
         return nullptr;
     }
-    uint32_t flags;
-    if (!parse_flags(args[3], flags)) return nullptr;
     Ref g(contiguous_of(g0)), x(g ? contiguous_of(x0) : nullptr), b(x ? contiguous_of(b0) : nullptr);
     if (!g || !x || !b) return nullptr;
     const at::Device device = x.t->flat.device();
@@ -623,6 +656,9 @@ PyObject *op_bias_gelu_backward(PyObject *, PyObject *const *args, Py_ssize_t na
 // matmul_bias_gelu(a, b, bias, flags, want_pre)
 PyObject *op_matmul_bias_gelu(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     ARGS(5, "matmul_bias_gelu(a, b, bias, flags, want_pre)");
+    uint32_t flags;
+    bool want_pre;
+    if (!parse_flags(args[3], flags) || !parse_truth(args[4], want_pre)) return nullptr;
     TENSOR(a, 0, "a");
     TENSOR(b, 1, "b");
     TENSOR(bias, 2, "bias");
@@ -632,9 +668,6 @@ PyObject *op_matmul_bias_gelu(PyObject *, PyObject *const *args, Py_ssize_t narg
         PyErr_SetString(PyExc_ValueError, "bias must be a contiguous [N] vector");
         return nullptr;
     }
-    uint32_t flags;
-    bool want_pre;
-    if (!parse_flags(args[3], flags) || !parse_truth(args[4], want_pre)) return nullptr;
     Ref pre, out;
     if (want_pre) {
         pre.reset(new_tensor(shape, a->flat.device()));
@@ -849,11 +882,11 @@ PyObject *bind(PyObject *, PyObject *table) {
 
 PyObject *raw_stream(PyObject *, PyObject *) { return PyLong_FromVoidPtr(current_stream()); }
 
-#define FAST(name, fn, doc) {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(fn)), METH_FASTCALL, doc}
+#define FAST(name, fn, doc) {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(guarded_fast<fn>)), METH_FASTCALL, doc}
 PyMethodDef module_methods[] = {
     FAST("setup", setup, "registers the Python side"),
     {"bind", bind, METH_O, "binds the library's entry points"},
-    {"current_stream", raw_stream, METH_NOARGS, "address of the current CUDA stream of the current device"},
+    {"current_stream", guarded<raw_stream>, METH_NOARGS, "address of the current CUDA stream of the current device"},
     FAST("empty", empty, "uninitialised row-major tensor"),
     FAST("matmul", op_matmul, "ops.matmul"),
     FAST("matmul_backward", op_matmul_backward, "ops.matmul_backward"),

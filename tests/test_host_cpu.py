@@ -42,3 +42,25 @@ def test_switches_without_a_truth_value(F):
             F.matmul_backward(y, x, w, **{kw: NoTruth()})
     with pytest.raises(RuntimeError, match="no truth value"):
         F.matmul_bias_gelu(x, w, b, want_pre=NoTruth())
+
+
+def test_tensor_without_storage(F):
+    """An object that was never initialised has no `storage`: every use says so, none ends the process."""
+    t, v = bare(F, (4, 4)), bare(F, (4,))
+    uses = [lambda: t.storage, lambda: t.ptr, lambda: t.permute((1, 0)), lambda: t.numpy(), lambda: F.matmul(t, t),
+            lambda: F.matmul_backward(t, t, t), lambda: F.matmul_bias_gelu(t, t, v), lambda: F.add(t, v),
+            lambda: F.add_backward(t, (4, 4), (4,)), lambda: F.bias_gelu(t, v), lambda: F.bias_gelu_backward(t, t, v),
+            lambda: F.softmax(t), lambda: F.softmax_backward(t, t), lambda: F.permute_backward(t, (1, 0), (4, 4)),
+            lambda: F.clip_and_step([t], [t], [t], [t], lr=1e-3)]
+    for use in uses:
+        with pytest.raises(AttributeError, match="storage"):
+            use()
+
+
+def test_no_device_is_an_error_not_an_abort(F):
+    import torch
+    if torch.cuda.is_available():
+        pytest.skip("there is a device")
+    for use in (lambda: F.device_status(), lambda: F.tensor.current_stream(), lambda: F.DeviceTensor.empty((2, 2))):
+        with pytest.raises(RuntimeError):
+            use()
