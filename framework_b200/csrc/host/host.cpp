@@ -249,7 +249,7 @@ bool make_view(const TensorObj *t, mni_b200_view &v) {
     v.ndim = static_cast<int32_t>(t->shape.size());
     for (int i = 0; i < v.ndim; ++i) {
         v.shape[i] = t->shape[static_cast<size_t>(i)];
-        v.stride[i] = t->stride[static_cast<size_t>(i)];
+        v.stride[i] = static_cast<size_t>(i) < t->stride.size() ? t->stride[static_cast<size_t>(i)] : 0;   // none given: 0
     }
     return true;
 }
@@ -303,6 +303,10 @@ PyObject *permuted(TensorObj *t, const Dims &dims) {
         if (list) PyErr_Format(PyExc_ValueError, "invalid permutation %R", list);
         Py_XDECREF(list);
         Py_XDECREF(given);
+        return nullptr;
+    }
+    if (t->stride.size() < nd) {
+        PyErr_SetString(PyExc_IndexError, "the tensor has fewer strides than dimensions");
         return nullptr;
     }
     TensorObj *r = alloc_tensor(g_class);

@@ -52,3 +52,21 @@ def test_copies_and_checkpoints_keep_layout_and_contents(F):
         assert u.shape == t.shape and u.strides == t.strides and np.array_equal(u.numpy(), want)
     deep.storage.zero_()
     assert np.array_equal(t.numpy(), want)
+
+
+@pytest.mark.gpu
+def test_fewer_strides_than_dimensions(F):
+    """A dimension without a stride is not advanced along; there is nothing to permute it with."""
+    import torch
+    flat = torch.arange(16, dtype=torch.float32, device="cuda")
+    t = F.DeviceTensor(flat, (4, 4), (1,))
+    assert np.array_equal(t.contiguous().numpy(), np.repeat(np.arange(4, dtype=np.float32)[:, None], 4, 1))
+    with pytest.raises(IndexError):
+        t.permute((1, 0))
+    u = F.DeviceTensor(flat, (16,))
+    u.shape = (4, 4)                    # the strides are those of before
+    assert not u.is_contiguous()
+    with pytest.raises(IndexError):
+        u.permute((1, 0))
+    u.strides = (4, 1)
+    assert u.is_contiguous() and np.array_equal(u.numpy(), flat.cpu().numpy().reshape(4, 4))
