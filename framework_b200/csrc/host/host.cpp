@@ -128,7 +128,10 @@ bool has_storage(const TensorObj *t) {
     return false;
 }
 
-bool parse_ints(PyObject *seq, Dims &out) {
+// How an item that is no int becomes one: as int() does (extents and strides of a new tensor), as an index (dimensions), or only
+// if it equals one (a shape that is compared with a tensor's; -1, which no extent is, if it does not).
+enum class Ints { kConvert, kIndex, kEqual };
+bool parse_ints(PyObject *seq, Dims &out, Ints how = Ints::kConvert) {
     PyObject *fast = PySequence_Fast(seq, "expected a sequence of integers");
     if (!fast) return false;
     const Py_ssize_t n = PySequence_Fast_GET_SIZE(fast);
@@ -139,10 +142,13 @@ bool parse_ints(PyObject *seq, Dims &out) {
         if (PyLong_CheckExact(item)) {
             v = PyLong_AsLongLong(item);
         } else {
-            PyObject *as_int = PyNumber_Long(item);
+            PyObject *as_int = how == Ints::kIndex ? PyNumber_Index(item) : PyNumber_Long(item);
             if (!as_int) { Py_DECREF(fast); return false; }
             v = PyLong_AsLongLong(as_int);
+            const int equal = how == Ints::kEqual ? PyObject_RichCompareBool(as_int, item, Py_EQ) : 1;
             Py_DECREF(as_int);
+            if (equal < 0) { Py_DECREF(fast); return false; }
+            if (equal == 0) v = -1;
         }
         if (v == -1 && PyErr_Occurred()) { Py_DECREF(fast); return false; }
         out[static_cast<size_t>(i)] = v;
@@ -323,7 +329,7 @@ PyObject *permuted(TensorObj *t, const Dims &dims) {
 }
 PyObject *permute(PyObject *self, PyObject *arg) {
     Dims dims;
-    if (!has_storage(reinterpret_cast<TensorObj *>(self)) || !parse_ints(arg, dims)) return nullptr;
+    if (!has_storage(reinterpret_cast<TensorObj *>(self)) || !parse_ints(arg, dims, Ints::kIndex)) return nullptr;
     return permuted(reinterpret_cast<TensorObj *>(self), dims);
 }
 
@@ -594,7 +600,7 @@ PyObject *op_add_backward(PyObject *, PyObject *const *args, Py_ssize_t nargs) {
     if (!parse_flags(args[3], flags)) return nullptr;
     TENSOR(grad, 0, "grad");
     Dims a_shape, b_shape;
-    if (!parse_ints(args[1], a_shape) || !parse_ints(args[2], b_shape)) return nullptr;
+    if (!parse_ints(args[1], a_shape, Ints::kEqual) || !parse_ints(args[2], b_shape, Ints::kEqual)) return nullptr;
     if (grad->shape != a_shape || b_shape.size() != 1 || grad->shape.empty() || b_shape[0] != grad->shape.back()) {
         PyErr_SetString(PyExc_NotImplementedError, "only the Linear bias add ([..., N] + [N]) is on this path");
         return nullptr;
@@ -755,7 +761,7 @@ PyObject *op_permute_backward(PyObject *, PyObject *const *args, Py_ssize_t narg
     ARGS(3, "permute_backward(grad, dims, orig_shape)");
     TENSOR(grad, 0, "grad");
     Dims dims, orig;
-    if (!parse_ints(args[1], dims) || !parse_ints(args[2], orig)) return nullptr;
+    if (!parse_ints(args[1], dims, Ints::kIndex) || !parse_ints(args[2], orig, Ints::kEqual)) return nullptr;
     const size_t nd = dims.size();
     bool ok = grad->shape.size() == nd;
     Dims inverse, want;

@@ -70,3 +70,20 @@ def test_fewer_strides_than_dimensions(F):
         u.permute((1, 0))
     u.strides = (4, 1)
     assert u.is_contiguous() and np.array_equal(u.numpy(), flat.cpu().numpy().reshape(4, 4))
+
+
+@pytest.mark.gpu
+def test_dimensions_and_shapes_that_are_no_integers(F):
+    t, y = F.DeviceTensor.empty((2, 3)), F.DeviceTensor.empty((2, 3))
+    for dims in ((1.5, 0), (1.0, 0.0), ("1", "0"), (None, 0)):
+        with pytest.raises(TypeError):
+            t.permute(dims)
+        with pytest.raises(TypeError):
+            F.permute_backward(t, dims, (3, 2))
+    assert t.permute((np.int64(1), 0)).shape == (3, 2)
+    assert F.permute_backward(t, (1, 0), (3.0, 2)).shape == (3, 2)
+    with pytest.raises(ValueError):
+        F.permute_backward(t, (1, 0), (3.5, 2))
+    assert F.add_backward(y, (2.0, 3), (3,))[0].shape == (2, 3)
+    with pytest.raises(NotImplementedError):
+        F.add_backward(y, (2.5, 3), (3,))
