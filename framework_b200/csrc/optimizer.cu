@@ -11,7 +11,9 @@
 #include <string.h>
 
 #include <algorithm>
-#include <mutex>
+#include <iterator>
+#include <map>
+#include <vector>
 
 namespace mni {
 
@@ -247,6 +249,63 @@ int launch_norm(int count, const float *const *grad, const int64_t *n, double *o
     return MNI_B200_OK;
 }
 
+// Memory that the step of entry `entry` writes.
+struct Span { uintptr_t begin, end; int64_t entry; };
+
+// Whether the steps of two entries touch the same memory.  A model's tensors mostly come in the order of their addresses: four
+// sorted runs that only need merging.
+bool entries_overlap(int64_t count, float *const *const (&arrays)[4], const int64_t *n) {
+    std::vector<Span> spans;
+    spans.reserve(static_cast<size_t>(4 * count));
+    auto less = [](const Span &a, const Span &b) { return a.begin < b.begin; };
+    std::ptrdiff_t runs[5] = {0, 0, 0, 0, 0};
+    for (int k = 0; k < 4; ++k) {
+        for (int64_t i = 0; i < count; ++i) {
+            const uintptr_t at = reinterpret_cast<uintptr_t>(arrays[k][i]);
+            if (n[i] > 0) spans.push_back(Span{at, at + static_cast<uintptr_t>(n[i]) * sizeof(float), i});
+        }
+        runs[k + 1] = static_cast<std::ptrdiff_t>(spans.size());
+        const auto first = spans.begin() + runs[k];
+        if (!std::is_sorted(first, spans.end(), less)) std::sort(first, spans.end(), less);
+    }
+    const auto at = spans.begin();
+    std::inplace_merge(at, at + runs[1], at + runs[2], less);
+    std::inplace_merge(at + runs[2], at + runs[3], at + runs[4], less);
+    std::inplace_merge(at, at + runs[2], at + runs[4], less);
+    Span reach{0, 0, -1};
+    for (const Span &s : spans) {
+        if (s.begin < reach.end && s.entry != reach.entry) return true;
+        if (s.end > reach.end) reach = s;
+    }
+    return false;
+}
+
+// How many entries from the start of the list one launch may take: up to the first that touches what an earlier one writes.
+int64_t disjoint_entries(int64_t count, float *const *const (&arrays)[4], const int64_t *n) {
+    std::map<uintptr_t, uintptr_t> taken;                     // begin -> end, disjoint
+    for (int64_t i = 0; i < count; ++i) {
+        if (n[i] == 0) continue;
+        Span own[4];
+        for (int k = 0; k < 4; ++k) {
+            const uintptr_t at = reinterpret_cast<uintptr_t>(arrays[k][i]);
+            own[k] = Span{at, at + static_cast<uintptr_t>(n[i]) * sizeof(float), i};
+        }
+        std::sort(own, own + 4, [](const Span &a, const Span &b) { return a.begin < b.begin; });
+        int parts = 1;                                        // an entry's own arrays may overlap
+        for (int k = 1; k < 4; ++k) {
+            if (own[k].begin < own[parts - 1].end) own[parts - 1].end = std::max(own[parts - 1].end, own[k].end);
+            else own[parts++] = own[k];
+        }
+        for (int k = 0; k < parts; ++k) {
+            const auto next = taken.upper_bound(own[k].begin);
+            if (next != taken.end() && next->first < own[k].end) return i;
+            if (next != taken.begin() && std::prev(next)->second > own[k].begin) return i;
+        }
+        for (int k = 0; k < parts; ++k) taken[own[k].begin] = own[k].end;
+    }
+    return count;
+}
+
 }  // namespace
 
 double *norm_sumsq_ptr() {
@@ -254,10 +313,19 @@ double *norm_sumsq_ptr() {
     return cudaGetSymbolAddress(&p, g_norm_sumsq) == cudaSuccess ? static_cast<double *>(p) : nullptr;
 }
 
+// Entries that touch the same memory (tied parameters given twice) are stepped one after the other, in list order: the blocks of
+// one launch run in any order, so a launch ends before an entry that overlaps one of its own.
 int launch_adamw_list(const AdamWArgs &a, int64_t count, float *const *param, float *const *m, float *const *v,
                       float *const *grad, const int64_t *n, bool dependent, cudaStream_t stream) {
-    for (int64_t i = 0; i < count; i += kMaxList) {
-        const int k = static_cast<int>(std::min<int64_t>(kMaxList, count - i));
+    float *const *const arrays[4] = {param, m, v, grad};
+    const bool overlap = count > 1 && entries_overlap(count, arrays, n);
+    for (int64_t i = 0, k64 = 0; i < count; i += k64) {
+        k64 = std::min<int64_t>(kMaxList, count - i);
+        if (overlap) {
+            float *const *const rest[4] = {param + i, m + i, v + i, grad + i};
+            k64 = disjoint_entries(k64, rest, n + i);
+        }
+        const int k = static_cast<int>(k64);
         // the parameter block is copied at every launch, so a short list takes a short one
         auto launch = k <= 16 ? launch_step<16> : k <= 128 ? launch_step<128> : launch_step<kMaxList>;
         const int rc = launch(a, k, param + i, m + i, v + i, grad + i, n + i, dependent && i == 0, stream);

@@ -209,7 +209,8 @@ MNI_B200_API int mni_b200_grad_norm_sq(int64_t count, const float *const *grads,
                                        void *stream);
 /*
  * ... and clip_and_step (ops/optimizer.rs:247-276): the norm over all gradients, then the clipped AdamW step of every
- * tensor, gradients left scaled as grad_clip_f32 leaves them.  One launch each for lists of up to 512 tensors.  With a
+ * tensor, gradients left scaled as grad_clip_f32 leaves them.  One launch each for lists of up to 512 tensors; entries
+ * that share memory (tied parameters given twice) are stepped one after the other, in list order.  With a
  * non-null `norm` (host memory) the call waits until the norm before clipping is known and stores it there; the
  * step itself may still be running, in stream order with whatever follows.
  */

@@ -131,3 +131,44 @@ def test_parameter_lists_around_the_chunk_and_launch_limits(F, oracle, sizes, mi
     for name in "pmvg":
         for d, r in zip(dev[name], host[name]):
             assert r.size == 0 or float(np.max(np.abs(d.numpy() - r))) <= 2e-6 * (1 + float(np.abs(r).max())), name
+
+
+@pytest.mark.parametrize("max_norm", [0.0, 0.5])
+def test_tensors_that_share_memory_are_stepped_in_list_order(F, max_norm):
+    """Tied parameters given twice, a parameter that overlaps another's part, state shared by two parameters: bit for bit what
+    the list gives one tensor at a time."""
+    import torch
+    n = 70_000
+    rng = np.random.default_rng(11)
+    host = [(scale * rng.standard_normal(4 * n)).astype(np.float32) for scale in (1.0, 0.1, 0.01, 1.0)]
+    host[2] = np.abs(host[2])
+    # (param, m, v, grad) as ranges of the four buffers: start and length
+    entries = [(0, n), (n, n), (0, n), (2 * n, n), (2 * n + n // 2, n), (0, n), (n, 0), (3 * n + n // 2, 5), (n, n)]
+
+    def lists():
+        bufs = [torch.from_numpy(a).cuda() for a in host]
+        out = [[F.DeviceTensor(b[s:s + max(k, 1)], (k,)) for s, k in entries] for b in bufs]
+        out[2][3] = F.DeviceTensor(bufs[2][n:2 * n], (n,))               # v of another entry
+        return bufs, out
+    cfg = dict(lr=1e-3, weight_decay=0.01, step=3, max_grad_norm=max_norm)
+    got_bufs, (p, m, v, g) = lists()
+    launches = F.launch_count()
+    norm = F.clip_and_step(p, m, v, g, **cfg)
+    launches = F.launch_count() - launches
+    want_bufs, (p, m, v, g) = lists()
+    sumsq = F.ops._grad_sumsq(g)
+    for one in zip(p, m, v, g):
+        F.adamw_step(*one, grad_sumsq=sumsq, **cfg)
+    assert norm == float(np.sqrt(np.float32(sumsq.item())))
+    for a, b in zip(got_bufs, want_bufs):
+        assert torch.equal(a, b)
+    assert launches == 1 + 3             # the norm, then entries 0-1, 2-3 and 4-8: a launch ends before an overlap
+
+
+def test_tensors_that_only_touch_need_one_launch(F):
+    import torch
+    flat = [torch.rand(3000, device="cuda") for _ in range(4)]
+    lists = [[F.DeviceTensor(b[s:s + 1000], (1000,)) for s in (2000, 0, 1000)] for b in flat]
+    launches = F.launch_count()
+    F.clip_and_step(*lists, lr=1e-3)
+    assert F.launch_count() - launches == 2
