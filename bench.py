@@ -68,7 +68,7 @@ class Workload:
 
     @property
     def out_shape(self):
-        from framework_b200.ops import broadcast_shape
+        from framework_b200.shapes import broadcast_shape
         m, _, n = self.mkn
         return broadcast_shape(self.a_shape[:-2], self.b_logical[:-2]) + (m, n)
 

@@ -121,16 +121,26 @@ def host_is_stale() -> bool:
 
 def build_host(force: bool = False) -> str:
     """Compiles the host extension into lib/_host.so (about ten seconds); returns its path.  The file is put in place
-    by a rename, so that processes that build it at the same time each see a whole one."""
+    by a rename, so that whoever loads it meanwhile sees a whole one; of processes that find it missing at the same time
+    (the ranks of a fresh tree) one compiles, under a file lock, and the others take what it has built."""
     if not force and not host_is_stale():
         return HOST_PATH
+    import fcntl
+    os.makedirs(os.path.dirname(HOST_PATH), exist_ok=True)
+    with open(HOST_PATH + ".lock", "w") as lock:
+        fcntl.flock(lock, fcntl.LOCK_EX)
+        if force or host_is_stale():
+            _compile_host()
+    return HOST_PATH
+
+
+def _compile_host() -> None:
     import sysconfig
     import torch
     root = os.path.dirname(torch.__file__)
     inc = [os.path.join(_ROOT, "include"), os.path.join(root, "include"),
            os.path.join(root, "include", "torch", "csrc", "api", "include"), sysconfig.get_paths()["include"],
            os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")]
-    os.makedirs(os.path.dirname(HOST_PATH), exist_ok=True)
     tmp = f"{HOST_PATH}.{os.getpid()}.tmp"
     subprocess.check_call(
         ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
@@ -141,13 +151,16 @@ def build_host(force: bool = False) -> str:
     with open(f"{tmp}.id", "w") as f:
         f.write(host_source_hash() + "\n")
     os.replace(f"{tmp}.id", _hash_file())
-    return HOST_PATH
 
 
 def load_host():
     """The host extension as a module, compiled first if it is missing or was built from another source."""
     import torch  # noqa: F401  (the extension links against torch's libraries, which torch loads)
-    build_host()
+    try:
+        build_host()
+    except (OSError, subprocess.CalledProcessError) as e:
+        raise ImportError(f"{HOST_PATH} is missing or was built from another source, and cannot be built here ({e}): build it "
+                          "with `python -m framework_b200.build`") from e
     loader = importlib.machinery.ExtensionFileLoader("_host", HOST_PATH)
     spec = importlib.util.spec_from_file_location("_host", HOST_PATH, loader=loader)
     module = importlib.util.module_from_spec(spec)

@@ -12,25 +12,8 @@ from __future__ import annotations
 from typing import Optional, Sequence, Tuple
 
 from . import _lib
-from .tensor import DeviceTensor, _host, current_stream, row_major_strides
-
-
-def broadcast_shape(a: Sequence[int], b: Sequence[int]) -> tuple:
-    """utils.rs:3-20.  Raises where the reference panics."""
-    nd = max(len(a), len(b))
-    out = []
-    for i in range(nd):
-        da = 1 if i < nd - len(a) else a[i - (nd - len(a))]
-        db = 1 if i < nd - len(b) else b[i - (nd - len(b))]
-        if da == db:
-            out.append(da)
-        elif da == 1:
-            out.append(db)
-        elif db == 1:
-            out.append(da)
-        else:
-            raise ValueError(f"shapes {list(a)} and {list(b)} are not broadcastable")
-    return tuple(out)
+from .shapes import broadcast_shape, row_major_strides
+from .tensor import DeviceTensor, _host, current_stream
 
 
 def _matmul_out_shape(a: DeviceTensor, b: DeviceTensor) -> tuple:

@@ -15,24 +15,9 @@ import numpy as np
 import torch
 
 from . import _lib, build
+from .shapes import row_major_strides, shape_size  # noqa: F401
 
 _host = build.load_host()
-
-
-def row_major_strides(shape: Sequence[int]) -> tuple:
-    """tensor.rs:7-17 compute_strides."""
-    st, acc = [], 1
-    for s in reversed(shape):
-        st.append(acc)
-        acc *= int(s)
-    return tuple(reversed(st))
-
-
-def shape_size(shape: Sequence[int]) -> int:
-    n = 1
-    for s in shape:
-        n *= int(s)
-    return n
 
 
 def current_stream() -> int:

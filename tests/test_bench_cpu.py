@@ -54,3 +54,24 @@ def test_cpu_samples_are_bounded_leading_slices(bench):
     assert "leading" in what
     whole, what = bench.cpu_sample_workload(bench.WORKLOADS["c1"], budget_gflop=150.0)
     assert whole.a_shape == (512, 512) and what == "whole step"
+
+
+def test_reference_arm_loads_no_native_code_of_the_package(bench):
+    """What the reference arm takes from the package -- shapes and shards of the workloads -- maps none of its libraries."""
+    import subprocess
+    import sys
+    code = """
+import importlib.util, sys
+spec = importlib.util.spec_from_file_location("bench_module", "bench.py")
+bench = importlib.util.module_from_spec(spec)
+spec.loader.exec_module(bench)
+for wl in bench.WORKLOADS.values():
+    bench.config_dict(wl, 8, "f32")
+    shard = bench.shard_workload(wl, 1, 8)
+    if wl.kind not in ("softmax", "adamw"):
+        shard.out_shape, shard.batch, shard.flops, bench.cpu_sample_workload(wl, budget_gflop=150.0)
+assert "framework_b200.sharding" in sys.modules
+maps = open("/proc/self/maps").read()
+assert "framework_b200" not in maps, [line for line in maps.splitlines() if "framework_b200" in line]
+"""
+    subprocess.run([sys.executable, "-c", code], check=True, cwd=ROOT)

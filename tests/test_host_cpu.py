@@ -1,4 +1,7 @@
 """CPU: what the native operator front end refuses, before it touches a device."""
+import threading
+import time
+
 import pytest
 
 
@@ -64,3 +67,55 @@ def test_no_device_is_an_error_not_an_abort(F):
     for use in (lambda: F.device_status(), lambda: F.tensor.current_stream(), lambda: F.DeviceTensor.empty((2, 2))):
         with pytest.raises(RuntimeError):
             use()
+
+
+def test_one_of_several_compiles_the_extension(monkeypatch, tmp_path):
+    from framework_b200 import build
+    monkeypatch.setattr(build, "HOST_PATH", str(tmp_path / "lib" / "_host.so"))
+    runs = []
+
+    def compiler(cmd, **kw):
+        runs.append(cmd)
+        time.sleep(0.2)
+        open(cmd[cmd.index("-o") + 1], "w").close()
+    monkeypatch.setattr(build.subprocess, "check_call", compiler)
+    threads = [threading.Thread(target=build.build_host) for _ in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert len(runs) == 1 and not build.host_is_stale()
+    build.build_host(force=True)
+    assert len(runs) == 2
+
+
+def test_no_compiler_is_an_import_error(monkeypatch, tmp_path):
+    from framework_b200 import build
+    monkeypatch.setattr(build, "HOST_PATH", str(tmp_path / "lib" / "_host.so"))
+
+    def no_compiler(cmd, **kw):
+        raise FileNotFoundError(2, "No such file or directory", cmd[0])
+    monkeypatch.setattr(build.subprocess, "check_call", no_compiler)
+    with pytest.raises(ImportError, match="framework_b200.build"):
+        build.load_host()
+
+
+def test_names_of_the_package():
+    import subprocess
+    import sys
+    from conftest import ROOT
+    code = """
+import sys
+import framework_b200 as F
+assert "framework_b200.ops" not in sys.modules and {"matmul", "DeviceTensor", "ops"} <= set(dir(F))
+assert F.matmul is F.ops.matmul and F.DeviceTensor is F.tensor.DeviceTensor and F.broadcast_shape((2, 1), (3,)) == (2, 3)
+from framework_b200 import *
+assert all(name in globals() for name in F.__all__)
+try:
+    F.nothing
+except AttributeError as e:
+    assert "nothing" in str(e)
+else:
+    raise AssertionError
+"""
+    subprocess.run([sys.executable, "-c", code], check=True, cwd=ROOT)
