@@ -1255,7 +1255,6 @@ int mni_b200_workspace_query(const mni_b200_view *a, const mni_b200_view *b, uin
     for (int d = dc.ndim - 1; d >= 0; --d) { dc.stride[d] = acc; acc *= dc.shape[d]; }
     mni_b200_view dc_strided = dc;
     for (int d = 0; d < dc.ndim; ++d) dc_strided.stride[d] = dc.stride[d] * 2;
-    float *fake = reinterpret_cast<float *>(static_cast<uintptr_t>(256));
     size_t need = 0;
     auto dry = [&](auto body) -> int {
         Call c;
@@ -1264,15 +1263,23 @@ int mni_b200_workspace_query(const mni_b200_view *a, const mni_b200_view *b, uin
         need = std::max(need, c.arena.used);
         return r;
     };
-    rc = dry([&](Call &c) { return fwd_body(c, a, b, fake, nullptr); });
-    if (rc) return rc;
-    rc = dry([&](Call &c) { return bwd_body(c, a, b, &dc, fake, fake, fake); });
-    if (rc) return rc;
-    rc = dry([&](Call &c) { return bwd_body(c, a, b, &dc_strided, fake, fake, fake); });
-    if (rc) return rc;
-    // bias + GELU forward without a `pre` output: when the epilogue cannot be fused the product needs a temporary
-    rc = dry([&](Call &c) { return fwd_gelu_body(c, a, b, fake, nullptr, fake); });
-    if (rc) return rc;
+    // Outputs on a 16-byte boundary and off it take different plans, and so do calls for both gradients, which may run
+    // side by side on half of the SMs each, and calls for one of them.
+    for (const uintptr_t at : {uintptr_t{256}, uintptr_t{260}}) {
+        float *out = reinterpret_cast<float *>(at);
+        rc = dry([&](Call &c) { return fwd_body(c, a, b, out, nullptr); });
+        if (rc) return rc;
+        for (const mni_b200_view *grad : {&dc, &dc_strided})
+            for (int want = 1; want < 8; ++want) {
+                rc = dry([&](Call &c) {
+                    return bwd_body(c, a, b, grad, (want & 1) ? out : nullptr, (want & 2) ? out : nullptr, (want & 4) ? out : nullptr);
+                });
+                if (rc) return rc;
+            }
+        // bias + GELU forward without a `pre` output: when the epilogue cannot be fused the product needs a temporary
+        rc = dry([&](Call &c) { return fwd_gelu_body(c, a, b, out, nullptr, out); });
+        if (rc) return rc;
+    }
     // the pointwise entry points on the forward output: column-sum partials
     const int64_t rows = s.batch * s.M;
     need = std::max(need, (colsum_partial_bytes(std::max<int64_t>(rows, 1), std::max<int64_t>(s.N, 1), st->sm_count) + 255) &

@@ -253,9 +253,10 @@ MNI_B200_API int mni_b200_contiguous(const mni_b200_view *src, float *dst, void 
  * with MNI_B200_ERR_WORKSPACE rather than allocate.  mni_b200_workspace_query
  * returns an upper bound, for operands a and b as given (their strides and
  * alignment count), over: mni_b200_matmul_fwd; mni_b200_matmul_bias_gelu_fwd
- * with or without a `pre` output; mni_b200_matmul_bwd with da, db and dbias and
- * ANY view of the output gradient (contiguous, or strided so that it has to be
- * gathered first); and the pointwise entry points (add_bias_bwd, bias_gelu_bwd)
+ * with or without a `pre` output; mni_b200_matmul_bwd with any of da, db and
+ * dbias (a call for one gradient can need more than one for both) and ANY view
+ * of the output gradient (contiguous, or strided so that it has to be gathered
+ * first); and the pointwise entry points (add_bias_bwd, bias_gelu_bwd)
  * applied to tensors no larger than a, b or the forward output.
  * The flags given are the flags the later calls must use.
  *

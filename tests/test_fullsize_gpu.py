@@ -7,6 +7,8 @@ e * sum|v| a worst-case alignment of signs would give."""
 import numpy as np
 import pytest
 
+from conftest import Guarded, regression_bound_3xtf32, rel_fro
+
 pytestmark = pytest.mark.gpu
 
 
@@ -124,3 +126,46 @@ def test_caller_provided_workspace(F):
     finally:
         F._lib.check(lib.mni_b200_workspace_set(None, 0))
     assert np.array_equal(F.matmul(a, w).numpy(), ref_c)
+
+
+@pytest.mark.parametrize("m,k,n,batch", [(1728, 3648, 1728, ()), (512, 512, 512, ()), (2048, 3072, 768, ()), (16, 4096, 4096, ()),
+                                         (9, 4096, 4095, ()), (333, 64, 333, (6,)), (1000, 333, 777, ()), (40, 2048, 1000, ())])
+def test_queried_scratch_serves_every_form_of_a_call(F, m, k, n, batch):
+    """Each gradient alone, both, with and without the bias gradient, from a contiguous and a strided output gradient, into
+    aligned and unaligned outputs, and the forward with GELU: all inside a buffer of exactly the queried size."""
+    import ctypes as C
+    import torch
+    rng = np.random.default_rng(m)
+    t = F.DeviceTensor.from_numpy
+    x, w = rng.standard_normal(batch + (m, k)).astype(np.float32), rng.standard_normal(batch + (k, n)).astype(np.float32)
+    dy, bias = rng.standard_normal(batch + (m, n)).astype(np.float32), rng.standard_normal(n).astype(np.float32)
+    dx, dw, db_ = t(x), t(w), t(bias)
+    strided = torch.zeros(batch + (m, 2 * n), device="cuda")[..., ::2]
+    strided.copy_(torch.from_numpy(dy))
+    lib, need = F._lib.lib(), C.c_size_t(0)
+    F._lib.check(lib.mni_b200_workspace_query(dx.view_struct(), dw.view_struct(), 0, C.byref(need)))
+    buf = torch.empty(need.value + 512, dtype=torch.uint8, device="cuda")
+    base = (buf.data_ptr() + 255) // 256 * 256
+    guard = buf[base - buf.data_ptr() + need.value:]
+    guard.fill_(0x5A)
+    batch_k = max(m, k, n)
+    want = {"da": dy @ np.swapaxes(w, -1, -2), "db": np.swapaxes(x, -1, -2) @ dy, "dbias": dy.reshape(-1, n).sum(0)}
+    F._lib.check(lib.mni_b200_workspace_set(C.c_void_p(base), max(need.value, 1)))
+    try:
+        for grad in (t(dy), F.DeviceTensor.from_torch(strided)):
+            for off in (0, 1):
+                for names in (("da",), ("db",), ("da", "db"), ("da", "dbias"), ("db", "dbias"), ("da", "db", "dbias"), ("dbias",)):
+                    out = {nm: Guarded(F, want[nm].shape, misalign=off) for nm in names}
+                    F.matmul_backward(grad, dx, dw, need_da="da" in names, need_db="db" in names, want_dbias="dbias" in names,
+                                      **{nm: g.tensor for nm, g in out.items()})
+                    F.device_status()
+                    for nm, g in out.items():
+                        g.check(nm)
+                        assert rel_fro(g.tensor.numpy(), want[nm]) <= regression_bound_3xtf32(batch_k), (names, nm, off)
+        for pre in (True, False):
+            F.matmul_bias_gelu(dx, dw, db_, want_pre=pre)
+        F.matmul(dx, dw)
+        F.device_status()
+    finally:
+        F._lib.check(lib.mni_b200_workspace_set(None, 0))
+    assert bool((guard == 0x5A).all())
