@@ -838,6 +838,13 @@ int launch_skinny_dw(const float *x, int64_t ldx, const float *dy, int64_t lddy,
     long long slabs = std::max<long long>(1, static_cast<long long>(device_sm_count()) * (mt > 8 ? 5 : 8) / strips);
     long long k_per = std::max<long long>(8, (K + slabs - 1) / slabs);
     k_per = std::min<long long>(k_per, mt > 8 ? 512 : 1024);
+    // A grid has at most 65535 slabs: beyond, several launches.
+    const long long k_most = 65535 * k_per;
+    if (K > k_most) {
+        const int rc = launch_skinny_dw(x + k_most, ldx, dy, lddy, dW + k_most * lddw, lddw, accumulate, M, N, K - k_most, stream);
+        if (rc) return rc;
+        K = k_most;
+    }
     slabs = (K + k_per - 1) / k_per;
     dim3 grid(strips, static_cast<unsigned>(slabs));
     const size_t smem = static_cast<size_t>(mt) * k_per * sizeof(float2);

@@ -65,3 +65,20 @@ def test_few_rows_units_from_before_a_row(F, m, k, n, offset):
         dw = dw.tensor
         for got, want, length in ((y, x64 @ w64, k), (dx, dy64 @ w64.T, n), (dw, x64.T @ dy64, m)):
             assert rel_fro(got.numpy(), want) <= regression_bound_3xtf32(length)
+
+
+def test_weight_gradient_of_more_slabs_than_a_grid_has(F):
+    """9 rows in slabs of 512 weight rows: the first length past 65535 slabs."""
+    import torch
+    k = 65535 * 512 + 1
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    x, dy = torch.randn((9, k), generator=gen, device="cuda"), torch.randn((9, 1), generator=gen, device="cuda")
+    dw = Guarded(F, (k, 1))
+    t = F.DeviceTensor.from_torch
+    F.matmul_backward(t(dy), t(x), F.DeviceTensor.empty((k, 1)), need_da=False, db=dw.tensor)
+    F.device_status()
+    dw.check("dw")
+    want = (x * dy).sum(0, dtype=torch.float64)
+    got = dw.tensor.storage.double()
+    assert float((got - want).norm() / want.norm()) <= regression_bound_3xtf32(9)
+    assert float((got - want)[-600:].abs().max()) <= 1e-5
