@@ -296,12 +296,21 @@ namespace {
 template <bool GELU>
 int launch_bias(const float *y, const float *bias, float *out, int64_t rows, int64_t n, cudaStream_t stream) {
     if (rows == 0 || n == 0) return MNI_B200_OK;
-    if (n >= (1LL << 31)) return fail(MNI_B200_ERR_TOO_LARGE, "bias of %lld columns", static_cast<long long>(n));
+    // The kernel's flat index stays below 2^31, the last block's included: longer rows go out in pieces of columns.
+    constexpr int64_t kMostUnits = (1LL << 31) - 8192, kPiece = 1LL << 30;
+    if (n > kMostUnits) {
+        for (int64_t r = 0; r < rows; ++r)
+            for (int64_t c = 0; c < n; c += kPiece) {
+                const int rc = launch_bias<GELU>(y + r * n + c, bias + c, out + r * n + c, 1, std::min(kPiece, n - c), stream);
+                if (rc) return rc;
+            }
+        return MNI_B200_OK;
+    }
     const bool quads = ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
     const bool aligned = quads && n % 4 == 0 && (reinterpret_cast<uintptr_t>(bias) & 15) == 0;
     // whole groups of rows per launch, so that every launch's flat index stays below 2^31 and its start keeps the
     // alignment (a multiple of four rows)
-    const int64_t limit = ((1LL << 31) - 8192) / n;
+    const int64_t limit = kMostUnits / n;
     const int64_t step = std::max<int64_t>(1, limit >= 4 ? limit / 4 * 4 : limit);
     for (int64_t r = 0; r < rows; r += step) {
         const int64_t total = std::min(step, rows - r) * n;

@@ -164,3 +164,16 @@ def test_small_products_in_one_launch(F, m, k, n, layout):
         for got, want, c in zip((y, da, db, dbias), (a64 @ b64 + bias, g64 @ b64.T, a64.T @ g64, g64.sum(0)), c0):
             got.check(fully_written=not accumulate)
             assert rel_fro(got.tensor.numpy(), want + (c if accumulate else 0)) <= regression_bound_3xtf32(max(m, k, n))
+
+
+@pytest.mark.parametrize("n,misalign", [(2 ** 31 - 5, 1), (2 ** 31 + 3, 0)])
+def test_bias_rows_past_the_flat_index(F, n, misalign):
+    """A row whose elements a 32-bit index does not count, added in place."""
+    import torch
+    y, bias = torch.rand(n + 8, device="cuda"), torch.empty(n, device="cuda")
+    bias.copy_(y[misalign:misalign + n])
+    F._lib.check(F._lib.lib().mni_b200_add_bias(y.data_ptr() + 4 * misalign, bias.data_ptr(), y.data_ptr() + 4 * misalign, 1, n, 0))
+    torch.cuda.synchronize()
+    step = 1 << 28
+    for at in range(0, n, step):
+        assert torch.equal(y[misalign + at:misalign + min(n, at + step)], 2 * bias[at:at + step]), at
