@@ -959,7 +959,7 @@ bool pdl_enabled() {
 namespace {
 constexpr int kMaxSwitches = 48;
 struct EnvSnapshot {
-    int depth = 0, count = 0;
+    int depth = 0, count = 0;             // count > kMaxSwitches: more than fit, and the environment is asked as outside a scope
     const char *entry[kMaxSwitches];      // "NAME=value"
 };
 thread_local EnvSnapshot t_env;
@@ -969,13 +969,16 @@ EnvScope::EnvScope() {
     if (t_env.depth++ != 0) return;
     t_env.count = 0;
     for (char **e = environ; e && *e; ++e)
-        if ((*e)[0] == 'M' && strncmp(*e, "MNI_B200_", 9) == 0 && t_env.count < kMaxSwitches) t_env.entry[t_env.count++] = *e;
+        if ((*e)[0] == 'M' && strncmp(*e, "MNI_B200_", 9) == 0) {
+            if (t_env.count == kMaxSwitches) { ++t_env.count; break; }
+            t_env.entry[t_env.count++] = *e;
+        }
 }
 EnvScope::~EnvScope() { --t_env.depth; }
 
 const char *env_value(const char *name) {
     const char *v = nullptr;
-    if (t_env.depth == 0) {
+    if (t_env.depth == 0 || t_env.count > kMaxSwitches) {
         v = getenv(name);
     } else {
         for (int i = 0; i < t_env.count; ++i) {
@@ -1293,6 +1296,7 @@ int mni_b200_plan_describe(const mni_b200_view *a, const mni_b200_view *b, int b
     if (!out || out_len == 0) return fail(MNI_B200_ERR_ARG, "out is null or empty");
     if (sm_count < 8 || sm_count > 4096) return fail(MNI_B200_ERR_ARG, "sm_count %d out of range", sm_count);
     out[0] = 0;
+    EnvScope env;
     Shapes s;
     int rc = analyse(a, b, s);
     if (rc) return rc;

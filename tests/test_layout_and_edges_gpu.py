@@ -177,3 +177,17 @@ def test_bias_rows_past_the_flat_index(F, n, misalign):
     step = 1 << 28
     for at in range(0, n, step):
         assert torch.equal(y[misalign + at:misalign + min(n, at + step)], 2 * bias[at:at + step]), at
+
+
+def test_a_call_honours_a_switch_however_many_are_set(F, monkeypatch):
+    x, w, dy = (F.DeviceTensor.from_numpy(np.ones(s, np.float32)) for s in ((32, 64), (64, 32), (32, 32)))
+
+    def launches():
+        before = F.launch_count()
+        F.matmul_backward(dy, x, w)
+        return F.launch_count() - before
+    assert launches() == 1                       # both products in one f32 kernel
+    for i in range(60):
+        monkeypatch.setenv(f"MNI_B200_UNUSED_{i}", "1")
+    monkeypatch.setenv("MNI_B200_TINY", "0")
+    assert launches() >= 2

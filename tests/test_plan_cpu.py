@@ -174,6 +174,16 @@ def test_exchanged_operands_keep_to_the_plans_that_store_transposed(plan, monkey
     assert (cut["exchanged"], cut["tail_ways"]) == (0, 3)
 
 
+@pytest.mark.parametrize("others", [0, 46, 47, 48, 60])
+def test_a_switch_counts_however_many_are_set(plan, monkeypatch, others):
+    for i in range(others):
+        monkeypatch.setenv(f"MNI_B200_UNUSED_{i}", "1")
+    monkeypatch.setenv("MNI_B200_BN", "64")
+    assert tensor_plan(plan((4096, 1024), (1024, 4096)), "forward")["bn"] == 64
+    monkeypatch.delenv("MNI_B200_BN")
+    assert tensor_plan(plan((4096, 1024), (1024, 4096)), "forward")["bn"] == 256
+
+
 def test_errors_are_the_calls_own(plan):
     from framework_b200 import _lib
     with pytest.raises(_lib.MniError) as ei:
