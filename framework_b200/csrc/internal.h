@@ -222,9 +222,10 @@ int launch_tiny(const TinyProduct *products, int count, const TinyColumns *colum
 int launch_add_bias(const float *y, const float *bias, float *out, int64_t rows, int64_t n,
                     cudaStream_t stream);
 size_t colsum_partial_bytes(int64_t rows, int64_t n, int sm_count);
-// out = column sums of dy[rows, n] (row pitch ld); copy != null also receives dy (pitch n) in the same pass
+// out = column sums of dy[rows, n] (row pitch ld); copy != null also receives dy (pitch n) in the same pass.  ticket_bank: 1 for
+// calls whose partial sums are not in the library's scratch
 int launch_colsum(const float *dy, int64_t ld, float *copy, float *out, int64_t rows, int64_t n, bool accumulate,
-                  float *partial, int sm_count, cudaStream_t stream);
+                  float *partial, int sm_count, cudaStream_t stream, int ticket_bank = 0);
 int launch_copy(const float *src, float *dst, int64_t n, cudaStream_t stream);
 int launch_softmax_fwd(const float *x, float *out, int64_t outer, int64_t dim, int64_t inner, cudaStream_t stream);
 int launch_softmax_bwd(const float *dy, const float *out, float *dx, int64_t outer, int64_t dim, int64_t inner,

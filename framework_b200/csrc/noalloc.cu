@@ -17,6 +17,7 @@
 //   * All calls on a device use the same array, and it keeps whatever the previous call left in
 //     it.  Nothing in it has to start at zero: the first kernel of a call writes every slot the
 //     second kernel of that call reads, so stale contents are never observed.
+//   * Its finish tickets are its own as well (bank 1 of the column sums): a call may run beside the library's other calls.
 //   * Two calls that run on the GPU at the same time (different streams, or different host
 //     threads without ordering) write the same array and corrupt each other's sums.  Issue them
 //     on one stream, or order them with events.
@@ -98,5 +99,5 @@ extern "C" MNI_B200_API int mni_b200_add_bias_bwd_noalloc(const float *dy, float
         if (!accumulate) MNI_CUDA(cudaMemsetAsync(dbias, 0, static_cast<size_t>(n) * sizeof(float), s));
         return MNI_B200_OK;
     }
-    return mni::launch_colsum(dy, n, d_y != dy ? d_y : nullptr, dbias, rows, n, accumulate, st->scratch, st->sm_count, s);
+    return mni::launch_colsum(dy, n, d_y != dy ? d_y : nullptr, dbias, rows, n, accumulate, st->scratch, st->sm_count, s, 1);
 }

@@ -23,7 +23,10 @@ int grid_for(long long work_items, int threads) {
 // one launch does what took two (and, with a copy of dy wanted, three): 5.5 -> 2.0 us of launches for a small layer.
 // A strip summed by one block needs neither scratch nor ticket.
 constexpr int kMaxStrips = 1024;             // several slabs per strip only up to this many strips (see colsum_slabs)
-__device__ unsigned int g_colsum_tickets[kMaxStrips];   // zero between launches
+// Zero between launches.  Bank 1 belongs to the entry point that allocates nothing, whose partial sums are its own too: its
+// calls may run beside the others'.
+constexpr int kTicketBanks = 2;
+__device__ unsigned int g_colsum_tickets[kTicketBanks * kMaxStrips];
 
 __device__ __forceinline__ void store_cols(float *dst, long long col, long long n, const float4 &s) {
     dst[0] = s.x;
@@ -48,8 +51,9 @@ __device__ __forceinline__ float4 fold_warps(float4 (*red)[32], const float4 &ac
 }
 // The end of a column-sum block: `acc` is this thread's sum over the block's rows.
 __device__ __forceinline__ void finish_colsum(const float4 &acc, float4 (*red)[32], float *partial, float *out,
-                                              long long n, int accumulate) {
+                                              long long n, int accumulate, int bank) {
     __shared__ unsigned int s_last;
+    unsigned int *const ticket = g_colsum_tickets + bank * kMaxStrips + blockIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const long long col = (static_cast<long long>(blockIdx.x) * 32 + lane) * 4;
     float4 s = fold_warps(red, acc);
@@ -59,7 +63,7 @@ __device__ __forceinline__ void finish_colsum(const float4 &acc, float4 (*red)[3
             if (col < n) store_cols(partial + static_cast<long long>(blockIdx.y) * n + col, col, n, s);
             __threadfence();
             __syncwarp();
-            if (lane == 0) s_last = atomicAdd(&g_colsum_tickets[blockIdx.x], 1u) == static_cast<unsigned>(slabs - 1);
+            if (lane == 0) s_last = atomicAdd(ticket, 1u) == static_cast<unsigned>(slabs - 1);
         }
         __syncthreads();
         if (!s_last) return;
@@ -76,7 +80,7 @@ __device__ __forceinline__ void finish_colsum(const float4 &acc, float4 (*red)[3
             }
         }
         s = fold_warps(red, t);
-        if (threadIdx.x == 0) g_colsum_tickets[blockIdx.x] = 0u;
+        if (threadIdx.x == 0) *ticket = 0u;
     }
     if (warp == 0 && col < n) {
         if (accumulate) {
@@ -92,7 +96,7 @@ __device__ __forceinline__ void finish_colsum(const float4 &acc, float4 (*red)[3
 template <bool COPY>
 __global__ void __launch_bounds__(256)
 colsum_kernel(const float *__restrict__ dy, long long ld, float *__restrict__ copy, float *__restrict__ partial,
-              float *__restrict__ out, long long rows, long long n, long long rows_per, int accumulate) {
+              float *__restrict__ out, long long rows, long long n, long long rows_per, int accumulate, int bank) {
     __shared__ float4 red[8][32];
     grid_dependency_trigger();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -136,7 +140,7 @@ colsum_kernel(const float *__restrict__ dy, long long ld, float *__restrict__ co
             acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
         }
     }
-    finish_colsum(acc, red, partial, out, n, accumulate);
+    finish_colsum(acc, red, partial, out, n, accumulate, bank);
 }
 
 // ---- bias + GELU (tanh form), the fused pointwise op that follows the MLP up-projection --------
@@ -252,7 +256,7 @@ bias_gelu_bwd_kernel(const float *__restrict__ grad, const float *__restrict__ x
             }
         }
     }
-    finish_colsum(acc, red, partial, dbias, n, accumulate);
+    finish_colsum(acc, red, partial, dbias, n, accumulate, 0);
 }
 
 struct UnbArgs {
@@ -352,13 +356,13 @@ size_t colsum_partial_bytes(int64_t rows, int64_t n, int sm_count) {
 }
 
 int launch_colsum(const float *dy, int64_t ld, float *copy, float *out, int64_t rows, int64_t n, bool accumulate,
-                  float *partial, int sm_count, cudaStream_t stream) {
+                  float *partial, int sm_count, cudaStream_t stream, int ticket_bank) {
     if (n == 0) return MNI_B200_OK;
     const int slabs = colsum_slabs(rows, n, sm_count);
     const long long rows_per = (rows + slabs - 1) / slabs;
     dim3 grid(static_cast<unsigned>((n + 127) / 128), static_cast<unsigned>(slabs));
     const cudaError_t e = launch_dependent(copy ? colsum_kernel<true> : colsum_kernel<false>, grid, dim3(256), 0, stream, dy,
-                                           ld, copy, partial, out, rows, n, rows_per, accumulate ? 1 : 0);
+                                           ld, copy, partial, out, rows, n, rows_per, accumulate ? 1 : 0, ticket_bank);
     if (e != cudaSuccess) return fail(MNI_B200_ERR_CUDA, "colsum_kernel launch failed: %s", cudaGetErrorString(e));
     MNI_LAUNCH_CHECK("colsum_kernel");
     return MNI_B200_OK;

@@ -116,3 +116,23 @@ def test_refuses_sizes_beyond_the_built_in_scratch(F):
     # the regular entry point takes the same size
     F._lib.check(lib.mni_b200_add_bias_bwd(dy.data_ptr(), None, db.data_ptr(), 2, n, 0, current_stream()))
     torch.cuda.synchronize()
+
+
+def test_runs_beside_the_regular_entry_point(F):
+    """Its partial sums and its finish tickets are its own: a call on one stream and a regular one on another."""
+    import torch
+    lib = F._lib.lib()
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    dy = [torch.randn((4096, 1024), generator=gen, device="cuda") for _ in range(2)]
+    out = [torch.empty((200, 1024), device="cuda") for _ in range(2)]
+    fns = (lib.mni_b200_add_bias_bwd, lib.mni_b200_add_bias_bwd_noalloc)
+    for fn, s, d, o in zip(fns, streams, dy, out):
+        F._lib.check(fn(d.data_ptr(), None, o[0].data_ptr(), 4096, 1024, 0, s.cuda_stream))
+        torch.cuda.synchronize()
+    for i in range(1, 200):
+        for fn, s, d, o in zip(fns, streams, dy, out):
+            F._lib.check(fn(d.data_ptr(), None, o[i].data_ptr(), 4096, 1024, 0, s.cuda_stream))
+    torch.cuda.synchronize()
+    for o in out:
+        assert torch.equal(o, o[:1].expand_as(o))
