@@ -809,9 +809,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         const long long t_wg0 = p.prof ? clock64() : 0;
                         if (lane == 0 && in_flight == p.epi_patches) {   // the patch must have been read by its store
                             if (p.epi_patches == 1) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-                            else if (p.epi_patches == 2) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-                            else if (p.epi_patches == 4) asm volatile("cp.async.bulk.wait_group.read 3;" ::: "memory");
-                            else asm volatile("cp.async.bulk.wait_group.read 7;" ::: "memory");
+                            else asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
                             --in_flight;
                         }
                         __syncwarp();
@@ -1691,18 +1689,8 @@ Plan make_plan(const GemmProblem &p, int sm_count) {
     const size_t raw = static_cast<size_t>(BM + pl.bn / pl.cg) * pl.bk * 4;
     const size_t stage = p.fast_tf32 ? raw : (pl.ta ? raw + static_cast<size_t>(pl.bn) * pl.bk * 4 : 2 * raw);
     const size_t budget = 227 * 1024;
-    // Tiles with a short contraction spend their time in the epilogue: give it more TMA stores in
-    // flight (staging patches) and the main loop fewer stages.  Long contractions get the deepest pipeline.
-    const long long iters_per_tile = p.fold * ((p.K + pl.bk - 1) / pl.bk);
-    pl.patches = 1;   // staging patches per epilogue warp
-    (void)iters_per_tile;
-    const int pt_env = env_int("MNI_B200_EPI_PATCHES", 0);
-    if (pt_env == 1 || pt_env == 2 || pt_env == 4) pl.patches = pt_env;
-    size_t fixed = kFixedSmemNoEpi + static_cast<size_t>(kEpiWarps * pl.patches) * kEpiBufBytes;
-    while (pl.patches > 2 && (budget - fixed) / stage < 2) {
-        pl.patches /= 2;
-        fixed = kFixedSmemNoEpi + static_cast<size_t>(kEpiWarps * pl.patches) * kEpiBufBytes;
-    }
+    pl.patches = env_int("MNI_B200_EPI_PATCHES", 1) == 2 ? 2 : 1;   // staging patches per epilogue warp
+    const size_t fixed = kFixedSmemNoEpi + static_cast<size_t>(kEpiWarps * pl.patches) * kEpiBufBytes;
     pl.stages = static_cast<int>(std::min<size_t>(kMaxStages, (budget - fixed) / stage));
     if (pl.ta) pl.stages = std::min(pl.stages, (512 - 2 * pl.bn) / (2 * pl.bk));   // one TMEM slot per stage
     const int st_env = env_int("MNI_B200_STAGES", 0);

@@ -174,6 +174,16 @@ def test_exchanged_operands_keep_to_the_plans_that_store_transposed(plan, monkey
     assert (cut["exchanged"], cut["tail_ways"]) == (0, 3)
 
 
+def test_staging_patches_are_one_or_two(plan, monkeypatch):
+    """A patch per epilogue warp more costs pipeline stages; any other number than two leaves the default."""
+    def stages():
+        return tensor_plan(plan((4096, 1024), (1024, 4096)), "forward")["stages"]
+    default = stages()
+    for value, same in (("1", True), ("2", False), ("3", True), ("4", True), ("8", True)):
+        monkeypatch.setenv("MNI_B200_EPI_PATCHES", value)
+        assert (stages() == default) == same, value
+
+
 @pytest.mark.parametrize("others", [0, 46, 47, 48, 60])
 def test_a_switch_counts_however_many_are_set(plan, monkeypatch, others):
     for i in range(others):
