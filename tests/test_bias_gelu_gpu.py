@@ -3,7 +3,7 @@ matmul -> bias_gelu, against the CPU oracle (ops/fused.rs:251-277, :317-352 rest
 import numpy as np
 import pytest
 
-from conftest import tol_3xtf32
+from conftest import rel_fro, tol_3xtf32
 
 pytestmark = pytest.mark.gpu
 
@@ -77,3 +77,49 @@ def test_batched_broadcast_weight_with_gelu(F, oracle):
     F.device_status()
     assert pre.shape == (3, 160, 256)
     assert float(np.max(np.abs(out.numpy() - rout))) <= 1.2 * tol_3xtf32(96, a, w) + 4e-6
+
+
+def _exact(v):
+    v = v.astype(np.float64)
+    u2 = 2 * 0.7978845608028654 * (v + 0.044715 * v ** 3)
+    s = 1 / (1 + np.exp(-u2))
+    return u2, v * s, s + v * s * (1 / (1 + np.exp(u2))) * 2 * 0.7978845608028654 * (1 + 3 * 0.044715 * v ** 2)
+
+
+def _gelu_and_derivative(F, v):
+    n = 1024
+    x = F.DeviceTensor.from_numpy(v.reshape(-1, n))
+    zero, one = (F.DeviceTensor.from_numpy(np.full(s, c, np.float32)) for s, c in (((n,), 0), (x.shape, 1)))
+    return F.bias_gelu(x, zero).numpy().ravel(), F.bias_gelu_backward(one, x, zero)[0].numpy().ravel()
+
+
+def test_gelu_is_as_exact_as_the_tanh_form_in_single_precision(F):
+    """Normally distributed inputs, error in the 2-norm against float64: 0.5 v (1 + tanhf(u)) and its derivative in f32 are off
+    by 3.84e-8 and 4.50e-8."""
+    v = np.random.default_rng(0).standard_normal(1 << 20).astype(np.float32)
+    _, gelu, grad = _exact(v)
+    got, dgot = _gelu_and_derivative(F, v)
+    assert rel_fro(got, gelu) <= 3.84e-8 and rel_fro(dgot, grad) <= 4.50e-8
+
+
+def test_gelu_pointwise(F):
+    """Positive v: the rounding of the result, and the error of e = exp(-2u) < 1, two units and more where e is small, in
+    1 + e: three units of 2^-24 together.  Negative v: the error of the exponential, (2 + 1.2 |2u|) units, and of 2u itself, two
+    roundings times |2u|.  The derivative is s plus v s (1 - s) 2u', |v 2u'| <= 3 |2u|, with such an error in each factor."""
+    v = np.linspace(-10, 10, 1 << 20).astype(np.float32)
+    u2, gelu, grad = _exact(v)
+    got, dgot = _gelu_and_derivative(F, v)
+    relative = np.where(v >= 0, 3 * 2.0 ** -24, (4 + 3.2 * np.abs(u2)) * 2.0 ** -23)
+    assert np.all(np.abs(got - gelu) <= relative * np.abs(gelu) + 1e-37)
+    terms = np.where(v >= 0, 1.2, np.exp(np.minimum(u2, 0)) * (1 + 3 * np.abs(u2)))
+    assert np.all(np.abs(dgot - grad) <= 2 * relative * terms + 1e-36)
+
+
+def test_gelu_of_extreme_inputs(F):
+    v = np.zeros(1024, np.float32)
+    v[:9] = [np.inf, -np.inf, np.nan, 1e13, -1e13, 3e38, -3e38, 88, -88]
+    got, dgot = _gelu_and_derivative(F, v)
+    assert got[0] == np.inf and np.isnan(got[1]) and np.isnan(got[2])       # as 0.5 v (1 + tanh u) gives them
+    assert np.array_equal(got[3:9], np.maximum(v[3:9], 0))
+    assert list(dgot[[3, 4, 7, 8]]) == [1, 0, 1, 0] and np.all(np.isnan(dgot[:3]))
+    assert not got[9:].any() and np.all(dgot[9:] == 0.5)
