@@ -80,11 +80,20 @@ constexpr int64_t kSkinnyDxRows = 5, kSkinnyDwRows = 8;
 // 16-byte aligned it would have to gather first.
 constexpr int64_t kRowsAligned = 15, kRowsUnaligned = 16;
 
-// Limits of the one-launch f32 kernel (tiny.cu): it needs about 1.9 us and 1 us per 64 contraction elements, whatever the
-// rest of the shape, up to M * N * K = 8 M (192^3: forward 5.0 us against 7.7, backward 5.8 against 8.9; 256^3 is level;
-// K = 512 loses).  Up to 8 rows the streaming kernels are the competition.
-constexpr int64_t kTinyContraction = 320, kTinyContractionFewRows = 128;
+// Limits of the one-launch f32 kernel (tiny.cu): it needs about 1.9 us and 1 us per 64 contraction elements, up to M * N * K =
+// 8 M (192^3: forward 5.0 us against 7.7, backward 5.8 against 8.9; 256^3 is level; K = 512 loses), and up to so many 32 x 32
+// tiles of output -- three a block slot and more queue up and store element by element (2048 x 1 x 4096, 8192 tiles: 62 us
+// against 13).  An eager call gains from one launch in place of two to four; under capture only device time counts, and one
+// product with aligned output rows is the tensor path's from fewer tiles on (104 x 1 x 4776, 600 tiles: 7.0 us against 5.5; rows
+// of 19247: 6.7 against 12.1), two gradients' with contractions from 256 on (17 x 992 x 256: 8.7 against 7.3).
+constexpr int64_t kTinyContraction = 320, kTinyContractionFewRows = 128, kTinyContractionCaptured = 240;
 constexpr int kTinyWork = 1 << 23;
+constexpr int64_t kTinyTiles = 800, kTinyTilesCaptured = 400;
+// Up to 8 rows the streaming kernels are the competition.  For one product they win but where the tiles are few and five rows
+// or more, or a short contraction, share them (8 x 8 x 4512 forward 3.3 us against 4.8, 8 x 90 x 1656 4.1 / 6.3; but 8 x 128 x
+// 8192 6.1 / 4.8, 1 x 128 x 4096 5.6 / 3.1, input gradient 8 x 496 x 8 2.7 / 2.6).  A backward call for both gradients they make in two launches on two
+// streams: eager 8 x 12704 x 8 8.1 us against 14.8, captured 7.7 / 6.3, 4 x 4096 x 64 5.7 / 3.8, 8 x 2048 x 127 5.5 / 6.7.
+constexpr int64_t kTinyTilesFewRows = 256, kTinyTilesFewest = 8;
 
 bool env_flag(const char *name, int dflt) { return env_int(name, dflt) != 0; }
 
@@ -448,16 +457,42 @@ bool rows_wanted(uint32_t flags, const Shapes &s, const mni_b200_view &w) {
            s.M <= (aligned ? kRowsAligned : kRowsUnaligned);
 }
 
-// Small enough for the one-launch f32 kernel: a single matrix product whose longest contraction (forward K, backward
-// M and N) and whose work are both small, operands readable along one of their dims.  MNI_B200_TINY overrides the limit on
-// M * N * K (0: never).
-bool tiny_wanted(uint32_t flags, const Shapes &s, const mni_b200_view &a, const mni_b200_view &b, const mni_b200_view *dc) {
+// What the one-launch f32 kernel would compute for a call.
+enum TinyCall { kTinyForward, kTinyForwardGelu, kTinyGradA, kTinyGradB, kTinyGradBoth };
+
+// Small enough for the one-launch f32 kernel: a single matrix product whose contraction (forward K, backward M and N), work and
+// tiles are all small, operands readable along one of their dims.  MNI_B200_TINY overrides the limit on M * N * K (0: never).
+bool tiny_wanted(const Call &c, TinyCall call, const Shapes &s, const mni_b200_view &a, const mni_b200_view &b, const mni_b200_view *dc) {
     auto readable = [](const mni_b200_view &v) { return v.stride[v.ndim - 1] == 1 || v.stride[v.ndim - 2] == 1; };
     const uint32_t forced = MNI_B200_FORCE_TENSOR_PATH | MNI_B200_FORCE_SKINNY_PATH | MNI_B200_FORCE_PACK | MNI_B200_PRECISION_TF32;
-    return (flags & forced) == 0 && ((flags >> 16) & 0xffu) == 0 && s.batch == 1 && s.a_batch == 1 && s.b_batch == 1 &&
-           (dc ? std::max(s.M, s.N) : s.K) <= (s.M <= 8 ? kTinyContractionFewRows : kTinyContraction) &&
-           std::max({s.M, s.N, s.K}) <= kTinyWork && s.M * s.N * s.K <= env_int("MNI_B200_TINY", kTinyWork) && readable(a) &&
-           readable(b) && (!dc || readable(*dc));
+    if ((c.flags & forced) != 0 || ((c.flags >> 16) & 0xffu) != 0 || s.batch != 1 || s.a_batch != 1 || s.b_batch != 1 ||
+        (dc ? std::max(s.M, s.N) : s.K) > (s.M <= 8 ? kTinyContractionFewRows : kTinyContraction) ||
+        std::max({s.M, s.N, s.K}) > kTinyWork || s.M * s.N * s.K > env_int("MNI_B200_TINY", kTinyWork) || !readable(a) ||
+        !readable(b) || (dc && !readable(*dc)))
+        return false;
+    const int64_t m = (s.M + 31) / 32, n = (s.N + 31) / 32, k = (s.K + 31) / 32;
+    const bool da = call == kTinyGradA || call == kTinyGradBoth, db = call == kTinyGradB || call == kTinyGradBoth;
+    const int64_t tiles = dc ? (da ? m * k : 0) + (db ? k * n : 0) : m * n;
+    if (s.M > 8) {
+        if (c.capturing && call == kTinyGradBoth) return tiles <= kTinyTiles && std::max(s.M, s.N) <= kTinyContractionCaptured;
+        const bool aligned_rows = (call == kTinyGradA ? s.K : s.N) % 4 == 0;
+        return tiles <= (c.capturing && call != kTinyGradBoth && aligned_rows ? kTinyTilesCaptured : kTinyTiles);
+    }
+    if (tiles <= kTinyTilesFewest && (dc ? std::max(s.M, s.N) : s.K) <= 32) return true;
+    const bool rows_unit = dc ? dc->stride[dc->ndim - 1] == 1 || s.N == 1 : a.stride[a.ndim - 1] == 1 || s.K == 1;
+    const bool weight_aligned = (reinterpret_cast<uintptr_t>(b.ptr) & 15) == 0 && b.stride[b.ndim - 1] == 1 &&
+                                b.stride[b.ndim - 2] % 4 == 0 && s.N % 4 == 0;
+    switch (call) {
+        case kTinyForward:
+            return tiles <= (s.K > 64 ? kTinyTilesFewRows / 2 : kTinyTilesFewRows) &&
+                   (!rows_unit || (weight_aligned && (s.M > 4 || s.K <= 64)));
+        case kTinyForwardGelu: return tiles <= kTinyTilesFewRows;
+        case kTinyGradA: return tiles <= kTinyTilesFewRows && !rows_unit;
+        case kTinyGradB: return tiles <= kTinyTilesFewRows && (!c.capturing || s.M > 2);
+        default:
+            if (!c.capturing) return tiles <= kTinyTiles;
+            return tiles <= (s.M > 4 ? kTinyTilesCaptured : s.M > 2 ? kTinyTilesFewRows / 2 : kTinyTilesFewest);
+    }
 }
 
 // ------------------------------------------------------------------ forward
@@ -471,7 +506,7 @@ int fwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, float *out
     if (s.K == 0) return zero_or_bias_fill(c, out, s.batch * s.M, s.N, bias, accumulate);
 
     if (!*c.label) c.label = "forward: ";
-    if (tiny_wanted(c.flags, s, *a, *b, nullptr)) {
+    if (tiny_wanted(c, kTinyForward, s, *a, *b, nullptr)) {
         c.note("small f32 kernel");
         if (c.dry()) return MNI_B200_OK;
         const TinyProduct p{a->ptr, b->ptr, out, bias, static_cast<int>(s.M), static_cast<int>(s.N), static_cast<int>(s.K),
@@ -540,7 +575,14 @@ int fwd_gelu_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const
     if (!bias || !out) return fail(MNI_B200_ERR_ARG, "bias and out must not be null");
     const uint32_t saved_flags = c.flags;
     c.flags &= ~static_cast<uint32_t>(MNI_B200_ACCUMULATE_C);
-    const bool skinny = (c.flags & MNI_B200_FORCE_SKINNY_PATH) != 0 || tiny_wanted(c.flags, s, *a, *b, nullptr) ||
+    if (s.K > 0 && tiny_wanted(c, kTinyForwardGelu, s, *a, *b, nullptr)) {
+        c.flags = saved_flags;
+        if (c.dry()) return MNI_B200_OK;
+        const TinyProduct p{a->ptr, b->ptr, pre, bias, static_cast<int>(s.M), static_cast<int>(s.N), static_cast<int>(s.K), 0,
+                            a->stride[a->ndim - 2], a->stride[a->ndim - 1], b->stride[b->ndim - 2], b->stride[b->ndim - 1], s.N, out};
+        return launch_tiny(&p, 1, nullptr, c.stream);
+    }
+    const bool skinny = (c.flags & MNI_B200_FORCE_SKINNY_PATH) != 0 ||
                         ((c.flags & MNI_B200_FORCE_TENSOR_PATH) == 0 && s.M <= skinny_fwd_row_limit(s.N));
     if (s.K > 0 && !skinny) {
         GemmProblem p;
@@ -649,7 +691,7 @@ int bwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const mni_
     const bool da_wanted = da && a_elems > 0 && s.N > 0 && g_batch > 0;
     const bool db_wanted = db && b_elems > 0 && s.M > 0 && g_batch > 0;
     if (g_batch == 1 && s.M > 0 && s.N > 0 && s.K > 0 && (da || db) && (!dbias || dc->stride[gn - 1] == 1) &&
-        tiny_wanted(c.flags, s, *a, *b, dc)) {
+        tiny_wanted(c, da && db ? kTinyGradBoth : da ? kTinyGradA : kTinyGradB, s, *a, *b, dc)) {
         c.label = "grad_a, grad_b, grad_bias: ";
         c.note("small f32 kernel");
         c.label = "";
@@ -1259,12 +1301,16 @@ int mni_b200_workspace_query(const mni_b200_view *a, const mni_b200_view *b, uin
     mni_b200_view dc_strided = dc;
     for (int d = 0; d < dc.ndim; ++d) dc_strided.stride[d] = dc.stride[d] * 2;
     size_t need = 0;
-    auto dry = [&](auto body) -> int {
-        Call c;
-        c.st = st; c.arena.dry = true; c.stream = nullptr; c.flags = flags;
-        const int r = body(c);
-        need = std::max(need, c.arena.used);
-        return r;
+    auto dry = [&](auto body) -> int {             // eager and captured calls are planned differently
+        for (const bool capturing : {false, true}) {
+            Call c;
+            c.st = st; c.arena.dry = true; c.stream = nullptr; c.flags = flags;
+            c.capturing = capturing;
+            const int r = body(c);
+            if (r) return r;
+            need = std::max(need, c.arena.used);
+        }
+        return MNI_B200_OK;
     };
     // Outputs on a 16-byte boundary and off it take different plans, and so do calls for both gradients, which may run
     // side by side on half of the SMs each, and calls for one of them.

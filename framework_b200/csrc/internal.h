@@ -201,12 +201,14 @@ RowsLaunch launch_rows_bt_fwd, launch_rows_bt_dx;      // W stored [N, K], seen 
 
 // Products too small for the tensor path, all of a call's in one launch (tiny.cu):
 //   c[m, n] = sum_k a[m, k] . b[k, n] (+ bias) (+ c), each operand with a unit stride in one of its dims
+// act != null (in the first of a call's products, and then in all): c (may be null) = the sum alone, act = gelu(sum + bias)
 struct TinyProduct {
     const float *a, *b;
     float *c;
     const float *bias;
     int M, N, K, accumulate;
     long long a_m, a_k, b_k, b_n, ldc;
+    float *act = nullptr;
 };
 //   out[j] (+)= sum_r src[r, j]
 struct TinyColumns {

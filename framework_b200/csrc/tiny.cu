@@ -8,6 +8,10 @@
 // with a private slice of shared memory (no barrier in the loop) and the next run's loads in registers while the current
 // one is multiplied: a lane keeps 8 x 4 outputs, so three 16-byte reads feed 32 FMAs.  The warps' sums are added in warp
 // order: results do not depend on scheduling.
+//
+// Its stores are single elements and a tile's 256 threads take a slot whatever the tile holds, so it is for calls of few tiles:
+// api.cu has the limits.
+#include "activation.h"
 #include "internal.h"
 
 #include <algorithm>
@@ -72,6 +76,8 @@ __device__ __forceinline__ void load_step(Lane &l, int K, float (&v)[8]) {
     l.k += kRun * kWarps;
 }
 
+// ACT: the products are followed by bias + GELU (its registers cost the others 0.5 us in 6).
+template <bool ACT>
 __global__ void __launch_bounds__(kThreads)
 tiny_kernel(const __grid_constant__ Jobs jobs) {
     __shared__ __align__(16) float mem[kWarps * kTile * kPitch];     // operand slices [warp][2][kRun][kPitch], then the sums
@@ -152,10 +158,16 @@ tiny_kernel(const __grid_constant__ Jobs jobs) {
         s.x += t.x; s.y += t.y; s.z += t.z; s.w += t.w;
     }
     float out[4] = {s.x, s.y, s.z, s.w};
-    float *dst = p.c + (m0 + row) * p.ldc + n0 + col;
+    const long long at = (m0 + row) * p.ldc + n0 + col;
+    float *dst = p.c + at;
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
         if (n0 + col + e >= p.N) break;
+        if (ACT) {
+            if (p.c) dst[e] = out[e];
+            p.act[at + e] = gelu_tanh(out[e] + __ldg(p.bias + n0 + col + e));
+            continue;
+        }
         if (p.bias) out[e] += __ldg(p.bias + n0 + col + e);
         if (p.accumulate) out[e] += dst[e];
         dst[e] = out[e];
@@ -182,7 +194,7 @@ int launch_tiny(const TinyProduct *products, int count, const TinyColumns *colum
         blocks += static_cast<unsigned>((columns->n + 31) / 32);
     }
     if (blocks == 0) return MNI_B200_OK;
-    const cudaError_t e = launch_dependent(tiny_kernel, dim3(blocks), dim3(kThreads), 0, stream, jobs);
+    const cudaError_t e = launch_dependent(products[0].act ? tiny_kernel<true> : tiny_kernel<false>, dim3(blocks), dim3(kThreads), 0, stream, jobs);
     if (e != cudaSuccess) return fail(MNI_B200_ERR_CUDA, "tiny_kernel launch failed: %s", cudaGetErrorString(e));
     MNI_LAUNCH_CHECK("tiny_kernel");
     return MNI_B200_OK;

@@ -191,3 +191,49 @@ def test_a_call_honours_a_switch_however_many_are_set(F, monkeypatch):
         monkeypatch.setenv(f"MNI_B200_UNUSED_{i}", "1")
     monkeypatch.setenv("MNI_B200_TINY", "0")
     assert launches() >= 2
+
+
+@pytest.mark.parametrize("m,k,n", [(1, 1, 1), (9, 8, 7), (31, 33, 32), (33, 65, 129), (8, 128, 1024), (320, 320, 64), (3, 70, 517)])
+@pytest.mark.parametrize("want_pre", [False, True])
+def test_small_products_with_gelu_in_one_launch(F, m, k, n, want_pre):
+    rng = _rng(8, m, k, n)
+    a, b = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((k, n)).astype(np.float32) / np.sqrt(k).astype(np.float32)
+    bias = rng.standard_normal(n).astype(np.float32)
+    launches = F.launch_count()
+    pre, out = F.matmul_bias_gelu(*(F.DeviceTensor.from_numpy(x) for x in (a, b, bias)), want_pre=want_pre)
+    F.device_status()
+    assert F.launch_count() - launches == 1
+    want = a.astype(np.float64) @ b.astype(np.float64)
+    assert (pre is not None) == want_pre and (not want_pre or rel_fro(pre.numpy(), want) <= regression_bound_3xtf32(k))
+    v = want + bias
+    assert rel_fro(out.numpy(), 0.5 * v * (1 + np.tanh(0.7978845608028654 * (v + 0.044715 * v ** 3)))) <= regression_bound_3xtf32(k)
+
+
+@pytest.mark.parametrize("m,k,n", [(9, 40, 7000), (700, 40, 900), (8, 96, 7900), (8, 100, 8300), (4, 64, 8000), (5, 65, 33)])
+def test_products_around_the_limits_of_the_small_kernel(F, m, k, n):
+    """Either side of the tile limits, eager and captured, whose limits differ: the same products."""
+    import torch
+    rng = _rng(9, m, k, n)
+    a, b, g = (rng.standard_normal(s).astype(np.float32) for s in ((m, k), (k, n), (m, n)))
+    ad, bd, gd = (F.DeviceTensor.from_numpy(x) for x in (a, b, g))
+    a64, b64, g64 = (x.astype(np.float64) for x in (a, b, g))
+    outs = [Guarded(F, s) for s in ((m, n), (m, k), (k, n), (n,))]
+
+    def call():
+        F.matmul(ad, bd, out=outs[0].tensor)
+        F.matmul_backward(gd, ad, bd, da=outs[1].tensor, db=outs[2].tensor, dbias=outs[3].tensor, want_dbias=True)
+
+    def check():
+        F.device_status()
+        for got, want in zip(outs, (a64 @ b64, g64 @ b64.T, a64.T @ g64, g64.sum(0))):
+            got.check()
+            assert rel_fro(got.tensor.numpy(), want) <= regression_bound_3xtf32(max(m, k, n))
+    call()
+    check()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        call()
+    for o in outs:
+        o.tensor.storage.zero_()
+    graph.replay()
+    check()

@@ -174,6 +174,22 @@ def test_exchanged_operands_keep_to_the_plans_that_store_transposed(plan, monkey
     assert (cut["exchanged"], cut["tail_ways"]) == (0, 3)
 
 
+def test_small_products_are_those_of_few_tiles(plan):
+    """The one-launch f32 kernel takes calls of at most 800 tiles of 32 x 32, and of few rows only where the streaming kernels,
+    which read the weight in 16-byte units, do not do better."""
+    def small(m, k, n, backward=0):
+        return all("small f32 kernel" in line for line in plan((m, k), (k, n), backward=backward))
+    for shape in ((32, 64, 32), (128, 128, 128), (192, 192, 192), (9, 8, 7), (700, 3, 1000), (8, 8, 4512), (8, 90, 1656), (2, 8, 3568), (1, 1, 1)):
+        assert small(*shape), shape
+    for shape in ((2048, 1, 4096), (100000, 2, 40), (65536, 128, 1), (9, 1, 900000), (1024, 8, 1024), (4096, 4, 512),      # tiles
+                  (1, 128, 65536), (1, 64, 131072), (8, 16, 65536), (1, 128, 1024), (8, 8, 37266), (1, 8, 19862), (256, 512, 64), (8, 128, 8192)):
+        assert not small(*shape), shape
+    for shape in ((32, 64, 32), (8, 12704, 8), (4, 4096, 64), (100, 1, 300)):
+        assert small(*shape, backward=2), shape
+    for shape in ((1, 65536, 128), (300, 27000, 1), (1, 131072, 64), (8, 65536, 16)):
+        assert not small(*shape, backward=2), shape
+
+
 def test_staging_patches_are_one_or_two(plan, monkeypatch):
     """A patch per epilogue warp more costs pipeline stages; any other number than two leaves the default."""
     def stages():
