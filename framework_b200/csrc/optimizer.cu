@@ -3,7 +3,7 @@
 //
 // HBM-bound: the step reads grad and reads and writes param, m and v once (28 bytes per element), the norm reads grad
 // once more.  A model's parameters are a list of tensors from a few hundred elements to millions, so the unit of work
-// is a chunk of 4096 elements of whichever tensor: ONE launch covers up to kMaxList tensors, whose addresses travel as
+// is a chunk of whichever tensor: ONE launch covers up to kMaxList tensors, whose addresses travel as
 // a kernel parameter, and a block finds its chunk's tensor by bisection over the chunk offsets (constant memory).
 // 74 tensors, 42.5 M elements: 222 launches and 1158 us a step before, of which the device worked ~400.
 #include "internal.h"
@@ -20,7 +20,11 @@ namespace mni {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kChunk = 4096;                 // elements per block of the step: 4 vectors of each array per thread
+constexpr int kChunk = 4096;                 // elements per block of the norm
+// Elements per block of the step.  A list: four vectors of each array per thread, which pay for finding the block's tensor (74
+// tensors, 42.5 M elements: 221 us; 226 with one vector).  A single tensor: one, as what such a call waits for is a block's
+// later vectors (65 536 elements 7.8 us against 3.4) or a nearly empty third round of blocks (5 M 25.2 / 19.8; 50 M 224 / 215).
+__host__ __device__ constexpr int step_chunk(int cap) { return cap == 1 ? 1024 : 4096; }
 constexpr int kMaxList = 512;                // tensors per launch (24 KB of kernel parameters at most)
 constexpr int kMaxNormBlocks = 1024;
 
@@ -70,19 +74,20 @@ __device__ __forceinline__ float clip_scale(const double *sumsq, float max_norm)
 // fetched before the wait (the norm kernel was launched the ordinary way, so whatever wrote the operands is complete
 // once it runs).
 template <int CAP>
-__global__ void __launch_bounds__(kThreads, 4)
+__global__ void __launch_bounds__(kThreads, CAP == 1 ? 6 : 4)
 adamw_list_kernel(const __grid_constant__ StepList<CAP> list, const AdamWArgs a) {
+    constexpr int CHUNK = step_chunk(CAP);
     const unsigned chunk = list.first[list.count] - 1 - blockIdx.x;
     const int t = find_tensor(list.first, list.count, chunk);
-    const long long base = static_cast<long long>(chunk - list.first[t]) * kChunk, n = list.n[t];
+    const long long base = static_cast<long long>(chunk - list.first[t]) * CHUNK, n = list.n[t];
     float *param = list.param[t], *m = list.m[t], *v = list.v[t], *grad = list.grad[t];
     const bool vec = ((reinterpret_cast<uintptr_t>(param) | reinterpret_cast<uintptr_t>(m) |
                        reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(grad)) & 15) == 0;
-    if (vec && base + kChunk <= n) {
-        constexpr int U = 2;
-        float scale = 1.0f;
+    float scale = 1.0f;
+    if (vec && base + CHUNK <= n) {
+        constexpr int PER = CHUNK / (kThreads * 4), U = PER < 2 ? PER : 2;
 #pragma unroll
-        for (int h = 0; h < kChunk / (kThreads * 4 * U); ++h) {
+        for (int h = 0; h < PER / U; ++h) {
             float4 p[U], mm[U], vv[U], g[U];
             long long at[U];
 #pragma unroll
@@ -114,17 +119,36 @@ adamw_list_kernel(const __grid_constant__ StepList<CAP> list, const AdamWArgs a)
         }
         return;
     }
-    // a tensor's last, partial chunk, or one that is not 16-byte aligned
-    grid_dependency_wait();
-    const float scale = clip_scale(a.sumsq, a.max_norm);
-    const long long end = min(n, base + kChunk);
-    for (long long i = base + threadIdx.x; i < end; i += kThreads) {
-        float g = grad[i];
-        if (scale != 1.0f) {
-            g *= scale;
-            if (a.write_grad) grad[i] = g;
+    // A tensor's last, partial chunk, or one that is not 16-byte aligned: four elements of each array of a thread on their way
+    // together (one after the other they cost a round trip to memory each: 3100 elements 11.6 us, now 3.0).
+    const long long end = min(n, base + CHUNK);
+#pragma unroll 1
+    for (int h = 0; h < CHUNK; h += 4 * kThreads) {
+        const long long i0 = base + h + threadIdx.x;
+        float p[4], mm[4], vv[4], g[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const long long i = i0 + u * kThreads;
+            if (i >= end) continue;
+            p[u] = param[i]; mm[u] = m[i]; vv[u] = v[i];
+            g[u] = __ldcs(grad + i);
         }
-        adamw_one(param[i], m[i], v[i], g, a);
+        if (h == 0) {
+            grid_dependency_wait();
+            scale = clip_scale(a.sumsq, a.max_norm);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const long long i = i0 + u * kThreads;
+            if (i >= end) continue;
+            if (scale != 1.0f) {
+                g[u] *= scale;
+                if (a.write_grad) grad[i] = g[u];
+            }
+            adamw_one(p[u], mm[u], vv[u], g[u], a);
+            param[i] = p[u]; m[i] = mm[u]; v[i] = vv[u];
+        }
+        if (i0 + 4 * kThreads - threadIdx.x >= end) break;
     }
 }
 
@@ -202,7 +226,7 @@ sumsq_list_kernel(const __grid_constant__ NormList<CAP> list, double *out, int a
     }
 }
 
-unsigned chunks_of(int64_t n) { return static_cast<unsigned>((n + kChunk - 1) / kChunk); }
+unsigned chunks_of(int64_t n, int chunk) { return static_cast<unsigned>((n + chunk - 1) / chunk); }
 
 template <int CAP>
 int launch_step(const AdamWArgs &a, int count, float *const *param, float *const *m, float *const *v, float *const *grad,
@@ -215,7 +239,7 @@ int launch_step(const AdamWArgs &a, int count, float *const *param, float *const
         const int k = list.count++;
         list.param[k] = param[i]; list.m[k] = m[i]; list.v[k] = v[i]; list.grad[k] = grad[i];
         list.n[k] = n[i];
-        list.first[k + 1] = list.first[k] + chunks_of(n[i]);
+        list.first[k + 1] = list.first[k] + chunks_of(n[i], step_chunk(CAP));
     }
     if (list.count == 0) return MNI_B200_OK;
     const dim3 grid(list.first[list.count]), block(kThreads);
@@ -240,7 +264,7 @@ int launch_norm(int count, const float *const *grad, const int64_t *n, double *o
         const int k = list.count++;
         list.grad[k] = grad[i];
         list.n[k] = n[i];
-        list.first[k + 1] = list.first[k] + chunks_of(n[i]);
+        list.first[k + 1] = list.first[k] + chunks_of(n[i], kChunk);
     }
     const unsigned chunks = list.first[list.count];
     const unsigned blocks = std::max(1u, std::min(chunks, static_cast<unsigned>(std::min(6 * sm_count, kMaxNormBlocks))));
@@ -252,9 +276,25 @@ int launch_norm(int count, const float *const *grad, const int64_t *n, double *o
 // Memory that the step of entry `entry` writes.
 struct Span { uintptr_t begin, end; int64_t entry; };
 
-// Whether the steps of two entries touch the same memory.  A model's tensors mostly come in the order of their addresses: four
-// sorted runs that only need merging.
+// Whether the steps of two entries touch the same memory.  A model's tensors mostly come in the order of their addresses, each
+// kind in a buffer of its own, where one look at each settles it; or else as four sorted runs that only need merging.  (The
+// kernel of a short list's norm is over in 5 us, and the step is launched behind this check.)
 bool entries_overlap(int64_t count, float *const *const (&arrays)[4], const int64_t *n) {
+    Span range[4];
+    bool settled = true;
+    for (int k = 0; k < 4 && settled; ++k) {
+        range[k] = Span{0, 0, -1};
+        for (int64_t i = 0; i < count && settled; ++i) {
+            if (n[i] == 0) continue;
+            const uintptr_t at = reinterpret_cast<uintptr_t>(arrays[k][i]);
+            settled = at >= range[k].end;
+            if (range[k].entry < 0) range[k].begin = at;
+            range[k].end = at + static_cast<uintptr_t>(n[i]) * sizeof(float);
+            range[k].entry = i;
+        }
+        for (int j = 0; j < k && settled; ++j) settled = range[k].begin >= range[j].end || range[j].begin >= range[k].end;
+    }
+    if (settled) return false;
     std::vector<Span> spans;
     spans.reserve(static_cast<size_t>(4 * count));
     auto less = [](const Span &a, const Span &b) { return a.begin < b.begin; };
@@ -327,7 +367,7 @@ int launch_adamw_list(const AdamWArgs &a, int64_t count, float *const *param, fl
         }
         const int k = static_cast<int>(k64);
         // the parameter block is copied at every launch, so a short list takes a short one
-        auto launch = k <= 16 ? launch_step<16> : k <= 128 ? launch_step<128> : launch_step<kMaxList>;
+        auto launch = k == 1 ? launch_step<1> : k <= 16 ? launch_step<16> : k <= 128 ? launch_step<128> : launch_step<kMaxList>;
         const int rc = launch(a, k, param + i, m + i, v + i, grad + i, n + i, dependent && i == 0, stream);
         if (rc) return rc;
     }

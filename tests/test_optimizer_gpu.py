@@ -135,8 +135,10 @@ def test_parameter_lists_around_the_chunk_and_launch_limits(F, oracle, sizes, mi
 
 @pytest.mark.parametrize("max_norm", [0.0, 0.5])
 def test_tensors_that_share_memory_are_stepped_in_list_order(F, max_norm):
-    """Tied parameters given twice, a parameter that overlaps another's part, state shared by two parameters: bit for bit what
-    the list gives one tensor at a time."""
+    """Tied parameters given twice, a parameter that overlaps another's part, state shared by two parameters: what the list gives
+    one tensor at a time.  The kernels of a list and of one tensor may contract the same expressions differently, four
+    roundings a step of terms below 1 + |x|, and no element is stepped more than three times; a step left out or taken out of turn
+    is three orders of magnitude above that."""
     import torch
     n = 70_000
     rng = np.random.default_rng(11)
@@ -161,7 +163,7 @@ def test_tensors_that_share_memory_are_stepped_in_list_order(F, max_norm):
         F.adamw_step(*one, grad_sumsq=sumsq, **cfg)
     assert norm == float(np.sqrt(np.float32(sumsq.item())))
     for a, b in zip(got_bufs, want_bufs):
-        assert torch.equal(a, b)
+        assert bool(((a - b).abs() <= 12 * 2.0 ** -24 * (1 + b.abs())).all())
     assert launches == 1 + 3             # the norm, then entries 0-1, 2-3 and 4-8: a launch ends before an overlap
 
 
@@ -172,3 +174,25 @@ def test_tensors_that_only_touch_need_one_launch(F):
     launches = F.launch_count()
     F.clip_and_step(*lists, lr=1e-3)
     assert F.launch_count() - launches == 2
+
+
+@pytest.mark.parametrize("sizes,misalign", [([1, 255, 1023, 1024, 1025, 2047], 0), ([1025, 1024, 300], 3), ([5000], 0), ([1021], 1), ([4095, 4097, 8193], 0),
+                                            ([4096, 9000], 2), ([3072], 0)])
+def test_step_around_its_chunk(F, oracle, sizes, misalign):
+    """A single tensor is stepped 1024 elements a block, a list 4096, partial and unaligned chunks four elements at a time."""
+    import torch
+    rng = np.random.default_rng(sum(sizes))
+    host = {name: [np.abs(scale * rng.standard_normal(n)).astype(np.float32) for n in sizes]
+            for name, scale in (("p", 1.0), ("m", 0.1), ("v", 0.01), ("g", 1.0))}
+    flat = {name: [torch.full((n + misalign + 4,), 7.0, device="cuda") for n in sizes] for name in host}
+    dev = {name: [F.DeviceTensor(f[misalign:misalign + n], (n,)) for f, n in zip(flat[name], sizes)] for name in host}
+    for name in host:
+        for d, a in zip(dev[name], host[name]):
+            d.storage.copy_(torch.from_numpy(a))
+    cfg = dict(lr=1e-3, weight_decay=0.01, step=2, max_grad_norm=0.3)
+    oracle.clip_and_step(host["p"], host["m"], host["v"], host["g"], beta1=0.9, beta2=0.999, eps=1e-8, **cfg)
+    F.clip_and_step(dev["p"], dev["m"], dev["v"], dev["g"], **cfg)
+    for name in host:
+        for d, r, f, n in zip(dev[name], host[name], flat[name], sizes):
+            assert float(np.max(np.abs(d.numpy() - r))) <= 2e-6 * (1 + float(np.abs(r).max())), name
+            assert bool((f[:misalign] == 7).all()) and bool((f[misalign + n:] == 7).all())
