@@ -1599,16 +1599,43 @@ struct Plan {
 
 constexpr size_t kFixedSmemNoEpi = 1024 + kBarBytes;
 
-// Split tail of `tiles` 256-wide pair tiles: after at least one whole round, a last wave that fills at most half of the
-// slots, in a schedule that would idle more than a fifth of them, is cut into two to four units per tile of at least 128
-// contraction elements each.  1: no cut.
-long long cut_ways(long long tiles, long long slots, long long k) {
-    const long long full = tiles / slots, rem = tiles - full * slots;
-    const long long ways = rem > 0 ? std::min<long long>(slots / rem, 4) : 1;
-    const double eff = static_cast<double>(tiles) / static_cast<double>((full + 1) * slots);
-    return full >= 1 && ways >= 2 && eff < 0.80 && k / ways >= 128 ? ways : 1;
-}
+// Split tail of `tiles` 256-wide pair tiles: the last wave's tiles cut into `ways` units each (1: not), and what the schedule then
+// takes, in rounds of whole tiles, and the finish in microseconds.
+struct Cut {
+    long long ways;
+    double rounds, finish_us;
+};
+constexpr double kPairNs = 30.0;             // main loop of a 256-wide pair, 3xTF32, per contraction element
+// Microseconds of a finish kernel that adds `parts` partial results of `bytes` each: its launch and its traffic.
+double finish_us(double parts, double bytes) { return 1.5 + (parts + 1.0) * bytes * 1e-6 / 3.0; }
 
+// After at least one whole round, a last wave that fills at most half of the slots, in a schedule that would idle more than a
+// fifth of them, is cut into two to four units per tile of at least 128 contraction elements each.  Otherwise, where a round
+// takes long, into as many units as even out best over several short rounds, if that saves 6 % and 5 us: 3xTF32 contractions from
+// about 3000 on with 0.5 to 0.8 or 1.5 to 1.75 waves of tiles (74 pairs; us whole / balanced tail / cut): 2048 x 4096 x 1280
+// 128 / 91 / 92, 2048 x 8192 x 1280 242 / 174 / 176, 1536 x 8192 x 2048 239 / 197 / 191, 2048 x 8192 x 3584 500 / 436 / 439,
+// 2048 x 3072 x 3584 177 / 169 / 168; at K = 2048, 121 / 117 / -, it would save 4.6 %.  Not in single-pass mode, whose long units
+// lose more by giving up their running sum (2048 x 8192 x 3584 200 / 209 / 231).
+Cut cut_tail(long long tiles, long long slots, long long k, bool single_pass) {
+    const long long full = tiles / slots, rem = tiles - full * slots;
+    const double tile_bytes = 4.0 * 2 * BM * 256;
+    const Cut whole{1, static_cast<double>(rem > 0 ? full + 1 : full), 0.0};
+    if (rem == 0) return whole;
+    const long long ways = std::min<long long>(slots / rem, 4);
+    const double eff = static_cast<double>(tiles) / static_cast<double>((full + 1) * slots);
+    if (full >= 1 && ways >= 2 && eff < 0.80 && k / ways >= 128)
+        return Cut{ways, static_cast<double>(full) + 1.0 / static_cast<double>(ways), finish_us(static_cast<double>(ways), tile_bytes * static_cast<double>(rem))};
+    if (single_pass) return whole;
+    const double round_us = static_cast<double>(k) * kPairNs * 1e-3;
+    Cut best = whole;
+    for (long long w = 2; w <= 6 && k / w >= 256; ++w) {
+        const Cut c{w, static_cast<double>(full) + static_cast<double>((rem * w + slots - 1) / slots) / static_cast<double>(w),
+                    finish_us(static_cast<double>(w), tile_bytes * static_cast<double>(rem))};
+        if (c.rounds * round_us + c.finish_us < best.rounds * round_us + best.finish_us) best = c;
+    }
+    const double saved = (whole.rounds - best.rounds) * round_us - best.finish_us;
+    return saved > 5.0 && saved > 0.06 * whole.rounds * round_us ? best : whole;
+}
 // Longest accumulation chain in tensor memory, in k-blocks (MNI_B200_CHUNK_K contraction elements; 0 = no limit).  The fused
 // activation needs the whole sum in one accumulator.
 int chunk_iters_for(const GemmProblem &p, int bk) {
@@ -1652,6 +1679,12 @@ Plan make_plan(const GemmProblem &p, int sm_count) {
                 const double t = rounds * (k_eff / sp) * c_ns + (sp > 1 ? 1500.0 + (sp + 1) * out_bytes / 3000.0 : 0.0);
                 if (t < best) { best = t; pl.bn = bn; model_splits = sp; }
             }
+            // ... or a single, partly filled wave of 256-wide pairs cut like a last one
+            if (bn == 256 && cg == 2 && !p.exchanged && tiles < slots) {
+                const Cut cut = cut_tail(tiles, slots, p.fold * ((p.K + 15) / 16) * 16, p.fast_tf32);
+                const double t = cut.rounds * k_eff * kPairNs + cut.finish_us * 1e3;
+                if (cut.ways > 1 && t < 0.97 * best) { best = t; pl.bn = bn; model_splits = 1; }
+            }
         }
         pl.est_us = best * 1e-3 + kFixedUs;
     }
@@ -1667,12 +1700,12 @@ Plan make_plan(const GemmProblem &p, int sm_count) {
             const int cg = pair_for(bn);
             const long long tiles = static_cast<long long>(p.batch) * ((p.M + BM * cg - 1) / (BM * cg)) * ((p.N + bn - 1) / bn);
             const long long slots = std::max(1, sm_count / cg);
-            const double loop = k_us * (bn == 256 ? (cg == 2 ? 30.0 : 33.0) : (bn == 128 ? 19.0 : 13.0)) + (bn == 256 ? 0.5 : (bn == 128 ? 1.0 : 0.65));
+            const double loop = k_us * (bn == 256 ? (cg == 2 ? kPairNs : 33.0) : (bn == 128 ? 19.0 : 13.0)) + (bn == 256 ? 0.5 : (bn == 128 ? 1.0 : 0.65));
             const double write = unaligned * (bn == 256 ? (cg == 2 ? 3.7 : 4.5) : (bn == 128 ? 2.2 : 1.5));
             double rounds = static_cast<double>((tiles + slots - 1) / slots);
             if (bn == 256 && cg == 2) {
-                const long long ways = cut_ways(tiles, slots, p.fold * ((p.K + 15) / 16) * 16);
-                if (ways > 1) rounds += 1.0 / static_cast<double>(ways) - 0.75;
+                const Cut cut = cut_tail(tiles, slots, p.fold * ((p.K + 15) / 16) * 16, p.fast_tf32);
+                if (cut.ways > 1) rounds = cut.rounds + 0.25;
             }
             const double t = rounds * std::max(loop, write);
             if (t < best) { best = t; pl.bn = bn; }
@@ -1710,6 +1743,17 @@ Plan make_plan(const GemmProblem &p, int sm_count) {
     } else if (tiles * 2 <= slots && iters >= 8) {
         // Few output tiles and a long contraction: split K so that the whole GPU works.
         splits = static_cast<int>(std::min<long long>(slots / tiles, iters / 4));
+    } else if (pl.ta && iters * pl.bk >= 2048) {
+        // Narrow tiles in a few long rounds: the contraction split two to four ways where that evens them out by 6 % and 5 us
+        // (100 x [384 x 4096 x 64], 300 tiles on 148 SMs: 182 -> 172 us; 200 x [128 x 2048 x 64]: 74 -> 68).
+        const double round_us = static_cast<double>(iters * pl.bk) * (pl.bn == 128 ? 20.5e-3 : 16.0e-3);
+        const double bytes = 4.0 * static_cast<double>(p.batch) * static_cast<double>(p.M) * static_cast<double>(p.N);
+        const double whole = static_cast<double>((tiles + slots - 1) / slots) * round_us;
+        double best = std::min(0.94 * whole, whole - 5.0);
+        for (int sp = 2; sp <= 4; ++sp) {
+            const double t = static_cast<double>((tiles * sp + slots - 1) / slots) / sp * round_us + finish_us(sp, bytes);
+            if (t < best) { best = t; splits = sp; }
+        }
     }
     splits = static_cast<int>(std::max<long long>(1, std::min<long long>(std::min<long long>(splits, iters), 64)));
     pl.splits = splits;
@@ -1721,9 +1765,10 @@ Plan make_plan(const GemmProblem &p, int sm_count) {
     pl.sk_first_tile = 0;
     pl.tail_ways = pl.tail_tiles = 0;
     pl.running = false;
-    // MNI_B200_STREAMK=1 turns it on where whole tiles would idle more than 8 % of the slot-rounds.  Off by default: parking
-    // and adding the shared tiles costs more than the idle slots at every size measured (24 x [512 x 512 x 64] 19.9 us
-    // against 12.4, 6 x 700^3 42.1 / 29.0, 3000 x 1000 x 900 45.8 / 37.7, 1000 x 2000 x 3000 63.8 / 65.4).
+    // MNI_B200_STREAMK=1 turns it on where whole tiles would idle more than 8 % of the slot-rounds.  Off by default: where the
+    // contraction is short, parking and adding the shared tiles costs more than the idle slots (24 x [512 x 512 x 64] 19.9 us
+    // against 12.4, 6 x 700^3 42.1 / 29.0, 3000 x 1000 x 900 45.8 / 37.7), where it is long the cut below is as fast and its
+    // accumulation chains are shorter.
     // MNI_B200_STREAMK=0 turns the split tail below off as well.
     const int sk_env = env_int("MNI_B200_STREAMK", -1);
     // The split tail's partial tiles are added by one small kernel.  2048 x 3072, K = 768 (96 tiles on 74 pairs): two
@@ -1731,10 +1776,11 @@ Plan make_plan(const GemmProblem &p, int sm_count) {
     // Neither it nor the running sum is built for exchanged operands, whose patches leave transposed (the planner's own
     // choice there is a 64-wide tile; MNI_B200_BN=256 makes it a 256-wide pair).
     if (splits == 1 && sk_env < 0 && p.force_splits <= 0 && pl.cg == 2 && pl.bn == 256 && !p.exchanged) {
-        const long long ways = cut_ways(tiles, slots, iters * pl.bk);
-        if (ways > 1) {
-            pl.tail_ways = static_cast<int>(ways);
+        const Cut cut = cut_tail(tiles, slots, iters * pl.bk, p.fast_tf32);
+        if (cut.ways > 1) {
+            pl.tail_ways = static_cast<int>(cut.ways);
             pl.tail_tiles = static_cast<int>(tiles % slots);
+            pl.grid = static_cast<int>(std::min<long long>(tiles + pl.tail_tiles * (cut.ways - 1), slots)) * pl.cg;
             return pl;
         }
     }

@@ -237,3 +237,31 @@ def test_products_around_the_limits_of_the_small_kernel(F, m, k, n):
         o.tensor.storage.zero_()
     graph.replay()
     check()
+
+
+@pytest.mark.parametrize("m,k,n,batch", [
+    (2048, 3072, 1280, ()),       # 40 tiles of 256 x 256 on 74 pairs, no whole round: cut into three units each
+    (1530, 4100, 2047, ()),       # 48, ragged edges, unaligned rows
+    (2040, 3080, 3500, ())])      # 112: one round and 38 tiles cut into three
+@pytest.mark.parametrize("mode", ["plain", "accumulate", "gelu"])
+def test_long_contractions_cut_into_several_rounds_of_units(F, m, k, n, batch, mode):
+    rng = _rng(10, m, k, n)
+    a, b = rng.standard_normal(batch + (m, k)).astype(np.float32), rng.standard_normal(batch + (k, n)).astype(np.float32)
+    b /= np.sqrt(k).astype(np.float32)
+    bias, c0 = rng.standard_normal(n).astype(np.float32), rng.standard_normal(batch + (m, n)).astype(np.float32)
+    ad, bd, biasd = (F.DeviceTensor.from_numpy(x) for x in (a, b, bias))
+    assert "tail_ways=0" not in F.plan_describe(a.shape, b.shape)[0]
+    want = a.astype(np.float64) @ b.astype(np.float64)
+    if mode == "gelu":
+        pre, got = F.matmul_bias_gelu(ad, bd, biasd)
+        F.device_status()
+        # one accumulator holds a unit's whole share of the contraction here: 2.35e-9 an element and pass of it
+        assert rel_fro(pre.numpy(), want) <= regression_bound_3xtf32(k) + 7.1e-9 * k / 3
+        v = want + bias
+        assert rel_fro(got.numpy(), 0.5 * v * (1 + np.tanh(0.7978845608028654 * (v + 0.044715 * v ** 3)))) <= regression_bound_3xtf32(k) + 7.1e-9 * k / 3
+        return
+    out = Guarded(F, want.shape, init=c0 if mode == "accumulate" else None)
+    F.matmul(ad, bd, biasd, out=out.tensor, flags=F._lib.ACCUMULATE_C if mode == "accumulate" else 0)
+    F.device_status()
+    out.check("product", fully_written=mode != "accumulate")
+    assert rel_fro(out.tensor.numpy(), want + bias + (c0 if mode == "accumulate" else 0)) <= regression_bound_3xtf32(k)

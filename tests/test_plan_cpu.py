@@ -174,6 +174,20 @@ def test_exchanged_operands_keep_to_the_plans_that_store_transposed(plan, monkey
     assert (cut["exchanged"], cut["tail_ways"]) == (0, 3)
 
 
+def test_long_contractions_over_a_ragged_wave_are_cut(plan):
+    """A partly filled wave of 256-wide pairs, alone or last, is cut into units where the contraction is long enough to pay for
+    adding them; the grid is then full.  Narrow tiles in a few long rounds are split."""
+    def f(m, k, n, batch=(), **kw):
+        return tensor_plan(plan(batch + (m, k), batch + (k, n), **kw), "forward")
+    for m, k, n, ways in ((2048, 4096, 1280, 5), (1536, 8192, 2048, 3), (1280, 8192, 2560, 4), (2048, 3072, 3584, 3)):
+        p = f(m, k, n)
+        assert (p["bn"], p["pair"], p["splits"], p["tail_ways"], p["grid"], p["running"]) == (256, 1, 1, ways, 148, 0), p
+    for m, k, n in ((2048, 2048, 3584), (2048, 1024, 3584), (4096, 1024, 4096), (8192, 8192, 8192), (2048, 2048, 1280)):
+        assert f(m, k, n)["tail_ways"] == 0, (m, k, n)
+    assert f(2048, 8192, 3584, flags=1)["tail_ways"] == 0
+    assert f(384, 4096, 64, (100,))["splits"] > 1 and f(384, 512, 64, (100,))["splits"] == 1
+
+
 def test_small_products_are_those_of_few_tiles(plan):
     """The one-launch f32 kernel takes calls of at most 800 tiles of 32 x 32, and of few rows only where the streaming kernels,
     which read the weight in 16-byte units, do not do better."""
