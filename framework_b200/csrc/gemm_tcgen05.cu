@@ -804,8 +804,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         }
                     }
                     // Stages the 32 values of this lane's row into the warp's next patch and hands the
-                    // patch to the TMA unit (store, or reduce-add for C += ...).
-                    auto emit = [&](const CUtensorMap *map, bool reduce) {
+                    // patch to the TMA unit (store, or reduce-add for C += ...).  `gelu`: applied to the staged row, four
+                    // elements at a time: unrolled over the row's registers its code, which few calls run, took the place of the
+                    // others' in the instruction cache (100 x [256 x 512 x 64] 19.3 -> 21.7 us).
+                    auto emit = [&](const CUtensorMap *map, bool reduce, bool gelu = false) {
                         const long long t_wg0 = p.prof ? clock64() : 0;
                         if (lane == 0 && in_flight == p.epi_patches) {   // the patch must have been read by its store
                             if (p.epi_patches == 1) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
@@ -828,6 +830,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                                 *reinterpret_cast<float4 *>(dst + ((j ^ (lane & 7)) << 4)) =
                                     make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
                                                 __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
+                            if (gelu) {
+#pragma unroll 1
+                                for (int j = 0; j < 8; ++j) {
+                                    float4 *const at = reinterpret_cast<float4 *>(dst + ((j ^ (lane & 7)) << 4));   // no bank conflicts
+                                    const float4 x = *at;
+                                    *at = make_float4(gelu_tanh(x.x), gelu_tanh(x.y), gelu_tanh(x.z), gelu_tanh(x.w));
+                                }
+                            }
                         }
                         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                         __syncwarp();
@@ -868,9 +878,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         }
                     }
                     if (do_act) {
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(gelu_tanh(__uint_as_float(v[j])));
-                        emit(&tmD, false);
+                        emit(&tmD, false, true);
                     } else if (part) {
                         emit(&tmP, add_piece);
                     } else if (RUN || use_tma) {
