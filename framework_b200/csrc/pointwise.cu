@@ -34,10 +34,11 @@ __device__ __forceinline__ void store_cols(float *dst, long long col, long long 
     if (col + 2 < n) dst[2] = s.z;
     if (col + 3 < n) dst[3] = s.w;
 }
-// Adds the 8 warps' values in warp order; the result is valid in warp 0.
+// Adds the 8 warps' values in warp order; the result is valid in warp 0.  AGAIN: red may still be read from an earlier fold.
+template <bool AGAIN>
 __device__ __forceinline__ float4 fold_warps(float4 (*red)[32], const float4 &acc) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    __syncthreads();                          // red may still be read from an earlier fold
+    if (AGAIN) __syncthreads();
     red[warp][lane] = acc;
     __syncthreads();
     float4 s = red[0][lane];
@@ -56,7 +57,7 @@ __device__ __forceinline__ void finish_colsum(const float4 &acc, float4 (*red)[3
     unsigned int *const ticket = g_colsum_tickets + bank * kMaxStrips + blockIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const long long col = (static_cast<long long>(blockIdx.x) * 32 + lane) * 4;
-    float4 s = fold_warps(red, acc);
+    float4 s = fold_warps<false>(red, acc);
     const int slabs = static_cast<int>(gridDim.y);
     if (slabs > 1) {
         if (warp == 0) {
@@ -79,7 +80,7 @@ __device__ __forceinline__ void finish_colsum(const float4 &acc, float4 (*red)[3
                 if (col + 3 < n) t.w += __ldcg(p + 3);
             }
         }
-        s = fold_warps(red, t);
+        s = fold_warps<true>(red, t);
         if (threadIdx.x == 0) *ticket = 0u;
     }
     if (warp == 0 && col < n) {
