@@ -83,12 +83,13 @@ constexpr int64_t kRowsAligned = 15, kRowsUnaligned = 16;
 // Limits of the one-launch f32 kernel (tiny.cu): it needs about 1.9 us and 1 us per 64 contraction elements, up to M * N * K =
 // 8 M (192^3: forward 5.0 us against 7.7, backward 5.8 against 8.9; 256^3 is level; K = 512 loses), and up to so many 32 x 32
 // tiles of output -- three a block slot and more queue up and store element by element (2048 x 1 x 4096, 8192 tiles: 62 us
-// against 13).  An eager call gains from one launch in place of two to four; under capture only device time counts, and one
-// product with aligned output rows is the tensor path's from fewer tiles on (104 x 1 x 4776, 600 tiles: 7.0 us against 5.5; rows
-// of 19247: 6.7 against 12.1), two gradients' with contractions from 256 on (17 x 992 x 256: 8.7 against 7.3).
-constexpr int64_t kTinyContraction = 320, kTinyContractionFewRows = 128, kTinyContractionCaptured = 240;
+// against 13).  An eager call gains from one launch in place of two to four (491 x 8 x 1746, 880 tiles: 8.5 against 11.5), the
+// two gradients of a backward call more (13 x 5616 x 99, 880 tiles: 11.0 against 15.6; 48 x 18120 x 3, 1701: 16.7 / 17.1).  Under
+// capture only device time counts, and one product with aligned output rows and more than the 64 rows that are computed exchanged
+// is the tensor path's from fewer tiles on (104 x 1 x 4776, 600 tiles: 7.0 against 5.5; but 20 x 3 x 16904 5.7 / 7.2).
+constexpr int64_t kTinyContraction = 320, kTinyContractionFewRows = 128;
 constexpr int kTinyWork = 1 << 23;
-constexpr int64_t kTinyTiles = 800, kTinyTilesCaptured = 400;
+constexpr int64_t kTinyTiles = 900, kTinyTilesBoth = 1200, kTinyTilesCaptured = 400;
 // Up to 8 rows the streaming kernels are the competition.  For one product they win but where the tiles are few and five rows
 // or more, or a short contraction, share them (8 x 8 x 4512 forward 3.3 us against 4.8, 8 x 90 x 1656 4.1 / 6.3; but 8 x 128 x
 // 8192 6.1 / 4.8, 1 x 128 x 4096 5.6 / 3.1, input gradient 8 x 496 x 8 2.7 / 2.6).  A backward call for both gradients they make in two launches on two
@@ -474,9 +475,9 @@ bool tiny_wanted(const Call &c, TinyCall call, const Shapes &s, const mni_b200_v
     const bool da = call == kTinyGradA || call == kTinyGradBoth, db = call == kTinyGradB || call == kTinyGradBoth;
     const int64_t tiles = dc ? (da ? m * k : 0) + (db ? k * n : 0) : m * n;
     if (s.M > 8) {
-        if (c.capturing && call == kTinyGradBoth) return tiles <= kTinyTiles && std::max(s.M, s.N) <= kTinyContractionCaptured;
-        const bool aligned_rows = (call == kTinyGradA ? s.K : s.N) % 4 == 0;
-        return tiles <= (c.capturing && call != kTinyGradBoth && aligned_rows ? kTinyTilesCaptured : kTinyTiles);
+        if (call == kTinyGradBoth) return tiles <= kTinyTilesBoth;
+        const bool aligned_rows = (call == kTinyGradA ? s.K : s.N) % 4 == 0, exchanged = (call == kTinyGradB ? s.K : s.M) <= 64;
+        return tiles <= (c.capturing && aligned_rows && !exchanged ? kTinyTilesCaptured : kTinyTiles);
     }
     if (tiles <= kTinyTilesFewest && (dc ? std::max(s.M, s.N) : s.K) <= 32) return true;
     const bool rows_unit = dc ? dc->stride[dc->ndim - 1] == 1 || s.N == 1 : a.stride[a.ndim - 1] == 1 || s.K == 1;
