@@ -79,6 +79,10 @@ constexpr int64_t kSkinnyDxRows = 5, kSkinnyDwRows = 8;
 // rows, the narrowest tile of the tensor path, that path wastes nothing on an aligned weight; one whose rows are not
 // 16-byte aligned it would have to gather first.
 constexpr int64_t kRowsAligned = 15, kRowsUnaligned = 16;
+// ... of an aligned weight with short contractions only, or up to 16 M elements with at least as many outputs: larger ones the
+// tensor path streams better (9 rows, weight not in L2, us here / there: 1024 x 4096 forward 7.9 / 10.4, 4096 x 4096 19.1 / 19.2,
+// 2792 x 3880 14.6 / 15.7 and its dx 19.9 / 15.6, 8192 x 8192 66 / 57, 4096 x 12000 75 / 55, 6000 x 3000 27 / 21).
+constexpr int64_t kRowsShort = 1024, kRowsElements = 1 << 24;
 
 // Limits of the one-launch f32 kernel (tiny.cu): it needs about 1.9 us and 1 us per 64 contraction elements, up to M * N * K =
 // 8 M (192^3: forward 5.0 us against 7.7, backward 5.8 against 8.9; 256^3 is level; K = 512 loses), and up to so many 32 x 32
@@ -448,14 +452,20 @@ int analyse(const mni_b200_view *a, const mni_b200_view *b, Shapes &s) {
     return MNI_B200_OK;
 }
 
+bool aligned_weight(const Shapes &s, const mni_b200_view &w) {
+    const int64_t s0 = w.stride[w.ndim - 2], s1 = w.stride[w.ndim - 1];
+    return (reinterpret_cast<uintptr_t>(w.ptr) & 15) == 0 && (s1 == 1 ? s0 : s1) % 4 == 0 && (s1 == 1 ? s.N : s.K) % 4 == 0;
+}
 // Few rows against one weight, not forced onto another path.
 bool rows_wanted(uint32_t flags, const Shapes &s, const mni_b200_view &w) {
-    const int64_t s0 = w.stride[w.ndim - 2], s1 = w.stride[w.ndim - 1];
-    const bool aligned = (reinterpret_cast<uintptr_t>(w.ptr) & 15) == 0 && (s1 == 1 ? s0 : s1) % 4 == 0 &&
-                         (s1 == 1 ? s.N : s.K) % 4 == 0;
     return (flags & (MNI_B200_FORCE_TENSOR_PATH | MNI_B200_FORCE_SKINNY_PATH | MNI_B200_FORCE_PACK)) == 0 &&
            ((flags >> 16) & 0xffu) == 0 && s.batch == 1 && s.a_batch == 1 && s.b_batch == 1 &&
-           s.M <= (aligned ? kRowsAligned : kRowsUnaligned);
+           s.M <= (aligned_weight(s, w) ? kRowsAligned : kRowsUnaligned);
+}
+// Whether the product of `outs` outputs a row and a contraction of `total` is one the warp-level kernels take.
+bool rows_take(const Shapes &s, const mni_b200_view &w, int64_t outs, int64_t total, int sm_count) {
+    return rows_supported(s.M, outs, total, sm_count) &&
+           (!aligned_weight(s, w) || total <= kRowsShort || (outs >= total && outs * total <= kRowsElements));
 }
 
 // What the one-launch f32 kernel would compute for a call.
@@ -533,7 +543,7 @@ int fwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, float *out
         }
     }
 
-    if (rows_wanted(c.flags, s, *b) && rows_supported(s.M, s.N, s.K, c.st->sm_count) && (a->stride[a->ndim - 1] == 1 || s.K == 1)) {
+    if (rows_wanted(c.flags, s, *b) && rows_take(s, *b, s.N, s.K, c.st->sm_count) && (a->stride[a->ndim - 1] == 1 || s.K == 1)) {
         const int64_t ldx = a->stride[a->ndim - 2], sk = b->stride[b->ndim - 2], sn = b->stride[b->ndim - 1];
         if (sn == 1 || sk == 1) {                      // W as stored [K, N], or [N, K] seen through a transposing view
             c.note("streaming (few rows) forward kernel");
@@ -714,15 +724,14 @@ int bwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const mni_
                            dc->stride[gn - 1] == 1 && b->stride[b->ndim - 1] == 1 && s.K > 1 &&
                            skinny_dx_supported(dc->ptr, dc->stride[gn - 2], b->ptr, b->stride[b->ndim - 2], s.M, s.N);
     const bool rows_ok = rows_wanted(c.flags, s, *b) && g_batch == 1 && (dc->stride[gn - 1] == 1 || s.N == 1);
+    // ... and those of the remaining few-row products that stream the weight through the warp-level kernels
+    const int64_t b_sk = b->stride[b->ndim - 2], b_sn = b->stride[b->ndim - 1];
+    const bool rows_dx = da_wanted && !skinny_dx && rows_ok && rows_take(s, *b, s.K, s.N, c.st->sm_count) && (b_sn == 1 || b_sk == 1);
     const bool skinny_dw = db_wanted &&
                            ((c.flags & MNI_B200_FORCE_SKINNY_PATH) != 0 || rows_ok ||
                             ((c.flags & MNI_B200_FORCE_TENSOR_PATH) == 0 && s.M <= kSkinnyDwRows)) &&
                            s.batch == 1 && g_batch == 1 && s.M <= 16 && (a->stride[a->ndim - 1] == 1 || s.K == 1) &&
                            (dc->stride[gn - 1] == 1 || s.N == 1);
-
-    // ... and those of the remaining few-row products that stream the weight through the warp-level kernels
-    const int64_t b_sk = b->stride[b->ndim - 2], b_sn = b->stride[b->ndim - 1];
-    const bool rows_dx = da_wanted && !skinny_dx && rows_ok && rows_supported(s.M, s.K, s.N, c.st->sm_count) && (b_sn == 1 || b_sk == 1);
     const bool streamed_dx = skinny_dx || rows_dx, streamed_dw = skinny_dw;
 
     // grad_a and grad_b do not depend on each other.  grad_b of a small problem goes to the library's side stream
@@ -782,7 +791,12 @@ int bwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const mni_
     }
     const int pair_env = env_int("MNI_B200_BWD_PAIR", -1);
     const bool pair = pairable && (pair_env > 0 || (pair_env < 0 && beside && !c.capturing));
-    const bool overlap = side_on && !pair && da && db && a_elems > 0 && b_elems > 0 && beside;
+    // Streamed gradients that each keep HBM busy on their own run one after the other: of one row against a very large weight
+    // (8192 x 8192 97 us against 111 side by side, 4096 x 20000 120 / 137; four rows 120 / 111), and the streaming dW of 9 to 12
+    // rows with whichever kernel computes dx (4096 x 4096 40 / 44, 5504 x 7680 87 / 92, 4096 x 20000 148 / 164; 15 rows 49 / 50).
+    const bool in_turn = skinny_dw && da_wanted && ((s.M == 1 && s.K * s.N >= (int64_t{1} << 26)) ||
+                                                    (s.M > 8 && s.M <= 12 && s.K * s.N >= (int64_t{1} << 24)));
+    const bool overlap = side_on && !pair && da && db && a_elems > 0 && b_elems > 0 && beside && !in_turn;
     const bool side_dbias = side_on && dbias && (da || db) && work > 0;
     // Two tensor-core products side by side: each persistent grid is planned for half of the SMs, so that both are
     // resident at once instead of the second queueing behind the first's CTAs (measured under graph replay: 512^3

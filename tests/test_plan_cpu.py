@@ -188,6 +188,24 @@ def test_long_contractions_over_a_ragged_wave_are_cut(plan):
     assert f(384, 4096, 64, (100,))["splits"] > 1 and f(384, 512, 64, (100,))["splits"] == 1
 
 
+def test_nine_to_fifteen_rows_against_aligned_weights(plan):
+    """The warp-level kernels take them with short contractions, or up to 16 M elements with as many outputs as the contraction
+    is long; the tensor path streams larger weights better, and then takes both gradients."""
+    for k, n, fwd, dx in ((1024, 4096, True, False), (4096, 4096, True, True), (2792, 3880, True, False), (8192, 8192, False, False),
+                          (4096, 12000, False, False), (6000, 3000, False, False), (8191, 8191, True, True)):
+        assert ("few rows" in plan((9, k), (k, n))[0]) == fwd, (k, n)
+        b = by_label(plan((9, k), (k, n), backward=1))
+        assert ("few rows" in b["grad_a"][0][2]) == dx and "streaming" in b["grad_b"][0][2], (k, n)
+
+
+def test_streamed_gradients_that_fill_the_memory_run_in_turn(plan):
+    def beside(m, k, n):
+        return any("side" in line for line in plan((m, k), (k, n), backward=1))
+    for shape, want in (((1, 4096, 4096), True), ((4, 8192, 8192), True), ((1, 8192, 8192), False), ((9, 4096, 4096), False),
+                        ((12, 4096, 12000), False), ((9, 1024, 4096), True), ((15, 4096, 4096), True)):
+        assert beside(*shape) == want, shape
+
+
 def test_small_products_are_those_of_few_tiles(plan):
     """The one-launch f32 kernel takes calls of at most 900 tiles of 32 x 32 (two gradients 1200), and of few rows only where the streaming kernels,
     which read the weight in 16-byte units, do not do better."""
