@@ -407,6 +407,7 @@ int run_gemm(Call &c, GemmProblem &p) {
     p.force_splits = static_cast<int>((c.flags >> 16) & 0xffu);
     p.flag_bank = c.flag_bank;
     p.dep_mode = c.dep_mode;
+    p.beside = c.sm_share > 1;
     if (p.M > 0x7fffffffLL || p.N > 0x7fffffffLL || p.K > 0x7fffffffLL || p.batch * p.fold > 0x7fffffffLL ||
         p.batch * ((p.M + 127) / 128) * ((p.N + 63) / 64) > 0x3fffffffLL)
         return fail(MNI_B200_ERR_TOO_LARGE, "GEMM %lld x %lld x %lld (batch %lld) exceeds the kernels' int32 indexing",
@@ -773,6 +774,8 @@ int bwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const mni_
                 return p;
             };
             const GemmProblem pa = problem(s.M, s.K, s.N, oa, na, *a, da), pb = problem(s.K, s.N, s.M, ob, nb, *b, db);
+            GemmProblem pa_half = pa, pb_half = pb;
+            pa_half.beside = pb_half.beside = true;
             const int all = c.gemm_sms();
             c.sm_share = 2;
             const int half = c.gemm_sms();
@@ -781,12 +784,12 @@ int bwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const mni_
                 // Larger products go side by side where the cost model says so by a margin: where one of them, or both, would
                 // leave SMs idle on its own or need a split of the contraction to fill them (2048 x 3072 x 768: 97.6 -> 81.4 us).
                 const double whole_a = gemm_tc_estimate_us(pa, all), whole_b = gemm_tc_estimate_us(pb, all);
-                const double half_a = gemm_tc_estimate_us(pa, half), half_b = gemm_tc_estimate_us(pb, half);
+                const double half_a = gemm_tc_estimate_us(pa_half, half), half_b = gemm_tc_estimate_us(pb_half, half);
                 beside = whole_a > 0 && whole_b > 0 && half_a > 0 && half_b > 0 && std::max(half_a, half_b) < 0.9 * (whole_a + whole_b);
             }
             // CTA pairs take both SMs of a unit, lone CTAs are dealt out one to a unit: launched first, these would leave
             // the pairs hardly a whole unit until they end (16 rows x 4096^2, grad_b in pairs after grad_a: 47 us against 37).
-            b_first = beside && !gemm_tc_uses_pairs(pa, half) && gemm_tc_uses_pairs(pb, half);
+            b_first = beside && !gemm_tc_uses_pairs(pa_half, half) && gemm_tc_uses_pairs(pb_half, half);
         }
     }
     const int pair_env = env_int("MNI_B200_BWD_PAIR", -1);

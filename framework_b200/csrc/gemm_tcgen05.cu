@@ -1623,8 +1623,9 @@ double finish_us(double parts, double bytes) { return 1.5 + (parts + 1.0) * byte
 // about 3000 on with 0.5 to 0.8 or 1.5 to 1.75 waves of tiles (74 pairs; us whole / balanced tail / cut): 2048 x 4096 x 1280
 // 128 / 91 / 92, 2048 x 8192 x 1280 242 / 174 / 176, 1536 x 8192 x 2048 239 / 197 / 191, 2048 x 8192 x 3584 500 / 436 / 439,
 // 2048 x 3072 x 3584 177 / 169 / 168; at K = 2048, 121 / 117 / -, it would save 4.6 %.  Not in single-pass mode, whose long units
-// lose more by giving up their running sum (2048 x 8192 x 3584 200 / 209 / 231).
-Cut cut_tail(long long tiles, long long slots, long long k, bool single_pass) {
+// lose more by giving up their running sum (2048 x 8192 x 3584 200 / 209 / 231), and not beside another product, which uses the
+// SMs that the wave leaves.  `round_only`: neither.
+Cut cut_tail(long long tiles, long long slots, long long k, bool round_only) {
     const long long full = tiles / slots, rem = tiles - full * slots;
     const double tile_bytes = 4.0 * 2 * BM * 256;
     const Cut whole{1, static_cast<double>(rem > 0 ? full + 1 : full), 0.0};
@@ -1633,7 +1634,7 @@ Cut cut_tail(long long tiles, long long slots, long long k, bool single_pass) {
     const double eff = static_cast<double>(tiles) / static_cast<double>((full + 1) * slots);
     if (full >= 1 && ways >= 2 && eff < 0.80 && k / ways >= 128)
         return Cut{ways, static_cast<double>(full) + 1.0 / static_cast<double>(ways), finish_us(static_cast<double>(ways), tile_bytes * static_cast<double>(rem))};
-    if (single_pass) return whole;
+    if (round_only) return whole;
     const double round_us = static_cast<double>(k) * kPairNs * 1e-3;
     Cut best = whole;
     for (long long w = 2; w <= 6 && k / w >= 256; ++w) {
@@ -1689,7 +1690,7 @@ Plan make_plan(const GemmProblem &p, int sm_count) {
             }
             // ... or a single, partly filled wave of 256-wide pairs cut like a last one
             if (bn == 256 && cg == 2 && !p.exchanged && tiles < slots) {
-                const Cut cut = cut_tail(tiles, slots, p.fold * ((p.K + 15) / 16) * 16, p.fast_tf32);
+                const Cut cut = cut_tail(tiles, slots, p.fold * ((p.K + 15) / 16) * 16, p.fast_tf32 || p.beside);
                 const double t = cut.rounds * k_eff * kPairNs + cut.finish_us * 1e3;
                 if (cut.ways > 1 && t < 0.97 * best) { best = t; pl.bn = bn; model_splits = 1; }
             }
@@ -1712,7 +1713,7 @@ Plan make_plan(const GemmProblem &p, int sm_count) {
             const double write = unaligned * (bn == 256 ? (cg == 2 ? 3.7 : 4.5) : (bn == 128 ? 2.2 : 1.5));
             double rounds = static_cast<double>((tiles + slots - 1) / slots);
             if (bn == 256 && cg == 2) {
-                const Cut cut = cut_tail(tiles, slots, p.fold * ((p.K + 15) / 16) * 16, p.fast_tf32);
+                const Cut cut = cut_tail(tiles, slots, p.fold * ((p.K + 15) / 16) * 16, p.fast_tf32 || p.beside);
                 if (cut.ways > 1) rounds = cut.rounds + 0.25;
             }
             const double t = rounds * std::max(loop, write);
@@ -1784,7 +1785,7 @@ Plan make_plan(const GemmProblem &p, int sm_count) {
     // Neither it nor the running sum is built for exchanged operands, whose patches leave transposed (the planner's own
     // choice there is a 64-wide tile; MNI_B200_BN=256 makes it a 256-wide pair).
     if (splits == 1 && sk_env < 0 && p.force_splits <= 0 && pl.cg == 2 && pl.bn == 256 && !p.exchanged) {
-        const Cut cut = cut_tail(tiles, slots, iters * pl.bk, p.fast_tf32);
+        const Cut cut = cut_tail(tiles, slots, iters * pl.bk, p.fast_tf32 || p.beside);
         if (cut.ways > 1) {
             pl.tail_ways = static_cast<int>(cut.ways);
             pl.tail_tiles = static_cast<int>(tiles % slots);

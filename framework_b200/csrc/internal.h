@@ -137,6 +137,7 @@ struct GemmProblem {
     bool accumulate = false;       // C += ...
     bool fast_tf32 = false;        // one TF32 pass instead of the 3-pass split
     int force_splits = 0;          // tests
+    bool beside = false;           // another product runs on the SMs that this one is not planned for
     bool exchanged = false;        // the kernel's view of a product whose operands it exchanges: it computes C^T
     // Two products of one call that do not depend on each other (grad_a and grad_b) are launched back to back on
     // one stream as a pair: the first (1) lets its dependent start only after its own wait for earlier work has

@@ -206,6 +206,13 @@ def test_streamed_gradients_that_fill_the_memory_run_in_turn(plan):
         assert beside(*shape) == want, shape
 
 
+def test_a_wave_beside_another_product_is_left_whole(plan):
+    """24 pair tiles on half of the device, the other half busy with grad_a."""
+    b = plan((19, 104, 1847), (1847, 661), b_strides=(1, 1847), backward=1)
+    assert any("side by side" in line for line in b)
+    assert tensor_plan(b, "grad_b")["tail_ways"] == 0
+
+
 def test_small_products_are_those_of_few_tiles(plan):
     """The one-launch f32 kernel takes calls of at most 900 tiles of 32 x 32 (two gradients 1200), and of few rows only where the streaming kernels,
     which read the weight in 16-byte units, do not do better."""
