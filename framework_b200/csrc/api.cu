@@ -72,7 +72,8 @@ double overlap_work_limit() {
 
 // Row counts up to which the streaming kernels beat the tensor path (measured at K = N = 4096 with a weight
 // that is not in L2: dx 19.4 vs 23.6 us at 5 rows and 31.0 vs 23.7 at 8; dW 14 vs 16.9 at 8 rows, 15.5 at 12, 20.7 at
-// 15: beyond 8 rows it goes with the rows.cu kernels, whose dx it runs in front of).  The forward's limit depends on which of its two kernels can run: skinny_fwd_row_limit.
+// 15: beyond 8 rows it goes with the calls of few rows below).  The forward's limit depends on which of its two kernels can
+// run: skinny_fwd_row_limit.
 constexpr int64_t kSkinnyDxRows = 5, kSkinnyDwRows = 8;
 
 // Rows up to which the warp-level streaming kernels (rows.cu) take a product the FFMA kernels above do not.  From 16

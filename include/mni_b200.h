@@ -288,7 +288,7 @@ MNI_B200_API int mni_b200_sm_reserve(int sms);
  * output gradient and both gradients (backward = 1; 2 = with the bias gradient too) would launch for
  * these operands and flags on a device with `sm_count` SMs -- one line of text per launch: the product
  * it belongs to, the kernel, and for the tensor-core kernel its tile width, CTA pairing, contraction
- * split, balanced tail, grid and the number of pieces a long contraction is summed in.  Operand
+ * split, cut or balanced tail, grid and the number of pieces a long contraction is summed in.  Operand
  * pointers are only inspected for alignment.  Pure host arithmetic: touches no device, so the planner
  * can be checked where there is none.  (No counterpart in the reference.)
  */

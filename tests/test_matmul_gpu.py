@@ -739,8 +739,10 @@ def test_balanced_tail_with_a_long_contraction(F, oracle, monkeypatch):
 
 def test_shard_of_the_broadcast_weight_problem_takes_the_default_tail(F, oracle):
     """One rank's share of an 8-rank run of the broadcast-weight configuration ([8,1024,768].[768,3072]): its input
-    gradient has 96 pair-tiles for 74 pairs, which the default policy runs with the balanced tail.  First and last
-    128 rows of dA against the CPU backend."""
+    gradient has 96 pair-tiles for 74 pairs, a last wave that the default policy cuts into several units a tile.  First and
+    last 128 rows of dA against the CPU backend."""
+    assert any(line.startswith("grad_a") and "tail_ways=3" in line
+               for line in F.plan_describe((8, 1024, 768), (768, 3072), backward=1))
     rng = np.random.default_rng(94)
     a = rng.standard_normal((8, 1024, 768), dtype=np.float32)
     w = (0.02 * rng.standard_normal((768, 3072))).astype(np.float32)

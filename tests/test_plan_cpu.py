@@ -1,7 +1,7 @@
 """CPU: the launch planner, pinned at the benchmark configurations.
 
 Which kernel a product takes -- tile width, CTA pairing, the A operand from tensor memory, the split of the
-contraction, the balanced tail, how many SMs two side-by-side products get, streaming kernels for few rows,
+contraction, the cut or balanced tail, how many SMs two side-by-side products get, streaming kernels for few rows,
 pieces of a long contraction -- is host arithmetic over shapes, strides and the SM count, so it is checked here
 without a device through `mni_b200_plan_describe`.  The pins are the plans the measured numbers were taken
 with: a change of the planner that moves one of them is a performance change and must be re-measured.  (The
@@ -55,7 +55,7 @@ def test_default_benchmark_shape_whole_and_as_an_eighth(plan):
         assert dw["pieces"] == batches // 2                  # (batches * 1024 / 2) / 1024
         assert not any("side by side" in line for line in bwd)        # large products run one after the other
         # whole: 768 pair-tiles = 10.4 rounds, the ragged wave is left alone; an eighth: 96 tiles on 74 pairs
-        # would be two rounds at 0.65 -> balanced tail
+        # would be two rounds at 0.65 -> the last wave's 22 tiles are cut
         assert da["tail"] == (1 if batches == 8 else 0) and da["grid"] == 148
 
 
