@@ -37,6 +37,8 @@ struct DeviceState {
     int cc_major = 0;
     uint8_t *ws = nullptr;        // library-owned scratch
     size_t ws_bytes = 0;
+    bool ws_recorded = false;     // some graph holds its address
+    std::vector<uint8_t *> retired;   // scratch outgrown since, kept for the graphs that hold its address (mni_b200_release frees it)
     uint8_t *user_ws = nullptr;   // caller-provided scratch (takes precedence)
     size_t user_bytes = 0;
     unsigned int *err_word = nullptr;
@@ -174,13 +176,18 @@ int scratch_base(DeviceState &st, size_t bytes, cudaStream_t stream, uint8_t **b
     if (bytes > st.ws_bytes) {
         const size_t want = bytes + bytes / 4 + (1u << 20);
         // Growing frees the old buffer, which a capturing stream must not do (it would end the capture in
-        // an error) and which would leave the nodes already recorded with a dangling address.
+        // an error).
         if (st.ws && stream_is_capturing(stream))
             return fail(MNI_B200_ERR_WORKSPACE,
                         "scratch would have to grow from %zu to %zu bytes while the stream is capturing: run the call "
                         "once before the capture, or hand the library a buffer (mni_b200_workspace_set)",
                         st.ws_bytes, bytes);
-        if (st.ws) {
+        if (st.ws && st.ws_recorded) {
+            st.retired.push_back(st.ws);
+            st.ws = nullptr;
+            st.ws_bytes = 0;
+            st.ws_recorded = false;
+        } else if (st.ws) {
             // cudaFree waits for work that may still read the old buffer.
             cudaError_t e = cudaFree(st.ws);
             st.ws = nullptr;
@@ -196,6 +203,7 @@ int scratch_base(DeviceState &st, size_t bytes, cudaStream_t stream, uint8_t **b
         st.ws = static_cast<uint8_t *>(p);
         st.ws_bytes = want;
     }
+    if (!st.ws_recorded && stream_is_capturing(stream)) st.ws_recorded = true;
     *base = st.ws;
     return MNI_B200_OK;
 }
@@ -347,6 +355,8 @@ struct Call {
     bool capturing = false;    // the stream records into a graph
     int flag_bank = 0;         // 1 while launches go to the library's side stream / for the second product of a pair
     int dep_mode = 0;          // GemmProblem::dep_mode of the tensor-path launches issued now
+    bool used_half = false;    // some product of the call is computed from 16-bit halves
+    bool no_half = false;      // there is no scratch for operands as 16-bit halves
     GemmFinish *defer = nullptr;       // where the next product leaves its split-K finish instead of launching it
     int sm_share = 1;          // 2 while grad_a and grad_b run side by side: each is planned for half of the SMs
     std::string *plan_log = nullptr;   // mni_b200_plan_describe: one line per launch the call would make
@@ -356,7 +366,8 @@ struct Call {
     }
     // SMs the persistent tensor-core grids are planned for: all of them minus the caller's reservation, divided
     // between the products that run at the same time (kept even, CTA pairs take two)
-    int gemm_sms() const { return std::max(8, ((st->sm_count - st->sm_reserve) / sm_share) & ~1); }
+    int gemm_sms(int share) const { return std::max(8, ((st->sm_count - st->sm_reserve) / share) & ~1); }
+    int gemm_sms() const { return gemm_sms(sm_share); }
     bool dry() const { return arena.dry; }
     float *at(size_t off) const { return reinterpret_cast<float *>(base + off); }
 };
@@ -419,6 +430,122 @@ int run_gemm(Call &c, GemmProblem &p) {
     if (c.plan_log) c.note(gemm_tc_describe(p, c.gemm_sms()));
     if (c.dry()) return MNI_B200_OK;
     return launch_gemm_tc(p, pbytes ? c.at(poff) : nullptr, c.st->err_word, c.gemm_sms(), c.stream, c.defer);
+}
+
+// ------------------------------------------------------------------ large products from 16-bit halves
+// A view as matrices with a unit stride along their columns (swapped: the view's last two dims are exchanged for that).
+bool view_to_half(const mni_b200_view &v, HalfView &h, bool *swapped) {
+    const int nd = v.ndim;
+    *swapped = v.stride[nd - 1] != 1;
+    if (*swapped && v.stride[nd - 2] != 1) return false;
+    const int r = *swapped ? nd - 1 : nd - 2, k = *swapped ? nd - 2 : nd - 1;
+    h.src = v.ptr;
+    h.rows = v.shape[r];
+    h.cols = v.shape[k];
+    h.ld = v.stride[r];
+    int nb = 0;
+    int64_t bs[MNI_B200_MAX_DIMS], bt[MNI_B200_MAX_DIMS];
+    h.batch = 1;
+    for (int d = 0; d < nd - 2; ++d) {
+        h.batch *= v.shape[d];
+        if (v.shape[d] == 1) continue;
+        if (v.stride[d] == 0) return false;
+        if (nb > 0 && bt[nb - 1] == v.stride[d] * v.shape[d]) {
+            bs[nb - 1] *= v.shape[d];
+            bt[nb - 1] = v.stride[d];
+        } else {
+            bs[nb] = v.shape[d];
+            bt[nb] = v.stride[d];
+            ++nb;
+        }
+    }
+    if (nb > 3) return false;
+    for (int i = 0; i < 3; ++i) { h.bshape[i] = 1; h.bstride[i] = 0; }
+    for (int i = 0; i < nb; ++i) { h.bshape[3 - nb + i] = bs[i]; h.bstride[3 - nb + i] = bt[i]; }
+    h.pitch = round_up(h.cols, 64);
+    h.matrix = h.rows * h.pitch;
+    h.plane = h.batch * h.matrix;
+    return h.ld >= 0 && h.batch * h.rows < 0x7fffffffLL && h.batch * ((h.rows + 15) / 16) * ((h.pitch + 511) / 512) < 0x1fffffffLL;
+}
+
+// The 16-bit planes of a call's operands.
+struct Halves {
+    HalfView view[kMaxHalves];
+    bool swapped[kMaxHalves];
+    int count = 0, blocks = 0, planes = 3;
+    unsigned int *status = nullptr;
+    // operand i with its last dim contracted, or (transposed) the one before
+    HalfOperand operand(int i, bool transposed) const {
+        const HalfView &v = view[i];
+        HalfOperand o;
+        o.ptr = v.dst;
+        o.k_major = swapped[i] == transposed;
+        o.rows = o.k_major ? v.rows : v.cols;
+        o.kdim = o.k_major ? v.cols : v.rows;
+        o.pitch = v.pitch; o.matrix = v.matrix; o.plane = v.plane;
+        o.batch = v.batch;
+        o.planes = planes;
+        o.exp = v.exp;
+        return o;
+    }
+};
+
+// Whether a call may be computed from 16-bit planes, and is large enough for it to be worth finding out whether that pays.
+constexpr double kHalfWork = 4.0e9;                // M * N * K of its products
+bool half_possible(const Call &c, double work) {
+    const uint32_t forced = MNI_B200_FORCE_TENSOR_PATH | MNI_B200_FORCE_SKINNY_PATH | MNI_B200_FORCE_PACK;
+    return !c.no_half && (c.flags & forced) == 0 && ((c.flags >> 16) & 0xffu) == 0 &&
+           (work >= kHalfWork || env_int("MNI_B200_HALF", -1) > 0);
+}
+// Whether it pays: `f32_us` the estimate for the products from f32 operands, `half_us` from 16-bit planes, which the pass over the
+// operands' `elements` comes on top of (8 bytes an element, 6 in single-pass mode, at 5.2 TB/s, and 7 us for its two launches).
+// Measured with and without, us, sustained: forward 2048 x 768 x 3072 55 / 62, 2048^3 65 / 62, 8192 x 768 x 3072 143 / 125,
+// 4096 x 1024 x 4096 137 / 114, 4096^3 480 / 338, 1024 x 8192 x 1024 70 / 90, 8192 x 8192 x 512 291 / 308; single pass 3072^3
+// 80 / 82, 4096^3 218 / 178.  MNI_B200_HALF=0 / 1: never / wherever it can be done.
+bool half_pays(const Call &c, double f32_us, double half_us, double elements) {
+    const int env = env_int("MNI_B200_HALF", -1);
+    if (env >= 0) return env > 0;
+    const double bytes = (c.flags & MNI_B200_PRECISION_TF32) != 0 ? 6.0 : 8.0;
+    return half_us + 7.0 + bytes * elements / 5.2e6 < 0.95 * f32_us;
+}
+// Gathering an operand that TMA cannot describe, in microseconds.
+double gather_us(const mni_b200_view &v) {
+    Operand probe;
+    return view_to_operand(v, false, probe) ? 0.0 : 3.0 + 8.0 * static_cast<double>(prod(v.shape, v.ndim)) / 4.0e6;
+}
+
+// sums_out: also the column sums of the first view.
+int make_halves(Call &c, std::initializer_list<const mni_b200_view *> views, Halves &h, float *sums_out = nullptr, bool accumulate = false) {
+    for (const mni_b200_view *v : views) {
+        if (!view_to_half(*v, h.view[h.count], &h.swapped[h.count])) return fail(MNI_B200_ERR_ARG, "internal: operand has no halves");
+        ++h.count;
+    }
+    h.planes = (c.flags & MNI_B200_PRECISION_TF32) != 0 ? 2 : 3;
+    h.blocks = half_blocks(h.view, h.count, c.st->sm_count);
+    const size_t words = static_cast<size_t>(h.blocks) + kMaxHalves, head = c.arena.reserve(4 * words);
+    size_t at[kMaxHalves];
+    for (int i = 0; i < h.count; ++i) at[i] = c.arena.reserve(static_cast<size_t>(h.view[i].plane) * 2 * h.planes);
+    const size_t sums_at = sums_out ? c.arena.reserve(half_columns_bytes(h.view[0], h.blocks)) : 0;
+    c.used_half = true;
+    c.note("operands into 16-bit planes");
+    if (c.dry()) return MNI_B200_OK;
+    h.status = reinterpret_cast<unsigned int *>(c.at(head));
+    for (int i = 0; i < h.count; ++i) {
+        h.view[i].dst = c.at(at[i]);
+        h.view[i].exp = reinterpret_cast<int *>(h.status + h.blocks + i);
+    }
+    HalfColumns sums;
+    if (sums_out) sums = HalfColumns{c.at(sums_at), sums_out, accumulate ? 1 : 0};
+    return launch_split_half(h.view, h.count, h.planes, h.status, h.blocks, sums, c.stream);
+}
+
+// The product `p` from operands `a` and `b`; p.C and the rest as for the general path.
+int run_halves(Call &c, GemmProblem p, const Halves &h, const HalfOperand &a, const HalfOperand &b) {
+    p.ha = &a;
+    p.hb = &b;
+    p.half_status = h.status;
+    p.half_statuses = h.blocks;
+    return run_gemm(c, p);
 }
 
 int zero_or_bias_fill(Call &c, float *out, int64_t rows, int64_t n, const float *bias, bool accumulate) {
@@ -509,6 +636,40 @@ bool tiny_wanted(const Call &c, TinyCall call, const Shapes &s, const mni_b200_v
 }
 
 // ------------------------------------------------------------------ forward
+// a . b on the tensor path; `p` without its operands.
+int forward_product(Call &c, const Shapes &s, const mni_b200_view *a, const mni_b200_view *b, GemmProblem &p) {
+    HalfView probe;
+    bool swapped;
+    bool half = s.M > 128 && s.N > 128 && s.K >= 64 && half_possible(c, static_cast<double>(s.batch) * s.M * s.N * s.K) &&
+                view_to_half(*a, probe, &swapped) && view_to_half(*b, probe, &swapped);
+    if (half) {
+        p.fast_tf32 = (c.flags & MNI_B200_PRECISION_TF32) != 0;
+        half = half_pays(c, gemm_estimate_us(p, false, c.gemm_sms()) + gather_us(*a) + gather_us(*b), gemm_estimate_us(p, true, c.gemm_sms()),
+                         static_cast<double>(s.a_batch) * s.M * s.K + static_cast<double>(s.b_batch) * s.K * s.N);
+    }
+    const mni_b200_view *const a_given = a, *const b_given = b;
+    int rc = MNI_B200_OK;
+    if (!half || c.plan_log) {
+        mni_b200_view packed[kMaxGathers];
+        rc = pack_undescribable(c, {&a, &b}, packed);
+        if (rc) return rc;
+        rc = make_operand(*a, false, p.A);
+        if (rc) return rc;
+        rc = make_operand(*b, true, p.B);
+        if (rc) return rc;
+        p.A.batch = s.a_batch;
+        p.B.batch = s.b_batch;
+        rc = run_gemm(c, p);
+        if (!half || rc) return rc;
+        c.note("with scratch for 16-bit operands, instead of these:");
+    }
+    Halves h;
+    rc = make_halves(c, {a_given, b_given}, h);
+    if (rc) return rc;
+    const HalfOperand x = h.operand(0, false), y = h.operand(1, true);
+    return run_halves(c, p, h, x, y);
+}
+
 int fwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, float *out, const float *bias) {
     Shapes s;
     int rc = analyse(a, b, s);
@@ -557,15 +718,6 @@ int fwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, float *out
     }
 
     GemmProblem p;
-    mni_b200_view packed[kMaxGathers];
-    rc = pack_undescribable(c, {&a, &b}, packed);
-    if (rc) return rc;
-    rc = make_operand(*a, false, p.A);
-    if (rc) return rc;
-    rc = make_operand(*b, true, p.B);
-    if (rc) return rc;
-    p.A.batch = s.a_batch;
-    p.B.batch = s.b_batch;
     p.M = s.M; p.N = s.N; p.K = s.K;
     p.batch = s.batch;
     p.fold = 1;
@@ -574,7 +726,7 @@ int fwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, float *out
     p.c_bstride = s.M * s.N;
     p.bias = bias;
     p.accumulate = accumulate;
-    return run_gemm(c, p);
+    return forward_product(c, s, a, b, p);
 }
 
 // Forward with the bias + GELU epilogue: pre = a . b (optional output), out = gelu(pre + bias).
@@ -599,15 +751,6 @@ int fwd_gelu_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const
                         ((c.flags & MNI_B200_FORCE_TENSOR_PATH) == 0 && s.M <= skinny_fwd_row_limit(s.N));
     if (s.K > 0 && !skinny) {
         GemmProblem p;
-        mni_b200_view packed[kMaxGathers];
-        rc = pack_undescribable(c, {&a, &b}, packed);
-        if (rc) return rc;
-        rc = make_operand(*a, false, p.A);
-        if (rc) return rc;
-        rc = make_operand(*b, true, p.B);
-        if (rc) return rc;
-        p.A.batch = s.a_batch;
-        p.B.batch = s.b_batch;
         p.M = s.M; p.N = s.N; p.K = s.K;
         p.batch = s.batch;
         p.C = pre; p.D = out;
@@ -616,7 +759,7 @@ int fwd_gelu_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const
         p.fast_tf32 = (c.flags & MNI_B200_PRECISION_TF32) != 0;
         p.force_splits = static_cast<int>((c.flags >> 16) & 0xffu);
         if (gemm_tc_can_fuse_activation(p, c.gemm_sms())) {
-            rc = run_gemm(c, p);
+            rc = forward_product(c, s, a, b, p);
             c.flags = saved_flags;
             return rc;
         }
@@ -647,8 +790,10 @@ bool single_product(const int64_t *ob, int onb, const mni_b200_view &target, boo
 
 // One gradient: G[ob.., R, Cn] = X . Y (a GEMM over `kdim`) reduced to `target`'s shape.
 //   X supplies the rows, Y the columns; both already as Operands with flat batch counts.
+//   h != null: from these halves instead.
 int grad_gemm(Call &c, Operand X, Operand Y, int64_t R, int64_t Cn, int64_t kdim, const int64_t *ob, int onb,
-              const mni_b200_view &target, float *out, bool accumulate) {
+              const mni_b200_view &target, float *out, bool accumulate, const Halves *h = nullptr, const HalfOperand *hx = nullptr,
+              const HalfOperand *hy = nullptr) {
     const int64_t obatch = prod(ob, onb);
     const int64_t tbatch = prod(target.shape, target.ndim - 2);
     bool same = false;
@@ -660,13 +805,13 @@ int grad_gemm(Call &c, Operand X, Operand Y, int64_t R, int64_t Cn, int64_t kdim
     if (same || obatch == 1) {
         p.batch = obatch; p.fold = 1;
         p.C = out; p.ldc = Cn; p.c_bstride = R * Cn; p.accumulate = accumulate;
-        return run_gemm(c, p);
+        return h ? run_halves(c, p, *h, *hx, *hy) : run_gemm(c, p);
     }
     if (tbatch == 1) {
         // The operand was broadcast over every batch: sum the batches inside the contraction.
         p.batch = 1; p.fold = obatch;
         p.C = out; p.ldc = Cn; p.c_bstride = R * Cn; p.accumulate = accumulate;
-        return run_gemm(c, p);
+        return h ? run_halves(c, p, *h, *hx, *hy) : run_gemm(c, p);
     }
     // Partial broadcast: full batched product into scratch, then the device-side unbroadcast.
     const size_t bytes = static_cast<size_t>(obatch * R * Cn) * sizeof(float);
@@ -681,6 +826,39 @@ int grad_gemm(Call &c, Operand X, Operand Y, int64_t R, int64_t Cn, int64_t kdim
     for (int i = 0; i < onb; ++i) gshape[i] = ob[i];
     gshape[onb] = R; gshape[onb + 1] = Cn;
     return launch_unbroadcast(c.at(off), gshape, onb + 2, target.shape, target.ndim, out, accumulate, c.stream);
+}
+
+// Whether the gradients on the tensor path are computed from 16-bit planes: one product each, of operands that have them.
+bool bwd_half_wanted(const Call &c, const Shapes &s, const mni_b200_view &a, const mni_b200_view &b, const mni_b200_view &dc, bool da,
+                     bool db, int64_t g_batch, double work) {
+    if ((!da && !db) || s.M < 64 || s.N < 64 || s.K <= 128 || (da && s.M <= 128) || (db && s.N <= 128) || !half_possible(c, work)) return false;
+    HalfView probe;
+    bool swapped;
+    if (!view_to_half(dc, probe, &swapped)) return false;
+    double elements = static_cast<double>(g_batch) * s.M * s.N, f32_us = 0, half_us = 0, beside_us = 0, gathers_us = gather_us(dc);
+    const int all = c.gemm_sms(1), halved = c.gemm_sms(2);
+    auto product = [&](const mni_b200_view &other, const mni_b200_view &target, int64_t rows, int64_t cols, int64_t k) {
+        int64_t ob[MNI_B200_MAX_DIMS];
+        bool same;
+        const int nb = broadcast_shape(other.shape, other.ndim - 2, dc.shape, dc.ndim - 2, ob);
+        if (nb < 0 || !single_product(ob, nb, target, &same) || !view_to_half(other, probe, &swapped)) return false;
+        const int64_t count = prod(ob, nb);
+        GemmProblem p;
+        p.M = rows; p.N = cols; p.K = k;
+        p.batch = same ? count : 1;
+        p.fold = same ? 1 : count;
+        p.ldc = cols; p.c_bstride = rows * cols;
+        p.fast_tf32 = (c.flags & MNI_B200_PRECISION_TF32) != 0;
+        f32_us += gemm_estimate_us(p, false, all);
+        gathers_us += gather_us(other);
+        half_us += gemm_estimate_us(p, true, all);
+        beside_us = std::max(beside_us, gemm_estimate_us(p, false, halved));
+        elements += static_cast<double>(prod(other.shape, other.ndim));
+        return true;
+    };
+    if (da && !product(b, a, s.M, s.K, s.N)) return false;
+    if (db && !product(a, b, s.K, s.N, s.M)) return false;
+    return half_pays(c, gathers_us + (da && db ? std::min(f32_us, beside_us) : f32_us), half_us, elements);
 }
 
 int bwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const mni_b200_view *dc, float *da,
@@ -812,13 +990,23 @@ int bwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const mni_
     mni_b200_view packed[kMaxGathers];
     const bool da_tensor = da_wanted && !streamed_dx, db_tensor = db_wanted && !streamed_dw;
     const mni_b200_view *const dc_given = dc, *const a_given = a, *const b_given = b;
-    c.label = "operands: ";
-    if (da_tensor && db_tensor) rc = pack_undescribable(c, {&dc, &b, &a}, packed);
-    else if (da_tensor) rc = pack_undescribable(c, {&dc, &b}, packed);
-    else if (db_tensor) rc = pack_undescribable(c, {&dc, &a}, packed);
-    c.label = "";
+    auto pack = [&]() -> int {
+        c.label = "operands: ";
+        int r = MNI_B200_OK;
+        if (da_tensor && db_tensor) r = pack_undescribable(c, {&dc, &b, &a}, packed);
+        else if (da_tensor) r = pack_undescribable(c, {&dc, &b}, packed);
+        else if (db_tensor) r = pack_undescribable(c, {&dc, &a}, packed);
+        c.label = "";
+        return r;
+    };
+    // From 16-bit operands, one product after the other on all SMs, instead of everything above and below but the column sums.
+    const bool half = bwd_half_wanted(c, s, *a, *b, *dc, da_tensor, db_tensor, g_batch, work), halves_now = half && !c.plan_log;
+    if (halves_now) c.sm_share = 1;
+    else rc = pack();
     if (rc) return rc;
-    const bool fork = !c.dry() && (overlap || side_dbias);
+    // ... whose pass over dc can make them too
+    const bool halves_dbias = halves_now && dbias && dc->stride[gn - 1] == 1;
+    const bool fork = !c.dry() && ((overlap && !halves_now) || (side_dbias && !halves_dbias));
     if (fork) {
         MNI_CUDA(cudaEventRecord(c.st->ev_fork, main_stream));
         MNI_CUDA(cudaStreamWaitEvent(c.st->side, c.st->ev_fork, 0));
@@ -839,7 +1027,7 @@ int bwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const mni_
 
     if (share_sms) c.note("grad_a and grad_b side by side, each planned for half of the SMs");
     else if (overlap) c.note("grad_b on the side stream beside grad_a");
-    if (dbias) {
+    if (dbias && !halves_dbias) {
         // Column sums over every row of dc (ops/elementwise.rs:224-229 via utils::unbroadcast).
         c.label = "grad_bias: ";
         if (side_dbias && !c.dry()) c.stream = c.st->side;
@@ -875,6 +1063,31 @@ int bwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const mni_
     }
 
     c.stream = main_stream;
+
+    auto halves = [&]() -> int {
+        Halves h;
+        c.label = "gradients: ";
+        if (c.plan_log) c.note("with scratch for 16-bit operands, instead of these:");
+        float *const sums = halves_dbias ? dbias : nullptr;
+        int r = da_tensor && db_tensor ? make_halves(c, {dc_given, b_given, a_given}, h, sums, acc_dbias)
+                : da_tensor            ? make_halves(c, {dc_given, b_given}, h, sums, acc_dbias)
+                                       : make_halves(c, {dc_given, a_given}, h, sums, acc_dbias);
+        int64_t ob[MNI_B200_MAX_DIMS];
+        if (r == MNI_B200_OK && da_tensor) {
+            c.label = "grad_a: ";
+            const int onb = broadcast_shape(dc_given->shape, gn - 2, b_given->shape, b_given->ndim - 2, ob);
+            const HalfOperand x = h.operand(0, false), y = h.operand(1, false);
+            r = grad_gemm(c, Operand{}, Operand{}, s.M, s.K, s.N, ob, onb, *a_given, da, acc_da, &h, &x, &y);
+        }
+        if (r == MNI_B200_OK && db_tensor) {
+            c.label = "grad_b: ";
+            const int onb = broadcast_shape(a_given->shape, a_given->ndim - 2, dc_given->shape, gn - 2, ob);
+            const HalfOperand x = h.operand(da_tensor ? 2 : 1, true), y = h.operand(0, true);
+            r = grad_gemm(c, Operand{}, Operand{}, s.K, s.N, s.M, ob, onb, *b_given, db, acc_db, &h, &x, &y);
+        }
+        return r;
+    };
+    if (halves_now) return halves();
 
     GemmFinish finish[2];              // of a pair: launched after both products
     // What the first (0) or second (1) product issued is launched with: an independent pair on one stream, or the second
@@ -963,6 +1176,10 @@ int bwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const mni_
     const bool both = finish[0] && finish[1];
     if (rc == MNI_B200_OK && finish[0]) rc = finish[0](both ? 1 : 0, c.stream);
     if (rc == MNI_B200_OK && finish[1]) rc = finish[1](both ? 2 : 0, c.stream);
+    if (rc == MNI_B200_OK && half) {
+        c.sm_share = 1;
+        rc = halves();
+    }
     return rc;
 }
 
@@ -975,24 +1192,30 @@ int with_scratch(uint32_t flags, void *stream, Body body) {
     if (rc) return rc;
     std::lock_guard<std::mutex> lock(st->mu);
     const bool capturing = stream_is_capturing(static_cast<cudaStream_t>(stream));
-    Call dry;
-    dry.capturing = capturing;
-    dry.st = st; dry.arena.st = st; dry.arena.dry = true; dry.stream = static_cast<cudaStream_t>(stream); dry.flags = flags;
-    rc = body(dry);
-    if (rc) return rc;
     Call real;
     real.capturing = capturing;
     real.st = st; real.arena.st = st; real.arena.dry = false; real.stream = static_cast<cudaStream_t>(stream); real.flags = flags;
-    if (dry.arena.used > 0) {
-        rc = scratch_base(*st, dry.arena.used, real.stream, &real.base);
+    size_t sized = 0;
+    while (true) {
+        Call dry;
+        dry.capturing = capturing;
+        dry.no_half = real.no_half;
+        dry.st = st; dry.arena.st = st; dry.arena.dry = true; dry.stream = static_cast<cudaStream_t>(stream); dry.flags = flags;
+        rc = body(dry);
         if (rc) return rc;
+        sized = dry.arena.used;
+        if (sized == 0) break;
+        rc = scratch_base(*st, sized, real.stream, &real.base);
+        if (rc == MNI_B200_OK) break;
+        // Scratch for the operands' halves cannot be had: the call goes without them, as it needs little or none then.
+        if (!dry.used_half || real.no_half) return rc;
+        real.no_half = true;
     }
     rc = body(real);
     // Both passes must have planned the same launches: a real pass that asked for more scratch than was sized
     // would have written past it.
-    if (rc == MNI_B200_OK && real.arena.used > dry.arena.used)
-        return fail(MNI_B200_ERR_WORKSPACE, "internal: the call used %zu bytes of scratch, %zu were sized", real.arena.used,
-                    dry.arena.used);
+    if (rc == MNI_B200_OK && real.arena.used > sized)
+        return fail(MNI_B200_ERR_WORKSPACE, "internal: the call used %zu bytes of scratch, %zu were sized", real.arena.used, sized);
     return rc;
 }
 
@@ -1418,11 +1641,16 @@ int mni_b200_release(void) {
     int rc = device_state(&st);
     if (rc) return rc;
     std::lock_guard<std::mutex> lock(st->mu);
+    if (st->ws || !st->retired.empty()) MNI_CUDA(cudaDeviceSynchronize());
     if (st->ws) {
-        MNI_CUDA(cudaDeviceSynchronize());
         MNI_CUDA(cudaFree(st->ws));
         st->ws = nullptr;
         st->ws_bytes = 0;
+        st->ws_recorded = false;
+    }
+    while (!st->retired.empty()) {
+        MNI_CUDA(cudaFree(st->retired.back()));
+        st->retired.pop_back();
     }
     return MNI_B200_OK;
 }

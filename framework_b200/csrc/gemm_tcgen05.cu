@@ -28,6 +28,18 @@
 //               tails.  Split-K partials go through the same path into scratch.  Outputs whose row
 //               pitch is not a multiple of 16 bytes take a plain-store fallback.
 //
+// Large products take their operands as 16-bit planes instead, which half.cu makes of them beforehand (kHalfThree, kHalfOne): the
+// f16 pipe has the eleven bits of TF32 at twice the rate.  Nothing is split here then; the split warps only relay "landed".
+//   kHalfThree  per k-block of 64: hi*hi into one accumulator, lo*hi and hi*lo (scaled by 2^12) into another, both of them all of
+//               tensor memory.  The epilogue takes both into its registers and the next unit begins; the large terms' chain is a
+//               third as long as in 3xTF32, and its rounding a sixth (1.24e-6 -> 3.5e-7 at K = 512, 7.6e-6 -> 1.25e-6 at 2048
+//               to 3072), so a piece may be 4096 long.  Bound by the power cap in a loop, by L2 (16 KB a CTA and 16 elements) at
+//               full clocks.  8192^3: 24.9 cycles per element of a tile for the pipe's 24, 3.7 -> 2.4 ms a product with the pass
+//               over the operands; as one accumulator with hi staged a second time, 33 cycles and 2.8 ms (L2).
+//   kHalfOne    hi*hi alone, accumulators double-buffered as in single-pass TF32: 10 cycles for the pipe's 8 (L2: 8 KB a CTA and
+//               16 elements), 1.9 -> 1.2 ms.
+// Operands whose range f16 does not hold come as three (two) bf16 planes through the same stages.
+//
 // CG = 2: two CTAs of a cluster share a 256 x BN tile (cta_group::2 MMAs issued by the leader).
 // Work is dealt out as whole tiles, round-robin over the CTAs (pairs).  The tiles of a badly ragged wave are cut into
 // several units each, whose partial tiles go to scratch and are added by tail_finish_kernel (cut_tail has the rule).  On
@@ -50,6 +62,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <cmath>
 #include <mutex>
 #include <unordered_map>
 
@@ -67,6 +80,9 @@ constexpr long long kWaitCycles = 4000000000LL;            // default limit of e
 
 enum OperandMode { kKMajor = 0, kMnMultiBox = 1, kMnSingleBox = 2 };
 enum TailMode { kWholeTiles = 0, kBalanced = 1, kCutTiles = 2, kRunningSum = 3 };
+// How a product is computed: operands as f32 (three TF32 passes, or one), or as the 16-bit halves that split_half_kernel has made
+// of them (three passes, or one).
+enum PassMode { kThreePass = 0, kOnePass = 1, kHalfThree = 2, kHalfOne = 3 };
 enum EpilogueMode { kEpiPlainStores = 0, kEpiTmaStore = 1, kEpiTmaReduce = 2, kEpiVectorStores = 3 };
 
 struct KParams {
@@ -116,6 +132,10 @@ struct KParams {
     int sk_first_tile;         // tiles below this index are dealt out whole, round-robin
     float *sk_partial;         // two parked accumulator tiles per CTA: [cta][2][epilogue warp][chunk][8][lane] float4
     unsigned int *sk_flags;    // ready flags [cta][2][epilogue warp] (1 = parked), then tickets [tile][rank][epilogue warp]
+    // 16-bit halves: what split_half_kernel left beside them
+    const int *a_exp, *b_exp;              // the operands were multiplied by 2^exponent
+    const unsigned int *half_status;       // a word per block of it: != 0, some operand's range does not fit
+    int half_statuses;
 };
 
 // ------------------------------------------------------------------ PTX helpers
@@ -289,6 +309,17 @@ __device__ __forceinline__ void umma_tf32_pair(uint32_t d_tmem, uint32_t a_lo, u
         "mov.b64 db, {%3, %4};\n\t"
         "setp.ne.b32 p, %6, 0;\n\t"
         "tcgen05.mma.cta_group::2.kind::tf32 [%0], da, db, %5, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void umma_f16_pair(uint32_t d_tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo,
+                                              uint32_t b_hi, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+        "mov.b64 da, {%1, %2};\n\t"
+        "mov.b64 db, {%3, %4};\n\t"
+        "setp.ne.b32 p, %6, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], da, db, %5, p;\n\t}"
         ::"r"(d_tmem), "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)
         : "memory");
 }
@@ -479,6 +510,13 @@ __device__ __forceinline__ void load_operand(int mode, uint32_t dst, const CUten
     }
 }
 
+// The same for a tile of 16-bit halves: 64 elements of the contiguous dimension wide, 128 rows.
+__device__ __forceinline__ void load_half(int mode, uint32_t dst, const CUtensorMap *map, uint32_t bar, int k0, int row0, int batch,
+                                          int plane) {
+    if (mode == kKMajor) tma_load_5d(dst, map, bar, k0, row0, batch, plane, 0);
+    else tma_load_5d(dst, map, bar, 0, k0, row0 >> 6, batch, plane);
+}
+
 // CG = 1: one CTA computes a 128 x BN tile.  CG = 2: a pair of CTAs (a 2-CTA cluster) computes a
 // 256 x BN tile with cta_group::2 MMAs issued by the pair's leader; each CTA stages its own 128 rows
 // of A and half (BN/2 rows) of B, so shared-memory and L2 traffic per flop drop by a third.
@@ -501,26 +539,34 @@ struct RegShare {
     static constexpr int kSplitGroups = FAST ? 1 : 2, kLaunch = FAST ? 128 : 96;
     static_assert(2 * kEpilogue + kSplitGroups * kSplit + kIssue <= (3 + kSplitGroups) * kLaunch, "more registers than the launch has");
 };
-template <int BN, int BK, bool FAST, int NS, int CG, bool TA = false, int TAIL = kWholeTiles, int SG = 1>
+// ... and of the two-accumulator variant, 168 of 384 threads at launch: two epilogue warpgroups and the one of all other roles.
+constexpr int kTwoEpilogue = 232, kTwoIssue = 40, kTwoLaunch = 168;
+static_assert(2 * kTwoEpilogue + kTwoIssue <= 3 * kTwoLaunch, "more registers than the launch has");
+template <int BN, int BK, int MODE, int NS, int CG, bool TA = false, int TAIL = kWholeTiles, int SG = 1>
 __global__ void __launch_bounds__(gemm_threads(NS, TAIL == kRunningSum), 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmD,
                const __grid_constant__ CUtensorMap tmP, const __grid_constant__ KParams p) {
     constexpr bool SK = TAIL == kBalanced, CUT = TAIL == kCutTiles;
+    constexpr bool HALF = MODE == kHalfThree || MODE == kHalfOne, FAST = MODE != kThreePass;   // FAST: the split warps split nothing
+    static_assert(!HALF || (BN == 256 && BK == 64 && CG == 2 && !TA && !SK), "16-bit halves are built for 256-wide pairs");
+    constexpr uint32_t ELT = HALF ? 2 : 4;                 // bytes of a staged element
     constexpr int BNL = BN / CG;                           // B rows staged by this CTA
-    constexpr uint32_t A_BYTES = BM * BK * 4;
-    constexpr uint32_t B_BYTES = BNL * BK * 4;
+    constexpr uint32_t A_BYTES = BM * BK * ELT;
+    constexpr uint32_t B_BYTES = BNL * BK * ELT;
     constexpr uint32_t RAW_BYTES = A_BYTES + B_BYTES;
     // RUN: a unit's running sum over its pieces takes 128 registers of every epilogue thread, so the warps are laid out in
     // whole warpgroups -- TMA and MMA (and two idle), split, epilogue -- that trade registers.
-    constexpr bool RUN = TAIL == kRunningSum;
+    // TWO: the large and the small terms of a piece in an accumulator each, all of tensor memory; the epilogue takes both into its
+    // registers, whole, before anything is stored, and the next piece begins.
+    constexpr bool TWO = MODE == kHalfThree, RUN = TAIL == kRunningSum || TWO;
     static_assert(!RUN || (BN == 256 && CG == 2), "running sums are built for 256-wide pairs");
-    constexpr int SPLIT0 = RUN ? 4 : 2, EPI0 = SPLIT0 + NS;   // first split and first epilogue warp
+    constexpr int SPLIT0 = RUN && !TWO ? 4 : 2, EPI0 = SPLIT0 + NS;   // first split and first epilogue warp
     static_assert(!TA || (!FAST && CG == 1 && BK == 32 && NS == 8 && BN <= 128), "unsupported A-from-TMEM variant");
     constexpr uint32_t STAGE_BYTES = FAST ? RAW_BYTES : (TA ? A_BYTES + 2 * B_BYTES : 2 * RAW_BYTES);
     constexpr uint32_t STAGE16 = STAGE_BYTES >> 4;
     constexpr uint32_t LO16 = (TA ? B_BYTES : RAW_BYTES) >> 4;   // lo copy relative to its raw tile, 16-byte units
-    constexpr int KSTEPS = BK / 8;
+    constexpr int KSTEPS = BK / (HALF ? 16 : 8);
     constexpr uint32_t TMEM_COLS = TA ? 512 : 2 * BN;      // double-buffered accumulator (+ the A slots)
     constexpr uint32_t TA_COL0 = 2 * BN;                   // first column of the A slots
     constexpr uint32_t TA_SLOT = 2 * BK;                   // hi | lo
@@ -560,7 +606,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     if (threadIdx.x == 0) {
         for (int s = 0; s < p.stages; ++s) {
             mbar_init(bar_full + 8u * s, 1);
-            mbar_init(bar_xform + 8u * s, CG * NS / SG);   // one arrival per split warp (of the k-block's group; of both CTAs for a pair)
+            mbar_init(bar_xform + 8u * s, HALF ? CG : CG * NS / SG);   // one arrival per split warp (of the k-block's group; of both CTAs for a pair)
             mbar_init(bar_empty + 8u * s, 1);
         }
         for (int i = 0; i < 2; ++i) {
@@ -595,12 +641,27 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     // an independent pair needs nothing from the first: it runs beside it and waits for it only before it ends.
     if (p.dep_mode != 2) grid_dependency_wait();
     if (p.dep_mode == 1 && threadIdx.x == 0) grid_dependency_trigger();
-
+    // HALF: wide if some operand's range did not fit f16, and the planes hold bf16 thirds, unscaled.
+    float unscale = 1.f;
+    bool wide = false;
+    if constexpr (HALF) {
+        unsigned int status = 0;
+        for (int i = threadIdx.x; i < p.half_statuses; i += blockDim.x) status |= __ldcg(p.half_status + i);
+        int ea = __ldcg(p.a_exp), eb = __ldcg(p.b_exp);          // at most 60 either way
+        wide = __syncthreads_or(status & 1u) != 0;
+        if (wide) {
+            const bool huge = __syncthreads_or(status & 2u) != 0;
+            ea = half_wide_exponent(ea, huge);
+            eb = half_wide_exponent(eb, huge);
+        }
+        unscale = __uint_as_float(static_cast<uint32_t>(127 - ea - eb) << 23);
+    }
+    const int planes = TWO ? (wide ? 3 : 2) : (wide ? 2 : 1);     // HALF
 
     // The epilogue comes first: it is the branch whose register share the running-sum variants raise.
     if (warp >= EPI0) {
         // RUN: the warpgroups trade registers; the increase waits for the others' decrease
-        if constexpr (RUN) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(RegShare<FAST>::kEpilogue));
+        if constexpr (RUN) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(TWO ? kTwoEpilogue : RegShare<FAST>::kEpilogue));
         // ------------------------------------------------------------ epilogue
         const int q = warp & 3;                       // TMEM lane quarter this warp may read
         const int ew = warp - EPI0;               // 0..7: warps ew and ew+4 share a lane quarter ...
@@ -619,8 +680,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         const int my_cta = static_cast<int>(blockIdx.x);                 // slot * CG + rank in the pair
         uint32_t run[RUN ? CHUNKS : 1][32];           // RUN: sum of the unit's pieces so far
         while (ok && work_next<TAIL>(p, wi, t)) {
-            const int buf = acc_it & 1;
-            const uint32_t acc_phase = (acc_it >> 1) & 1;
+            const int buf = TWO ? 0 : acc_it & 1;
+            const uint32_t acc_phase = TWO ? acc_it & 1 : (acc_it >> 1) & 1;
             ok = mbar_wait(bar_acc_full + 8u * buf, acc_phase, abort_flag, p.err, 0x500u | buf, waited, timed, p.wait_cycles);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
@@ -701,14 +762,30 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         }
                     }
                 }
-                if (p.prof) t_ld += clock64() - t_ld0;
                 // the accumulator has been read: the MMA warp may refill it while this sum goes out
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) {
-                    if (CG == 2 && cta_rank != 0) mbar_arrive_cta(bar_acc_empty + 8u * buf, 0u);
-                    else mbar_arrive(bar_acc_empty + 8u * buf);
+                auto release = [&](int slot) {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) {
+                        if (CG == 2 && cta_rank != 0) mbar_arrive_cta(bar_acc_empty + 8u * slot, 0u);
+                        else mbar_arrive(bar_acc_empty + 8u * slot);
+                    }
+                };
+                release(buf);
+                if constexpr (TWO) {
+                    const float small_scale = wide ? 1.f : 1.f / (1 << kHalfLoShift);
+#pragma unroll
+                    for (int c = 0; c < CHUNKS; ++c) {
+                        uint32_t x[32];
+                        tmem_ld32_issue(tbase + BN + (chunk_lo + c) * 32, x);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int e = 0; e < 32; ++e)
+                            run[c][e] = __float_as_uint(fmaf(__uint_as_float(x[e]), small_scale, __uint_as_float(run[c][e])));
+                    }
+                    release(1);
                 }
+                if (p.prof) t_ld += clock64() - t_ld0;
                 ++acc_it;
                 if (!last_piece) continue;
             }
@@ -726,6 +803,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         tmem_ld32_issue(tbase + chunk * 32, v);
                         tmem_ld_wait();
                         if (p.prof) t_ld += clock64() - t_ld0;
+                    }
+                    if constexpr (HALF) {
+#pragma unroll
+                        for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) * unscale);
                     }
                     if (park_it) {
                         // [j][lane] order: one instruction of the warp writes 512 contiguous bytes
@@ -855,7 +936,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         }
                         if (++patch == p.epi_patches) patch = 0;
                     };
-                    const bool do_act = !RUN && fuse && p.act != 0;          // host guarantees use_tma in this mode
+                    const bool do_act = (!RUN || HALF) && fuse && p.act != 0;          // host guarantees use_tma in this mode
                     if (do_act && p.store_pre) emit(&tmC, false);    // the raw product, what the tape saves
                     if (fuse && p.bias != nullptr && add_piece) {
                         // the bias went in with the first piece
@@ -883,7 +964,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         emit(&tmD, false, true);
                     } else if (part) {
                         emit(&tmP, add_piece);
-                    } else if (RUN || use_tma) {
+                    } else if ((RUN && !HALF) || use_tma) {
                         emit(&tmC, (p.epi_mode == kEpiTmaReduce && fuse) || add_piece);
                     } else {
                         float *out0 = fuse ? p.C + static_cast<long long>(t.bt) * p.c_bstride + static_cast<long long>(row0) * p.ldc
@@ -987,7 +1068,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
     } else {
     if constexpr (RUN) {
-        if (warp < SPLIT0) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(RegShare<FAST>::kIssue));
+        if (TWO) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kTwoIssue));
+        else if (warp < SPLIT0) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(RegShare<FAST>::kIssue));
         else asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(RegShare<FAST>::kSplit));
     }
     if (warp == 0) {
@@ -1015,6 +1097,34 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 batch_coords(t.bt * p.fold + f, p.b_batch, p.b_d1, p.b_d2, p.fd_b_cnt, p.fd_b_d1, p.fd_b_d2, b0, b1, b2);
                 const int rowA = t.tm * (BM * CG) + static_cast<int>(cta_rank) * BM;
                 const int rowB = t.tn * BN + static_cast<int>(cta_rank) * BNL;
+                if constexpr (HALF) {
+                    // The planes of a k-block are staged one after the other, each in a stage of its own.  The plane is the map's
+                    // second batch coordinate.
+                    for (int it = t.it0; ok && it < t.it1; ++it) {
+                        for (int plane = 0; plane < planes; ++plane) {
+                            ok = mbar_wait_warp(bar_empty + 8u * stage, phase ^ 1u, abort_flag, p.err, 0x100u | stage, waited, timed, p.wait_cycles);
+                            if (!ok) break;
+                            const uint32_t full = bar_full + 8u * stage;
+                            ++armed;
+                            if (elect_one()) {
+                                mbar_arrive_expect_tx(full, RAW_BYTES);
+                                if (armed != p.withhold_at) {
+                                    load_half(p.a_mode, dstA, &tmA, full, kk * BK, rowA, a2, plane);
+                                    load_half(p.b_mode, dstA + A_BYTES, &tmB, full, kk * BK, rowB, b2, plane);
+                                }
+                            }
+                            if (++stage == p.stages) { stage = 0; phase ^= 1u; dstA = dstA0; } else { dstA += STAGE_BYTES; }
+                        }
+                        if (++kk == p.kiters) {
+                            kk = 0;
+                            ++f;
+                            if (p.fold > 1) {
+                                batch_coords(t.bt * p.fold + f, p.a_batch, p.a_d1, p.a_d2, p.fd_a_cnt, p.fd_a_d1, p.fd_a_d2, a0, a1, a2);
+                                batch_coords(t.bt * p.fold + f, p.b_batch, p.b_d1, p.b_d2, p.fd_b_cnt, p.fd_b_d1, p.fd_b_d2, b0, b1, b2);
+                            }
+                        }
+                    }
+                } else
                 for (int it = t.it0; it < t.it1; ++it) {
                     ok = mbar_wait_warp(bar_empty + 8u * stage, phase ^ 1u, abort_flag, p.err, 0x100u | stage, waited, timed, p.wait_cycles);
                     if (!ok) break;
@@ -1067,7 +1177,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             uint32_t a_lo = a_lo0, b_lo = b_lo0;
             const uint32_t a_hi = p.a_desc_hi, b_hi = p.b_desc_hi;
             const uint32_t a_ks = p.a_kstep, b_ks = p.b_kstep;
-            const uint32_t idesc = p.idesc;
+            const uint32_t idesc = HALF && wide ? p.idesc | (1u << 7) | (1u << 10) : p.idesc;     // bf16 operands
             // A lone CTA in single-pass mode consumes the TMA barrier directly; otherwise the split warps
             // (of both CTAs, for a pair) announce the stage on the leader's barrier.
             const uint32_t ready0 = (FAST && CG == 1) ? bar_full : bar_xform;
@@ -1075,13 +1185,66 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             TileCoord wt;
             while (ok && work_next<TAIL>(p, wi, wt)) {
                 const int iters = wt.it1 - wt.it0;
-                const int buf = acc_it & 1;
-                const uint32_t acc_phase = (acc_it >> 1) & 1;
+                const int buf = TWO ? 0 : acc_it & 1;
+                const uint32_t acc_phase = TWO ? acc_it & 1 : (acc_it >> 1) & 1;
                 ok = mbar_wait_warp(bar_acc_empty + 8u * buf, acc_phase ^ 1u, abort_flag, p.err, 0x200u | buf, waited_acc, timed, p.wait_cycles);
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(buf * BN);
                 uint32_t accumulate = 0;
+                if constexpr (HALF) {
+                    auto next = [&] {
+                        if (++stage == p.stages) { stage = 0; phase ^= 1u; a_lo = a_lo0; b_lo = b_lo0; }
+                        else { a_lo += STAGE16; b_lo += STAGE16; }
+                    };
+                    for (int it = 0; it < iters; ++it) {
+                        ok = mbar_wait_warp(ready0 + 8u * stage, phase, abort_flag, p.err, 0x300u | stage, waited, timed, p.wait_cycles);
+                        if (!ok) break;
+                        tc_fence_after();
+                        const uint32_t hi_stage = static_cast<uint32_t>(stage), ah = a_lo, bh = b_lo;
+                        if (elect_one()) {
+#pragma unroll
+                            for (int ks = 0; ks < KSTEPS; ++ks)
+                                umma_f16_pair(d_tmem, ah + ks * a_ks, a_hi, bh + ks * b_ks, b_hi, idesc, ks == 0 ? accumulate : 1u);
+                            if (planes == 1) umma_commit_pair(bar_empty + 8u * hi_stage);
+                        }
+                        __syncwarp();
+                        next();
+                        // The products with the planes below hi: into an accumulator of their own (TWO) or the same.
+                        uint32_t small_acc = TWO ? accumulate : 1u;
+                        for (int plane = 1; plane < planes; ++plane) {
+                            ok = mbar_wait_warp(ready0 + 8u * stage, phase, abort_flag, p.err, 0x300u | stage, waited, timed, p.wait_cycles);
+                            if (!ok) break;
+                            if (TWO && it == 0 && plane == 1) {     // its accumulator comes free a little later than the other
+                                ok = mbar_wait_warp(bar_acc_empty + 8u, acc_phase ^ 1u, abort_flag, p.err, 0x201u, waited_acc, timed, p.wait_cycles);
+                                if (!ok) break;
+                            }
+                            tc_fence_after();
+                            const uint32_t d_small = d_tmem + (TWO ? BN : 0);
+                            if (elect_one()) {
+#pragma unroll
+                                for (int ks = 0; ks < KSTEPS; ++ks) {
+                                    umma_f16_pair(d_small, a_lo + ks * a_ks, a_hi, bh + ks * b_ks, b_hi, idesc, ks == 0 ? small_acc : 1u);
+                                    umma_f16_pair(d_small, ah + ks * a_ks, a_hi, b_lo + ks * b_ks, b_hi, idesc, 1u);
+                                    if (TWO && wide && plane == 1)
+                                        umma_f16_pair(d_small, a_lo + ks * a_ks, a_hi, b_lo + ks * b_ks, b_hi, idesc, 1u);
+                                }
+                                umma_commit_pair(bar_empty + 8u * stage);
+                                if (plane + 1 == planes) umma_commit_pair(bar_empty + 8u * hi_stage);
+                            }
+                            __syncwarp();
+                            small_acc = 1u;
+                            next();
+                        }
+                        if (!ok) break;
+                        accumulate = 1u;
+                    }
+                    if (ok && elect_one()) umma_commit_pair(bar_acc_full + 8u * buf);
+                    __syncwarp();
+                    if (!ok) break;
+                    ++acc_it;
+                } else
+                {
                 for (int it = 0; it < iters; ++it) {
                     if (!next_ready) {
                         ok = mbar_wait_warp(ready0 + 8u * stage, phase, abort_flag, p.err, 0x300u | stage, waited, timed, p.wait_cycles);
@@ -1107,6 +1270,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                                 umma_tf32_ts(d_tmem, at + BK, bk, b_hi, idesc, acc_first);
                                 umma_tf32_ts(d_tmem, at, bk + LO16, b_hi, idesc, 1u);
                                 umma_tf32_ts(d_tmem, at, bk, b_hi, idesc, 1u);
+                            } else if constexpr (HALF) {
                             } else if constexpr (CG == 2 && FAST) {
                                 umma_tf32_pair(d_tmem, ak, a_hi, bk, b_hi, idesc, acc_first);
                             } else if constexpr (CG == 2) {
@@ -1136,13 +1300,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 if constexpr (CG == 2) { if (elect_one()) umma_commit_pair(bar_acc_full + 8u * buf); }
                 else { if (elect_one()) umma_commit(bar_acc_full + 8u * buf); }
                 ++acc_it;
+                }
             }
             if (p.prof && lane == 0) {
                 atomicAdd(p.prof + 1, static_cast<unsigned long long>(waited_acc));
                 atomicAdd(p.prof + 2, static_cast<unsigned long long>(waited));
             }
         }
-    } else if (RUN && warp < SPLIT0) {
+    } else if (RUN && !TWO && warp < SPLIT0) {
         // idle: the rest of the first warpgroup
     } else {
         // ------------------------------------------------------------ hi/lo split
@@ -1170,8 +1335,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             constexpr int U = !EXACT ? 1 : (PER % 4 == 0) ? 4 : (PER % 2 == 0 ? 2 : 1);
             WorkIter wi = work_begin(p, unit0, unit_step);
             TileCoord wt;
+            if (HALF && warp != SPLIT0) ok = false;           // one warp relays there
             while (ok && work_next<TAIL>(p, wi, wt)) {
-                const int iters = wt.it1 - wt.it0;
+                int iters = wt.it1 - wt.it0;
+                if (HALF) iters *= planes;                        // each takes a stage
                 for (int it = 0; it < iters; ++it) {
                     if (SG == 2 && ((kb++ & 1) != group)) {    // the other group's k-block
                         if (++stage == p.stages) { stage = 0; phase ^= 1u; }
@@ -1466,7 +1633,7 @@ struct MapKey {
     cuuint64_t dims[5];
     cuuint64_t strides[4];
     cuuint32_t box[5];
-    int swz;
+    int swz;                       // and the element type
     bool operator==(const MapKey &o) const { return memcmp(this, &o, sizeof(MapKey)) == 0; }
 };
 struct MapKeyHash {
@@ -1484,8 +1651,8 @@ struct MapKeyHash {
 };
 constexpr size_t kMapCacheEntries = 512;
 
-CUresult encode(CUtensorMap *map, const float *ptr, const cuuint64_t *dims, const cuuint64_t *strides,
-                const cuuint32_t *box, CUtensorMapSwizzle swz) {
+CUresult encode(CUtensorMap *map, const void *ptr, const cuuint64_t *dims, const cuuint64_t *strides,
+                const cuuint32_t *box, CUtensorMapSwizzle swz, CUtensorMapDataType type = CU_TENSOR_MAP_DATA_TYPE_FLOAT32) {
     static thread_local std::unordered_map<MapKey, CUtensorMap, MapKeyHash> cache;
     static const bool use_cache = env_int("MNI_B200_MAP_CACHE", 1) != 0;
     MapKey key;
@@ -1493,13 +1660,13 @@ CUresult encode(CUtensorMap *map, const float *ptr, const cuuint64_t *dims, cons
     key.ptr = ptr;
     for (int i = 0; i < 5; ++i) { key.dims[i] = dims[i]; key.box[i] = box[i]; }
     for (int i = 0; i < 4; ++i) key.strides[i] = strides[i];
-    key.swz = static_cast<int>(swz);
+    key.swz = static_cast<int>(swz) + 256 * static_cast<int>(type);
     if (use_cache) {
         auto it = cache.find(key);
         if (it != cache.end()) { *map = it->second; return CUDA_SUCCESS; }
     }
     const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
-    const CUresult r = encode_fn()(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 5, const_cast<float *>(ptr), dims, strides, box,
+    const CUresult r = encode_fn()(map, type, 5, const_cast<void *>(ptr), dims, strides, box,
                                    estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r == CUDA_SUCCESS && use_cache) {
@@ -1581,6 +1748,29 @@ int make_operand_map(CUtensorMap *map, const Operand &op, int box_rows, int bk, 
     return MNI_B200_OK;
 }
 
+// Tensor map of an operand in 16-bit halves.  K-major: (kdim, rows, batch, plane) in boxes of 64 x 128.  MN-major: (64 contiguous
+// rows, kdim, chunks of 64 rows, batch, plane) in boxes of 64 x 64 x 2; the pitch is a multiple of 64 there.
+int make_half_map(CUtensorMap *map, const HalfOperand &op, int *mode) {
+    if (!encode_fn()) return fail(MNI_B200_ERR_CUDA, "cuTensorMapEncodeTiled entry point not found");
+    cuuint64_t dims[5], strides[4];
+    cuuint32_t box[5] = {64, 128, 1, 1, 1};
+    const cuuint64_t pitch = static_cast<cuuint64_t>(op.pitch) * 2, matrix = static_cast<cuuint64_t>(op.matrix) * 2,
+                     plane = static_cast<cuuint64_t>(op.plane) * 2, batch = static_cast<cuuint64_t>(op.batch);
+    if (op.k_major) {
+        dims[0] = static_cast<cuuint64_t>(op.kdim); dims[1] = static_cast<cuuint64_t>(op.rows); dims[2] = batch; dims[3] = static_cast<cuuint64_t>(op.planes); dims[4] = 1;
+        strides[0] = pitch; strides[1] = matrix; strides[2] = plane; strides[3] = 2 * plane;
+        *mode = kKMajor;
+    } else {
+        dims[0] = 64; dims[1] = static_cast<cuuint64_t>(op.kdim); dims[2] = static_cast<cuuint64_t>((op.rows + 63) / 64); dims[3] = batch; dims[4] = static_cast<cuuint64_t>(op.planes);
+        strides[0] = pitch; strides[1] = 128; strides[2] = matrix; strides[3] = plane;
+        box[1] = 64; box[2] = 2;
+        *mode = kMnSingleBox;
+    }
+    const CUresult r = encode(map, op.ptr, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_DATA_TYPE_FLOAT16);
+    if (r != CUDA_SUCCESS) return fail(MNI_B200_ERR_CUDA, "cuTensorMapEncodeTiled(halves) failed (%d)", static_cast<int>(r));
+    return MNI_B200_OK;
+}
+
 // Tensor map of the output (or of the split-K partial buffer): dims (N, M, batches), 32 x 32 boxes.
 int make_output_map(CUtensorMap *map, float *ptr, int64_t N, int64_t M, int64_t batches, int64_t ld, int64_t bstride) {
     cuuint64_t dims[5] = {static_cast<cuuint64_t>(N), static_cast<cuuint64_t>(M), static_cast<cuuint64_t>(batches), 1, 1};
@@ -1627,7 +1817,7 @@ double finish_us(double parts, double bytes) { return 1.5 + (parts + 1.0) * byte
 // 2048 x 3072 x 3584 177 / 169 / 168; at K = 2048, 121 / 117 / -, it would save 4.6 %.  Not in single-pass mode, whose long units
 // lose more by giving up their running sum (2048 x 8192 x 3584 200 / 209 / 231), and not beside another product, which uses the
 // SMs that the wave leaves.  `round_only`: neither.
-Cut cut_tail(long long tiles, long long slots, long long k, bool round_only) {
+Cut cut_tail(long long tiles, long long slots, long long k, bool round_only, double pair_ns = kPairNs) {
     const long long full = tiles / slots, rem = tiles - full * slots;
     const double tile_bytes = 4.0 * 2 * BM * 256;
     const Cut whole{1, static_cast<double>(rem > 0 ? full + 1 : full), 0.0};
@@ -1637,7 +1827,7 @@ Cut cut_tail(long long tiles, long long slots, long long k, bool round_only) {
     if (full >= 1 && ways >= 2 && eff < 0.80 && k / ways >= 128)
         return Cut{ways, static_cast<double>(full) + 1.0 / static_cast<double>(ways), finish_us(static_cast<double>(ways), tile_bytes * static_cast<double>(rem))};
     if (round_only) return whole;
-    const double round_us = static_cast<double>(k) * kPairNs * 1e-3;
+    const double round_us = static_cast<double>(k) * pair_ns * 1e-3;
     Cut best = whole;
     for (long long w = 2; w <= 6 && k / w >= 256; ++w) {
         const Cut c{w, static_cast<double>(full) + static_cast<double>((rem * w + slots - 1) / slots) / static_cast<double>(w),
@@ -1649,12 +1839,53 @@ Cut cut_tail(long long tiles, long long slots, long long k, bool round_only) {
 }
 // Longest accumulation chain in tensor memory, in k-blocks (MNI_B200_CHUNK_K contraction elements; 0 = no limit).  The fused
 // activation needs the whole sum in one accumulator.
+constexpr int kHalfChunkK = 4096;
 int chunk_iters_for(const GemmProblem &p, int bk) {
-    const int chunk_k = env_int("MNI_B200_CHUNK_K", 1024);
+    const int chunk_k = env_int("MNI_B200_CHUNK_K", p.ha ? kHalfChunkK : 1024);
     return (chunk_k > 0 && p.D == nullptr) ? std::max(1, chunk_k / bk) : 0;
 }
 
+// Main loop of a 256-wide pair over 16-bit planes, nanoseconds per contraction element, in a loop of calls (the pipe's own 12.6
+// and 4.2 at 1.9 GHz are out of reach of the power, and of L2, which feeds 32 and 16 KB a pair and 16 elements).
+double half_pair_ns(const GemmProblem &p) { return p.fast_tf32 ? 7.0 : 16.5; }
+
+// Products of 16-bit halves: 256-wide pairs throughout.  Few tiles: the contraction is split until the pairs are busy; a ragged
+// last wave is cut as cut_tail says.
+Plan make_half_plan(const GemmProblem &p, int sm_count) {
+    Plan pl{};
+    pl.bn = 256;
+    pl.bk = 64;
+    pl.cg = 2;
+    pl.patches = 1;
+    const size_t stage = static_cast<size_t>(BM + 128) * pl.bk * 2, fixed = 1024 + kBarBytes + static_cast<size_t>(kEpiWarps) * kEpiBufBytes;
+    pl.stages = static_cast<int>(std::min<size_t>(kMaxStages, (227 * 1024 - fixed) / stage));
+    pl.smem = fixed + static_cast<size_t>(pl.stages) * stage;
+    const int slots = std::max(1, sm_count / 2);
+    pl.tiles_m = static_cast<int>((p.M + 255) / 256);
+    pl.tiles_n = static_cast<int>((p.N + 255) / 256);
+    const long long tiles = static_cast<long long>(p.batch) * pl.tiles_m * pl.tiles_n;
+    const long long iters = p.fold * ((p.K + pl.bk - 1) / pl.bk);
+    long long splits = 1;
+    if (tiles * 2 <= slots && iters >= 8) splits = std::max<long long>(1, std::min<long long>(slots / tiles, iters / 4));
+    pl.splits = static_cast<int>(std::min<long long>(splits, 64));
+    const long long units = tiles * pl.splits;
+    pl.grid = static_cast<int>(std::min<long long>(units, slots)) * 2;
+    if (pl.splits == 1) {
+        const Cut cut = cut_tail(tiles, slots, iters * pl.bk, false, half_pair_ns(p));
+        if (cut.ways > 1) {
+            pl.tail_ways = static_cast<int>(cut.ways);
+            pl.tail_tiles = static_cast<int>(tiles % slots);
+            pl.grid = static_cast<int>(std::min<long long>(tiles + pl.tail_tiles * (cut.ways - 1), slots)) * 2;
+            return pl;
+        }
+    }
+    const long long chunk = chunk_iters_for(p, pl.bk), unit_len = (iters + pl.splits - 1) / pl.splits;
+    pl.running = chunk > 0 && unit_len > chunk + (chunk >> 3);
+    return pl;
+}
+
 Plan make_plan(const GemmProblem &p, int sm_count) {
+    if (p.ha) return make_half_plan(p, sm_count);
     Plan pl;
     pl.bn = p.N <= 64 ? 64 : (p.N <= 128 ? 128 : 256);
     const int bn_env = env_int("MNI_B200_BN", 0);
@@ -1835,7 +2066,7 @@ uint32_t desc_hi_bits(uint32_t sbo_bytes, uint32_t layout_type) {
     return ((sbo_bytes >> 4) & 0x3FFFu) | (1u << 14) | (layout_type << 29);
 }
 
-template <int BN, int BK, bool FAST, int NS, int CG, bool TA = false, int TAIL = kWholeTiles, int SG = 1>
+template <int BN, int BK, int MODE, int NS, int CG, bool TA = false, int TAIL = kWholeTiles, int SG = 1>
 cudaError_t launch_variant(const Plan &pl, const CUtensorMap &tmA, const CUtensorMap &tmB, const CUtensorMap &tmC,
                            const CUtensorMap &tmD, const CUtensorMap &tmP, const KParams &k, cudaStream_t stream) {
     // The shared-memory opt-in is an attribute of the function on ONE device: set once per device of the process
@@ -1846,7 +2077,7 @@ cudaError_t launch_variant(const Plan &pl, const CUtensorMap &tmA, const CUtenso
     if (attr != cudaSuccess) return attr;
     const uint64_t bit = 1ull << (dev & 63);
     if ((opted_in.load(std::memory_order_acquire) & bit) == 0) {
-        attr = cudaFuncSetAttribute(gemm_tc_kernel<BN, BK, FAST, NS, CG, TA, TAIL, SG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        attr = cudaFuncSetAttribute(gemm_tc_kernel<BN, BK, MODE, NS, CG, TA, TAIL, SG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     227 * 1024);
         if (attr != cudaSuccess) return attr;
         opted_in.fetch_or(bit, std::memory_order_release);
@@ -1865,7 +2096,7 @@ cudaError_t launch_variant(const Plan &pl, const CUtensorMap &tmA, const CUtenso
     attrs[1].val.clusterDim.z = 1;
     cfg.attrs = attrs;
     cfg.numAttrs = CG == 2 ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, gemm_tc_kernel<BN, BK, FAST, NS, CG, TA, TAIL, SG>, tmA, tmB, tmC, tmD, tmP, k);
+    return cudaLaunchKernelEx(&cfg, gemm_tc_kernel<BN, BK, MODE, NS, CG, TA, TAIL, SG>, tmA, tmB, tmC, tmD, tmP, k);
 }
 
 }  // namespace
@@ -1924,7 +2155,7 @@ GemmProblem kernel_view(const GemmProblem &p, bool *transposed) {
     *transposed = false;
     const bool storable = (reinterpret_cast<uintptr_t>(p.C) & 15) == 0 && p.ldc % 4 == 0 && p.c_bstride % 4 == 0 &&
                           p.N % 4 == 0 && env_int("MNI_B200_NO_TMA_STORE", 0) == 0 && env_int("MNI_B200_EPI_VECTOR", 0) == 0;
-    if (p.D != nullptr || p.M > 64 || p.N < 256 || !storable || env_int("MNI_B200_TRANSPOSE_OUT", 1) == 0) return p;
+    if (p.ha != nullptr || p.D != nullptr || p.M > 64 || p.N < 256 || !storable || env_int("MNI_B200_TRANSPOSE_OUT", 1) == 0) return p;
     GemmProblem q = p;
     std::swap(q.A, q.B);
     std::swap(q.M, q.N);
@@ -1962,6 +2193,27 @@ double gemm_tc_estimate_us(const GemmProblem &p, int sm_count) {
     return p.fast_tf32 ? 0.0 : make_plan(kernel_view(p, &transposed), sm_count).est_us;
 }
 
+double gemm_estimate_us(const GemmProblem &p0, bool half, int sm_count) {
+    static const HalfOperand any;
+    GemmProblem p = p0;
+    p.ha = half ? &any : nullptr;
+    bool transposed = false;
+    p = kernel_view(p, &transposed);
+    const Plan pl = make_plan(p, sm_count);
+    if (pl.est_us > 0 && !p.fast_tf32) return pl.est_us;
+    const double k = static_cast<double>(p.K) * static_cast<double>(p.fold);
+    const double ns = half ? half_pair_ns(p) : (p.fast_tf32 ? 13.0 : kPairNs) * (pl.bn == 256 ? 1.0 : (pl.bn == 128 ? 0.65 : 0.45));
+    const double slots = std::max(1, sm_count / pl.cg), tiles = static_cast<double>(p.batch) * pl.tiles_m * pl.tiles_n;
+    const double out = 4.0 * static_cast<double>(p.batch) * static_cast<double>(p.M) * static_cast<double>(p.N);
+    double rounds = std::ceil(tiles * pl.splits / slots) / pl.splits, finish = pl.splits > 1 ? finish_us(pl.splits, out) : 0.0;
+    if (pl.tail_ways) {
+        rounds = std::floor(tiles / slots) + std::ceil(pl.tail_tiles * pl.tail_ways / slots) / pl.tail_ways;
+        finish = finish_us(pl.tail_ways, 4.0 * BM * pl.cg * pl.bn * pl.tail_tiles);
+    }
+    const double round_us = half ? k * ns * 1e-3 + (p.fast_tf32 ? 1.0 : 4.5) : std::max(k * ns * 1e-3, pl.bn == 256 ? 3.7 : 1.5);
+    return (half ? 8.0 : 5.0) + rounds * round_us + finish;
+}
+
 std::string gemm_tc_describe(const GemmProblem &p0, int sm_count) {
     bool transposed = false;
     const GemmProblem p = kernel_view(p0, &transposed);
@@ -1973,9 +2225,9 @@ std::string gemm_tc_describe(const GemmProblem &p0, int sm_count) {
     const int pieces = (ci > 0 && len > ci + ci / 8) ? static_cast<int>((len + ci - 1) / ci) : 1;
     char buf[320];
     snprintf(buf, sizeof(buf),
-             "tensor m=%lld n=%lld k=%lld batch=%lld fold=%lld bn=%d bk=%d pair=%d tmem_a=%d stages=%d splits=%d "
+             "%s m=%lld n=%lld k=%lld batch=%lld fold=%lld bn=%d bk=%d pair=%d tmem_a=%d stages=%d splits=%d "
              "tail=%d grid=%d exchanged=%d single_pass=%d pieces=%d mma_n=%d tail_ways=%d running=%d",
-             static_cast<long long>(p.M), static_cast<long long>(p.N), static_cast<long long>(p.K),
+             p.ha ? "halves" : "tensor", static_cast<long long>(p.M), static_cast<long long>(p.N), static_cast<long long>(p.K),
              static_cast<long long>(p.batch), static_cast<long long>(p.fold), pl.bn, pl.bk, pl.cg == 2 ? 1 : 0,
              pl.ta ? 1 : 0, pl.stages, pl.splits, pl.sk || pl.tail_ways ? 1 : 0, pl.grid, transposed ? 1 : 0, p.fast_tf32 ? 1 : 0,
              pieces, mma_n_for(p, pl), pl.tail_ways, pl.running ? 1 : 0);
@@ -2043,13 +2295,14 @@ int launch_gemm_tc(const GemmProblem &p0, float *partial, uint32_t *err_word, in
     CUtensorMap tmA, tmB, tmC, tmD, tmP;
     if (p.D != nullptr && !gemm_tc_can_fuse_activation(p, sm_count))
         return fail(MNI_B200_ERR_ARG, "fused activation requested for a problem that cannot carry it");
-    int rc = make_operand_map(&tmA, p.A, BM, pl.bk, &k.a_mode);
+    const bool half = p.ha != nullptr;
+    int rc = half ? make_half_map(&tmA, *p.ha, &k.a_mode) : make_operand_map(&tmA, p.A, BM, pl.bk, &k.a_mode);
     if (rc) return rc;
     // B rows that exist in a tile wider than the output: with a K-major B (one box of whole rows) only those are
     // loaded, split and multiplied; the shared memory behind them is never read.
     const int mma_n = mma_n_for(p, pl);
     k.b_rows_live = (p.B.k_major && mma_n < pl.bn) ? mma_n : pl.bn / pl.cg;
-    rc = make_operand_map(&tmB, p.B, k.b_rows_live, pl.bk, &k.b_mode);
+    rc = half ? make_half_map(&tmB, *p.hb, &k.b_mode) : make_operand_map(&tmB, p.B, k.b_rows_live, pl.bk, &k.b_mode);
     if (rc) return rc;
 
     // Epilogue: TMA store when the destination rows are 16-byte aligned, plain stores otherwise.
@@ -2142,6 +2395,26 @@ int launch_gemm_tc(const GemmProblem &p0, float *partial, uint32_t *err_word, in
     else { k.a_desc_hi = desc_hi_bits(mn_sbo, mn_layout); k.a_desc_lbo = ((mn_lbo >> 4) & 0x3FFFu) << 16; k.a_kstep = 64; }
     if (p.B.k_major) { k.b_desc_hi = desc_hi_bits(k_sbo, k_layout); k.b_desc_lbo = 0; k.b_kstep = 2; }
     else { k.b_desc_hi = desc_hi_bits(mn_sbo, mn_layout); k.b_desc_lbo = ((mn_lbo >> 4) & 0x3FFFu) << 16; k.b_kstep = 64; }
+    if (half) {
+        // kind::f16: f16 operands, 16-deep k-steps.  K-major rows of 64 elements, one swizzle span (k-step 32 bytes); MN-major chunks
+        // of 64 rows, LBO apart, of 64 k-lines in groups of 8 (k-step two groups).
+        const uint32_t hi = desc_hi_bits(1024, 2), lbo = static_cast<uint32_t>((pl.bk * 128) >> 4) << 16;
+        k.idesc = (1u << 4) | ((p.ha->k_major ? 0u : 1u) << 15) | ((p.hb->k_major ? 0u : 1u) << 16) | (32u << 17) | (16u << 24);
+        k.a_desc_hi = k.b_desc_hi = hi;
+        k.a_desc_lbo = p.ha->k_major ? 0 : lbo;
+        k.b_desc_lbo = p.hb->k_major ? 0 : lbo;
+        k.a_kstep = p.ha->k_major ? 2 : 128;
+        k.b_kstep = p.hb->k_major ? 2 : 128;
+        k.b_rows_live = 128;
+        k.a_batch = static_cast<int>(p.ha->batch); k.a_d1 = 1; k.a_d2 = k.a_batch;
+        k.b_batch = static_cast<int>(p.hb->batch); k.b_d1 = 1; k.b_d2 = k.b_batch;
+        k.fd_a_cnt = make_fastdiv(k.a_batch); k.fd_a_d1 = make_fastdiv(1); k.fd_a_d2 = make_fastdiv(k.a_d2);
+        k.fd_b_cnt = make_fastdiv(k.b_batch); k.fd_b_d1 = make_fastdiv(1); k.fd_b_d2 = make_fastdiv(k.b_d2);
+        k.a_exp = p.ha->exp;
+        k.b_exp = p.hb->exp;
+        k.half_status = p.half_status;
+        k.half_statuses = p.half_statuses;
+    }
     k.C = p.C;
     k.ldc = p.ldc;
     k.c_bstride = p.c_bstride;
@@ -2182,39 +2455,48 @@ int launch_gemm_tc(const GemmProblem &p0, float *partial, uint32_t *err_word, in
     }
     const bool running = pl.running && (k.epi_mode == kEpiTmaStore || k.epi_mode == kEpiTmaReduce);
     cudaError_t e = cudaErrorInvalidValue;
-    if (pl.sk) {
-        if (pl.ta && pl.bn == 64 && split_groups == 2) e = launch_variant<64, 32, false, 8, 1, true, kBalanced, 2>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
-        else if (pl.ta && pl.bn == 64) e = launch_variant<64, 32, false, 8, 1, true, kBalanced>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
-        else if (pl.ta && pl.bn == 128 && split_groups == 2) e = launch_variant<128, 32, false, 8, 1, true, kBalanced, 2>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
-        else if (pl.ta && pl.bn == 128) e = launch_variant<128, 32, false, 8, 1, true, kBalanced>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
-        else if (!p.fast_tf32 && pl.bk == 16) e = launch_variant<256, 16, false, 8, 2, false, kBalanced>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
-        else if (!p.fast_tf32 && pl.bk == 32) e = launch_variant<256, 32, false, 8, 2, false, kBalanced>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
-        else if (pl.bk == 16) e = launch_variant<256, 16, true, 4, 2, false, kBalanced>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
-        else e = launch_variant<256, 32, true, 4, 2, false, kBalanced>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+    if (half) {
+        if (p.fast_tf32) {
+            if (running) e = launch_variant<256, 64, kHalfOne, 4, 2, false, kRunningSum>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+            else if (pl.tail_ways) e = launch_variant<256, 64, kHalfOne, 4, 2, false, kCutTiles>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+            else e = launch_variant<256, 64, kHalfOne, 4, 2>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+        } else {
+            if (pl.tail_ways) e = launch_variant<256, 64, kHalfThree, 2, 2, false, kCutTiles>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+            else e = launch_variant<256, 64, kHalfThree, 2, 2>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+        }
+    } else if (pl.sk) {
+        if (pl.ta && pl.bn == 64 && split_groups == 2) e = launch_variant<64, 32, kThreePass, 8, 1, true, kBalanced, 2>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+        else if (pl.ta && pl.bn == 64) e = launch_variant<64, 32, kThreePass, 8, 1, true, kBalanced>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+        else if (pl.ta && pl.bn == 128 && split_groups == 2) e = launch_variant<128, 32, kThreePass, 8, 1, true, kBalanced, 2>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+        else if (pl.ta && pl.bn == 128) e = launch_variant<128, 32, kThreePass, 8, 1, true, kBalanced>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+        else if (!p.fast_tf32 && pl.bk == 16) e = launch_variant<256, 16, kThreePass, 8, 2, false, kBalanced>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+        else if (!p.fast_tf32 && pl.bk == 32) e = launch_variant<256, 32, kThreePass, 8, 2, false, kBalanced>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+        else if (pl.bk == 16) e = launch_variant<256, 16, kOnePass, 4, 2, false, kBalanced>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+        else e = launch_variant<256, 32, kOnePass, 4, 2, false, kBalanced>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
     } else if (running && p.fast_tf32) {
-        e = launch_variant<256, 32, true, 4, 2, false, kRunningSum>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+        e = launch_variant<256, 32, kOnePass, 4, 2, false, kRunningSum>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
     } else if (running) {
-        e = launch_variant<256, 16, false, 8, 2, false, kRunningSum>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+        e = launch_variant<256, 16, kThreePass, 8, 2, false, kRunningSum>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
     } else if (pl.tail_ways) {
-        if (!p.fast_tf32 && pl.bk == 16) e = launch_variant<256, 16, false, 8, 2, false, kCutTiles>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
-        else if (!p.fast_tf32) e = launch_variant<256, 32, false, 8, 2, false, kCutTiles>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
-        else if (pl.bk == 16) e = launch_variant<256, 16, true, 4, 2, false, kCutTiles>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
-        else e = launch_variant<256, 32, true, 4, 2, false, kCutTiles>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+        if (!p.fast_tf32 && pl.bk == 16) e = launch_variant<256, 16, kThreePass, 8, 2, false, kCutTiles>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+        else if (!p.fast_tf32) e = launch_variant<256, 32, kThreePass, 8, 2, false, kCutTiles>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+        else if (pl.bk == 16) e = launch_variant<256, 16, kOnePass, 4, 2, false, kCutTiles>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+        else e = launch_variant<256, 32, kOnePass, 4, 2, false, kCutTiles>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
     } else if (pl.ta) {
-        if (pl.bn == 64 && split_groups == 2) e = launch_variant<64, 32, false, 8, 1, true, kWholeTiles, 2>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
-        else if (pl.bn == 64) e = launch_variant<64, 32, false, 8, 1, true>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
-        else if (split_groups == 2) e = launch_variant<128, 32, false, 8, 1, true, kWholeTiles, 2>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
-        else e = launch_variant<128, 32, false, 8, 1, true>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+        if (pl.bn == 64 && split_groups == 2) e = launch_variant<64, 32, kThreePass, 8, 1, true, kWholeTiles, 2>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+        else if (pl.bn == 64) e = launch_variant<64, 32, kThreePass, 8, 1, true>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+        else if (split_groups == 2) e = launch_variant<128, 32, kThreePass, 8, 1, true, kWholeTiles, 2>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+        else e = launch_variant<128, 32, kThreePass, 8, 1, true>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
     }
 #define MNI_VARIANT(BN_, BK_)                                                                         \
-    if (pl.cg == 1 && !pl.ta && pl.bn == BN_ && pl.bk == BK_) {                                                 \
-        if (p.fast_tf32) e = launch_variant<BN_, BK_, true, 4, 1>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);      \
-        else e = launch_variant<BN_, BK_, false, 8, 1>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);                 \
+    if (!half && pl.cg == 1 && !pl.ta && pl.bn == BN_ && pl.bk == BK_) {                                                 \
+        if (p.fast_tf32) e = launch_variant<BN_, BK_, kOnePass, 4, 1>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);      \
+        else e = launch_variant<BN_, BK_, kThreePass, 8, 1>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);                 \
     }
 #define MNI_PAIR_VARIANT(BN_, BK_)                                                                    \
-    if (pl.cg == 2 && !pl.sk && !pl.tail_ways && !running && pl.bn == BN_ && pl.bk == BK_) {                                                 \
-        if (p.fast_tf32) e = launch_variant<BN_, BK_, true, 4, 2>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);      \
-        else e = launch_variant<BN_, BK_, false, 8, 2>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);                 \
+    if (!half && pl.cg == 2 && !pl.sk && !pl.tail_ways && !running && pl.bn == BN_ && pl.bk == BK_) {                                                 \
+        if (p.fast_tf32) e = launch_variant<BN_, BK_, kOnePass, 4, 2>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);      \
+        else e = launch_variant<BN_, BK_, kThreePass, 8, 2>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);                 \
     }
     MNI_PAIR_VARIANT(64, 32) MNI_PAIR_VARIANT(128, 32) MNI_PAIR_VARIANT(256, 16) MNI_PAIR_VARIANT(256, 32)
 #undef MNI_PAIR_VARIANT

@@ -1,0 +1,367 @@
+// Operands of large products in 16-bit planes for the f16 tensor pipe, which runs at twice the rate of TF32 and has the same
+// eleven significant bits: x * 2^e = hi + lo * 2^-12 with hi and lo in f16, e chosen for the whole operand.
+//
+// e comes from 1024 sampled elements, so one pass over the operand is enough; the largest sample lands in [2^6, 2^7).  Above it
+// there is room for elements 256 times as large, below it every element of at least 2^-21 of it keeps 22 bits.  What f16 does not
+// hold is found by the same pass and reported in the block's status word; a second kernel then writes three bf16 planes, whose
+// range is that of f32, and the products take those:
+//   - an element beyond 2^15 after scaling, an infinity or a NaN;
+//   - a stretch of a row or of a column (256 elements, 32 elements) that consists of smaller elements than that, zeros aside: in
+//     its row or column of the product the bits they lose would be the leading ones;
+//   - a tile in which more than a sixteenth of the elements are that small.
+#include "internal.h"
+
+#include <cuda_fp16.h>
+
+#include <algorithm>
+
+namespace mni {
+
+namespace {
+
+constexpr int kThreads = 256, kTileRows = 16, kTileCols = 512;     // 64 threads x 8 columns, 4 groups of 4 rows
+constexpr int kBlocksPerSm = 3;
+constexpr float kLargest = 32768.f, kSmallest = 1.f / 32768.f;
+constexpr int kMaxExp = kHalfMaxExp, kTargetExp = 6;
+// Status word of a block: some element, row, column or tile did not fit; some element is beyond 2^30 after scaling.
+constexpr unsigned kUnfit = 1, kHuge = 2;
+
+struct View {
+    const float *src;
+    uint16_t *dst;                      // first plane; the others follow `plane` elements apart
+    long long ld, b0, b1, b2;           // source strides
+    long long matrix, plane;
+    int rows, cols, pitch;
+    FastDiv rows_d, d1, d2;
+    FastDiv tiles_r, tiles_strip;       // tiles of a strip of columns: of one matrix, of all of them
+    int first_tile;
+    unsigned total_rows;
+    int vec;                            // rows are 16-byte aligned
+    int *exp;
+};
+struct ViewList {
+    View v[kMaxHalves];
+    int count, tiles;
+    unsigned int *status;
+    int statuses;                       // = blocks of split_half_kernel
+    HalfColumns sums;                   // of the first view
+};
+
+__device__ __forceinline__ const float *matrix_source(const View &v, int batch) {
+    const int q2 = fd_div(batch, v.d2), q1 = fd_div(q2, v.d1);
+    return v.src + (batch - q2 * static_cast<int>(v.d2.d)) * v.b2 + (q2 - q1 * static_cast<int>(v.d1.d)) * v.b1 + q1 * v.b0;
+}
+struct Tile {
+    int strip, batch, r0, c0;           // r0: first row of the tile, c0: first column of its strip
+};
+__device__ __forceinline__ Tile tile_at(const View &v, int rel) {
+    Tile t;
+    t.strip = fd_div(rel, v.tiles_strip);
+    const int in = rel - t.strip * static_cast<int>(v.tiles_strip.d);
+    t.batch = fd_div(in, v.tiles_r);
+    t.r0 = (in - t.batch * static_cast<int>(v.tiles_r.d)) * kTileRows;
+    t.c0 = t.strip * kTileCols;
+    return t;
+}
+__device__ __forceinline__ int first_tile_of(const ViewList &list, int block) {
+    return static_cast<int>(static_cast<long long>(list.tiles) * block / list.statuses);
+}
+
+// The exponent of the operand's scale, the same in every block that asks.
+__device__ int operand_exponent(const View &v, unsigned *biggest) {
+    unsigned m = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const unsigned s = i * kThreads + threadIdx.x;
+        const int row = static_cast<int>((static_cast<unsigned long long>(s) * v.total_rows) >> 10);
+        unsigned h = (s + 1u) * 0x9E3779B1u;
+        h = (h ^ (h >> 15)) * 0x85EBCA77u;
+        h ^= h >> 13;
+        const int col = static_cast<int>(__umulhi(h, static_cast<unsigned>(v.cols)));
+        const int batch = fd_div(row, v.rows_d);
+        const float x = __ldg(matrix_source(v, batch) + (row - batch * v.rows) * v.ld + col);
+        m = max(m, __float_as_uint(x) & 0x7fffffffu);
+    }
+    m = __reduce_max_sync(0xffffffffu, m);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) biggest[threadIdx.x >> 5] = m;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < kThreads / 32; ++w) m = max(m, biggest[w]);
+    const int field = static_cast<int>(m >> 23);                    // 255: infinity or NaN, which the pass will find
+    return (m == 0 || field == 255) ? 0 : max(-kMaxExp, min(kMaxExp, kTargetExp + 127 - field));
+}
+
+// Bound by memory: 4 bytes read and 4 (LO) or 2 written an element.  A block takes consecutive tiles of a strip of columns, so
+// that what it finds about columns, and their sums (SUMS: of the first view, for the bias gradient), stay in registers until
+// the strip ends.
+template <bool LO, bool SUMS>
+__global__ void __launch_bounds__(kThreads, kBlocksPerSm)
+split_half_kernel(const __grid_constant__ ViewList list) {
+    __shared__ unsigned shared[4][kTileCols], shared_n[4][kTileCols / 4];
+    __shared__ int smalls;
+    grid_dependency_trigger();
+    grid_dependency_wait();
+    const int t0 = first_tile_of(list, blockIdx.x), t1 = first_tile_of(list, blockIdx.x + 1);
+    const int tc = threadIdx.x & 63, group = threadIdx.x >> 6;
+    const unsigned limit = __float_as_uint(kLargest), small = __float_as_uint(kSmallest);
+    unsigned bad = 0, cmax[8], few[2];             // few: small elements of the columns, a byte each
+    float sum[8];
+    int n_small = 0, rows_seen = 0;
+    int j = -1, strip = -1;
+    float scale = 1.f;
+    auto begin_strip = [&] {
+#pragma unroll
+        for (int c = 0; c < 8; ++c) { cmax[c] = 0; if (SUMS) sum[c] = 0.f; }
+        few[0] = few[1] = 0;
+        n_small = rows_seen = 0;
+    };
+    auto end_strip = [&] {
+        if (__syncthreads_or(n_small)) {
+            if (threadIdx.x == 0) smalls = 0;
+#pragma unroll
+            for (int c = 0; c < 8; ++c) shared[group][tc * 8 + c] = cmax[c];
+            shared_n[group][tc * 2] = few[0];
+            shared_n[group][tc * 2 + 1] = few[1];
+            __syncthreads();
+            if (n_small) atomicAdd(&smalls, n_small);
+            for (int c = threadIdx.x; c < kTileCols; c += kThreads) {
+                unsigned m = 0, n = 0;
+#pragma unroll
+                for (int g = 0; g < 4; ++g) {
+                    m = max(m, shared[g][c]);
+                    n += (shared_n[g][c >> 2] >> (8 * (c & 3))) & 255u;
+                }
+                if (n >= 8u && m < small) bad |= kUnfit;
+            }
+            __syncthreads();
+            const int width = min(kTileCols, list.v[j].cols - strip * kTileCols);
+            if (smalls > 16 + rows_seen * width / 16) bad |= kUnfit;
+        }
+        if (SUMS && j == 0) {
+            __syncthreads();
+            float *const mine = reinterpret_cast<float *>(&shared[0][0]);
+#pragma unroll
+            for (int c = 0; c < 8; ++c) mine[group * kTileCols + tc * 8 + c] = sum[c];
+            __syncthreads();
+            float *const out = list.sums.partial + static_cast<long long>(blockIdx.x + strip) * kTileCols;
+            for (int c = threadIdx.x; c < kTileCols; c += kThreads)
+                out[c] = (mine[c] + mine[kTileCols + c]) + (mine[2 * kTileCols + c] + mine[3 * kTileCols + c]);
+            __syncthreads();
+        }
+    };
+    for (int tile = t0; tile < t1; ++tile) {
+        int at = 0;
+        while (at + 1 < list.count && tile >= list.v[at + 1].first_tile) ++at;
+        const View &v = list.v[at];
+        const Tile t = tile_at(v, tile - v.first_tile);
+        const int r0 = t.r0 + group, c0 = t.c0 + tc * 8;
+        const float *src = matrix_source(v, t.batch) + r0 * v.ld + c0;
+        const bool whole = v.vec && c0 + 8 <= v.cols;
+        float x[4][8];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float *row = src + 4 * i * v.ld;
+            if (r0 + 4 * i < v.rows && whole) {
+                const float4 a = __ldg(reinterpret_cast<const float4 *>(row)), b = __ldg(reinterpret_cast<const float4 *>(row) + 1);
+                x[i][0] = a.x; x[i][1] = a.y; x[i][2] = a.z; x[i][3] = a.w;
+                x[i][4] = b.x; x[i][5] = b.y; x[i][6] = b.z; x[i][7] = b.w;
+            } else {
+#pragma unroll
+                for (int c = 0; c < 8; ++c) x[i][c] = (r0 + 4 * i < v.rows && c0 + c < v.cols) ? __ldg(row + c) : 0.f;
+            }
+        }
+        if (at != j || t.strip != strip) {         // the loads above are on their way meanwhile
+            if (j >= 0) end_strip();
+            if (at != j) {
+                const int e = operand_exponent(v, &shared[0][0]);
+                __syncthreads();
+                scale = __uint_as_float(static_cast<unsigned>(127 + e) << 23);
+                if (tile == v.first_tile && threadIdx.x == 0) *v.exp = e;
+            }
+            j = at;
+            strip = t.strip;
+            begin_strip();
+        }
+        rows_seen += min(kTileRows, v.rows - t.r0);
+        uint16_t *dst = v.dst + t.batch * v.matrix + static_cast<long long>(r0) * v.pitch + c0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (r0 + 4 * i >= v.rows) break;       // the same for the whole warp
+            uint4 hi, lo;
+            unsigned *const h = &hi.x, *const l = &lo.x;
+            unsigned big = 0, least = 0xffffffffu;
+#pragma unroll
+            for (int c = 0; c < 8; c += 2) {
+                if (SUMS) { sum[c] += x[i][c]; sum[c + 1] += x[i][c + 1]; }
+                const float a = x[i][c] * scale, b = x[i][c + 1] * scale;
+                const unsigned ua = __float_as_uint(a) & 0x7fffffffu, ub = __float_as_uint(b) & 0x7fffffffu;
+                cmax[c] = max(cmax[c], ua);
+                cmax[c + 1] = max(cmax[c + 1], ub);
+                big = max(big, max(ua, ub));
+                least = min(least, min(ua - 1u, ub - 1u));         // a zero wraps round to the largest
+                const __half2 h2 = __floats2half2_rn(a, b);
+                h[c / 2] = *reinterpret_cast<const unsigned *>(&h2);
+                if (LO) {
+                    const float2 back = __half22float2(h2);
+                    constexpr float up = 1 << kHalfLoShift;
+                    const __half2 l2 = __floats2half2_rn((a - back.x) * up, (b - back.y) * up);
+                    l[c / 2] = *reinterpret_cast<const unsigned *>(&l2);
+                }
+            }
+            if (big > limit) bad |= big > __float_as_uint(1073741824.f) ? kUnfit | kHuge : kUnfit;
+            if (__any_sync(0xffffffffu, least < small - 1u)) {
+                int n = 0;
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    const unsigned u = __float_as_uint(x[i][c] * scale) & 0x7fffffffu;
+                    if (u - 1u < small - 1u) {
+                        ++n;
+                        if (((few[c / 4] >> (8 * (c & 3))) & 255u) < 63u) few[c / 4] += 1u << (8 * (c & 3));
+                    }
+                }
+                n_small += n;
+                if (__reduce_add_sync(0xffffffffu, n) >= 16 && !__any_sync(0xffffffffu, big >= small)) bad |= kUnfit;
+            }
+            if (c0 < v.pitch) {
+                *reinterpret_cast<uint4 *>(dst + static_cast<long long>(4 * i) * v.pitch) = hi;
+                if (LO) *reinterpret_cast<uint4 *>(dst + v.plane + static_cast<long long>(4 * i) * v.pitch) = lo;
+            }
+        }
+    }
+    if (j >= 0) end_strip();
+    bad = (__syncthreads_or(bad & kUnfit) ? kUnfit : 0u) | (__syncthreads_or(bad & kHuge) ? kHuge : 0u);
+    if (threadIdx.x == 0) list.status[blockIdx.x] = bad;
+}
+
+// Finishes the column sums.  And if the pass above found an operand that f16 does not hold: all of them again, as sums of three
+// (or two) bf16, whose range is that of f32.  half_wide_exponent has their scale.
+template <int PLANES>
+__global__ void __launch_bounds__(kThreads)
+split_wide_kernel(const __grid_constant__ ViewList list) {
+    __shared__ float part[8][32];
+    grid_dependency_trigger();
+    grid_dependency_wait();
+    unsigned status = 0;
+    for (int i = threadIdx.x; i < list.statuses; i += kThreads) status |= __ldcg(list.status + i);
+    const HalfColumns &sums = list.sums;
+    if (sums.out) {
+        const View &v = list.v[0];
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, per_strip = static_cast<int>(v.tiles_strip.d);
+        for (int c32 = blockIdx.x * 32; c32 < v.cols; c32 += gridDim.x * 32) {
+            // the blocks that took tiles of this strip
+            const int strip = c32 / kTileCols, first = strip * per_strip, last = first + per_strip - 1;
+            int b0 = static_cast<int>(static_cast<long long>(first) * list.statuses / list.tiles);
+            while (b0 > 0 && first_tile_of(list, b0) > first) --b0;
+            while (first_tile_of(list, b0 + 1) <= first) ++b0;
+            int b1 = static_cast<int>(static_cast<long long>(last) * list.statuses / list.tiles);
+            while (b1 > 0 && first_tile_of(list, b1) > last) --b1;
+            while (first_tile_of(list, b1 + 1) <= last) ++b1;
+            float s = 0.f;
+            for (int b = b0 + warp; b <= b1; b += 8)
+                s += __ldcg(sums.partial + static_cast<long long>(b + strip) * kTileCols + (c32 % kTileCols) + lane);
+            part[warp][lane] = s;
+            __syncthreads();
+            if (warp == 0 && c32 + lane < v.cols) {
+#pragma unroll
+                for (int w = 1; w < 8; ++w) s += part[w][lane];
+                sums.out[c32 + lane] = sums.accumulate ? sums.out[c32 + lane] + s : s;
+            }
+            __syncthreads();
+        }
+    }
+    if (!__syncthreads_or(status & kUnfit)) return;
+    const bool huge = __syncthreads_or(status & kHuge);
+    for (int tile = blockIdx.x; tile < list.tiles; tile += gridDim.x) {
+        int at = 0;
+        while (at + 1 < list.count && tile >= list.v[at + 1].first_tile) ++at;
+        const View &v = list.v[at];
+        const Tile t = tile_at(v, tile - v.first_tile);
+        const int c0 = t.c0 + (threadIdx.x & 63) * 8;
+        const float scale = __uint_as_float(static_cast<unsigned>(127 + half_wide_exponent(__ldcg(v.exp), huge)) << 23);
+        if (c0 >= v.pitch) continue;
+        for (int r = t.r0 + (threadIdx.x >> 6); r < min(v.rows, t.r0 + kTileRows); r += 4) {
+            const float *src = matrix_source(v, t.batch) + r * v.ld + c0;
+            uint16_t *dst = v.dst + t.batch * v.matrix + static_cast<long long>(r) * v.pitch + c0;
+            float x[8];
+#pragma unroll
+            for (int c = 0; c < 8; ++c) x[c] = c0 + c < v.cols ? __ldg(src + c) * scale : 0.f;
+#pragma unroll
+            for (int plane = 0; plane < PLANES; ++plane) {
+                uint4 out;
+                unsigned *const o = &out.x;
+#pragma unroll
+                for (int c = 0; c < 8; c += 2) {
+                    // cut, not rounded, so that the largest f32 does not become infinite
+                    const unsigned a = __float_as_uint(x[c]) & 0xffff0000u, b = __float_as_uint(x[c + 1]) & 0xffff0000u;
+                    o[c / 2] = (a >> 16) | b;
+                    x[c] -= __uint_as_float(a);
+                    x[c + 1] -= __uint_as_float(b);
+                }
+                *reinterpret_cast<uint4 *>(dst + plane * v.plane) = out;
+            }
+        }
+    }
+}
+
+long long strips_of(const HalfView &v) { return (v.pitch + kTileCols - 1) / kTileCols; }
+long long tiles_of(const HalfView &v) { return v.batch * ((v.rows + kTileRows - 1) / kTileRows) * strips_of(v); }
+
+}  // namespace
+
+size_t half_columns_bytes(const HalfView &first, int blocks) {
+    return static_cast<size_t>(blocks + strips_of(first)) * kTileCols * sizeof(float);
+}
+
+int half_blocks(const HalfView *views, int count, int sm_count) {
+    long long tiles = 0;
+    for (int i = 0; i < count; ++i) tiles += tiles_of(views[i]);
+    return static_cast<int>(std::min<long long>(tiles, static_cast<long long>(sm_count) * kBlocksPerSm));
+}
+
+int launch_split_half(const HalfView *views, int count, int planes, unsigned int *status, int blocks, const HalfColumns &sums,
+                      cudaStream_t stream) {
+    ViewList list{};
+    list.count = count;
+    list.status = status;
+    list.statuses = blocks;
+    list.sums = sums;
+    long long tiles = 0;
+    for (int i = 0; i < count; ++i) {
+        const HalfView &h = views[i];
+        View &v = list.v[i];
+        v.src = h.src;
+        v.dst = static_cast<uint16_t *>(h.dst);
+        v.ld = h.ld;
+        v.b0 = h.bstride[0]; v.b1 = h.bstride[1]; v.b2 = h.bstride[2];
+        v.matrix = h.matrix;
+        v.plane = h.plane;
+        v.rows = static_cast<int>(h.rows);
+        v.cols = static_cast<int>(h.cols);
+        v.pitch = static_cast<int>(h.pitch);
+        v.rows_d = make_fastdiv(h.rows);
+        v.d1 = make_fastdiv(h.bshape[1]);
+        v.d2 = make_fastdiv(h.bshape[2]);
+        v.tiles_r = make_fastdiv((h.rows + kTileRows - 1) / kTileRows);
+        v.tiles_strip = make_fastdiv(h.batch * ((h.rows + kTileRows - 1) / kTileRows));
+        v.first_tile = static_cast<int>(tiles);
+        v.total_rows = static_cast<unsigned>(h.batch * h.rows);
+        v.vec = (reinterpret_cast<uintptr_t>(h.src) & 15) == 0 && h.ld % 4 == 0 && h.bstride[0] % 4 == 0 && h.bstride[1] % 4 == 0 &&
+                h.bstride[2] % 4 == 0;
+        v.exp = h.exp;
+        tiles += tiles_of(h);
+    }
+    list.tiles = static_cast<int>(tiles);
+    const dim3 grid(static_cast<unsigned>(blocks));
+    const auto split = planes == 3 ? (sums.out ? split_half_kernel<true, true> : split_half_kernel<true, false>)
+                                   : (sums.out ? split_half_kernel<false, true> : split_half_kernel<false, false>);
+    cudaError_t e = launch_dependent(split, grid, dim3(kThreads), 0, stream, list);
+    if (e != cudaSuccess) return fail(MNI_B200_ERR_CUDA, "split_half_kernel launch failed: %s", cudaGetErrorString(e));
+    MNI_LAUNCH_CHECK("split_half_kernel");
+    e = launch_dependent(planes == 3 ? split_wide_kernel<3> : split_wide_kernel<2>, grid, dim3(kThreads), 0, stream, list);
+    if (e != cudaSuccess) return fail(MNI_B200_ERR_CUDA, "split_wide_kernel launch failed: %s", cudaGetErrorString(e));
+    MNI_LAUNCH_CHECK("split_wide_kernel");
+    return MNI_B200_OK;
+}
+
+}  // namespace mni

@@ -126,6 +126,24 @@ struct Operand {
     int64_t batch = 1;             // product of bshape
 };
 
+// An operand in 16-bit planes (half.cu), each [batch][rows or k][pitch], and the exponent its values were multiplied by.
+struct HalfOperand {
+    const void *ptr = nullptr;
+    bool k_major = true;
+    int64_t rows = 0, kdim = 0, pitch = 0;
+    int64_t matrix = 0, plane = 0;   // elements of one matrix, of one plane
+    int64_t batch = 1;
+    int planes = 3;                  // that there is room for
+    const int *exp = nullptr;
+};
+// lo = (x - hi) * 2^kHalfLoShift: the whole range of f16 serves the part below hi's last bit
+constexpr int kHalfLoShift = 12;
+// f16 planes: exponents lie within this either way.
+constexpr int kHalfMaxExp = 60;
+// The exponent of bf16 planes, from that of f16 ones.  Numbers so small that their parts would run into bf16's smallest are
+// scaled, unless the operand holds some that are not (huge); scaled ones stay below 1, so that no product overflows by it.
+__host__ __device__ inline int half_wide_exponent(int e, bool huge) { return e == kHalfMaxExp && !huge ? 24 : 0; }
+
 struct GemmProblem {
     Operand A, B;                  // C[M,N] = sum_k A[m,k] * B[n,k]
     int64_t M = 0, N = 0, K = 0;
@@ -147,6 +165,10 @@ struct GemmProblem {
     int flag_bank = 0;             // 1 for launches on the library's side stream: their own set of balanced-tail flags
     // Optional second output D = gelu(C + bias) written by the same epilogue (C itself is skipped if null).
     float *D = nullptr;
+    // The operands in 16-bit planes (A and B are not read then) and the status words of the kernel that made them.
+    const HalfOperand *ha = nullptr, *hb = nullptr;
+    const unsigned int *half_status = nullptr;
+    int half_statuses = 0;
 };
 
 // Bytes of split-K partial storage launch_gemm_tc would use for this problem (0 if none).
@@ -163,6 +185,8 @@ int launch_gemm_tc(const GemmProblem &p, float *partial, uint32_t *err_word, int
 bool gemm_tc_uses_pairs(const GemmProblem &p, int sm_count);
 // The plan's cost model for this problem in microseconds (0: the model does not cover it).
 double gemm_tc_estimate_us(const GemmProblem &p, int sm_count);
+// Microseconds of a product: from f32 operands, or from 16-bit planes of them (without the pass that makes those).
+double gemm_estimate_us(const GemmProblem &p, bool half, int sm_count);
 // One line of text naming the kernel variant, tiling, split and grid launch_gemm_tc would use for this problem
 // on a device with `sm_count` SMs.  Pure host arithmetic: touches no device.
 std::string gemm_tc_describe(const GemmProblem &p, int sm_count);
@@ -262,6 +286,26 @@ struct GatherView {
 };
 constexpr int kMaxGathers = 3;
 int launch_gather(const GatherView *views, int count, cudaStream_t stream);
+// Matrices to be made into 16-bit planes (half.cu): `batch` of them, rows x cols, unit stride along cols.
+struct HalfView {
+    const float *src;
+    int64_t bshape[3], bstride[3], batch;
+    int64_t rows, cols, ld;
+    void *dst;                     // the planes, rows of `pitch` elements (a multiple of 64)
+    int64_t pitch, matrix, plane;
+    int *exp;                      // on the device: the exponent the values were multiplied by
+};
+constexpr int kMaxHalves = 3;
+int half_blocks(const HalfView *views, int count, int sm_count);      // blocks of the first launch, and its status words
+// Column sums of the first view's rows, for the bias gradient (out null: none).
+struct HalfColumns {
+    float *partial = nullptr, *out = nullptr;
+    int accumulate = 0;
+};
+size_t half_columns_bytes(const HalfView &first, int blocks);
+// planes: 3, for products in full precision (f16 hi and lo, or three bf16), or 2, for single-pass ones (f16 hi, or two bf16)
+int launch_split_half(const HalfView *views, int count, int planes, unsigned int *status, int blocks, const HalfColumns &sums,
+                      cudaStream_t stream);
 // device-side utils::unbroadcast: out[orig] (+)= sum over broadcast dims of grad[gshape]
 int launch_unbroadcast(const float *grad, const int64_t *gshape, int gnd, const int64_t *oshape, int ond,
                        float *out, bool accumulate, cudaStream_t stream);

@@ -74,7 +74,7 @@ typedef enum mni_b200_status {
 
 /* flags (OR together) */
 #define MNI_B200_PRECISION_3XTF32   0u        /* default: hi/lo split, 3 tensor-core passes, ~f32 accuracy  */
-#define MNI_B200_PRECISION_TF32     (1u << 0) /* fast mode: one TF32 pass                                   */
+#define MNI_B200_PRECISION_TF32     (1u << 0) /* fast mode: one pass over operands of 11 significant bits   */
 #define MNI_B200_ACCUMULATE_C       (1u << 1) /* fwd: c  += a.b (+bias)   instead of overwrite              */
 #define MNI_B200_ACCUMULATE_DA      (1u << 2) /* bwd: da += ...                                             */
 #define MNI_B200_ACCUMULATE_DB      (1u << 3) /* bwd: db += ...                                             */
@@ -262,12 +262,18 @@ MNI_B200_API int mni_b200_contiguous(const mni_b200_view *src, float *dst, void 
  *
  * CUDA graphs.  Every call may be recorded by a capturing stream (the side stream
  * is forked and joined with events, which capture follows).  The recorded nodes
- * hold the scratch address of the moment: a library-owned buffer that grows later
- * is freed and leaves such a graph with a dangling address, and it cannot grow
- * during a capture at all (the call then fails with MNI_B200_ERR_WORKSPACE and
- * records nothing).  A caller that replays graphs hands the library a buffer of
- * the queried size with mni_b200_workspace_set and keeps it for the graph's life,
- * or runs each captured call once beforehand and makes no larger call afterwards.
+ * hold the scratch address of the moment; a library-owned buffer that is outgrown
+ * later is kept for them until mni_b200_release.  It cannot grow during a capture
+ * (the call then fails with MNI_B200_ERR_WORKSPACE and records nothing): a caller
+ * that replays graphs hands the library a buffer of the queried size with
+ * mni_b200_workspace_set and keeps it for the graph's life, or runs each captured
+ * call once beforehand.
+ *
+ * Large products are computed from 16-bit planes of their operands in scratch, 6
+ * bytes an operand element (4 with MNI_B200_PRECISION_TF32).  Where that cannot be
+ * had -- a smaller buffer was given, no memory is left, a capture may not grow it --
+ * the call computes them from the f32 operands instead, which needs what it did
+ * before and takes longer; it does not fail for it.
  */
 MNI_B200_API int mni_b200_workspace_set(void *ptr, size_t bytes);
 MNI_B200_API int mni_b200_workspace_query(const mni_b200_view *a, const mni_b200_view *b, uint32_t flags,
@@ -315,7 +321,7 @@ MNI_B200_API int mni_b200_role_wait_cycles(uint64_t out[8], int reset);
 /* Number of kernels this library has launched in this process (all threads). */
 MNI_B200_API uint64_t mni_b200_launch_count(void);
 
-/* Releases the library-owned scratch of the current device (synchronises it). */
+/* Releases the library-owned scratch of the current device (synchronises it), that of graphs recorded so far included. */
 MNI_B200_API int mni_b200_release(void);
 
 #ifdef __cplusplus

@@ -1,0 +1,186 @@
+"""GPU: large products from 16-bit planes of their operands (half.cu and the f16 variants of the tensor-core kernel).
+
+MNI_B200_HALF=1 takes every product there that can go, so that the edges of tiles, of k-blocks and of pieces are reached at small
+sizes.  Reference: float64.  Bounds: hi and lo keep 22 bits of each operand and the dropped lo x lo is 2^-24, together below 4e-7
+of a product's norm; the f32 accumulate of the f16 pipe loses up to 0.75e-9 per element of a chain of at most 4608 (measured, K =
+4096: 3.1e-6).  Three bf16 planes keep 24 bits.  In single-pass mode f16 rounds to 11 bits: 2^-12 at most, per operand."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from conftest import Guarded, rel_fro
+
+pytestmark = pytest.mark.gpu
+
+
+def _bound(k, single=False):
+    return 6e-4 if single else 5e-7 + 1e-9 * min(k, 4608)
+
+
+@pytest.fixture
+def planes(monkeypatch):
+    monkeypatch.setenv("MNI_B200_HALF", "1")
+
+
+SHAPES = [
+    # m, k, n, batch, weight shared
+    (256, 192, 256, (), False),           # whole tiles
+    (129, 130, 131, (), False),           # a little more than a block in every dimension
+    (500, 333, 777, (), False),           # nothing aligned
+    (384, 4160, 512, (), False),          # a unit of just more than a chain
+    (300, 9300, 260, (), False),          # split contraction, several pieces a unit
+    (2560, 5000, 2560, (), False),        # many tiles of two pieces
+    (2048, 416, 3072, (), False),         # a last wave cut into units
+    (300, 200, 260, (5,), False),
+    (256, 192, 320, (2, 3), True),        # the weight gradient sums over the batch
+]
+
+
+@pytest.mark.parametrize("m,k,n,batch,shared,bt", [s + (bt,) for s in SHAPES for bt in (False, True) if not bt or s[0] * s[2] < 4e6])
+@pytest.mark.parametrize("single", [False, True])
+def test_forward_and_gradients(F, planes, m, k, n, batch, shared, bt, single):
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(m + k + n)
+    def normal(*s):
+        return torch.randn(s, generator=gen, device="cuda")
+    wb = () if shared else batch
+    x, w, dy, bias = normal(*batch, m, k), normal(*wb, *((n, k) if bt else (k, n))), normal(*batch, m, n), normal(n)
+    wv = w.transpose(-1, -2) if bt else w
+    t = F.DeviceTensor.from_torch
+    dw_view = t(w).permute(tuple(range(len(wb))) + (len(wb) + 1, len(wb))) if bt else t(w)
+    flags = F._lib.PRECISION_TF32 if single else 0
+    y = Guarded(F, batch + (m, n), init=np.ones(batch + (m, n), np.float32))
+    F.matmul(t(x), dw_view, t(bias), out=y.tensor, flags=flags | F._lib.ACCUMULATE_C)
+    da, db, dbias = Guarded(F, batch + (m, k)), Guarded(F, wb + (k, n)), Guarded(F, (n,))
+    F.matmul_backward(t(dy), t(x), dw_view, want_dbias=True, da=da.tensor, db=db.tensor, dbias=dbias.tensor, flags=flags)
+    F.device_status()
+    product = x.double() @ wv.double()
+    want = {"y": product + bias.double() + 1, "da": dy.double() @ wv.double().transpose(-1, -2),
+            "db": x.double().transpose(-1, -2) @ dy.double(), "dbias": dy.double().reshape(-1, n).sum(0)}
+    if shared:
+        want["db"] = want["db"].sum(tuple(range(len(batch))))
+    fold = int(np.prod(batch)) if shared else 1
+    for got, name, length in ((y, "y", k), (da, "da", n), (db, "db", m * fold), (dbias, "dbias", 0)):
+        got.check(name, fully_written=name != "y")
+        assert rel_fro(got.tensor.numpy(), want[name].cpu().numpy()) <= (1e-6 if name == "dbias" else _bound(length, single)), name
+
+
+@pytest.mark.parametrize("n,misalign,want_pre", [(512, 0, True), (512, 0, False), (500, 0, True), (501, 1, True)])
+def test_gelu_epilogue_and_unaligned_outputs(F, planes, n, misalign, want_pre):
+    rng = np.random.default_rng(n)
+    a, w, bias = (rng.standard_normal(s).astype(np.float32) for s in ((600, 300), (300, n), (n,)))
+    w /= np.sqrt(np.float32(300))
+    t = F.DeviceTensor.from_numpy
+    pre, out = F.matmul_bias_gelu(t(a), t(w), t(bias), want_pre=want_pre)
+    plain = Guarded(F, (600, n), misalign=misalign)
+    F.matmul(t(a), t(w), t(bias), out=plain.tensor)
+    F.device_status()
+    want = a.astype(np.float64) @ w
+    plain.check("product")
+    assert rel_fro(plain.tensor.numpy(), want + bias) <= _bound(300)
+    v = want + bias
+    assert rel_fro(out.numpy(), 0.5 * v * (1 + np.tanh(0.7978845608028654 * (v + 0.044715 * v ** 3)))) <= _bound(300)
+    assert (pre is not None) == want_pre and (pre is None or rel_fro(pre.numpy(), want) <= _bound(300))
+
+
+def _ranges():
+    rng = np.random.default_rng(1)
+    m, k, n = 300, 512, 272
+    x, w = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((k, n)).astype(np.float32)
+    def put(a, at, v):
+        a = a.copy()
+        a[at] = v
+        return a
+    spread = np.logspace(-12, 0, k).astype(np.float32)
+    few = np.logspace(-4, 0, k).astype(np.float32)
+    eye = np.eye(k, n, dtype=np.float32)
+    return {
+        "small": (x * np.float32(1e-30), w), "large": (x * np.float32(1e30), w * np.float32(1e-20)),
+        "subnormal": (x * np.float32(1e-39), w), "largest": (np.full((m, k), 3.4e38, np.float32), eye),
+        "row": (put(x, 5, x[5] * np.float32(1e-12)), w), "column": (x, put(w, (slice(None), 7), w[:, 7] * np.float32(1e-12))),
+        "contraction": (x * spread, w / spread[:, None]), "contraction within range": (x * few, w / few[:, None]),
+        "outlier": (put(x, (3, 4), 1e8), w), "zeros": (x * 0, w), "zero rows": (put(x, slice(10, 200), 0), w),
+        "exponents": (np.sign(x) * np.exp2(-40 * rng.random((m, k))).astype(np.float32), eye),
+        "infinity": (put(x, (3, 4), np.inf), w), "nan": (x, put(w, (3, 4), np.nan)),
+    }
+
+
+@pytest.mark.parametrize("name", list(_ranges()))
+@pytest.mark.parametrize("single", [False, True])
+def test_any_range_of_values(F, planes, monkeypatch, name, single):
+    """Row by row and column by column: what f16 does not hold goes through bf16 planes, and nothing loses its leading bits."""
+    x, w = _ranges()[name]
+    t = F.DeviceTensor.from_numpy
+    flags = F._lib.PRECISION_TF32 if single else 0
+    got = F.matmul(t(x), t(w), flags=flags).numpy()
+    F.device_status()
+    monkeypatch.setenv("MNI_B200_HALF", "0")
+    general = F.matmul(t(x), t(w), flags=flags).numpy()
+    finite = np.isfinite(general)
+    assert np.array_equal(finite, np.isfinite(got))
+    if not finite.all():
+        return
+    want = x.astype(np.float64) @ w.astype(np.float64)
+    for axis in (0, 1):
+        error = np.sqrt(((got - want) ** 2).sum(axis))
+        assert (error <= (1e-3 if single else 2e-6) * np.sqrt((want ** 2).sum(axis))).all(), axis
+
+
+def test_without_scratch_for_the_planes_the_product_comes_from_f32(F, planes, monkeypatch):
+    """A buffer that the general path fits in and the planes do not, and a capture that may not grow the library's own."""
+    import torch
+    rng = np.random.default_rng(9)
+    a, b, g = (rng.standard_normal(s).astype(np.float32) for s in ((512, 512), (512, 512), (512, 512)))
+    t = F.DeviceTensor.from_numpy
+    ad, bd, gd = t(a), t(b), t(g)
+    want = {"y": a.astype(np.float64) @ b, "da": g.astype(np.float64) @ b.T, "db": a.T.astype(np.float64) @ g}
+    lib, general = F._lib.lib(), 32 << 20
+    buf = torch.empty(general + 256, dtype=torch.uint8, device="cuda")
+    small = t(rng.standard_normal((4096, 4096)).astype(np.float32))
+    F._lib.check(lib.mni_b200_workspace_set(C.c_void_p((buf.data_ptr() + 255) // 256 * 256), general))
+    try:
+        y, (da, db) = F.matmul(ad, bd), F.matmul_backward(gd, ad, bd)
+        launches = F.launch_count()
+        F.matmul(small, small)                       # its planes need 200 MB
+        assert F.launch_count() - launches <= 2      # the product and a finish
+        F.device_status()
+    finally:
+        F._lib.check(lib.mni_b200_workspace_set(None, 0))
+    for got, name in ((y, "y"), (da, "da"), (db, "db")):
+        assert rel_fro(got.numpy(), want[name]) <= 5e-6, name
+    F._lib.check(lib.mni_b200_release())
+    monkeypatch.setenv("MNI_B200_HALF", "0")
+    F.matmul(small, small)                           # scratch for this, eagerly
+    monkeypatch.setenv("MNI_B200_HALF", "1")
+    out, stream = F.DeviceTensor.empty((4096, 4096)), torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            F.matmul(small, small, out=out)
+    F.matmul(small, small)                           # its planes make the library's scratch grow: the graph keeps its own
+    out.torch_view().zero_()
+    graph.replay()
+    F.device_status()
+    s = small.torch_view().double()
+    assert float((out.torch_view().double() - s @ s).norm() / (s @ s).norm()) <= 2e-5
+
+
+def test_queried_scratch_holds_the_planes(F, planes):
+    import torch
+    rng = np.random.default_rng(4)
+    a, b, g = (F.DeviceTensor.from_numpy(rng.standard_normal(s).astype(np.float32)) for s in ((700, 333), (333, 500), (700, 500)))
+    lib, need = F._lib.lib(), C.c_size_t(0)
+    F._lib.check(lib.mni_b200_workspace_query(a.view_struct(), b.view_struct(), 0, C.byref(need)))
+    buf = torch.full((need.value + 4352,), 0x5A, dtype=torch.uint8, device="cuda")
+    base = (buf.data_ptr() + 255) // 256 * 256
+    F._lib.check(lib.mni_b200_workspace_set(C.c_void_p(base), need.value))
+    try:
+        before = F.launch_count()
+        F.matmul(a, b)
+        assert F.launch_count() - before >= 3         # the passes over the operands, the product
+        F.matmul_backward(g, a, b, want_dbias=True)
+        F.device_status()
+    finally:
+        F._lib.check(lib.mni_b200_workspace_set(None, 0))
+    assert bool((buf[base - buf.data_ptr() + need.value:] == 0x5A).all())
