@@ -45,11 +45,17 @@ __device__ __forceinline__ float4 unit_grad(const float4 &g, const float4 &s, fl
     return make_float4(s.x * (g.x - dot), s.y * (g.y - dot), s.z * (g.z - dot), s.w * (g.w - dot));
 }
 
+// The row of this warp.  From the last one down: what the kernel before wrote last is what L2 still holds (scores of 100 MB
+// between their product, this pass and the next product: attention 288 -> 277 us a pass, the forward's share 7, the backward's 5).
+__device__ __forceinline__ long long last_rows_first() {
+    return (gridDim.x - 1 - blockIdx.x) * static_cast<long long>(kRowsPerBlock) + (threadIdx.x >> 5);
+}
+
 template <typename V, int CH>
 __global__ void __launch_bounds__(kRowsPerBlock * 32)
 softmax_rows_fwd_kernel(const V *__restrict__ x, V *__restrict__ out, long long rows, int len) {
     grid_dependency_trigger();
-    const long long row = blockIdx.x * static_cast<long long>(kRowsPerBlock) + (threadIdx.x >> 5);
+    const long long row = last_rows_first();
     const int lane = threadIdx.x & 31;
     grid_dependency_wait();
     if (row >= rows) return;
@@ -82,7 +88,7 @@ template <typename V, int CH>
 __global__ void __launch_bounds__(kRowsPerBlock * 32)
 softmax_rows_bwd_kernel(const V *__restrict__ dy, const V *__restrict__ out, V *__restrict__ dx, long long rows, int len) {
     grid_dependency_trigger();
-    const long long row = blockIdx.x * static_cast<long long>(kRowsPerBlock) + (threadIdx.x >> 5);
+    const long long row = last_rows_first();
     const int lane = threadIdx.x & 31;
     grid_dependency_wait();
     if (row >= rows) return;
