@@ -499,14 +499,16 @@ bool half_possible(const Call &c, double work) {
 }
 // Whether it pays: `f32_us` the estimate for the products from f32 operands, `half_us` from 16-bit planes, which the pass over the
 // operands' `elements` comes on top of (8 bytes an element, 6 in single-pass mode, at 5.2 TB/s, and 7 us for its two launches).
-// Measured with and without, us, sustained: forward 2048 x 768 x 3072 55 / 62, 2048^3 65 / 62, 8192 x 768 x 3072 143 / 125,
-// 4096 x 1024 x 4096 137 / 114, 4096^3 480 / 338, 1024 x 8192 x 1024 70 / 90, 8192 x 8192 x 512 291 / 308; single pass 3072^3
-// 80 / 82, 4096^3 218 / 178.  MNI_B200_HALF=0 / 1: never / wherever it can be done.
+// Measured with f32 operands / 16-bit planes, us, in a loop: forward 2048 x 768 x 3072 56 / 63, 2048^3 67 / 68, 8192 x 768 x 3072
+// 142 / 131, 4096 x 1024 x 4096 133 / 110, 4096^3 516 / 339, 1024 x 8192 x 1024 70 / 83, 8192 x 8192 x 512 252 / 282; backward
+// 2048 x 768 x 3072 113 / 107, 2048^3 133 / 107, 8192 x 768 x 3072 322 / 242, 4096^3 1071 / 612, 512 x 4096 x 4096 144 / 147;
+// single pass forward 3072^3 79 / 80, 4096^3 219 / 159, backward 162 / 128, 440 / 258.  MNI_B200_HALF=0 / 1: never / wherever it
+// can be done.
 bool half_pays(const Call &c, double f32_us, double half_us, double elements) {
     const int env = env_int("MNI_B200_HALF", -1);
     if (env >= 0) return env > 0;
-    const double bytes = (c.flags & MNI_B200_PRECISION_TF32) != 0 ? 6.0 : 8.0;
-    return half_us + 7.0 + bytes * elements / 5.2e6 < 0.95 * f32_us;
+    const bool single = (c.flags & MNI_B200_PRECISION_TF32) != 0;
+    return half_us + 7.0 + (single ? 6.0 : 8.0) * elements / 5.2e6 < (single ? 0.92 : 0.96) * f32_us;
 }
 // Gathering an operand that TMA cannot describe, in microseconds.
 double gather_us(const mni_b200_view &v) {
@@ -539,13 +541,32 @@ int make_halves(Call &c, std::initializer_list<const mni_b200_view *> views, Hal
     return launch_split_half(h.view, h.count, h.planes, h.status, h.blocks, sums, c.stream);
 }
 
-// The product `p` from operands `a` and `b`; p.C and the rest as for the general path.
-int run_halves(Call &c, GemmProblem p, const Halves &h, const HalfOperand &a, const HalfOperand &b) {
-    p.ha = &a;
-    p.hb = &b;
-    p.half_status = h.status;
-    p.half_statuses = h.blocks;
-    return run_gemm(c, p);
+// One or two products, p[i] of operands x[i] and y[i], in one launch.
+int run_halves(Call &c, GemmProblem *p, int count, const Halves &h, const HalfOperand *x, const HalfOperand *y, const char *const *labels) {
+    for (int i = 0; i < count; ++i) {
+        p[i].ha = &x[i];
+        p[i].hb = &y[i];
+        p[i].half_status = h.status;
+        p[i].half_statuses = h.blocks;
+        p[i].fast_tf32 = (c.flags & MNI_B200_PRECISION_TF32) != 0;
+    }
+    size_t bytes[2] = {0, 0};
+    float *partial[2] = {nullptr, nullptr};
+    gemm_halves_partial_bytes(p, count, c.gemm_sms(), bytes);
+    for (int i = 0; i < count; ++i) {
+        const size_t at = bytes[i] ? c.arena.reserve(bytes[i]) : 0;
+        if (bytes[i] && !c.dry()) partial[i] = c.at(at);
+    }
+    if (c.plan_log) {
+        std::string lines[2];
+        gemm_halves_describe(p, count, c.gemm_sms(), lines);
+        for (int i = 0; i < count; ++i) {
+            if (labels) c.label = labels[i];
+            c.note(lines[i]);
+        }
+    }
+    if (c.dry()) return MNI_B200_OK;
+    return launch_gemm_halves(p, count, partial, c.st->err_word, c.gemm_sms(), c.stream);
 }
 
 int zero_or_bias_fill(Call &c, float *out, int64_t rows, int64_t n, const float *bias, bool accumulate) {
@@ -644,7 +665,7 @@ int forward_product(Call &c, const Shapes &s, const mni_b200_view *a, const mni_
                 view_to_half(*a, probe, &swapped) && view_to_half(*b, probe, &swapped);
     if (half) {
         p.fast_tf32 = (c.flags & MNI_B200_PRECISION_TF32) != 0;
-        half = half_pays(c, gemm_estimate_us(p, false, c.gemm_sms()) + gather_us(*a) + gather_us(*b), gemm_estimate_us(p, true, c.gemm_sms()),
+        half = half_pays(c, gemm_estimate_us(p, c.gemm_sms()) + gather_us(*a) + gather_us(*b), gemm_halves_estimate_us(&p, 1, c.gemm_sms()),
                          static_cast<double>(s.a_batch) * s.M * s.K + static_cast<double>(s.b_batch) * s.K * s.N);
     }
     const mni_b200_view *const a_given = a, *const b_given = b;
@@ -667,7 +688,7 @@ int forward_product(Call &c, const Shapes &s, const mni_b200_view *a, const mni_
     rc = make_halves(c, {a_given, b_given}, h);
     if (rc) return rc;
     const HalfOperand x = h.operand(0, false), y = h.operand(1, true);
-    return run_halves(c, p, h, x, y);
+    return run_halves(c, &p, 1, h, &x, &y, nullptr);
 }
 
 int fwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, float *out, const float *bias) {
@@ -790,10 +811,8 @@ bool single_product(const int64_t *ob, int onb, const mni_b200_view &target, boo
 
 // One gradient: G[ob.., R, Cn] = X . Y (a GEMM over `kdim`) reduced to `target`'s shape.
 //   X supplies the rows, Y the columns; both already as Operands with flat batch counts.
-//   h != null: from these halves instead.
 int grad_gemm(Call &c, Operand X, Operand Y, int64_t R, int64_t Cn, int64_t kdim, const int64_t *ob, int onb,
-              const mni_b200_view &target, float *out, bool accumulate, const Halves *h = nullptr, const HalfOperand *hx = nullptr,
-              const HalfOperand *hy = nullptr) {
+              const mni_b200_view &target, float *out, bool accumulate) {
     const int64_t obatch = prod(ob, onb);
     const int64_t tbatch = prod(target.shape, target.ndim - 2);
     bool same = false;
@@ -805,13 +824,13 @@ int grad_gemm(Call &c, Operand X, Operand Y, int64_t R, int64_t Cn, int64_t kdim
     if (same || obatch == 1) {
         p.batch = obatch; p.fold = 1;
         p.C = out; p.ldc = Cn; p.c_bstride = R * Cn; p.accumulate = accumulate;
-        return h ? run_halves(c, p, *h, *hx, *hy) : run_gemm(c, p);
+        return run_gemm(c, p);
     }
     if (tbatch == 1) {
         // The operand was broadcast over every batch: sum the batches inside the contraction.
         p.batch = 1; p.fold = obatch;
         p.C = out; p.ldc = Cn; p.c_bstride = R * Cn; p.accumulate = accumulate;
-        return h ? run_halves(c, p, *h, *hx, *hy) : run_gemm(c, p);
+        return run_gemm(c, p);
     }
     // Partial broadcast: full batched product into scratch, then the device-side unbroadcast.
     const size_t bytes = static_cast<size_t>(obatch * R * Cn) * sizeof(float);
@@ -828,37 +847,48 @@ int grad_gemm(Call &c, Operand X, Operand Y, int64_t R, int64_t Cn, int64_t kdim
     return launch_unbroadcast(c.at(off), gshape, onb + 2, target.shape, target.ndim, out, accumulate, c.stream);
 }
 
-// Whether the gradients on the tensor path are computed from 16-bit planes: one product each, of operands that have them.
+// The gradients on the tensor path as products of 16-bit planes, the one of the longer contraction first: units that take
+// longer are better dealt out early.
+struct HalfGrads {
+    GemmProblem p[2];
+    bool is_a[2];                      // grad_a = dc . b^T, or grad_b = a^T . dc
+    int count = 0;
+};
+// Whether they are computed so: one product each, of operands that have planes, and worth it.
 bool bwd_half_wanted(const Call &c, const Shapes &s, const mni_b200_view &a, const mni_b200_view &b, const mni_b200_view &dc, bool da,
-                     bool db, int64_t g_batch, double work) {
+                     bool db, int64_t g_batch, double work, HalfGrads &g) {
     if ((!da && !db) || s.M < 64 || s.N < 64 || s.K <= 128 || (da && s.M <= 128) || (db && s.N <= 128) || !half_possible(c, work)) return false;
     HalfView probe;
     bool swapped;
     if (!view_to_half(dc, probe, &swapped)) return false;
-    double elements = static_cast<double>(g_batch) * s.M * s.N, f32_us = 0, half_us = 0, beside_us = 0, gathers_us = gather_us(dc);
+    double elements = static_cast<double>(g_batch) * s.M * s.N, f32_us = 0, beside_us = 0, gathers_us = gather_us(dc);
     const int all = c.gemm_sms(1), halved = c.gemm_sms(2);
-    auto product = [&](const mni_b200_view &other, const mni_b200_view &target, int64_t rows, int64_t cols, int64_t k) {
+    auto product = [&](const mni_b200_view &other, const mni_b200_view &target, int64_t rows, int64_t cols, int64_t k, bool is_a) {
         int64_t ob[MNI_B200_MAX_DIMS];
         bool same;
         const int nb = broadcast_shape(other.shape, other.ndim - 2, dc.shape, dc.ndim - 2, ob);
         if (nb < 0 || !single_product(ob, nb, target, &same) || !view_to_half(other, probe, &swapped)) return false;
         const int64_t count = prod(ob, nb);
-        GemmProblem p;
+        g.is_a[g.count] = is_a;
+        GemmProblem &p = g.p[g.count++];
         p.M = rows; p.N = cols; p.K = k;
         p.batch = same ? count : 1;
         p.fold = same ? 1 : count;
         p.ldc = cols; p.c_bstride = rows * cols;
         p.fast_tf32 = (c.flags & MNI_B200_PRECISION_TF32) != 0;
-        f32_us += gemm_estimate_us(p, false, all);
+        f32_us += gemm_estimate_us(p, all);
         gathers_us += gather_us(other);
-        half_us += gemm_estimate_us(p, true, all);
-        beside_us = std::max(beside_us, gemm_estimate_us(p, false, halved));
+        beside_us = std::max(beside_us, (p.fast_tf32 ? 1.25 : 1.1) * gemm_estimate_us(p, halved));   // they slow one another down
         elements += static_cast<double>(prod(other.shape, other.ndim));
         return true;
     };
-    if (da && !product(b, a, s.M, s.K, s.N)) return false;
-    if (db && !product(a, b, s.K, s.N, s.M)) return false;
-    return half_pays(c, gathers_us + (da && db ? std::min(f32_us, beside_us) : f32_us), half_us, elements);
+    if (da && !product(b, a, s.M, s.K, s.N, true)) return false;
+    if (db && !product(a, b, s.K, s.N, s.M, false)) return false;
+    if (g.count == 2 && g.p[1].K * g.p[1].fold > g.p[0].K * g.p[0].fold) {
+        std::swap(g.p[0], g.p[1]);
+        std::swap(g.is_a[0], g.is_a[1]);
+    }
+    return half_pays(c, gathers_us + (da && db ? std::min(f32_us, beside_us) : f32_us), gemm_halves_estimate_us(g.p, g.count, all), elements);
 }
 
 int bwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const mni_b200_view *dc, float *da,
@@ -999,8 +1029,9 @@ int bwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const mni_
         c.label = "";
         return r;
     };
-    // From 16-bit operands, one product after the other on all SMs, instead of everything above and below but the column sums.
-    const bool half = bwd_half_wanted(c, s, *a, *b, *dc, da_tensor, db_tensor, g_batch, work), halves_now = half && !c.plan_log;
+    // From 16-bit planes, in one launch on all SMs, instead of everything above and below but the column sums.
+    HalfGrads half_grads;
+    const bool half = bwd_half_wanted(c, s, *a, *b, *dc, da_tensor, db_tensor, g_batch, work, half_grads), halves_now = half && !c.plan_log;
     if (halves_now) c.sm_share = 1;
     else rc = pack();
     if (rc) return rc;
@@ -1072,19 +1103,18 @@ int bwd_body(Call &c, const mni_b200_view *a, const mni_b200_view *b, const mni_
         int r = da_tensor && db_tensor ? make_halves(c, {dc_given, b_given, a_given}, h, sums, acc_dbias)
                 : da_tensor            ? make_halves(c, {dc_given, b_given}, h, sums, acc_dbias)
                                        : make_halves(c, {dc_given, a_given}, h, sums, acc_dbias);
-        int64_t ob[MNI_B200_MAX_DIMS];
-        if (r == MNI_B200_OK && da_tensor) {
-            c.label = "grad_a: ";
-            const int onb = broadcast_shape(dc_given->shape, gn - 2, b_given->shape, b_given->ndim - 2, ob);
-            const HalfOperand x = h.operand(0, false), y = h.operand(1, false);
-            r = grad_gemm(c, Operand{}, Operand{}, s.M, s.K, s.N, ob, onb, *a_given, da, acc_da, &h, &x, &y);
+        if (r) return r;
+        HalfOperand x[2], y[2];
+        const char *labels[2];
+        for (int i = 0; i < half_grads.count; ++i) {
+            const bool is_a = half_grads.is_a[i];
+            labels[i] = is_a ? "grad_a: " : "grad_b: ";
+            x[i] = is_a ? h.operand(0, false) : h.operand(da_tensor ? 2 : 1, true);
+            y[i] = is_a ? h.operand(1, false) : h.operand(0, true);
+            half_grads.p[i].C = is_a ? da : db;
+            half_grads.p[i].accumulate = is_a ? acc_da : acc_db;
         }
-        if (r == MNI_B200_OK && db_tensor) {
-            c.label = "grad_b: ";
-            const int onb = broadcast_shape(a_given->shape, a_given->ndim - 2, dc_given->shape, gn - 2, ob);
-            const HalfOperand x = h.operand(da_tensor ? 2 : 1, true), y = h.operand(0, true);
-            r = grad_gemm(c, Operand{}, Operand{}, s.K, s.N, s.M, ob, onb, *b_given, db, acc_db, &h, &x, &y);
-        }
+        r = run_halves(c, half_grads.p, half_grads.count, h, x, y, labels);
         return r;
     };
     if (halves_now) return halves();

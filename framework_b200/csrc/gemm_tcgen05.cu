@@ -64,6 +64,7 @@
 #include <algorithm>
 #include <cmath>
 #include <mutex>
+#include <type_traits>
 #include <unordered_map>
 
 namespace mni {
@@ -136,6 +137,18 @@ struct KParams {
     const int *a_exp, *b_exp;              // the operands were multiplied by 2^exponent
     const unsigned int *half_status;       // a word per block of it: != 0, some operand's range does not fit
     int half_statuses;
+};
+
+// What a launch computes: one product, or (16-bit planes) two that need nothing from each other, the units of the second dealt
+// out after those of the first to the CTA pairs whose turn it is.
+struct Product {
+    CUtensorMap A, B, C, D, P;
+    KParams p;
+};
+template <int N>
+struct Products {
+    Product s[N];
+    int count;
 };
 
 // ------------------------------------------------------------------ PTX helpers
@@ -533,20 +546,21 @@ __device__ __forceinline__ void load_half(int mode, uint32_t dst, const CUtensor
 __host__ __device__ constexpr int gemm_threads(int ns, bool run) { return 32 * ((run ? 4 : 2) + ns + kEpiWarps); }
 // Register shares of the running-sum variants, in registers per thread, out of what the launch gives each thread (96 of
 // 640 threads, 128 of 512 in single-pass mode): two epilogue warpgroups, the split's and the one that issues.
-template <bool FAST>
+template <int MODE>
 struct RegShare {
-    static constexpr int kEpilogue = FAST ? 216 : 168, kSplit = FAST ? 40 : 48, kIssue = FAST ? 40 : 48;
-    static constexpr int kSplitGroups = FAST ? 1 : 2, kLaunch = FAST ? 128 : 96;
+    static constexpr bool kPlain = MODE == kThreePass, kOneF32 = MODE == kOnePass;
+    static constexpr int kEpilogue = kPlain ? 168 : kOneF32 ? 216 : 208, kSplit = kOneF32 ? 40 : 48, kIssue = kOneF32 ? 40 : 48;
+    static constexpr int kSplitGroups = kPlain ? 2 : 1, kLaunch = kPlain ? 96 : 128;
     static_assert(2 * kEpilogue + kSplitGroups * kSplit + kIssue <= (3 + kSplitGroups) * kLaunch, "more registers than the launch has");
 };
 // ... and of the two-accumulator variant, 168 of 384 threads at launch: two epilogue warpgroups and the one of all other roles.
-constexpr int kTwoEpilogue = 232, kTwoIssue = 40, kTwoLaunch = 168;
+constexpr int kTwoEpilogue = 224, kTwoIssue = 56, kTwoLaunch = 168;
 static_assert(2 * kTwoEpilogue + kTwoIssue <= 3 * kTwoLaunch, "more registers than the launch has");
+__host__ __device__ constexpr int product_slots(int mode) { return mode == kHalfThree || mode == kHalfOne ? 2 : 1; }
 template <int BN, int BK, int MODE, int NS, int CG, bool TA = false, int TAIL = kWholeTiles, int SG = 1>
 __global__ void __launch_bounds__(gemm_threads(NS, TAIL == kRunningSum), 1)
-gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-               const __grid_constant__ CUtensorMap tmC, const __grid_constant__ CUtensorMap tmD,
-               const __grid_constant__ CUtensorMap tmP, const __grid_constant__ KParams p) {
+gemm_tc_kernel(const __grid_constant__ Products<product_slots(MODE)> g) {
+    const KParams &p = g.s[0].p;                           // what every product of the launch shares is read there
     constexpr bool SK = TAIL == kBalanced, CUT = TAIL == kCutTiles;
     constexpr bool HALF = MODE == kHalfThree || MODE == kHalfOne, FAST = MODE != kThreePass;   // FAST: the split warps split nothing
     static_assert(!HALF || (BN == 256 && BK == 64 && CG == 2 && !TA && !SK), "16-bit halves are built for 256-wide pairs");
@@ -599,9 +613,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     if (threadIdx.x == 0 && p.dep_mode != 1) grid_dependency_trigger();
     if (warp == 0 && lane == 1) {
         // descriptor fetches overlap the barrier and TMEM set-up
-        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmA)) : "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmB)) : "memory");
-        asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmC)) : "memory");
+        for (int prod = 0; prod < (HALF ? g.count : 1); ++prod) {
+            asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&g.s[prod].A)) : "memory");
+            asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&g.s[prod].B)) : "memory");
+            asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&g.s[prod].C)) : "memory");
+        }
     }
     if (threadIdx.x == 0) {
         for (int s = 0; s < p.stages; ++s) {
@@ -642,28 +658,28 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     if (p.dep_mode != 2) grid_dependency_wait();
     if (p.dep_mode == 1 && threadIdx.x == 0) grid_dependency_trigger();
     // HALF: wide if some operand's range did not fit f16, and the planes hold bf16 thirds, unscaled.
-    float unscale = 1.f;
-    bool wide = false;
+    bool wide = false, huge = false;
     if constexpr (HALF) {
         unsigned int status = 0;
         for (int i = threadIdx.x; i < p.half_statuses; i += blockDim.x) status |= __ldcg(p.half_status + i);
-        int ea = __ldcg(p.a_exp), eb = __ldcg(p.b_exp);          // at most 60 either way
         wide = __syncthreads_or(status & 1u) != 0;
-        if (wide) {
-            const bool huge = __syncthreads_or(status & 2u) != 0;
-            ea = half_wide_exponent(ea, huge);
-            eb = half_wide_exponent(eb, huge);
-        }
-        unscale = __uint_as_float(static_cast<uint32_t>(127 - ea - eb) << 23);
+        if (wide) huge = __syncthreads_or(status & 2u) != 0;
     }
+    // The products of the launch, as every role walks them: first_unit is this CTA pair's first unit of one.
+    const int products = HALF ? g.count : 1;
+    auto first_unit = [&](int prod) {
+        if (prod == 0) return unit0;
+        const int at = unit0 - g.s[0].p.units % unit_step;
+        return at < 0 ? at + unit_step : at;
+    };
     const int planes = TWO ? (wide ? 3 : 2) : (wide ? 2 : 1);     // HALF
 
     // The epilogue comes first: it is the branch whose register share the running-sum variants raise.
     if (warp >= EPI0) {
         // RUN: the warpgroups trade registers; the increase waits for the others' decrease
-        if constexpr (RUN) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(TWO ? kTwoEpilogue : RegShare<FAST>::kEpilogue));
+        if constexpr (RUN) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(TWO ? kTwoEpilogue : RegShare<MODE>::kEpilogue));
         // ------------------------------------------------------------ epilogue
-        const int q = warp & 3;                       // TMEM lane quarter this warp may read
+        const int quarter = warp & 3;                       // TMEM lane quarter this warp may read
         const int ew = warp - EPI0;               // 0..7: warps ew and ew+4 share a lane quarter ...
         constexpr int CHUNKS = BN / 32 / (kEpiWarps / 4);   // ... and take half of the tile's 32-column chunks each
         const int chunk_lo = (ew >> 2) * CHUNKS;
@@ -673,13 +689,24 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         int in_flight = 0;                            // bulk groups committed by lane 0 and not yet waited for
         bool ok = true;
         long long waited = 0, t_ld = 0, t_wg = 0;
-        const bool use_tma = p.epi_mode == kEpiTmaStore || p.epi_mode == kEpiTmaReduce;
-        const bool bias_vec = (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0;
-        WorkIter wi = work_begin(p, unit0, unit_step);
-        TileCoord t;
         const int my_cta = static_cast<int>(blockIdx.x);                 // slot * CG + rank in the pair
+        bool any_tma = false;
+        for (int prod = 0; ok && prod < products; ++prod) {
+        const Product &w = g.s[HALF ? prod : 0];
+        const KParams &q = HALF ? w.p : p;
+        float unscale = 1.f;
+        if constexpr (HALF) {
+            int ea = __ldcg(q.a_exp), eb = __ldcg(q.b_exp);          // at most 60 either way
+            if (wide) { ea = half_wide_exponent(ea, huge); eb = half_wide_exponent(eb, huge); }
+            unscale = __uint_as_float(static_cast<uint32_t>(127 - ea - eb) << 23);
+        }
+        const bool use_tma = q.epi_mode == kEpiTmaStore || q.epi_mode == kEpiTmaReduce;
+        any_tma |= use_tma;
+        const bool bias_vec = (reinterpret_cast<uintptr_t>(q.bias) & 15) == 0;
+        WorkIter wi = work_begin(q, first_unit(prod), unit_step);
+        TileCoord t;
         uint32_t run[RUN ? CHUNKS : 1][32];           // RUN: sum of the unit's pieces so far
-        while (ok && work_next<TAIL>(p, wi, t)) {
+        while (ok && work_next<TAIL>(q, wi, t)) {
             const int buf = TWO ? 0 : acc_it & 1;
             const uint32_t acc_phase = TWO ? acc_it & 1 : (acc_it >> 1) & 1;
             ok = mbar_wait(bar_acc_full + 8u * buf, acc_phase, abort_flag, p.err, 0x500u | buf, waited, timed, p.wait_cycles);
@@ -687,7 +714,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             if (!ok) break;
             tc_fence_after();
             const bool part = CUT && t.part >= 0;            // of the split tail: a raw partial tile, always through TMA
-            const bool fuse = p.splits == 1 && !part;
+            const bool fuse = q.splits == 1 && !part;
             const bool tma_here = use_tma || part;
             const bool later_piece = t.chunk > 0;     // a later piece of this unit's contraction: added to the earlier ones
             const bool last_piece = wi.piece_it >= wi.piece_end;
@@ -698,9 +725,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 in_flight = 0;
                 __syncwarp();
             }
-            const int row0 = t.tm * (BM * CG) + static_cast<int>(cta_rank) * BM + q * 32;
-            const int cbatch = fuse ? t.bt : t.split * p.batch + t.bt;
-            const uint32_t tbase = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + static_cast<uint32_t>(buf * BN);
+            const int row0 = t.tm * (BM * CG) + static_cast<int>(cta_rank) * BM + quarter * 32;
+            const int cbatch = fuse ? t.bt : t.split * q.batch + t.bt;
+            const uint32_t tbase = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(buf * BN);
             // Shared tile of the balanced tail.  Each (tile, CTA rank, epilogue warp) region has a ticket; the
             // units of the tile arrive in any order, all but the last park their accumulator (and raise a
             // ready flag), the last one adds the parked ones to its own in slot order -- the sum does not
@@ -709,7 +736,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             bool reducer = false;
             const int nslots = static_cast<int>(gridDim.x) / CG;
             if (SK && t.shared) {
-                const long long per_tile = p.fold * p.kiters;
+                const long long per_tile = q.fold * q.kiters;
                 const long long tile_begin = static_cast<long long>(t.tile - p.sk_first_tile) * per_tile;
                 const long long tile_end = tile_begin + per_tile;
                 seg_first = unit0;
@@ -720,7 +747,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             }
             bool waited_contrib = false, parked = false;
             unsigned int *ticket = nullptr;
-            if (SK && t.shared && seg_count > 1 && row0 < p.M && t.tn * BN + chunk_lo * 32 < p.N) {
+            if (SK && t.shared && seg_count > 1 && row0 < q.M && t.tn * BN + chunk_lo * 32 < q.N) {
                 const size_t region = (static_cast<size_t>(t.tile - p.sk_first_tile) * CG + cta_rank) * kEpiWarps + ew;
                 ticket = p.sk_flags + static_cast<size_t>(gridDim.x) * 2 * kEpiWarps + region;
                 unsigned int old = 0;
@@ -734,7 +761,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             size_t others[kSkMaxShare - 1];
             int n_others = 0, n_before = 0;
             if (SK && reducer) {
-                const long long tile_begin = static_cast<long long>(t.tile - p.sk_first_tile) * (p.fold * p.kiters);
+                const long long tile_begin = static_cast<long long>(t.tile - p.sk_first_tile) * (q.fold * q.kiters);
                 for (int j = seg_first; j < seg_first + seg_count; ++j) {
                     if (j == unit0) continue;
                     const int idx = (j == seg_first && sk_range_begin(p, j, nslots) < tile_begin) ? 1 : 0;
@@ -789,12 +816,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 ++acc_it;
                 if (!last_piece) continue;
             }
-            if (row0 < p.M) {
+            if (row0 < q.M) {
 #pragma unroll(RUN ? CHUNKS : 1)
                 for (int c = 0; c < CHUNKS; ++c) {
                     const int chunk = chunk_lo + c;
                     const int col0 = t.tn * BN + chunk * 32;
-                    if (col0 >= p.N) break;           // warp-uniform
+                    if (col0 >= q.N) break;           // warp-uniform
                     uint32_t loaded[32];
                     uint32_t (&v)[32] = RUN ? run[RUN ? c : 0] : loaded;
                     if constexpr (!RUN) {
@@ -927,7 +954,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         if (lane == 0) {
                             const uint32_t src = smem_u32(my_stage + patch * kEpiBufBytes);
                             const int c0 = part ? chunk * 32 : (!RUN && p.transpose_out) ? row0 : col0;
-                            const int c1 = part ? static_cast<int>(cta_rank) * BM + q * 32 : (!RUN && p.transpose_out) ? col0 : row0;
+                            const int c1 = part ? static_cast<int>(cta_rank) * BM + quarter * 32 : (!RUN && p.transpose_out) ? col0 : row0;
                             const int c2 = part ? t.part : cbatch;
                             if (reduce) tma_reduce_add_5d(map, src, c0, c1, c2);
                             else tma_store_5d(map, src, c0, c1, c2);
@@ -936,19 +963,19 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         }
                         if (++patch == p.epi_patches) patch = 0;
                     };
-                    const bool do_act = (!RUN || HALF) && fuse && p.act != 0;          // host guarantees use_tma in this mode
-                    if (do_act && p.store_pre) emit(&tmC, false);    // the raw product, what the tape saves
-                    if (fuse && p.bias != nullptr && add_piece) {
+                    const bool do_act = (!RUN || HALF) && fuse && q.act != 0;          // host guarantees use_tma in this mode
+                    if (do_act && q.store_pre) emit(&w.C, false);    // the raw product, what the tape saves
+                    if (fuse && q.bias != nullptr && add_piece) {
                         // the bias went in with the first piece
-                    } else if (!RUN && fuse && p.bias != nullptr && p.transpose_out) {
-                        const float b = row0 + lane < p.M ? __ldg(p.bias + row0 + lane) : 0.f;   // one bias value per row here
+                    } else if (!RUN && fuse && q.bias != nullptr && p.transpose_out) {
+                        const float b = row0 + lane < q.M ? __ldg(q.bias + row0 + lane) : 0.f;   // one bias value per row here
 #pragma unroll
                         for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + b);
-                    } else if (fuse && p.bias != nullptr) {
-                        if (bias_vec && col0 + 32 <= p.N) {
+                    } else if (fuse && q.bias != nullptr) {
+                        if (bias_vec && col0 + 32 <= q.N) {
 #pragma unroll
                             for (int j = 0; j < 8; ++j) {
-                                const float4 b = __ldg(reinterpret_cast<const float4 *>(p.bias + col0) + j);
+                                const float4 b = __ldg(reinterpret_cast<const float4 *>(q.bias + col0) + j);
                                 v[4 * j + 0] = __float_as_uint(__uint_as_float(v[4 * j + 0]) + b.x);
                                 v[4 * j + 1] = __float_as_uint(__uint_as_float(v[4 * j + 1]) + b.y);
                                 v[4 * j + 2] = __float_as_uint(__uint_as_float(v[4 * j + 2]) + b.z);
@@ -957,23 +984,23 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         } else {
 #pragma unroll
                             for (int j = 0; j < 32; ++j)
-                                if (col0 + j < p.N) v[j] = __float_as_uint(__uint_as_float(v[j]) + __ldg(p.bias + col0 + j));
+                                if (col0 + j < q.N) v[j] = __float_as_uint(__uint_as_float(v[j]) + __ldg(q.bias + col0 + j));
                         }
                     }
                     if (do_act) {
-                        emit(&tmD, false, true);
+                        emit(&w.D, false, true);
                     } else if (part) {
-                        emit(&tmP, add_piece);
+                        emit(&w.P, add_piece);
                     } else if ((RUN && !HALF) || use_tma) {
-                        emit(&tmC, (p.epi_mode == kEpiTmaReduce && fuse) || add_piece);
+                        emit(&w.C, (q.epi_mode == kEpiTmaReduce && fuse) || add_piece);
                     } else {
-                        float *out0 = fuse ? p.C + static_cast<long long>(t.bt) * p.c_bstride + static_cast<long long>(row0) * p.ldc
-                                           : p.partial + (static_cast<long long>(cbatch) * p.M + row0) * p.partial_ld;
-                        const long long pitch = fuse ? p.ldc : p.partial_ld;
-                        const bool add = (fuse && p.accumulate) || add_piece;
-                        if (p.epi_mode == kEpiVectorStores && col0 + 32 <= p.N) {
+                        float *out0 = fuse ? q.C + static_cast<long long>(t.bt) * q.c_bstride + static_cast<long long>(row0) * q.ldc
+                                           : q.partial + (static_cast<long long>(cbatch) * q.M + row0) * q.partial_ld;
+                        const long long pitch = fuse ? q.ldc : q.partial_ld;
+                        const bool add = (fuse && q.accumulate) || add_piece;
+                        if (q.epi_mode == kEpiVectorStores && col0 + 32 <= q.N) {
                             // Each lane owns one row: four 32-byte stores write whole sectors, no staging.
-                            if (row0 + lane >= p.M) continue;
+                            if (row0 + lane >= q.M) continue;
                             float *dst = out0 + lane * pitch + col0;
 #pragma unroll
                             for (int j = 0; j < 4; ++j) {
@@ -1007,8 +1034,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                                 make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]),
                                             __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
                         __syncwarp();
-                        const int rows = min(32, p.M - row0);
-                        if (col0 + lane < p.N) {
+                        const int rows = min(32, q.M - row0);
+                        if (col0 + lane < q.N) {
                             float *dst = out0 + col0 + lane;
                             const uint8_t *src = my_stage + ((lane & 3) << 2);
 #pragma unroll 2
@@ -1058,9 +1085,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 ++acc_it;
             }
         }
+        }
         // The staging patches must have been read before the CTA gives up its shared memory; the global
         // writes themselves complete with the grid like any other store.
-        if ((use_tma || CUT) && lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        if ((any_tma || CUT) && lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
         if (p.prof && warp == EPI0 && lane == 0) {
             atomicAdd(p.prof + 4, static_cast<unsigned long long>(waited));
             atomicAdd(p.prof + 7, static_cast<unsigned long long>(t_wg));
@@ -1069,12 +1097,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     } else {
     if constexpr (RUN) {
         if (TWO) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kTwoIssue));
-        else if (warp < SPLIT0) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(RegShare<FAST>::kIssue));
-        else asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(RegShare<FAST>::kSplit));
+        else if (warp < SPLIT0) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(RegShare<MODE>::kIssue));
+        else asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(RegShare<MODE>::kSplit));
     }
-    if (warp == 0) {
+    if (warp == 0 || (HALF && warp == SPLIT0 + 1)) {
         // ------------------------------------------------------------ TMA producer
-        // The whole warp runs the loop; one elected lane issues the copies.
+        // The whole warp runs the loop; one elected lane issues the copies.  HALF: a stage holds a third of the time it holds
+        // in 3xTF32, so a second warp issues B's copies (the first arms the barrier).
+        const bool loads_a = !HALF || warp == 0, loads_b = !HALF || warp != 0;
         {
             int stage = 0;
             uint32_t phase = 0;
@@ -1084,17 +1114,23 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             constexpr uint32_t CHUNK_BYTES = 128u * BK;   // one 32-wide MN chunk: BK k-rows of 128 bytes
             const uint32_t dstA0 = smem_u32(stage_base);
             uint32_t dstA = dstA0;
-            WorkIter wi = work_begin(p, unit0, unit_step);
+#pragma unroll                             // parameters at constant addresses, so that what an MMA or a copy takes stays uniform
+            for (int prod = 0; prod < product_slots(MODE); ++prod) {
+            if (!ok || prod >= products) break;
+            const Product &w = g.s[HALF ? prod : 0];
+            const KParams &q = HALF ? w.p : p;
+            const int a_mode = q.a_mode, b_mode = q.b_mode, kiters = q.kiters;
+            WorkIter wi = work_begin(q, first_unit(prod), unit_step);
             TileCoord t;
-            while (ok && work_next<TAIL>(p, wi, t)) {
+            while (ok && work_next<TAIL>(q, wi, t)) {
                 int f = 0, kk = t.it0;
-                if (t.it0 >= p.kiters) {
-                    f = t.it0 / p.kiters;
-                    kk = t.it0 - f * p.kiters;
+                if (t.it0 >= q.kiters) {
+                    f = t.it0 / q.kiters;
+                    kk = t.it0 - f * q.kiters;
                 }
                 int a0, a1, a2, b0, b1, b2;
-                batch_coords(t.bt * p.fold + f, p.a_batch, p.a_d1, p.a_d2, p.fd_a_cnt, p.fd_a_d1, p.fd_a_d2, a0, a1, a2);
-                batch_coords(t.bt * p.fold + f, p.b_batch, p.b_d1, p.b_d2, p.fd_b_cnt, p.fd_b_d1, p.fd_b_d2, b0, b1, b2);
+                batch_coords(t.bt * q.fold + f, q.a_batch, q.a_d1, q.a_d2, q.fd_a_cnt, q.fd_a_d1, q.fd_a_d2, a0, a1, a2);
+                batch_coords(t.bt * q.fold + f, q.b_batch, q.b_d1, q.b_d2, q.fd_b_cnt, q.fd_b_d1, q.fd_b_d2, b0, b1, b2);
                 const int rowA = t.tm * (BM * CG) + static_cast<int>(cta_rank) * BM;
                 const int rowB = t.tn * BN + static_cast<int>(cta_rank) * BNL;
                 if constexpr (HALF) {
@@ -1107,20 +1143,20 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                             const uint32_t full = bar_full + 8u * stage;
                             ++armed;
                             if (elect_one()) {
-                                mbar_arrive_expect_tx(full, RAW_BYTES);
+                                if (loads_a) mbar_arrive_expect_tx(full, RAW_BYTES);
                                 if (armed != p.withhold_at) {
-                                    load_half(p.a_mode, dstA, &tmA, full, kk * BK, rowA, a2, plane);
-                                    load_half(p.b_mode, dstA + A_BYTES, &tmB, full, kk * BK, rowB, b2, plane);
+                                    if (loads_a) load_half(a_mode, dstA, &w.A, full, kk * BK, rowA, a2, plane);
+                                    if (loads_b) load_half(b_mode, dstA + A_BYTES, &w.B, full, kk * BK, rowB, b2, plane);
                                 }
                             }
                             if (++stage == p.stages) { stage = 0; phase ^= 1u; dstA = dstA0; } else { dstA += STAGE_BYTES; }
                         }
-                        if (++kk == p.kiters) {
+                        if (++kk == kiters) {
                             kk = 0;
                             ++f;
-                            if (p.fold > 1) {
-                                batch_coords(t.bt * p.fold + f, p.a_batch, p.a_d1, p.a_d2, p.fd_a_cnt, p.fd_a_d1, p.fd_a_d2, a0, a1, a2);
-                                batch_coords(t.bt * p.fold + f, p.b_batch, p.b_d1, p.b_d2, p.fd_b_cnt, p.fd_b_d1, p.fd_b_d2, b0, b1, b2);
+                            if (q.fold > 1) {
+                                batch_coords(t.bt * q.fold + f, q.a_batch, q.a_d1, q.a_d2, q.fd_a_cnt, q.fd_a_d1, q.fd_a_d2, a0, a1, a2);
+                                batch_coords(t.bt * q.fold + f, q.b_batch, q.b_d1, q.b_d2, q.fd_b_cnt, q.fd_b_d1, q.fd_b_d2, b0, b1, b2);
                             }
                         }
                     }
@@ -1132,24 +1168,25 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     const int k0 = kk * BK;
                     ++armed;
                     if (elect_one()) {
-                        mbar_arrive_expect_tx(full, A_BYTES + static_cast<uint32_t>(p.b_rows_live) * BK * 4u);
+                        mbar_arrive_expect_tx(full, A_BYTES + static_cast<uint32_t>(q.b_rows_live) * BK * 4u);
                         if (armed != p.withhold_at) {        // test hook: a stage that is armed and never filled
-                            load_operand(p.a_mode, dstA, &tmA, full, k0, rowA, BM / 32, CHUNK_BYTES, a0, a1, a2);
-                            load_operand(p.b_mode, dstA + A_BYTES, &tmB, full, k0, rowB, BNL / 32, CHUNK_BYTES, b0, b1, b2);
+                            load_operand(a_mode, dstA, &w.A, full, k0, rowA, BM / 32, CHUNK_BYTES, a0, a1, a2);
+                            load_operand(b_mode, dstA + A_BYTES, &w.B, full, k0, rowB, BNL / 32, CHUNK_BYTES, b0, b1, b2);
                         }
                     }
                     if (++stage == p.stages) { stage = 0; phase ^= 1u; dstA = dstA0; } else { dstA += STAGE_BYTES; }
-                    if (++kk == p.kiters) {
+                    if (++kk == kiters) {
                         kk = 0;
                         ++f;
-                        if (p.fold > 1) {
-                            batch_coords(t.bt * p.fold + f, p.a_batch, p.a_d1, p.a_d2, p.fd_a_cnt, p.fd_a_d1, p.fd_a_d2, a0, a1, a2);
-                            batch_coords(t.bt * p.fold + f, p.b_batch, p.b_d1, p.b_d2, p.fd_b_cnt, p.fd_b_d1, p.fd_b_d2, b0, b1, b2);
+                        if (q.fold > 1) {
+                            batch_coords(t.bt * q.fold + f, q.a_batch, q.a_d1, q.a_d2, q.fd_a_cnt, q.fd_a_d1, q.fd_a_d2, a0, a1, a2);
+                            batch_coords(t.bt * q.fold + f, q.b_batch, q.b_d1, q.b_d2, q.fd_b_cnt, q.fd_b_d1, q.fd_b_d2, b0, b1, b2);
                         }
                     }
                 }
             }
-            if (!ok) {
+            }
+            if (!ok && loads_a) {
                 // Aborting: let the copies already issued land before the CTA exits.
                 const int pending = min(armed, p.stages);
                 for (int i = 0; i < pending; ++i) {
@@ -1158,7 +1195,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     while (!mbar_try_wait(bar_full + 8u * stage, phase) && clock64() - t0 < p.wait_cycles / 8) {}
                 }
             }
-            if (p.prof && lane == 0) atomicAdd(p.prof + 0, static_cast<unsigned long long>(waited));
+            if (p.prof && lane == 0 && loads_a) atomicAdd(p.prof + 0, static_cast<unsigned long long>(waited));
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
@@ -1172,18 +1209,22 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             long long waited = 0, waited_acc = 0;
             bool next_ready = false;                   // the stage about to be consumed was already seen complete
             const uint32_t sa0 = smem_u32(stage_base);
-            const uint32_t a_lo0 = ((sa0 >> 4) & 0x3FFFu) | p.a_desc_lbo;
-            const uint32_t b_lo0 = (((sa0 + A_BYTES) >> 4) & 0x3FFFu) | p.b_desc_lbo;
-            uint32_t a_lo = a_lo0, b_lo = b_lo0;
-            const uint32_t a_hi = p.a_desc_hi, b_hi = p.b_desc_hi;
-            const uint32_t a_ks = p.a_kstep, b_ks = p.b_kstep;
-            const uint32_t idesc = HALF && wide ? p.idesc | (1u << 7) | (1u << 10) : p.idesc;     // bf16 operands
+#pragma unroll                             // parameters at constant addresses, so that what an MMA or a copy takes stays uniform
+            for (int prod = 0; prod < product_slots(MODE); ++prod) {
+            if (!ok || prod >= products) break;
+            const KParams &q = HALF ? g.s[prod].p : p;
+            const uint32_t a_lo0 = ((sa0 >> 4) & 0x3FFFu) | q.a_desc_lbo;
+            const uint32_t b_lo0 = (((sa0 + A_BYTES) >> 4) & 0x3FFFu) | q.b_desc_lbo;
+            uint32_t a_lo = a_lo0 + static_cast<uint32_t>(stage) * STAGE16, b_lo = b_lo0 + static_cast<uint32_t>(stage) * STAGE16;
+            const uint32_t a_hi = q.a_desc_hi, b_hi = q.b_desc_hi;
+            const uint32_t a_ks = q.a_kstep, b_ks = q.b_kstep;
+            const uint32_t idesc = HALF && wide ? q.idesc | (1u << 7) | (1u << 10) : q.idesc;     // bf16 operands
             // A lone CTA in single-pass mode consumes the TMA barrier directly; otherwise the split warps
             // (of both CTAs, for a pair) announce the stage on the leader's barrier.
             const uint32_t ready0 = (FAST && CG == 1) ? bar_full : bar_xform;
-            WorkIter wi = work_begin(p, unit0, unit_step);
+            WorkIter wi = work_begin(q, first_unit(prod), unit_step);
             TileCoord wt;
-            while (ok && work_next<TAIL>(p, wi, wt)) {
+            while (ok && work_next<TAIL>(q, wi, wt)) {
                 const int iters = wt.it1 - wt.it0;
                 const int buf = TWO ? 0 : acc_it & 1;
                 const uint32_t acc_phase = TWO ? acc_it & 1 : (acc_it >> 1) & 1;
@@ -1197,6 +1238,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         if (++stage == p.stages) { stage = 0; phase ^= 1u; a_lo = a_lo0; b_lo = b_lo0; }
                         else { a_lo += STAGE16; b_lo += STAGE16; }
                     };
+                    // Compiled for each number of planes: as a run-time number it cost a tenth of the pipe (8192^3: 27.1 cycles per
+                    // element of a tile instead of 24.4).
+                    auto k_loop = [&](auto plane_count) {
+                    constexpr int PLANES = decltype(plane_count)::value;
+                    constexpr bool WIDE = PLANES > (TWO ? 2 : 1);
                     for (int it = 0; it < iters; ++it) {
                         ok = mbar_wait_warp(ready0 + 8u * stage, phase, abort_flag, p.err, 0x300u | stage, waited, timed, p.wait_cycles);
                         if (!ok) break;
@@ -1206,13 +1252,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 #pragma unroll
                             for (int ks = 0; ks < KSTEPS; ++ks)
                                 umma_f16_pair(d_tmem, ah + ks * a_ks, a_hi, bh + ks * b_ks, b_hi, idesc, ks == 0 ? accumulate : 1u);
-                            if (planes == 1) umma_commit_pair(bar_empty + 8u * hi_stage);
+                            if (PLANES == 1) umma_commit_pair(bar_empty + 8u * hi_stage);
                         }
                         __syncwarp();
                         next();
                         // The products with the planes below hi: into an accumulator of their own (TWO) or the same.
                         uint32_t small_acc = TWO ? accumulate : 1u;
-                        for (int plane = 1; plane < planes; ++plane) {
+#pragma unroll
+                        for (int plane = 1; plane < PLANES; ++plane) {
                             ok = mbar_wait_warp(ready0 + 8u * stage, phase, abort_flag, p.err, 0x300u | stage, waited, timed, p.wait_cycles);
                             if (!ok) break;
                             if (TWO && it == 0 && plane == 1) {     // its accumulator comes free a little later than the other
@@ -1226,11 +1273,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                                 for (int ks = 0; ks < KSTEPS; ++ks) {
                                     umma_f16_pair(d_small, a_lo + ks * a_ks, a_hi, bh + ks * b_ks, b_hi, idesc, ks == 0 ? small_acc : 1u);
                                     umma_f16_pair(d_small, ah + ks * a_ks, a_hi, b_lo + ks * b_ks, b_hi, idesc, 1u);
-                                    if (TWO && wide && plane == 1)
+                                    if (TWO && WIDE && plane == 1)
                                         umma_f16_pair(d_small, a_lo + ks * a_ks, a_hi, b_lo + ks * b_ks, b_hi, idesc, 1u);
                                 }
                                 umma_commit_pair(bar_empty + 8u * stage);
-                                if (plane + 1 == planes) umma_commit_pair(bar_empty + 8u * hi_stage);
+                                if (plane + 1 == PLANES) umma_commit_pair(bar_empty + 8u * hi_stage);
                             }
                             __syncwarp();
                             small_acc = 1u;
@@ -1239,6 +1286,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         if (!ok) break;
                         accumulate = 1u;
                     }
+                    };
+                    if (wide) k_loop(std::integral_constant<int, TWO ? 3 : 2>{});
+                    else k_loop(std::integral_constant<int, TWO ? 2 : 1>{});
                     if (ok && elect_one()) umma_commit_pair(bar_acc_full + 8u * buf);
                     __syncwarp();
                     if (!ok) break;
@@ -1302,6 +1352,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 ++acc_it;
                 }
             }
+            }
             if (p.prof && lane == 0) {
                 atomicAdd(p.prof + 1, static_cast<unsigned long long>(waited_acc));
                 atomicAdd(p.prof + 2, static_cast<unsigned long long>(waited));
@@ -1333,10 +1384,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             constexpr int PER = (N4 + NT - 1) / NT;       // float4s per thread (the last round may be partial)
             constexpr bool EXACT = N4 % NT == 0;
             constexpr int U = !EXACT ? 1 : (PER % 4 == 0) ? 4 : (PER % 2 == 0 ? 2 : 1);
-            WorkIter wi = work_begin(p, unit0, unit_step);
-            TileCoord wt;
             if (HALF && warp != SPLIT0) ok = false;           // one warp relays there
-            while (ok && work_next<TAIL>(p, wi, wt)) {
+#pragma unroll                             // parameters at constant addresses, so that what an MMA or a copy takes stays uniform
+            for (int prod = 0; prod < product_slots(MODE); ++prod) {
+            if (!ok || prod >= products) break;
+            const KParams &q = HALF ? g.s[prod].p : p;
+            WorkIter wi = work_begin(q, first_unit(prod), unit_step);
+            TileCoord wt;
+            while (ok && work_next<TAIL>(q, wi, wt)) {
                 int iters = wt.it1 - wt.it0;
                 if (HALF) iters *= planes;                        // each takes a stage
                 for (int it = 0; it < iters; ++it) {
@@ -1354,7 +1409,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                       for (int h = 0; h < SG; ++h) {
                         const int half = SG == 2 ? h : group;
                         uint32_t hi[16], lo16[16];
-                        if (p.a_mode == kKMajor) {
+                        if (q.a_mode == kKMajor) {
                             // 128-byte rows, 16-byte chunk c of row r sits at chunk c ^ (r % 8)
                             const uint8_t *rp = sa + row * 128;
 #pragma unroll
@@ -1391,7 +1446,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                                                                          (TA ? A_BYTES : 0));
                     float4 *lo = const_cast<float4 *>(raw) + N4;
                     // float4s that hold data: all of them, or A and the live rows of B
-                    const int live4 = N4 - ((BNL - p.b_rows_live) * BK * 4 >> 4);
+                    const int live4 = N4 - ((BNL - q.b_rows_live) * BK * 4 >> 4);
 #pragma unroll
                     for (int g = 0; g < (FAST ? 0 : PER); g += U) {
                         float4 v[U];
@@ -1423,6 +1478,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     }
                     if (++stage == p.stages) { stage = 0; phase ^= 1u; }
                 }
+            }
             }
             if (p.prof && tid == 0) atomicAdd(p.prof + 3, static_cast<unsigned long long>(waited));
         }
@@ -1817,7 +1873,7 @@ double finish_us(double parts, double bytes) { return 1.5 + (parts + 1.0) * byte
 // 2048 x 3072 x 3584 177 / 169 / 168; at K = 2048, 121 / 117 / -, it would save 4.6 %.  Not in single-pass mode, whose long units
 // lose more by giving up their running sum (2048 x 8192 x 3584 200 / 209 / 231), and not beside another product, which uses the
 // SMs that the wave leaves.  `round_only`: neither.
-Cut cut_tail(long long tiles, long long slots, long long k, bool round_only, double pair_ns = kPairNs) {
+Cut cut_tail(long long tiles, long long slots, long long k, bool round_only) {
     const long long full = tiles / slots, rem = tiles - full * slots;
     const double tile_bytes = 4.0 * 2 * BM * 256;
     const Cut whole{1, static_cast<double>(rem > 0 ? full + 1 : full), 0.0};
@@ -1827,7 +1883,7 @@ Cut cut_tail(long long tiles, long long slots, long long k, bool round_only, dou
     if (full >= 1 && ways >= 2 && eff < 0.80 && k / ways >= 128)
         return Cut{ways, static_cast<double>(full) + 1.0 / static_cast<double>(ways), finish_us(static_cast<double>(ways), tile_bytes * static_cast<double>(rem))};
     if (round_only) return whole;
-    const double round_us = static_cast<double>(k) * pair_ns * 1e-3;
+    const double round_us = static_cast<double>(k) * kPairNs * 1e-3;
     Cut best = whole;
     for (long long w = 2; w <= 6 && k / w >= 256; ++w) {
         const Cut c{w, static_cast<double>(full) + static_cast<double>((rem * w + slots - 1) / slots) / static_cast<double>(w),
@@ -1847,45 +1903,139 @@ int chunk_iters_for(const GemmProblem &p, int bk) {
 
 // Main loop of a 256-wide pair over 16-bit planes, nanoseconds per contraction element, in a loop of calls (the pipe's own 12.6
 // and 4.2 at 1.9 GHz are out of reach of the power, and of L2, which feeds 32 and 16 KB a pair and 16 elements).
-double half_pair_ns(const GemmProblem &p) { return p.fast_tf32 ? 7.0 : 16.5; }
+double half_pair_ns(const GemmProblem &p) { return p.fast_tf32 ? 6.5 : 15.0; }
 
-// Products of 16-bit halves: 256-wide pairs throughout.  Few tiles: the contraction is split until the pairs are busy; a ragged
-// last wave is cut as cut_tail says.
-Plan make_half_plan(const GemmProblem &p, int sm_count) {
-    Plan pl{};
-    pl.bn = 256;
-    pl.bk = 64;
-    pl.cg = 2;
-    pl.patches = 1;
-    const size_t stage = static_cast<size_t>(BM + 128) * pl.bk * 2, fixed = 1024 + kBarBytes + static_cast<size_t>(kEpiWarps) * kEpiBufBytes;
-    pl.stages = static_cast<int>(std::min<size_t>(kMaxStages, (227 * 1024 - fixed) / stage));
-    pl.smem = fixed + static_cast<size_t>(pl.stages) * stage;
-    const int slots = std::max(1, sm_count / 2);
-    pl.tiles_m = static_cast<int>((p.M + 255) / 256);
-    pl.tiles_n = static_cast<int>((p.N + 255) / 256);
-    const long long tiles = static_cast<long long>(p.batch) * pl.tiles_m * pl.tiles_n;
-    const long long iters = p.fold * ((p.K + pl.bk - 1) / pl.bk);
-    long long splits = 1;
-    if (tiles * 2 <= slots && iters >= 8) splits = std::max<long long>(1, std::min<long long>(slots / tiles, iters / 4));
-    pl.splits = static_cast<int>(std::min<long long>(splits, 64));
-    const long long units = tiles * pl.splits;
-    pl.grid = static_cast<int>(std::min<long long>(units, slots)) * 2;
-    if (pl.splits == 1) {
-        const Cut cut = cut_tail(tiles, slots, iters * pl.bk, false, half_pair_ns(p));
-        if (cut.ways > 1) {
-            pl.tail_ways = static_cast<int>(cut.ways);
-            pl.tail_tiles = static_cast<int>(tiles % slots);
-            pl.grid = static_cast<int>(std::min<long long>(tiles + pl.tail_tiles * (cut.ways - 1), slots)) * 2;
-            return pl;
+// Longest of the CTA pairs' shares when groups of units of equal cost are dealt out one after the other, round-robin.
+struct UnitGroup {
+    long long count;
+    double cost;
+};
+double longest_share(const UnitGroup *groups, int n, int slots) {
+    auto share = [&](long long s) {
+        double load = 0.0;
+        long long at = 0;
+        for (int i = 0; i < n; ++i) {
+            const long long first = (s - at % slots + slots) % slots;       // this slot's first unit of the group
+            if (first < groups[i].count) load += static_cast<double>((groups[i].count - 1 - first) / slots + 1) * groups[i].cost;
+            at += groups[i].count;
         }
+        return load;
+    };
+    double most = share(0);            // it changes only where a group begins
+    long long at = 0;
+    for (int i = 0; i < n; ++i) {
+        at += groups[i].count;
+        most = std::max(most, share(at % slots));
     }
-    const long long chunk = chunk_iters_for(p, pl.bk), unit_len = (iters + pl.splits - 1) / pl.splits;
-    pl.running = chunk > 0 && unit_len > chunk + (chunk >> 3);
-    return pl;
+    return most;
+}
+
+// Plans for one or two products of 16-bit planes that share a launch: 256-wide pairs throughout, dealt out in the order given.
+// Where units are few, the contractions are split (for a finish kernel that adds the parts), or the last tiles are cut, so that
+// the pairs' shares even out.  Returns the estimated microseconds.  A unit costs its main loop and what the pipe waits between
+// units; a launch 8 us for its first operands and its last stores.
+double find_half_plans(const GemmProblem *p, int count, int sm_count, Plan *pl) {
+    const int slots = std::max(1, sm_count / 2);
+    const bool one = p[0].fast_tf32;
+    auto unit_us = [&](double k_us) { return std::max(k_us + (one ? 1.0 : 4.5), 4.5); };     // ... or its stores
+    struct {
+        long long tiles, iters, chunk;
+        double k_us, out_bytes;
+    } w[2];
+    for (int i = 0; i < count; ++i) {
+        Plan &q = pl[i] = Plan{};
+        q.bn = 256;
+        q.bk = 64;
+        q.cg = 2;
+        q.patches = 1;
+        const size_t stage = static_cast<size_t>(BM + 128) * q.bk * 2, fixed = 1024 + kBarBytes + static_cast<size_t>(kEpiWarps) * kEpiBufBytes;
+        q.stages = static_cast<int>(std::min<size_t>(kMaxStages, (227 * 1024 - fixed) / stage));
+        q.smem = fixed + static_cast<size_t>(q.stages) * stage;
+        q.tiles_m = static_cast<int>((p[i].M + 255) / 256);
+        q.tiles_n = static_cast<int>((p[i].N + 255) / 256);
+        q.splits = 1;
+        w[i].tiles = static_cast<long long>(p[i].batch) * q.tiles_m * q.tiles_n;
+        w[i].iters = p[i].fold * ((p[i].K + q.bk - 1) / q.bk);
+        w[i].chunk = chunk_iters_for(p[i], q.bk);
+        w[i].k_us = static_cast<double>(w[i].iters * q.bk) * half_pair_ns(p[i]) * 1e-3;
+        w[i].out_bytes = 4.0 * static_cast<double>(p[i].batch) * static_cast<double>(p[i].M) * static_cast<double>(p[i].N);
+    }
+    auto pieces = [&](int i, long long splits) { return w[i].chunk > 0 && (w[i].iters + splits - 1) / splits > w[i].chunk + (w[i].chunk >> 3); };
+    constexpr int kWays[] = {1, 2, 3, 4, 6, 8, 12, 16, 24, 32};
+    double best = 1e300;
+    int best_splits[2] = {1, 1}, best_cut = 1;
+    const int last = count - 1;
+    for (const int s0 : kWays)
+        for (const int s1 : kWays) {
+            const int splits[2] = {s0, s1};
+            if (count == 1 && s1 > 1) break;
+            bool ok = true;
+            double finish = 0.0;
+            UnitGroup g[3];
+            for (int i = 0; i < count; ++i) {
+                ok = ok && (splits[i] == 1 || (p[i].D == nullptr && w[i].iters / splits[i] >= 4 && w[i].tiles * splits[i] <= 2 * slots));
+                g[i] = UnitGroup{w[i].tiles * splits[i], unit_us(w[i].k_us / splits[i])};
+                if (splits[i] > 1) finish += finish_us(splits[i], w[i].out_bytes);
+            }
+            if (!ok) continue;
+            const double t = longest_share(g, count, slots) + finish;
+            if (t < best) { best = t; best_splits[0] = s0; best_splits[1] = s1; best_cut = 1; }
+            // ... or the tiles of the last product that the last, ragged wave holds, cut; not where a running sum would be given up
+            const long long rem = (g[0].count + (count == 2 ? g[1].count : 0)) % slots;
+            if (splits[last] > 1 || rem == 0 || rem > w[last].tiles || (one && (pieces(0, s0) || pieces(last, 1)))) continue;
+            for (int ways = 2; ways <= 6 && w[last].iters / ways >= 4; ++ways) {
+                g[last].count = w[last].tiles - rem;
+                g[count] = UnitGroup{rem * ways, unit_us(w[last].k_us / ways)};
+                const double c = longest_share(g, count + 1, slots) + finish + finish_us(ways, 4.0 * 2 * BM * 256 * static_cast<double>(rem));
+                if (c < 0.97 * best) { best = c; best_splits[0] = s0; best_splits[1] = s1; best_cut = ways; }
+            }
+        }
+    long long units = 0;
+    for (int i = 0; i < count; ++i) {
+        pl[i].splits = best_splits[i];
+        units += w[i].tiles * pl[i].splits;
+    }
+    if (best_cut > 1) {
+        pl[last].tail_ways = best_cut;
+        pl[last].tail_tiles = static_cast<int>(units % slots);
+        units += static_cast<long long>(pl[last].tail_tiles) * (best_cut - 1);
+    }
+    for (int i = 0; i < count; ++i) {
+        pl[i].grid = static_cast<int>(std::min<long long>(units, slots)) * 2;
+        pl[i].running = pieces(i, pl[i].splits);
+        pl[i].est_us = 8.0 + best;
+    }
+    return 8.0 + best;
+}
+
+// A call asks several times (the estimate, its scratch, the launch), and a loop of calls the same again: the last few answers are
+// kept, a pure function of the sizes.
+double make_half_plans(const GemmProblem *p, int count, int sm_count, Plan *pl) {
+    struct Entry {
+        int64_t key[14];
+        Plan pl[2];
+        double us;
+    };
+    static thread_local Entry entries[8];
+    static thread_local unsigned next = 0;
+    int64_t key[14] = {count, sm_count, chunk_iters_for(p[0], 64), p[0].fast_tf32};
+    for (int i = 0; i < count; ++i) {
+        const int64_t k[5] = {p[i].M, p[i].N, p[i].K, p[i].batch, p[i].fold * 2 + (p[i].D != nullptr ? 1 : 0)};
+        std::copy(k, k + 5, key + 4 + 5 * i);
+    }
+    for (const Entry &e : entries)
+        if (std::equal(key, key + 14, e.key)) {
+            std::copy(e.pl, e.pl + count, pl);
+            return e.us;
+        }
+    Entry &e = entries[next++ % 8];
+    e.us = find_half_plans(p, count, sm_count, e.pl);
+    std::copy(key, key + 14, e.key);
+    std::copy(e.pl, e.pl + count, pl);
+    return e.us;
 }
 
 Plan make_plan(const GemmProblem &p, int sm_count) {
-    if (p.ha) return make_half_plan(p, sm_count);
     Plan pl;
     pl.bn = p.N <= 64 ? 64 : (p.N <= 128 ? 128 : 256);
     const int bn_env = env_int("MNI_B200_BN", 0);
@@ -2067,8 +2217,7 @@ uint32_t desc_hi_bits(uint32_t sbo_bytes, uint32_t layout_type) {
 }
 
 template <int BN, int BK, int MODE, int NS, int CG, bool TA = false, int TAIL = kWholeTiles, int SG = 1>
-cudaError_t launch_variant(const Plan &pl, const CUtensorMap &tmA, const CUtensorMap &tmB, const CUtensorMap &tmC,
-                           const CUtensorMap &tmD, const CUtensorMap &tmP, const KParams &k, cudaStream_t stream) {
+cudaError_t launch_variant(const Plan &pl, const Product *const *w, int count, cudaStream_t stream) {
     // The shared-memory opt-in is an attribute of the function on ONE device: set once per device of the process
     // (a bit per device ordinal; setting it twice from two threads is harmless).
     static std::atomic<uint64_t> opted_in{0};
@@ -2096,7 +2245,10 @@ cudaError_t launch_variant(const Plan &pl, const CUtensorMap &tmA, const CUtenso
     attrs[1].val.clusterDim.z = 1;
     cfg.attrs = attrs;
     cfg.numAttrs = CG == 2 ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, gemm_tc_kernel<BN, BK, MODE, NS, CG, TA, TAIL, SG>, tmA, tmB, tmC, tmD, tmP, k);
+    Products<product_slots(MODE)> g;
+    for (int i = 0; i < product_slots(MODE); ++i) g.s[i] = *w[i < count ? i : 0];
+    g.count = count;
+    return cudaLaunchKernelEx(&cfg, gemm_tc_kernel<BN, BK, MODE, NS, CG, TA, TAIL, SG>, g);
 }
 
 }  // namespace
@@ -2164,23 +2316,27 @@ GemmProblem kernel_view(const GemmProblem &p, bool *transposed) {
     return q;
 }
 
-bool gemm_tc_can_fuse_activation(const GemmProblem &p, int sm_count) {
-    const Plan pl = make_plan(p, sm_count);
+static bool can_fuse_activation(const GemmProblem &p, const Plan &pl) {
     auto aligned = [&](const float *ptr) { return (reinterpret_cast<uintptr_t>(ptr) & 15) == 0; };
     return pl.splits == 1 && p.ldc % 4 == 0 && p.c_bstride % 4 == 0 && aligned(p.D) && (p.C == nullptr || aligned(p.C)) &&
            env_int("MNI_B200_NO_TMA_STORE", 0) == 0 && env_int("MNI_B200_EPI_VECTOR", 0) == 0;
 }
 
+bool gemm_tc_can_fuse_activation(const GemmProblem &p, int sm_count) { return can_fuse_activation(p, make_plan(p, sm_count)); }
+
 static int64_t partial_pitch(int64_t n) { return (n + 3) / 4 * 4; }
 
+static size_t partial_bytes(const GemmProblem &p, const Plan &pl, int64_t out_rows, int64_t out_cols);
 size_t gemm_tc_partial_bytes(const GemmProblem &p0, int sm_count) {
     bool transposed = false;
     const GemmProblem p = kernel_view(p0, &transposed);
-    const Plan pl = make_plan(p, sm_count);
+    return partial_bytes(p, make_plan(p, sm_count), p0.M, p0.N);
+}
+static size_t partial_bytes(const GemmProblem &p, const Plan &pl, int64_t out_rows, int64_t out_cols) {
     if (pl.sk) return static_cast<size_t>(pl.grid) * 2 * BM * pl.bn * sizeof(float);   // two parked accumulators per CTA
     if (pl.tail_ways) return static_cast<size_t>(pl.tail_tiles) * pl.tail_ways * BM * pl.cg * pl.bn * sizeof(float);
     if (pl.splits <= 1) return 0;
-    return static_cast<size_t>(pl.splits) * p.batch * p0.M * partial_pitch(p0.N) * sizeof(float);
+    return static_cast<size_t>(pl.splits) * p.batch * out_rows * partial_pitch(out_cols) * sizeof(float);
 }
 
 bool gemm_tc_uses_pairs(const GemmProblem &p, int sm_count) {
@@ -2193,16 +2349,13 @@ double gemm_tc_estimate_us(const GemmProblem &p, int sm_count) {
     return p.fast_tf32 ? 0.0 : make_plan(kernel_view(p, &transposed), sm_count).est_us;
 }
 
-double gemm_estimate_us(const GemmProblem &p0, bool half, int sm_count) {
-    static const HalfOperand any;
-    GemmProblem p = p0;
-    p.ha = half ? &any : nullptr;
+double gemm_estimate_us(const GemmProblem &p0, int sm_count) {
     bool transposed = false;
-    p = kernel_view(p, &transposed);
+    const GemmProblem p = kernel_view(p0, &transposed);
     const Plan pl = make_plan(p, sm_count);
     if (pl.est_us > 0 && !p.fast_tf32) return pl.est_us;
+    const double ns = (p.fast_tf32 ? 13.0 : kPairNs) * (pl.bn == 256 ? 1.0 : (pl.bn == 128 ? 0.65 : 0.45));
     const double k = static_cast<double>(p.K) * static_cast<double>(p.fold);
-    const double ns = half ? half_pair_ns(p) : (p.fast_tf32 ? 13.0 : kPairNs) * (pl.bn == 256 ? 1.0 : (pl.bn == 128 ? 0.65 : 0.45));
     const double slots = std::max(1, sm_count / pl.cg), tiles = static_cast<double>(p.batch) * pl.tiles_m * pl.tiles_n;
     const double out = 4.0 * static_cast<double>(p.batch) * static_cast<double>(p.M) * static_cast<double>(p.N);
     double rounds = std::ceil(tiles * pl.splits / slots) / pl.splits, finish = pl.splits > 1 ? finish_us(pl.splits, out) : 0.0;
@@ -2210,14 +2363,33 @@ double gemm_estimate_us(const GemmProblem &p0, bool half, int sm_count) {
         rounds = std::floor(tiles / slots) + std::ceil(pl.tail_tiles * pl.tail_ways / slots) / pl.tail_ways;
         finish = finish_us(pl.tail_ways, 4.0 * BM * pl.cg * pl.bn * pl.tail_tiles);
     }
-    const double round_us = half ? k * ns * 1e-3 + (p.fast_tf32 ? 1.0 : 4.5) : std::max(k * ns * 1e-3, pl.bn == 256 ? 3.7 : 1.5);
-    return (half ? 8.0 : 5.0) + rounds * round_us + finish;
+    return 5.0 + rounds * std::max(k * ns * 1e-3, pl.bn == 256 ? 3.7 : 1.5) + finish;
+}
+
+double gemm_halves_estimate_us(const GemmProblem *p, int count, int sm_count) {
+    Plan pl[2];
+    return make_half_plans(p, count, sm_count, pl);
+}
+
+void gemm_halves_partial_bytes(const GemmProblem *p, int count, int sm_count, size_t *bytes) {
+    Plan pl[2];
+    make_half_plans(p, count, sm_count, pl);
+    for (int i = 0; i < count; ++i) bytes[i] = partial_bytes(p[i], pl[i], p[i].M, p[i].N);
+}
+
+static std::string describe_plan(const GemmProblem &p, const Plan &pl, bool transposed, bool halves);
+void gemm_halves_describe(const GemmProblem *p, int count, int sm_count, std::string *lines) {
+    Plan pl[2];
+    make_half_plans(p, count, sm_count, pl);
+    for (int i = 0; i < count; ++i) lines[i] = describe_plan(p[i], pl[i], false, true);
 }
 
 std::string gemm_tc_describe(const GemmProblem &p0, int sm_count) {
     bool transposed = false;
     const GemmProblem p = kernel_view(p0, &transposed);
-    const Plan pl = make_plan(p, sm_count);
+    return describe_plan(p, make_plan(p, sm_count), transposed, false);
+}
+static std::string describe_plan(const GemmProblem &p, const Plan &pl, bool transposed, bool halves) {
     // pieces a whole unit's contraction is summed in (the kernel's first_piece rule)
     const long long iters = p.fold * ((p.K + pl.bk - 1) / pl.bk);
     const long long len = (iters + pl.splits - 1) / pl.splits;
@@ -2227,7 +2399,7 @@ std::string gemm_tc_describe(const GemmProblem &p0, int sm_count) {
     snprintf(buf, sizeof(buf),
              "%s m=%lld n=%lld k=%lld batch=%lld fold=%lld bn=%d bk=%d pair=%d tmem_a=%d stages=%d splits=%d "
              "tail=%d grid=%d exchanged=%d single_pass=%d pieces=%d mma_n=%d tail_ways=%d running=%d",
-             p.ha ? "halves" : "tensor", static_cast<long long>(p.M), static_cast<long long>(p.N), static_cast<long long>(p.K),
+             halves ? "planes" : "tensor", static_cast<long long>(p.M), static_cast<long long>(p.N), static_cast<long long>(p.K),
              static_cast<long long>(p.batch), static_cast<long long>(p.fold), pl.bn, pl.bk, pl.cg == 2 ? 1 : 0,
              pl.ta ? 1 : 0, pl.stages, pl.splits, pl.sk || pl.tail_ways ? 1 : 0, pl.grid, transposed ? 1 : 0, p.fast_tf32 ? 1 : 0,
              pieces, mma_n_for(p, pl), pl.tail_ways, pl.running ? 1 : 0);
@@ -2278,22 +2450,19 @@ int launch_tail_finish(const GemmProblem &p, const Plan &pl, const KParams &k, c
 }
 }  // namespace
 
-int launch_gemm_tc(const GemmProblem &p0, float *partial, uint32_t *err_word, int sm_count,
-                   cudaStream_t stream, GemmFinish *defer) {
-    if (p0.M <= 0 || p0.N <= 0 || p0.batch <= 0) return MNI_B200_OK;
-    bool transposed = false;
-    const GemmProblem p = kernel_view(p0, &transposed);       // p.M / p.N are the kernel's; oM / oN the output's
-    const int64_t oM = p0.M, oN = p0.N;
-    const Plan pl = make_plan(p, sm_count);
+// Fills in what one product of a launch needs.  oM / oN: the output's extents (p.M / p.N are the kernel's).
+static int make_product(const GemmProblem &p, const Plan &pl, bool transposed, int64_t oM, int64_t oN, float *partial, uint32_t *err_word,
+                        Product &w) {
     if (p.K <= 0) return fail(MNI_B200_ERR_ARG, "empty contraction reached the tensor-core launcher");
     if (transposed && (pl.tail_ways || pl.running))
         return fail(MNI_B200_ERR_ARG, "internal: a plan that stores no transposed patches for exchanged operands");
     if ((pl.splits > 1 || pl.sk || pl.tail_ways) && partial == nullptr)
         return fail(MNI_B200_ERR_WORKSPACE, "split-K launch without partial storage");
 
-    KParams k{};
-    CUtensorMap tmA, tmB, tmC, tmD, tmP;
-    if (p.D != nullptr && !gemm_tc_can_fuse_activation(p, sm_count))
+    KParams &k = w.p;
+    k = KParams{};
+    CUtensorMap &tmA = w.A, &tmB = w.B, &tmC = w.C, &tmD = w.D, &tmP = w.P;
+    if (p.D != nullptr && !can_fuse_activation(p, pl))
         return fail(MNI_B200_ERR_ARG, "fused activation requested for a problem that cannot carry it");
     const bool half = p.ha != nullptr;
     int rc = half ? make_half_map(&tmA, *p.ha, &k.a_mode) : make_operand_map(&tmA, p.A, BM, pl.bk, &k.a_mode);
@@ -2444,6 +2613,73 @@ int launch_gemm_tc(const GemmProblem &p0, float *partial, uint32_t *err_word, in
         if (pl.grid * 3 * kEpiWarps > kSkFlagCount) return fail(MNI_B200_ERR_CUDA, "balanced-tail flag array too small");
     }
 
+    return MNI_B200_OK;
+}
+static int launch_finish(const GemmProblem &p, const Plan &pl, const KParams &k, float *partial, int64_t oM, int64_t oN, cudaStream_t stream,
+                         GemmFinish *defer) {
+    if (pl.tail_ways) {
+        if (!defer) return launch_tail_finish(p, pl, k, partial, 0, stream);
+        *defer = [p, pl, k, partial](int dep_mode, cudaStream_t st) { return launch_tail_finish(p, pl, k, partial, dep_mode, st); };
+    } else if (pl.splits > 1) {
+        const SplitFinish f{partial, p.C, p.ldc, p.c_bstride, p.batch, oM, oN, p.bias, p.accumulate, pl.splits};
+        if (!defer) return launch_split_finish(f, 0, stream);
+        *defer = [f](int dep_mode, cudaStream_t st) { return launch_split_finish(f, dep_mode, st); };
+    }
+    return MNI_B200_OK;
+}
+
+int launch_gemm_halves(const GemmProblem *p, int count, float *const *partial, uint32_t *err_word, int sm_count, cudaStream_t stream) {
+    Plan pls[2];
+    make_half_plans(p, count, sm_count, pls);
+    Product w[2];
+    const Product *products[2] = {&w[0], &w[count - 1]};
+    bool cut = false, running = false, tma = true;
+    for (int i = 0; i < count; ++i) {
+        const int rc = make_product(p[i], pls[i], false, p[i].M, p[i].N, partial[i], err_word, w[i]);
+        if (rc) return rc;
+        cut = cut || pls[i].tail_ways > 0;
+        running = running || pls[i].running;
+        tma = tma && (w[i].p.epi_mode == kEpiTmaStore || w[i].p.epi_mode == kEpiTmaReduce) && p[i].D == nullptr;
+    }
+    const Plan &pl = pls[0];
+    cudaError_t e;
+    if (!p[0].fast_tf32) {
+        e = cut ? launch_variant<256, 64, kHalfThree, 2, 2, false, kCutTiles>(pl, products, count, stream)
+                : launch_variant<256, 64, kHalfThree, 2, 2>(pl, products, count, stream);
+    } else if (cut) {
+        e = launch_variant<256, 64, kHalfOne, 4, 2, false, kCutTiles>(pl, products, count, stream);
+    } else {
+        e = running && tma ? launch_variant<256, 64, kHalfOne, 4, 2, false, kRunningSum>(pl, products, count, stream)
+                           : launch_variant<256, 64, kHalfOne, 4, 2>(pl, products, count, stream);
+    }
+    if (e != cudaSuccess) return fail(MNI_B200_ERR_CUDA, "gemm_tc_kernel set-up failed: %s", cudaGetErrorString(e));
+    MNI_LAUNCH_CHECK("gemm_tc_kernel");
+    GemmFinish finish[2];
+    for (int i = 0; i < count; ++i) {
+        const int rc = launch_finish(p[i], pls[i], w[i].p, partial[i], p[i].M, p[i].N, stream, &finish[i]);
+        if (rc) return rc;
+    }
+    const bool both = finish[0] && finish[1];
+    for (int i = 0; i < count; ++i) {
+        const int rc = finish[i] ? finish[i](both ? i + 1 : 0, stream) : static_cast<int>(MNI_B200_OK);
+        if (rc) return rc;
+    }
+    return MNI_B200_OK;
+}
+
+int launch_gemm_tc(const GemmProblem &p0, float *partial, uint32_t *err_word, int sm_count,
+                   cudaStream_t stream, GemmFinish *defer) {
+    if (p0.M <= 0 || p0.N <= 0 || p0.batch <= 0) return MNI_B200_OK;
+    bool transposed = false;
+    const GemmProblem p = kernel_view(p0, &transposed);       // p.M / p.N are the kernel's; oM / oN the output's
+    const int64_t oM = p0.M, oN = p0.N;
+    const Plan pl = make_plan(p, sm_count);
+    Product w;
+    const int rc = make_product(p, pl, transposed, oM, oN, partial, err_word, w);
+    if (rc) return rc;
+    const KParams &k = w.p;
+    const Product *const products[1] = {&w};
+    constexpr int count = 1;
     // Two split groups pay when the k-loop is long enough for the second k-block in flight to matter (measured:
     // K = 512 per unit 33.6 -> 32.8 us per attention-shaped product, 128 k-blocks 57.9 -> 54.4 us; four k-blocks per
     // unit are no faster).  MNI_B200_SPLIT_GROUPS=1/2 forces either.
@@ -2455,48 +2691,39 @@ int launch_gemm_tc(const GemmProblem &p0, float *partial, uint32_t *err_word, in
     }
     const bool running = pl.running && (k.epi_mode == kEpiTmaStore || k.epi_mode == kEpiTmaReduce);
     cudaError_t e = cudaErrorInvalidValue;
-    if (half) {
-        if (p.fast_tf32) {
-            if (running) e = launch_variant<256, 64, kHalfOne, 4, 2, false, kRunningSum>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
-            else if (pl.tail_ways) e = launch_variant<256, 64, kHalfOne, 4, 2, false, kCutTiles>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
-            else e = launch_variant<256, 64, kHalfOne, 4, 2>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
-        } else {
-            if (pl.tail_ways) e = launch_variant<256, 64, kHalfThree, 2, 2, false, kCutTiles>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
-            else e = launch_variant<256, 64, kHalfThree, 2, 2>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
-        }
-    } else if (pl.sk) {
-        if (pl.ta && pl.bn == 64 && split_groups == 2) e = launch_variant<64, 32, kThreePass, 8, 1, true, kBalanced, 2>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
-        else if (pl.ta && pl.bn == 64) e = launch_variant<64, 32, kThreePass, 8, 1, true, kBalanced>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
-        else if (pl.ta && pl.bn == 128 && split_groups == 2) e = launch_variant<128, 32, kThreePass, 8, 1, true, kBalanced, 2>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
-        else if (pl.ta && pl.bn == 128) e = launch_variant<128, 32, kThreePass, 8, 1, true, kBalanced>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
-        else if (!p.fast_tf32 && pl.bk == 16) e = launch_variant<256, 16, kThreePass, 8, 2, false, kBalanced>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
-        else if (!p.fast_tf32 && pl.bk == 32) e = launch_variant<256, 32, kThreePass, 8, 2, false, kBalanced>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
-        else if (pl.bk == 16) e = launch_variant<256, 16, kOnePass, 4, 2, false, kBalanced>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
-        else e = launch_variant<256, 32, kOnePass, 4, 2, false, kBalanced>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+    if (pl.sk) {
+        if (pl.ta && pl.bn == 64 && split_groups == 2) e = launch_variant<64, 32, kThreePass, 8, 1, true, kBalanced, 2>(pl, products, count, stream);
+        else if (pl.ta && pl.bn == 64) e = launch_variant<64, 32, kThreePass, 8, 1, true, kBalanced>(pl, products, count, stream);
+        else if (pl.ta && pl.bn == 128 && split_groups == 2) e = launch_variant<128, 32, kThreePass, 8, 1, true, kBalanced, 2>(pl, products, count, stream);
+        else if (pl.ta && pl.bn == 128) e = launch_variant<128, 32, kThreePass, 8, 1, true, kBalanced>(pl, products, count, stream);
+        else if (!p.fast_tf32 && pl.bk == 16) e = launch_variant<256, 16, kThreePass, 8, 2, false, kBalanced>(pl, products, count, stream);
+        else if (!p.fast_tf32 && pl.bk == 32) e = launch_variant<256, 32, kThreePass, 8, 2, false, kBalanced>(pl, products, count, stream);
+        else if (pl.bk == 16) e = launch_variant<256, 16, kOnePass, 4, 2, false, kBalanced>(pl, products, count, stream);
+        else e = launch_variant<256, 32, kOnePass, 4, 2, false, kBalanced>(pl, products, count, stream);
     } else if (running && p.fast_tf32) {
-        e = launch_variant<256, 32, kOnePass, 4, 2, false, kRunningSum>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+        e = launch_variant<256, 32, kOnePass, 4, 2, false, kRunningSum>(pl, products, count, stream);
     } else if (running) {
-        e = launch_variant<256, 16, kThreePass, 8, 2, false, kRunningSum>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+        e = launch_variant<256, 16, kThreePass, 8, 2, false, kRunningSum>(pl, products, count, stream);
     } else if (pl.tail_ways) {
-        if (!p.fast_tf32 && pl.bk == 16) e = launch_variant<256, 16, kThreePass, 8, 2, false, kCutTiles>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
-        else if (!p.fast_tf32) e = launch_variant<256, 32, kThreePass, 8, 2, false, kCutTiles>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
-        else if (pl.bk == 16) e = launch_variant<256, 16, kOnePass, 4, 2, false, kCutTiles>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
-        else e = launch_variant<256, 32, kOnePass, 4, 2, false, kCutTiles>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+        if (!p.fast_tf32 && pl.bk == 16) e = launch_variant<256, 16, kThreePass, 8, 2, false, kCutTiles>(pl, products, count, stream);
+        else if (!p.fast_tf32) e = launch_variant<256, 32, kThreePass, 8, 2, false, kCutTiles>(pl, products, count, stream);
+        else if (pl.bk == 16) e = launch_variant<256, 16, kOnePass, 4, 2, false, kCutTiles>(pl, products, count, stream);
+        else e = launch_variant<256, 32, kOnePass, 4, 2, false, kCutTiles>(pl, products, count, stream);
     } else if (pl.ta) {
-        if (pl.bn == 64 && split_groups == 2) e = launch_variant<64, 32, kThreePass, 8, 1, true, kWholeTiles, 2>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
-        else if (pl.bn == 64) e = launch_variant<64, 32, kThreePass, 8, 1, true>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
-        else if (split_groups == 2) e = launch_variant<128, 32, kThreePass, 8, 1, true, kWholeTiles, 2>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
-        else e = launch_variant<128, 32, kThreePass, 8, 1, true>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);
+        if (pl.bn == 64 && split_groups == 2) e = launch_variant<64, 32, kThreePass, 8, 1, true, kWholeTiles, 2>(pl, products, count, stream);
+        else if (pl.bn == 64) e = launch_variant<64, 32, kThreePass, 8, 1, true>(pl, products, count, stream);
+        else if (split_groups == 2) e = launch_variant<128, 32, kThreePass, 8, 1, true, kWholeTiles, 2>(pl, products, count, stream);
+        else e = launch_variant<128, 32, kThreePass, 8, 1, true>(pl, products, count, stream);
     }
 #define MNI_VARIANT(BN_, BK_)                                                                         \
-    if (!half && pl.cg == 1 && !pl.ta && pl.bn == BN_ && pl.bk == BK_) {                                                 \
-        if (p.fast_tf32) e = launch_variant<BN_, BK_, kOnePass, 4, 1>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);      \
-        else e = launch_variant<BN_, BK_, kThreePass, 8, 1>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);                 \
+    if (pl.cg == 1 && !pl.ta && pl.bn == BN_ && pl.bk == BK_) {                                                 \
+        if (p.fast_tf32) e = launch_variant<BN_, BK_, kOnePass, 4, 1>(pl, products, count, stream);      \
+        else e = launch_variant<BN_, BK_, kThreePass, 8, 1>(pl, products, count, stream);                 \
     }
 #define MNI_PAIR_VARIANT(BN_, BK_)                                                                    \
-    if (!half && pl.cg == 2 && !pl.sk && !pl.tail_ways && !running && pl.bn == BN_ && pl.bk == BK_) {                                                 \
-        if (p.fast_tf32) e = launch_variant<BN_, BK_, kOnePass, 4, 2>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);      \
-        else e = launch_variant<BN_, BK_, kThreePass, 8, 2>(pl, tmA, tmB, tmC, tmD, tmP, k, stream);                 \
+    if (pl.cg == 2 && !pl.sk && !pl.tail_ways && !running && pl.bn == BN_ && pl.bk == BK_) {                                                 \
+        if (p.fast_tf32) e = launch_variant<BN_, BK_, kOnePass, 4, 2>(pl, products, count, stream);      \
+        else e = launch_variant<BN_, BK_, kThreePass, 8, 2>(pl, products, count, stream);                 \
     }
     MNI_PAIR_VARIANT(64, 32) MNI_PAIR_VARIANT(128, 32) MNI_PAIR_VARIANT(256, 16) MNI_PAIR_VARIANT(256, 32)
 #undef MNI_PAIR_VARIANT
@@ -2504,15 +2731,7 @@ int launch_gemm_tc(const GemmProblem &p0, float *partial, uint32_t *err_word, in
 #undef MNI_VARIANT
     if (e != cudaSuccess) return fail(MNI_B200_ERR_CUDA, "gemm_tc_kernel set-up failed: %s", cudaGetErrorString(e));
     MNI_LAUNCH_CHECK("gemm_tc_kernel");
-    if (pl.tail_ways) {
-        if (!defer) return launch_tail_finish(p, pl, k, partial, 0, stream);
-        *defer = [p, pl, k, partial](int dep_mode, cudaStream_t st) { return launch_tail_finish(p, pl, k, partial, dep_mode, st); };
-    } else if (pl.splits > 1) {
-        const SplitFinish f{partial, p.C, p.ldc, p.c_bstride, p.batch, oM, oN, p.bias, p.accumulate, pl.splits};
-        if (!defer) return launch_split_finish(f, 0, stream);
-        *defer = [f](int dep_mode, cudaStream_t st) { return launch_split_finish(f, dep_mode, st); };
-    }
-    return MNI_B200_OK;
+    return launch_finish(p, pl, k, partial, oM, oN, stream, defer);
 }
 
 }  // namespace mni

@@ -185,8 +185,13 @@ int launch_gemm_tc(const GemmProblem &p, float *partial, uint32_t *err_word, int
 bool gemm_tc_uses_pairs(const GemmProblem &p, int sm_count);
 // The plan's cost model for this problem in microseconds (0: the model does not cover it).
 double gemm_tc_estimate_us(const GemmProblem &p, int sm_count);
-// Microseconds of a product: from f32 operands, or from 16-bit planes of them (without the pass that makes those).
-double gemm_estimate_us(const GemmProblem &p, bool half, int sm_count);
+// Microseconds of a product from f32 operands.
+double gemm_estimate_us(const GemmProblem &p, int sm_count);
+// One or two independent products from 16-bit planes (GemmProblem::ha, hb), in one launch.  partial[i] must hold bytes[i].
+int launch_gemm_halves(const GemmProblem *p, int count, float *const *partial, uint32_t *err_word, int sm_count, cudaStream_t stream);
+void gemm_halves_partial_bytes(const GemmProblem *p, int count, int sm_count, size_t *bytes);
+double gemm_halves_estimate_us(const GemmProblem *p, int count, int sm_count);     // without the pass that makes the planes
+void gemm_halves_describe(const GemmProblem *p, int count, int sm_count, std::string *lines);
 // One line of text naming the kernel variant, tiling, split and grid launch_gemm_tc would use for this problem
 // on a device with `sm_count` SMs.  Pure host arithmetic: touches no device.
 std::string gemm_tc_describe(const GemmProblem &p, int sm_count);
