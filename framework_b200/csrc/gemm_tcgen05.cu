@@ -690,7 +690,6 @@ gemm_tc_kernel(const __grid_constant__ Products<product_slots(MODE)> g) {
         bool ok = true;
         long long waited = 0, t_ld = 0, t_wg = 0;
         const int my_cta = static_cast<int>(blockIdx.x);                 // slot * CG + rank in the pair
-        bool any_tma = false;
         for (int prod = 0; ok && prod < products; ++prod) {
         const Product &w = g.s[HALF ? prod : 0];
         const KParams &q = HALF ? w.p : p;
@@ -701,7 +700,6 @@ gemm_tc_kernel(const __grid_constant__ Products<product_slots(MODE)> g) {
             unscale = __uint_as_float(static_cast<uint32_t>(127 - ea - eb) << 23);
         }
         const bool use_tma = q.epi_mode == kEpiTmaStore || q.epi_mode == kEpiTmaReduce;
-        any_tma |= use_tma;
         const bool bias_vec = (reinterpret_cast<uintptr_t>(q.bias) & 15) == 0;
         WorkIter wi = work_begin(q, first_unit(prod), unit_step);
         TileCoord t;
@@ -1088,7 +1086,7 @@ gemm_tc_kernel(const __grid_constant__ Products<product_slots(MODE)> g) {
         }
         // The staging patches must have been read before the CTA gives up its shared memory; the global
         // writes themselves complete with the grid like any other store.
-        if ((any_tma || CUT) && lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
         if (p.prof && warp == EPI0 && lane == 0) {
             atomicAdd(p.prof + 4, static_cast<unsigned long long>(waited));
             atomicAdd(p.prof + 7, static_cast<unsigned long long>(t_wg));
@@ -1170,12 +1168,12 @@ gemm_tc_kernel(const __grid_constant__ Products<product_slots(MODE)> g) {
                     if (elect_one()) {
                         mbar_arrive_expect_tx(full, A_BYTES + static_cast<uint32_t>(q.b_rows_live) * BK * 4u);
                         if (armed != p.withhold_at) {        // test hook: a stage that is armed and never filled
-                            load_operand(a_mode, dstA, &w.A, full, k0, rowA, BM / 32, CHUNK_BYTES, a0, a1, a2);
-                            load_operand(b_mode, dstA + A_BYTES, &w.B, full, k0, rowB, BNL / 32, CHUNK_BYTES, b0, b1, b2);
+                            load_operand(q.a_mode, dstA, &w.A, full, k0, rowA, BM / 32, CHUNK_BYTES, a0, a1, a2);
+                            load_operand(q.b_mode, dstA + A_BYTES, &w.B, full, k0, rowB, BNL / 32, CHUNK_BYTES, b0, b1, b2);
                         }
                     }
                     if (++stage == p.stages) { stage = 0; phase ^= 1u; dstA = dstA0; } else { dstA += STAGE_BYTES; }
-                    if (++kk == kiters) {
+                    if (++kk == q.kiters) {
                         kk = 0;
                         ++f;
                         if (q.fold > 1) {
