@@ -524,7 +524,7 @@ int make_halves(Call &c, std::initializer_list<const mni_b200_view *> views, Hal
     }
     h.planes = (c.flags & MNI_B200_PRECISION_TF32) != 0 ? 2 : 3;
     h.blocks = half_blocks(h.view, h.count, c.st->sm_count);
-    const size_t words = static_cast<size_t>(h.blocks) + kMaxHalves, head = c.arena.reserve(4 * words);
+    const size_t words = static_cast<size_t>(h.blocks) + 1 + kMaxHalves, head = c.arena.reserve(4 * words);
     size_t at[kMaxHalves];
     for (int i = 0; i < h.count; ++i) at[i] = c.arena.reserve(static_cast<size_t>(h.view[i].plane) * 2 * h.planes);
     const size_t sums_at = sums_out ? c.arena.reserve(half_columns_bytes(h.view[0], h.blocks)) : 0;
@@ -534,7 +534,7 @@ int make_halves(Call &c, std::initializer_list<const mni_b200_view *> views, Hal
     h.status = reinterpret_cast<unsigned int *>(c.at(head));
     for (int i = 0; i < h.count; ++i) {
         h.view[i].dst = c.at(at[i]);
-        h.view[i].exp = reinterpret_cast<int *>(h.status + h.blocks + i);
+        h.view[i].exp = reinterpret_cast<int *>(h.status + h.blocks + 1 + i);
     }
     HalfColumns sums;
     if (sums_out) sums = HalfColumns{c.at(sums_at), sums_out, accumulate ? 1 : 0};
@@ -546,8 +546,7 @@ int run_halves(Call &c, GemmProblem *p, int count, const Halves &h, const HalfOp
     for (int i = 0; i < count; ++i) {
         p[i].ha = &x[i];
         p[i].hb = &y[i];
-        p[i].half_status = h.status;
-        p[i].half_statuses = h.blocks;
+        p[i].half_status = h.status + h.blocks;
         p[i].fast_tf32 = (c.flags & MNI_B200_PRECISION_TF32) != 0;
     }
     size_t bytes[2] = {0, 0};

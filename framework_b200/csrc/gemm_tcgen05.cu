@@ -135,8 +135,7 @@ struct KParams {
     unsigned int *sk_flags;    // ready flags [cta][2][epilogue warp] (1 = parked), then tickets [tile][rank][epilogue warp]
     // 16-bit halves: what split_half_kernel left beside them
     const int *a_exp, *b_exp;              // the operands were multiplied by 2^exponent
-    const unsigned int *half_status;       // a word per block of it: != 0, some operand's range does not fit
-    int half_statuses;
+    const unsigned int *half_status;       // bit 0: some operand's range did not fit
 };
 
 // What a launch computes: one product, or (16-bit planes) two that need nothing from each other, the units of the second dealt
@@ -660,10 +659,9 @@ gemm_tc_kernel(const __grid_constant__ Products<product_slots(MODE)> g) {
     // HALF: wide if some operand's range did not fit f16, and the planes hold bf16 thirds, unscaled.
     bool wide = false, huge = false;
     if constexpr (HALF) {
-        unsigned int status = 0;
-        for (int i = threadIdx.x; i < p.half_statuses; i += blockDim.x) status |= __ldcg(p.half_status + i);
-        wide = __syncthreads_or(status & 1u) != 0;
-        if (wide) huge = __syncthreads_or(status & 2u) != 0;
+        const unsigned int status = __ldcg(p.half_status);
+        wide = (status & 1u) != 0;
+        huge = (status & 2u) != 0;
     }
     // The products of the launch, as every role walks them: first_unit is this CTA pair's first unit of one.
     const int products = HALF ? g.count : 1;
@@ -2580,7 +2578,6 @@ static int make_product(const GemmProblem &p, const Plan &pl, bool transposed, i
         k.a_exp = p.ha->exp;
         k.b_exp = p.hb->exp;
         k.half_status = p.half_status;
-        k.half_statuses = p.half_statuses;
     }
     k.C = p.C;
     k.ldc = p.ldc;

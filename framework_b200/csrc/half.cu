@@ -44,6 +44,7 @@ struct ViewList {
     int count, tiles;
     unsigned int *status;
     int statuses;                       // = blocks of split_half_kernel
+    unsigned int *verdict;              // all of them in one word, for the products
     HalfColumns sums;                   // of the first view
 };
 
@@ -270,8 +271,9 @@ split_wide_kernel(const __grid_constant__ ViewList list) {
             __syncthreads();
         }
     }
-    if (!__syncthreads_or(status & kUnfit)) return;
-    const bool huge = __syncthreads_or(status & kHuge);
+    const bool unfit = __syncthreads_or(status & kUnfit), huge = __syncthreads_or(status & kHuge);
+    if (blockIdx.x == 0 && threadIdx.x == 0) *list.verdict = (unfit ? kUnfit : 0u) | (huge ? kHuge : 0u);
+    if (!unfit) return;
     for (int tile = blockIdx.x; tile < list.tiles; tile += gridDim.x) {
         int at = 0;
         while (at + 1 < list.count && tile >= list.v[at + 1].first_tile) ++at;
@@ -325,6 +327,7 @@ int launch_split_half(const HalfView *views, int count, int planes, unsigned int
     list.count = count;
     list.status = status;
     list.statuses = blocks;
+    list.verdict = status + blocks;
     list.sums = sums;
     long long tiles = 0;
     for (int i = 0; i < count; ++i) {

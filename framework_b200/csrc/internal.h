@@ -165,10 +165,9 @@ struct GemmProblem {
     int flag_bank = 0;             // 1 for launches on the library's side stream: their own set of balanced-tail flags
     // Optional second output D = gelu(C + bias) written by the same epilogue (C itself is skipped if null).
     float *D = nullptr;
-    // The operands in 16-bit planes (A and B are not read then) and the status words of the kernel that made them.
+    // The operands in 16-bit planes (A and B are not read then) and the status word of the launch that made them.
     const HalfOperand *ha = nullptr, *hb = nullptr;
     const unsigned int *half_status = nullptr;
-    int half_statuses = 0;
 };
 
 // Bytes of split-K partial storage launch_gemm_tc would use for this problem (0 if none).
@@ -301,7 +300,8 @@ struct HalfView {
     int *exp;                      // on the device: the exponent the values were multiplied by
 };
 constexpr int kMaxHalves = 3;
-int half_blocks(const HalfView *views, int count, int sm_count);      // blocks of the first launch, and its status words
+int half_blocks(const HalfView *views, int count, int sm_count);      // blocks of the launches
+// status: a word per block, and one for all of them behind those (bit 0: the planes are bf16, bit 1: see half_wide_exponent)
 // Column sums of the first view's rows, for the bias gradient (out null: none).
 struct HalfColumns {
     float *partial = nullptr, *out = nullptr;
