@@ -877,7 +877,7 @@ bool bwd_half_wanted(const Call &c, const Shapes &s, const mni_b200_view &a, con
         p.fast_tf32 = (c.flags & MNI_B200_PRECISION_TF32) != 0;
         f32_us += gemm_estimate_us(p, all);
         gathers_us += gather_us(other);
-        beside_us = std::max(beside_us, (p.fast_tf32 ? 1.25 : 1.1) * gemm_estimate_us(p, halved));   // they slow one another down
+        beside_us = std::max(beside_us, 1.25 * gemm_estimate_us(p, halved));   // beside one another they are that much slower
         elements += static_cast<double>(prod(other.shape, other.ndim));
         return true;
     };
