@@ -38,6 +38,7 @@ struct DeviceState {
     uint8_t *ws = nullptr;        // library-owned scratch
     size_t ws_bytes = 0;
     bool ws_recorded = false;     // some graph holds its address
+    size_t refused = SIZE_MAX;    // the least that could not be had for 16-bit planes: not tried again until mni_b200_release
     std::vector<uint8_t *> retired;   // scratch outgrown since, kept for the graphs that hold its address (mni_b200_release frees it)
     uint8_t *user_ws = nullptr;   // caller-provided scratch (takes precedence)
     size_t user_bytes = 0;
@@ -1234,10 +1235,15 @@ int with_scratch(uint32_t flags, void *stream, Body body) {
         if (rc) return rc;
         sized = dry.arena.used;
         if (sized == 0) break;
+        if (dry.used_half && !st->user_ws && sized >= st->refused && sized > st->ws_bytes) {
+            real.no_half = true;
+            continue;
+        }
         rc = scratch_base(*st, sized, real.stream, &real.base);
         if (rc == MNI_B200_OK) break;
-        // Scratch for the operands' halves cannot be had: the call goes without them, as it needs little or none then.
+        // Scratch for the operands' planes cannot be had: the call goes without them, as it needs little or none then.
         if (!dry.used_half || real.no_half) return rc;
+        if (!st->user_ws && !capturing) st->refused = sized;      // (growing frees and allocates: not on every call)
         real.no_half = true;
     }
     rc = body(real);
@@ -1670,6 +1676,7 @@ int mni_b200_release(void) {
     int rc = device_state(&st);
     if (rc) return rc;
     std::lock_guard<std::mutex> lock(st->mu);
+    st->refused = SIZE_MAX;
     if (st->ws || !st->retired.empty()) MNI_CUDA(cudaDeviceSynchronize());
     if (st->ws) {
         MNI_CUDA(cudaFree(st->ws));

@@ -1182,7 +1182,7 @@ gemm_tc_kernel(const __grid_constant__ Products<product_slots(MODE)> g) {
                 }
             }
             }
-            if (!ok && loads_a) {
+            if (!ok) {
                 // Aborting: let the copies already issued land before the CTA exits.
                 const int pending = min(armed, p.stages);
                 for (int i = 0; i < pending; ++i) {

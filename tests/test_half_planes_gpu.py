@@ -52,8 +52,10 @@ def test_forward_and_gradients(F, planes, m, k, n, batch, shared, bt, single):
     flags = F._lib.PRECISION_TF32 if single else 0
     y = Guarded(F, batch + (m, n), init=np.ones(batch + (m, n), np.float32))
     F.matmul(t(x), dw_view, t(bias), out=y.tensor, flags=flags | F._lib.ACCUMULATE_C)
-    da, db, dbias = Guarded(F, batch + (m, k)), Guarded(F, wb + (k, n)), Guarded(F, (n,))
-    F.matmul_backward(t(dy), t(x), dw_view, want_dbias=True, da=da.tensor, db=db.tensor, dbias=dbias.tensor, flags=flags)
+    add = bt                                      # one of the two layouts accumulates onto ones
+    da, db, dbias = (Guarded(F, s, init=np.ones(s, np.float32) if add else None) for s in (batch + (m, k), wb + (k, n), (n,)))
+    F.matmul_backward(t(dy), t(x), dw_view, want_dbias=True, da=da.tensor, db=db.tensor, dbias=dbias.tensor,
+                      flags=flags | (F._lib.ACCUMULATE_DA | F._lib.ACCUMULATE_DB | F._lib.ACCUMULATE_DBIAS if add else 0))
     F.device_status()
     product = x.double() @ wv.double()
     want = {"y": product + bias.double() + 1, "da": dy.double() @ wv.double().transpose(-1, -2),
@@ -62,8 +64,8 @@ def test_forward_and_gradients(F, planes, m, k, n, batch, shared, bt, single):
         want["db"] = want["db"].sum(tuple(range(len(batch))))
     fold = int(np.prod(batch)) if shared else 1
     for got, name, length in ((y, "y", k), (da, "da", n), (db, "db", m * fold), (dbias, "dbias", 0)):
-        got.check(name, fully_written=name != "y")
-        assert rel_fro(got.tensor.numpy(), want[name].cpu().numpy()) <= (1e-6 if name == "dbias" else _bound(length, single)), name
+        got.check(name, fully_written=name != "y" and not add)
+        assert rel_fro(got.tensor.numpy(), want[name].cpu().numpy() + (1 if add and name != "y" else 0)) <= (1e-6 if name == "dbias" else _bound(length, single)), name
 
 
 @pytest.mark.parametrize("n,misalign,want_pre", [(512, 0, True), (512, 0, False), (500, 0, True), (501, 1, True)])
@@ -184,3 +186,23 @@ def test_queried_scratch_holds_the_planes(F, planes):
     finally:
         F._lib.check(lib.mni_b200_workspace_set(None, 0))
     assert bool((buf[base - buf.data_ptr() + need.value:] == 0x5A).all())
+
+
+@pytest.mark.parametrize("flags", [0, 1])
+def test_wait_limit_runs_out_then_the_library_recovers(F, planes, monkeypatch, flags):
+    """As test_timeout_gpu.py does for the other variants: a stage that is armed and never filled."""
+    rng = np.random.default_rng(5)
+    a, b = (rng.standard_normal((512, 512), dtype=np.float32) for _ in range(2))
+    ad, bd = F.DeviceTensor.from_numpy(a), F.DeviceTensor.from_numpy(b)
+    F.device_status()
+    monkeypatch.setenv("MNI_B200_WAIT_CYCLES", "2000000")
+    monkeypatch.setenv("MNI_B200_TEST_WITHHOLD_KBLOCK", "3")
+    F.matmul(ad, bd, flags=flags)
+    with pytest.raises(F._lib.MniError) as ei:
+        F.device_status()
+    assert ei.value.status == 8
+    monkeypatch.delenv("MNI_B200_TEST_WITHHOLD_KBLOCK")
+    monkeypatch.delenv("MNI_B200_WAIT_CYCLES")
+    out = F.matmul(ad, bd, flags=flags)
+    assert F.device_status() == 0
+    assert rel_fro(out.numpy(), a.astype(np.float64) @ b) <= _bound(512, flags == 1)
