@@ -34,10 +34,10 @@
 //               tensor memory.  The epilogue takes both into its registers and the next unit begins; the large terms' chain is a
 //               third as long as in 3xTF32, and its rounding a sixth (1.24e-6 -> 3.5e-7 at K = 512, 7.6e-6 -> 1.25e-6 at 2048
 //               to 3072), so a piece may be 4096 long.  Bound by the power cap in a loop, by L2 (16 KB a CTA and 16 elements) at
-//               full clocks.  8192^3: 24.9 cycles per element of a tile for the pipe's 24, 3.7 -> 2.4 ms a product with the pass
-//               over the operands; as one accumulator with hi staged a second time, 33 cycles and 2.8 ms (L2).
-//   kHalfOne    hi*hi alone, accumulators double-buffered as in single-pass TF32: 10 cycles for the pipe's 8 (L2: 8 KB a CTA and
-//               16 elements), 1.9 -> 1.2 ms.
+//               full clocks.  8192^3: 24.4 cycles per element of a tile for the pipe's 24, 4.0 -> 2.5 ms a product with the pass
+//               over the operands, in a loop; as one accumulator with hi staged a second time, 33 cycles (L2).
+//   kHalfOne    hi*hi alone, accumulators double-buffered as in single-pass TF32: 9.4 cycles for the pipe's 8 (L2: 8 KB a CTA and
+//               16 elements), 1.8 -> 0.96 ms.
 // Operands whose range f16 does not hold come as three (two) bf16 planes through the same stages.
 //
 // CG = 2: two CTAs of a cluster share a 256 x BN tile (cta_group::2 MMAs issued by the leader).
