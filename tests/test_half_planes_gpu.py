@@ -206,3 +206,25 @@ def test_wait_limit_runs_out_then_the_library_recovers(F, planes, monkeypatch, f
     out = F.matmul(ad, bd, flags=flags)
     assert F.device_status() == 0
     assert rel_fro(out.numpy(), a.astype(np.float64) @ b) <= _bound(512, flags == 1)
+
+
+def test_replayed_graph_looks_at_the_values_each_time(F, planes):
+    """Scale and range are found on the device: a graph replayed with other values in the same buffers is right for those."""
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(8)
+    x, w = torch.randn(300, 500, generator=gen, device="cuda"), torch.randn(500, 400, generator=gen, device="cuda")
+    xt, wt, out = F.DeviceTensor.from_torch(x), F.DeviceTensor.from_torch(w), F.DeviceTensor.empty((300, 400))
+    F.matmul(xt, wt, out=out)                        # scratch
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            F.matmul(xt, wt, out=out)
+    first = x.clone()
+    spread = torch.logspace(-15, 10, 500, device="cuda")
+    for value in (first, first * 1e-20, first * spread, first * 1e25, first):
+        x.copy_(value)
+        graph.replay()
+        F.device_status()
+        want = x.double() @ w.double()
+        assert float((out.torch_view().double() - want).norm() / want.norm()) <= _bound(500)
