@@ -194,6 +194,11 @@ skinny_fwd_kernel(const float *__restrict__ x, long long ldx, const float *__res
 // register file, so a thread can keep 16 accumulator vectors (16 rows of x) and still have 192 bytes
 // on their way; and a k-group's chain of dependent DRAM round trips shrinks from one per batch to the
 // ring's fill.  No thread reads another thread's ring slots, so the loop needs no block barrier.
+// Weights of this many elements and more are asked into L2 before the kernel before has ended: the first rows of a block, what
+// its ring takes first.  us with three weights in turn, without / 4 / 12 / 24 / 64 rows: 1 x 4096 x 4096 14.1 / 13.8 / 13.5 / 13.5 / 14.1,
+// 8 rows 17.0 / 16.4 / 16.2 / 16.6 / 17.6, 8 x 8192 x 2048 18.7 / 18.1 / 17.1 / 17.5 / 18.7.  Smaller ones may be there already: 1 x 1000 x
+// 5000 8.4 / 8.8 (12 rows).
+constexpr int64_t kEarlyWeight = 1 << 23;
 constexpr int kRingThreads = 256;                           // COLS column-threads x GROUPS k-groups
 constexpr int kRingBatch = 4;                               // rows of W per cp.async group
 // Measured at K = N = 4096 (1 / 8 rows): 8 groups x 4 batches 15.4 / 18.7 us; 4 groups 17.0 / 20.1; 2 groups
@@ -210,7 +215,7 @@ __global__ void __launch_bounds__(kRingThreads, 2)
 skinny_fwd_ring_kernel(const float *__restrict__ x, long long ldx, const float *__restrict__ W, long long ldw,
                        float *__restrict__ partial, float *__restrict__ y, long long ldy,
                        const float *__restrict__ bias, int accumulate, int M, long long N, long long K, int k_per,
-                       int x_vec, int cluster) {
+                       int x_vec, int cluster, int early) {
     extern __shared__ __align__(16) float smem_f[];
     grid_dependency_trigger();
     float *xs = smem_f;                                                  // [MT][k_per], zero beyond M / K
@@ -239,6 +244,11 @@ skinny_fwd_ring_kernel(const float *__restrict__ x, long long ldx, const float *
         }
         cp_async_commit();                                               // empty groups keep the count uniform
     };
+    // A prefetch reads nothing, so W may be what the kernel before writes.  One lane per 128-byte line.
+    if (early && live && (threadIdx.x & 7) == 0) {
+        for (int r = g0; r < min(g0 + AHEAD * kRingBatch, min(kc, g0 + rpg)); ++r)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(wp + static_cast<long long>(r) * ldw));
+    }
     grid_dependency_wait();
     // The x slice goes first and asynchronously as well (16-byte pieces, zero-filled beyond M rows / kc
     // columns): staged with ordinary loads its 4 * MT * k_per bytes cost one L2 round trip per few elements
@@ -748,13 +758,14 @@ int launch_skinny_fwd(const float *x, int64_t ldx, const float *W, int64_t ldw, 
         cfg.numAttrs = pl.cluster ? 2 : 1;
         const int acc_i = accumulate ? 1 : 0, m_i = static_cast<int>(M), kper_i = static_cast<int>(pl.k_per);
         const int xvec_i = x_vec ? 1 : 0, cluster_i = pl.cluster ? 1 : 0;
+        const int early_i = N * K >= kEarlyWeight ? 1 : 0;
         const long long ldx_l = ldx, ldw_l = ldw, ldy_l = ldy, n_l = N, k_l = K;
 #define MNI_SKINNY_RING(MT)                                                                            \
     case MT:                                                                                           \
         cudaFuncSetAttribute(skinny_fwd_ring_kernel<MT, kRingGroups, kRingDepth>,                      \
                              cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024);                 \
         cudaLaunchKernelEx(&cfg, skinny_fwd_ring_kernel<MT, kRingGroups, kRingDepth>, x, ldx_l, W, ldw_l, partial, \
-                           y, ldy_l, bias, acc_i, m_i, n_l, k_l, kper_i, xvec_i, cluster_i);           \
+                           y, ldy_l, bias, acc_i, m_i, n_l, k_l, kper_i, xvec_i, cluster_i, early_i);  \
         break;
         switch (mt) {
             MNI_SKINNY_RING(1) MNI_SKINNY_RING(2) MNI_SKINNY_RING(4) MNI_SKINNY_RING(8) MNI_SKINNY_RING(16)

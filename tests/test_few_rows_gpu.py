@@ -82,3 +82,22 @@ def test_weight_gradient_of_more_slabs_than_a_grid_has(F):
     got = dw.tensor.storage.double()
     assert float((got - want).norm() / want.norm()) <= regression_bound_3xtf32(9)
     assert float((got - want)[-600:].abs().max()) <= 1e-5
+
+
+@pytest.mark.parametrize("m,k,n", [(1, 4096, 2044), (1, 4096, 2048), (5, 2099, 4000), (8, 65, 129060), (3, 16421, 516)])
+def test_weight_written_by_the_kernel_before(F, m, k, n):
+    """A long weight's first rows are asked into L2 before the kernel before has ended; what that kernel writes there is what the
+    product reads.  Sizes on both sides of the rule, ragged slices and strips."""
+    rng = np.random.default_rng([m, k, n])
+    x = rng.standard_normal((m, k)).astype(np.float32)
+    t = F.DeviceTensor.from_numpy
+    xd, w, y = t(x), F.DeviceTensor.empty((k, n)), Guarded(F, (m, n))
+    for turn in range(4):
+        u, v = rng.standard_normal((k, 3)).astype(np.float32), rng.standard_normal((3, n)).astype(np.float32)
+        ud, vd = t(u), t(v)
+        F.matmul(ud, vd, out=w)
+        F.matmul(xd, w, out=y.tensor)
+        F.device_status()
+        y.check(fully_written=True)
+        want = x.astype(np.float64) @ w.numpy().astype(np.float64)
+        assert rel_fro(y.tensor.numpy(), want) <= regression_bound_3xtf32(k), turn
