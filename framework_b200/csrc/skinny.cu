@@ -476,16 +476,23 @@ skinny_dw_kernel(const float *__restrict__ x, long long ldx, const float *__rest
 // L1/L2) and a shuffle tree folds the 32 lane sums.  W is read exactly once.
 constexpr int kDxThreads = 256;
 constexpr int kDxRows = 2;
-// FULL: M == MT and N a multiple of 512, so the loop carries no bounds tests and the compiler can issue
-// all 8 weight loads and all 4 * MT dy loads of a step before the first multiply.
-template <int MT, bool FULL>
-__global__ void __launch_bounds__(kDxThreads)
+// The rows of dy are a template argument and the steps of 512 columns of LONG rows carry no bounds tests, so that all loads of a
+// step are under way before its first multiply; what is left of a row is a step of its own.  With a test per row and position
+// the loads waited for the multiplies between them.  us with three weights in turn, before / now: 4096 x 4096 at 1 / 2 / 3 /
+// 4 / 5 rows 12.5 / 15.6 / 21.6 / 20.3 / 22.9 -> 10.6 / 11.9 / 12.0 / 12.3 / 13.0, 8192 x 8192 at 4 rows 69 -> 41.5.  (The next
+// step's weights loaded one step early: 11.7 / 12.3 / 12.9 / 13.0 / 14.5; bounds of three blocks per SM spill.)
+template <int MT, bool LONG>
+__global__ void __launch_bounds__(kDxThreads, LONG ? 2 : 1)
 skinny_dx_kernel(const float *__restrict__ dy, long long lddy, const float *__restrict__ W, long long ldw,
-                 float *__restrict__ dx, long long lddx, int accumulate, int M, long long N, long long K) {
+                 float *__restrict__ dx, long long lddx, int accumulate, long long N, long long K, int early) {
     grid_dependency_trigger();
     const int lane = threadIdx.x & 31;
     const long long gw = static_cast<long long>(blockIdx.x) * (kDxThreads / 32) + (threadIdx.x >> 5);
     const long long k0 = gw * kDxRows;
+    constexpr int P = 4;                                   // 128-float positions per step: 4 KB of weight per warp
+    // the first step's lines, as in the forward above
+    if (LONG && early && k0 + (lane >> 4) < K && (lane & 15) * 32 < N)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(W + (k0 + (lane >> 4)) * ldw + (lane & 15) * 32));
     grid_dependency_wait();
     if (k0 >= K) return;
     float acc[kDxRows][MT];
@@ -494,36 +501,48 @@ skinny_dx_kernel(const float *__restrict__ dy, long long lddy, const float *__re
 #pragma unroll
         for (int m = 0; m < MT; ++m) acc[r][m] = 0.f;
     const float *w0 = W + k0 * ldw;
-    const bool row1 = k0 + 1 < K;
-    const float *w1 = row1 ? w0 + ldw : w0;
-    // 512 floats of both rows per step: eight 16-byte weight loads in flight per lane (4 KB per warp),
-    // enough outstanding bytes per SM to keep HBM busy with 16 resident warps.
-    constexpr int P = 4;                                   // 128-float positions per step
-    for (long long n = lane * 4; n < N; n += 128 * P) {
-        float4 wa[P], wb[P];
+    const float *w1 = k0 + 1 < K ? w0 + ldw : w0;
+    struct Step { float4 a[P], b[P]; };
+    auto load = [&](Step &w, long long n) {
 #pragma unroll
         for (int q = 0; q < P; ++q) {
-            const long long nq = n + 128 * q;
-            if (FULL || nq < N) {
-                wa[q] = __ldcs(reinterpret_cast<const float4 *>(w0 + nq));
-                wb[q] = __ldcs(reinterpret_cast<const float4 *>(w1 + nq));
-            } else {
-                wa[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-                wb[q] = wa[q];
+            w.a[q] = __ldcs(reinterpret_cast<const float4 *>(w0 + n + 128 * q));
+            w.b[q] = __ldcs(reinterpret_cast<const float4 *>(w1 + n + 128 * q));
+        }
+    };
+    auto add = [&](const float4 &a, const float4 &b, int m, long long n) {
+        const float4 g = __ldg(reinterpret_cast<const float4 *>(dy + m * lddy + n));
+        acc[0][m] = fmaf(g.x, a.x, fmaf(g.y, a.y, fmaf(g.z, a.z, fmaf(g.w, a.w, acc[0][m]))));
+        acc[1][m] = fmaf(g.x, b.x, fmaf(g.y, b.y, fmaf(g.z, b.z, fmaf(g.w, b.w, acc[1][m]))));
+    };
+    auto multiply = [&](const Step &w, long long n) {
+#pragma unroll
+        for (int m = 0; m < MT; ++m)
+#pragma unroll
+            for (int q = 0; q < P; ++q) add(w.a[q], w.b[q], m, n + 128 * q);
+    };
+    long long n = lane * 4;
+    Step w;
+    if (LONG) {
+        const int steps = static_cast<int>(N / (128 * P));
+        for (int s = 0; s < steps; ++s, n += 128 * P) {
+            load(w, n);
+            multiply(w, n);
+        }
+    }
+    for (; n < N; n = LONG ? N : n + 128 * P) {            // LONG rows have one such step
+#pragma unroll
+        for (int q = 0; q < P; ++q) {
+            if (n + 128 * q < N) {
+                w.a[q] = __ldcs(reinterpret_cast<const float4 *>(w0 + n + 128 * q));
+                w.b[q] = __ldcs(reinterpret_cast<const float4 *>(w1 + n + 128 * q));
             }
         }
 #pragma unroll
-        for (int m = 0; m < MT; ++m) {
-            if (FULL || m < M) {
+        for (int q = 0; q < P; ++q) {
+            if (n + 128 * q < N) {
 #pragma unroll
-                for (int q = 0; q < P; ++q) {
-                    const long long nq = n + 128 * q;
-                    if (FULL || nq < N) {
-                        const float4 g = __ldg(reinterpret_cast<const float4 *>(dy + m * lddy + nq));
-                        acc[0][m] = fmaf(g.x, wa[q].x, fmaf(g.y, wa[q].y, fmaf(g.z, wa[q].z, fmaf(g.w, wa[q].w, acc[0][m]))));
-                        acc[1][m] = fmaf(g.x, wb[q].x, fmaf(g.y, wb[q].y, fmaf(g.z, wb[q].z, fmaf(g.w, wb[q].w, acc[1][m]))));
-                    }
-                }
+                for (int m = 0; m < MT; ++m) add(w.a[q], w.b[q], m, n + 128 * q);
             }
         }
     }
@@ -534,7 +553,7 @@ skinny_dx_kernel(const float *__restrict__ dy, long long lddy, const float *__re
             float v = acc[r][m];
 #pragma unroll
             for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-            if (lane == 0 && m < M && k0 + r < K) {
+            if (lane == 0 && k0 + r < K) {
                 float *dst = dx + m * lddx + k0 + r;
                 *dst = accumulate ? *dst + v : v;
             }
@@ -824,15 +843,24 @@ int launch_skinny_dx(const float *dy, int64_t lddy, const float *W, int64_t ldw,
     }
     const long long rows_per_block = (kDxThreads / 32) * kDxRows;
     const unsigned blocks = static_cast<unsigned>((K + rows_per_block - 1) / rows_per_block);
-    const bool full = M == mt && mt >= 4 && N % 512 == 0;   // measured: slower than the guarded loop for 1-2 rows
+    // One row against short weight rows, or two against very short ones, keep the tested loop, which takes fewer registers: there
+    // more blocks per SM count.  1 row, tested / not: 16384 x 600 8.3 / 9.4 us, 8192 x 1000 5.6 / 6.0, 20000 x 100 3.7 / 4.1;
+    // 2 rows: 20000 x 100 4.3 / 5.2, 16384 x 600 11.3 / 10.2, 8192 x 1000 7.9 / 6.3.
+    const bool whole = M > 2 || N >= (M == 1 ? 2048 : 512);
+    const int early = N * K >= kEarlyWeight ? 1 : 0;
     cudaError_t e = cudaErrorInvalidValue;
-#define MNI_SKINNY_DX(MT)                                                                              \
-    case MT:                                                                                           \
-        e = launch_dependent(dependent, full ? skinny_dx_kernel<MT, true> : skinny_dx_kernel<MT, false>, dim3(blocks), \
-                             dim3(kDxThreads), 0, stream, dy, lddy, W, ldw, dx, lddx, accumulate ? 1 : 0, static_cast<int>(M), N, K); \
-        break;
-    switch (mt) {
-        MNI_SKINNY_DX(1) MNI_SKINNY_DX(2) MNI_SKINNY_DX(4) MNI_SKINNY_DX(8)
+#define MNI_SKINNY_DX(MT, LONG)                                                                        \
+    e = launch_dependent(dependent, skinny_dx_kernel<MT, LONG>, dim3(blocks), dim3(kDxThreads), 0, stream, dy, lddy, W, ldw, \
+                         dx, lddx, accumulate ? 1 : 0, N, K, early)
+    switch (M) {
+        case 1: if (whole) MNI_SKINNY_DX(1, true); else MNI_SKINNY_DX(1, false); break;
+        case 2: if (whole) MNI_SKINNY_DX(2, true); else MNI_SKINNY_DX(2, false); break;
+        case 3: MNI_SKINNY_DX(3, true); break;
+        case 4: MNI_SKINNY_DX(4, true); break;
+        case 5: MNI_SKINNY_DX(5, true); break;
+        case 6: MNI_SKINNY_DX(6, true); break;
+        case 7: MNI_SKINNY_DX(7, true); break;
+        case 8: MNI_SKINNY_DX(8, true); break;
         default: return fail(MNI_B200_ERR_ARG, "skinny dx handles at most 8 rows");
     }
 #undef MNI_SKINNY_DX

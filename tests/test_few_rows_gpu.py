@@ -101,3 +101,21 @@ def test_weight_written_by_the_kernel_before(F, m, k, n):
         y.check(fully_written=True)
         want = x.astype(np.float64) @ w.numpy().astype(np.float64)
         assert rel_fro(y.tensor.numpy(), want) <= regression_bound_3xtf32(k), turn
+
+
+@pytest.mark.parametrize("k,n", [(4097, 2048), (33, 2052), (35, 508), (31, 516), (2, 2044), (16, 4), (2100, 4100)])
+@pytest.mark.parametrize("m", range(1, 9))
+def test_input_gradient_steps_and_what_is_left_of_a_row(F, m, k, n):
+    """Each row count's own kernel: whole steps of 512 columns, none, a last part; odd weight rows; short and long rows."""
+    rng = np.random.default_rng([m, k, n])
+    x, dy, w = (rng.standard_normal(s).astype(np.float32) for s in ((m, k), (m, n), (k, n)))
+    t = F.DeviceTensor.from_numpy
+    c = rng.standard_normal((m, k)).astype(np.float32)
+    for accumulate in (False, True):
+        dx = Guarded(F, (m, k), init=c if accumulate else None)
+        flags = F._lib.FORCE_SKINNY_PATH | (F._lib.ACCUMULATE_DA if accumulate else 0)
+        F.matmul_backward(t(dy), t(x), t(w), da=dx.tensor, need_db=False, flags=flags)
+        F.device_status()
+        dx.check(fully_written=not accumulate)
+        want = dy.astype(np.float64) @ w.astype(np.float64).T + (c if accumulate else 0)
+        assert rel_fro(dx.tensor.numpy(), want) <= regression_bound_3xtf32(n), accumulate
