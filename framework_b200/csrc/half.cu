@@ -2,13 +2,16 @@
 // eleven significant bits: x * 2^e = hi + lo * 2^-12 with hi and lo in f16, e chosen for the whole operand.
 //
 // e comes from 1024 sampled elements, so one pass over the operand is enough; the largest sample lands in [2^6, 2^7).  Above it
-// there is room for elements 256 times as large, below it every element of at least 2^-21 of it keeps 22 bits.  What f16 does not
-// hold is found by the same pass and reported in the block's status word; a second kernel then writes three bf16 planes, whose
-// range is that of f32, and the products take those:
+// there is room for elements 256 times as large, below it every element of at least 2^-14, which is 2^-20 of it or less, keeps 22
+// bits (11 where there is no lo).  What f16 does not hold is found by the same pass and reported in the block's status word; a
+// second kernel then writes three bf16 planes, whose range is that of f32, and the products take those:
 //   - an element beyond 2^15 after scaling, an infinity or a NaN;
-//   - a stretch of a row or of a column (256 elements, 32 elements) that consists of smaller elements than that, zeros aside: in
-//     its row or column of the product the bits they lose would be the leading ones;
-//   - a tile in which more than a sixteenth of the elements are that small.
+//   - a stretch of a row (256 elements) or of a column (what a block takes of it) in which more than a fifth of the elements are
+//     smaller than 2^-14, zeros not counted: in its row or column of the product the bits they lose could be the leading ones,
+//     where the stretch has nothing else as well as where the rest of it meets zeros.
+// So a small element that stays has four times as many ordinary ones beside it, in its row and in its column.  It carries an
+// absolute error of 2^-43 (2^-31 without lo) of the largest sample.  Of normally distributed elements one in 6e5 is small: two of
+// a stretch's first ten do not come about by chance.
 #include "internal.h"
 
 #include <cuda_fp16.h>
@@ -21,9 +24,10 @@ namespace {
 
 constexpr int kThreads = 256, kTileRows = 16, kTileCols = 512;     // 64 threads x 8 columns, 4 groups of 4 rows
 constexpr int kBlocksPerSm = 3;
-constexpr float kLargest = 32768.f, kSmallest = 1.f / 32768.f;
+constexpr float kLargest = 32768.f, kSmallest = 1.f / 16384.f;
+constexpr unsigned kOrdinary = 4;                  // this many ordinary elements to each small one
 constexpr int kMaxExp = kHalfMaxExp, kTargetExp = 6;
-// Status word of a block: some element, row, column or tile did not fit; some element is beyond 2^30 after scaling.
+// Status word of a block: some element, row or column did not fit; some element is beyond 2^30 after scaling.
 constexpr unsigned kUnfit = 1, kHuge = 2;
 
 struct View {
@@ -95,49 +99,46 @@ __device__ int operand_exponent(const View &v, unsigned *biggest) {
 
 // Bound by memory: 4 bytes read and 4 (LO) or 2 written an element.  A block takes consecutive tiles of a strip of columns, so
 // that what it finds about columns, and their sums (SUMS: of the first view, for the bias gradient), stay in registers until
-// the strip ends.
+// the strip ends.  The ordinary elements of a column are counted two columns at a time, in f16, which stops at 2048 and so errs
+// towards "unfit" only.
 template <bool LO, bool SUMS>
 __global__ void __launch_bounds__(kThreads, kBlocksPerSm)
 split_half_kernel(const __grid_constant__ ViewList list) {
-    __shared__ unsigned shared[4][kTileCols], shared_n[4][kTileCols / 4];
-    __shared__ int smalls;
+    __shared__ unsigned shared[4][kTileCols];
     grid_dependency_trigger();
     grid_dependency_wait();
     const int t0 = first_tile_of(list, blockIdx.x), t1 = first_tile_of(list, blockIdx.x + 1);
     const int tc = threadIdx.x & 63, group = threadIdx.x >> 6;
     const unsigned limit = __float_as_uint(kLargest), small = __float_as_uint(kSmallest);
-    unsigned bad = 0, cmax[8], few[2];             // few: small elements of the columns, a byte each
+    const __half2 none = __float2half2_rn(0.f), least_ordinary = __float2half2_rn(kSmallest);
+    unsigned bad = 0;
+    __half2 ordinary[4], few[4];                   // of the columns: elements of 2^-14 and more, smaller ones but zeros
     float sum[8];
-    int n_small = 0, rows_seen = 0;
+    bool some_small = false;
     int j = -1, strip = -1;
     float scale = 1.f;
     auto begin_strip = [&] {
 #pragma unroll
-        for (int c = 0; c < 8; ++c) { cmax[c] = 0; if (SUMS) sum[c] = 0.f; }
-        few[0] = few[1] = 0;
-        n_small = rows_seen = 0;
+        for (int c = 0; c < 4; ++c) ordinary[c] = few[c] = none;
+        if (SUMS) {
+#pragma unroll
+            for (int c = 0; c < 8; ++c) sum[c] = 0.f;
+        }
+        some_small = false;
     };
     auto end_strip = [&] {
-        if (__syncthreads_or(n_small)) {
-            if (threadIdx.x == 0) smalls = 0;
+        if (__syncthreads_or(some_small)) {
 #pragma unroll
-            for (int c = 0; c < 8; ++c) shared[group][tc * 8 + c] = cmax[c];
-            shared_n[group][tc * 2] = few[0];
-            shared_n[group][tc * 2 + 1] = few[1];
-            __syncthreads();
-            if (n_small) atomicAdd(&smalls, n_small);
-            for (int c = threadIdx.x; c < kTileCols; c += kThreads) {
-                unsigned m = 0, n = 0;
-#pragma unroll
-                for (int g = 0; g < 4; ++g) {
-                    m = max(m, shared[g][c]);
-                    n += (shared_n[g][c >> 2] >> (8 * (c & 3))) & 255u;
-                }
-                if (n >= 8u && m < small) bad |= kUnfit;
+            for (int c = 0; c < 8; ++c) {
+                const __half o = c & 1 ? __high2half(ordinary[c / 2]) : __low2half(ordinary[c / 2]);
+                const __half f = c & 1 ? __high2half(few[c / 2]) : __low2half(few[c / 2]);
+                shared[group][tc * 8 + c] = __half2uint_rz(o) | __half2uint_rz(f) << 16;
             }
             __syncthreads();
-            const int width = min(kTileCols, list.v[j].cols - strip * kTileCols);
-            if (smalls > 16 + rows_seen * width / 16) bad |= kUnfit;
+            for (int c = threadIdx.x; c < kTileCols; c += kThreads) {
+                const unsigned n = shared[0][c] + shared[1][c] + shared[2][c] + shared[3][c];      // at most 8192 each
+                if (kOrdinary * (n >> 16) > (n & 0xffffu)) bad |= kUnfit;
+            }
         }
         if (SUMS && j == 0) {
             __syncthreads();
@@ -184,7 +185,6 @@ split_half_kernel(const __grid_constant__ ViewList list) {
             strip = t.strip;
             begin_strip();
         }
-        rows_seen += min(kTileRows, v.rows - t.r0);
         uint16_t *dst = v.dst + t.batch * v.matrix + static_cast<long long>(r0) * v.pitch + c0;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -197,12 +197,11 @@ split_half_kernel(const __grid_constant__ ViewList list) {
                 if (SUMS) { sum[c] += x[i][c]; sum[c + 1] += x[i][c + 1]; }
                 const float a = x[i][c] * scale, b = x[i][c + 1] * scale;
                 const unsigned ua = __float_as_uint(a) & 0x7fffffffu, ub = __float_as_uint(b) & 0x7fffffffu;
-                cmax[c] = max(cmax[c], ua);
-                cmax[c + 1] = max(cmax[c + 1], ub);
                 big = max(big, max(ua, ub));
                 least = min(least, min(ua - 1u, ub - 1u));         // a zero wraps round to the largest
                 const __half2 h2 = __floats2half2_rn(a, b);
                 h[c / 2] = *reinterpret_cast<const unsigned *>(&h2);
+                ordinary[c / 2] = __hadd2(ordinary[c / 2], __hge2(__habs2(h2), least_ordinary));
                 if (LO) {
                     const float2 back = __half22float2(h2);
                     constexpr float up = 1 << kHalfLoShift;
@@ -212,17 +211,17 @@ split_half_kernel(const __grid_constant__ ViewList list) {
             }
             if (big > limit) bad |= big > __float_as_uint(1073741824.f) ? kUnfit | kHuge : kUnfit;
             if (__any_sync(0xffffffffu, least < small - 1u)) {
-                int n = 0;
+                unsigned n = 0;                                    // small ones below, ordinary ones above
 #pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    const unsigned u = __float_as_uint(x[i][c] * scale) & 0x7fffffffu;
-                    if (u - 1u < small - 1u) {
-                        ++n;
-                        if (((few[c / 4] >> (8 * (c & 3))) & 255u) < 63u) few[c / 4] += 1u << (8 * (c & 3));
-                    }
+                for (int c = 0; c < 8; c += 2) {
+                    const unsigned ua = __float_as_uint(x[i][c] * scale) & 0x7fffffffu, ub = __float_as_uint(x[i][c + 1] * scale) & 0x7fffffffu;
+                    const bool sa = ua - 1u < small - 1u, sb = ub - 1u < small - 1u;
+                    n += (sa ? 1u : ua ? 0x10000u : 0u) + (sb ? 1u : ub ? 0x10000u : 0u);
+                    few[c / 2] = __hadd2(few[c / 2], __floats2half2_rn(sa ? 1.f : 0.f, sb ? 1.f : 0.f));
                 }
-                n_small += n;
-                if (__reduce_add_sync(0xffffffffu, n) >= 16 && !__any_sync(0xffffffffu, big >= small)) bad |= kUnfit;
+                some_small = true;                                 // of the warp, that is
+                n = __reduce_add_sync(0xffffffffu, n);
+                if (kOrdinary * (n & 0xffffu) > n >> 16) bad |= kUnfit;
             }
             if (c0 < v.pitch) {
                 *reinterpret_cast<uint4 *>(dst + static_cast<long long>(4 * i) * v.pitch) = hi;

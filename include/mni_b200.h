@@ -273,7 +273,14 @@ MNI_B200_API int mni_b200_contiguous(const mni_b200_view *src, float *dst, void 
  * bytes an operand element (4 with MNI_B200_PRECISION_TF32).  Where that cannot be
  * had -- a smaller buffer was given, no memory is left, a capture may not grow it --
  * the call computes them from the f32 operands instead, which needs what it did
- * before and takes longer; it does not fail for it.
+ * before and takes longer; it does not fail for it.  The planes keep 22 bits of an
+ * element (11 with MNI_B200_PRECISION_TF32), except that one smaller than 2^-20 of
+ * the operand's largest may have an error of 2^-43 (2^-31) of that largest one
+ * where it is among others: where four in five of the non-zero elements beside it,
+ * in its row and in its column, are larger than that.  This shows in a result only
+ * where all those larger ones meet zeros of the other operand.  Operands with
+ * more small elements than that in any row or column keep all their bits, and take
+ * longer.
  */
 MNI_B200_API int mni_b200_workspace_set(void *ptr, size_t bytes);
 MNI_B200_API int mni_b200_workspace_query(const mni_b200_view *a, const mni_b200_view *b, uint32_t flags,

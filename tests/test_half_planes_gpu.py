@@ -108,10 +108,45 @@ def _ranges():
     }
 
 
+def _sparse():
+    """Small numbers in a row, a column or a matrix of few non-zeros, or beside large ones that meet zeros."""
+    rng = np.random.default_rng(2)
+    m, k, n = 300, 512, 272
+    x, w = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((k, n)).astype(np.float32)
+    cases = {}
+    for count, scale in ((1, 1e-8), (8, 1e-9), (8, 1e-12), (15, 1e-13), (100, 1e-7)):
+        a, b = x.copy(), w.copy()
+        a[5] = 0
+        b[:, 7] = 0
+        for c0 in range(0, k, 256):
+            at = c0 + rng.permutation(256)[:count]
+            a[5, at], b[at, 7] = x[5, at] * np.float32(scale), w[at, 7] * np.float32(scale)
+        cases[f"row of {count} at {scale:g}"], cases[f"column of {count} at {scale:g}"] = (a, w), (x, b)
+    a, b = x.copy(), w.copy()
+    a[5] *= np.float32(1e-10)
+    a[5, ::256] = 1
+    b[::256] = 0
+    cases["row behind ones"] = (a, b)
+    a, b = x.copy(), w.copy()
+    b[:, 7] *= np.float32(1e-10)
+    b[::16, 7] = 1
+    a[:, ::16] = 0
+    cases["column behind ones"] = (a, b)
+    a, b = x.copy(), w.copy()
+    a[5] = 0
+    a[5, 3], a[5, 7], b[3] = 1, 1e-10, 0
+    cases["one behind a one"] = (a, b)
+    long = rng.standard_normal((2048, n)).astype(np.float32)
+    for scale in (1e-6, 1e-8, 1e-12):                # none of the diagonal is among the samples that the scale comes from
+        cases[f"diagonal {scale:g}"] = (np.eye(2048, dtype=np.float32) * np.float32(scale), long)
+    cases["diagonal of many sizes"] = (np.diag(np.logspace(-14, 0, 2048).astype(np.float32)), long)
+    return cases
+
+
 @pytest.mark.parametrize("name", list(_ranges()))
 @pytest.mark.parametrize("single", [False, True])
 def test_any_range_of_values(F, planes, monkeypatch, name, single):
-    """Row by row and column by column: what f16 does not hold goes through bf16 planes, and nothing loses its leading bits."""
+    """Row by row and column by column: what f16 does not hold goes through bf16 planes.  Infinities and NaN as from f32 operands."""
     x, w = _ranges()[name]
     t = F.DeviceTensor.from_numpy
     flags = F._lib.PRECISION_TF32 if single else 0
@@ -123,10 +158,52 @@ def test_any_range_of_values(F, planes, monkeypatch, name, single):
     assert np.array_equal(finite, np.isfinite(got))
     if not finite.all():
         return
-    want = x.astype(np.float64) @ w.astype(np.float64)
-    for axis in (0, 1):
+    _by_rows_and_columns(got, x.astype(np.float64) @ w.astype(np.float64), single)
+
+
+def _by_rows_and_columns(got, want, single):
+    """Single pass: 2^-12 of every operand's element and a sum's rounding; else 2^-22 and that: 2e-6 at K = 512."""
+    for axis in (-1, -2):
         error = np.sqrt(((got - want) ** 2).sum(axis))
         assert (error <= (1e-3 if single else 2e-6) * np.sqrt((want ** 2).sum(axis))).all(), axis
+
+
+@pytest.mark.parametrize("name", list(_sparse()))
+@pytest.mark.parametrize("single", [False, True])
+def test_rows_and_columns_of_few_small_numbers(F, planes, name, single):
+    x, w = _sparse()[name]
+    t = F.DeviceTensor.from_numpy
+    got = F.matmul(t(x), t(w), flags=F._lib.PRECISION_TF32 if single else 0).numpy()
+    F.device_status()
+    _by_rows_and_columns(got, x.astype(np.float64) @ w.astype(np.float64), single)
+
+
+@pytest.mark.parametrize("single", [False, True])
+def test_ordinary_values_stay_in_f16(F, planes, single):
+    """The verdict of the pass, which follows the blocks' words at the start of the scratch: what f16 holds is not sent to the
+    planes that take longer."""
+    import torch
+    rng = np.random.default_rng(6)
+    def normal(*s):
+        return rng.standard_normal(s).astype(np.float32)
+    x, w = normal(1000, 700), normal(700, 520)
+    half_off = np.where(normal(1000, 700) > 0, x, 0).astype(np.float32)
+    cases = {"normal": (x, w), "uniform": (rng.random((1000, 700), np.float32), w), "halves": (half_off, w), "narrow": (normal(1000, 257), normal(257, 520)),
+             "few": (np.where(rng.random((1000, 700)) < 0.02, x, 0).astype(np.float32), w), "one hot": (np.eye(700, dtype=np.float32)[rng.integers(0, 700, 1000)], w),
+             "gelu": (0.5 * x * (1 + np.tanh(0.7978845608 * (x + 0.044715 * x ** 3))), w * np.float32(0.02)), "scaled rows": (x * np.float32(10) ** rng.uniform(-3, 1, (1000, 1)).astype(np.float32), w)}
+    lib, room = F._lib.lib(), 64 << 20
+    buf = torch.empty(room, dtype=torch.uint8, device="cuda")
+    F._lib.check(lib.mni_b200_workspace_set(C.c_void_p(buf.data_ptr()), room))
+    try:
+        for name, (a, b) in cases.items():
+            a, b = F.DeviceTensor.from_numpy(np.ascontiguousarray(a, np.float32)), F.DeviceTensor.from_numpy(b)
+            F.matmul(a, b, flags=F._lib.PRECISION_TF32 if single else 0)
+            F.device_status()
+            blocks = min(148 * 3, sum(-(-r // 16) * -(-(-(-c // 64) * 64) // 512) for r, c in (a.shape, b.shape)))
+            words = buf[:4 * (blocks + 1)].view(torch.int32)
+            assert int(words[blocks]) == 0 and not bool(words.any()), name
+    finally:
+        F._lib.check(lib.mni_b200_workspace_set(None, 0))
 
 
 def test_without_scratch_for_the_planes_the_product_comes_from_f32(F, planes, monkeypatch):
