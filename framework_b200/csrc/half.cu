@@ -6,9 +6,9 @@
 // bits (11 where there is no lo).  What f16 does not hold is found by the same pass and reported in the block's status word; a
 // second kernel then writes three bf16 planes, whose range is that of f32, and the products take those:
 //   - an element beyond 2^15 after scaling, an infinity or a NaN;
-//   - a stretch of a row (256 elements) or of a column (what a block takes of it) in which more than a fifth of the elements are
-//     smaller than 2^-14, zeros not counted: in its row or column of the product the bits they lose could be the leading ones,
-//     where the stretch has nothing else as well as where the rest of it meets zeros.
+//   - a stretch of a row (256 elements) or of a column (what a block takes of it in one matrix) in which more than a fifth of the
+//     elements are smaller than 2^-14, zeros not counted: in its row or column of the product the bits they lose could be the
+//     leading ones, where the stretch has nothing else as well as where the rest of it meets zeros.
 // So a small element that stays has four times as many ordinary ones beside it, in its row and in its column.  It carries an
 // absolute error of 2^-43 (2^-31 without lo) of the largest sample.  Of normally distributed elements one in 6e5 is small: two of
 // a stretch's first ten do not come about by chance.
@@ -98,8 +98,8 @@ __device__ int operand_exponent(const View &v, unsigned *biggest) {
 }
 
 // Bound by memory: 4 bytes read and 4 (LO) or 2 written an element.  A block takes consecutive tiles of a strip of columns, so
-// that what it finds about columns, and their sums (SUMS: of the first view, for the bias gradient), stay in registers until
-// the strip ends.  The ordinary elements of a column are counted two columns at a time, in f16, which stops at 2048 and so errs
+// that what it finds about columns stays in registers until the matrix ends, and their sums (SUMS: of the first view, for the
+// bias gradient) until the strip ends.  The ordinary elements of a column are counted two columns at a time, in f16, which stops at 2048 and so errs
 // towards "unfit" only.
 template <bool LO, bool SUMS>
 __global__ void __launch_bounds__(kThreads, kBlocksPerSm)
@@ -117,16 +117,12 @@ split_half_kernel(const __grid_constant__ ViewList list) {
     bool some_small = false;
     int j = -1, strip = -1;
     float scale = 1.f;
-    auto begin_strip = [&] {
+    auto begin_columns = [&] {
 #pragma unroll
         for (int c = 0; c < 4; ++c) ordinary[c] = few[c] = none;
-        if (SUMS) {
-#pragma unroll
-            for (int c = 0; c < 8; ++c) sum[c] = 0.f;
-        }
         some_small = false;
     };
-    auto end_strip = [&] {
+    auto end_columns = [&] {
         if (__syncthreads_or(some_small)) {
 #pragma unroll
             for (int c = 0; c < 8; ++c) {
@@ -140,6 +136,9 @@ split_half_kernel(const __grid_constant__ ViewList list) {
                 if (kOrdinary * (n >> 16) > (n & 0xffffu)) bad |= kUnfit;
             }
         }
+    };
+    auto end_strip = [&] {
+        end_columns();
         if (SUMS && j == 0) {
             __syncthreads();
             float *const mine = reinterpret_cast<float *>(&shared[0][0]);
@@ -183,7 +182,14 @@ split_half_kernel(const __grid_constant__ ViewList list) {
             }
             j = at;
             strip = t.strip;
-            begin_strip();
+            begin_columns();
+            if (SUMS) {
+#pragma unroll
+                for (int c = 0; c < 8; ++c) sum[c] = 0.f;
+            }
+        } else if (t.r0 == 0) {                    // the next matrix, whose columns are judged by themselves
+            end_columns();
+            begin_columns();
         }
         uint16_t *dst = v.dst + t.batch * v.matrix + static_cast<long long>(r0) * v.pitch + c0;
 #pragma unroll

@@ -179,6 +179,21 @@ def test_rows_and_columns_of_few_small_numbers(F, planes, name, single):
 
 
 @pytest.mark.parametrize("single", [False, True])
+def test_small_columns_beside_ordinary_ones_of_the_next_matrix(F, planes, single):
+    """A block of the pass takes ten tiles of 16 rows here and a matrix has four: no matrix has a block of its own."""
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    x, dy = (torch.randn(s, generator=gen, device="cuda") for s in ((555, 64, 200), (555, 64, 136)))
+    for b in range(555):
+        x[b, :, b % 200] *= 1e-12
+    t = F.DeviceTensor.from_torch
+    _, dw = F.matmul_backward(t(dy), t(x), t(torch.zeros(555, 200, 136, device="cuda")), need_da=False,
+                              flags=F._lib.PRECISION_TF32 if single else 0)
+    F.device_status()
+    _by_rows_and_columns(dw.numpy(), (x.double().transpose(1, 2) @ dy.double()).cpu().numpy(), single)
+
+
+@pytest.mark.parametrize("single", [False, True])
 def test_ordinary_values_stay_in_f16(F, planes, single):
     """The verdict of the pass, which follows the blocks' words at the start of the scratch: what f16 holds is not sent to the
     planes that take longer."""
