@@ -240,6 +240,17 @@ split_half_kernel(const __grid_constant__ ViewList list) {
     if (threadIdx.x == 0) list.status[blockIdx.x] = bad;
 }
 
+// The bf16 of plane `plane` in the upper half of a word, of what the planes before it left of an element.  Cut, not rounded, so that
+// the largest f32 does not become infinite.  Single-pass products (two planes) of an infinity come out infinite, as from f32
+// operands, if it meets the first plane of the other operand alone, whose second may be zero: the first plane has its sign, the
+// second, which is left of it then, itself.
+template <int PLANES>
+__device__ __forceinline__ unsigned wide_part(float x, int plane) {
+    const unsigned u = __float_as_uint(x);
+    if (PLANES == 2 && plane == 0 && (u & 0x7fffffffu) == 0x7f800000u) return (u & 0x80000000u) | 0x3f800000u;
+    return u & 0xffff0000u;
+}
+
 // Finishes the column sums.  And if the pass above found an operand that f16 does not hold: all of them again, as sums of three
 // (or two) bf16, whose range is that of f32.  half_wide_exponent has their scale.
 template <int PLANES>
@@ -299,8 +310,7 @@ split_wide_kernel(const __grid_constant__ ViewList list) {
                 unsigned *const o = &out.x;
 #pragma unroll
                 for (int c = 0; c < 8; c += 2) {
-                    // cut, not rounded, so that the largest f32 does not become infinite
-                    const unsigned a = __float_as_uint(x[c]) & 0xffff0000u, b = __float_as_uint(x[c + 1]) & 0xffff0000u;
+                    const unsigned a = wide_part<PLANES>(x[c], plane), b = wide_part<PLANES>(x[c + 1], plane);
                     o[c / 2] = (a >> 16) | b;
                     x[c] -= __uint_as_float(a);
                     x[c + 1] -= __uint_as_float(b);

@@ -221,6 +221,31 @@ def test_ordinary_values_stay_in_f16(F, planes, single):
         F._lib.check(lib.mni_b200_workspace_set(None, 0))
 
 
+@pytest.mark.parametrize("at", ["left", "right", "both"])
+@pytest.mark.parametrize("single", [False, True])
+def test_infinities_as_from_f32_operands(F, planes, monkeypatch, at, single):
+    """Against finite numbers of one bf16 and of more, of either sign, zero, and an infinity: the same infinities, the same NaN."""
+    rng = np.random.default_rng(7)
+    x, w = (rng.standard_normal(s).astype(np.float32) for s in ((300, 320), (320, 272)))
+    w[4, :4], x[:4, 5] = (1, -2, 0, 1e-30), (1, -2, 0, 1e-30)
+    if at != "right":
+        x[10, 4], x[11, 4] = np.inf, -np.inf
+    if at != "left":
+        w[5, 20], w[5, 21] = np.inf, -np.inf
+    if at == "both":
+        w[4, 30], w[4, 31] = np.inf, -np.inf
+    t = F.DeviceTensor.from_numpy
+    flags = F._lib.PRECISION_TF32 if single else 0
+    got = F.matmul(t(x), t(w), flags=flags).numpy()
+    F.device_status()
+    monkeypatch.setenv("MNI_B200_HALF", "0")
+    general = F.matmul(t(x), t(w), flags=flags).numpy()
+    assert np.array_equal(np.isnan(general), np.isnan(got)) and not np.isfinite(general).all()
+    infinite = np.isinf(general)
+    assert np.array_equal(infinite, np.isinf(got)) and np.array_equal(general[infinite], got[infinite])
+    assert infinite.any() == single                  # in three passes inf - inf is what is left of one
+
+
 def test_without_scratch_for_the_planes_the_product_comes_from_f32(F, planes, monkeypatch):
     """A buffer that the general path fits in and the planes do not, and a capture that may not grow the library's own."""
     import torch
