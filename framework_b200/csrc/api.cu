@@ -1235,7 +1235,8 @@ int with_scratch(uint32_t flags, void *stream, Body body) {
         if (rc) return rc;
         sized = dry.arena.used;
         if (sized == 0) break;
-        if (dry.used_half && !st->user_ws && sized >= st->refused && sized > st->ws_bytes) {
+        // Not what would have to be allocated in a capture, which that would end, nor what could not be had before.
+        if (dry.used_half && !st->user_ws && sized > st->ws_bytes && (capturing || sized >= st->refused)) {
             real.no_half = true;
             continue;
         }
@@ -1243,7 +1244,7 @@ int with_scratch(uint32_t flags, void *stream, Body body) {
         if (rc == MNI_B200_OK) break;
         // Scratch for the operands' planes cannot be had: the call goes without them, as it needs little or none then.
         if (!dry.used_half || real.no_half) return rc;
-        if (!st->user_ws && !capturing) st->refused = sized;      // (growing frees and allocates: not on every call)
+        if (!st->user_ws) st->refused = sized;                    // (growing frees and allocates: not on every call)
         real.no_half = true;
     }
     rc = body(real);

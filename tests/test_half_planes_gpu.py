@@ -285,6 +285,22 @@ def test_without_scratch_for_the_planes_the_product_comes_from_f32(F, planes, mo
     assert float((out.torch_view().double() - s @ s).norm() / (s @ s).norm()) <= 2e-5
 
 
+def test_capture_before_there_is_any_scratch(F):
+    """The first call after a release is a captured one: it allocates nothing, and needs nothing from f32 operands."""
+    import torch
+    x, w, out = (F.DeviceTensor.from_torch(torch.randn(s, device="cuda")) for s in ((4096, 1024), (1024, 4096), (4096, 4096)))
+    F._lib.check(F._lib.lib().mni_b200_release())
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            F.matmul(x, w, out=out)
+    graph.replay()
+    F.device_status()
+    want = x.torch_view().double() @ w.torch_view().double()
+    assert float((out.torch_view().double() - want).norm() / want.norm()) <= 2e-5
+
+
 def test_queried_scratch_holds_the_planes(F, planes):
     import torch
     rng = np.random.default_rng(4)
