@@ -183,12 +183,10 @@ int scratch_base(DeviceState &st, size_t bytes, cudaStream_t stream, uint8_t **b
                         "scratch would have to grow from %zu to %zu bytes while the stream is capturing: run the call "
                         "once before the capture, or hand the library a buffer (mni_b200_workspace_set)",
                         st.ws_bytes, bytes);
-        if (st.ws && st.ws_recorded) {
-            st.retired.push_back(st.ws);
-            st.ws = nullptr;
-            st.ws_bytes = 0;
-            st.ws_recorded = false;
-        } else if (st.ws) {
+        // What there is stays if the larger buffer cannot be had: calls that fit in it may be captured later on.
+        const bool keep = st.ws && st.ws_recorded;
+        const size_t old_bytes = keep ? 0 : st.ws_bytes;
+        if (st.ws && !keep) {
             // cudaFree waits for work that may still read the old buffer.
             cudaError_t e = cudaFree(st.ws);
             st.ws = nullptr;
@@ -196,11 +194,18 @@ int scratch_base(DeviceState &st, size_t bytes, cudaStream_t stream, uint8_t **b
             if (e != cudaSuccess) return fail(MNI_B200_ERR_WORKSPACE, "cudaFree(scratch): %s", cudaGetErrorString(e));
         }
         void *p = nullptr;
-        cudaError_t e = cudaMalloc(&p, want);
+        const cudaError_t e = cudaMalloc(&p, want);
         if (e != cudaSuccess) {
+            cudaGetLastError();
+            if (old_bytes && cudaMalloc(&p, old_bytes) == cudaSuccess) {
+                st.ws = static_cast<uint8_t *>(p);
+                st.ws_bytes = old_bytes;
+            }
             cudaGetLastError();
             return fail(MNI_B200_ERR_WORKSPACE, "cudaMalloc(%zu) for scratch failed: %s", want, cudaGetErrorString(e));
         }
+        if (keep) st.retired.push_back(st.ws);
+        st.ws_recorded = false;
         st.ws = static_cast<uint8_t *>(p);
         st.ws_bytes = want;
     }

@@ -301,6 +301,53 @@ def test_capture_before_there_is_any_scratch(F):
     assert float((out.torch_view().double() - want).norm() / want.norm()) <= 2e-5
 
 
+@pytest.fixture
+def little_memory():
+    """All of the device's memory but 80 MB taken, until release() is called."""
+    import torch
+    hog = []
+    def take():
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        hog.append(torch.empty(torch.cuda.mem_get_info()[0] - (80 << 20), dtype=torch.uint8, device="cuda"))
+    def release():
+        hog.clear()
+        torch.cuda.empty_cache()
+    yield take, release
+    release()
+
+
+@pytest.mark.parametrize("recorded", [False, True])
+def test_planes_that_do_not_fit_leave_the_scratch_there_was(F, little_memory, recorded):
+    """A small call that has run can be captured, although a larger one found no memory for its planes in between."""
+    import torch
+    x, w, out = (F.DeviceTensor.from_torch(torch.randn(s, device="cuda")) for s in ((8192, 1024), (1024, 8192), (8192, 8192)))
+    a, c = (F.DeviceTensor.from_torch(torch.randn(512, 512, device="cuda")) for _ in range(2))
+    want = a.torch_view().double() @ a.torch_view().double()
+    F._lib.check(F._lib.lib().mni_b200_release())
+    def small():
+        F.matmul(a, a, out=c)                        # four splits, in scratch
+    def capture(call):
+        stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+        with torch.cuda.stream(stream):
+            with torch.cuda.graph(graph, stream=stream):
+                call()
+        return graph
+    small()
+    capture(c.torch_view().zero_)                    # what torch needs for its first capture
+    first = capture(small) if recorded else None
+    little_memory[0]()
+    launches = F.launch_count()
+    F.matmul(x, w, out=out)                          # planes of 100 MB
+    assert F.launch_count() - launches == 1
+    for graph in (first, capture(small)):
+        if graph is not None:
+            c.torch_view().zero_()
+            graph.replay()
+            F.device_status()
+            assert float((c.torch_view().double() - want).norm() / want.norm()) <= 5e-6
+
+
 def test_queried_scratch_holds_the_planes(F, planes):
     import torch
     rng = np.random.default_rng(4)
