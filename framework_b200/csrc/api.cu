@@ -38,7 +38,8 @@ struct DeviceState {
     uint8_t *ws = nullptr;        // library-owned scratch
     size_t ws_bytes = 0;
     bool ws_recorded = false;     // some graph holds its address
-    size_t refused = SIZE_MAX;    // the least that could not be had for 16-bit planes: not tried again until mni_b200_release
+    size_t refused = SIZE_MAX;    // the least that could not be had for 16-bit planes, and what was free then: not tried again
+    size_t refused_free = 0;      // until more is (or mni_b200_release)
     std::vector<uint8_t *> retired;   // scratch outgrown since, kept for the graphs that hold its address (mni_b200_release frees it)
     uint8_t *user_ws = nullptr;   // caller-provided scratch (takes precedence)
     size_t user_bytes = 0;
@@ -165,6 +166,27 @@ bool stream_is_capturing(cudaStream_t stream) {
     return status != cudaStreamCaptureStatusNone;
 }
 
+// What is allocated where `bytes` of scratch are needed.
+size_t scratch_for(size_t bytes) { return bytes + bytes / 4 + (1u << 20); }
+
+// Whether scratch of this size, or less, was refused and there is no more memory than then.  Growing frees and allocates, which
+// calls that go on without it must not do each time.
+bool scratch_refused(const DeviceState &st, size_t bytes) {
+    if (bytes < st.refused) return false;
+    size_t free = 0, total = 0;
+    if (cudaMemGetInfo(&free, &total) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return free <= st.refused_free || free + (st.ws_recorded ? 0 : st.ws_bytes) < scratch_for(bytes);
+}
+void note_refused(DeviceState &st, size_t bytes) {
+    size_t free = 0, total = 0;
+    if (cudaMemGetInfo(&free, &total) != cudaSuccess) cudaGetLastError();
+    st.refused = bytes;
+    st.refused_free = free;
+}
+
 // Makes `bytes` of scratch available and returns its base.
 int scratch_base(DeviceState &st, size_t bytes, cudaStream_t stream, uint8_t **base) {
     if (st.user_ws) {
@@ -175,7 +197,7 @@ int scratch_base(DeviceState &st, size_t bytes, cudaStream_t stream, uint8_t **b
         return MNI_B200_OK;
     }
     if (bytes > st.ws_bytes) {
-        const size_t want = bytes + bytes / 4 + (1u << 20);
+        const size_t want = scratch_for(bytes);
         // Growing frees the old buffer, which a capturing stream must not do (it would end the capture in
         // an error).
         if (st.ws && stream_is_capturing(stream))
@@ -1241,7 +1263,7 @@ int with_scratch(uint32_t flags, void *stream, Body body) {
         sized = dry.arena.used;
         if (sized == 0) break;
         // Not what would have to be allocated in a capture, which that would end, nor what could not be had before.
-        if (dry.used_half && !st->user_ws && sized > st->ws_bytes && (capturing || sized >= st->refused)) {
+        if (dry.used_half && !st->user_ws && sized > st->ws_bytes && (capturing || scratch_refused(*st, sized))) {
             real.no_half = true;
             continue;
         }
@@ -1249,7 +1271,7 @@ int with_scratch(uint32_t flags, void *stream, Body body) {
         if (rc == MNI_B200_OK) break;
         // Scratch for the operands' planes cannot be had: the call goes without them, as it needs little or none then.
         if (!dry.used_half || real.no_half) return rc;
-        if (!st->user_ws) st->refused = sized;                    // (growing frees and allocates: not on every call)
+        if (!st->user_ws) note_refused(*st, sized);
         real.no_half = true;
     }
     rc = body(real);

@@ -348,6 +348,21 @@ def test_planes_that_do_not_fit_leave_the_scratch_there_was(F, little_memory, re
             assert float((c.torch_view().double() - want).norm() / want.norm()) <= 5e-6
 
 
+def test_planes_are_tried_again_once_there_is_memory(F, little_memory):
+    import torch
+    x, w, out = (F.DeviceTensor.from_torch(torch.randn(s, device="cuda")) for s in ((8192, 1024), (1024, 8192), (8192, 8192)))
+    F._lib.check(F._lib.lib().mni_b200_release())
+    def launches():
+        before = F.launch_count()
+        F.matmul(x, w, out=out)
+        return F.launch_count() - before
+    little_memory[0]()
+    assert (launches(), launches()) == (1, 1)
+    little_memory[1]()
+    assert (launches(), launches()) == (3, 3)        # two passes over the operands and the product
+    F.device_status()
+
+
 def test_queried_scratch_holds_the_planes(F, planes):
     import torch
     rng = np.random.default_rng(4)
