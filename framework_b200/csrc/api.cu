@@ -1593,9 +1593,11 @@ int mni_b200_workspace_query(const mni_b200_view *a, const mni_b200_view *b, uin
     Shapes s;
     rc = analyse(a, b, s);
     if (rc) return rc;
-    // The forward output's gradient, broadcast batch + [M, N], in the two forms that bound what a real one can
-    // need: contiguous and 256-byte aligned (read in place), and a view no descriptor covers (neither matrix
-    // dim has unit stride), which is gathered into scratch once for each of its three uses.
+    // The forward output's gradient, broadcast batch + [M, N], in the forms that bound what a real one can need: contiguous
+    // (read in place, column sums included), the same with M and N exchanged in memory (read in place, but gathered for the
+    // column sums), either on a 16-byte boundary or off it (gathered by products of f32 operands, which counts where these
+    // are compared with 16-bit planes), and a view no descriptor and no plane covers (neither matrix dim has unit stride),
+    // which is gathered into scratch once for each of its three uses.
     mni_b200_view dc{};
     dc.ptr = reinterpret_cast<const float *>(static_cast<uintptr_t>(256));
     dc.ndim = s.out_nb + 2;
@@ -1603,8 +1605,12 @@ int mni_b200_workspace_query(const mni_b200_view *a, const mni_b200_view *b, uin
     dc.shape[s.out_nb] = s.M; dc.shape[s.out_nb + 1] = s.N;
     int64_t acc = 1;
     for (int d = dc.ndim - 1; d >= 0; --d) { dc.stride[d] = acc; acc *= dc.shape[d]; }
-    mni_b200_view dc_strided = dc;
+    mni_b200_view dc_strided = dc, dc_exchanged = dc;
     for (int d = 0; d < dc.ndim; ++d) dc_strided.stride[d] = dc.stride[d] * 2;
+    dc_exchanged.stride[s.out_nb] = 1;
+    dc_exchanged.stride[s.out_nb + 1] = s.M;
+    mni_b200_view dc_off = dc, dc_exchanged_off = dc_exchanged;
+    dc_off.ptr = dc_exchanged_off.ptr = dc.ptr + 1;
     size_t need = 0;
     auto dry = [&](auto body) -> int {             // eager and captured calls are planned differently
         for (const bool capturing : {false, true}) {
@@ -1623,7 +1629,7 @@ int mni_b200_workspace_query(const mni_b200_view *a, const mni_b200_view *b, uin
         float *out = reinterpret_cast<float *>(at);
         rc = dry([&](Call &c) { return fwd_body(c, a, b, out, nullptr); });
         if (rc) return rc;
-        for (const mni_b200_view *grad : {&dc, &dc_strided})
+        for (const mni_b200_view *grad : {&dc, &dc_off, &dc_exchanged, &dc_exchanged_off, &dc_strided})
             for (int want = 1; want < 8; ++want) {
                 rc = dry([&](Call &c) {
                     return bwd_body(c, a, b, grad, (want & 1) ? out : nullptr, (want & 2) ? out : nullptr, (want & 4) ? out : nullptr);

@@ -383,6 +383,36 @@ def test_queried_scratch_holds_the_planes(F, planes):
     assert bool((buf[base - buf.data_ptr() + need.value:] == 0x5A).all())
 
 
+@pytest.mark.parametrize("shape", [(1024, 512, 768), (2048, 768, 3072), (512, 320, 512, 3)])
+@pytest.mark.parametrize("exchanged,off", [(False, 0), (False, 1), (True, 0), (True, 1)])
+def test_queried_scratch_serves_every_view_of_the_gradient(F, monkeypatch, shape, exchanged, off):
+    """The call takes the same launches from a buffer of the queried size as from the library's own scratch."""
+    import torch
+    (m, k, n), lead = shape[:3], shape[3:]
+    x, w = (F.DeviceTensor.from_torch(torch.randn(s, device="cuda")) for s in (lead + (m, k), lead + (k, n)))
+    size = m * n * int(np.prod(lead))
+    g = F.DeviceTensor(torch.randn(size + off, device="cuda")[off:], lead + ((n, m) if exchanged else (m, n)))
+    if exchanged:
+        g = g.permute(tuple(range(len(lead))) + (len(lead) + 1, len(lead)))
+    def launches(**kw):
+        before = F.launch_count()
+        F.matmul_backward(g, x, w, **kw)
+        return F.launch_count() - before
+    lib, need = F._lib.lib(), C.c_size_t(0)
+    wanted = [dict(want_dbias=True), dict(), dict(need_da=False, want_dbias=True), dict(need_db=False)]
+    for half in ("0", "1", None):
+        monkeypatch.setenv("MNI_B200_HALF", half) if half else monkeypatch.delenv("MNI_B200_HALF")
+        own = [launches(**kw) for kw in wanted]
+        F._lib.check(lib.mni_b200_workspace_query(x.view_struct(), w.view_struct(), 0, C.byref(need)))
+        buf = torch.empty(need.value + 256, dtype=torch.uint8, device="cuda")
+        F._lib.check(lib.mni_b200_workspace_set(C.c_void_p((buf.data_ptr() + 255) // 256 * 256), need.value))
+        try:
+            assert [launches(**kw) for kw in wanted] == own, half
+        finally:
+            F.device_status()
+            F._lib.check(lib.mni_b200_workspace_set(None, 0))
+
+
 @pytest.mark.parametrize("flags", [0, 1])
 def test_wait_limit_runs_out_then_the_library_recovers(F, planes, monkeypatch, flags):
     """As test_timeout_gpu.py does for the other variants: a stage that is armed and never filled."""
