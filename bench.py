@@ -130,14 +130,36 @@ WORKLOADS = {
 }
 HBM_BOUND = ("c3", "c5b1", "c5b4", "c5b16")
 SHARDED = ("c4", "c5a")            # partition across ranks (strong scaling); c2 is weak-scaled; the rest are replicas
-# DRAM bytes of one forward launch, from ncu captures of that launch summarised under profiles/
-# (dram__bytes_read.sum + dram__bytes_write.sum): a cited capture, not a measurement of this run.
+# DRAM bytes of one forward call, from ncu captures of its launches summarised under profiles/
+# (dram__bytes_read.sum + dram__bytes_write.sum): a cited capture, not a measurement of this run.  By workload, and by whether the
+# product is computed from 16-bit planes ("f16") or f32 operands ("tf32": MNI_B200_HALF=0 for these two).
 NCU_TRAFFIC = {
-    "c2": (34.11e6 + 19.63e6, "profiles/gemm_tc_kernel_c2_linear.md"),
+    ("c2", "f16"): (33.6e6 + 0.7e6 + 34.8e6 + 18.2e6, "profiles/gemm_tc_kernel_planes_c2.md"),
+    ("c2", "tf32"): (34.11e6 + 19.63e6, "profiles/gemm_tc_kernel_c2_linear.md"),
     # captured on a 1/8 shard (34.7 MB read + 46.3 MB written of 135.3 MB algorithmic; the output's last ~54 MB stay
     # in L2) and scaled to 64 batches: operands 210.7 MB, output 805.3 MB minus the same L2 residue
-    "c4": (210.7e6 + 805.3e6 - 54.4e6, "profiles/gemm_tc_kernel_c4_broadcast_weight.md (scaled from the 8-batch shard)"),
+    ("c4", "tf32"): (210.7e6 + 805.3e6 - 54.4e6, "profiles/gemm_tc_kernel_c4_broadcast_weight.md (scaled from the 8-batch shard)"),
 }
+
+
+def product_pipe(fn, outputs) -> str:
+    """"f16" for a call that is computed from 16-bit planes of its operands, else "tf32".  The library is asked: the same call kept to
+    f32 operands gives other bits in some output then, and the same bits otherwise (results are reproducible)."""
+    import torch
+    chosen = os.environ.get("MNI_B200_HALF")
+    fn()
+    before = [t.clone() for t in outputs]
+    try:
+        os.environ["MNI_B200_HALF"] = "0"
+        fn()
+    finally:
+        if chosen is None:
+            del os.environ["MNI_B200_HALF"]
+        else:
+            os.environ["MNI_B200_HALF"] = chosen
+    return "tf32" if all(torch.equal(a, b) for a, b in zip(before, outputs)) else "f16"
+
+
 C5A_PANELS = 4                      # row panels of dB, each reduced as soon as it is computed
 
 
@@ -589,9 +611,8 @@ def run_ours(args):
         if hbm_bound:
             entry.update(bound="hbm", frac=round(gbs / hbm_peak, 4))
         else:
-            # a call from 16-bit planes makes two launches before the product's own, and multiplies on the f16 pipe
-            entry["pipe"] = "f16" if n_launch >= 3 else "tf32"
-            pipe_peak = tf32_peak * (2 if n_launch >= 3 else 1)
+            entry["pipe"] = product_pipe(fn, [t.storage for t in prob.out.values()])
+            pipe_peak = tf32_peak * (2 if entry["pipe"] == "f16" else 1)
             issued = tfs * (1 if args.precision == "tf32" else 3)
             entry.update(bound="tensor", frac=round(tfs / pipe_peak, 4), issued_frac=round(issued / pipe_peak, 4))
         kernels.append(entry)
@@ -608,16 +629,14 @@ def run_ours(args):
                                      "note": "sum of algorithmic bytes / sum of the products' stand-alone times"},
                     "peak_source": "measured hbm_gbs" if "hbm_gbs" in peaks else "fallback 6650"}
     else:
-        traffic, source = (NCU_TRAFFIC.get(wl.name, (None, None))
+        traffic, source = (NCU_TRAFFIC.get((wl.name, first["pipe"]), (None, None))
                            if (args.precision != "tf32" and world == 1 and args.shard_of == 1) else (None, None))
         issued = first["tflops"] * (1 if args.precision == "tf32" else 3)
         f16 = first["pipe"] == "f16"
         pipe_peak = tf32_peak * (2 if f16 else 1)
-        if f16:
-            traffic, source = None, None               # the cited captures are of the f32-operand launch
         roofline = {"bound": "tensor", "achieved": first["tflops"], "peak": pipe_peak, "unit": "TFLOP/s",
                     "frac": first["tflops"] / pipe_peak, "traffic": traffic,
-                    "traffic_source": (f"cited from {source} (ncu dram read+write bytes of this launch), not measured by this run"
+                    "traffic_source": (f"cited from {source} (ncu dram read+write bytes of the call's launches), not measured by this run"
                                        if source else None),
                     "algorithmic_bytes": first["algorithmic_bytes"],
                     "kernel": f"gemm_tc_kernel ({first['call']}; the other products are in `kernels`)",

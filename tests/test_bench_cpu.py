@@ -47,6 +47,19 @@ def test_both_arms_print_the_same_config(bench):
     assert bench.config_dict(bench.WORKLOADS["c4"], 1, "3xtf32")["parallelism"] == "single GPU"
 
 
+def test_pipe_of_a_call_is_asked_of_the_library(bench, monkeypatch):
+    """By the results with and without 16-bit planes, however many launches a call makes; the caller's switch is put back."""
+    import torch
+    out = [torch.zeros(4), torch.zeros(2)]
+    def planes():
+        out[1].fill_(1.0 if os.environ.get("MNI_B200_HALF") == "0" else 1.0 + 2.0 ** -20)
+    for chosen in (None, "1"):
+        monkeypatch.setenv("MNI_B200_HALF", chosen) if chosen else monkeypatch.delenv("MNI_B200_HALF", raising=False)
+        assert bench.product_pipe(planes, out) == "f16"
+        assert bench.product_pipe(lambda: out[0].fill_(3.0), out) == "tf32"
+        assert os.environ.get("MNI_B200_HALF") == chosen
+
+
 def test_cpu_samples_are_bounded_leading_slices(bench):
     c4 = bench.WORKLOADS["c4"]
     small, what = bench.cpu_sample_workload(c4, budget_gflop=150.0)
