@@ -29,7 +29,13 @@ def test_calls_from_16_bit_planes(plan, a, b, flags, forward, backward):
     for backward_call, want in ((0, forward), (1, backward)):
         lines = plan(a, b, flags=flags, backward=backward_call)
         assert len(planes(lines)) == want, lines
-        assert ": tensor " in lines[0] or "tensor" in "".join(lines), lines
+        kinds = ["planes" if ": planes " in line else "f32" if ": tensor " in line else
+                 "instead" if "with scratch for 16-bit operands" in line else "" for line in lines]
+        named = [kind for kind in kinds if kind]
+        if want:
+            assert named == ["f32"] * named.count("f32") + ["instead"] + ["planes"] * want and named[0] == "f32", lines
+        else:
+            assert set(named) <= {"f32"}, lines
 
 
 @pytest.mark.parametrize("m,k,n", [(2048, 3072, 768), (1000, 1333, 2777), (700, 5000, 3000), (4096, 4096, 4096), (8192, 768, 3072)])
