@@ -480,9 +480,10 @@ constexpr int kDxRows = 2;
 // step are under way before its first multiply; what is left of a row is a step of its own.  With a test per row and position
 // the loads waited for the multiplies between them.  us with three weights in turn, before / now: 4096 x 4096 at 1 / 2 / 3 /
 // 4 / 5 rows 12.5 / 15.6 / 21.6 / 20.3 / 22.9 -> 10.6 / 11.9 / 12.0 / 12.3 / 13.0, 8192 x 8192 at 4 rows 69 -> 41.5.  (The next
-// step's weights loaded one step early: 11.7 / 12.3 / 12.9 / 13.0 / 14.5; bounds of three blocks per SM spill.)
-template <int MT, bool LONG>
-__global__ void __launch_bounds__(kDxThreads, LONG ? 2 : 1)
+// step's weights loaded one step early: 11.7 / 12.3 / 12.9 / 13.0 / 14.5.)  BLOCKS per SM that the registers are shared out for:
+// launch_skinny_dx has the rule.
+template <int MT, bool LONG, int BLOCKS>
+__global__ void __launch_bounds__(kDxThreads, BLOCKS)
 skinny_dx_kernel(const float *__restrict__ dy, long long lddy, const float *__restrict__ W, long long ldw,
                  float *__restrict__ dx, long long lddx, int accumulate, long long N, long long K, int early) {
     grid_dependency_trigger();
@@ -845,24 +846,35 @@ int launch_skinny_dx(const float *dy, int64_t lddy, const float *W, int64_t ldw,
     const unsigned blocks = static_cast<unsigned>((K + rows_per_block - 1) / rows_per_block);
     // One row against short weight rows, or two against very short ones, keep the tested loop, which takes fewer registers: there
     // more blocks per SM count.  1 row, tested / not: 16384 x 600 8.3 / 9.4 us, 8192 x 1000 5.6 / 6.0, 20000 x 100 3.7 / 4.1;
-    // 2 rows: 20000 x 100 4.3 / 5.2, 16384 x 600 11.3 / 10.2, 8192 x 1000 7.9 / 6.3.
+    // 2 rows: 20000 x 100 3.8 / 5.2, 30000 x 256 6.4 / 8.9, 16384 x 600 9.9 / 9.9, 8192 x 1000 7.1 / 6.0.
     const bool whole = M > 2 || N >= (M == 1 ? 2048 : 512);
+    // Two blocks per SM hold all of a step's loads, three fewer of them and take 1.4 times as long a round: three where they save
+    // rounds all the same, or where a block of up to two rows has little more than a step to do.  us at 1 / 2 / 3 / 4 / 5 rows, two /
+    // three blocks: 4864 x 4864 (1.03 rounds of two blocks) 17.7/20.5/21.2/23.0/25.9 / 15.1/16.3/17.7/20.5/20.5, 5000 x 1000 (1.06)
+    // 3.7/4.3/5.8/6.8/7.2 / 3.2/3.8/4.6/5.8/6.0, 7100 x 4096 (1.5) 17.3/19.8/20.2/21.8/24.1 / 17.6/19.3/20.4/22.0/20.5, 8192 x 1000
+    // (1.73) 5.5/6.0/7.1/7.9/8.5 / 5.7/6.7/8.2/10.0/11.0, 20000 x 1500 (4.2) 18.2/20.2/21.9/24.0/25.4 / 16.5/18.3/20.4/22.7/24.0,
+    // 32000 x 1024 (6.8) 16.6/19.7/20.8/22.4/24.0 / 17.7/20.3/22.1/25.8/26.0; 2 rows x 50000 x 768 28.1 / 25.8.
+    const long long sms = device_sm_count();
+    const long long rounds2 = (blocks + 2 * sms - 1) / (2 * sms), rounds3 = (blocks + 3 * sms - 1) / (3 * sms);
+    const bool three = rounds3 * 14 < rounds2 * 10 || (M <= 2 && N < 1024 && rounds2 > 2);
     const int early = N * K >= kEarlyWeight ? 1 : 0;
     cudaError_t e = cudaErrorInvalidValue;
-#define MNI_SKINNY_DX(MT, LONG)                                                                        \
-    e = launch_dependent(dependent, skinny_dx_kernel<MT, LONG>, dim3(blocks), dim3(kDxThreads), 0, stream, dy, lddy, W, ldw, \
+#define MNI_SKINNY_DX(MT, LONG, BLOCKS)                                                                \
+    e = launch_dependent(dependent, skinny_dx_kernel<MT, LONG, BLOCKS>, dim3(blocks), dim3(kDxThreads), 0, stream, dy, lddy, W, ldw, \
                          dx, lddx, accumulate ? 1 : 0, N, K, early)
+#define MNI_SKINNY_DX_LONG(MT) if (three) MNI_SKINNY_DX(MT, true, 3); else MNI_SKINNY_DX(MT, true, 2)
     switch (M) {
-        case 1: if (whole) MNI_SKINNY_DX(1, true); else MNI_SKINNY_DX(1, false); break;
-        case 2: if (whole) MNI_SKINNY_DX(2, true); else MNI_SKINNY_DX(2, false); break;
-        case 3: MNI_SKINNY_DX(3, true); break;
-        case 4: MNI_SKINNY_DX(4, true); break;
-        case 5: MNI_SKINNY_DX(5, true); break;
-        case 6: MNI_SKINNY_DX(6, true); break;
-        case 7: MNI_SKINNY_DX(7, true); break;
-        case 8: MNI_SKINNY_DX(8, true); break;
+        case 1: if (!whole) MNI_SKINNY_DX(1, false, 4); else MNI_SKINNY_DX_LONG(1); break;
+        case 2: if (!whole) MNI_SKINNY_DX(2, false, 4); else MNI_SKINNY_DX_LONG(2); break;
+        case 3: MNI_SKINNY_DX_LONG(3); break;
+        case 4: MNI_SKINNY_DX_LONG(4); break;
+        case 5: MNI_SKINNY_DX_LONG(5); break;
+        case 6: MNI_SKINNY_DX(6, true, 2); break;
+        case 7: MNI_SKINNY_DX(7, true, 2); break;
+        case 8: MNI_SKINNY_DX(8, true, 2); break;
         default: return fail(MNI_B200_ERR_ARG, "skinny dx handles at most 8 rows");
     }
+#undef MNI_SKINNY_DX_LONG
 #undef MNI_SKINNY_DX
     if (e != cudaSuccess) return fail(MNI_B200_ERR_CUDA, "skinny_dx_kernel launch failed: %s", cudaGetErrorString(e));
     MNI_LAUNCH_CHECK("skinny_dx_kernel");

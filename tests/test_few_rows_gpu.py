@@ -103,10 +103,11 @@ def test_weight_written_by_the_kernel_before(F, m, k, n):
         assert rel_fro(y.tensor.numpy(), want) <= regression_bound_3xtf32(k), turn
 
 
-@pytest.mark.parametrize("k,n", [(4097, 2048), (33, 2052), (35, 508), (31, 516), (2, 2044), (16, 4), (2100, 4100)])
+@pytest.mark.parametrize("k,n", [(4097, 2048), (33, 2052), (35, 508), (31, 516), (2, 2044), (16, 4), (2100, 4100), (4741, 2052), (9490, 516)])
 @pytest.mark.parametrize("m", range(1, 9))
 def test_input_gradient_steps_and_what_is_left_of_a_row(F, m, k, n):
-    """Each row count's own kernel: whole steps of 512 columns, none, a last part; odd weight rows; short and long rows."""
+    """Each row count's own kernel: whole steps of 512 columns, none, a last part; odd weight rows; short and long rows; two and
+    three blocks per SM."""
     rng = np.random.default_rng([m, k, n])
     x, dy, w = (rng.standard_normal(s).astype(np.float32) for s in ((m, k), (m, n), (k, n)))
     t = F.DeviceTensor.from_numpy
