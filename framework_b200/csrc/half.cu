@@ -8,7 +8,8 @@
 //   - an element beyond 2^15 after scaling, an infinity or a NaN;
 //   - a stretch of a row (256 elements) or of a column (what a block takes of it in one matrix) in which more than a fifth of the
 //     elements are smaller than 2^-14, zeros not counted: in its row or column of the product the bits they lose could be the
-//     leading ones, where the stretch has nothing else as well as where the rest of it meets zeros.
+//     leading ones, where the stretch has nothing else as well as where the rest of it meets zeros;
+//   - 64 columns of what a block takes of a matrix with more than 16 small elements that are more than a sixteenth of all.
 // So a small element that stays has four times as many ordinary ones beside it, in its row and in its column.  It carries an
 // absolute error of 2^-43 (2^-31 without lo) of the largest sample.  Of normally distributed elements one in 6e5 is small: two of
 // a stretch's first ten do not come about by chance.
@@ -131,10 +132,16 @@ split_half_kernel(const __grid_constant__ ViewList list) {
                 shared[group][tc * 8 + c] = __half2uint_rz(o) | __half2uint_rz(f) << 16;
             }
             __syncthreads();
+            unsigned smalls = 0, others = 0;
             for (int c = threadIdx.x; c < kTileCols; c += kThreads) {
                 const unsigned n = shared[0][c] + shared[1][c] + shared[2][c] + shared[3][c];      // at most 8192 each
                 if (kOrdinary * (n >> 16) > (n & 0xffffu)) bad |= kUnfit;
+                smalls += n >> 16;
+                others += n & 0xffffu;
             }
+            smalls = __reduce_add_sync(0xffffffffu, smalls);
+            others = __reduce_add_sync(0xffffffffu, others);
+            if (smalls > 16 + (smalls + others) / 16) bad |= kUnfit;
         }
     };
     auto end_strip = [&] {
