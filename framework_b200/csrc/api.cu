@@ -518,7 +518,9 @@ struct Halves {
     }
 };
 
-// Whether a call may be computed from 16-bit planes, and is large enough for it to be worth finding out whether that pays.
+// Whether a call may be computed from 16-bit planes, and is large enough for it to be worth finding out whether that pays.  Below
+// the line it seldom does; f32 operands / planes, us: forward 1280^3 30 / 38, 1024 x 768 x 3072 32 / 34, 1536^3 38 / 45; backward
+// 1280^3 46 / 47, 1024 x 3072 x 768 43 / 57, 8192 x 256 x 1024 44 / 62, but 1536^3 64 / 56 and 1000 x 1333 x 2777 113 / 89.
 constexpr double kHalfWork = 4.0e9;                // M * N * K of its products
 bool half_possible(const Call &c, double work) {
     const uint32_t forced = MNI_B200_FORCE_TENSOR_PATH | MNI_B200_FORCE_SKINNY_PATH | MNI_B200_FORCE_PACK;
@@ -530,8 +532,10 @@ bool half_possible(const Call &c, double work) {
 // Measured with f32 operands / 16-bit planes, us, in a loop: forward 2048 x 768 x 3072 56 / 63, 2048^3 67 / 68, 8192 x 768 x 3072
 // 142 / 131, 4096 x 1024 x 4096 133 / 110, 4096^3 516 / 339, 1024 x 8192 x 1024 70 / 83, 8192 x 8192 x 512 252 / 282; backward
 // 2048 x 768 x 3072 113 / 107, 2048^3 133 / 107, 8192 x 768 x 3072 322 / 242, 4096^3 1071 / 612, 512 x 4096 x 4096 144 / 147;
-// single pass forward 3072^3 79 / 80, 4096^3 219 / 159, backward 162 / 128, 440 / 258.  MNI_B200_HALF=0 / 1: never / wherever it
-// can be done.
+// single pass forward 3072^3 79 / 80, 4096^3 219 / 159, backward 162 / 128, 440 / 258.  Near the line, with three sets of operands
+// in turn: backward 2048 x 1024 x 2048 77 / 69, 2048^2 x 1024 78 / 74, 2048 x 3072 x 768 88 / 84, 4096 x 512 x 2048 82 / 77, 3000 x
+// 700 x 2000 96 / 79, 1500 x 1024 x 4096 118 / 96.  That is at the clocks the power cap leaves; in the first 2 ms after a pause
+// the same six take 66 / 68, 67 / 74, 74 / 85, 70 / 77, 84 / 78, 101 / 92.  MNI_B200_HALF=0 / 1: never / wherever it can be done.
 bool half_pays(const Call &c, double f32_us, double half_us, double elements) {
     const int env = env_int("MNI_B200_HALF", -1);
     if (env >= 0) return env > 0;
@@ -905,7 +909,7 @@ bool bwd_half_wanted(const Call &c, const Shapes &s, const mni_b200_view &a, con
         p.fast_tf32 = (c.flags & MNI_B200_PRECISION_TF32) != 0;
         f32_us += gemm_estimate_us(p, all);
         gathers_us += gather_us(other);
-        beside_us = std::max(beside_us, 1.25 * gemm_estimate_us(p, halved));   // beside one another they are that much slower
+        beside_us = std::max(beside_us, 1.25 * gemm_estimate_us(p, halved));   // beside one another they are that much slower (half_pays)
         elements += static_cast<double>(prod(other.shape, other.ndim));
         return true;
     };

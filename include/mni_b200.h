@@ -30,6 +30,7 @@
  *     kernels can run at the same time on one device (different streams with no
  *     event between them) race on them.  Keep a device's calls on one stream --
  *     what the reference does (device.rs:37) -- or order the streams with events.
+ *     Nearly every large product uses the scratch (see mni_b200_workspace_set).
  *     The library's own side stream is forked from and joined to the caller's
  *     stream inside one call and never overlaps the next call's kernels.
  */
@@ -263,14 +264,17 @@ MNI_B200_API int mni_b200_contiguous(const mni_b200_view *src, float *dst, void 
  * CUDA graphs.  Every call may be recorded by a capturing stream (the side stream
  * is forked and joined with events, which capture follows).  The recorded nodes
  * hold the scratch address of the moment; a library-owned buffer that is outgrown
- * later is kept for them until mni_b200_release.  It cannot grow during a capture
- * (the call then fails with MNI_B200_ERR_WORKSPACE and records nothing): a caller
+ * later is kept for them until mni_b200_release.  It cannot grow during a capture:
+ * a large product then goes on without the planes of the next paragraph, any other
+ * call fails with MNI_B200_ERR_WORKSPACE and records nothing.  A caller
  * that replays graphs hands the library a buffer of the queried size with
  * mni_b200_workspace_set and keeps it for the graph's life, or runs each captured
  * call once beforehand.
  *
  * Large products are computed from 16-bit planes of their operands in scratch, 6
- * bytes an operand element (4 with MNI_B200_PRECISION_TF32).  Where that cannot be
+ * bytes an operand element (4 with MNI_B200_PRECISION_TF32).  The library's own
+ * buffer is a quarter larger than the largest call needed and stays until
+ * mni_b200_release.  Where the planes cannot be
  * had -- a smaller buffer was given, no memory is left, a capture may not grow it --
  * the call computes them from the f32 operands instead, which needs what it did
  * before and takes longer; it does not fail for it.  The planes keep 22 bits of an
